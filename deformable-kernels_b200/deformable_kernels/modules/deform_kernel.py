@@ -80,7 +80,7 @@ class GlobalDeformKernel2d(nn.Module):
         n, c, h, w = x.shape
         if self._fused_head_ok(x):
             # pool, coordinate head, bank sampling and the per-plane scale in one call each way
-            return global_dk_scale(x, self.weight.view(c, *self.weight_shape), self.fc.weight, self.fc.bias, self._tap_bias)
+            return global_dk_scale(x, self.weight, self.fc.weight, self.fc.bias, self._tap_bias)
         weight = self.dynamic_weight(x, self.weight).to(x.dtype)
         if self._is_plane_scale() and x.is_cuda:
             # 1x1 depthwise: the per-sample grouped convolution is a per-plane scale
