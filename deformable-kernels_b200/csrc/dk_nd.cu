@@ -25,8 +25,19 @@ __global__ void nd_fwd_kernel(const T* __restrict__ data, const T* __restrict__ 
   st<T, A>(out + tid, v);
 }
 
-// grad wrt the array, gather form: one thread per (channel, cell) walks the batch and adds
-// grad_out[b, c] * (product over dimensions of the hat weight of this cell).
+// grad wrt the array: a cluster of blocks per 32 channels (nd_accumulate_bank)
+template <typename T>
+__global__ void __launch_bounds__(256) nd_bwd_data_cluster_kernel(const T* __restrict__ dy, const T* __restrict__ coord,
+                                                                  T* __restrict__ ddata, int B, int C, int D, int prod,
+                                                                  const NdShape sh) {
+  using A = typename Compute<T>::type;
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  nd_accumulate_bank<T, A, true>(reinterpret_cast<A*>(smem_raw), dy, coord, ddata, blockIdx.x % kNdCluster,
+                                 blockIdx.x / kNdCluster * 32, B, C, D, prod, sh);
+}
+
+// The same in gather form, for arrays whose accumulators do not fit in shared memory: one thread per (channel, cell)
+// walks the batch and adds grad_out[b, c] * (product over dimensions of the hat weight of this cell).
 template <typename T>
 __global__ void nd_bwd_data_kernel(const T* __restrict__ dy, const T* __restrict__ coord, T* __restrict__ ddata, int B,
                                    int C, int D, int prod, const NdShape sh) {
@@ -135,6 +146,11 @@ int nd_forward(const T* data, const T* coord, T* out, int B, int C, int D, int p
 template <typename T>
 int nd_backward_data(const T* dy, const T* coord, T* ddata, int B, int C, int D, int prod, const NdShape& sh,
                      cudaStream_t s) {
+  using A = typename Compute<T>::type;
+  const int warps = nd_acc_warps<A>(prod, B);
+  if (warps > 0)
+    return launch_nd_clusters(nd_bwd_data_cluster_kernel<T>, (unsigned)((C + 31) / 32), 32 * warps,
+                              (size_t)warps * prod * 32 * sizeof(A), s, dy, coord, ddata, B, C, D, prod, sh);
   unsigned grid;
   if (!grid_1d((long long)C * prod, 128, &grid)) return DK_ERR_UNSUPPORTED;
   nd_bwd_data_kernel<T><<<grid, 128, 0, s>>>(dy, coord, ddata, B, C, D, prod, sh);
