@@ -1,5 +1,6 @@
 // extern "C" surface of the library (see include/dk_b200.h): argument checks, dtype
 // dispatch, workspace carving.  No allocation, no synchronisation, no printing.
+#include <atomic>
 #include <mutex>
 
 #include "dk_common.cuh"
@@ -43,6 +44,40 @@ const DevAttr& attrs() {
   return a;
 }
 }  // namespace
+
+int raise_smem_limit(const void* kernel, size_t bytes) {
+  // open addressing over (kernel, device) keys that are never removed; a full neighbourhood only means asking the driver
+  // again.  `granted` is raised after the driver agreed, so a reader never sees more than is set.
+  struct Slot {
+    std::atomic<uint64_t> key{0};
+    std::atomic<size_t> granted{0};
+  };
+  static Slot table[1024];
+  int dev = 0;
+  cudaGetDevice(&dev);
+  const uint64_t key = (uint64_t)reinterpret_cast<uintptr_t>(kernel) * 64 + (unsigned)(dev & 63) + 1;
+  Slot* slot = nullptr;
+  for (uint64_t h = (key * 0x9e3779b97f4a7c15ull) >> 54, probe = 0; probe < 8; ++probe) {
+    Slot& t = table[(h + probe) & 1023];
+    uint64_t seen = t.key.load(std::memory_order_acquire);
+    if (seen == 0 && t.key.compare_exchange_strong(seen, key)) seen = key;
+    if (seen == key) {
+      slot = &t;
+      break;
+    }
+  }
+  if (slot && dev < 64 && slot->granted.load(std::memory_order_acquire) >= bytes) return DK_OK;
+  static std::mutex raise_mutex;
+  std::lock_guard<std::mutex> lock(raise_mutex);
+  if (slot && dev < 64 && slot->granted.load() >= bytes) return DK_OK;  // the limit is never lowered below another thread's
+  const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
+  if (e != cudaSuccess) {
+    set_last_cuda_error(e);
+    return DK_ERR_CUDA;
+  }
+  if (slot && dev < 64) slot->granted.store(bytes, std::memory_order_release);
+  return DK_OK;
+}
 
 int device_smem_optin() { return attrs().smem_optin; }
 int device_sm_count() { return attrs().sms; }

@@ -151,16 +151,12 @@ int check_launch();
 int device_smem_optin();  // max dynamic shared memory per block (opt-in), cached per device
 int device_sm_count();
 
+// Raises the kernel's dynamic shared-memory limit on the current device to `bytes`.  The driver is asked once per (kernel,
+// device, larger size): the call costs about as much host time as the launch itself.
+int raise_smem_limit(const void* kernel, size_t bytes);
 template <typename K>
 inline int enable_smem(K kernel, size_t bytes) {
-  if (bytes > 48 * 1024) {
-    cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
-    if (e != cudaSuccess) {
-      set_last_cuda_error(e);
-      return DK_ERR_CUDA;
-    }
-  }
-  return DK_OK;
+  return bytes > 48 * 1024 ? raise_smem_limit(reinterpret_cast<const void*>(kernel), bytes) : DK_OK;
 }
 
 // typed launchers implemented in dk_local.cu / dk_deform.cu / dk_nd.cu

@@ -442,13 +442,13 @@ Tensor plane_scale(const Tensor& input, const Tensor& scale) {
 
 struct GlobalDKScaleBackward : public Node {
   SavedVariable input, bank, fc_weight;
-  Tensor pooled, raw, coord, scale;  // not visible outside: no version to check
+  Tensor kept;  // pooled [N,C], scale [N,C], raw and coord [N,D], one after the other; not visible outside: no version to check
   int64_t first_dim = 1;             // where the bank's sampled dimensions start
 
   variable_list apply(variable_list&& grads) override {
     at::NoGradGuard no_grad;
     const Tensor x = input.unpack(), b = bank.unpack(), fw = fc_weight.unpack();
-    TORCH_CHECK(pooled.defined(), "Trying to backward through the graph a second time");
+    TORCH_CHECK(kept.defined(), "Trying to backward through the graph a second time");
     const c10::DeviceGuard guard(x.device());
     const Tensor dy = arrived(grads, x.sizes(), x);
     const NdShape sh = nd_shape(b, first_dim);
@@ -460,7 +460,9 @@ struct GlobalDKScaleBackward : public Node {
     if (task_should_compute_output(3)) dfb = empty_of(x, {sh.dims}, at::kFloat);
     const size_t bytes = lib.dk_global_dk_backward_workspace_bytes(n, c, sh.dims);
     Tensor ws = workspace(bytes, x);
-    check(lib.dk_global_dk_backward(cptr(dy), cptr(x), cptr(b), cptr(fw), cptr(pooled), cptr(raw), cptr(coord), cptr(scale),
+    const float* pooled = kept.const_data_ptr<float>();
+    const float *scale = pooled + (int64_t)n * c, *raw = scale + (int64_t)n * c, *coord = raw + (int64_t)n * sh.dims;
+    check(lib.dk_global_dk_backward(cptr(dy), cptr(x), cptr(b), cptr(fw), pooled, raw, coord, scale,
                                     mptr(dx), mptr(db), mptr(dfw), mptr(dfb), n, c, hw, sh.dims, sh.s.data(), dtype_code(x),
                                     mptr(ws), bytes, stream_of(x)),
           "global_dk_scale backward");
@@ -469,7 +471,7 @@ struct GlobalDKScaleBackward : public Node {
   std::string name() const override { return "GlobalDKScaleFunctionBackward"; }
   void release_variables() override {
     input.reset_data(), bank.reset_data(), fc_weight.reset_data();
-    pooled.reset(), raw.reset(), coord.reset(), scale.reset();
+    kept.reset();
   }
 };
 
@@ -490,7 +492,7 @@ Tensor global_dk_scale(const Tensor& input, const Tensor& bank, const Tensor& fc
                     "expected fc_weight [dims, C], fc_bias [dims], tap_bias [dims]");
   const int code = dtype_code(input);
   const bool grad = wants_grad({&input, &bank, &fc_weight, &fc_bias});
-  Tensor out, x, b, fw, pooled, raw, coord, scale;
+  Tensor out, x, b, fw, kept;
   {
     at::NoGradGuard no_grad;
     const c10::DeviceGuard guard(input.device());
@@ -498,19 +500,20 @@ Tensor global_dk_scale(const Tensor& input, const Tensor& bank, const Tensor& fc
     const Tensor fb = fc_bias.contiguous(), tb = tap_bias.contiguous();
     const int64_t n = x.size(0), c = x.size(1);
     out = empty_as(x, x.sizes());
-    pooled = empty_of(x, {n, c}, at::kFloat), scale = empty_of(x, {n, c}, at::kFloat);
-    raw = empty_of(x, {n, dims}, at::kFloat), coord = empty_of(x, {n, dims}, at::kFloat);
+    kept = empty_of(x, {2 * n * (c + dims)}, at::kFloat);
+    float* pooled = kept.mutable_data_ptr<float>();
+    float *scale = pooled + n * c, *raw = scale + n * c, *coord = raw + n * dims;
     const NdShape sh = nd_shape(b, first);
-    check(lib.dk_global_dk_forward(cptr(x), cptr(b), cptr(fw), cptr(fb), cptr(tb), mptr(out), mptr(pooled), mptr(raw),
-                                   mptr(coord), mptr(scale), as_int(n), as_int(c), as_int(x.size(2) * x.size(3)), sh.dims,
-                                   sh.s.data(), code, stream_of(x)),
+    check(lib.dk_global_dk_forward(cptr(x), cptr(b), cptr(fw), cptr(fb), cptr(tb), mptr(out), pooled, raw, coord, scale,
+                                   as_int(n), as_int(c), as_int(x.size(2) * x.size(3)), sh.dims, sh.s.data(), code,
+                                   stream_of(x)),
           "global_dk_scale forward");
   }
   if (grad) {
     auto node = std::make_shared<GlobalDKScaleBackward>();
     node->set_next_edges(collect_next_edges(input, bank, fc_weight, fc_bias, tap_bias));
     node->input = SavedVariable(x, false), node->bank = SavedVariable(b, false), node->fc_weight = SavedVariable(fw, false);
-    node->pooled = pooled, node->raw = raw, node->coord = coord, node->scale = scale;
+    node->kept = kept;
     node->first_dim = first;
     torch::autograd::set_history(out, node);
   }
