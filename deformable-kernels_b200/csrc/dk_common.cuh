@@ -201,6 +201,10 @@ bool local_bwd_ring_preferred(const Geom& g);  // the one-pass backward is expec
 int local_bwd_ring(const __half* dy, const __half* x, const __half* rot, const __half* w, __half* dx, __half* drot, __half* dw,
                    const Geom& g, void* ws, size_t ws_bytes, cudaStream_t s);  // all three gradients in one pass
 int ring_error_status();
+// tcgen05 kernels (dk_local_tc.cu), fp16 and fp32; DK_ERR_UNSUPPORTED = shape outside them
+template <typename T>
+int local_conv_tc(const T* src, const T* rot, const T* w, T* dst, const Geom& g, bool transposed, cudaStream_t s);
+int tc_error_status();
 size_t local_rot_mma_workspace(const Geom& g);
 int local_rot_mma(const __half* dy, const __half* x, const __half* rot, const __half* w, __half* drot, const Geom& g,
                   void* ws, size_t ws_bytes, cudaStream_t s);

@@ -139,6 +139,13 @@ static int launch_local_conv(const T* src, const T* rot, const T* w, T* dst, con
       if (rc != DK_ERR_UNSUPPORTED) return rc;
     }
   }
+  // fp32, and fp16 with channel counts the mma.sync kernels do not take (no multiple of 16)
+  if constexpr (sizeof(T) <= 4) {
+    if (mma_path_enabled()) {
+      const int rc = local_conv_tc<T>(src, rot, w, dst, g, TRANSPOSED, s);
+      if (rc != DK_ERR_UNSUPPORTED) return rc;
+    }
+  }
   const long long total = (long long)g.N * (TRANSPOSED ? g.HW : g.P);
   // 16 channels per thread amortise the sampling basis of a (pixel, tap); a call too small to fill the GPU that way
   // (under two blocks per SM) takes 4 channels per thread and blocks of 64 instead: four times the threads, a quarter

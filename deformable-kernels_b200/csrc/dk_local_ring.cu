@@ -46,6 +46,45 @@ int launch_reduce_rot_partials(const float* partial, __half* out, size_t n_out, 
 
 namespace {
 
+typedef CUresult (*EncodeTiledFn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*, const cuuint64_t*,
+                                  const cuuint32_t*, const cuuint32_t*, CUtensorMapInterleave, CUtensorMapSwizzle,
+                                  CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
+
+// The driver's tensor-map encoder, looked up through the runtime (the library links no driver library).
+EncodeTiledFn encode_tiled() {
+  static EncodeTiledFn fn = [] {
+    void* ptr = nullptr;
+    cudaDriverEntryPointQueryResult q = cudaDriverEntryPointSymbolNotFound;
+    if (cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &ptr, cudaEnableDefault, &q) != cudaSuccess ||
+        q != cudaDriverEntryPointSuccess)
+      ptr = nullptr;
+    (void)cudaGetLastError();
+    return reinterpret_cast<EncodeTiledFn>(ptr);
+  }();
+  return fn;
+}
+
+}  // namespace
+
+namespace ring {
+bool make_plane_row_map(CUtensorMap* tm, const void* base, int elem, int width, int rows, long long planes, int box_w,
+                        int box_planes) {
+  EncodeTiledFn enc = encode_tiled();
+  if (!enc) return false;
+  if ((reinterpret_cast<uintptr_t>(base) & 15) || (width * elem & 15) || box_w > 256 || box_planes > 256 || (box_w * elem & 15))
+    return false;
+  const cuuint64_t dims[3] = {(cuuint64_t)width, (cuuint64_t)rows, (cuuint64_t)planes};
+  const cuuint64_t strides[2] = {(cuuint64_t)width * elem, (cuuint64_t)width * rows * elem};
+  const cuuint32_t box[3] = {(cuuint32_t)box_w, 1u, (cuuint32_t)box_planes};
+  const cuuint32_t estr[3] = {1u, 1u, 1u};
+  return enc(tm, elem == 2 ? CU_TENSOR_MAP_DATA_TYPE_FLOAT16 : CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 3, const_cast<void*>(base), dims,
+             strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
+             CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
+}
+}  // namespace ring
+
+namespace {
+
 constexpr int kErrTimeout = 1;
 
 // Zero-initialised by the loader; set when a bounded wait ran out (see dk_ring.cuh).
@@ -1369,37 +1408,8 @@ __global__ void __launch_bounds__(MAXT, 1) ring_bwd_kernel(const __grid_constant
 }
 
 // ------------------------------------------------------------------ host side
-typedef CUresult (*EncodeTiledFn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*, const cuuint64_t*,
-                                  const cuuint32_t*, const cuuint32_t*, CUtensorMapInterleave, CUtensorMapSwizzle,
-                                  CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
-
-// The driver's tensor-map encoder, looked up through the runtime (the library links no driver library).
-EncodeTiledFn encode_tiled() {
-  static EncodeTiledFn fn = [] {
-    void* ptr = nullptr;
-    cudaDriverEntryPointQueryResult q = cudaDriverEntryPointSymbolNotFound;
-    if (cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &ptr, cudaEnableDefault, &q) != cudaSuccess ||
-        q != cudaDriverEntryPointSuccess)
-      ptr = nullptr;
-    (void)cudaGetLastError();
-    return reinterpret_cast<EncodeTiledFn>(ptr);
-  }();
-  return fn;
-}
-
-// fp16 planes [planes][rows][width] viewed as a rank-3 tensor; one box = `box_w` halves of one row of
-// `box_planes` consecutive planes.  Elements outside the tensor are delivered as zeros.
 bool make_row_map(CUtensorMap* tm, const __half* base, int width, int rows, long long planes, int box_w, int box_planes) {
-  EncodeTiledFn enc = encode_tiled();
-  if (!enc) return false;
-  if ((reinterpret_cast<uintptr_t>(base) & 15) || (width & 7) || box_w > 256 || box_planes > 256 || (box_w & 7)) return false;
-  const cuuint64_t dims[3] = {(cuuint64_t)width, (cuuint64_t)rows, (cuuint64_t)planes};
-  const cuuint64_t strides[2] = {(cuuint64_t)width * 2, (cuuint64_t)width * rows * 2};
-  const cuuint32_t box[3] = {(cuuint32_t)box_w, 1u, (cuuint32_t)box_planes};
-  const cuuint32_t estr[3] = {1u, 1u, 1u};
-  return enc(tm, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 3, const_cast<__half*>(base), dims, strides, box, estr,
-             CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
-             CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
+  return make_plane_row_map(tm, base, 2, width, rows, planes, box_w, box_planes);
 }
 
 // Input widths the kernels are instantiated for; scope 4 x 4.  The kernels themselves take any width: rows that are not
@@ -1885,7 +1895,7 @@ int local_ring_plan_query(const Geom& g, int pass, long long out[8]) {
 int ring_error_status() {
   int v = 0;
   if (cudaMemcpyFromSymbol(&v, g_ring_error, sizeof(int)) != cudaSuccess) return -1;
-  return v;
+  return v ? v : tc_error_status();
 }
 
 // forward (transposed = false) or grad-input (transposed = true); DK_ERR_UNSUPPORTED = not a ring shape

@@ -1,0 +1,935 @@
+// Local deformable kernel on the fifth-generation tensor cores (tcgen05 + TMEM), fp16 and fp32 storage.
+//
+// The resampled kernel is a contraction with hat products, K[c, p, tap] = sum_cell W[c, cell] * beta[p, tap, cell]
+// (dk_local_mma.cu).  Here the channels are the 128 rows of a tcgen05.mma: W stays in TMEM, the hat products of a step's 64
+// pixels and the three taps of one kernel row are the 192 columns in shared memory, and the result is read back one channel
+// per lane.  A lane then owns 8 consecutive pixels of ONE channel: its source window is one 16-byte shared-memory load per
+// row plus the two edge values, shared by nine taps.
+//
+// With mma.sync fragments (8 channels x 2 pixels per lane) the same step executes 166 warp-instructions per 128 outputs: 27
+// loads of 4 bytes, 45 for the hat products that every warp builds for itself, 9 mma, 36 multiply-adds, 30 for indices and
+// waits.  Here hat products are built once per block by warps of their own, the mma are issued by one warp, and a consumer
+// warp is left with 72 multiply-adds, 15 loads and the stores per 256 outputs.
+//
+// fp16: K leaves the tensor cores rounded to fp16 (relative 2^-11, like the tensors themselves) and meets x in the
+// mixed-precision multiply-add (exact product, fp32 sum), as in dk_local_ring.cu.
+// fp32: W and the hat products are split into two fp16 pieces each, scaled by powers of two so that no piece is subnormal
+// (W per channel, the hat products by 2^15); the four products of the pieces, summed in fp32, are exact to 2^-23 of the
+// channel's largest bank value, like the four fp32 products and additions it replaces.
+//
+// A block walks through a contiguous range of 8-pixel segments of the destination rows (sample, row, column octet, in
+// memory order) for up to CG channels; 8 segments are a step.  Roles:
+//   16 consumer warps  team j (4 warps, one per quarter of the TMEM lanes) takes segments 2j, 2j + 1 of every step: waits
+//                      for the accumulators of one kernel row, multiplies, leaves the results in shared memory
+//   1 MMA warp         issues the tcgen05.mma, two sets of accumulators
+//   1 or 3 loaders     source rows through a ring of row slots: TMA where rows are multiples of 16 bytes (out-of-range
+//                      elements arrive as zeros = the convolution padding), else cp.async pieces or elements, 3 warps
+//   6 or 4 beta warps  lane = destination pixel: 18 offsets, nine taps of 16 hat products, written as the B operand
+//   4 or 6 store warps results of a step from shared memory, consecutive pixels on consecutive lanes (written straight from
+//                      the consumers' registers, one channel per lane, every store touches 32 lines)
+// Every hand-over is an mbarrier used once per step (or per set of accumulators) by the same warps, in order.
+#include <cstring>
+#include <type_traits>
+
+#include "dk_tc.cuh"
+
+namespace dk {
+
+using namespace ring;
+using namespace tc;
+using mma::hat;
+
+namespace {
+
+__device__ int g_tc_error;  // set when a bounded wait ran out
+
+constexpr int kTeams = 4;
+constexpr int kConsumers = 16;
+constexpr int kHelpers = 12;  // MMA, loaders, hat products, stores
+constexpr int kThreads = 32 * (kConsumers + kHelpers);
+// registers: 72 per thread at launch, then 88 for the four consumer warpgroups and 48 for the three of the helpers
+constexpr int kRegsLaunch = 72, kRegsConsumer = 88, kRegsHelper = 48;
+static_assert(kConsumers * kRegsConsumer + kHelpers * kRegsHelper <= (kConsumers + kHelpers) * kRegsLaunch, "register shares");
+constexpr int kLoaders = 3;                         // warps that fetch rows without TMA
+constexpr int kStepSegs = 8;
+constexpr int kSlotCols = 48;                       // three taps x 16 pixels
+constexpr int kSetCols = kTeams * kSlotCols;        // one set of accumulators
+constexpr int kBankCol = 2 * kSetCols;              // the bank behind the two sets
+constexpr int kDepth = 4;                           // steps in flight, as seen by the row ring
+constexpr int kMaxBuf = 3;                          // buffers of hat products
+constexpr int kBars = 2 * kDepth + 2 * kMaxBuf + 6;
+constexpr int kPairRow = 6 * 256;                   // hat products of two segments and one kernel row: 48 columns x 32 bytes
+constexpr int kPiece = 3 * kTeams * kPairRow;       // of a step: [kernel row][pair][segment, tap: 8 columns][two halves of the cells]
+constexpr int kMinSmem = 120 * 1024;                // one block per SM: it takes all of TMEM
+
+// Hat products: two warps per step, each pair of warps with a buffer of its own, so that a warp sees every reuse of its buffer
+// (a barrier's phase can only be told from the one before it).
+template <typename T>
+__host__ __device__ constexpr int beta_warps(int loaders) {
+  return loaders == 1 && sizeof(T) == 2 ? 6 : 4;
+}
+
+enum Mode { kFwd1 = 0, kFwd2 = 1, kData1 = 2, kData2 = 3 };  // forward, grad-input; stride 1, 2
+
+struct ConvParams {
+  int N, C;
+  int Hs, Ws;  // source plane
+  int Hg, Wg;  // plane of the segments: destination (kData2: grad-output)
+  int Hd, Wd;  // destination plane
+  int Ho, Wo;  // plane of the offsets
+  int nseg;    // segments per row
+  int L;       // stream rows per sample
+  int R;       // slots in the row ring
+  int pitch;   // bytes per channel row in a slot: an odd multiple of 16
+  int CG;      // channels per block
+  int box_c;   // channels per TMA box
+  int full;    // quads of 32-channel groups
+  int rest;    // groups beyond them
+  int segs;    // N * Hg * nseg
+  int steps_per_cta;
+  unsigned magic_seg, magic_row;  // ceil(2^32 / nseg), ceil(2^32 / Hg)
+  int scW, cells;
+  float uh0, uw0;
+  int store;  // bytes per store of a result row: 16, 4 or 2
+};
+
+struct SegPos {
+  int n, g, s;
+};
+__device__ __forceinline__ SegPos seg_pos(int b, const ConvParams& p) {
+  SegPos r;
+  const int row = p.nseg == 1 ? b : (int)__umulhi((unsigned)b, p.magic_seg);
+  r.s = b - row * p.nseg;
+  r.n = p.Hg == 1 ? row : (int)__umulhi((unsigned)row, p.magic_row);
+  r.g = row - r.n * p.Hg;
+  return r;
+}
+
+template <int MODE> struct Walk {
+  static constexpr int S = MODE == kFwd2 ? 2 : 1;        // stream rows per segment row
+  static constexpr int rows = MODE == kData2 ? 2 : 3;    // stream rows a segment reads
+  static constexpr int first = MODE == kData2 ? 0 : -1;  // source row of a sample's first stream row
+  static constexpr int xs = MODE == kFwd2 ? 2 : 1;       // source columns per segment column
+};
+
+// ------------------------------------------------------------------ consumers' operands
+// One item = one segment (8 pixels) and one kernel row of the lane's channel: 24 kernel values (tap-major; pixels p and
+// p + 4 in adjacent columns) and the source window.
+template <typename T, int MODE> struct Item;
+
+template <int MODE> struct Item<__half, MODE> {
+  static constexpr int NW = MODE == kFwd2 ? 8 : 4;
+  unsigned k[12];        // fp16 pairs (p, p + 4)
+  unsigned w[NW];        // source columns 0 .. 7 (15) of the segment
+  unsigned left, right;  // columns -1 and 8
+  __device__ __forceinline__ void load(unsigned tmem, const char* row) {
+    ld24(k, tmem);
+    const __half* x = reinterpret_cast<const __half*>(row);
+#pragma unroll
+    for (int i = 0; i < NW / 4; ++i) {
+      const uint4 q = *reinterpret_cast<const uint4*>(x + 8 * i);
+      w[4 * i] = q.x, w[4 * i + 1] = q.y, w[4 * i + 2] = q.z, w[4 * i + 3] = q.w;
+    }
+    if (MODE != kData2) left = *reinterpret_cast<const unsigned short*>(x - 1);
+    if (MODE != kFwd2) right = *reinterpret_cast<const unsigned short*>(x + 8);
+  }
+  // a += source column I * half KH of kk
+  template <int I, int KH> __device__ __forceinline__ void mac(float& a, unsigned kk) const {
+    if constexpr (I < 0) mma::fma_hh<0, KH>(a, left, kk);
+    else if constexpr (I >= 2 * NW) mma::fma_hh<0, KH>(a, right, kk);
+    else mma::fma_hh<I & 1, KH>(a, w[I / 2], kk);
+  }
+  template <int LO, int HI, int Q> __device__ __forceinline__ void tap(float& a, float& b) const {
+    mac<LO, 0>(a, k[Q]);
+    mac<HI, 1>(b, k[Q]);
+  }
+};
+
+template <int MODE> struct Item<float, MODE> {
+  static constexpr int NW = MODE == kFwd2 ? 16 : 8;
+  unsigned k[24];
+  float w[NW], left, right;
+  __device__ __forceinline__ void load(unsigned tmem, const char* row) {
+    ld24(k, tmem);
+    const float* x = reinterpret_cast<const float*>(row);
+#pragma unroll
+    for (int i = 0; i < NW / 4; ++i) {
+      const float4 q = *reinterpret_cast<const float4*>(x + 4 * i);
+      w[4 * i] = q.x, w[4 * i + 1] = q.y, w[4 * i + 2] = q.z, w[4 * i + 3] = q.w;
+    }
+    if (MODE != kData2) left = x[-1];
+    if (MODE != kFwd2) right = x[8];
+  }
+  template <int I> __device__ __forceinline__ float at() const {
+    if constexpr (I < 0) return left;
+    else if constexpr (I >= NW) return right;
+    else return w[I];
+  }
+  template <int LO, int HI, int Q> __device__ __forceinline__ void tap(float& a, float& b) const {
+    a = fmaf(at<LO>(), __uint_as_float(k[2 * Q]), a);
+    b = fmaf(at<HI>(), __uint_as_float(k[2 * Q + 1]), b);
+  }
+};
+
+// acc += window * kernel row.  Source column of tap t and pixel p: p xs + t - 1 (kData2: p, and p + 1 for the third tap);
+// kData2 keeps the even destination columns in acc[0..8) and the odd ones in acc[8..16).
+template <typename T, int MODE, int N>
+__device__ __forceinline__ void multiply(float (&acc)[N], const Item<T, MODE>& it) {
+  constexpr int XS = Walk<MODE>::xs;
+  constexpr bool D = MODE == kData2;
+#define DK_TAP(t, p)                                                                                             \
+  it.template tap<D ? p + (t == 2) : p * XS + t - 1, D ? p + 4 + (t == 2) : (p + 4) * XS + t - 1, t * 4 + p>( \
+      acc[(D && t ? 8 : 0) + p], acc[(D && t ? 8 : 0) + p + 4]);
+#define DK_TAPS(t) DK_TAP(t, 0) DK_TAP(t, 1) DK_TAP(t, 2) DK_TAP(t, 3)
+  DK_TAPS(0) DK_TAPS(1) DK_TAPS(2)
+#undef DK_TAPS
+#undef DK_TAP
+}
+
+// `count` consecutive values v[0..count) of one channel row to global memory (kData2)
+template <typename T, int NV>
+__device__ __forceinline__ void store_row(T* __restrict__ d, const float (&v)[NV], int count, bool vec) {
+  constexpr int V = 16 / sizeof(T);
+#pragma unroll
+  for (int i = 0; i < NV; i += V) {
+    if (vec && count >= i + V) {
+      if constexpr (sizeof(T) == 2)
+        *reinterpret_cast<uint4*>(d + i) = make_uint4(mma::pack2(v[i], v[i + 1]), mma::pack2(v[i + 2], v[i + 3]),
+                                                      mma::pack2(v[i + 4], v[i + 5]), mma::pack2(v[i + 6], v[i + 7]));
+      else
+        *reinterpret_cast<float4*>(d + i) = make_float4(v[i], v[i + 1], v[i + 2], v[i + 3]);
+    } else {
+#pragma unroll
+      for (int k = i; k < i + V; ++k)
+        if (k < count) st<T, float>(d + k, v[k]);
+    }
+  }
+}
+
+// ------------------------------------------------------------------ bank in TMEM
+// A tiles: `full` quads of groups in order, then four variants of the remaining 1 to 3 groups.  Variant v puts them on the
+// quarters of the lanes (= consumer warps) that pair (v - step) mod 4 of a step uses, so that over four pairs every quarter
+// gets the same number of groups.  Index of the remaining group on quarter q, -1: none.
+__device__ __forceinline__ int rest_index(int rest, int v, int q) {
+  if (rest == 1) return q == v ? 0 : -1;
+  if (rest == 2) return (q >> 1) == (v & 1) ? (q & 1) : -1;
+  return q == v ? -1 : q - (q > v);
+}
+
+// the 16 cells of one channel as fp16 pieces: hi[8], lo[8] (two cells each); `inv` undoes the scaling of fp32 banks and of
+// the hat products they meet
+template <typename T>
+__device__ __forceinline__ void bank_pieces(unsigned (&hi)[8], unsigned (&lo)[8], float& inv, const T* __restrict__ w, int cells,
+                                            bool ok) {
+  float v[16];
+#pragma unroll
+  for (int i = 0; i < 16; ++i) v[i] = ok && i < cells ? ld<float>(w + i) : 0.f;
+  if constexpr (std::is_same<T, __half>::value) {
+#pragma unroll
+    for (int i = 0; i < 8; ++i) hi[i] = mma::pack2(v[2 * i], v[2 * i + 1]), lo[i] = 0;
+    inv = 1.f;
+  } else {
+    float top = 0.f;
+#pragma unroll
+    for (int i = 0; i < 16; ++i) top = fmaxf(top, fabsf(v[i]));
+    int e = 0;
+    if (top > 0.f && top < INFINITY) frexpf(top, &e);
+    const int shift = min(15 - e, 100);  // largest magnitude in [2^14, 2^15)
+    const float sc = ldexpf(1.f, shift);
+    inv = ldexpf(1.f, -15 - shift);
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+      const float a = v[2 * i] * sc, b = v[2 * i + 1] * sc;
+      hi[i] = mma::pack2(a, b);
+      lo[i] = mma::pack2(a - mma::lo2f(hi[i]), b - mma::hi2f(hi[i]));
+    }
+  }
+}
+
+// ------------------------------------------------------------------ hat products
+// Tap column t of kernel row v of segment pixel (g, x): the offsets' pixel (qh, qw) and the tap (fh, fw).
+template <int MODE>
+__device__ __forceinline__ void tap_of(int v, int t, int g, int x, int& qh, int& qw, int& fh, int& fw) {
+  if (MODE == kFwd1 || MODE == kFwd2) {
+    qh = g, qw = x, fh = v, fw = t;
+  } else if (MODE == kData1) {
+    qh = g + v - 1, qw = x + t - 1, fh = 2 - v, fw = 2 - t;
+  } else {  // 2 x 2 patch: (0, tap 1) -> even row; (0, tap 2), (1, tap 0) -> odd row; columns alike
+    qh = g + (v == 2), qw = x + (t == 2), fh = v == 0 ? 1 : (v == 1 ? 2 : 0), fw = t == 0 ? 1 : (t == 1 ? 2 : 0);
+  }
+}
+
+// 16 hat products of one tap: cells (2i, 2i + 1) in hi[i] (and, scaled by 2^15, the rest in lo[i] for fp32)
+template <bool SC44, bool SPLIT>
+__device__ __forceinline__ void hat_products(unsigned (&hi)[8], unsigned (&lo)[8], float u, float v, bool ok, int scW, int cells) {
+  float b[16];
+  if (SC44) {
+    float hu[4], hv[4];
+#pragma unroll
+    for (int a = 0; a < 4; ++a) {
+      hu[a] = ok ? hat(u - (float)a) : 0.f;
+      hv[a] = hat(v - (float)a);
+      if (SPLIT) hu[a] *= 32768.f;
+    }
+    const uint64_t v01 = pack_f2(hv[0], hv[1]), v23 = pack_f2(hv[2], hv[3]);
+#pragma unroll
+    for (int a = 0; a < 4; ++a) {
+      const uint64_t uu = pack_f2(hu[a], hu[a]);
+      const float2 r = unpack_f2(mul2(uu, v01)), q = unpack_f2(mul2(uu, v23));
+      b[4 * a] = r.x, b[4 * a + 1] = r.y, b[4 * a + 2] = q.x, b[4 * a + 3] = q.y;
+    }
+  } else {
+    int a = 0, c = 0;
+#pragma unroll
+    for (int i = 0; i < 16; ++i) {
+      b[i] = ok && i < cells ? hat(u - (float)a) * hat(v - (float)c) * (SPLIT ? 32768.f : 1.f) : 0.f;
+      if (++c == scW) c = 0, ++a;
+    }
+  }
+#pragma unroll
+  for (int i = 0; i < 8; ++i) {
+    hi[i] = mma::pack2(b[2 * i], b[2 * i + 1]);
+    if (SPLIT) lo[i] = mma::pack2(b[2 * i] - mma::lo2f(hi[i]), b[2 * i + 1] - mma::hi2f(hi[i]));
+  }
+}
+
+__device__ __forceinline__ void sts16(unsigned a, unsigned x, unsigned y, unsigned z, unsigned w) {
+  asm volatile("st.shared.v4.b32 [%0], {%1,%2,%3,%4};\n" ::"r"(a), "r"(x), "r"(y), "r"(z), "r"(w) : "memory");
+}
+
+// The offsets of one pixel as they lie in memory: nine (vertical, horizontal) pairs; absent ones read as zero.
+template <typename T> struct Offsets {
+  T r[9][2];
+  unsigned ok;  // taps whose offsets exist
+};
+
+// one beta warp: half a step (32 pixels, lane = pixel: segment lane / 8, column lane % 8)
+template <typename T, int MODE>
+__device__ __forceinline__ void fetch_offsets(Offsets<T>& o, const T* __restrict__ rot, int seg, int hi_seg, const ConvParams& p,
+                                              int lane) {
+  const int b = seg + (lane >> 3);
+  const SegPos sp = seg_pos(min(b, hi_seg - 1), p);
+  const int x = sp.s * 8 + (lane & 7), P = p.Ho * p.Wo;
+  const bool live = b < hi_seg && x < p.Wg;
+  const T* rn = rot + (size_t)sp.n * 18 * P;
+  o.ok = 0;
+#pragma unroll
+  for (int i = 0; i < 9; ++i) {
+    int qh, qw, fh, fw;
+    tap_of<MODE>(i / 3, i % 3, sp.g, x, qh, qw, fh, fw);
+    const bool ok = live && qh >= 0 && qh < p.Ho && qw >= 0 && qw < p.Wo;
+    o.ok |= (unsigned)ok << i;
+    const T* a = rn + ((fh * 3 + fw) * 2) * P + qh * p.Wo + qw;
+    o.r[i][0] = ok ? __ldg(a) : T(0.f);
+    o.r[i][1] = ok ? __ldg(a + P) : T(0.f);
+  }
+}
+
+template <typename T, int MODE, bool SC44>
+__device__ __forceinline__ void write_hats(unsigned buf, const Offsets<T>& o, int half, const ConvParams& p, int lane) {
+  constexpr bool SPLIT = std::is_same<T, float>::value;
+  const int sl = lane >> 3, px = lane & 7;
+  // row of this pixel inside its 8-row core matrix: pixels p and p + 4 are neighbours
+  const unsigned dst = buf + (half * 2 + (sl >> 1)) * kPairRow + (sl & 1) * (3 * 256) + ((px & 3) * 2 + (px >> 2)) * 16;
+#pragma unroll
+  for (int i = 0; i < 9; ++i) {
+    int qh, qw, fh, fw;
+    tap_of<MODE>(i / 3, i % 3, 0, 0, qh, qw, fh, fw);
+    // same association as the reference: (tap index + offset) + (scope - kernel) / 2
+    const float u = ((float)fh + static_cast<float>(o.r[i][0])) + p.uh0, w = ((float)fw + static_cast<float>(o.r[i][1])) + p.uw0;
+    unsigned hi[8], lo[8];
+    hat_products<SC44, SPLIT>(hi, lo, u, w, (o.ok >> i) & 1, p.scW, p.cells);
+    const unsigned a = dst + (i / 3) * (kTeams * kPairRow) + (i % 3) * 256;
+    sts16(a, hi[0], hi[1], hi[2], hi[3]);
+    sts16(a + 128, hi[4], hi[5], hi[6], hi[7]);
+    if (SPLIT) {
+      sts16(a + kPiece, lo[0], lo[1], lo[2], lo[3]);
+      sts16(a + kPiece + 128, lo[4], lo[5], lo[6], lo[7]);
+    }
+  }
+}
+
+// ------------------------------------------------------------------ source rows without TMA
+// Loader warp lw of NL: source row `row` of channels c0 .. c0 + cg - 1 of sample n into a slot.
+template <typename T, int NL>
+__device__ __forceinline__ void copy_row(char* slot, const T* __restrict__ src, int n, int c0, int cg, int row, const ConvParams& p,
+                                         int lw, int lane) {
+  const int bytes = p.Ws * (int)sizeof(T);
+  if (row < 0 || row >= p.Hs) {  // a row of the padding
+    for (int c = lw; c < cg; c += NL) {
+      uint4* d = reinterpret_cast<uint4*>(slot + (size_t)c * p.pitch);
+      for (int i = lane; i < p.pitch / 16; i += 32) d[i] = make_uint4(0, 0, 0, 0);
+    }
+    return;
+  }
+  const size_t plane = (size_t)p.Hs * bytes;
+  const char* g0 = reinterpret_cast<const char*>(src) + ((size_t)n * p.C + c0) * plane + (size_t)row * bytes;
+  char* d0 = slot + 16;
+  const unsigned align = (unsigned)(reinterpret_cast<uintptr_t>(src) | (unsigned)bytes);
+  const int unit = (align & 7) == 0 ? 8 : ((align & 3) == 0 ? 4 : 2);
+  const int per = bytes / unit;  // copies per channel row
+  // a lane keeps its piece of the row and walks down the channels, several channels per step where rows are short
+  const int chs = per <= 16 ? 32 / per : 1;
+  for (int i = lane; i < (per <= 16 ? chs * per : per); i += 32) {
+    const int sub = per <= 16 ? i / per : 0, first = lw * chs + sub, step = NL * chs;
+    const int pc = i - sub * per;
+    const char* g = g0 + (size_t)first * plane + pc * unit;
+    char* d = d0 + first * p.pitch + pc * unit;
+    const size_t gs = (size_t)step * plane;
+    const int ds = step * p.pitch;
+    if (unit == 8) {
+#pragma unroll 4
+      for (int c = first; c < cg; c += step, g += gs, d += ds) cp_async8(d, g);
+    } else if (unit == 4) {
+#pragma unroll 4
+      for (int c = first; c < cg; c += step, g += gs, d += ds) mma::cp_async4(d, g);
+    } else {
+      for (int c = first; c < cg; c += 8 * step, g += 8 * gs, d += 8 * ds) {  // eight independent loads in flight
+        unsigned short v[8];
+#pragma unroll
+        for (int k = 0; k < 8; ++k)
+          if (c + k * step < cg) v[k] = __ldg(reinterpret_cast<const unsigned short*>(g + k * gs));
+#pragma unroll
+        for (int k = 0; k < 8; ++k)
+          if (c + k * step < cg) *reinterpret_cast<unsigned short*>(d + k * ds) = v[k];
+      }
+    }
+  }
+}
+
+// ------------------------------------------------------------------ forward and grad-input
+// staged results: [channel][64 pixels], an odd number of 16-byte units per channel (lanes = channels write 16 bytes each)
+template <typename T> __host__ __device__ constexpr int out_pitch() { return kStepSegs * 8 * (int)sizeof(T) + 16; }
+
+struct ConvSmem {  // byte offsets behind the row ring
+  unsigned beta, inv, out, bars, total;
+};
+template <typename T, int MODE>
+__host__ __device__ inline ConvSmem conv_smem(unsigned ring_bytes, int groups, int nbuf) {
+  constexpr bool SPLIT = std::is_same<T, float>::value;
+  ConvSmem m;
+  m.beta = (ring_bytes + 32 + 127) & ~127u;  // 32: what the last channel row's right edge may read
+  m.inv = m.beta + nbuf * kPiece * (SPLIT ? 2 : 1);
+  m.out = m.inv + (SPLIT ? groups * 128 : 0);
+  m.bars = m.out + (MODE == kData2 ? 0 : groups * 32 * out_pitch<T>());
+  m.total = m.bars + kBars * 8 + 16;
+  return m;
+}
+
+template <typename T, int MODE, bool SC44, int NL>
+__global__ void __launch_bounds__(kThreads, 1)
+    tc_conv_kernel(const __grid_constant__ CUtensorMap tm, const T* __restrict__ src, const T* __restrict__ rot,
+                   const T* __restrict__ bank, T* __restrict__ dst, const ConvParams p) {
+  extern __shared__ __align__(1024) char smem[];
+  using Wk = Walk<MODE>;
+  constexpr bool SPLIT = std::is_same<T, float>::value, STAGED = MODE != kData2;
+  constexpr int PIECES = SPLIT ? 2 : 1, E = sizeof(T);
+  constexpr int NB = beta_warps<T>(NL), NBUF = NB / 2, NS = kHelpers - 1 - NL - NB;
+  constexpr int kOutPitch = out_pitch<T>();
+  const int warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0), lane = threadIdx.x & 31;
+  const int c0 = blockIdx.y * p.CG, cg = min(p.CG, p.C - c0);
+  const int groups = p.full * 4 + p.rest, rounds = p.full + (p.rest ? 1 : 0);
+  const unsigned slot_bytes = (unsigned)p.CG * p.pitch, ring_bytes = slot_bytes * p.R;
+  const ConvSmem sm = conv_smem<T, MODE>(ring_bytes, groups, NBUF);
+  const unsigned base = smem_u32(smem);
+  const unsigned x_full = base + sm.bars, step_done = x_full + 8 * kDepth, b_full = step_done + 8 * kDepth;
+  const unsigned b_free = b_full + 8 * kMaxBuf, t_full = b_free + 8 * kMaxBuf, t_empty = t_full + 16, o_full = t_empty + 16,
+                 o_free = o_full + 8;
+  float* inv_s = reinterpret_cast<float*>(smem + sm.inv);
+  volatile int* tail = reinterpret_cast<volatile int*>(smem + sm.bars + kBars * 8);  // TMEM address, abort flag
+
+  const int lo = blockIdx.x * p.steps_per_cta * kStepSegs, hi = min(lo + p.steps_per_cta * kStepSegs, p.segs);
+  const int steps = (hi - lo + kStepSegs - 1) / kStepSegs;
+  const SegPos s_lo = seg_pos(lo, p);
+  const int j_first = s_lo.n * p.L + s_lo.g * Wk::S;  // first stream row
+  const unsigned magic_r = (unsigned)((0x100000000ull + (unsigned)p.R - 1) / (unsigned)p.R);
+
+  // ---- set-up: the padding that no copy writes is zero
+  if (NL == 1) {
+    for (int i = threadIdx.x; i < p.R * p.CG; i += kThreads) *reinterpret_cast<uint4*>(smem + (size_t)i * p.pitch) = make_uint4(0, 0, 0, 0);
+  } else {
+    for (unsigned i = threadIdx.x * 16; i < ring_bytes; i += kThreads * 16) *reinterpret_cast<uint4*>(smem + i) = make_uint4(0, 0, 0, 0);
+  }
+  if (threadIdx.x < 2) *reinterpret_cast<uint4*>(smem + ring_bytes + threadIdx.x * 16) = make_uint4(0, 0, 0, 0);
+  fence_proxy_async();
+  if (threadIdx.x == 0) {
+    for (int i = 0; i < kDepth; ++i) {
+      mbar_init(x_full + 8 * i, NL == 1 ? 1 : 64 * NL);
+      mbar_init(step_done + 8 * i, kConsumers);
+    }
+    for (int i = 0; i < NBUF; ++i) {
+      mbar_init(b_full + 8 * i, 2);
+      mbar_init(b_free + 8 * i, 1);
+    }
+    for (int i = 0; i < 2; ++i) {
+      mbar_init(t_full + 8 * i, 1);
+      mbar_init(t_empty + 8 * i, kConsumers);
+    }
+    mbar_init(o_full, kConsumers);
+    mbar_init(o_free, NS);
+    fence_barrier_init();
+    tail[1] = 0;
+  }
+  if (warp == kConsumers) tmem_alloc_all(smem_u32(const_cast<int*>(tail)));
+  fence_before();
+  __syncthreads();
+  fence_after();
+  const unsigned tmem = __shfl_sync(0xffffffffu, (unsigned)tail[0], 0);
+  volatile int* abort_flag = tail + 1;
+  if (warp < kConsumers) {  // bank -> TMEM
+    const int q = warp & 3, tiles = p.full + (p.rest ? 4 : 0);
+    for (int i = warp >> 2; i < tiles; i += kTeams) {
+      int grp = i * 4 + q;
+      if (i >= p.full) {
+        const int k = rest_index(p.rest, i - p.full, q);
+        grp = k < 0 ? -1 : p.full * 4 + k;
+      }
+      const int ch = grp * 32 + lane;
+      const bool ok = grp >= 0 && ch < cg;
+      unsigned h[8], l[8];
+      float inv;
+      bank_pieces<T>(h, l, inv, bank + (size_t)(c0 + (ok ? ch : 0)) * p.cells, p.cells, ok);
+      const unsigned a = tmem + ((unsigned)(q * 32) << 16) + kBankCol + i * 8 * PIECES;
+      st8(a, h);
+      if (SPLIT) {
+        st8(a + 8, l);
+        if (grp >= 0) inv_s[grp * 32 + lane] = inv;
+      }
+    }
+    wait_st();
+  }
+  fence_before();
+  __syncthreads();
+  fence_after();
+
+  if (warp < kConsumers) {
+    // ================================================================ consumers
+    regs_inc<kRegsConsumer>();
+    const int q = warp & 3, team = warp >> 2;
+    const unsigned lanes = (unsigned)(q * 32) << 16;
+    const bool vec = p.store == 16;
+    constexpr int NA = MODE == kData2 ? 16 : 8;
+    int use = 0;
+    for (int s = 0; s < steps; ++s) {
+      const int seg0 = lo + s * kStepSegs + team * 2;  // this pair's two segments
+      SegPos sp[2];
+      unsigned xr[2][Wk::rows];
+      bool live[2];
+#pragma unroll
+      for (int h = 0; h < 2; ++h) {
+        live[h] = seg0 + h < hi;
+        sp[h] = seg_pos(live[h] ? seg0 + h : lo, p);
+        const int k = sp[h].n * p.L + sp[h].g * Wk::S - j_first;
+#pragma unroll
+        for (int v = 0; v < Wk::rows; ++v) {
+          const int kk = k + v, sl = kk - (int)__umulhi((unsigned)kk, magic_r) * p.R;
+          xr[h][v] = sl * slot_bytes + 16 + sp[h].s * (8 * Wk::xs * E);
+        }
+      }
+      if (!wait_bar(x_full + 8 * (s & (kDepth - 1)), (s / kDepth) & 1, abort_flag)) break;
+      if (STAGED && s > 0 && !wait_bar(o_free, (s - 1) & 1, abort_flag)) break;
+      bool ok = true;
+      for (int rd = 0; rd < rounds; ++rd) {
+        int grp = rd * 4 + q;
+        if (rd == p.full) {
+          const int k = rest_index(p.rest, (team + s) & 3, q);
+          grp = k < 0 ? -1 : p.full * 4 + k;
+        }
+        if (grp < 0) {  // no group for this quarter: only keep step with the sets of accumulators
+          for (int v = 0; v < 3; ++v, ++use) {
+            ok = wait_bar(t_full + 8 * (use & 1), (use >> 1) & 1, abort_flag);
+            if (!ok) break;
+            if (lane == 0) mbar_arrive(t_empty + 8 * (use & 1));
+          }
+          if (!ok) break;
+          continue;
+        }
+        const int ch = grp * 32 + lane;
+        const char* xc = smem + ch * p.pitch;
+        const float inv = SPLIT ? inv_s[ch] : 1.f;
+        float acc[2][NA];
+#pragma unroll
+        for (int h = 0; h < 2; ++h)
+#pragma unroll
+          for (int i = 0; i < NA; ++i) acc[h][i] = 0.f;
+        // items (kernel row, segment) in order; fp16 fetches the next item while it multiplies this one
+        constexpr int NI = SPLIT ? 1 : 2;
+        Item<T, MODE> item[NI];
+        auto fetch = [&](Item<T, MODE>& it, int i) -> bool {
+          const int v = i >> 1, h = i & 1, set = (use + v) & 1;
+          if (h == 0) {
+            if (!wait_bar(t_full + 8 * set, ((use + v) >> 1) & 1, abort_flag)) return false;
+            fence_after();
+            __syncwarp();
+          }
+          constexpr int row_of[3] = {0, MODE == kData2 ? 0 : 1, MODE == kData2 ? 1 : 2};
+          it.load(tmem + lanes + set * kSetCols + team * kSlotCols + h * 24, xc + xr[h][row_of[v]]);
+          return true;
+        };
+        auto fetched = [&](Item<T, MODE>& it, int i) {
+          wait_ld(it.k);
+          if (i & 1) {  // both segments' accumulators of this kernel row are in registers
+            fence_before();
+            if (lane == 0) mbar_arrive(t_empty + 8 * ((use + (i >> 1)) & 1));
+          }
+        };
+        if (NI == 2) {
+          ok = fetch(item[0], 0);
+          if (!ok) break;
+          fetched(item[0], 0);
+        }
+#pragma unroll
+        for (int i = 0; i < 6; ++i) {
+          if (NI == 2) {
+            if (i < 5) {
+              ok = fetch(item[(i + 1) % NI], i + 1);
+              if (!ok) break;
+            }
+            multiply<T, MODE>(acc[i & 1], item[i % NI]);
+            if (i < 5) fetched(item[(i + 1) % NI], i + 1);
+          } else {
+            ok = fetch(item[0], i);
+            if (!ok) break;
+            fetched(item[0], i);
+            multiply<T, MODE>(acc[i & 1], item[0]);
+          }
+          if (MODE == kData2 && (i < 2 || i > 3)) {  // kernel row 0 completes the even row of the patch, 2 the odd one
+            const int h = i & 1, row = 2 * sp[h].g + (i > 3), col = 16 * sp[h].s;
+            if (live[h] && ch < cg && row < p.Hd) {
+              float o[16];
+#pragma unroll
+              for (int k = 0; k < 8; ++k) o[2 * k] = acc[h][k] * inv, o[2 * k + 1] = acc[h][NA - 8 + k] * inv;
+              store_row<T, 16>(dst + (((size_t)sp[h].n * p.C + c0 + ch) * p.Hd + row) * p.Wd + col, o, p.Wd - col, vec);
+            }
+#pragma unroll
+            for (int k = 0; k < NA; ++k) acc[h][k] = 0.f;
+          }
+        }
+        if (!ok) break;
+        use += 3;
+        if (STAGED) {
+          char* o = smem + sm.out + ch * kOutPitch + team * (16 * E);
+#pragma unroll
+          for (int h = 0; h < 2; ++h) {
+            if constexpr (E == 2) {
+              *reinterpret_cast<uint4*>(o + 16 * h) = make_uint4(mma::pack2(acc[h][0], acc[h][1]), mma::pack2(acc[h][2], acc[h][3]),
+                                                                 mma::pack2(acc[h][4], acc[h][5]), mma::pack2(acc[h][6], acc[h][7]));
+            } else {
+#pragma unroll
+              for (int k = 0; k < 8; k += 4)
+                *reinterpret_cast<float4*>(o + 32 * h + 4 * k) =
+                    make_float4(acc[h][k] * inv, acc[h][k + 1] * inv, acc[h][k + 2] * inv, acc[h][k + 3] * inv);
+            }
+          }
+        }
+      }
+      if (!ok) break;
+      __syncwarp();
+      if (lane == 0) {
+        mbar_arrive(step_done + 8 * (s & (kDepth - 1)));
+        if (STAGED) mbar_arrive(o_full);
+      }
+    }
+  } else if (warp == kConsumers) {
+    // ================================================================ MMA
+    regs_dec<kRegsHelper>();
+    constexpr unsigned idesc_all = idesc_f16(128, kSetCols, false, false, SPLIT), idesc_pair = idesc_f16(128, kSlotCols, false, false, SPLIT);
+    int use = 0;
+    bool ok = true;
+    for (int s = 0, bi = 0, turn = 0; s < steps && ok; ++s) {
+      ok = wait_bar(b_full + 8 * bi, turn & 1, abort_flag);
+      if (!ok) break;
+      fence_after();
+      const unsigned buf = base + sm.beta + bi * (PIECES * kPiece);
+      for (int rd = 0; rd < rounds && ok; ++rd) {
+        for (int v = 0; v < 3; ++v, ++use) {
+          const int set = use & 1;
+          if (use >= 2) {
+            ok = wait_bar(t_empty + 8 * set, ((use >> 1) - 1) & 1, abort_flag);
+            if (!ok) break;
+            fence_after();
+          }
+          const unsigned d = tmem + set * kSetCols;
+          const uint64_t b = sdesc(buf + v * (kTeams * kPairRow), 128, 256);
+          if (elect_one()) {
+            if (rd < p.full) {
+              const unsigned a = tmem + kBankCol + rd * 8 * PIECES;
+              mma_ts(d, a, b, idesc_all, false);
+              if (SPLIT) {
+                mma_ts(d, a, b + (kPiece >> 4), idesc_all, true);
+                mma_ts(d, a + 8, b, idesc_all, true);
+                mma_ts(d, a + 8, b + (kPiece >> 4), idesc_all, true);
+              }
+            } else {  // the remaining groups sit on other lanes for every pair
+#pragma unroll
+              for (int j = 0; j < kTeams; ++j) {
+                const unsigned a = tmem + kBankCol + (p.full + ((j + s) & 3)) * 8 * PIECES, dj = d + j * kSlotCols;
+                const uint64_t bj = b + j * (kPairRow >> 4);
+                mma_ts(dj, a, bj, idesc_pair, false);
+                if (SPLIT) {
+                  mma_ts(dj, a, bj + (kPiece >> 4), idesc_pair, true);
+                  mma_ts(dj, a + 8, bj, idesc_pair, true);
+                  mma_ts(dj, a + 8, bj + (kPiece >> 4), idesc_pair, true);
+                }
+              }
+            }
+            commit(t_full + 8 * set);
+          }
+          __syncwarp();
+        }
+      }
+      if (ok && elect_one()) commit(b_free + 8 * bi);
+      __syncwarp();
+      if (++bi == NBUF) bi = 0, ++turn;
+    }
+  } else if (warp <= kConsumers + NL) {
+    // ================================================================ source rows
+    regs_dec<kRegsHelper>();
+    const int lw = warp - kConsumers - 1;
+    int next = 0, done = 0;
+    bool ok = true;
+    for (int s = 0; s < steps && ok; ++s) {
+      const SegPos e = seg_pos(min(lo + s * kStepSegs + kStepSegs - 1, hi - 1), p);
+      const int last = e.n * p.L + e.g * Wk::S + Wk::rows - 1 - j_first;
+      // steps that must be over: those that read the rows about to be overwritten, and the last user of this step's barrier
+      while (done < s) {
+        const SegPos f = seg_pos(lo + done * kStepSegs, p);
+        const int first_row = f.n * p.L + f.g * Wk::S - j_first;
+        if (done > s - kDepth && (next > last || first_row > last - p.R)) break;
+        ok = wait_bar(step_done + 8 * (done & (kDepth - 1)), (done / kDepth) & 1, abort_flag);
+        if (!ok) break;
+        ++done;
+      }
+      if (!ok) break;
+      const unsigned bar = x_full + 8 * (s & (kDepth - 1));
+      if (NL == 1) {
+        if (lane == 0) {
+          if (last >= next) mbar_arrive_expect_tx(bar, (unsigned)(last - next + 1) * slot_bytes);
+          else mbar_arrive(bar);
+        }
+        __syncwarp();
+      }
+      for (; next <= last; ++next) {
+        const int sl = next - (int)__umulhi((unsigned)next, magic_r) * p.R;
+        const int j = j_first + next, n = j / p.L, row = j - n * p.L + Wk::first;
+        if (NL == 1) {
+          if (lane == 0)
+            for (int c = 0; c < p.CG; c += p.box_c)
+              tma_load_3d(base + sl * slot_bytes + c * p.pitch, &tm, -(16 / E), row, n * p.C + c0 + c, bar);
+        } else {
+          copy_row<T, NL>(smem + (size_t)sl * slot_bytes, src, n, c0, cg, row, p, lw, lane);
+        }
+      }
+      if (NL != 1) {
+        cp_async_arrive_noinc(bar);
+        mbar_arrive(bar);
+      }
+    }
+  } else if (warp <= kConsumers + NL + NB) {
+    // ================================================================ hat products
+    regs_dec<kRegsHelper>();
+    const int w = warp - kConsumers - 1 - NL, half = w & 1, bi = w >> 1;
+    Offsets<T> off;
+    if (bi < steps) fetch_offsets<T, MODE>(off, rot, lo + bi * kStepSegs + half * 4, hi, p, lane);
+    for (int s = bi, turn = 0; s < steps; s += NBUF, ++turn) {
+      if (turn > 0 && !wait_bar(b_free + 8 * bi, (turn - 1) & 1, abort_flag)) break;
+      write_hats<T, MODE, SC44>(base + sm.beta + bi * (PIECES * kPiece), off, half, p, lane);
+      fence_proxy_async();
+      __syncwarp();
+      if (lane == 0) mbar_arrive(b_full + 8 * bi);
+      if (s + NBUF < steps) fetch_offsets<T, MODE>(off, rot, lo + (s + NBUF) * kStepSegs + half * 4, hi, p, lane);
+    }
+  } else {
+    // ================================================================ results to memory
+    regs_dec<kRegsHelper>();
+    const int w = warp - kConsumers - 1 - NL - NB;
+    const size_t plane = (size_t)p.Hd * p.Wd;
+    for (int s = 0; s < steps && STAGED; ++s) {
+      const int seg = lo + s * kStepSegs;
+      // where this lane's share of a channel's 64 staged values goes: `store` bytes of a segment
+      if (p.store == 16) {
+        constexpr int PC = kStepSegs * 8 * E / 16, PS = PC / kStepSegs;  // 16-byte pieces per channel, per segment
+        const int i = lane % PC, b = seg + i / PS;
+        const SegPos sp = seg_pos(min(b, hi - 1), p);
+        const int col = 8 * sp.s + (i % PS) * (16 / E);
+        T* d = dst + ((size_t)sp.n * p.C + c0) * plane + (size_t)sp.g * p.Wd + col;
+        const char* o = smem + sm.out + i * 16;
+        if (!wait_bar(o_full, s & 1, abort_flag)) break;
+        if (b < hi && col < p.Wd) {
+#pragma unroll 4
+          for (int c = w * (32 / PC) + lane / PC; c < cg; c += NS * (32 / PC))
+            *reinterpret_cast<uint4*>(d + c * plane) = *reinterpret_cast<const uint4*>(o + c * kOutPitch);
+        }
+      } else {
+        if (!wait_bar(o_full, s & 1, abort_flag)) break;
+        const int per = 8 * E / p.store;
+        for (int i = lane; i < kStepSegs * per; i += 32) {
+          const int b = seg + i / per;
+          const SegPos sp = seg_pos(min(b, hi - 1), p);
+          const int col = 8 * sp.s + (i % per) * (p.store / E);
+          if (b < hi && col < p.Wd) {
+            T* d = dst + ((size_t)sp.n * p.C + c0) * plane + (size_t)sp.g * p.Wd + col;
+            const char* o = smem + sm.out + i * p.store;
+            if (p.store == 4) {
+#pragma unroll 4
+              for (int c = w; c < cg; c += NS) *reinterpret_cast<unsigned*>(d + c * plane) = *reinterpret_cast<const unsigned*>(o + c * kOutPitch);
+            } else {
+#pragma unroll 4
+              for (int c = w; c < cg; c += NS)
+                *reinterpret_cast<unsigned short*>(d + c * plane) = *reinterpret_cast<const unsigned short*>(o + c * kOutPitch);
+            }
+          }
+        }
+      }
+      __syncwarp();
+      if (lane == 0) mbar_arrive(o_free);
+    }
+  }
+  __syncwarp();
+  fence_before();
+  __syncthreads();
+  if (*abort_flag) {
+    // a wait ran out: report it, and leave the shared memory that copies may still write to for a while
+    if (threadIdx.x == 0) atomicExch(&g_tc_error, 2);
+    for (int i = 0; i < 64; ++i) __nanosleep(1000);
+  }
+  if (warp == kConsumers) {
+    fence_after();
+    tmem_free_all(tmem);
+  }
+}
+
+// ------------------------------------------------------------------ host side
+bool tc_shape(const Geom& g) {
+  if (g.kH != 3 || g.kW != 3 || g.dH != 1 || g.dW != 1 || g.pH != 1 || g.pW != 1) return false;
+  if (g.sH != g.sW || (g.sH != 1 && g.sH != 2)) return false;
+  return g.G == 1 && g.cells <= 16;
+}
+
+// most stream rows that `segments` consecutive segments can read
+int step_rows(int nseg, int Hg, int S, int L, int rows, int segments) {
+  const int span = (nseg - 1 + segments - 1) / nseg;      // segment rows beyond the first
+  const int crossings = span ? (span + Hg - 1) / Hg : 0;  // samples beyond the first
+  return span * S + crossings * (L - Hg * S) + rows;
+}
+
+struct ConvPlan {
+  bool ok;
+  bool tma;
+  int ctas, splits;
+  size_t smem;
+  ConvParams p;
+};
+
+template <typename T, int MODE>
+ConvPlan plan_conv(const Geom& g, const void* src, const void* dst) {
+  using Wk = Walk<MODE>;
+  ConvPlan pl;
+  pl.ok = false;
+  ConvParams& p = pl.p;
+  constexpr bool kData = MODE == kData1 || MODE == kData2;
+  constexpr int E = sizeof(T), PIECES = E == 4 ? 2 : 1;
+  p.N = g.N, p.C = g.C, p.Ho = g.Ho, p.Wo = g.Wo;
+  p.Hs = kData ? g.Ho : g.H, p.Ws = kData ? g.Wo : g.W;
+  p.Hd = kData ? g.H : g.Ho, p.Wd = kData ? g.W : g.Wo;
+  p.Hg = MODE == kData2 ? g.Ho : p.Hd, p.Wg = MODE == kData2 ? g.Wo : p.Wd;
+  p.nseg = (p.Wg + 7) / 8;
+  p.L = MODE == kFwd2 ? 2 * g.Ho + 1 : (MODE == kData2 ? g.Ho + 1 : p.Hs + 2);
+  const long long rows = (long long)g.N * p.Hg, segs = rows * p.nseg;
+  if (segs > 0x3fffffffLL || (long long)g.N * p.L > 0x3fffffffLL) return pl;
+  // the divisions by nseg, Hg and the ring depth are multiplications that need these products below 2^32
+  if (segs * p.nseg > 0xffffffffLL || rows * p.Hg > 0xffffffffLL) return pl;
+  p.segs = (int)segs;
+  p.magic_seg = (unsigned)((0x100000000ull + p.nseg - 1) / p.nseg);
+  p.magic_row = (unsigned)((0x100000000ull + p.Hg - 1) / p.Hg);
+  p.scW = g.scW, p.cells = g.cells;
+  p.uh0 = 0.5f * (g.scH - 3), p.uw0 = 0.5f * (g.scW - 3);
+  p.store = E;
+  if ((reinterpret_cast<uintptr_t>(dst) & 15) == 0 && (p.Wd * E) % 16 == 0) p.store = 16;
+  else if ((reinterpret_cast<uintptr_t>(dst) & 3) == 0 && (p.Wd * E) % 4 == 0) p.store = 4;
+  // padded row: 16 bytes in front; the column behind the last segment is the next row's front
+  p.pitch = ((1 + (p.nseg * 8 * Wk::xs * E) / 16) | 1) * 16;
+  if (p.pitch < 16 + p.Ws * E || p.pitch > 1152) return pl;
+  pl.tma = (reinterpret_cast<uintptr_t>(src) & 15) == 0 && (p.Ws * E) % 16 == 0 && p.pitch / E <= 256;
+  const int nbuf = beta_warps<T>(pl.tma ? 1 : kLoaders) / 2;
+  const int need = step_rows(p.nseg, p.Hg, Wk::S, p.L, Wk::rows, kStepSegs);
+  const int want = step_rows(p.nseg, p.Hg, Wk::S, p.L, Wk::rows, kStepSegs * kDepth);
+  const int groups = (g.C + 31) / 32, steps = (p.segs + kStepSegs - 1) / kStepSegs, sms = device_sm_count();
+  const size_t budget = (size_t)device_smem_optin();
+  long long best = -1;
+  for (int per = groups; per >= 1; --per) {  // groups per block
+    const int splits = (groups + per - 1) / per;
+    if ((groups + splits - 1) / splits != per || splits > 65535) continue;  // as many blocks with a better balance exist
+    const int full = per / 4, rest = per % 4;
+    if ((full + (rest ? 4 : 0)) * 8 * PIECES > 512 - kBankCol) continue;
+    int cg = splits == 1 ? (g.C + 7) & ~7 : per * 32;
+    const int boxes = (cg + 255) / 256;
+    cg = (cg + 8 * boxes - 1) / (8 * boxes) * (8 * boxes);  // boxes start on 128 bytes
+    if (splits > 1 && cg != per * 32) continue;
+    const size_t slot = (size_t)cg * p.pitch, fixed = conv_smem<T, MODE>(0, per, nbuf).total + 160;
+    if (fixed + slot * (need + 1) > budget) continue;
+    int R = (int)((budget - fixed) / slot);
+    if (R > want + 2) R = want + 2;
+    const bool shallow = R < need + 2 * Wk::S + 1;
+    long long cx = sms / splits > 0 ? sms / splits : 1;
+    if (cx > steps) cx = steps;
+    const int spc = (int)((steps + cx - 1) / cx);
+    const long long waves = ((long long)((steps + spc - 1) / spc) * splits + sms - 1) / sms;
+    // time of a block ~ steps x (groups + the hat products, about one group's work), plus its set-up
+    const long long cost = waves * ((long long)(spc + 2) * (per + 1) * (shallow ? 5 : 4));
+    if (best < 0 || cost < best) {
+      best = cost;
+      pl.ok = true;
+      p.CG = cg, p.box_c = cg / boxes, p.full = full, p.rest = rest, p.R = R;
+      p.steps_per_cta = spc;
+      pl.ctas = (steps + spc - 1) / spc, pl.splits = splits;
+      pl.smem = conv_smem<T, MODE>((unsigned)(slot * R), per, nbuf).total;
+      if (pl.smem < kMinSmem) pl.smem = kMinSmem;
+    }
+  }
+  return pl;
+}
+
+template <typename T, int MODE>
+int launch_conv(const T* src, const T* rot, const T* w, T* dst, const Geom& g, cudaStream_t s) {
+  const ConvPlan pl = plan_conv<T, MODE>(g, src, dst);
+  if (!pl.ok) return DK_ERR_UNSUPPORTED;
+  CUtensorMap tm;
+  std::memset(&tm, 0, sizeof(tm));
+  if (pl.tma && !make_plane_row_map(&tm, src, sizeof(T), pl.p.Ws, pl.p.Hs, (long long)g.N * g.C, pl.p.pitch / (int)sizeof(T), pl.p.box_c))
+    return DK_ERR_UNSUPPORTED;
+  const bool sc44 = g.scH == 4 && g.scW == 4;
+  auto run = [&](auto kern) {
+    // the roles' register shares add up to what a launch with this many registers allocates, not to less
+    static const bool shares_fit = [&] {
+      cudaFuncAttributes at;
+      return cudaFuncGetAttributes(&at, kern) == cudaSuccess && at.numRegs >= kRegsLaunch;
+    }();
+    if (!shares_fit) return (int)DK_ERR_UNSUPPORTED;
+    const int rc = enable_smem(kern, pl.smem);
+    if (rc) return rc;
+    kern<<<dim3(pl.ctas, pl.splits), kThreads, pl.smem, s>>>(tm, src, rot, w, dst, pl.p);
+    return check_launch();
+  };
+  if (pl.tma) return sc44 ? run(tc_conv_kernel<T, MODE, true, 1>) : run(tc_conv_kernel<T, MODE, false, 1>);
+  return sc44 ? run(tc_conv_kernel<T, MODE, true, kLoaders>) : run(tc_conv_kernel<T, MODE, false, kLoaders>);
+}
+
+}  // namespace
+
+template <typename T>
+int local_conv_tc(const T* src, const T* rot, const T* w, T* dst, const Geom& g, bool transposed, cudaStream_t s) {
+  if (!tc_shape(g)) return DK_ERR_UNSUPPORTED;
+  if (!transposed) return g.sH == 1 ? launch_conv<T, kFwd1>(src, rot, w, dst, g, s) : launch_conv<T, kFwd2>(src, rot, w, dst, g, s);
+  return g.sH == 1 ? launch_conv<T, kData1>(src, rot, w, dst, g, s) : launch_conv<T, kData2>(src, rot, w, dst, g, s);
+}
+template int local_conv_tc<float>(const float*, const float*, const float*, float*, const Geom&, bool, cudaStream_t);
+template int local_conv_tc<__half>(const __half*, const __half*, const __half*, __half*, const Geom&, bool, cudaStream_t);
+
+int tc_error_status() {
+  int v = 0;
+  if (cudaMemcpyFromSymbol(&v, g_tc_error, sizeof(int)) != cudaSuccess) return -1;
+  return v;
+}
+
+}  // namespace dk

@@ -81,6 +81,11 @@ __device__ __forceinline__ void prefetch_tensormap(const CUtensorMap* tm) {
   asm volatile("prefetch.tensormap [%0];\n" ::"l"(tm) : "memory");
 }
 
+// Planes [planes][rows][width] of `elem`-byte values viewed as a rank-3 tensor; one box = `box_w` values of one row of
+// `box_planes` consecutive planes.  Elements outside the tensor are delivered as zeros.  false: TMA cannot fetch such rows.
+bool make_plane_row_map(CUtensorMap* tm, const void* base, int elem, int width, int rows, long long planes, int box_w,
+                        int box_planes);
+
 // Bookkeeping of one ring of n slots (any n from 2 up, not only powers of two: shared memory decides the depth).
 // Fill number k goes to slot k mod n and is phase k / n ("turn") of that slot's two barriers.  A phase can only
 // be told from its parity, so a consumer may wait on the "full" barrier of fill k only once the slot has been
