@@ -411,7 +411,7 @@ __device__ __forceinline__ void beta_direct(unsigned (&bf)[9][2], const __half* 
       const int orow = S == 1 ? tr : tr >> 1, ocol = S == 1 ? tc : tc >> 1;
       rok[f] = tr >= 0 && (S == 1 || !(tr & 1)) && orow < Hs;
       cok[f] = pc < Wd && tc >= 0 && (S == 1 || !(tc & 1)) && ocol < Ws;
-      roff[f] = rok[f] ? orow * rb.Wp : 0;
+      roff[f] = (rok[f] ? orow : max(rb.row_lo, 0)) * rb.Wp;  // an unused tap reads (and ignores) some row of the band
       coff[f] = cok[f] ? ocol : 0;
     }
   }
