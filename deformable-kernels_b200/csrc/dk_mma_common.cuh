@@ -149,6 +149,8 @@ __device__ __forceinline__ void group_sync(int bar_id, int nt) {
   if (bar_id == 0) __syncthreads();
   else asm volatile("bar.sync %0, %1;\n" ::"r"(bar_id), "r"(nt) : "memory");
 }
+// WIDE: with the warp-per-row copies of odd widths above 16 (kernels short of registers leave them out where they meet no such rows)
+template <bool WIDE>
 __device__ __forceinline__ void load_band_group(__half* __restrict__ band, const Band& b, const __half* __restrict__ src, int n,
                                                 int C, int c0, int cnt, int Hs, int Ws, int tid, int nt, int bar_id) {
   const int lane = tid & 31, warp = tid >> 5, nwarps = nt >> 5;
@@ -162,9 +164,28 @@ __device__ __forceinline__ void load_band_group(__half* __restrict__ band, const
     for (int i = tid; i < nv; i += nt) b4[i] = z;
     if (r_e <= r_s) return;
     group_sync(bar_id, nt);
-    // 2-byte copies: a thread takes one (channel, row) and walks along it, eight independent loads in flight
     const int rows = r_e - r_s;
     const int tasks = cnt * rows;
+    if (WIDE && Ws > 16) {
+      // 2-byte copies, a warp per (channel, row): neighbours on neighbouring lanes, up to four loads in flight each (with a
+      // row per thread every lane is on a line of its own)
+      for (int t = warp; t < tasks; t += nwarps) {
+        const int j = t / rows, r = r_s + (t - j * rows);
+        const __half* sp = s0 + (size_t)j * plane + (size_t)r * Ws + lane;
+        __half* dp = band + j * b.pitch_c + kSlack + (r * b.Wp - b.org) + lane;
+        for (int left = Ws - lane; left > 0; left -= 128, sp += 128, dp += 128) {
+          __half v[4];
+#pragma unroll
+          for (int k = 0; k < 4; ++k)
+            if (32 * k < left) v[k] = __ldg(sp + 32 * k);
+#pragma unroll
+          for (int k = 0; k < 4; ++k)
+            if (32 * k < left) dp[32 * k] = v[k];
+        }
+      }
+      return;
+    }
+    // short rows: a thread takes one (channel, row) and walks along it, eight independent loads in flight
     for (int t = tid; t < tasks; t += nt) {
       const int j = t / rows, r = r_s + (t - j * rows);
       const __half* sp = s0 + (size_t)j * plane + (size_t)r * Ws;
@@ -238,11 +259,12 @@ __device__ __forceinline__ void flat_copies(__half* __restrict__ band, int pitch
 // leave lanes idle on the last pass over a row and walk through the channels one after the other.  Same instruction count
 // (measured), 3-4 % less time in the four kernels.
 // Odd row widths, and bands without a row inside the image, go through load_band_group.
+template <bool WIDE>
 __device__ __forceinline__ void load_band_flat(__half* __restrict__ band, const Band& b, const __half* __restrict__ src, int n,
                                                int C, int c0, int cnt, int Hs, int Ws, int tid, int nt, int bar_id) {
   const int r_s = max(b.row_lo, 0), r_e = min(b.row_lo + b.RB, Hs);
   if (b.mode == 0 || r_e <= r_s) {
-    load_band_group(band, b, src, n, C, c0, cnt, Hs, Ws, tid, nt, bar_id);
+    load_band_group<WIDE>(band, b, src, n, C, c0, cnt, Hs, Ws, tid, nt, bar_id);
     return;
   }
   const size_t plane = (size_t)Hs * Ws;
@@ -273,9 +295,10 @@ __device__ __forceinline__ void load_band_flat(__half* __restrict__ band, const 
     }
   }
 }
+template <bool WIDE = true>
 __device__ __forceinline__ void load_band(__half* __restrict__ band, const Band& b, const __half* __restrict__ src, int n, int C,
                                           int c0, int cnt, int Hs, int Ws) {
-  load_band_flat(band, b, src, n, C, c0, cnt, Hs, Ws, threadIdx.x, blockDim.x, 0);
+  load_band_flat<WIDE>(band, b, src, n, C, c0, cnt, Hs, Ws, threadIdx.x, blockDim.x, 0);
 }
 
 // Offset (in halves, even) of the window of pixel pair (ow, ow+1), row selector 0, inside a channel band.
