@@ -205,6 +205,11 @@ int ring_error_status();
 template <typename T>
 int local_conv_tc(const T* src, const T* rot, const T* w, T* dst, const Geom& g, bool transposed, cudaStream_t s);
 int tc_error_status();
+// fp32 gradients towards offsets and bank (dk_local_f32.cu); the bank's leave as *blocks partial sums [block][C][cells]
+int local_rot_f32(const float* dy, const float* x, const float* rot, const float* w, float* drot, const Geom& g, cudaStream_t s);
+size_t local_filter_f32_workspace(const Geom& g);
+int local_filter_f32(const float* dy, const float* x, const float* rot, float* partial, const Geom& g, size_t ws_bytes, int* blocks,
+                     cudaStream_t s);
 size_t local_rot_mma_workspace(const Geom& g);
 int local_rot_mma(const __half* dy, const __half* x, const __half* rot, const __half* w, __half* drot, const Geom& g,
                   void* ws, size_t ws_bytes, cudaStream_t s);

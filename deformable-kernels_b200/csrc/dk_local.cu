@@ -255,6 +255,10 @@ int local_backward_rotation(const T* dy, const T* x, const T* rot, const T* w, T
       if (rc != DK_ERR_UNSUPPORTED) return rc;
     }
   }
+  if constexpr (std::is_same<T, float>::value) {
+    const int rc = local_rot_f32(dy, x, rot, w, drot, g, s);
+    if (rc != DK_ERR_UNSUPPORTED) return rc;
+  }
   constexpr int NW = 8;
   const long long bx = ((long long)g.N * g.P + 31) / 32;
   if (bx > 0x7fffffffLL || g.G > 65535) return DK_ERR_UNSUPPORTED;
@@ -657,6 +661,16 @@ int local_backward_filter(const T* dy, const T* x, const T* rot, T* dw, const Ge
       const int rc = local_filter_mma(dy, x, rot, dw, g, ws, ws_bytes, s);
       if (rc != DK_ERR_UNSUPPORTED) return rc;
     }
+  }
+  if constexpr (std::is_same<T, float>::value) {
+    int blocks = 0;
+    const int rc = local_filter_f32(dy, x, rot, reinterpret_cast<float*>(ws), g, ws_bytes, &blocks, s);
+    if (rc == DK_OK) {
+      const int n_out = g.C * g.cells;
+      reduce_partials_kernel<T><<<(n_out + 31) / 32, 256, 0, s>>>(reinterpret_cast<const float*>(ws), dw, n_out, blocks);
+      return check_launch();
+    }
+    if (rc != DK_ERR_UNSUPPORTED) return rc;
   }
   return filter_backward<T, false>(dy, x, nullptr, rot, dw, g, ws, ws_bytes, s);
 }

@@ -1,0 +1,367 @@
+// Offset and bank gradients of the local deformable kernel in fp32 (3 x 3 taps, scopes up to 4 x 4).
+//
+// Both consume the products dK = dy * x, and both are dense in the 16 bank cells here: with the hat products the sampled
+// cells need no data-dependent addresses, so every bank value and every hat product is one broadcast read for a whole warp.
+//   bank      lanes = channels: dW[c, cell] += dK * hat_u * hat_v, 16 accumulators per lane kept in registers over all of the
+//             block's pixels; x and dy of a pixel tile come through shared memory (fetched with neighbours on neighbouring
+//             lanes, read back one channel per lane), the hats of a (pixel, tap) are two 16-byte broadcasts
+//   offsets   lanes = pixels: G[tap, cell] += dK * W[c, cell], a warp per kernel row (48 accumulators), channel after channel;
+//             then the floor-based derivative weights contract G
+// Bound by multiply-adds: 21 (bank) and 17 (offsets) per pixel, tap and channel.  The kernels before gathered four cells per
+// tap with an address per lane, read x and dy one channel per lane from global memory (a line per lane) and added into
+// shared memory: N = 64, C = 144, 56 x 56: bank 2088 us, offsets 394 us.
+#include <cuda_runtime.h>
+
+#include "dk_common.cuh"
+
+namespace dk {
+
+namespace {
+
+struct TilePlan {
+  int TH, TW;                 // output pixels of a tile
+  int across, down;           // tiles per row of tiles, per sample
+  int tiles;                  // over the batch
+  int XH, XW;                 // source rows and columns of a tile
+  int xpitch, ypitch;         // words per channel in shared memory, odd
+  unsigned magic_x, magic_y;  // ceil(2^32 / XW), ceil(2^32 / TW)
+  int per_block, blocks;      // tiles per block, blocks (bank)
+  size_t smem;
+};
+
+TilePlan tile_plan(const Geom& g, int pixels) {
+  TilePlan t;
+  const int widest = pixels < 32 ? pixels : 32;
+  t.across = (g.Wo + widest - 1) / widest;
+  t.TW = (g.Wo + t.across - 1) / t.across;
+  t.TH = pixels / t.TW;
+  if (t.TH > g.Ho) t.TH = g.Ho;
+  t.down = (g.Ho + t.TH - 1) / t.TH;
+  t.TH = (g.Ho + t.down - 1) / t.down;
+  t.tiles = g.N * t.down * t.across;
+  t.XH = (t.TH - 1) * g.sH + 3;
+  t.XW = (t.TW - 1) * g.sW + 3;
+  t.xpitch = (t.XH * t.XW) | 1;
+  t.ypitch = (t.TH * t.TW) | 1;
+  t.magic_x = (unsigned)((0x100000000ull + t.XW - 1) / t.XW);
+  t.magic_y = t.TW == 1 ? 0 : (unsigned)((0x100000000ull + t.TW - 1) / t.TW);
+  t.per_block = 1;
+  t.blocks = t.tiles;
+  t.smem = 0;
+  return t;
+}
+
+// two fp32 multiply-adds in one instruction: the pipe needs as long as for two, but the loads beside them get issue slots
+__device__ __forceinline__ unsigned long long pair(float a, float b) {
+  unsigned long long r;
+  asm("mov.b64 %0, {%1, %2};\n" : "=l"(r) : "f"(a), "f"(b));
+  return r;
+}
+__device__ __forceinline__ float2 unpair(unsigned long long v) {
+  float2 r;
+  asm("mov.b64 {%0, %1}, %2;\n" : "=f"(r.x), "=f"(r.y) : "l"(v));
+  return r;
+}
+__device__ __forceinline__ void fma2(unsigned long long& acc, unsigned long long a, unsigned long long b) {
+  asm("fma.rn.f32x2 %0, %1, %2, %0;\n" : "+l"(acc) : "l"(a), "l"(b));
+}
+
+__device__ __forceinline__ int over(int e, int d, unsigned magic) { return d == 1 ? e : (int)__umulhi((unsigned)e, magic); }
+__device__ __forceinline__ float hat1(float t) { return __saturatef(1.f - fabsf(t)); }  // max(0, 1 - |t|)
+
+struct TilePos {
+  int n, oh0, ow0;
+};
+__device__ __forceinline__ TilePos tile_pos(int tile, const TilePlan& t) {
+  TilePos p;
+  const int row = tile / t.across;
+  p.ow0 = (tile - row * t.across) * t.TW;
+  p.n = row / t.down;
+  p.oh0 = (row - p.n * t.down) * t.TH;
+  return p;
+}
+
+// 4 bytes from global to shared memory, asynchronously; zero where !ok (the address is not read then)
+__device__ __forceinline__ void copy4(float* dst, const float* src, bool ok) {
+  asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;\n" ::"r"((unsigned)__cvta_generic_to_shared(dst)), "l"(src),
+               "r"(ok ? 4 : 0));
+}
+__device__ __forceinline__ void copies_done() { asm volatile("cp.async.wait_all;\n" ::: "memory"); }
+
+// x and dy of channels c0 .. c0 + 31 of one tile; what lies outside the planes or beyond the last channel is zero.  All of a
+// warp's copies are in flight at once (loads into registers, four at a time, took as long as the arithmetic).
+template <int S>
+__device__ __forceinline__ void stage_tile(float* xs, float* ys, const float* __restrict__ x, const float* __restrict__ dy, const Geom& g,
+                                           const TilePlan& t, const TilePos& tp, int c0, int warp, int warps, int lane) {
+  const int xe = t.XH * t.XW, ye = t.TH * t.TW;
+  const float* x0 = x + ((size_t)tp.n * g.C + c0) * g.HW;
+  const float* y0 = dy + ((size_t)tp.n * g.C + c0) * g.P;
+  const int n_c = min(32, g.C - c0);
+  for (int e = lane; e < xe; e += 32) {
+    const int r = over(e, t.XW, t.magic_x), ih = tp.oh0 * S - 1 + r, iw = tp.ow0 * S - 1 + (e - r * t.XW);
+    const bool in = ih >= 0 && ih < g.H && iw >= 0 && iw < g.W;
+    const float* src = x0 + (in ? ih * g.W + iw : 0);
+    for (int ch = warp; ch < 32; ch += warps) copy4(xs + ch * t.xpitch + e, src + (size_t)(ch < n_c ? ch : 0) * g.HW, in && ch < n_c);
+  }
+  for (int e = lane; e < ye; e += 32) {
+    const int r = over(e, t.TW, t.magic_y), oh = tp.oh0 + r, ow = tp.ow0 + (e - r * t.TW);
+    const bool in = oh < g.Ho && ow < g.Wo;
+    const float* src = y0 + (in ? oh * g.Wo + ow : 0);
+    for (int ch = warp; ch < 32; ch += warps) copy4(ys + ch * t.ypitch + e, src + (size_t)(ch < n_c ? ch : 0) * g.P, in && ch < n_c);
+  }
+}
+
+// ------------------------------------------------------------------ bank
+constexpr int kBankWarps = 8;
+
+template <int S>
+__global__ void __launch_bounds__(32 * kBankWarps, 2) f32_bank_kernel(const float* __restrict__ dy, const float* __restrict__ x,
+                                                                      const float* __restrict__ rot, float* __restrict__ partial,
+                                                                      const Geom g, const TilePlan t) {
+  extern __shared__ __align__(16) float smem_f[];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int c0 = blockIdx.y * 32, px = t.TH * t.TW;
+  float4* hats = reinterpret_cast<float4*>(smem_f);  // [pixel][tap][hat_u | hat_v]
+  float* xs = smem_f + (size_t)px * 72;
+  float* ys = xs + 32 * t.xpitch;
+  const float uh0 = 0.5f * (float)(g.scH - 3), uw0 = 0.5f * (float)(g.scW - 3);
+  unsigned long long acc[2][4];  // cell rows (2i, 2i + 1) of column k
+#pragma unroll
+  for (int i = 0; i < 8; ++i) acc[i >> 2][i & 3] = 0;
+  const int first = blockIdx.x * t.per_block, last = min(first + t.per_block, t.tiles);
+  for (int tile = first; tile < last; ++tile) {
+    const TilePos tp = tile_pos(tile, t);
+    __syncthreads();
+    stage_tile<S>(xs, ys, x, dy, g, t, tp, c0, warp, kBankWarps, lane);
+    for (int i = threadIdx.x; i < px * 9; i += 32 * kBankWarps) {
+      const int tap = i / px, p = i - tap * px, r = over(p, t.TW, t.magic_y);
+      const int oh = tp.oh0 + r, ow = tp.ow0 + (p - r * t.TW), fh = tap / 3, fw = tap - fh * 3;
+      float u = -8.f, v = -8.f;  // samples nothing
+      if (oh < g.Ho && ow < g.Wo) {
+        const float* rp = rot + ((size_t)tp.n * 18 + 2 * tap) * g.P + oh * g.Wo + ow;
+        u = ((float)fh + __ldg(rp)) + uh0;
+        v = ((float)fw + __ldg(rp + g.P)) + uw0;
+      }
+      float4 hu, hv;
+      hu.x = hat1(u), hu.y = g.scH > 1 ? hat1(u - 1.f) : 0.f, hu.z = g.scH > 2 ? hat1(u - 2.f) : 0.f, hu.w = g.scH > 3 ? hat1(u - 3.f) : 0.f;
+      hv.x = hat1(v), hv.y = g.scW > 1 ? hat1(v - 1.f) : 0.f, hv.z = g.scW > 2 ? hat1(v - 2.f) : 0.f, hv.w = g.scW > 3 ? hat1(v - 3.f) : 0.f;
+      hats[(p * 9 + tap) * 2] = hu;
+      hats[(p * 9 + tap) * 2 + 1] = hv;
+    }
+    copies_done();
+    __syncthreads();
+    for (int p = warp; p < px; p += kBankWarps) {
+      const int r = over(p, t.TW, t.magic_y);
+      const float* xp = xs + lane * t.xpitch + r * S * t.XW + (p - r * t.TW) * S;
+      const float yv = ys[lane * t.ypitch + p];
+      const float4* hp = hats + p * 18;
+#pragma unroll
+      for (int i = 0; i < 9; ++i) {
+        const float dk = yv * xp[(i / 3) * t.XW + i % 3];
+        const ulonglong2 hu = *reinterpret_cast<const ulonglong2*>(hp + 2 * i);
+        const float4 hv = hp[2 * i + 1];
+        const float b[4] = {dk * hv.x, dk * hv.y, dk * hv.z, dk * hv.w};
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+          const unsigned long long bb = pair(b[k], b[k]);
+          fma2(acc[0][k], hu.x, bb);
+          fma2(acc[1][k], hu.y, bb);
+        }
+      }
+    }
+  }
+  __syncthreads();
+  float* red = smem_f;  // [warp][cell][lane]
+#pragma unroll
+  for (int i = 0; i < 8; ++i) {
+    const float2 v = unpair(acc[i >> 2][i & 3]);
+    const int cell = (i >> 2) * 8 + (i & 3);
+    red[(warp * 16 + cell) * 32 + lane] = v.x;
+    red[(warp * 16 + cell + 4) * 32 + lane] = v.y;
+  }
+  __syncthreads();
+  for (int i = threadIdx.x; i < 32 * 16; i += 32 * kBankWarps) {
+    const int cell = i >> 5, a = cell >> 2, b = cell & 3, c = c0 + (i & 31);
+    if (c < g.C && a < g.scH && b < g.scW) {
+      float s = 0.f;
+#pragma unroll
+      for (int w = 0; w < kBankWarps; ++w) s += red[w * 512 + i];
+      partial[((size_t)blockIdx.x * g.C + c) * g.cells + a * g.scW + b] = s;
+    }
+  }
+}
+
+// ------------------------------------------------------------------ offsets
+// 12 warps: kernel row x (PQ quads of 32 pixels, 4 / PQ shares of the channels).  Few pixels in the call: fewer pixels per
+// block and more shares.
+constexpr int kOffWarps = 12;
+
+template <int S, int PQ>
+__global__ void __launch_bounds__(32 * kOffWarps, 2) f32_offsets_kernel(const float* __restrict__ dy, const float* __restrict__ x,
+                                                                        const float* __restrict__ rot, const float* __restrict__ w,
+                                                                        float* __restrict__ drot, const Geom g, const TilePlan t) {
+  constexpr int SH = 4 / PQ;
+  extern __shared__ __align__(16) float smem_f[];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int fh = warp % 3, k = warp / 3, quad = k % PQ, share = k / PQ;
+  float* ws = smem_f;  // [channel][16 cells]
+  float* xs = ws + 32 * 16;
+  float* ys = xs + 32 * t.xpitch;
+  const TilePos tp = tile_pos(blockIdx.x, t);
+  const int px = t.TH * t.TW;
+  const int p = quad * 32 + lane, pc = p < px ? p : 0, r = over(pc, t.TW, t.magic_y), col = pc - r * t.TW;
+  const int xo = (r * S + fh) * t.XW + col * S;
+  unsigned long long G2[3][8];  // cells (2i, 2i + 1)
+#pragma unroll
+  for (int i = 0; i < 24; ++i) G2[i / 8][i % 8] = 0;
+  for (int c0 = 0; c0 < g.C; c0 += 32) {
+    __syncthreads();
+    stage_tile<S>(xs, ys, x, dy, g, t, tp, c0, warp, kOffWarps, lane);
+    for (int i = threadIdx.x; i < 32 * 16; i += 32 * kOffWarps) {
+      const int c = c0 + (i >> 4), a = (i >> 2) & 3, b = i & 3;
+      ws[i] = c < g.C && a < g.scH && b < g.scW ? __ldg(w + (size_t)c * g.cells + a * g.scW + b) : 0.f;
+    }
+    copies_done();
+    __syncthreads();
+    const int n_c = min(32, g.C - c0);
+#pragma unroll 2
+    for (int ch = share; ch < n_c; ch += SH) {
+      const float yv = ys[ch * t.ypitch + pc];
+      const float* xp = xs + ch * t.xpitch + xo;
+      unsigned long long d[3];
+#pragma unroll
+      for (int a = 0; a < 3; ++a) {
+        const float v = yv * xp[a];
+        d[a] = pair(v, v);
+      }
+      const ulonglong2* wp = reinterpret_cast<const ulonglong2*>(ws + ch * 16);
+#pragma unroll
+      for (int q = 0; q < 4; ++q) {
+        const ulonglong2 wv = wp[q];
+#pragma unroll
+        for (int a = 0; a < 3; ++a) {
+          fma2(G2[a][2 * q], d[a], wv.x);
+          fma2(G2[a][2 * q + 1], d[a], wv.y);
+        }
+      }
+    }
+  }
+  float G[3][16];
+#pragma unroll
+  for (int i = 0; i < 24; ++i) {
+    const float2 v = unpair(G2[i / 8][i % 8]);
+    G[i / 8][2 * (i % 8)] = v.x, G[i / 8][2 * (i % 8) + 1] = v.y;
+  }
+  float* red = smem_f + (size_t)(quad * 3 + fh) * 48 * 32;  // [tap, cell][lane]
+#pragma unroll
+  for (int s = 1; s < SH; ++s) {
+    __syncthreads();
+    if (share == s) {
+#pragma unroll
+      for (int i = 0; i < 48; ++i) red[i * 32 + lane] = G[i / 16][i % 16];
+    }
+    __syncthreads();
+    if (share == 0) {
+#pragma unroll
+      for (int i = 0; i < 48; ++i) G[i / 16][i % 16] += red[i * 32 + lane];
+    }
+  }
+  const int oh = tp.oh0 + r, ow = tp.ow0 + col;
+  if (share != 0 || p >= px || oh >= g.Ho || ow >= g.Wo) return;
+  const float uh0 = 0.5f * (float)(g.scH - 3), uw0 = 0.5f * (float)(g.scW - 3);
+  const int ih = oh * S - 1 + fh;
+#pragma unroll
+  for (int fw = 0; fw < 3; ++fw) {
+    const int iw = ow * S - 1 + fw, tap = fh * 3 + fw;
+    const size_t o = ((size_t)tp.n * 18 + 2 * tap) * g.P + oh * g.Wo + ow;
+    const float u = ((float)fh + __ldg(rot + o)) + uh0, v = ((float)fw + __ldg(rot + o + g.P)) + uw0;
+    const bool used = ih >= 0 && ih < g.H && iw >= 0 && iw < g.W && u > -1.f && v > -1.f && u < (float)g.scH && v < (float)g.scW;
+    float gu = 0.f, gv = 0.f;
+    if (used) {
+      const float fu = floorf(u), fv = floorf(v), lh = u - fu, lw = v - fv;
+      const int a0 = (int)fu, b0 = (int)fv;
+      float hv[4], dv[4];
+#pragma unroll
+      for (int b = 0; b < 4; ++b) {
+        hv[b] = b == b0 ? 1.f - lw : (b == b0 + 1 ? lw : 0.f);
+        dv[b] = b == b0 ? -1.f : (b == b0 + 1 ? 1.f : 0.f);
+      }
+#pragma unroll
+      for (int a = 0; a < 4; ++a) {
+        const float hu = a == a0 ? 1.f - lh : (a == a0 + 1 ? lh : 0.f), du = a == a0 ? -1.f : (a == a0 + 1 ? 1.f : 0.f);
+        float su = 0.f, sv = 0.f;
+#pragma unroll
+        for (int b = 0; b < 4; ++b) {
+          su = fmaf(hv[b], G[fw][4 * a + b], su);
+          sv = fmaf(dv[b], G[fw][4 * a + b], sv);
+        }
+        gu = fmaf(du, su, gu);
+        gv = fmaf(hu, sv, gv);
+      }
+    }
+    drot[o] = gu;
+    drot[o + g.P] = gv;
+  }
+}
+
+// ------------------------------------------------------------------ host side
+bool f32_shape(const Geom& g) {
+  return g.kH == 3 && g.kW == 3 && g.dH == 1 && g.dW == 1 && g.pH == 1 && g.pW == 1 && g.sH == g.sW && (g.sH == 1 || g.sH == 2) &&
+         g.G == 1 && g.scH <= 4 && g.scW <= 4 && (long long)g.N * g.P < 0x3fffffff;
+}
+
+// Tiles of up to 128 pixels; smaller ones while that leaves SMs without a block; then as many blocks as are resident at once.
+TilePlan bank_plan(const Geom& g) {
+  const int groups = (g.C + 31) / 32;
+  TilePlan t = tile_plan(g, 128);
+  for (int px = 64; px >= 16 && (long long)t.tiles * groups < 2LL * device_sm_count(); px /= 2) t = tile_plan(g, px);
+  int want = 2 * device_sm_count() / groups;
+  if (want < 1) want = 1;
+  t.per_block = (t.tiles + want - 1) / want;
+  t.blocks = (t.tiles + t.per_block - 1) / t.per_block;
+  t.smem = ((size_t)t.TH * t.TW * 72 + 32 * (size_t)(t.xpitch + t.ypitch)) * sizeof(float);
+  const size_t red = (size_t)kBankWarps * 512 * sizeof(float);
+  if (t.smem < red) t.smem = red;
+  return t;
+}
+
+}  // namespace
+
+size_t local_filter_f32_workspace(const Geom& g) {
+  return f32_shape(g) ? (size_t)bank_plan(g).blocks * g.C * g.cells * sizeof(float) : 0;
+}
+
+int local_filter_f32(const float* dy, const float* x, const float* rot, float* partial, const Geom& g, size_t ws_bytes, int* blocks,
+                     cudaStream_t s) {
+  if (!f32_shape(g)) return DK_ERR_UNSUPPORTED;
+  const TilePlan t = bank_plan(g);
+  if (t.smem > (size_t)device_smem_optin() || (g.C + 31) / 32 > 65535) return DK_ERR_UNSUPPORTED;
+  if (partial == nullptr || ws_bytes < (size_t)t.blocks * g.C * g.cells * sizeof(float)) return DK_ERR_WORKSPACE;
+  auto kern = g.sH == 1 ? f32_bank_kernel<1> : f32_bank_kernel<2>;
+  const int rc = enable_smem(kern, t.smem);
+  if (rc) return rc;
+  kern<<<dim3(t.blocks, (g.C + 31) / 32), 32 * kBankWarps, t.smem, s>>>(dy, x, rot, partial, g, t);
+  *blocks = t.blocks;
+  return check_launch();
+}
+
+int local_rot_f32(const float* dy, const float* x, const float* rot, const float* w, float* drot, const Geom& g, cudaStream_t s) {
+  if (!f32_shape(g)) return DK_ERR_UNSUPPORTED;
+  TilePlan t = tile_plan(g, 128);
+  int pq = 4;
+  while (pq > 1 && t.tiles < 2 * device_sm_count()) t = tile_plan(g, 32 * (pq /= 2));
+  size_t words = 512 + 32 * (size_t)(t.xpitch + t.ypitch);
+  const size_t red = (size_t)pq * 3 * 48 * 32;
+  if (pq < 4 && words < red) words = red;
+  t.smem = words * sizeof(float);
+  if (t.smem > (size_t)device_smem_optin()) return DK_ERR_UNSUPPORTED;
+  void (*kern)(const float*, const float*, const float*, const float*, float*, const Geom, const TilePlan) =
+      g.sH == 1 ? (pq == 4 ? f32_offsets_kernel<1, 4> : pq == 2 ? f32_offsets_kernel<1, 2> : f32_offsets_kernel<1, 1>)
+                : (pq == 4 ? f32_offsets_kernel<2, 4> : pq == 2 ? f32_offsets_kernel<2, 2> : f32_offsets_kernel<2, 1>);
+  const int rc = enable_smem(kern, t.smem);
+  if (rc) return rc;
+  kern<<<t.tiles, 32 * kOffWarps, t.smem, s>>>(dy, x, rot, w, drot, g, t);
+  return check_launch();
+}
+
+}  // namespace dk

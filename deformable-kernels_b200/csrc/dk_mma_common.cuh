@@ -149,7 +149,7 @@ __device__ __forceinline__ void group_sync(int bar_id, int nt) {
   if (bar_id == 0) __syncthreads();
   else asm volatile("bar.sync %0, %1;\n" ::"r"(bar_id), "r"(nt) : "memory");
 }
-// WIDE: with the warp-per-row copies of odd widths above 16 (kernels short of registers leave them out where they meet no such rows)
+// WIDE: with the warp-per-row copies of odd widths above 64 (kernels short of registers leave them out where they meet no such rows)
 template <bool WIDE>
 __device__ __forceinline__ void load_band_group(__half* __restrict__ band, const Band& b, const __half* __restrict__ src, int n,
                                                 int C, int c0, int cnt, int Hs, int Ws, int tid, int nt, int bar_id) {
@@ -166,9 +166,10 @@ __device__ __forceinline__ void load_band_group(__half* __restrict__ band, const
     group_sync(bar_id, nt);
     const int rows = r_e - r_s;
     const int tasks = cnt * rows;
-    if (WIDE && Ws > 16) {
-      // 2-byte copies, a warp per (channel, row): neighbours on neighbouring lanes, up to four loads in flight each (with a
-      // row per thread every lane is on a line of its own)
+    if (WIDE && Ws > 64) {
+      // 2-byte copies, a warp per (channel, row): neighbours on neighbouring lanes, up to four loads in flight each.  With a row per
+      // thread every lane is on a line of its own, but the lines are reused and more loads are in flight: on rows of 31 that is
+      // the faster way (forward 29 against 49 us), on rows of 85 and 101 it is not (121 against 83, 66 against 41 us)
       for (int t = warp; t < tasks; t += nwarps) {
         const int j = t / rows, r = r_s + (t - j * rows);
         const __half* sp = s0 + (size_t)j * plane + (size_t)r * Ws + lane;
