@@ -406,7 +406,7 @@ __global__ void filter_kernel(const T* __restrict__ dy, const T* __restrict__ x,
 template <typename T, bool DEFORM>
 __global__ void filter_plane_kernel(const T* __restrict__ dy, const T* __restrict__ x, const T* __restrict__ off,
                                     const T* __restrict__ rot, typename Compute<T>::type* __restrict__ partial,
-                                    const Geom g, const int pitch, const int batch) {
+                                    const Geom g, const int pitch, const int batch, const int parts) {
   using A = typename Compute<T>::type;
   using Entry = TapEntry<A, DEFORM>;
   extern __shared__ __align__(16) unsigned char smem_raw[];
@@ -424,7 +424,8 @@ __global__ void filter_plane_kernel(const T* __restrict__ dy, const T* __restric
   for (int i = lane; i < g.cells * 32; i += 32) acc[i] = (A)0;
   const T* myplane = planes + (size_t)lane * pitch;
 
-  for (int n = blockIdx.x; n < g.N; n += gridDim.x) {
+  const int part = blockIdx.x % parts;
+  for (int n = blockIdx.x / parts; n < g.N; n += gridDim.x / parts) {
     __syncthreads();
     for (int ch = warp; ch < 32; ch += warps) {
       if (j0 + ch < g.Cg) {
@@ -433,7 +434,7 @@ __global__ void filter_plane_kernel(const T* __restrict__ dy, const T* __restric
         for (int i = lane; i < g.HW; i += 32) dp[i] = __ldg(sp + i);
       }
     }
-    for (int base = 0; base < g.P; base += batch) {
+    for (int base = part * batch; base < g.P; base += batch * parts) {
       const int nb = min(batch, g.P - base);
       __syncthreads();
       for (int i = threadIdx.x; i < nb * g.taps; i += blockDim.x) {
@@ -513,7 +514,7 @@ __global__ void filter_plane_kernel(const T* __restrict__ dy, const T* __restric
 
 struct PlanePlan {
   bool ok;
-  int warps, batch, pitch, slots, chan_blocks;
+  int warps, batch, pitch, slots, parts, chan_blocks;
   size_t smem, ws_bytes;
 };
 
@@ -540,7 +541,13 @@ static PlanePlan plane_plan(const Geom& g) {
   if (slots > g.N) slots = g.N;
   if (slots < 1) slots = 1;
   pl.slots = (int)slots;
-  pl.ws_bytes = (size_t)pl.slots * g.C * g.cells * sizeof(A);
+  // fewer samples than it takes to fill the GPU: several blocks share a sample's pixels, each with a copy of the planes
+  // (N = 16, C = 192, 28 x 28 fp32: 96 blocks became 384, 213 -> 150 us)
+  long long parts = (2LL * 148 + slots * chan_ctas - 1) / (slots * chan_ctas);
+  const long long most = g.P / (4 * pl.batch);
+  if (parts > most) parts = most;
+  pl.parts = parts < 1 ? 1 : (int)parts;
+  pl.ws_bytes = (size_t)pl.slots * pl.parts * g.C * g.cells * sizeof(A);
   pl.ok = pl.smem <= 226 * 1024 && pl.chan_blocks <= 65535 && g.G <= 65535 && g.Cg >= 32;
   return pl;
 }
@@ -626,12 +633,12 @@ static int filter_backward(const T* dy, const T* x, const T* off, const T* rot, 
       auto kern = filter_plane_kernel<T, DEFORM>;
       int rc = enable_smem(kern, pp.smem);
       if (rc) return rc;
-      kern<<<dim3(pp.slots, pp.chan_blocks, g.G), pp.warps * 32, pp.smem, s>>>(dy, x, off, rot, reinterpret_cast<A*>(ws), g,
-                                                                            pp.pitch, pp.batch);
+      kern<<<dim3(pp.slots * pp.parts, pp.chan_blocks, g.G), pp.warps * 32, pp.smem, s>>>(dy, x, off, rot, reinterpret_cast<A*>(ws), g,
+                                                                            pp.pitch, pp.batch, pp.parts);
       rc = check_launch();
       if (rc) return rc;
       const int n_out = g.C * g.cells;
-      reduce_partials_kernel<T><<<(n_out + 31) / 32, 256, 0, s>>>(reinterpret_cast<const A*>(ws), dw, n_out, pp.slots);
+      reduce_partials_kernel<T><<<(n_out + 31) / 32, 256, 0, s>>>(reinterpret_cast<const A*>(ws), dw, n_out, pp.slots * pp.parts);
       return check_launch();
     }
   }

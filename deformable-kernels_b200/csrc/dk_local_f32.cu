@@ -7,9 +7,10 @@
 //             lanes, read back one channel per lane), the hats of a (pixel, tap) are two 16-byte broadcasts
 //   offsets   lanes = pixels: G[tap, cell] += dK * W[c, cell], a warp per kernel row (48 accumulators), channel after channel;
 //             then the floor-based derivative weights contract G
-// Bound by multiply-adds: 21 (bank) and 17 (offsets) per pixel, tap and channel.  The kernels before gathered four cells per
-// tap with an address per lane, read x and dy one channel per lane from global memory (a line per lane) and added into
-// shared memory: N = 64, C = 144, 56 x 56: bank 2088 us, offsets 394 us.
+// Bound by instruction issue: 21 (bank) and 17 (offsets) multiply-adds per pixel, tap and channel, packed in pairs, beside
+// the loads.  The bank kernel before gathered four cells per tap with an address per lane, read x and dy one channel per lane
+// from global memory (a line per lane) and added into shared memory: N = 64, C = 144, 56 x 56 2088 -> 384 us (stride 2 562 ->
+// 119, N = 32, C = 384, 14 x 14 115 -> 39).
 #include <cuda_runtime.h>
 
 #include "dk_common.cuh"
@@ -82,33 +83,41 @@ __device__ __forceinline__ TilePos tile_pos(int tile, const TilePlan& t) {
 }
 
 // 4 bytes from global to shared memory, asynchronously; zero where !ok (the address is not read then)
-__device__ __forceinline__ void copy4(float* dst, const float* src, bool ok) {
-  asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;\n" ::"r"((unsigned)__cvta_generic_to_shared(dst)), "l"(src),
-               "r"(ok ? 4 : 0));
+__device__ __forceinline__ void copy4(unsigned dst, const float* src, bool ok) {
+  asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;\n" ::"r"(dst), "l"(src), "r"(ok ? 4 : 0));
 }
 __device__ __forceinline__ void copies_done() { asm volatile("cp.async.wait_all;\n" ::: "memory"); }
 
-// x and dy of channels c0 .. c0 + 31 of one tile; what lies outside the planes or beyond the last channel is zero.  All of a
-// warp's copies are in flight at once (loads into registers, four at a time, took as long as the arithmetic).
-template <int S>
+// One tile (rows x cols from row r0, column q0 of H x W planes) of 32 planes, the first n_c of which exist, into shared
+// memory; zero outside the planes.  All of a warp's copies are in flight at once, and a lane keeps its place in the tile and
+// walks down the channels: two additions per copy (with the whole address computed for each, the copies were half of all
+// instructions).
+template <int WARPS>
+__device__ __forceinline__ void stage_planes(float* s, const float* __restrict__ g0, int rows, int cols, unsigned magic, int pitch, int r0,
+                                             int q0, int H, int W, int n_c, int warp, int lane) {
+  const size_t plane = (size_t)H * W;
+  const unsigned s0 = (unsigned)__cvta_generic_to_shared(s) + 4u * (unsigned)(warp * pitch);
+  const unsigned d_step = 4u * (unsigned)(WARPS * pitch);
+  for (int e = lane; e < rows * cols; e += 32) {
+    const int r = over(e, cols, magic), ih = r0 + r, iw = q0 + (e - r * cols);
+    const bool in = ih >= 0 && ih < H && iw >= 0 && iw < W;
+    const float* src = g0 + (size_t)warp * plane + (in ? ih * W + iw : 0);
+    unsigned dst = s0 + 4u * e;
+#pragma unroll
+    for (int ch = 0; ch < 32; ch += WARPS) {
+      if (ch + warp < 32) copy4(dst, src, in && ch + warp < n_c);
+      dst += d_step;
+      src += WARPS * plane;
+    }
+  }
+}
+template <int S, int WARPS>
 __device__ __forceinline__ void stage_tile(float* xs, float* ys, const float* __restrict__ x, const float* __restrict__ dy, const Geom& g,
-                                           const TilePlan& t, const TilePos& tp, int c0, int warp, int warps, int lane) {
-  const int xe = t.XH * t.XW, ye = t.TH * t.TW;
-  const float* x0 = x + ((size_t)tp.n * g.C + c0) * g.HW;
-  const float* y0 = dy + ((size_t)tp.n * g.C + c0) * g.P;
+                                           const TilePlan& t, const TilePos& tp, int c0, int warp, int lane) {
   const int n_c = min(32, g.C - c0);
-  for (int e = lane; e < xe; e += 32) {
-    const int r = over(e, t.XW, t.magic_x), ih = tp.oh0 * S - 1 + r, iw = tp.ow0 * S - 1 + (e - r * t.XW);
-    const bool in = ih >= 0 && ih < g.H && iw >= 0 && iw < g.W;
-    const float* src = x0 + (in ? ih * g.W + iw : 0);
-    for (int ch = warp; ch < 32; ch += warps) copy4(xs + ch * t.xpitch + e, src + (size_t)(ch < n_c ? ch : 0) * g.HW, in && ch < n_c);
-  }
-  for (int e = lane; e < ye; e += 32) {
-    const int r = over(e, t.TW, t.magic_y), oh = tp.oh0 + r, ow = tp.ow0 + (e - r * t.TW);
-    const bool in = oh < g.Ho && ow < g.Wo;
-    const float* src = y0 + (in ? oh * g.Wo + ow : 0);
-    for (int ch = warp; ch < 32; ch += warps) copy4(ys + ch * t.ypitch + e, src + (size_t)(ch < n_c ? ch : 0) * g.P, in && ch < n_c);
-  }
+  stage_planes<WARPS>(xs, x + ((size_t)tp.n * g.C + c0) * g.HW, t.XH, t.XW, t.magic_x, t.xpitch, tp.oh0 * S - 1, tp.ow0 * S - 1, g.H, g.W,
+                      n_c, warp, lane);
+  stage_planes<WARPS>(ys, dy + ((size_t)tp.n * g.C + c0) * g.P, t.TH, t.TW, t.magic_y, t.ypitch, tp.oh0, tp.ow0, g.Ho, g.Wo, n_c, warp, lane);
 }
 
 // ------------------------------------------------------------------ bank
@@ -132,7 +141,7 @@ __global__ void __launch_bounds__(32 * kBankWarps, 2) f32_bank_kernel(const floa
   for (int tile = first; tile < last; ++tile) {
     const TilePos tp = tile_pos(tile, t);
     __syncthreads();
-    stage_tile<S>(xs, ys, x, dy, g, t, tp, c0, warp, kBankWarps, lane);
+    stage_tile<S, kBankWarps>(xs, ys, x, dy, g, t, tp, c0, warp, lane);
     for (int i = threadIdx.x; i < px * 9; i += 32 * kBankWarps) {
       const int tap = i / px, p = i - tap * px, r = over(p, t.TW, t.magic_y);
       const int oh = tp.oh0 + r, ow = tp.ow0 + (p - r * t.TW), fh = tap / 3, fw = tap - fh * 3;
@@ -192,8 +201,7 @@ __global__ void __launch_bounds__(32 * kBankWarps, 2) f32_bank_kernel(const floa
 }
 
 // ------------------------------------------------------------------ offsets
-// 12 warps: kernel row x (PQ quads of 32 pixels, 4 / PQ shares of the channels).  Few pixels in the call: fewer pixels per
-// block and more shares.
+// 12 warps: kernel row x (PQ quads of 32 pixels, 4 / PQ shares of the channels); the shares' sums meet in shared memory.
 constexpr int kOffWarps = 12;
 
 template <int S, int PQ>
@@ -216,7 +224,7 @@ __global__ void __launch_bounds__(32 * kOffWarps, 2) f32_offsets_kernel(const fl
   for (int i = 0; i < 24; ++i) G2[i / 8][i % 8] = 0;
   for (int c0 = 0; c0 < g.C; c0 += 32) {
     __syncthreads();
-    stage_tile<S>(xs, ys, x, dy, g, t, tp, c0, warp, kOffWarps, lane);
+    stage_tile<S, kOffWarps>(xs, ys, x, dy, g, t, tp, c0, warp, lane);
     for (int i = threadIdx.x; i < 32 * 16; i += 32 * kOffWarps) {
       const int c = c0 + (i >> 4), a = (i >> 2) & 3, b = i & 3;
       ws[i] = c < g.C && a < g.scH && b < g.scW ? __ldg(w + (size_t)c * g.cells + a * g.scW + b) : 0.f;
@@ -224,17 +232,17 @@ __global__ void __launch_bounds__(32 * kOffWarps, 2) f32_offsets_kernel(const fl
     copies_done();
     __syncthreads();
     const int n_c = min(32, g.C - c0);
-#pragma unroll 2
-    for (int ch = share; ch < n_c; ch += SH) {
-      const float yv = ys[ch * t.ypitch + pc];
-      const float* xp = xs + ch * t.xpitch + xo;
+    const float *yp = ys + share * t.ypitch + pc, *xp = xs + share * t.xpitch + xo;
+    const ulonglong2* wp = reinterpret_cast<const ulonglong2*>(ws + share * 16);
+#pragma unroll 4
+    for (int ch = share; ch < n_c; ch += SH, yp += SH * t.ypitch, xp += SH * t.xpitch, wp += SH * 4) {
+      const float yv = *yp;
       unsigned long long d[3];
 #pragma unroll
       for (int a = 0; a < 3; ++a) {
         const float v = yv * xp[a];
         d[a] = pair(v, v);
       }
-      const ulonglong2* wp = reinterpret_cast<const ulonglong2*>(ws + ch * 16);
 #pragma unroll
       for (int q = 0; q < 4; ++q) {
         const ulonglong2 wv = wp[q];
@@ -347,17 +355,21 @@ int local_filter_f32(const float* dy, const float* x, const float* rot, float* p
 
 int local_rot_f32(const float* dy, const float* x, const float* rot, const float* w, float* drot, const Geom& g, cudaStream_t s) {
   if (!f32_shape(g)) return DK_ERR_UNSUPPORTED;
+  // Calls with few pixels only: the general kernel (32 pixels per block, gathered cells) leaves SMs without a block there.
+  // N = 2, C = 64, 28 x 28: 13.6 -> 10.7 us; N = 32, C = 960, 7 x 7: 109 -> 82.  With the GPU full it is as fast or faster
+  // (N = 64, C = 144, 56 x 56: 383 against 392 us, stride 2: 117 against 161).
   TilePlan t = tile_plan(g, 128);
-  int pq = 4;
-  while (pq > 1 && t.tiles < 2 * device_sm_count()) t = tile_plan(g, 32 * (pq /= 2));
+  if (t.tiles >= 2 * device_sm_count()) return DK_ERR_UNSUPPORTED;
+  int pq = 2;
+  t = tile_plan(g, 64);
+  if (t.tiles < 2 * device_sm_count()) pq = 1, t = tile_plan(g, 32);
   size_t words = 512 + 32 * (size_t)(t.xpitch + t.ypitch);
   const size_t red = (size_t)pq * 3 * 48 * 32;
-  if (pq < 4 && words < red) words = red;
+  if (words < red) words = red;
   t.smem = words * sizeof(float);
   if (t.smem > (size_t)device_smem_optin()) return DK_ERR_UNSUPPORTED;
   void (*kern)(const float*, const float*, const float*, const float*, float*, const Geom, const TilePlan) =
-      g.sH == 1 ? (pq == 4 ? f32_offsets_kernel<1, 4> : pq == 2 ? f32_offsets_kernel<1, 2> : f32_offsets_kernel<1, 1>)
-                : (pq == 4 ? f32_offsets_kernel<2, 4> : pq == 2 ? f32_offsets_kernel<2, 2> : f32_offsets_kernel<2, 1>);
+      g.sH == 1 ? (pq == 2 ? f32_offsets_kernel<1, 2> : f32_offsets_kernel<1, 1>) : (pq == 2 ? f32_offsets_kernel<2, 2> : f32_offsets_kernel<2, 1>);
   const int rc = enable_smem(kern, t.smem);
   if (rc) return rc;
   kern<<<t.tiles, 32 * kOffWarps, t.smem, s>>>(dy, x, rot, w, drot, g, t);

@@ -16,7 +16,7 @@
 // values and five FMAs per (pixel, tap, channel) and is bound by instruction issue.
 //
 // Covers: fp16, 3x3 kernel, dilation 1, pad 1, stride 1 or 2 (equal in h and w), one rotation
-// group, at most 16 bank cells, channels a multiple of 16.
+// group, at most 16 bank cells.
 // Everything else stays on the SIMT kernels of dk_local.cu.
 #include <cstdlib>
 #include <cstring>
@@ -825,6 +825,29 @@ __global__ void reduce_bank_partials_kernel(const float* __restrict__ partial, _
   if (lane == 0) out[i] = __float2half_rn(s);
 }
 
+// both second stages in one launch: the first rot_blocks blocks sum offset gradients, the others bank gradients
+__global__ void reduce_both_partials_kernel(const float* __restrict__ rot_partial, __half* __restrict__ drot, size_t n_rot, int groups,
+                                            unsigned rot_blocks, const float* __restrict__ partial, __half* __restrict__ out, int C,
+                                            int cells, int nblocks) {
+  if (blockIdx.x < rot_blocks) {
+    const size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= n_rot) return;
+    float s = 0.f;
+    for (int k = 0; k < groups; ++k) s += rot_partial[(size_t)k * n_rot + i];
+    drot[i] = __float2half_rn(s);
+    return;
+  }
+  const int i = (int)(blockIdx.x - rot_blocks) * (blockDim.x >> 5) + (threadIdx.x >> 5);
+  const int lane = threadIdx.x & 31;
+  if (i >= C * cells) return;
+  const int c = i / cells, cell = i - c * cells;
+  float s = 0.f;
+  for (int k = lane; k < nblocks; k += 32) s += partial[((size_t)k * C + c) * 16 + cell];
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+  if (lane == 0) out[i] = __float2half_rn(s);
+}
+
 FiltPlan filt_plan_search(const Geom& g) {
   FiltPlan pl;
   const int S = g.sH;
@@ -1380,8 +1403,13 @@ int local_gw_mma(const __half* dy, const __half* x, const __half* rot, const __h
     const size_t n_out = (size_t)g.N * 18 * g.P;
     const size_t blocks = (n_out + 255) / 256;
     if (blocks > 0x7fffffffULL) return DK_ERR_UNSUPPORTED;
-    reduce_rot_partials_kernel<<<(unsigned)blocks, 256, 0, s>>>(gpart, drot, n_out, pl.groups);
-    if ((rc = check_launch())) return rc;
+    const size_t bank_blocks = ((size_t)g.C * g.cells + 7) / 8;
+    if (blocks + bank_blocks <= 0x7fffffffULL) {
+      reduce_both_partials_kernel<<<(unsigned)(blocks + bank_blocks), 256, 0, s>>>(gpart, drot, n_out, pl.groups, (unsigned)blocks, partial,
+                                                                                  dw, g.C, g.cells, pl.blocks_x);
+      return check_launch();
+    }
+    return DK_ERR_UNSUPPORTED;
   }
   const int n_out = g.C * g.cells;
   reduce_bank_partials_kernel<<<(n_out + 7) / 8, 256, 0, s>>>(partial, dw, g.C, g.cells, pl.blocks_x);

@@ -46,7 +46,7 @@ typedef enum dk_dtype { DK_F32 = 0, DK_F16 = 1, DK_F64 = 2 } dk_dtype;
 
 /* Devices and numeric limits.  Every pointer of a call must belong to the CURRENT device (cudaGetDevice()): the library
  * launches there, on the given stream, and never checks ownership.  fp16 calls on the tensor-core path (3x3, pad 1,
- * stride 1 or 2, at most 16 bank cells, channels a multiple of 16): forward and grad-input take the resampled kernel
+ * stride 1 or 2, at most 16 bank cells): forward and grad-input take the resampled kernel
  * value of a (pixel, tap, channel) from the tensor cores rounded to fp16 (relative 2^-11, the precision of the tensors
  * themselves), multiply it exactly with the fp16 input and sum in fp32;
  * grad-offsets and grad-bank feed the products grad_output * input to the tensor cores as fp16, so
