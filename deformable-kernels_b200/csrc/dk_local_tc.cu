@@ -402,7 +402,7 @@ __device__ __forceinline__ void copy_row(char* slot, const T* __restrict__ src, 
 template <typename T> __host__ __device__ constexpr int out_pitch() { return kStepSegs * 8 * (int)sizeof(T) + 16; }
 
 struct ConvSmem {  // byte offsets behind the row ring
-  unsigned beta, inv, out, bars, total;
+  unsigned beta, inv, out, segs, bars, total;
 };
 template <typename T, int MODE>
 __host__ __device__ inline ConvSmem conv_smem(unsigned ring_bytes, int groups, int nbuf) {
@@ -411,7 +411,8 @@ __host__ __device__ inline ConvSmem conv_smem(unsigned ring_bytes, int groups, i
   m.beta = (ring_bytes + 32 + 127) & ~127u;  // 32: what the last channel row's right edge may read
   m.inv = m.beta + nbuf * kPiece * (SPLIT ? 2 : 1);
   m.out = m.inv + (SPLIT ? groups * 128 : 0);
-  m.bars = m.out + (MODE == kData2 ? 0 : groups * 32 * out_pitch<T>());
+  m.segs = m.out + (MODE == kData2 ? 0 : groups * 32 * out_pitch<T>());
+  m.bars = m.segs + kDepth * kStepSegs * 16;
   m.total = m.bars + kBars * 8 + 16;
   return m;
 }
@@ -511,24 +512,14 @@ __global__ void __launch_bounds__(kThreads, 1)
     constexpr int NA = MODE == kData2 ? 16 : 8;
     int use = 0;
     for (int s = 0; s < steps; ++s) {
-      const int seg0 = lo + s * kStepSegs + team * 2;  // this pair's two segments
-      SegPos sp[2];
-      unsigned xr[2][Wk::rows];
-      bool live[2];
-#pragma unroll
-      for (int h = 0; h < 2; ++h) {
-        live[h] = seg0 + h < hi;
-        sp[h] = seg_pos(live[h] ? seg0 + h : lo, p);
-        const int k = sp[h].n * p.L + sp[h].g * Wk::S - j_first;
-#pragma unroll
-        for (int v = 0; v < Wk::rows; ++v) {
-          const int kk = k + v, sl = kk - (int)__umulhi((unsigned)kk, magic_r) * p.R;
-          xr[h][v] = sl * slot_bytes + 16 + sp[h].s * (8 * Wk::xs * E);
-        }
-      }
       if (!wait_bar(x_full + 8 * (s & (kDepth - 1)), (s / kDepth) & 1, abort_flag)) break;
-      if (STAGED && s > 0 && !wait_bar(o_free, (s - 1) & 1, abort_flag)) break;
-      bool ok = true;
+      // this pair's two segments, as the first loader left them: offsets of the source windows in the ring, and where the
+      // segment lies (worked out by every consumer warp for itself, this was a third of all instructions at 96 channels)
+      int4 sd[2];
+#pragma unroll
+      for (int h = 0; h < 2; ++h)
+        sd[h] = *reinterpret_cast<const int4*>(smem + sm.segs + ((s & (kDepth - 1)) * kStepSegs + team * 2 + h) * 16);
+      bool ok = true, out_free = s == 0;
       for (int rd = 0; rd < rounds; ++rd) {
         int grp = rd * 4 + q;
         if (rd == p.full) {
@@ -563,7 +554,7 @@ __global__ void __launch_bounds__(kThreads, 1)
             __syncwarp();
           }
           constexpr int row_of[3] = {0, MODE == kData2 ? 0 : 1, MODE == kData2 ? 1 : 2};
-          it.load(tmem + lanes + set * kSetCols + team * kSlotCols + h * 24, xc + xr[h][row_of[v]]);
+          it.load(tmem + lanes + set * kSetCols + team * kSlotCols + h * 24, xc + (row_of[v] == 0 ? sd[h].x : row_of[v] == 1 ? sd[h].y : sd[h].z));
           return true;
         };
         auto fetched = [&](Item<T, MODE>& it, int i) {
@@ -594,12 +585,12 @@ __global__ void __launch_bounds__(kThreads, 1)
             multiply<T, MODE>(acc[i & 1], item[0]);
           }
           if (MODE == kData2 && (i < 2 || i > 3)) {  // kernel row 0 completes the even row of the patch, 2 the odd one
-            const int h = i & 1, row = 2 * sp[h].g + (i > 3), col = 16 * sp[h].s;
-            if (live[h] && ch < cg && row < p.Hd) {
+            const int h = i & 1, row = 2 * (sd[h].w >> 8) + (i > 3), col = 16 * (sd[h].w & 255);
+            if (sd[h].w >= 0 && ch < cg && row < p.Hd) {
               float o[16];
 #pragma unroll
               for (int k = 0; k < 8; ++k) o[2 * k] = acc[h][k] * inv, o[2 * k + 1] = acc[h][NA - 8 + k] * inv;
-              store_row<T, 16>(dst + (((size_t)sp[h].n * p.C + c0 + ch) * p.Hd + row) * p.Wd + col, o, p.Wd - col, vec);
+              store_row<T, 16>(dst + (((size_t)sd[h].z * p.C + c0 + ch) * p.Hd + row) * p.Wd + col, o, p.Wd - col, vec);
             }
 #pragma unroll
             for (int k = 0; k < NA; ++k) acc[h][k] = 0.f;
@@ -608,6 +599,11 @@ __global__ void __launch_bounds__(kThreads, 1)
         if (!ok) break;
         use += 3;
         if (STAGED) {
+          if (!out_free) {  // the results of the step before are on their way
+            ok = wait_bar(o_free, (s - 1) & 1, abort_flag);
+            if (!ok) break;
+            out_free = true;
+          }
           char* o = smem + sm.out + ch * kOutPitch + team * (16 * E);
 #pragma unroll
           for (int h = 0; h < 2; ++h) {
@@ -623,6 +619,7 @@ __global__ void __launch_bounds__(kThreads, 1)
           }
         }
       }
+      if (STAGED && ok && !out_free) ok = wait_bar(o_free, (s - 1) & 1, abort_flag);  // a step without a group for this warp
       if (!ok) break;
       __syncwarp();
       if (lane == 0) {
@@ -702,6 +699,21 @@ __global__ void __launch_bounds__(kThreads, 1)
       }
       if (!ok) break;
       const unsigned bar = x_full + 8 * (s & (kDepth - 1));
+      if (lw == 0 && lane < kStepSegs) {
+        // {ring offsets of the rows it reads; kData2: two of them, sample, segment row and column (negative: no segment)}
+        const int b = lo + s * kStepSegs + lane;
+        const SegPos q = seg_pos(min(b, hi - 1), p);
+        const int k = q.n * p.L + q.g * Wk::S - j_first;
+        int o[3];
+#pragma unroll
+        for (int v = 0; v < 3; ++v) {
+          const int kk = k + (v < Wk::rows ? v : 0), sl = kk - (int)__umulhi((unsigned)kk, magic_r) * p.R;
+          o[v] = sl * (int)slot_bytes + 16 + q.s * (8 * Wk::xs * E);
+        }
+        *reinterpret_cast<int4*>(smem + sm.segs + ((s & (kDepth - 1)) * kStepSegs + lane) * 16) =
+            MODE == kData2 ? make_int4(o[0], o[1], q.n, b < hi ? q.g * 256 + q.s : -1) : make_int4(o[0], o[1], o[2], 0);
+      }
+      __syncwarp();
       if (NL == 1) {
         if (lane == 0) {
           if (last >= next) mbar_arrive_expect_tx(bar, (unsigned)(last - next + 1) * slot_bytes);
@@ -849,7 +861,7 @@ ConvPlan plan_conv(const Geom& g, const void* src, const void* dst) {
   else if ((reinterpret_cast<uintptr_t>(dst) & 3) == 0 && (p.Wd * E) % 4 == 0) p.store = 4;
   // padded row: 16 bytes in front; the column behind the last segment is the next row's front
   p.pitch = ((1 + (p.nseg * 8 * Wk::xs * E) / 16) | 1) * 16;
-  if (p.pitch < 16 + p.Ws * E || p.pitch > 1152) return pl;
+  if (p.pitch < 16 + p.Ws * E || p.pitch > 1152 || p.Hg >= (1 << 22)) return pl;
   pl.tma = (reinterpret_cast<uintptr_t>(src) & 15) == 0 && (p.Ws * E) % 16 == 0 && p.pitch / E <= 256;
   const int nbuf = beta_warps<T>(pl.tma ? 1 : kLoaders) / 2;
   const int need = step_rows(p.nseg, p.Hg, Wk::S, p.L, Wk::rows, kStepSegs);
