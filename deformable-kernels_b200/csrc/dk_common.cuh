@@ -208,6 +208,10 @@ int tc_error_status();
 // fp32 gradients towards offsets and bank (dk_local_f32.cu); the bank's leave as *blocks partial sums [block][C][cells]
 int local_rot_f32(const float* dy, const float* x, const float* rot, const float* w, float* drot, const Geom& g, cudaStream_t s);
 size_t local_filter_f32_workspace(const Geom& g);
+size_t deform_bank_workspace(const Geom& g);
+template <typename T>
+int deform_bank(const T* dy, const T* x, const T* off, const T* rot, float* partial, const Geom& g, size_t ws_bytes, int* blocks,
+                cudaStream_t s);
 int local_filter_f32(const float* dy, const float* x, const float* rot, float* partial, const Geom& g, size_t ws_bytes, int* blocks,
                      cudaStream_t s);
 size_t local_rot_mma_workspace(const Geom& g);

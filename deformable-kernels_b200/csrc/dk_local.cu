@@ -133,7 +133,17 @@ static int launch_local_conv(const T* src, const T* rot, const T* w, T* dst, con
   using A = typename Compute<T>::type;
   if constexpr (std::is_same<T, __half>::value) {
     if (mma_path_enabled()) {
-      int rc = local_conv_ring(src, rot, w, dst, g, TRANSPOSED, s);
+      int rc = DK_ERR_UNSUPPORTED;
+      // stride 1, rows that TMA fetches, three 32-channel groups or more: a pair of groups leaves half of the consumer warps
+      // idle at a time.  Against the band kernels on rows of 16 .. 96, 72 .. 384 channels 1.0 to 1.6 times as fast (C = 384,
+      // 32 x 32: 45 -> 29 us); against the ring kernels (rows of 112 / 56) up to 96 channels only (C = 96, 112 x 112: 283 ->
+      // 253 us, grad-input 300 -> 286; C = 144, 56 x 56, batch 32: 35 -> 40).
+      const bool ring_row = g.W == 112 || g.W == 56;
+      if (g.sH == 1 && g.W % 8 == 0 && g.C > 64 && (!ring_row || g.C <= 96)) {
+        rc = local_conv_tc<T>(src, rot, w, dst, g, TRANSPOSED, s);
+        if (rc != DK_ERR_UNSUPPORTED) return rc;
+      }
+      rc = local_conv_ring(src, rot, w, dst, g, TRANSPOSED, s);
       if (rc != DK_ERR_UNSUPPORTED) return rc;
       rc = local_conv_mma(src, rot, w, dst, g, TRANSPOSED, s);
       if (rc != DK_ERR_UNSUPPORTED) return rc;
@@ -626,6 +636,16 @@ template <typename T, bool DEFORM>
 static int filter_backward(const T* dy, const T* x, const T* off, const T* rot, T* dw, const Geom& g, void* ws,
                            size_t ws_bytes, cudaStream_t s, bool fit = false) {
   using A = typename Compute<T>::type;
+  if constexpr (DEFORM && sizeof(T) <= 4) {
+    int blocks = 0;
+    int rc = deform_bank<T>(dy, x, off, rot, reinterpret_cast<float*>(ws), g, ws_bytes, &blocks, s);
+    if (rc == DK_OK) {
+      const int n_out = g.C * g.cells;
+      reduce_partials_kernel<T><<<(n_out + 31) / 32, 256, 0, s>>>(reinterpret_cast<const A*>(ws), dw, n_out, blocks);
+      return check_launch();
+    }
+    if (rc != DK_ERR_UNSUPPORTED) return rc;
+  }
   if (DEFORM) {
     const PlanePlan pp = plane_plan<T, DEFORM>(g);
     if (pp.ok && pp.smem <= (size_t)device_smem_optin()) {

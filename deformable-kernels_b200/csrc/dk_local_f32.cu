@@ -1,4 +1,5 @@
-// Offset and bank gradients of the local deformable kernel in fp32 (3 x 3 taps, scopes up to 4 x 4).
+// Offset and bank gradients of the local deformable kernel in fp32, and the bank gradient of DK + DCN where the tensor-core
+// kernels do not apply (3 x 3 taps, scopes up to 4 x 4).
 //
 // Both consume the products dK = dy * x, and both are dense in the 16 bank cells here: with the hat products the sampled
 // cells need no data-dependent addresses, so every bank value and every hat product is one broadcast read for a whole warp.
@@ -312,7 +313,129 @@ __global__ void __launch_bounds__(32 * kOffWarps, 2) f32_offsets_kernel(const fl
   }
 }
 
+// ------------------------------------------------------------------ bank of DK + DCN
+// The same with x read by bilinear sampling: a warp per tap and a lane per pixel sample the 32 channels first (corners and
+// coefficients once per pixel and tap, neighbours on neighbouring lanes) and leave the samples in shared memory, where the
+// lanes take a channel each.  Before, every lane followed its own channel through global memory, or through whole planes on
+// chip with read-modify-writes of the bank cells in shared memory: 16 x 192 channels of 28 x 28, 3 x 3 scope, 167 -> 112 us;
+// 13 x 96 of 80 x 80 (planes too big to hold) 1324 -> 391; fp16, 13 x 88 of 80 x 80, 1177 -> 377.  Bound by the latency of
+// the corner loads.
+constexpr int kTapWarps = 9;
+constexpr int kSamplePitch = 32 * 9 + 1;
+
+template <typename T>
+__global__ void __launch_bounds__(32 * kTapWarps, 2) deform_bank_kernel(const T* __restrict__ dy, const T* __restrict__ x,
+                                                                        const T* __restrict__ off, const T* __restrict__ rot,
+                                                                        float* __restrict__ partial, const Geom g, const TilePlan t) {
+  extern __shared__ __align__(16) float smem_f[];
+  const int lane = threadIdx.x & 31, tap = threadIdx.x >> 5;
+  const int c0 = blockIdx.y * 32, n_c = min(32, g.C - c0), px = t.TH * t.TW;
+  float4* hats = reinterpret_cast<float4*>(smem_f);  // [pixel][tap][hat_u | hat_v]
+  float* xs = smem_f + 32 * 72;                      // [channel][pixel][tap]
+  float* ys = xs + 32 * kSamplePitch;                // [channel][33]
+  const float uh0 = 0.5f * (float)(g.scH - 3), uw0 = 0.5f * (float)(g.scW - 3);
+  const int fh = tap / 3, fw = tap - fh * 3;
+  unsigned long long acc[2][4];
+#pragma unroll
+  for (int i = 0; i < 8; ++i) acc[i >> 2][i & 3] = 0;
+  const int first = blockIdx.x * t.per_block, last = min(first + t.per_block, t.tiles);
+  const int r = over(lane, t.TW, t.magic_y);
+  for (int tile = first; tile < last; ++tile) {
+    const TilePos tp = tile_pos(tile, t);
+    const int oh = tp.oh0 + r, ow = tp.ow0 + (lane - r * t.TW);
+    const bool live = lane < px && oh < g.Ho && ow < g.Wo;
+    const size_t o = ((size_t)tp.n * 18 + 2 * tap) * g.P + (live ? oh * g.Wo + ow : 0);
+    Bilinear<float> bi;
+    float sc[4] = {0.f, 0.f, 0.f, 0.f};
+    bool used = false;
+    float4 hu = make_float4(0.f, 0.f, 0.f, 0.f), hv = hu;
+    if (live) {
+      used = image_setup<float>((float)(oh * g.sH - g.pH + fh * g.dH) + ld<float>(off + o),
+                                (float)(ow * g.sW - g.pW + fw * g.dW) + ld<float>(off + o + g.P), g, bi);
+      if (used) {
+        bilinear_value_coefs(bi, sc);
+        const float u = ((float)fh + ld<float>(rot + o)) + uh0, v = ((float)fw + ld<float>(rot + o + g.P)) + uw0;
+        hu.x = hat1(u), hu.y = g.scH > 1 ? hat1(u - 1.f) : 0.f, hu.z = g.scH > 2 ? hat1(u - 2.f) : 0.f, hu.w = g.scH > 3 ? hat1(u - 3.f) : 0.f;
+        hv.x = hat1(v), hv.y = g.scW > 1 ? hat1(v - 1.f) : 0.f, hv.z = g.scW > 2 ? hat1(v - 2.f) : 0.f, hv.w = g.scW > 3 ? hat1(v - 3.f) : 0.f;
+      }
+    }
+    __syncthreads();  // the tile before has been read
+    hats[(lane * 9 + tap) * 2] = hu;
+    hats[(lane * 9 + tap) * 2 + 1] = hv;
+    {
+      const T* xc = x + ((size_t)tp.n * g.C + c0) * g.HW;
+      float* d = xs + lane * 9 + tap;
+      int q[4] = {0, 0, 0, 0};
+      if (used) q[0] = bi.idx[0], q[1] = bi.idx[1], q[2] = bi.idx[2], q[3] = bi.idx[3];
+#pragma unroll 4
+      for (int ch = 0; ch < n_c; ++ch, xc += g.HW, d += kSamplePitch) {
+        float v = 0.f;
+        if (used) v = sc[0] * ld<float>(xc + q[0]) + sc[1] * ld<float>(xc + q[1]) + sc[2] * ld<float>(xc + q[2]) + sc[3] * ld<float>(xc + q[3]);
+        *d = v;
+      }
+    }
+    {
+      const T* yc = dy + ((size_t)tp.n * g.C + c0) * g.P + (live ? oh * g.Wo + ow : 0);
+      for (int ch = tap; ch < n_c; ch += kTapWarps) ys[ch * 33 + lane] = live ? ld<float>(yc + (size_t)ch * g.P) : 0.f;
+    }
+    __syncthreads();
+    if (lane < n_c) {
+      for (int p = tap; p < px; p += kTapWarps) {
+        const float* xp = xs + lane * kSamplePitch + p * 9;
+        const float yv = ys[lane * 33 + p];
+        const float4* hp = hats + p * 18;
+#pragma unroll
+        for (int i = 0; i < 9; ++i) {
+          const float dk = yv * xp[i];
+          const ulonglong2 a = *reinterpret_cast<const ulonglong2*>(hp + 2 * i);
+          const float4 b = hp[2 * i + 1];
+          const float bb[4] = {dk * b.x, dk * b.y, dk * b.z, dk * b.w};
+#pragma unroll
+          for (int k = 0; k < 4; ++k) {
+            const unsigned long long w2 = pair(bb[k], bb[k]);
+            fma2(acc[0][k], a.x, w2);
+            fma2(acc[1][k], a.y, w2);
+          }
+        }
+      }
+    }
+  }
+  __syncthreads();
+  float* red = smem_f;  // [warp][cell][lane]
+#pragma unroll
+  for (int i = 0; i < 8; ++i) {
+    const float2 v = unpair(acc[i >> 2][i & 3]);
+    const int cell = (i >> 2) * 8 + (i & 3);
+    red[(tap * 16 + cell) * 32 + lane] = v.x;
+    red[(tap * 16 + cell + 4) * 32 + lane] = v.y;
+  }
+  __syncthreads();
+  for (int i = threadIdx.x; i < 32 * 16; i += 32 * kTapWarps) {
+    const int cell = i >> 5, a = cell >> 2, b = cell & 3, c = c0 + (i & 31);
+    if (c < g.C && a < g.scH && b < g.scW) {
+      float sum = 0.f;
+#pragma unroll
+      for (int w = 0; w < kTapWarps; ++w) sum += red[w * 512 + i];
+      partial[((size_t)blockIdx.x * g.C + c) * g.cells + a * g.scW + b] = sum;
+    }
+  }
+}
+constexpr size_t kDeformBankSmem = (32 * 72 + 32 * (size_t)kSamplePitch + 32 * 33) * sizeof(float);
+static_assert(kDeformBankSmem >= (size_t)kTapWarps * 512 * sizeof(float), "the warps' sums reuse the tile's room");
+
 // ------------------------------------------------------------------ host side
+bool deform_bank_shape(const Geom& g) {
+  return g.kH == 3 && g.kW == 3 && g.G == 1 && g.scH <= 4 && g.scW <= 4 && (long long)g.N * g.P < 0x3fffffff && (g.C + 31) / 32 <= 65535;
+}
+TilePlan deform_bank_plan(const Geom& g) {
+  TilePlan t = tile_plan(g, 32);
+  int want = 4 * device_sm_count() / ((g.C + 31) / 32);
+  if (want < 1) want = 1;
+  t.per_block = (t.tiles + want - 1) / want;
+  t.blocks = (t.tiles + t.per_block - 1) / t.per_block;
+  t.smem = kDeformBankSmem;
+  return t;
+}
 bool f32_shape(const Geom& g) {
   return g.kH == 3 && g.kW == 3 && g.dH == 1 && g.dW == 1 && g.pH == 1 && g.pW == 1 && g.sH == g.sW && (g.sH == 1 || g.sH == 2) &&
          g.G == 1 && g.scH <= 4 && g.scW <= 4 && (long long)g.N * g.P < 0x3fffffff;
@@ -375,5 +498,24 @@ int local_rot_f32(const float* dy, const float* x, const float* rot, const float
   kern<<<t.tiles, 32 * kOffWarps, t.smem, s>>>(dy, x, rot, w, drot, g, t);
   return check_launch();
 }
+
+size_t deform_bank_workspace(const Geom& g) {
+  return deform_bank_shape(g) ? (size_t)deform_bank_plan(g).blocks * g.C * g.cells * sizeof(float) : 0;
+}
+
+template <typename T>
+int deform_bank(const T* dy, const T* x, const T* off, const T* rot, float* partial, const Geom& g, size_t ws_bytes, int* blocks,
+                cudaStream_t s) {
+  if (!deform_bank_shape(g)) return DK_ERR_UNSUPPORTED;
+  const TilePlan t = deform_bank_plan(g);
+  if (partial == nullptr || ws_bytes < (size_t)t.blocks * g.C * g.cells * sizeof(float)) return DK_ERR_WORKSPACE;
+  const int rc = enable_smem(deform_bank_kernel<T>, t.smem);
+  if (rc) return rc;
+  deform_bank_kernel<T><<<dim3(t.blocks, (g.C + 31) / 32), 32 * kTapWarps, t.smem, s>>>(dy, x, off, rot, partial, g, t);
+  *blocks = t.blocks;
+  return check_launch();
+}
+template int deform_bank<float>(const float*, const float*, const float*, const float*, float*, const Geom&, size_t, int*, cudaStream_t);
+template int deform_bank<__half>(const __half*, const __half*, const __half*, const __half*, float*, const Geom&, size_t, int*, cudaStream_t);
 
 }  // namespace dk
