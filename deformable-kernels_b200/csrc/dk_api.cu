@@ -304,8 +304,11 @@ int dk_deform_sample_depthwise_forward(const void* input, const void* offset, co
 size_t dk_deform_sample_depthwise_backward_data_workspace_bytes(const dk_geom* g, int dtype) {
   Geom gg;
   if (!make_geom(g, &gg) || !dtype_ok(dtype)) return 0;
-  if (dtype != DK_F16) return 0;
-  return align256((size_t)gg.N * gg.C * gg.HW * sizeof(float));
+  if (dtype == DK_F64) return 0;
+  size_t need = dtype == DK_F16 ? align256((size_t)gg.N * gg.C * gg.HW * sizeof(float)) : 0;
+  const size_t bins = align256(deform_bins_workspace(gg, dtype == DK_F16 ? 2 : 4));
+  if (bins > need) need = bins;
+  return need;
 }
 
 int dk_deform_sample_depthwise_backward_data(const void* grad_output, const void* offset, const void* rotation,
@@ -420,9 +423,10 @@ int dk_deform_sample_depthwise_backward(const void* grad_output, const void* inp
     return rc;
   }
   if (grad_input) {
-    if (data_ws && (!workspace || workspace_bytes < data_ws)) return DK_ERR_WORKSPACE;
-    rc = dk_deform_sample_depthwise_backward_data(grad_output, offset, rotation, filter, grad_input, g, dtype, workspace,
-                                                  data_ws, stream);
+    const bool room = workspace && workspace_bytes >= data_ws;
+    if (dtype == DK_F16 && !room) return DK_ERR_WORKSPACE;  // fp32 falls back to a kernel that needs none
+    rc = dk_deform_sample_depthwise_backward_data(grad_output, offset, rotation, filter, grad_input, g, dtype,
+                                                  room ? workspace : nullptr, room ? data_ws : 0, stream);
     if (rc) return rc;
   }
   bool bank_done = false;

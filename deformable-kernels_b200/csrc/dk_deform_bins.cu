@@ -1,0 +1,314 @@
+// Grad-input of DK + DCN where the tensor-core kernel does not apply (fp32; fp16 with channels that are no multiple of 16, other
+// scopes, planes beyond 56 x 56), one offset group.
+//
+// The scatter of dy * k into the four corners of every sample point is 36 float additions to colliding addresses per output,
+// and shared memory adds floats with a compare-and-swap loop: 0.25 ms for 16 x 192 channels of 28 x 28 (350 G additions / s),
+// as slow as additions in L2.  But where a sample lands does not depend on the channel.  So the samples (pixel, tap) are first
+// sorted by the cell of the input grid they fall into, once for all channels (dcn_bins_kernel), and then a warp walks through
+// the cells of a row with 32 channels on its lanes and the four corner sums in registers: no atomics, no collisions, one
+// multiply-add per corner (dcn_gather_kernel).
+#include <cooperative_groups.h>
+
+#include "dk_common.cuh"
+
+namespace dk {
+namespace {
+
+namespace cg = cooperative_groups;
+
+constexpr int kSortBlocks = 8, kSortThreads = 1024;  // a cluster of 8 blocks sorts one sample
+constexpr int kGatherWarps = 8;
+
+struct BinPlan {
+  int bins, rec_per_n, Cp, groups;  // (H + 1) x (W + 1) cells; taps * P samples; channels rounded up to 32
+  int R, bands, segs;               // destination rows of a block, blocks per plane, pieces of a row of cells
+  size_t starts_bytes, recs_bytes, bytes, sort_smem, gather_smem;
+};
+
+// one sample point: corner coefficients of the image and of the bank, {bank cell * 32, column of the cell, pixel * Cp, 0}
+struct Rec {
+  float4 ci, cb;
+  int4 at;
+};
+
+// cell of sample i = tap * P + p, or -1 where it adds nothing
+template <typename T>
+__device__ __forceinline__ int sample_cell(int i, int n, const T* __restrict__ off, const T* __restrict__ rot, const Geom& g, Rec* rec,
+                                           int Cp) {
+  const int tap = i / g.P, p = i - tap * g.P, fh = tap / g.kW, fw = tap - fh * g.kW;
+  const int oh = p / g.Wo, ow = p - oh * g.Wo;
+  const size_t o = ((size_t)n * g.taps + tap) * 2 * g.P + p;
+  const float ph = (float)(oh * g.sH - g.pH + fh * g.dH) + ld<float>(off + o);
+  const float pw = (float)(ow * g.sW - g.pW + fw * g.dW) + ld<float>(off + o + g.P);
+  const float u = ((float)fh + ld<float>(rot + o)) + (float)(g.scH - g.kH) * 0.5f;
+  const float v = ((float)fw + ld<float>(rot + o + g.P)) + (float)(g.scW - g.kW) * 0.5f;
+  // written so that NaN fails; what passes is in range for the conversions below
+  if (!(ph > -1.f && pw > -1.f && ph < (float)g.H && pw < (float)g.W)) return -1;
+  if (!(u > -1.f && v > -1.f && u < (float)g.scH && v < (float)g.scW)) return -1;
+  const float fph = floorf(ph), fpw = floorf(pw);
+  const int h0 = (int)fph, w0 = (int)fpw;
+  if (rec != nullptr) {
+    const float lh = ph - fph, lw = pw - fpw, hh = 1.f - lh, hw = 1.f - lw;
+    const float fu = floorf(u), fv = floorf(v), lu = u - fu, lv = v - fv, hu = 1.f - lu, hv = 1.f - lv;
+    rec->ci = make_float4(hh * hw, hh * lw, lh * hw, lh * lw);
+    rec->cb = make_float4(hu * hv, hu * lv, lu * hv, lu * lv);
+    rec->at = make_int4((((int)fu + 1) * (g.scW + 2) + (int)fv + 1) * 32, w0 + 1, p * Cp, 0);
+  }
+  return (h0 + 1) * (g.W + 1) + w0 + 1;
+}
+
+// Counting sort of the samples of one (n) by cell: every block of the cluster counts its share in shared memory, the blocks
+// share the prefix sums (an eighth of the cells each, through distributed shared memory), then every block places its samples.
+// The clusters after the first N turn dy [C][P] into [P][Cp], so that 32 channels of a pixel are one line for the gather.
+template <typename T>
+__global__ void __launch_bounds__(kSortThreads) dcn_bins_kernel(const T* __restrict__ dy, const T* __restrict__ off,
+                                                                const T* __restrict__ rot, int* __restrict__ starts,
+                                                                Rec* __restrict__ recs, T* __restrict__ dyt, const Geom g,
+                                                                const BinPlan t) {
+  extern __shared__ __align__(16) int hist[];
+  __shared__ int slices[kSortBlocks], warp_sum[32];
+  __shared__ float tile[32][33];
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int n = blockIdx.x / kSortBlocks, rank = blockIdx.x - n * kSortBlocks;
+  if (n >= g.N) {
+    const int tiles_p = (g.P + 31) / 32;
+    const long long tiles = (long long)g.N * t.groups * tiles_p;
+    const long long step = gridDim.x - (long long)g.N * kSortBlocks;
+    for (long long k = blockIdx.x - (long long)g.N * kSortBlocks; k < tiles; k += step) {
+      const int m = (int)(k / (t.groups * tiles_p)), r = (int)(k - (long long)m * t.groups * tiles_p);
+      const int grp = r / tiles_p, p0 = (r - grp * tiles_p) * 32;
+      const int c = grp * 32 + warp;
+      __syncthreads();
+      tile[warp][lane] = (c < g.C && p0 + lane < g.P) ? ld<float>(dy + ((size_t)m * g.C + c) * g.P + p0 + lane) : 0.f;
+      __syncthreads();
+      if (p0 + warp < g.P) st<T, float>(dyt + ((size_t)m * g.P + p0 + warp) * t.Cp + grp * 32 + lane, tile[lane][warp]);
+    }
+    return;
+  }
+  cg::cluster_group cluster = cg::this_cluster();
+  for (int i = tid; i < t.bins; i += kSortThreads) hist[i] = 0;
+  __syncthreads();
+  for (int i = rank * kSortThreads + tid; i < t.rec_per_n; i += kSortBlocks * kSortThreads) {
+    const int cell = sample_cell<T>(i, n, off, rot, g, nullptr, 0);
+    if (cell >= 0) atomicAdd(&hist[cell], 1);
+  }
+  cluster.sync();
+  const int per = (t.bins + kSortBlocks - 1) / kSortBlocks, q = (per + kSortThreads - 1) / kSortThreads;
+  const int hi = min((rank + 1) * per, t.bins), lo = rank * per + tid * q, end = min(lo + q, hi);
+  int sum = 0;
+  for (int b = lo; b < end; ++b)
+    for (int k = 0; k < kSortBlocks; ++k) sum += cluster.map_shared_rank(hist, k)[b];
+  int scan = sum;
+#pragma unroll
+  for (int d = 1; d < 32; d <<= 1) {
+    const int o = __shfl_up_sync(0xffffffffu, scan, d);
+    if (lane >= d) scan += o;
+  }
+  if (lane == 31) warp_sum[warp] = scan;
+  __syncthreads();
+  int base = 0, total = 0;
+  for (int w = 0; w < kSortThreads / 32; ++w) {
+    if (w < warp) base += warp_sum[w];
+    total += warp_sum[w];
+  }
+  if (tid < kSortBlocks) cluster.map_shared_rank(slices, tid)[rank] = total;
+  cluster.sync();
+  int run = base + scan - sum, before = 0;
+  for (int k = 0; k < rank; ++k) before += slices[k];
+  run += before;
+  int* out = starts + (size_t)n * (t.bins + 1);
+  for (int b = lo; b < end; ++b) {
+    out[b] = run;
+    for (int k = 0; k < kSortBlocks; ++k) {
+      int* h = cluster.map_shared_rank(hist, k) + b;
+      const int c = *h;
+      *h = run;
+      run += c;
+    }
+  }
+  if (rank == kSortBlocks - 1 && tid == 0) out[t.bins] = before + total;
+  cluster.sync();
+  Rec* to = recs + (size_t)n * t.rec_per_n;
+  for (int i = rank * kSortThreads + tid; i < t.rec_per_n; i += kSortBlocks * kSortThreads) {
+    Rec r;
+    const int cell = sample_cell<T>(i, n, off, rot, g, &r, t.Cp);
+    if (cell >= 0) to[atomicAdd(&hist[cell], 1)] = r;
+  }
+}
+
+// Block = 32 channels of R rows of dx.  A unit of a warp is a piece of a row of cells: the samples of a cell add to
+// S00 .. S11, which at the end of the cell go to its four corners; the right-hand pair is carried to the next cell.  Even rows
+// of cells write their two rows of dx first, then the odd rows add theirs, so no element has two writers.  What a piece
+// carries past its end waits in `seam`.  A sample costs three shared loads of its record, one line of dy, four bank reads
+// and eight multiply-adds per 32 channels.
+template <typename T>
+__global__ void __launch_bounds__(32 * kGatherWarps) dcn_gather_kernel(const T* __restrict__ dyt, const int* __restrict__ starts,
+                                                                       const Rec* __restrict__ recs, const T* __restrict__ w,
+                                                                       T* __restrict__ dx, const Geom g, const BinPlan t) {
+  extern __shared__ __align__(16) float4 smem4[];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int n = blockIdx.x / t.bands, r0 = (blockIdx.x - n * t.bands) * t.R, rows = min(t.R, g.H - r0);
+  const int c0 = blockIdx.y * 32, n_c = min(32, g.C - c0), bw = g.scW + 2, W1 = g.W + 1;
+  float4* stage = smem4 + warp * 96;                                   // [32 records]
+  float* bank = reinterpret_cast<float*>(smem4 + kGatherWarps * 96);   // [cell of the zero-bordered bank][channel]
+  float* seam = bank + (g.scH + 2) * bw * 32;                          // [row of cells][piece][upper | lower][channel]
+  float* acc = seam + (t.R + 1) * t.segs * 64;                         // [row][column][33]
+  for (int i = threadIdx.x; i < (g.scH + 2) * bw * 32; i += 32 * kGatherWarps) {
+    const int cell = i >> 5, a = cell / bw - 1, b = cell - (a + 1) * bw - 1, c = i & 31;
+    bank[i] = (c < n_c && a >= 0 && a < g.scH && b >= 0 && b < g.scW) ? ld<float>(w + (size_t)(c0 + c) * g.cells + a * g.scW + b) : 0.f;
+  }
+  __syncthreads();
+  const T* yl = dyt + (size_t)n * g.P * t.Cp + c0 + lane;
+  const int* st_n = starts + (size_t)n * (t.bins + 1);
+  const float4* rc_n = reinterpret_cast<const float4*>(recs + (size_t)n * t.rec_per_n);
+  const float* bl = bank + lane;
+  for (int phase = 0; phase < 2; ++phase) {
+    const int n_rows = (rows + 2 - phase) >> 1;  // rows of cells r0 - 1 .. r0 + rows - 1, every other one
+    for (int unit = warp; unit < n_rows * t.segs; unit += kGatherWarps) {
+      const int k = unit / t.segs, seg = unit - k * t.segs, i = 2 * k + phase;  // row r0 - 1 + i of the plane
+      const int b0 = seg * W1 / t.segs, b1 = (seg + 1) * W1 / t.segs;
+      const int* sr = st_n + (r0 + i) * W1;
+      const int first = __ldg(sr + b0), last = __ldg(sr + b1);
+      float* up = i >= 1 ? acc + (size_t)(i - 1) * g.W * 33 + lane : nullptr;
+      float* low = i < rows ? acc + (size_t)i * g.W * 33 + lane : nullptr;
+      int cur = b0;
+      float s00 = 0.f, s01 = 0.f, s10 = 0.f, s11 = 0.f, cu = 0.f, cl = 0.f;
+      auto flush = [&]() {
+        if (cur > 0) {
+          const int o = (cur - 1) * 33;
+          if (up) up[o] = phase ? up[o] + (s00 + cu) : s00 + cu;
+          if (low) low[o] = phase ? low[o] + (s10 + cl) : s10 + cl;
+        }
+        cu = s01, cl = s11;
+        s00 = s01 = s10 = s11 = 0.f;
+        ++cur;
+      };
+      float4 next[3];
+      auto fetch = [&](int at) {
+        const int lim = (last - at) * 3;
+#pragma unroll
+        for (int j = 0; j < 3; ++j)
+          if (lane + 32 * j < lim) next[j] = __ldg(rc_n + (size_t)at * 3 + lane + 32 * j);
+      };
+      if (first < last) fetch(first);
+      for (int at = first; at < last; at += 32) {
+        __syncwarp();
+#pragma unroll
+        for (int j = 0; j < 3; ++j) stage[lane + 32 * j] = next[j];
+        __syncwarp();
+        if (at + 32 < last) fetch(at + 32);
+        const int cnt = min(32, last - at);
+        for (int k0 = 0; k0 < cnt; k0 += 8) {
+          float yv[8];
+#pragma unroll
+          for (int j = 0; j < 8; ++j)
+            if (k0 + j < cnt) yv[j] = ld<float>(yl + reinterpret_cast<const int*>(stage + (k0 + j) * 3 + 2)[2]);
+#pragma unroll
+          for (int j = 0; j < 8; ++j) {
+            if (k0 + j < cnt) {
+              const float4 ci = stage[(k0 + j) * 3], cb = stage[(k0 + j) * 3 + 1];
+              const int2 a2 = *reinterpret_cast<const int2*>(stage + (k0 + j) * 3 + 2);
+              while (cur < a2.y) flush();
+              const float* bk = bl + a2.x;
+              const float kv = cb.x * bk[0] + cb.y * bk[32] + cb.z * bk[bw * 32] + cb.w * bk[bw * 32 + 32];
+              const float v = kv * yv[j];
+              s00 += ci.x * v, s01 += ci.y * v, s10 += ci.z * v, s11 += ci.w * v;
+            }
+          }
+        }
+      }
+      while (cur < b1) flush();
+      seam[((i * t.segs + seg) * 2) * 32 + lane] = cu;
+      seam[((i * t.segs + seg) * 2 + 1) * 32 + lane] = cl;
+    }
+    __syncthreads();
+  }
+  if (t.segs > 1) {
+    for (int u = warp; u < rows * (t.segs - 1); u += kGatherWarps) {
+      const int d = u / (t.segs - 1), seg = u - d * (t.segs - 1), b = (seg + 1) * W1 / t.segs;
+      acc[((size_t)d * g.W + b - 1) * 33 + lane] +=
+          seam[(((d + 1) * t.segs + seg) * 2) * 32 + lane] + seam[((d * t.segs + seg) * 2 + 1) * 32 + lane];
+    }
+    __syncthreads();
+  }
+  const int span = rows * g.W;
+  for (int c = warp; c < n_c; c += kGatherWarps) {
+    T* o = dx + ((size_t)n * g.C + c0 + c) * g.HW + (size_t)r0 * g.W;
+    for (int e = lane; e < span; e += 32) st<T, float>(o + e, acc[e * 33 + c]);
+  }
+}
+
+size_t round256(size_t v) { return (v + 255) & ~(size_t)255; }
+
+bool bin_plan(const Geom& g, size_t elem, BinPlan& t) {
+  const long long bins = (long long)(g.H + 1) * (g.W + 1), recs = (long long)g.taps * g.P;
+  t.groups = (g.C + 31) / 32;
+  t.Cp = 32 * t.groups;
+  if (g.G != 1 || bins * 4 > 160 * 1024 || recs > 0x3fffffff || (long long)g.P * t.Cp > 0x7fffffff || t.groups > 65535) return false;
+  t.bins = (int)bins, t.rec_per_n = (int)recs;
+  // rows of a block: up to 56 KB of sums, three blocks (24 warps) on an SM; more and smaller blocks where they would not
+  // fill the chip (a row of cells between two blocks is walked through twice)
+  const int row = g.W * 33 * 4, sms = device_sm_count();
+  int R = 56 * 1024 / row;
+  if (R < 1) return false;
+  const long long planes = (long long)g.N * t.groups;
+  int bands = (g.H + R - 1) / R;
+  const long long fill = (2 * (long long)sms + planes - 1) / planes;
+  if (fill > bands) bands = (int)(fill < (g.H + 1) / 2 ? fill : (g.H + 1) / 2);
+  t.R = (g.H + bands - 1) / bands;
+  t.bands = (g.H + t.R - 1) / t.R;
+  // pieces of a row so that both halves of the rows give every warp one
+  t.segs = (2 * kGatherWarps + t.R) / (t.R + 1);
+  if (t.segs > (g.W + 1) / 4) t.segs = (g.W + 1) / 4 > 0 ? (g.W + 1) / 4 : 1;
+  t.sort_smem = (size_t)t.bins * 4;
+  t.gather_smem = (size_t)kGatherWarps * 1536 + ((size_t)(g.scH + 2) * (g.scW + 2) * 32 + (size_t)(t.R + 1) * t.segs * 64 + (size_t)t.R * g.W * 33) * 4;
+  if (t.gather_smem > 110 * 1024 || (long long)g.N * t.bands > 0x7fffffff || (long long)g.N * kSortBlocks > 0x3fffffff) return false;
+  t.starts_bytes = round256((size_t)g.N * (t.bins + 1) * sizeof(int));
+  t.recs_bytes = round256((size_t)g.N * t.rec_per_n * sizeof(Rec));
+  t.bytes = t.starts_bytes + t.recs_bytes + round256((size_t)g.N * g.P * t.Cp * elem);
+  return true;
+}
+
+}  // namespace
+
+size_t deform_bins_workspace(const Geom& g, size_t elem) {
+  BinPlan t;
+  return bin_plan(g, elem, t) ? t.bytes : 0;
+}
+
+template <typename T>
+int deform_data_bins(const T* dy, const T* off, const T* rot, const T* w, T* dx, const Geom& g, void* ws, size_t ws_bytes, cudaStream_t s) {
+  BinPlan t;
+  if (!bin_plan(g, sizeof(T), t) || ws == nullptr || ws_bytes < t.bytes) return DK_ERR_UNSUPPORTED;
+  int* starts = reinterpret_cast<int*>(ws);
+  Rec* recs = reinterpret_cast<Rec*>(reinterpret_cast<char*>(ws) + t.starts_bytes);
+  T* dyt = reinterpret_cast<T*>(reinterpret_cast<char*>(ws) + t.starts_bytes + t.recs_bytes);
+  int rc = enable_smem(dcn_bins_kernel<T>, t.sort_smem);
+  if (rc) return rc;
+  rc = enable_smem(dcn_gather_kernel<T>, t.gather_smem);
+  if (rc) return rc;
+  const long long tiles = (long long)g.N * t.groups * ((g.P + 31) / 32);
+  long long movers = (tiles + 4 * kSortBlocks - 1) / (4 * kSortBlocks);
+  if (movers > 2 * device_sm_count() / kSortBlocks) movers = 2 * device_sm_count() / kSortBlocks;
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3((unsigned)((g.N + movers) * kSortBlocks));
+  cfg.blockDim = dim3(kSortThreads);
+  cfg.dynamicSmemBytes = t.sort_smem;
+  cfg.stream = s;
+  cudaLaunchAttribute attr;
+  attr.id = cudaLaunchAttributeClusterDimension;
+  attr.val.clusterDim.x = kSortBlocks, attr.val.clusterDim.y = attr.val.clusterDim.z = 1;
+  cfg.attrs = &attr;
+  cfg.numAttrs = 1;
+  const cudaError_t e = cudaLaunchKernelEx(&cfg, dcn_bins_kernel<T>, dy, off, rot, starts, recs, dyt, g, t);
+  if (e != cudaSuccess) {
+    set_last_cuda_error(e);
+    return DK_ERR_CUDA;
+  }
+  dcn_gather_kernel<T><<<dim3((unsigned)(g.N * t.bands), t.groups), 32 * kGatherWarps, t.gather_smem, s>>>(dyt, starts, recs, w, dx, g, t);
+  return check_launch();
+}
+template int deform_data_bins<float>(const float*, const float*, const float*, const float*, float*, const Geom&, void*, size_t, cudaStream_t);
+template int deform_data_bins<__half>(const __half*, const __half*, const __half*, const __half*, __half*, const Geom&, void*, size_t, cudaStream_t);
+
+}  // namespace dk
