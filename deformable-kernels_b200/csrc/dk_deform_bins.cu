@@ -17,11 +17,11 @@ namespace {
 namespace cg = cooperative_groups;
 
 constexpr int kSortBlocks = 8, kSortThreads = 1024;  // a cluster of 8 blocks sorts one sample
-constexpr int kGatherWarps = 8;
+constexpr int kGatherWarps = 8, kMovePixels = 128;
 
 struct BinPlan {
-  int bins, rec_per_n, Cp, groups;  // (H + 1) x (W + 1) cells; taps * P samples; channels rounded up to 32
-  int R, bands, segs;               // destination rows of a block, blocks per plane, pieces of a row of cells
+  int bins, rec_per_n, Cp, groups;  // (H + 1) x (W + 1) cells; taps * P samples; channels rounded up to those of a block
+  int V, R, bands, segs;               // destination rows of a block, blocks per plane, pieces of a row of cells
   size_t starts_bytes, recs_bytes, bytes, sort_smem, gather_smem;
 };
 
@@ -59,7 +59,8 @@ __device__ __forceinline__ int sample_cell(int i, int n, const T* __restrict__ o
 
 // Counting sort of the samples of one (n) by cell: every block of the cluster counts its share in shared memory, the blocks
 // share the prefix sums (an eighth of the cells each, through distributed shared memory), then every block places its samples.
-// The clusters after the first N turn dy [C][P] into [P][Cp], so that 32 channels of a pixel are one line for the gather.
+// The clusters after the first N turn dy [C][P] into [P + 1][Cp] (the last pixel is zero), so that the channels of a pixel are
+// neighbours for the gather.
 template <typename T>
 __global__ void __launch_bounds__(kSortThreads) dcn_bins_kernel(const T* __restrict__ dy, const T* __restrict__ off,
                                                                 const T* __restrict__ rot, int* __restrict__ starts,
@@ -67,21 +68,27 @@ __global__ void __launch_bounds__(kSortThreads) dcn_bins_kernel(const T* __restr
                                                                 const BinPlan t) {
   extern __shared__ __align__(16) int hist[];
   __shared__ int slices[kSortBlocks], warp_sum[32];
-  __shared__ float tile[32][33];
+  __shared__ float tile[kMovePixels * 33];
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int n = blockIdx.x / kSortBlocks, rank = blockIdx.x - n * kSortBlocks;
   if (n >= g.N) {
-    const int tiles_p = (g.P + 31) / 32;
-    const long long tiles = (long long)g.N * t.groups * tiles_p;
-    const long long step = gridDim.x - (long long)g.N * kSortBlocks;
-    for (long long k = blockIdx.x - (long long)g.N * kSortBlocks; k < tiles; k += step) {
-      const int m = (int)(k / (t.groups * tiles_p)), r = (int)(k - (long long)m * t.groups * tiles_p);
-      const int grp = r / tiles_p, p0 = (r - grp * tiles_p) * 32;
-      const int c = grp * 32 + warp;
+    const int tiles_p = (g.P + 1 + kMovePixels - 1) / kMovePixels, per_n = t.Cp / 32 * tiles_p, step = gridDim.x - g.N * kSortBlocks;
+    for (int k = blockIdx.x - g.N * kSortBlocks; k < g.N * per_n; k += step) {
+      const int m = k / per_n, r = k - m * per_n, grp = r / tiles_p, p0 = (r - grp * tiles_p) * kMovePixels;
+      const T* from = dy + ((size_t)m * g.C + min(grp * 32 + warp, g.C - 1)) * g.P;
+      const bool has = grp * 32 + warp < g.C;
+      float v[kMovePixels / 32];
+#pragma unroll
+      for (int e = 0; e < kMovePixels / 32; ++e)
+        v[e] = has && p0 + e * 32 + lane < g.P ? ld<float>(from + p0 + e * 32 + lane) : 0.f;
       __syncthreads();
-      tile[warp][lane] = (c < g.C && p0 + lane < g.P) ? ld<float>(dy + ((size_t)m * g.C + c) * g.P + p0 + lane) : 0.f;
+#pragma unroll
+      for (int e = 0; e < kMovePixels / 32; ++e) tile[(e * 32 + lane) * 33 + warp] = v[e];
       __syncthreads();
-      if (p0 + warp < g.P) st<T, float>(dyt + ((size_t)m * g.P + p0 + warp) * t.Cp + grp * 32 + lane, tile[lane][warp]);
+      T* to = dyt + ((size_t)m * (g.P + 1) + p0 + warp) * t.Cp + grp * 32 + lane;
+#pragma unroll
+      for (int e = 0; e < kMovePixels / 32; ++e)
+        if (p0 + warp + e * 32 <= g.P) st<T, float>(to + (size_t)e * 32 * t.Cp, tile[(warp + e * 32) * 33 + lane]);
     }
     return;
   }
@@ -136,32 +143,53 @@ __global__ void __launch_bounds__(kSortThreads) dcn_bins_kernel(const T* __restr
   }
 }
 
-// Block = 32 channels of R rows of dx.  A unit of a warp is a piece of a row of cells: the samples of a cell add to
+// one or two neighbouring channels
+template <typename T, int V>
+__device__ __forceinline__ void get(const T* p, float (&v)[V]) {
+  if constexpr (V == 1) {
+    v[0] = static_cast<float>(*p);
+  } else if constexpr (sizeof(T) == 4) {
+    const float2 q = *reinterpret_cast<const float2*>(p);
+    v[0] = q.x, v[1] = q.y;
+  } else {
+    const float2 q = __half22float2(*reinterpret_cast<const __half2*>(p));
+    v[0] = q.x, v[1] = q.y;
+  }
+}
+template <int V>
+__device__ __forceinline__ void put(float* p, const float (&v)[V]) {
+  if constexpr (V == 1) *p = v[0];
+  else *reinterpret_cast<float2*>(p) = make_float2(v[0], v[1]);
+}
+
+// Block = 32 V channels of R rows of dx, V channels on a lane.  A unit of a warp is a piece of a row of cells: the samples of a cell add to
 // S00 .. S11, which at the end of the cell go to its four corners; the right-hand pair is carried to the next cell.  Even rows
 // of cells write their two rows of dx first, then the odd rows add theirs, so no element has two writers.  What a piece
-// carries past its end waits in `seam`.  A sample costs three shared loads of its record, one line of dy, four bank reads
-// and eight multiply-adds per 32 channels.
-template <typename T>
+// carries past its end waits in `seam`.  A sample costs four shared loads of its record, one line of dy, four bank reads
+// and nine multiplications or multiply-adds per channel.
+template <typename T, int V>
 __global__ void __launch_bounds__(32 * kGatherWarps) dcn_gather_kernel(const T* __restrict__ dyt, const int* __restrict__ starts,
                                                                        const Rec* __restrict__ recs, const T* __restrict__ w,
                                                                        T* __restrict__ dx, const Geom g, const BinPlan t) {
+  constexpr int CB = 32 * V, PITCH = V == 1 ? 33 : 66;
   extern __shared__ __align__(16) float4 smem4[];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int n = blockIdx.x / t.bands, r0 = (blockIdx.x - n * t.bands) * t.R, rows = min(t.R, g.H - r0);
-  const int c0 = blockIdx.y * 32, n_c = min(32, g.C - c0), bw = g.scW + 2, W1 = g.W + 1;
+  const int c0 = blockIdx.y * CB, n_c = min(CB, g.C - c0), bw = g.scW + 2, W1 = g.W + 1;
   float4* stage = smem4 + warp * 96;                                   // [32 records]
   float* bank = reinterpret_cast<float*>(smem4 + kGatherWarps * 96);   // [cell of the zero-bordered bank][channel]
-  float* seam = bank + (g.scH + 2) * bw * 32;                          // [row of cells][piece][upper | lower][channel]
-  float* acc = seam + (t.R + 1) * t.segs * 64;                         // [row][column][33]
-  for (int i = threadIdx.x; i < (g.scH + 2) * bw * 32; i += 32 * kGatherWarps) {
-    const int cell = i >> 5, a = cell / bw - 1, b = cell - (a + 1) * bw - 1, c = i & 31;
+  float* seam = bank + (g.scH + 2) * bw * CB;                          // [row of cells][piece][upper | lower][channel]
+  float* acc = seam + (t.R + 1) * t.segs * 2 * CB;                     // [row][column][PITCH]
+  for (int i = threadIdx.x; i < (g.scH + 2) * bw * CB; i += 32 * kGatherWarps) {
+    const int cell = i / CB, a = cell / bw - 1, b = cell - (a + 1) * bw - 1, c = i % CB;
     bank[i] = (c < n_c && a >= 0 && a < g.scH && b >= 0 && b < g.scW) ? ld<float>(w + (size_t)(c0 + c) * g.cells + a * g.scW + b) : 0.f;
   }
   __syncthreads();
-  const T* yl = dyt + (size_t)n * g.P * t.Cp + c0 + lane;
+  const T* yl = dyt + (size_t)n * (g.P + 1) * t.Cp + c0 + V * lane;
   const int* st_n = starts + (size_t)n * (t.bins + 1);
   const float4* rc_n = reinterpret_cast<const float4*>(recs + (size_t)n * t.rec_per_n);
-  const float* bl = bank + lane;
+  const float* bl = bank + V * lane;
+  const float4 none = make_float4(0.f, 0.f, 0.f, 0.f);
   for (int phase = 0; phase < 2; ++phase) {
     const int n_rows = (rows + 2 - phase) >> 1;  // rows of cells r0 - 1 .. r0 + rows - 1, every other one
     for (int unit = warp; unit < n_rows * t.segs; unit += kGatherWarps) {
@@ -169,26 +197,40 @@ __global__ void __launch_bounds__(32 * kGatherWarps) dcn_gather_kernel(const T* 
       const int b0 = seg * W1 / t.segs, b1 = (seg + 1) * W1 / t.segs;
       const int* sr = st_n + (r0 + i) * W1;
       const int first = __ldg(sr + b0), last = __ldg(sr + b1);
-      float* up = i >= 1 ? acc + (size_t)(i - 1) * g.W * 33 + lane : nullptr;
-      float* low = i < rows ? acc + (size_t)i * g.W * 33 + lane : nullptr;
+      float* up = i >= 1 ? acc + (i - 1) * g.W * PITCH + V * lane : nullptr;
+      float* low = i < rows ? acc + i * g.W * PITCH + V * lane : nullptr;
       int cur = b0;
-      float s00 = 0.f, s01 = 0.f, s10 = 0.f, s11 = 0.f, cu = 0.f, cl = 0.f;
+      float s00[V] = {}, s01[V] = {}, s10[V] = {}, s11[V] = {}, cu[V] = {}, cl[V] = {};
       auto flush = [&]() {
         if (cur > 0) {
-          const int o = (cur - 1) * 33;
-          if (up) up[o] = phase ? up[o] + (s00 + cu) : s00 + cu;
-          if (low) low[o] = phase ? low[o] + (s10 + cl) : s10 + cl;
+          const int o = (cur - 1) * PITCH;
+#pragma unroll
+          for (int j = 0; j < V; ++j) cu[j] += s00[j], cl[j] += s10[j];
+          if (up) {
+            if (phase)
+              for (int j = 0; j < V; ++j) cu[j] += up[o + j];
+            put<V>(up + o, cu);
+          }
+          if (low) {
+            if (phase)
+              for (int j = 0; j < V; ++j) cl[j] += low[o + j];
+            put<V>(low + o, cl);
+          }
         }
-        cu = s01, cl = s11;
-        s00 = s01 = s10 = s11 = 0.f;
+#pragma unroll
+        for (int j = 0; j < V; ++j) cu[j] = s01[j], cl[j] = s11[j], s00[j] = s01[j] = s10[j] = s11[j] = 0.f;
         ++cur;
       };
+      // records beyond the last one: no weight, the zero pixel, no new cell
       float4 next[3];
       auto fetch = [&](int at) {
         const int lim = (last - at) * 3;
 #pragma unroll
-        for (int j = 0; j < 3; ++j)
-          if (lane + 32 * j < lim) next[j] = __ldg(rc_n + (size_t)at * 3 + lane + 32 * j);
+        for (int j = 0; j < 3; ++j) {
+          const int e = lane + 32 * j;
+          next[j] = e < lim ? __ldg(rc_n + (size_t)at * 3 + e) : none;
+          if (e >= lim && e % 3 == 2) next[j].z = __int_as_float(g.P * t.Cp);
+        }
       };
       if (first < last) fetch(first);
       for (int at = first; at < last; at += 32) {
@@ -199,42 +241,44 @@ __global__ void __launch_bounds__(32 * kGatherWarps) dcn_gather_kernel(const T* 
         if (at + 32 < last) fetch(at + 32);
         const int cnt = min(32, last - at);
         for (int k0 = 0; k0 < cnt; k0 += 8) {
-          float yv[8];
+          float yv[8][V];
 #pragma unroll
-          for (int j = 0; j < 8; ++j)
-            if (k0 + j < cnt) yv[j] = ld<float>(yl + reinterpret_cast<const int*>(stage + (k0 + j) * 3 + 2)[2]);
+          for (int j = 0; j < 8; ++j) get<T, V>(yl + reinterpret_cast<const int*>(stage + (k0 + j) * 3 + 2)[2], yv[j]);
 #pragma unroll
           for (int j = 0; j < 8; ++j) {
-            if (k0 + j < cnt) {
-              const float4 ci = stage[(k0 + j) * 3], cb = stage[(k0 + j) * 3 + 1];
-              const int2 a2 = *reinterpret_cast<const int2*>(stage + (k0 + j) * 3 + 2);
-              while (cur < a2.y) flush();
-              const float* bk = bl + a2.x;
-              const float kv = cb.x * bk[0] + cb.y * bk[32] + cb.z * bk[bw * 32] + cb.w * bk[bw * 32 + 32];
-              const float v = kv * yv[j];
-              s00 += ci.x * v, s01 += ci.y * v, s10 += ci.z * v, s11 += ci.w * v;
+            const float4 ci = stage[(k0 + j) * 3], cb = stage[(k0 + j) * 3 + 1];
+            const int2 at2 = *reinterpret_cast<const int2*>(stage + (k0 + j) * 3 + 2);
+            while (cur < at2.y) flush();
+            const float* bk = bl + at2.x * V;
+            float b0v[V], b1v[V], b2v[V], b3v[V];
+            get<float, V>(bk, b0v), get<float, V>(bk + CB, b1v), get<float, V>(bk + bw * CB, b2v), get<float, V>(bk + bw * CB + CB, b3v);
+#pragma unroll
+            for (int e = 0; e < V; ++e) {
+              const float kv = cb.x * b0v[e] + cb.y * b1v[e] + cb.z * b2v[e] + cb.w * b3v[e];
+              const float v = kv * yv[j][e];
+              s00[e] += ci.x * v, s01[e] += ci.y * v, s10[e] += ci.z * v, s11[e] += ci.w * v;
             }
           }
         }
       }
       while (cur < b1) flush();
-      seam[((i * t.segs + seg) * 2) * 32 + lane] = cu;
-      seam[((i * t.segs + seg) * 2 + 1) * 32 + lane] = cl;
+      put<V>(seam + ((i * t.segs + seg) * 2) * CB + V * lane, cu);
+      put<V>(seam + ((i * t.segs + seg) * 2 + 1) * CB + V * lane, cl);
     }
     __syncthreads();
   }
   if (t.segs > 1) {
     for (int u = warp; u < rows * (t.segs - 1); u += kGatherWarps) {
       const int d = u / (t.segs - 1), seg = u - d * (t.segs - 1), b = (seg + 1) * W1 / t.segs;
-      acc[((size_t)d * g.W + b - 1) * 33 + lane] +=
-          seam[(((d + 1) * t.segs + seg) * 2) * 32 + lane] + seam[((d * t.segs + seg) * 2 + 1) * 32 + lane];
+      for (int j = lane; j < CB; j += 32)
+        acc[(d * g.W + b - 1) * PITCH + j] += seam[(((d + 1) * t.segs + seg) * 2) * CB + j] + seam[((d * t.segs + seg) * 2 + 1) * CB + j];
     }
     __syncthreads();
   }
   const int span = rows * g.W;
   for (int c = warp; c < n_c; c += kGatherWarps) {
     T* o = dx + ((size_t)n * g.C + c0 + c) * g.HW + (size_t)r0 * g.W;
-    for (int e = lane; e < span; e += 32) st<T, float>(o + e, acc[e * 33 + c]);
+    for (int e = lane; e < span; e += 32) st<T, float>(o + e, acc[e * PITCH + c]);
   }
 }
 
@@ -242,14 +286,17 @@ size_t round256(size_t v) { return (v + 255) & ~(size_t)255; }
 
 bool bin_plan(const Geom& g, size_t elem, BinPlan& t) {
   const long long bins = (long long)(g.H + 1) * (g.W + 1), recs = (long long)g.taps * g.P;
-  t.groups = (g.C + 31) / 32;
-  t.Cp = 32 * t.groups;
-  if (g.G != 1 || bins * 4 > 160 * 1024 || recs > 0x3fffffff || (long long)g.P * t.Cp > 0x7fffffff || t.groups > 65535) return false;
+  // two channels on a lane share the record and the walk through the cells
+  t.V = g.C > 32 ? 2 : 1;
+  t.groups = (g.C + 32 * t.V - 1) / (32 * t.V);
+  t.Cp = 32 * t.V * t.groups;
+  if (g.G != 1 || bins * 4 > 160 * 1024 || recs > 0x3fffffff || ((long long)g.P + 1) * t.Cp > 0x7fffffff || t.groups > 65535) return false;
+  if ((long long)g.N * (t.Cp / 32) * (g.P / kMovePixels + 1) > 0x3fffffff) return false;
   t.bins = (int)bins, t.rec_per_n = (int)recs;
-  // rows of a block: up to 56 KB of sums, three blocks (24 warps) on an SM; more and smaller blocks where they would not
-  // fill the chip (a row of cells between two blocks is walked through twice)
-  const int row = g.W * 33 * 4, sms = device_sm_count();
-  int R = 56 * 1024 / row;
+  // rows of a block: up to 72 KB of sums, two blocks on an SM; more and smaller blocks where they would not fill the chip (a
+  // row of cells between two blocks is walked through twice)
+  const int row = g.W * (t.V == 1 ? 33 : 66) * 4, sms = device_sm_count();
+  int R = 72 * 1024 / row;
   if (R < 1) return false;
   const long long planes = (long long)g.N * t.groups;
   int bands = (g.H + R - 1) / R;
@@ -261,11 +308,11 @@ bool bin_plan(const Geom& g, size_t elem, BinPlan& t) {
   t.segs = (2 * kGatherWarps + t.R) / (t.R + 1);
   if (t.segs > (g.W + 1) / 4) t.segs = (g.W + 1) / 4 > 0 ? (g.W + 1) / 4 : 1;
   t.sort_smem = (size_t)t.bins * 4;
-  t.gather_smem = (size_t)kGatherWarps * 1536 + ((size_t)(g.scH + 2) * (g.scW + 2) * 32 + (size_t)(t.R + 1) * t.segs * 64 + (size_t)t.R * g.W * 33) * 4;
+  t.gather_smem = (size_t)kGatherWarps * 1536 + ((size_t)(g.scH + 2) * (g.scW + 2) * 32 * t.V + (size_t)(t.R + 1) * t.segs * 64 * t.V) * 4 + (size_t)t.R * row;
   if (t.gather_smem > 110 * 1024 || (long long)g.N * t.bands > 0x7fffffff || (long long)g.N * kSortBlocks > 0x3fffffff) return false;
   t.starts_bytes = round256((size_t)g.N * (t.bins + 1) * sizeof(int));
   t.recs_bytes = round256((size_t)g.N * t.rec_per_n * sizeof(Rec));
-  t.bytes = t.starts_bytes + t.recs_bytes + round256((size_t)g.N * g.P * t.Cp * elem);
+  t.bytes = t.starts_bytes + t.recs_bytes + round256((size_t)g.N * (g.P + 1) * t.Cp * elem);
   return true;
 }
 
@@ -285,10 +332,11 @@ int deform_data_bins(const T* dy, const T* off, const T* rot, const T* w, T* dx,
   T* dyt = reinterpret_cast<T*>(reinterpret_cast<char*>(ws) + t.starts_bytes + t.recs_bytes);
   int rc = enable_smem(dcn_bins_kernel<T>, t.sort_smem);
   if (rc) return rc;
-  rc = enable_smem(dcn_gather_kernel<T>, t.gather_smem);
+  auto gather = t.V == 1 ? dcn_gather_kernel<T, 1> : dcn_gather_kernel<T, 2>;
+  rc = enable_smem(gather, t.gather_smem);
   if (rc) return rc;
-  const long long tiles = (long long)g.N * t.groups * ((g.P + 31) / 32);
-  long long movers = (tiles + 4 * kSortBlocks - 1) / (4 * kSortBlocks);
+  const long long tiles = (long long)g.N * (t.Cp / 32) * (g.P / kMovePixels + 1);
+  long long movers = (tiles + kSortBlocks - 1) / kSortBlocks;
   if (movers > 2 * device_sm_count() / kSortBlocks) movers = 2 * device_sm_count() / kSortBlocks;
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3((unsigned)((g.N + movers) * kSortBlocks));
@@ -305,7 +353,7 @@ int deform_data_bins(const T* dy, const T* off, const T* rot, const T* w, T* dx,
     set_last_cuda_error(e);
     return DK_ERR_CUDA;
   }
-  dcn_gather_kernel<T><<<dim3((unsigned)(g.N * t.bands), t.groups), 32 * kGatherWarps, t.gather_smem, s>>>(dyt, starts, recs, w, dx, g, t);
+  gather<<<dim3((unsigned)(g.N * t.bands), t.groups), 32 * kGatherWarps, t.gather_smem, s>>>(dyt, starts, recs, w, dx, g, t);
   return check_launch();
 }
 template int deform_data_bins<float>(const float*, const float*, const float*, const float*, float*, const Geom&, void*, size_t, cudaStream_t);
