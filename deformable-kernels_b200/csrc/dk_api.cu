@@ -306,8 +306,10 @@ size_t dk_deform_sample_depthwise_backward_data_workspace_bytes(const dk_geom* g
   if (!make_geom(g, &gg) || !dtype_ok(dtype)) return 0;
   if (dtype == DK_F64) return 0;
   size_t need = dtype == DK_F16 ? align256((size_t)gg.N * gg.C * gg.HW * sizeof(float)) : 0;
-  const size_t bins = align256(deform_bins_workspace(gg, dtype == DK_F16 ? 2 : 4));
-  if (bins > need) need = bins;
+  if (dtype != DK_F16 || deform_data_mma_workspace(gg) == 0) {
+    const size_t bins = align256(deform_bins_workspace(gg, dtype == DK_F16 ? 2 : 4));
+    if (bins > need) need = bins;
+  }
   return need;
 }
 

@@ -6,7 +6,9 @@
 // as slow as additions in L2.  But where a sample lands does not depend on the channel.  So the samples (pixel, tap) are first
 // sorted by the cell of the input grid they fall into, once for all channels (dcn_bins_kernel), and then a warp walks through
 // the cells of a row with 32 channels on its lanes and the four corner sums in registers: no atomics, no collisions, one
-// multiply-add per corner (dcn_gather_kernel).
+// multiply-add per corner (dcn_gather_kernel).  16 x 192 of 28 x 28: 245 -> 71 us (19 of them the sort); 13 x 96 of 80 x 80:
+// 985 -> 281, in fp16 912 -> 281; 64 x 384 of 14 x 14: 640 -> 111; 32 x 72 of 56 x 56, stride 2: 124 -> 101.  The gather is
+// bound by issue (1.6 instructions per cycle and SM over about 20 warps), the sort by the latency of its five steps.
 #include <cooperative_groups.h>
 
 #include "dk_common.cuh"
@@ -21,6 +23,7 @@ constexpr int kGatherWarps = 8, kMovePixels = 128;
 
 struct BinPlan {
   int bins, rec_per_n, Cp, groups;  // (H + 1) x (W + 1) cells; taps * P samples; channels rounded up to those of a block
+  int movers;                       // first block that transposes dy
   int V, R, bands, segs;               // destination rows of a block, blocks per plane, pieces of a row of cells
   size_t starts_bytes, recs_bytes, bytes, sort_smem, gather_smem;
 };
@@ -59,10 +62,10 @@ __device__ __forceinline__ int sample_cell(int i, int n, const T* __restrict__ o
 
 // Counting sort of the samples of one (n) by cell: every block of the cluster counts its share in shared memory, the blocks
 // share the prefix sums (an eighth of the cells each, through distributed shared memory), then every block places its samples.
-// The clusters after the first N turn dy [C][P] into [P + 1][Cp] (the last pixel is zero), so that the channels of a pixel are
+// The clusters beyond the first N (or, where they are few, all blocks before they sort) turn dy [C][P] into [P + 1][Cp] (the last pixel is zero), so that the channels of a pixel are
 // neighbours for the gather.
 template <typename T>
-__global__ void __launch_bounds__(kSortThreads) dcn_bins_kernel(const T* __restrict__ dy, const T* __restrict__ off,
+__global__ void __launch_bounds__(kSortThreads, 2) dcn_bins_kernel(const T* __restrict__ dy, const T* __restrict__ off,
                                                                 const T* __restrict__ rot, int* __restrict__ starts,
                                                                 Rec* __restrict__ recs, T* __restrict__ dyt, const Geom g,
                                                                 const BinPlan t) {
@@ -71,16 +74,16 @@ __global__ void __launch_bounds__(kSortThreads) dcn_bins_kernel(const T* __restr
   __shared__ float tile[kMovePixels * 33];
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int n = blockIdx.x / kSortBlocks, rank = blockIdx.x - n * kSortBlocks;
-  if (n >= g.N) {
-    const int tiles_p = (g.P + 1 + kMovePixels - 1) / kMovePixels, per_n = t.Cp / 32 * tiles_p, step = gridDim.x - g.N * kSortBlocks;
-    for (int k = blockIdx.x - g.N * kSortBlocks; k < g.N * per_n; k += step) {
+  {
+    const int tiles_p = (g.P + 1 + kMovePixels - 1) / kMovePixels, per_n = t.Cp / 32 * tiles_p, from = t.movers, step = gridDim.x - from;
+    for (int k = blockIdx.x - from; k >= 0 && k < g.N * per_n; k += step) {
       const int m = k / per_n, r = k - m * per_n, grp = r / tiles_p, p0 = (r - grp * tiles_p) * kMovePixels;
-      const T* from = dy + ((size_t)m * g.C + min(grp * 32 + warp, g.C - 1)) * g.P;
+      const T* src = dy + ((size_t)m * g.C + min(grp * 32 + warp, g.C - 1)) * g.P;
       const bool has = grp * 32 + warp < g.C;
       float v[kMovePixels / 32];
 #pragma unroll
       for (int e = 0; e < kMovePixels / 32; ++e)
-        v[e] = has && p0 + e * 32 + lane < g.P ? ld<float>(from + p0 + e * 32 + lane) : 0.f;
+        v[e] = has && p0 + e * 32 + lane < g.P ? ld<float>(src + p0 + e * 32 + lane) : 0.f;
       __syncthreads();
 #pragma unroll
       for (int e = 0; e < kMovePixels / 32; ++e) tile[(e * 32 + lane) * 33 + warp] = v[e];
@@ -90,8 +93,8 @@ __global__ void __launch_bounds__(kSortThreads) dcn_bins_kernel(const T* __restr
       for (int e = 0; e < kMovePixels / 32; ++e)
         if (p0 + warp + e * 32 <= g.P) st<T, float>(to + (size_t)e * 32 * t.Cp, tile[(warp + e * 32) * 33 + lane]);
     }
-    return;
   }
+  if (n >= g.N) return;
   cg::cluster_group cluster = cg::this_cluster();
   for (int i = tid; i < t.bins; i += kSortThreads) hist[i] = 0;
   __syncthreads();
@@ -104,6 +107,7 @@ __global__ void __launch_bounds__(kSortThreads) dcn_bins_kernel(const T* __restr
   const int hi = min((rank + 1) * per, t.bins), lo = rank * per + tid * q, end = min(lo + q, hi);
   int sum = 0;
   for (int b = lo; b < end; ++b)
+#pragma unroll
     for (int k = 0; k < kSortBlocks; ++k) sum += cluster.map_shared_rank(hist, k)[b];
   int scan = sum;
 #pragma unroll
@@ -126,11 +130,13 @@ __global__ void __launch_bounds__(kSortThreads) dcn_bins_kernel(const T* __restr
   int* out = starts + (size_t)n * (t.bins + 1);
   for (int b = lo; b < end; ++b) {
     out[b] = run;
+    int c[kSortBlocks];
+#pragma unroll
+    for (int k = 0; k < kSortBlocks; ++k) c[k] = cluster.map_shared_rank(hist, k)[b];
+#pragma unroll
     for (int k = 0; k < kSortBlocks; ++k) {
-      int* h = cluster.map_shared_rank(hist, k) + b;
-      const int c = *h;
-      *h = run;
-      run += c;
+      cluster.map_shared_rank(hist, k)[b] = run;
+      run += c[k];
     }
   }
   if (rank == kSortBlocks - 1 && tid == 0) out[t.bins] = before + total;
@@ -168,7 +174,7 @@ __device__ __forceinline__ void put(float* p, const float (&v)[V]) {
 // carries past its end waits in `seam`.  A sample costs four shared loads of its record, one line of dy, four bank reads
 // and nine multiplications or multiply-adds per channel.
 template <typename T, int V>
-__global__ void __launch_bounds__(32 * kGatherWarps) dcn_gather_kernel(const T* __restrict__ dyt, const int* __restrict__ starts,
+__global__ void __launch_bounds__(32 * kGatherWarps, 3) dcn_gather_kernel(const T* __restrict__ dyt, const int* __restrict__ starts,
                                                                        const Rec* __restrict__ recs, const T* __restrict__ w,
                                                                        T* __restrict__ dx, const Geom g, const BinPlan t) {
   constexpr int CB = 32 * V, PITCH = V == 1 ? 33 : 66;
@@ -286,27 +292,30 @@ size_t round256(size_t v) { return (v + 255) & ~(size_t)255; }
 
 bool bin_plan(const Geom& g, size_t elem, BinPlan& t) {
   const long long bins = (long long)(g.H + 1) * (g.W + 1), recs = (long long)g.taps * g.P;
-  // two channels on a lane share the record and the walk through the cells
-  t.V = g.C > 32 ? 2 : 1;
-  t.groups = (g.C + 32 * t.V - 1) / (32 * t.V);
+  // Two channels on a lane share the record and the walk through the cells (1.3 times the time of one).  A block walks R + 1
+  // rows of cells, half of them at a time, in pieces so that every warp gets one; what it does besides costs about three
+  // rows.  Up to 72 KB of sums, two blocks on an SM.  16 x 192 of 28 x 28: (V, R) = (1, 3) 94, (1, 7) 76, (2, 3) 75, (2, 7)
+  // 75 us; 64 x 384 of 14 x 14: 219, 146, 144, 112; 4 x 64 of 50 x 84: 83, 126, 93, -, and (2, 1) 71.
+  const int sms = device_sm_count();
+  long long best = -1;
+  for (int V = 1; V <= (g.C > 32 ? 2 : 1); ++V) {
+    for (int R = 1; R < kGatherWarps; R = 2 * R + 1) {
+      const int groups = (g.C + 32 * V - 1) / (32 * V), held = R < g.H ? R : g.H;
+      if ((long long)held * g.W * (V == 1 ? 33 : 66) * 4 > 72 * 1024) continue;
+      const long long blocks = (long long)g.N * groups * ((g.H + R - 1) / R), cost = (blocks + sms - 1) / sms * (R + 4) * (V == 1 ? 10 : 13);
+      if (best >= 0 && cost >= best) continue;
+      best = cost;
+      t.V = V, t.groups = groups, t.R = held, t.bands = (g.H + R - 1) / R;
+      t.segs = 2 * kGatherWarps / (R + 1);
+    }
+  }
+  if (best < 0) return false;
+  if (t.segs > (g.W + 1) / 4) t.segs = (g.W + 1) / 4 > 0 ? (g.W + 1) / 4 : 1;
+  const int row = g.W * (t.V == 1 ? 33 : 66) * 4;
   t.Cp = 32 * t.V * t.groups;
   if (g.G != 1 || bins * 4 > 160 * 1024 || recs > 0x3fffffff || ((long long)g.P + 1) * t.Cp > 0x7fffffff || t.groups > 65535) return false;
   if ((long long)g.N * (t.Cp / 32) * (g.P / kMovePixels + 1) > 0x3fffffff) return false;
   t.bins = (int)bins, t.rec_per_n = (int)recs;
-  // rows of a block: up to 72 KB of sums, two blocks on an SM; more and smaller blocks where they would not fill the chip (a
-  // row of cells between two blocks is walked through twice)
-  const int row = g.W * (t.V == 1 ? 33 : 66) * 4, sms = device_sm_count();
-  int R = 72 * 1024 / row;
-  if (R < 1) return false;
-  const long long planes = (long long)g.N * t.groups;
-  int bands = (g.H + R - 1) / R;
-  const long long fill = (2 * (long long)sms + planes - 1) / planes;
-  if (fill > bands) bands = (int)(fill < (g.H + 1) / 2 ? fill : (g.H + 1) / 2);
-  t.R = (g.H + bands - 1) / bands;
-  t.bands = (g.H + t.R - 1) / t.R;
-  // pieces of a row so that both halves of the rows give every warp one
-  t.segs = (2 * kGatherWarps + t.R) / (t.R + 1);
-  if (t.segs > (g.W + 1) / 4) t.segs = (g.W + 1) / 4 > 0 ? (g.W + 1) / 4 : 1;
   t.sort_smem = (size_t)t.bins * 4;
   t.gather_smem = (size_t)kGatherWarps * 1536 + ((size_t)(g.scH + 2) * (g.scW + 2) * 32 * t.V + (size_t)(t.R + 1) * t.segs * 64 * t.V) * 4 + (size_t)t.R * row;
   if (t.gather_smem > 110 * 1024 || (long long)g.N * t.bands > 0x7fffffff || (long long)g.N * kSortBlocks > 0x3fffffff) return false;
@@ -336,10 +345,12 @@ int deform_data_bins(const T* dy, const T* off, const T* rot, const T* w, T* dx,
   rc = enable_smem(gather, t.gather_smem);
   if (rc) return rc;
   const long long tiles = (long long)g.N * (t.Cp / 32) * (g.P / kMovePixels + 1);
-  long long movers = (tiles + kSortBlocks - 1) / kSortBlocks;
-  if (movers > 2 * device_sm_count() / kSortBlocks) movers = 2 * device_sm_count() / kSortBlocks;
+  long long clusters = (tiles + kSortBlocks - 1) / kSortBlocks;
+  if (clusters > 2 * device_sm_count() / kSortBlocks) clusters = 2 * device_sm_count() / kSortBlocks;
+  if (clusters < g.N) clusters = g.N;
+  t.movers = 3 * clusters >= 4 * (long long)g.N ? g.N * kSortBlocks : 0;
   cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3((unsigned)((g.N + movers) * kSortBlocks));
+  cfg.gridDim = dim3((unsigned)(clusters * kSortBlocks));
   cfg.blockDim = dim3(kSortThreads);
   cfg.dynamicSmemBytes = t.sort_smem;
   cfg.stream = s;
