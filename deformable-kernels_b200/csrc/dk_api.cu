@@ -370,6 +370,13 @@ int dk_deform_sample_depthwise_backward_rotation(const void* grad_output, const 
                                                P_(T, filter), (T*)nullptr, M_(T, grad_rotation), gg, (cudaStream_t)stream))
 }
 
+/* Whether the fused backward takes the kernels with channels on the lanes: where no tensor-core kernel applies. */
+static bool deform_by_rows(const Geom& g, int dtype) {
+  if (dtype == DK_F16)
+    return deform_data_mma_workspace(g) == 0 && deform_coords_mma_workspace(g) == 0 && deform_filter_mma_workspace(g) == 0;
+  return dtype == DK_F32;
+}
+
 /* First region of the fused backward's workspace: used by grad-input, then (same stream) by the offset gradients. */
 static size_t deform_front_ws(const dk_geom* g, int dtype) {
   size_t need = dk_deform_sample_depthwise_backward_data_workspace_bytes(g, dtype);
@@ -377,6 +384,10 @@ static size_t deform_front_ws(const dk_geom* g, int dtype) {
   if (dtype == DK_F16 && make_geom(g, &gg)) {
     const size_t c = align256(deform_coords_mma_workspace(gg));
     if (c > need) need = c;
+  }
+  if (make_geom(g, &gg) && deform_by_rows(gg, dtype)) {
+    const size_t rows = align256(deform_rows_workspace(gg, dtype == DK_F16 ? 2 : 4));
+    if (rows > need) need = rows;
   }
   return need;
 }
@@ -423,6 +434,27 @@ int dk_deform_sample_depthwise_backward(const void* grad_output, const void* inp
       rc = deform_filter_mma(P_(__half, grad_output), P_(__half, input), P_(__half, offset), nullptr, M_(__half, grad_filter),
                              gg, (char*)workspace + data_ws, filt_ws, s);
     return rc;
+  }
+  if (deform_by_rows(gg, dtype)) {
+    bool bank_done = false;
+    if (dtype == DK_F16)
+      rc = deform_backward_rows<__half>(P_(__half, grad_output), P_(__half, input), P_(__half, offset), P_(__half, rotation),
+                                        P_(__half, filter), M_(__half, grad_input), M_(__half, grad_offset), M_(__half, grad_rotation),
+                                        M_(__half, grad_filter), gg, workspace, workspace_bytes < data_ws ? 0 : data_ws,
+                                        (cudaStream_t)stream, &bank_done);
+    else
+      rc = deform_backward_rows<float>(P_(float, grad_output), P_(float, input), P_(float, offset), P_(float, rotation),
+                                       P_(float, filter), M_(float, grad_input), M_(float, grad_offset), M_(float, grad_rotation),
+                                       M_(float, grad_filter), gg, workspace, workspace_bytes < data_ws ? 0 : data_ws,
+                                       (cudaStream_t)stream, &bank_done);
+    if (rc == DK_OK && (bank_done || !grad_filter)) return rc;
+    if (rc == DK_OK) {
+      if (workspace_bytes < data_ws + filt_ws) return DK_ERR_WORKSPACE;
+      return dk_deform_sample_depthwise_backward_filter(grad_output, input, offset, rotation, grad_filter, g, dtype,
+                                                        (char*)workspace + data_ws, filt_ws, stream);
+    }
+    if (rc != DK_ERR_UNSUPPORTED) return rc;
+    rc = DK_OK;
   }
   if (grad_input) {
     const bool room = workspace && workspace_bytes >= data_ws;

@@ -103,6 +103,21 @@ __device__ __forceinline__ void bilinear_dv_coefs(const Bilinear<A>& b, A (&c)[4
   c[3] = b.m[3] ? b.lh : (A)0;
 }
 
+// two fp32 multiply-adds in one instruction: the pipe needs as long as for two, but the loads beside them get issue slots
+__device__ __forceinline__ unsigned long long pair(float a, float b) {
+  unsigned long long r;
+  asm("mov.b64 %0, {%1, %2};\n" : "=l"(r) : "f"(a), "f"(b));
+  return r;
+}
+__device__ __forceinline__ float2 unpair(unsigned long long v) {
+  float2 r;
+  asm("mov.b64 {%0, %1}, %2;\n" : "=f"(r.x), "=f"(r.y) : "l"(v));
+  return r;
+}
+__device__ __forceinline__ void fma2(unsigned long long& acc, unsigned long long a, unsigned long long b) {
+  asm("fma.rn.f32x2 %0, %1, %2, %0;\n" : "+l"(acc) : "l"(a), "l"(b));
+}
+
 // Bank coordinate of one tap: u = f + r + (scope - kernel)/2.  (The reference adds
 // the last term in double and narrows, csrc/filter_sample_depthwise_cuda_kernel.cu:338-341;
 // for the multiples of 0.5 that occur this equals the single correctly rounded add done here.)
@@ -212,6 +227,12 @@ size_t deform_data_mma_workspace(const Geom& g);
 size_t deform_bins_workspace(const Geom& g, size_t elem);
 template <typename T>
 int deform_data_bins(const T* dy, const T* off, const T* rot, const T* w, T* dx, const Geom& g, void* ws, size_t ws_bytes, cudaStream_t s);
+size_t deform_rows_workspace(const Geom& g, size_t elem);
+template <typename T>
+int deform_backward_rows(const T* dy, const T* x, const T* off, const T* rot, const T* w, T* dx, T* doff, T* drot, T* dw, const Geom& g,
+                         void* ws, size_t ws_bytes, cudaStream_t s, bool* bank_done);
+template <typename T>
+int reduce_bank(const float* partial, T* dw, int n_out, int blocks, cudaStream_t s);
 size_t deform_bank_workspace(const Geom& g);
 template <typename T>
 int deform_bank(const T* dy, const T* x, const T* off, const T* rot, float* partial, const Geom& g, size_t ws_bytes, int* blocks,

@@ -23,9 +23,10 @@ constexpr int kGatherWarps = 8, kMovePixels = 128;
 
 struct BinPlan {
   int bins, rec_per_n, Cp, groups;  // (H + 1) x (W + 1) cells; taps * P samples; channels rounded up to those of a block
-  int movers;                       // first block that transposes dy
+  int movers, sorted;               // first block that transposes; samples to sort (N or none)
   int V, R, bands, segs;               // destination rows of a block, blocks per plane, pieces of a row of cells
-  size_t starts_bytes, recs_bytes, bytes, sort_smem, gather_smem;
+  int bank_blocks;                  // partial bank gradients
+  size_t starts_bytes, recs_bytes, dyt_bytes, bytes, xt_bytes, bankt_bytes, all_bytes, sort_smem, gather_smem;
 };
 
 // one sample point: corner coefficients of the image and of the bank, {bank cell * 32, column of the cell, pixel * Cp, 0}
@@ -34,67 +35,96 @@ struct Rec {
   int4 at;
 };
 
-// cell of sample i = tap * P + p, or -1 where it adds nothing
+// where sample (n, tap, p) falls in the image and in the bank: upper left corner (-1 .. last) and the fractions
+struct Point {
+  int h0, w0, u0, v0;
+  float lh, lw, lu, lv;
+};
+
 template <typename T>
-__device__ __forceinline__ int sample_cell(int i, int n, const T* __restrict__ off, const T* __restrict__ rot, const Geom& g, Rec* rec,
-                                           int Cp) {
-  const int tap = i / g.P, p = i - tap * g.P, fh = tap / g.kW, fw = tap - fh * g.kW;
-  const int oh = p / g.Wo, ow = p - oh * g.Wo;
+__device__ __forceinline__ bool sample_point(int n, int tap, int p, const T* __restrict__ off, const T* __restrict__ rot, const Geom& g,
+                                             Point& q) {
+  const int fh = tap / g.kW, fw = tap - fh * g.kW, oh = p / g.Wo, ow = p - oh * g.Wo;
   const size_t o = ((size_t)n * g.taps + tap) * 2 * g.P + p;
   const float ph = (float)(oh * g.sH - g.pH + fh * g.dH) + ld<float>(off + o);
   const float pw = (float)(ow * g.sW - g.pW + fw * g.dW) + ld<float>(off + o + g.P);
   const float u = ((float)fh + ld<float>(rot + o)) + (float)(g.scH - g.kH) * 0.5f;
   const float v = ((float)fw + ld<float>(rot + o + g.P)) + (float)(g.scW - g.kW) * 0.5f;
   // written so that NaN fails; what passes is in range for the conversions below
-  if (!(ph > -1.f && pw > -1.f && ph < (float)g.H && pw < (float)g.W)) return -1;
-  if (!(u > -1.f && v > -1.f && u < (float)g.scH && v < (float)g.scW)) return -1;
-  const float fph = floorf(ph), fpw = floorf(pw);
-  const int h0 = (int)fph, w0 = (int)fpw;
+  if (!(ph > -1.f && pw > -1.f && ph < (float)g.H && pw < (float)g.W)) return false;
+  if (!(u > -1.f && v > -1.f && u < (float)g.scH && v < (float)g.scW)) return false;
+  const float fph = floorf(ph), fpw = floorf(pw), fu = floorf(u), fv = floorf(v);
+  q.h0 = (int)fph, q.w0 = (int)fpw, q.u0 = (int)fu, q.v0 = (int)fv;
+  q.lh = ph - fph, q.lw = pw - fpw, q.lu = u - fu, q.lv = v - fv;
+  return true;
+}
+
+// cell of sample i = tap * P + p, or -1 where it adds nothing
+template <typename T>
+__device__ __forceinline__ int sample_cell(int i, int n, const T* __restrict__ off, const T* __restrict__ rot, const Geom& g, Rec* rec,
+                                           int Cp) {
+  const int tap = i / g.P, p = i - tap * g.P;
+  Point q;
+  if (!sample_point(n, tap, p, off, rot, g, q)) return -1;
   if (rec != nullptr) {
-    const float lh = ph - fph, lw = pw - fpw, hh = 1.f - lh, hw = 1.f - lw;
-    const float fu = floorf(u), fv = floorf(v), lu = u - fu, lv = v - fv, hu = 1.f - lu, hv = 1.f - lv;
-    rec->ci = make_float4(hh * hw, hh * lw, lh * hw, lh * lw);
-    rec->cb = make_float4(hu * hv, hu * lv, lu * hv, lu * lv);
-    rec->at = make_int4((((int)fu + 1) * (g.scW + 2) + (int)fv + 1) * 32, w0 + 1, p * Cp, 0);
+    const float hh = 1.f - q.lh, hw = 1.f - q.lw, hu = 1.f - q.lu, hv = 1.f - q.lv;
+    rec->ci = make_float4(hh * hw, hh * q.lw, q.lh * hw, q.lh * q.lw);
+    rec->cb = make_float4(hu * hv, hu * q.lv, q.lu * hv, q.lu * q.lv);
+    rec->at = make_int4(((q.u0 + 1) * (g.scW + 2) + q.v0 + 1) * 32, q.w0 + 1, p * Cp, 0);
   }
-  return (h0 + 1) * (g.W + 1) + w0 + 1;
+  return (q.h0 + 1) * (g.W + 1) + q.w0 + 1;
+}
+
+template <typename T>
+__device__ __forceinline__ void move_channels(const T* __restrict__ src, T* __restrict__ dst, int P, const Geom& g, const BinPlan& t,
+                                              float* tile) {
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int tiles_p = (P + 1 + kMovePixels - 1) / kMovePixels, per_n = t.Cp / 32 * tiles_p;
+  for (int k = blockIdx.x - t.movers; k >= 0 && k < g.N * per_n; k += gridDim.x - t.movers) {
+    const int m = k / per_n, r = k - m * per_n, grp = r / tiles_p, p0 = (r - grp * tiles_p) * kMovePixels;
+    const T* from = src + ((size_t)m * g.C + min(grp * 32 + warp, g.C - 1)) * P;
+    const bool has = grp * 32 + warp < g.C;
+    float v[kMovePixels / 32];
+#pragma unroll
+    for (int e = 0; e < kMovePixels / 32; ++e)
+      v[e] = has && p0 + e * 32 + lane < P ? ld<float>(from + p0 + e * 32 + lane) : 0.f;
+    __syncthreads();
+#pragma unroll
+    for (int e = 0; e < kMovePixels / 32; ++e) tile[(e * 32 + lane) * 33 + warp] = v[e];
+    __syncthreads();
+    T* to = dst + ((size_t)m * (P + 1) + p0 + warp) * t.Cp + grp * 32 + lane;
+#pragma unroll
+    for (int e = 0; e < kMovePixels / 32; ++e)
+      if (p0 + warp + e * 32 <= P) st<T, float>(to + (size_t)e * 32 * t.Cp, tile[(warp + e * 32) * 33 + lane]);
+  }
 }
 
 // Counting sort of the samples of one (n) by cell: every block of the cluster counts its share in shared memory, the blocks
 // share the prefix sums (an eighth of the cells each, through distributed shared memory), then every block places its samples.
-// The clusters beyond the first N (or, where they are few, all blocks before they sort) turn dy [C][P] into [P + 1][Cp] (the last pixel is zero), so that the channels of a pixel are
-// neighbours for the gather.
+// The clusters beyond the first (or, where they are few, all blocks before they sort) bring dy, x and the bank into the order
+// in which the channels of a pixel or cell are neighbours: [P + 1][Cp] and [H W + 1][Cp] with a last pixel of zeros, and
+// [scH + 2][scW + 2][Cp] with a border of zeros.  x and the bank only where the other gradients want them.
 template <typename T>
 __global__ void __launch_bounds__(kSortThreads, 2) dcn_bins_kernel(const T* __restrict__ dy, const T* __restrict__ off,
                                                                 const T* __restrict__ rot, int* __restrict__ starts,
-                                                                Rec* __restrict__ recs, T* __restrict__ dyt, const Geom g,
-                                                                const BinPlan t) {
+                                                                Rec* __restrict__ recs, T* __restrict__ dyt,
+                                                                const T* __restrict__ x, T* __restrict__ xt, const T* __restrict__ w,
+                                                                float* __restrict__ bankt, const Geom g, const BinPlan t) {
   extern __shared__ __align__(16) int hist[];
   __shared__ int slices[kSortBlocks], warp_sum[32];
   __shared__ float tile[kMovePixels * 33];
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int n = blockIdx.x / kSortBlocks, rank = blockIdx.x - n * kSortBlocks;
-  {
-    const int tiles_p = (g.P + 1 + kMovePixels - 1) / kMovePixels, per_n = t.Cp / 32 * tiles_p, from = t.movers, step = gridDim.x - from;
-    for (int k = blockIdx.x - from; k >= 0 && k < g.N * per_n; k += step) {
-      const int m = k / per_n, r = k - m * per_n, grp = r / tiles_p, p0 = (r - grp * tiles_p) * kMovePixels;
-      const T* src = dy + ((size_t)m * g.C + min(grp * 32 + warp, g.C - 1)) * g.P;
-      const bool has = grp * 32 + warp < g.C;
-      float v[kMovePixels / 32];
-#pragma unroll
-      for (int e = 0; e < kMovePixels / 32; ++e)
-        v[e] = has && p0 + e * 32 + lane < g.P ? ld<float>(src + p0 + e * 32 + lane) : 0.f;
-      __syncthreads();
-#pragma unroll
-      for (int e = 0; e < kMovePixels / 32; ++e) tile[(e * 32 + lane) * 33 + warp] = v[e];
-      __syncthreads();
-      T* to = dyt + ((size_t)m * (g.P + 1) + p0 + warp) * t.Cp + grp * 32 + lane;
-#pragma unroll
-      for (int e = 0; e < kMovePixels / 32; ++e)
-        if (p0 + warp + e * 32 <= g.P) st<T, float>(to + (size_t)e * 32 * t.Cp, tile[(warp + e * 32) * 33 + lane]);
+  move_channels(dy, dyt, g.P, g, t, tile);
+  if (xt != nullptr) {
+    move_channels(x, xt, g.HW, g, t, tile);
+    const int cells = (g.scH + 2) * (g.scW + 2);
+    for (int i = (blockIdx.x - t.movers) * kSortThreads + tid; i >= 0 && i < cells * t.Cp; i += (gridDim.x - t.movers) * kSortThreads) {
+      const int cell = i / t.Cp, c = i - cell * t.Cp, a = cell / (g.scW + 2) - 1, b = cell - (a + 1) * (g.scW + 2) - 1;
+      bankt[i] = c < g.C && a >= 0 && a < g.scH && b >= 0 && b < g.scW ? ld<float>(w + (size_t)c * g.cells + a * g.scW + b) : 0.f;
     }
   }
-  if (n >= g.N) return;
+  if (n >= t.sorted) return;
   cg::cluster_group cluster = cg::this_cluster();
   for (int i = tid; i < t.bins; i += kSortThreads) hist[i] = 0;
   __syncthreads();
@@ -288,6 +318,201 @@ __global__ void __launch_bounds__(32 * kGatherWarps, 3) dcn_gather_kernel(const 
   }
 }
 
+// ------------------------------------------------------------------ the other gradients, channels on the lanes
+// With x, dy and the bank in channel order a corner of a sample is one line for 32 (64) channels instead of one line per lane, and
+// the corner indices and fractions, worked out by one lane per sample, are shared by all channels.  Corners outside the image
+// read the zero pixel, cells outside the bank its zero border, so nothing is masked.  A unit of a warp is 32 pixels of a tap.
+constexpr int kRowWarps = 8;
+
+// offsets of the four corners; {1 - lh, lh, 1 - lw, lw}; for the coordinates the same of the bank and {dy, bank cell}, for the bank
+// the hat functions of its rows and columns and {dy}
+struct TapRec {
+  int4 idx;
+  float4 im, a, b;
+  int4 at;
+};
+
+template <typename T, bool BANK>
+__device__ __forceinline__ void tap_record(int flat, int total, int tap, const T* __restrict__ off, const T* __restrict__ rot, const Geom& g,
+                                           int Cp, TapRec* to) {
+  const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f);
+  TapRec r;
+  const int nothing = g.HW * Cp;  // the zero pixels of the first sample
+  r.idx = make_int4(nothing, nothing, nothing, nothing), r.im = r.a = r.b = zero, r.at = make_int4(g.P * Cp, 0, 0, 0);
+  if (flat < total) {
+    const int n = flat / g.P, p = flat - n * g.P;
+    Point q;
+    if (sample_point(n, tap, p, off, rot, g, q)) {
+      const int base = n * (g.HW + 1);
+      const bool r0 = q.h0 >= 0, r1 = q.h0 + 1 < g.H, k0 = q.w0 >= 0, k1 = q.w0 + 1 < g.W;
+      const int px = q.h0 * g.W + q.w0;
+      r.idx.x = (base + (r0 && k0 ? px : g.HW)) * Cp, r.idx.y = (base + (r0 && k1 ? px + 1 : g.HW)) * Cp;
+      r.idx.z = (base + (r1 && k0 ? px + g.W : g.HW)) * Cp, r.idx.w = (base + (r1 && k1 ? px + g.W + 1 : g.HW)) * Cp;
+      r.im = make_float4(1.f - q.lh, q.lh, 1.f - q.lw, q.lw);
+      r.at.x = (n * (g.P + 1) + p) * Cp;
+      if (BANK) {
+        float* hu = reinterpret_cast<float*>(&r.a);
+        float* hv = reinterpret_cast<float*>(&r.b);
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+          hu[k] = k >= g.scH ? 0.f : k == q.u0 ? 1.f - q.lu : k == q.u0 + 1 ? q.lu : 0.f;
+          hv[k] = k >= g.scW ? 0.f : k == q.v0 ? 1.f - q.lv : k == q.v0 + 1 ? q.lv : 0.f;
+        }
+      } else {
+        r.a = make_float4(1.f - q.lu, q.lu, 1.f - q.lv, q.lv);
+        r.at.y = ((q.u0 + 1) * (g.scW + 2) + q.v0 + 1) * Cp;
+      }
+    }
+  }
+  *to = r;
+}
+
+// Both offset gradients.  S warps share the channels of a unit; the sum over the lanes leaves a quarter of the four sums on each.
+// 28 multiplications and additions per sample and channel, nine loads of a line.
+template <typename T, int V, bool ROT>
+__global__ void __launch_bounds__(32 * kRowWarps, 3) dcn_coords_kernel(const T* __restrict__ dyt, const T* __restrict__ xt,
+                                                                       const float* __restrict__ bankt, const T* __restrict__ off,
+                                                                       const T* __restrict__ rot, T* __restrict__ doff,
+                                                                       T* __restrict__ drot, const Geom g, const int Cp, const int S) {
+  __shared__ TapRec recs[kRowWarps][32];
+  __shared__ __align__(16) float out[kRowWarps][32][4];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, share = warp % S;
+  const int total = g.N * g.P, tiles = (total + 31) / 32, u = blockIdx.x * (kRowWarps / S) + warp / S;
+  const int tap = u / tiles, flat0 = (u - tap * tiles) * 32, cnt = tap < g.taps ? min(32, total - flat0) : 0;
+  if (cnt > 0) tap_record<T, false>(flat0 + lane, total, tap, off, rot, g, Cp, &recs[warp][lane]);
+  __syncwarp();
+  const int row = (g.scW + 2) * Cp;
+  for (int j = 0; j < cnt; j += 2) {
+    float s[2][4] = {};
+#pragma unroll 1
+    for (int c = (share * 32 + lane) * V; c < Cp; c += S * 32 * V) {
+      float x[2][4][V], k[2][4][V], y[2][V];
+#pragma unroll
+      for (int h = 0; h < 2; ++h) {
+        const TapRec& r = recs[warp][j + h];
+        const int4 idx = r.idx;
+        const int2 at = *reinterpret_cast<const int2*>(&r.at);
+        get<T, V>(xt + idx.x + c, x[h][0]), get<T, V>(xt + idx.y + c, x[h][1]), get<T, V>(xt + idx.z + c, x[h][2]), get<T, V>(xt + idx.w + c, x[h][3]);
+        get<T, V>(dyt + at.x + c, y[h]);
+        const float* bk = bankt + at.y + c;
+        get<float, V>(bk, k[h][0]), get<float, V>(bk + Cp, k[h][1]), get<float, V>(bk + row, k[h][2]), get<float, V>(bk + row + Cp, k[h][3]);
+      }
+#pragma unroll
+      for (int h = 0; h < 2; ++h) {
+        const float4 im = recs[warp][j + h].im, b = recs[warp][j + h].a;
+#pragma unroll
+        for (int e = 0; e < V; ++e) {
+          const float top = im.z * x[h][0][e] + im.w * x[h][1][e], low = im.z * x[h][2][e] + im.w * x[h][3][e];
+          const float ktop = b.z * k[h][0][e] + b.w * k[h][1][e], klow = b.z * k[h][2][e] + b.w * k[h][3][e];
+          const float yk = y[h][e] * (b.x * ktop + b.y * klow);
+          s[h][0] += yk * (low - top);
+          s[h][1] += yk * (im.x * (x[h][1][e] - x[h][0][e]) + im.y * (x[h][3][e] - x[h][2][e]));
+          if (ROT) {
+            const float yx = y[h][e] * (im.x * top + im.y * low);
+            s[h][2] += yx * (klow - ktop);
+            s[h][3] += yx * (b.x * (k[h][1][e] - k[h][0][e]) + b.y * (k[h][3][e] - k[h][2][e]));
+          }
+        }
+      }
+    }
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+      float a, b;
+      if (ROT) {
+        const bool up = lane & 16;
+        a = (up ? s[h][2] : s[h][0]) + __shfl_xor_sync(0xffffffffu, up ? s[h][0] : s[h][2], 16);
+        b = (up ? s[h][3] : s[h][1]) + __shfl_xor_sync(0xffffffffu, up ? s[h][1] : s[h][3], 16);
+      } else {
+        a = s[h][0] + __shfl_xor_sync(0xffffffffu, s[h][0], 16);
+        b = s[h][1] + __shfl_xor_sync(0xffffffffu, s[h][1], 16);
+      }
+      a = (lane & 8 ? b : a) + __shfl_xor_sync(0xffffffffu, lane & 8 ? a : b, 8);
+      a += __shfl_xor_sync(0xffffffffu, a, 4);
+      a += __shfl_xor_sync(0xffffffffu, a, 2);
+      a += __shfl_xor_sync(0xffffffffu, a, 1);
+      if ((lane & 7) == 0) out[warp][j + h][lane >> 3] = a;
+    }
+  }
+  __syncthreads();
+  if (share == 0 && lane < cnt) {
+    float4 sum = *reinterpret_cast<const float4*>(out[warp][lane]);
+    for (int k = 1; k < S; ++k) {
+      const float4 o = *reinterpret_cast<const float4*>(out[warp + k][lane]);
+      sum.x += o.x, sum.y += o.y, sum.z += o.z, sum.w += o.w;
+    }
+    const int n = (flat0 + lane) / g.P, p = flat0 + lane - n * g.P;
+    const size_t o = ((size_t)n * g.taps + tap) * 2 * g.P + p;
+    if (doff) st<T, float>(doff + o, sum.x), st<T, float>(doff + o + g.P, sum.y);
+    if (ROT) st<T, float>(drot + o, sum.z), st<T, float>(drot + o + g.P, sum.w);
+  }
+}
+
+// Bank gradient, dense in up to 4 x 4 cells (deform_bank_kernel with the samples taken by the lanes that use them).
+template <typename T, int V>
+__global__ void __launch_bounds__(32 * kRowWarps, 2) dcn_bank_kernel(const T* __restrict__ dyt, const T* __restrict__ xt,
+                                                                     const T* __restrict__ off, const T* __restrict__ rot,
+                                                                     float* __restrict__ partial, const Geom g, const int Cp) {
+  constexpr int CB = 32 * V;
+  __shared__ __align__(16) float room[kRowWarps * 16 * CB > kRowWarps * 32 * 20 ? kRowWarps * 16 * CB : kRowWarps * 32 * 20];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, c0 = blockIdx.y * CB, c = c0 + V * lane;
+  TapRec* recs = reinterpret_cast<TapRec*>(room) + warp * 32;
+  const int total = g.N * g.P, tiles = (total + 31) / 32;
+  unsigned long long acc[V][2][4] = {};
+  for (int u = blockIdx.x * kRowWarps + warp; u < g.taps * tiles; u += gridDim.x * kRowWarps) {
+    const int tap = u / tiles, flat0 = (u - tap * tiles) * 32, cnt = min(32, total - flat0);
+    __syncwarp();
+    tap_record<T, true>(flat0 + lane, total, tap, off, rot, g, Cp, recs + lane);
+    __syncwarp();
+    for (int j = 0; j < cnt; j += 4) {
+      float x[4][4][V], y[4][V];
+#pragma unroll
+      for (int h = 0; h < 4; ++h) {
+        const int4 idx = recs[j + h].idx;
+        get<T, V>(xt + idx.x + c, x[h][0]), get<T, V>(xt + idx.y + c, x[h][1]), get<T, V>(xt + idx.z + c, x[h][2]), get<T, V>(xt + idx.w + c, x[h][3]);
+        get<T, V>(dyt + recs[j + h].at.x + c, y[h]);
+      }
+#pragma unroll
+      for (int h = 0; h < 4; ++h) {
+        const float4 im = recs[j + h].im, hv = recs[j + h].b;
+        const ulonglong2 hu = *reinterpret_cast<const ulonglong2*>(&recs[j + h].a);
+#pragma unroll
+        for (int e = 0; e < V; ++e) {
+          const float dk = y[h][e] * (im.x * (im.z * x[h][0][e] + im.w * x[h][1][e]) + im.y * (im.z * x[h][2][e] + im.w * x[h][3][e]));
+          const float bb[4] = {dk * hv.x, dk * hv.y, dk * hv.z, dk * hv.w};
+#pragma unroll
+          for (int k = 0; k < 4; ++k) {
+            const unsigned long long w2 = pair(bb[k], bb[k]);
+            fma2(acc[e][0][k], hu.x, w2);
+            fma2(acc[e][1][k], hu.y, w2);
+          }
+        }
+      }
+    }
+  }
+  __syncthreads();
+#pragma unroll
+  for (int e = 0; e < V; ++e) {
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+      const float2 v = unpair(acc[e][i >> 2][i & 3]);
+      const int cell = (i >> 2) * 8 + (i & 3);
+      room[(warp * 16 + cell) * CB + V * lane + e] = v.x;
+      room[(warp * 16 + cell + 4) * CB + V * lane + e] = v.y;
+    }
+  }
+  __syncthreads();
+  for (int i = threadIdx.x; i < 16 * CB; i += 32 * kRowWarps) {
+    const int cell = i / CB, a = cell >> 2, b = cell & 3, ch = c0 + i % CB;
+    if (ch < g.C && a < g.scH && b < g.scW) {
+      float sum = 0.f;
+#pragma unroll
+      for (int k = 0; k < kRowWarps; ++k) sum += room[k * 16 * CB + i];
+      partial[((size_t)blockIdx.x * g.C + ch) * g.cells + a * g.scW + b] = sum;
+    }
+  }
+}
+
+// ------------------------------------------------------------------ host side
 size_t round256(size_t v) { return (v + 255) & ~(size_t)255; }
 
 bool bin_plan(const Geom& g, size_t elem, BinPlan& t) {
@@ -321,8 +546,21 @@ bool bin_plan(const Geom& g, size_t elem, BinPlan& t) {
   if (t.gather_smem > 110 * 1024 || (long long)g.N * t.bands > 0x7fffffff || (long long)g.N * kSortBlocks > 0x3fffffff) return false;
   t.starts_bytes = round256((size_t)g.N * (t.bins + 1) * sizeof(int));
   t.recs_bytes = round256((size_t)g.N * t.rec_per_n * sizeof(Rec));
-  t.bytes = t.starts_bytes + t.recs_bytes + round256((size_t)g.N * (g.P + 1) * t.Cp * elem);
+  t.dyt_bytes = round256((size_t)g.N * (g.P + 1) * t.Cp * elem);
+  t.bytes = t.starts_bytes + t.recs_bytes + t.dyt_bytes;
+  const int V = t.Cp % 64 == 0 ? 2 : 1;
+  const long long units = (long long)g.taps * (((long long)g.N * g.P + 31) / 32), most = (units + kRowWarps - 1) / kRowWarps;
+  t.bank_blocks = 2 * sms / (t.Cp / (32 * V));
+  if (t.bank_blocks < 1) t.bank_blocks = 1;
+  if (t.bank_blocks > most) t.bank_blocks = (int)most;
+  t.xt_bytes = round256((size_t)g.N * (g.HW + 1) * t.Cp * elem);
+  t.bankt_bytes = round256((size_t)(g.scH + 2) * (g.scW + 2) * t.Cp * sizeof(float));
+  t.all_bytes = t.bytes + t.xt_bytes + t.bankt_bytes + (size_t)t.bank_blocks * g.C * g.cells * sizeof(float);
   return true;
+}
+// the kernels above index all samples of x, dy and the units with 32 bits
+bool rows_shape(const Geom& g, const BinPlan& t) {
+  return (long long)g.N * (g.HW + 1) * t.Cp < 0x7fffffff && (long long)g.N * (g.P + 1) * t.Cp < 0x7fffffff && (long long)g.N * g.P * g.taps < 0x3fffffff;
 }
 
 }  // namespace
@@ -331,24 +569,25 @@ size_t deform_bins_workspace(const Geom& g, size_t elem) {
   BinPlan t;
   return bin_plan(g, elem, t) ? t.bytes : 0;
 }
+size_t deform_rows_workspace(const Geom& g, size_t elem) {
+  BinPlan t;
+  return bin_plan(g, elem, t) && rows_shape(g, t) ? t.all_bytes : 0;
+}
 
 template <typename T>
-int deform_data_bins(const T* dy, const T* off, const T* rot, const T* w, T* dx, const Geom& g, void* ws, size_t ws_bytes, cudaStream_t s) {
-  BinPlan t;
-  if (!bin_plan(g, sizeof(T), t) || ws == nullptr || ws_bytes < t.bytes) return DK_ERR_UNSUPPORTED;
-  int* starts = reinterpret_cast<int*>(ws);
-  Rec* recs = reinterpret_cast<Rec*>(reinterpret_cast<char*>(ws) + t.starts_bytes);
-  T* dyt = reinterpret_cast<T*>(reinterpret_cast<char*>(ws) + t.starts_bytes + t.recs_bytes);
-  int rc = enable_smem(dcn_bins_kernel<T>, t.sort_smem);
+static int launch_bins(const T* dy, const T* x, const T* off, const T* rot, const T* w, bool sort, int* starts, Rec* recs, T* dyt, T* xt,
+                       float* bankt, const Geom& g, BinPlan& t, cudaStream_t s) {
+  const int rc = enable_smem(dcn_bins_kernel<T>, t.sort_smem);
   if (rc) return rc;
-  auto gather = t.V == 1 ? dcn_gather_kernel<T, 1> : dcn_gather_kernel<T, 2>;
-  rc = enable_smem(gather, t.gather_smem);
-  if (rc) return rc;
-  const long long tiles = (long long)g.N * (t.Cp / 32) * (g.P / kMovePixels + 1);
-  long long clusters = (tiles + kSortBlocks - 1) / kSortBlocks;
+  t.sorted = sort ? g.N : 0;
+  long long tiles = (long long)g.N * (t.Cp / 32) * (g.P / kMovePixels + 1);
+  if (xt != nullptr) tiles += (long long)g.N * (t.Cp / 32) * (g.HW / kMovePixels + 1);
+  long long clusters = t.sorted + (tiles + kSortBlocks - 1) / kSortBlocks;
   if (clusters > 2 * device_sm_count() / kSortBlocks) clusters = 2 * device_sm_count() / kSortBlocks;
-  if (clusters < g.N) clusters = g.N;
-  t.movers = 3 * clusters >= 4 * (long long)g.N ? g.N * kSortBlocks : 0;
+  if (clusters < t.sorted) clusters = t.sorted;
+  if (clusters < 1) clusters = 1;
+  t.movers = 3 * clusters >= 4 * (long long)t.sorted ? t.sorted * kSortBlocks : 0;
+  if (clusters * kSortBlocks <= t.movers) t.movers = 0;
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3((unsigned)(clusters * kSortBlocks));
   cfg.blockDim = dim3(kSortThreads);
@@ -359,15 +598,80 @@ int deform_data_bins(const T* dy, const T* off, const T* rot, const T* w, T* dx,
   attr.val.clusterDim.x = kSortBlocks, attr.val.clusterDim.y = attr.val.clusterDim.z = 1;
   cfg.attrs = &attr;
   cfg.numAttrs = 1;
-  const cudaError_t e = cudaLaunchKernelEx(&cfg, dcn_bins_kernel<T>, dy, off, rot, starts, recs, dyt, g, t);
+  const cudaError_t e = cudaLaunchKernelEx(&cfg, dcn_bins_kernel<T>, dy, off, rot, starts, recs, dyt, x, xt, w, bankt, g, t);
   if (e != cudaSuccess) {
     set_last_cuda_error(e);
     return DK_ERR_CUDA;
   }
+  return check_launch();
+}
+
+template <typename T>
+static int launch_gather(const T* dyt, const int* starts, const Rec* recs, const T* w, T* dx, const Geom& g, const BinPlan& t, cudaStream_t s) {
+  auto gather = t.V == 1 ? dcn_gather_kernel<T, 1> : dcn_gather_kernel<T, 2>;
+  const int rc = enable_smem(gather, t.gather_smem);
+  if (rc) return rc;
   gather<<<dim3((unsigned)(g.N * t.bands), t.groups), 32 * kGatherWarps, t.gather_smem, s>>>(dyt, starts, recs, w, dx, g, t);
   return check_launch();
 }
-template int deform_data_bins<float>(const float*, const float*, const float*, const float*, float*, const Geom&, void*, size_t, cudaStream_t);
-template int deform_data_bins<__half>(const __half*, const __half*, const __half*, const __half*, __half*, const Geom&, void*, size_t, cudaStream_t);
+
+template <typename T>
+int deform_data_bins(const T* dy, const T* off, const T* rot, const T* w, T* dx, const Geom& g, void* ws, size_t ws_bytes, cudaStream_t s) {
+  BinPlan t;
+  if (!bin_plan(g, sizeof(T), t) || ws == nullptr || ws_bytes < t.bytes) return DK_ERR_UNSUPPORTED;
+  char* at = reinterpret_cast<char*>(ws);
+  int* starts = reinterpret_cast<int*>(at);
+  Rec* recs = reinterpret_cast<Rec*>(at + t.starts_bytes);
+  T* dyt = reinterpret_cast<T*>(at + t.starts_bytes + t.recs_bytes);
+  const int rc = launch_bins<T>(dy, nullptr, off, rot, w, true, starts, recs, dyt, nullptr, nullptr, g, t, s);
+  return rc ? rc : launch_gather<T>(dyt, starts, recs, w, dx, g, t, s);
+}
+
+// The wanted gradients (null: not wanted) from one pass that brings the operands into channel order.  The bank gradient, where
+// the scope is larger than 4 x 4, is left to the caller (*bank_done).
+template <typename T>
+int deform_backward_rows(const T* dy, const T* x, const T* off, const T* rot, const T* w, T* dx, T* doff, T* drot, T* dw, const Geom& g,
+                         void* ws, size_t ws_bytes, cudaStream_t s, bool* bank_done) {
+  BinPlan t;
+  *bank_done = false;
+  const bool bank = dw != nullptr && g.scH <= 4 && g.scW <= 4, coords = doff != nullptr || drot != nullptr;
+  if (!bin_plan(g, sizeof(T), t) || !rows_shape(g, t) || ws == nullptr || ws_bytes < t.all_bytes) return DK_ERR_UNSUPPORTED;
+  if (!dx && !coords && !bank) return DK_ERR_UNSUPPORTED;
+  char* at = reinterpret_cast<char*>(ws);
+  int* starts = reinterpret_cast<int*>(at);
+  Rec* recs = reinterpret_cast<Rec*>(at + t.starts_bytes);
+  T* dyt = reinterpret_cast<T*>(at + t.starts_bytes + t.recs_bytes);
+  T* xt = reinterpret_cast<T*>(at + t.bytes);
+  float* bankt = reinterpret_cast<float*>(at + t.bytes + t.xt_bytes);
+  float* partial = reinterpret_cast<float*>(at + t.bytes + t.xt_bytes + t.bankt_bytes);
+  int rc = launch_bins<T>(dy, x, off, rot, w, dx != nullptr, starts, recs, dyt, coords || bank ? xt : nullptr, bankt, g, t, s);
+  if (rc) return rc;
+  if (dx && (rc = launch_gather<T>(dyt, starts, recs, w, dx, g, t, s))) return rc;
+  const int V = t.Cp % 64 == 0 ? 2 : 1, groups = t.Cp / (32 * V), units = g.taps * ((g.N * g.P + 31) / 32);
+  if (coords) {
+    // warps share a unit's channels until there are 16 on every SM
+    int S = 1;
+    while (S < kRowWarps && 2 * S <= groups && (long long)units * S < 16 * device_sm_count()) S *= 2;
+    auto kern = V == 2 ? (drot ? dcn_coords_kernel<T, 2, true> : dcn_coords_kernel<T, 2, false>)
+                       : (drot ? dcn_coords_kernel<T, 1, true> : dcn_coords_kernel<T, 1, false>);
+    const int per_block = kRowWarps / S;
+    kern<<<(units + per_block - 1) / per_block, 32 * kRowWarps, 0, s>>>(dyt, xt, bankt, off, rot, doff, drot, g, t.Cp, S);
+    if ((rc = check_launch())) return rc;
+  }
+  if (bank) {
+    auto kern = V == 2 ? dcn_bank_kernel<T, 2> : dcn_bank_kernel<T, 1>;
+    kern<<<dim3(t.bank_blocks, groups), 32 * kRowWarps, 0, s>>>(dyt, xt, off, rot, partial, g, t.Cp);
+    if ((rc = check_launch())) return rc;
+    if ((rc = reduce_bank<T>(partial, dw, g.C * g.cells, t.bank_blocks, s))) return rc;
+    *bank_done = true;
+  }
+  return DK_OK;
+}
+#define DK_INSTANTIATE_BINS(T)                                                                                                         \
+  template int deform_data_bins<T>(const T*, const T*, const T*, const T*, T*, const Geom&, void*, size_t, cudaStream_t);              \
+  template int deform_backward_rows<T>(const T*, const T*, const T*, const T*, const T*, T*, T*, T*, T*, const Geom&, void*, size_t,   \
+                                       cudaStream_t, bool*);
+DK_INSTANTIATE_BINS(float)
+DK_INSTANTIATE_BINS(__half)
 
 }  // namespace dk

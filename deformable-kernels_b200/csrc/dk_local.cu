@@ -632,6 +632,15 @@ FilterPlan filter_plan_fit(const Geom& g, size_t acc_bytes, size_t max_bytes) {
   return pl;
 }
 
+// sums partial bank gradients [blocks][n_out] in order
+template <typename T>
+int reduce_bank(const float* partial, T* dw, int n_out, int blocks, cudaStream_t s) {
+  reduce_partials_kernel<T><<<(n_out + 31) / 32, 256, 0, s>>>(partial, dw, n_out, blocks);
+  return check_launch();
+}
+template int reduce_bank<float>(const float*, float*, int, int, cudaStream_t);
+template int reduce_bank<__half>(const float*, __half*, int, int, cudaStream_t);
+
 template <typename T, bool DEFORM>
 static int filter_backward(const T* dy, const T* x, const T* off, const T* rot, T* dw, const Geom& g, void* ws,
                            size_t ws_bytes, cudaStream_t s, bool fit = false) {

@@ -53,21 +53,6 @@ TilePlan tile_plan(const Geom& g, int pixels) {
   return t;
 }
 
-// two fp32 multiply-adds in one instruction: the pipe needs as long as for two, but the loads beside them get issue slots
-__device__ __forceinline__ unsigned long long pair(float a, float b) {
-  unsigned long long r;
-  asm("mov.b64 %0, {%1, %2};\n" : "=l"(r) : "f"(a), "f"(b));
-  return r;
-}
-__device__ __forceinline__ float2 unpair(unsigned long long v) {
-  float2 r;
-  asm("mov.b64 {%0, %1}, %2;\n" : "=f"(r.x), "=f"(r.y) : "l"(v));
-  return r;
-}
-__device__ __forceinline__ void fma2(unsigned long long& acc, unsigned long long a, unsigned long long b) {
-  asm("fma.rn.f32x2 %0, %1, %2, %0;\n" : "+l"(acc) : "l"(a), "l"(b));
-}
-
 __device__ __forceinline__ int over(int e, int d, unsigned magic) { return d == 1 ? e : (int)__umulhi((unsigned)e, magic); }
 __device__ __forceinline__ float hat1(float t) { return __saturatef(1.f - fabsf(t)); }  // max(0, 1 - |t|)
 

@@ -1,4 +1,4 @@
-"""DK + DCN bank and input gradients where the tensor-core kernels do not apply (fp32; fp16 with channels that are no multiple of
+"""DK + DCN gradients where the tensor-core kernels do not apply (fp32; fp16 with channels that are no multiple of
 16 or planes beyond 56 x 56): remainders of the 32-channel groups, of the 32-pixel tiles and of the bands and pieces of rows,
 single pixels, other strides, paddings and dilations, scopes other than 4 x 4, samples far outside, NaN offsets."""
 import pytest
@@ -16,18 +16,31 @@ SHAPES = [
 
 @pytest.mark.parametrize("n,c,h,w,stride,pad,dil,scope", SHAPES)
 @pytest.mark.parametrize("dtype", [torch.float32, torch.float16])
-def test_input_and_bank_gradient(n, c, h, w, stride, pad, dil, scope, dtype):
+def test_gradients(n, c, h, w, stride, pad, dil, scope, dtype):
     from deformable_kernels.ops.deform_kernel.functions import deform_sample_depthwise
     from oracle import dk_oracle as O
     case = make_case(n, c, h, w, scope=scope, stride=stride, pad=pad, dil=dil, rot_std=0.8, off_std=1.5, seed=c + h)
     if h > 4:
         case["offset"][0, 0, 0, 0], case["offset"][0, 3, -1, -1], case["offset"][0, 8, 1, 1] = float("nan"), 1e9, -float("inf")
     x, o, r, wt, dy = (case[k].to(dtype).to(DEV) for k in ("input", "offset", "rotation", "weight", "grad_output"))
-    x.requires_grad_(True), wt.requires_grad_(True)
-    dx, dw = torch.autograd.grad(deform_sample_depthwise(x, o, r, wt, **case["args"]), [x, wt], dy)
+    leaves = [t.requires_grad_(True) for t in (x, o, r, wt)]
+    got = torch.autograd.grad(deform_sample_depthwise(*leaves, **case["args"]), leaves, dy)
     up = torch.float32 if dtype == torch.float16 else torch.float64
     a = [case[k].to(dtype).to(up) for k in ("grad_output", "input", "offset", "rotation", "weight")]
     want = O.deform_sample_depthwise_backward(*a, **case["args"])
     tol = 2e-3 if dtype == torch.float16 else 1e-5
-    assert rel_err(dx, want[0].to(dtype)) < tol
-    assert rel_err(dw, want[3].to(dtype)) < tol
+    for g, w in zip(got, want):
+        assert rel_err(g, w.to(dtype)) < tol
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.float16])
+def test_subsets_of_the_gradients_agree(dtype):
+    from deformable_kernels.ops.deform_kernel.functions import deform_sample_depthwise
+    case = make_case(2, 72, 11, 13, rot_std=0.8, off_std=1.5, seed=5)
+    x, o, r, wt, dy = (case[k].to(dtype).to(DEV) for k in ("input", "offset", "rotation", "weight", "grad_output"))
+    leaves = [t.requires_grad_(True) for t in (x, o, r, wt)]
+    full = torch.autograd.grad(deform_sample_depthwise(*leaves, **case["args"]), leaves, dy)
+    for i, leaf in enumerate(leaves):
+        args = [t if t is leaf else t.detach() for t in leaves]
+        one, = torch.autograd.grad(deform_sample_depthwise(*args, **case["args"]), [leaf], dy)
+        assert rel_err(one, full[i]) < (2e-3 if dtype == torch.float16 else 1e-5)
