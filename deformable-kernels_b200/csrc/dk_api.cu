@@ -304,13 +304,8 @@ int dk_deform_sample_depthwise_forward(const void* input, const void* offset, co
 size_t dk_deform_sample_depthwise_backward_data_workspace_bytes(const dk_geom* g, int dtype) {
   Geom gg;
   if (!make_geom(g, &gg) || !dtype_ok(dtype)) return 0;
-  if (dtype == DK_F64) return 0;
-  size_t need = dtype == DK_F16 ? align256((size_t)gg.N * gg.C * gg.HW * sizeof(float)) : 0;
-  if (dtype != DK_F16 || deform_data_mma_workspace(gg) == 0) {
-    const size_t bins = align256(deform_bins_workspace(gg, dtype == DK_F16 ? 2 : 4));
-    if (bins > need) need = bins;
-  }
-  return need;
+  if (dtype != DK_F16) return 0;
+  return align256((size_t)gg.N * gg.C * gg.HW * sizeof(float));
 }
 
 int dk_deform_sample_depthwise_backward_data(const void* grad_output, const void* offset, const void* rotation,
@@ -370,11 +365,12 @@ int dk_deform_sample_depthwise_backward_rotation(const void* grad_output, const 
                                                P_(T, filter), (T*)nullptr, M_(T, grad_rotation), gg, (cudaStream_t)stream))
 }
 
-/* Whether the fused backward takes the kernels with channels on the lanes: where no tensor-core kernel applies. */
-static bool deform_by_rows(const Geom& g, int dtype) {
-  if (dtype == DK_F16)
-    return deform_data_mma_workspace(g) == 0 && deform_coords_mma_workspace(g) == 0 && deform_filter_mma_workspace(g) == 0;
-  return dtype == DK_F32;
+/* Whether the fused backward takes the kernels with channels on the lanes: where no tensor-core kernel applies; for
+ * grad-input alone (`data`) where that one has none. */
+static bool deform_by_rows(const Geom& g, int dtype, bool data) {
+  if (dtype != DK_F16) return dtype == DK_F32;
+  return deform_data_mma_workspace(g) == 0 &&
+         (data || (deform_coords_mma_workspace(g) == 0 && deform_filter_mma_workspace(g) == 0));
 }
 
 /* First region of the fused backward's workspace: used by grad-input, then (same stream) by the offset gradients. */
@@ -385,7 +381,7 @@ static size_t deform_front_ws(const dk_geom* g, int dtype) {
     const size_t c = align256(deform_coords_mma_workspace(gg));
     if (c > need) need = c;
   }
-  if (make_geom(g, &gg) && deform_by_rows(gg, dtype)) {
+  if (make_geom(g, &gg) && deform_by_rows(gg, dtype, true)) {
     const size_t rows = align256(deform_rows_workspace(gg, dtype == DK_F16 ? 2 : 4));
     if (rows > need) need = rows;
   }
@@ -435,32 +431,29 @@ int dk_deform_sample_depthwise_backward(const void* grad_output, const void* inp
                              gg, (char*)workspace + data_ws, filt_ws, s);
     return rc;
   }
-  if (deform_by_rows(gg, dtype)) {
+  if (deform_by_rows(gg, dtype, true)) {
+    const bool all = deform_by_rows(gg, dtype, false);
+    const size_t room = workspace && workspace_bytes >= data_ws ? data_ws : 0;
     bool bank_done = false;
-    if (dtype == DK_F16)
-      rc = deform_backward_rows<__half>(P_(__half, grad_output), P_(__half, input), P_(__half, offset), P_(__half, rotation),
-                                        P_(__half, filter), M_(__half, grad_input), M_(__half, grad_offset), M_(__half, grad_rotation),
-                                        M_(__half, grad_filter), gg, workspace, workspace_bytes < data_ws ? 0 : data_ws,
-                                        (cudaStream_t)stream, &bank_done);
-    else
-      rc = deform_backward_rows<float>(P_(float, grad_output), P_(float, input), P_(float, offset), P_(float, rotation),
-                                       P_(float, filter), M_(float, grad_input), M_(float, grad_offset), M_(float, grad_rotation),
-                                       M_(float, grad_filter), gg, workspace, workspace_bytes < data_ws ? 0 : data_ws,
-                                       (cudaStream_t)stream, &bank_done);
-    if (rc == DK_OK && (bank_done || !grad_filter)) return rc;
-    if (rc == DK_OK) {
-      if (workspace_bytes < data_ws + filt_ws) return DK_ERR_WORKSPACE;
-      return dk_deform_sample_depthwise_backward_filter(grad_output, input, offset, rotation, grad_filter, g, dtype,
-                                                        (char*)workspace + data_ws, filt_ws, stream);
+#define DK_ROWS(T)                                                                                                             \
+  deform_backward_rows<T>(P_(T, grad_output), P_(T, input), P_(T, offset), P_(T, rotation), P_(T, filter), M_(T, grad_input), \
+                          all ? M_(T, grad_offset) : nullptr, all ? M_(T, grad_rotation) : nullptr,                           \
+                          all ? M_(T, grad_filter) : nullptr, gg, workspace, room, (cudaStream_t)stream, &bank_done)
+    rc = dtype == DK_F16 ? DK_ROWS(__half) : DK_ROWS(float);
+#undef DK_ROWS
+    if (rc == DK_OK) {  // what is left
+      grad_input = nullptr;
+      if (all) grad_offset = grad_rotation = nullptr;
+      if (bank_done) grad_filter = nullptr;
+    } else if (rc != DK_ERR_UNSUPPORTED) {
+      return rc;
     }
-    if (rc != DK_ERR_UNSUPPORTED) return rc;
     rc = DK_OK;
   }
   if (grad_input) {
-    const bool room = workspace && workspace_bytes >= data_ws;
-    if (dtype == DK_F16 && !room) return DK_ERR_WORKSPACE;  // fp32 falls back to a kernel that needs none
-    rc = dk_deform_sample_depthwise_backward_data(grad_output, offset, rotation, filter, grad_input, g, dtype,
-                                                  room ? workspace : nullptr, room ? data_ws : 0, stream);
+    if (dtype == DK_F16 && (!workspace || workspace_bytes < data_ws)) return DK_ERR_WORKSPACE;
+    rc = dk_deform_sample_depthwise_backward_data(grad_output, offset, rotation, filter, grad_input, g, dtype, workspace,
+                                                  data_ws, stream);
     if (rc) return rc;
   }
   bool bank_done = false;

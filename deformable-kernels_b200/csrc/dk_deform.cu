@@ -251,10 +251,6 @@ int deform_backward_data(const T* dy, const T* off, const T* rot, const T* w, T*
       if (rc != DK_ERR_UNSUPPORTED) return rc;
     }
   }
-  if constexpr (sizeof(T) <= 4) {
-    const int rc = deform_data_bins<T>(dy, off, rot, w, dx, g, ws, ws_bytes, s);
-    if (rc != DK_ERR_UNSUPPORTED) return rc;
-  }
   {
     // planes of 8 channels in shared memory, when they fit
     constexpr int CP = 8;

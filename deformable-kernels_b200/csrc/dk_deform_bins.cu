@@ -1,4 +1,4 @@
-// Grad-input of DK + DCN where the tensor-core kernel does not apply (fp32; fp16 with channels that are no multiple of 16, other
+// Gradients of DK + DCN where the tensor-core kernels do not apply (fp32; fp16 with channels that are no multiple of 16, other
 // scopes, planes beyond 56 x 56), one offset group.
 //
 // The scatter of dy * k into the four corners of every sample point is 36 float additions to colliding addresses per output,
@@ -192,6 +192,11 @@ __device__ __forceinline__ void get(const T* p, float (&v)[V]) {
     v[0] = q.x, v[1] = q.y;
   }
 }
+// the same at a byte offset: one addition and no 64-bit address per load
+template <typename T, int V>
+__device__ __forceinline__ void get_at(const T* base, unsigned off, float (&v)[V]) {
+  get<T, V>(reinterpret_cast<const T*>(reinterpret_cast<const char*>(base) + off), v);
+}
 template <int V>
 __device__ __forceinline__ void put(float* p, const float (&v)[V]) {
   if constexpr (V == 1) *p = v[0];
@@ -322,9 +327,13 @@ __global__ void __launch_bounds__(32 * kGatherWarps, 3) dcn_gather_kernel(const 
 // With x, dy and the bank in channel order a corner of a sample is one line for 32 (64) channels instead of one line per lane, and
 // the corner indices and fractions, worked out by one lane per sample, are shared by all channels.  Corners outside the image
 // read the zero pixel, cells outside the bank its zero border, so nothing is masked.  A unit of a warp is 32 pixels of a tap.
+// Offsets, with x and dy brought into channel order for it alone: 16 x 192 of 28 x 28 120 -> 70 us, 8 x 960 of 7 x 7 222 -> 33; bank
+// 167 -> 62.  All gradients from one preparation: 16 x 192 of 28 x 28 531 -> 183 us, 13 x 96 of 80 x 80 2704 -> 773, fp16 13 x 88
+// of 80 x 80 2424 -> 713, 64 x 384 of 14 x 14 1061 -> 300, 32 x 72 of 56 x 56 at stride 2 551 -> 265.  Bound by issue: 28
+// multiply-adds beside nine loads and their addresses.
 constexpr int kRowWarps = 8;
 
-// offsets of the four corners; {1 - lh, lh, 1 - lw, lw}; for the coordinates the same of the bank and {dy, bank cell}, for the bank
+// byte offsets of the four corners; {1 - lh, lh, 1 - lw, lw}; for the coordinates the same of the bank and {dy, bank cell}, for the bank
 // the hat functions of its rows and columns and {dy}
 struct TapRec {
   int4 idx;
@@ -337,8 +346,9 @@ __device__ __forceinline__ void tap_record(int flat, int total, int tap, const T
                                            int Cp, TapRec* to) {
   const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f);
   TapRec r;
-  const int nothing = g.HW * Cp;  // the zero pixels of the first sample
-  r.idx = make_int4(nothing, nothing, nothing, nothing), r.im = r.a = r.b = zero, r.at = make_int4(g.P * Cp, 0, 0, 0);
+  const unsigned px_bytes = Cp * (unsigned)sizeof(T);
+  const int nothing = (int)(g.HW * px_bytes);  // the zero pixels of the first sample
+  r.idx = make_int4(nothing, nothing, nothing, nothing), r.im = r.a = r.b = zero, r.at = make_int4((int)(g.P * px_bytes), 0, 0, 0);
   if (flat < total) {
     const int n = flat / g.P, p = flat - n * g.P;
     Point q;
@@ -346,10 +356,10 @@ __device__ __forceinline__ void tap_record(int flat, int total, int tap, const T
       const int base = n * (g.HW + 1);
       const bool r0 = q.h0 >= 0, r1 = q.h0 + 1 < g.H, k0 = q.w0 >= 0, k1 = q.w0 + 1 < g.W;
       const int px = q.h0 * g.W + q.w0;
-      r.idx.x = (base + (r0 && k0 ? px : g.HW)) * Cp, r.idx.y = (base + (r0 && k1 ? px + 1 : g.HW)) * Cp;
-      r.idx.z = (base + (r1 && k0 ? px + g.W : g.HW)) * Cp, r.idx.w = (base + (r1 && k1 ? px + g.W + 1 : g.HW)) * Cp;
+      r.idx.x = (int)((base + (r0 && k0 ? px : g.HW)) * px_bytes), r.idx.y = (int)((base + (r0 && k1 ? px + 1 : g.HW)) * px_bytes);
+      r.idx.z = (int)((base + (r1 && k0 ? px + g.W : g.HW)) * px_bytes), r.idx.w = (int)((base + (r1 && k1 ? px + g.W + 1 : g.HW)) * px_bytes);
       r.im = make_float4(1.f - q.lh, q.lh, 1.f - q.lw, q.lw);
-      r.at.x = (n * (g.P + 1) + p) * Cp;
+      r.at.x = (int)((n * (g.P + 1) + p) * px_bytes);
       if (BANK) {
         float* hu = reinterpret_cast<float*>(&r.a);
         float* hv = reinterpret_cast<float*>(&r.b);
@@ -360,7 +370,7 @@ __device__ __forceinline__ void tap_record(int flat, int total, int tap, const T
         }
       } else {
         r.a = make_float4(1.f - q.lu, q.lu, 1.f - q.lv, q.lv);
-        r.at.y = ((q.u0 + 1) * (g.scW + 2) + q.v0 + 1) * Cp;
+        r.at.y = ((q.u0 + 1) * (g.scW + 2) + q.v0 + 1) * Cp * (int)sizeof(float);
       }
     }
   }
@@ -381,21 +391,23 @@ __global__ void __launch_bounds__(32 * kRowWarps, 3) dcn_coords_kernel(const T* 
   const int tap = u / tiles, flat0 = (u - tap * tiles) * 32, cnt = tap < g.taps ? min(32, total - flat0) : 0;
   if (cnt > 0) tap_record<T, false>(flat0 + lane, total, tap, off, rot, g, Cp, &recs[warp][lane]);
   __syncwarp();
-  const int row = (g.scW + 2) * Cp;
+  const unsigned cell = Cp * sizeof(float), row = (g.scW + 2) * cell;
   for (int j = 0; j < cnt; j += 2) {
     float s[2][4] = {};
 #pragma unroll 1
     for (int c = (share * 32 + lane) * V; c < Cp; c += S * 32 * V) {
+      const unsigned cb = c * (unsigned)sizeof(T);
       float x[2][4][V], k[2][4][V], y[2][V];
 #pragma unroll
       for (int h = 0; h < 2; ++h) {
         const TapRec& r = recs[warp][j + h];
         const int4 idx = r.idx;
         const int2 at = *reinterpret_cast<const int2*>(&r.at);
-        get<T, V>(xt + idx.x + c, x[h][0]), get<T, V>(xt + idx.y + c, x[h][1]), get<T, V>(xt + idx.z + c, x[h][2]), get<T, V>(xt + idx.w + c, x[h][3]);
-        get<T, V>(dyt + at.x + c, y[h]);
-        const float* bk = bankt + at.y + c;
-        get<float, V>(bk, k[h][0]), get<float, V>(bk + Cp, k[h][1]), get<float, V>(bk + row, k[h][2]), get<float, V>(bk + row + Cp, k[h][3]);
+        get_at<T, V>(xt, idx.x + cb, x[h][0]), get_at<T, V>(xt, idx.y + cb, x[h][1]), get_at<T, V>(xt, idx.z + cb, x[h][2]), get_at<T, V>(xt, idx.w + cb, x[h][3]);
+        get_at<T, V>(dyt, at.x + cb, y[h]);
+        const unsigned bk = at.y + c * (unsigned)sizeof(float);
+        get_at<float, V>(bankt, bk, k[h][0]), get_at<float, V>(bankt, bk + cell, k[h][1]);
+        get_at<float, V>(bankt, bk + row, k[h][2]), get_at<float, V>(bankt, bk + row + cell, k[h][3]);
       }
 #pragma unroll
       for (int h = 0; h < 2; ++h) {
@@ -454,7 +466,7 @@ __global__ void __launch_bounds__(32 * kRowWarps, 2) dcn_bank_kernel(const T* __
                                                                      float* __restrict__ partial, const Geom g, const int Cp) {
   constexpr int CB = 32 * V;
   __shared__ __align__(16) float room[kRowWarps * 16 * CB > kRowWarps * 32 * 20 ? kRowWarps * 16 * CB : kRowWarps * 32 * 20];
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, c0 = blockIdx.y * CB, c = c0 + V * lane;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, c0 = blockIdx.y * CB, cb = (c0 + V * lane) * (int)sizeof(T);
   TapRec* recs = reinterpret_cast<TapRec*>(room) + warp * 32;
   const int total = g.N * g.P, tiles = (total + 31) / 32;
   unsigned long long acc[V][2][4] = {};
@@ -468,8 +480,8 @@ __global__ void __launch_bounds__(32 * kRowWarps, 2) dcn_bank_kernel(const T* __
 #pragma unroll
       for (int h = 0; h < 4; ++h) {
         const int4 idx = recs[j + h].idx;
-        get<T, V>(xt + idx.x + c, x[h][0]), get<T, V>(xt + idx.y + c, x[h][1]), get<T, V>(xt + idx.z + c, x[h][2]), get<T, V>(xt + idx.w + c, x[h][3]);
-        get<T, V>(dyt + recs[j + h].at.x + c, y[h]);
+        get_at<T, V>(xt, idx.x + cb, x[h][0]), get_at<T, V>(xt, idx.y + cb, x[h][1]), get_at<T, V>(xt, idx.z + cb, x[h][2]), get_at<T, V>(xt, idx.w + cb, x[h][3]);
+        get_at<T, V>(dyt, recs[j + h].at.x + cb, y[h]);
       }
 #pragma unroll
       for (int h = 0; h < 4; ++h) {
@@ -527,7 +539,7 @@ bool bin_plan(const Geom& g, size_t elem, BinPlan& t) {
     for (int R = 1; R < kGatherWarps; R = 2 * R + 1) {
       const int groups = (g.C + 32 * V - 1) / (32 * V), held = R < g.H ? R : g.H;
       if ((long long)held * g.W * (V == 1 ? 33 : 66) * 4 > 72 * 1024) continue;
-      const long long blocks = (long long)g.N * groups * ((g.H + R - 1) / R), cost = (blocks + sms - 1) / sms * (R + 4) * (V == 1 ? 10 : 13);
+      const long long blocks = (long long)g.N * groups * ((g.H + R - 1) / R), cost = (blocks + 2 * sms - 1) / (2 * sms) * (R + 4) * (V == 1 ? 10 : 13);
       if (best >= 0 && cost >= best) continue;
       best = cost;
       t.V = V, t.groups = groups, t.R = held, t.bands = (g.H + R - 1) / R;
@@ -558,17 +570,13 @@ bool bin_plan(const Geom& g, size_t elem, BinPlan& t) {
   t.all_bytes = t.bytes + t.xt_bytes + t.bankt_bytes + (size_t)t.bank_blocks * g.C * g.cells * sizeof(float);
   return true;
 }
-// the kernels above index all samples of x, dy and the units with 32 bits
+// the kernels above address all samples of x and dy with 32 bits of bytes
 bool rows_shape(const Geom& g, const BinPlan& t) {
-  return (long long)g.N * (g.HW + 1) * t.Cp < 0x7fffffff && (long long)g.N * (g.P + 1) * t.Cp < 0x7fffffff && (long long)g.N * g.P * g.taps < 0x3fffffff;
+  return t.xt_bytes < 0xf0000000u && t.dyt_bytes < 0xf0000000u && (long long)g.N * g.P * g.taps < 0x3fffffff;
 }
 
 }  // namespace
 
-size_t deform_bins_workspace(const Geom& g, size_t elem) {
-  BinPlan t;
-  return bin_plan(g, elem, t) ? t.bytes : 0;
-}
 size_t deform_rows_workspace(const Geom& g, size_t elem) {
   BinPlan t;
   return bin_plan(g, elem, t) && rows_shape(g, t) ? t.all_bytes : 0;
@@ -615,18 +623,6 @@ static int launch_gather(const T* dyt, const int* starts, const Rec* recs, const
   return check_launch();
 }
 
-template <typename T>
-int deform_data_bins(const T* dy, const T* off, const T* rot, const T* w, T* dx, const Geom& g, void* ws, size_t ws_bytes, cudaStream_t s) {
-  BinPlan t;
-  if (!bin_plan(g, sizeof(T), t) || ws == nullptr || ws_bytes < t.bytes) return DK_ERR_UNSUPPORTED;
-  char* at = reinterpret_cast<char*>(ws);
-  int* starts = reinterpret_cast<int*>(at);
-  Rec* recs = reinterpret_cast<Rec*>(at + t.starts_bytes);
-  T* dyt = reinterpret_cast<T*>(at + t.starts_bytes + t.recs_bytes);
-  const int rc = launch_bins<T>(dy, nullptr, off, rot, w, true, starts, recs, dyt, nullptr, nullptr, g, t, s);
-  return rc ? rc : launch_gather<T>(dyt, starts, recs, w, dx, g, t, s);
-}
-
 // The wanted gradients (null: not wanted) from one pass that brings the operands into channel order.  The bank gradient, where
 // the scope is larger than 4 x 4, is left to the caller (*bank_done).
 template <typename T>
@@ -636,6 +632,9 @@ int deform_backward_rows(const T* dy, const T* x, const T* off, const T* rot, co
   *bank_done = false;
   const bool bank = dw != nullptr && g.scH <= 4 && g.scW <= 4, coords = doff != nullptr || drot != nullptr;
   if (!bin_plan(g, sizeof(T), t) || !rows_shape(g, t) || ws == nullptr || ws_bytes < t.all_bytes) return DK_ERR_UNSUPPORTED;
+  // one gradient alone has to pay for bringing x and dy into channel order: offsets of 16 x 192 of 28 x 28 120 -> 77 us, but
+  // 32 x 72 of 56 x 56, stride 2, 100 -> 134; bank of 1 x 960 of 7 x 7 12 -> 19
+  if (!dx && !(coords && bank) && (g.C < 96 || (!coords && (long long)g.N * g.P < 2048))) return DK_ERR_UNSUPPORTED;
   if (!dx && !coords && !bank) return DK_ERR_UNSUPPORTED;
   char* at = reinterpret_cast<char*>(ws);
   int* starts = reinterpret_cast<int*>(at);
@@ -667,11 +666,9 @@ int deform_backward_rows(const T* dy, const T* x, const T* off, const T* rot, co
   }
   return DK_OK;
 }
-#define DK_INSTANTIATE_BINS(T)                                                                                                         \
-  template int deform_data_bins<T>(const T*, const T*, const T*, const T*, T*, const Geom&, void*, size_t, cudaStream_t);              \
-  template int deform_backward_rows<T>(const T*, const T*, const T*, const T*, const T*, T*, T*, T*, T*, const Geom&, void*, size_t,   \
-                                       cudaStream_t, bool*);
-DK_INSTANTIATE_BINS(float)
-DK_INSTANTIATE_BINS(__half)
+template int deform_backward_rows<float>(const float*, const float*, const float*, const float*, const float*, float*, float*, float*, float*,
+                                        const Geom&, void*, size_t, cudaStream_t, bool*);
+template int deform_backward_rows<__half>(const __half*, const __half*, const __half*, const __half*, const __half*, __half*, __half*, __half*,
+                                         __half*, const Geom&, void*, size_t, cudaStream_t, bool*);
 
 }  // namespace dk

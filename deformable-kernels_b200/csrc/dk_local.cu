@@ -646,8 +646,9 @@ static int filter_backward(const T* dy, const T* x, const T* off, const T* rot, 
                            size_t ws_bytes, cudaStream_t s, bool fit = false) {
   using A = typename Compute<T>::type;
   if constexpr (DEFORM && sizeof(T) <= 4) {
+    // planes of less than two tiles keep the kernels below (8 x 960 of 7 x 7: 24 us against 28)
     int blocks = 0;
-    int rc = deform_bank<T>(dy, x, off, rot, reinterpret_cast<float*>(ws), g, ws_bytes, &blocks, s);
+    int rc = g.P < 64 ? (int)DK_ERR_UNSUPPORTED : deform_bank<T>(dy, x, off, rot, reinterpret_cast<float*>(ws), g, ws_bytes, &blocks, s);
     if (rc == DK_OK) {
       const int n_out = g.C * g.cells;
       reduce_partials_kernel<T><<<(n_out + 31) / 32, 256, 0, s>>>(reinterpret_cast<const A*>(ws), dw, n_out, blocks);
