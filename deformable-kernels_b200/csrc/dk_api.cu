@@ -301,6 +301,35 @@ int dk_deform_sample_depthwise_forward(const void* input, const void* offset, co
                                        (cudaStream_t)stream))
 }
 
+/* Whether the forward and the fused backward take the kernels with channels on the lanes: where no tensor-core kernel applies; for
+ * grad-input alone (`data`) where that one has none. */
+static bool deform_by_rows(const Geom& g, int dtype, bool data) {
+  if (dtype != DK_F16) return dtype == DK_F32;
+  return deform_data_mma_workspace(g) == 0 &&
+         (data || (deform_coords_mma_workspace(g) == 0 && deform_filter_mma_workspace(g) == 0));
+}
+
+size_t dk_deform_sample_depthwise_forward_workspace_bytes(const dk_geom* g, int dtype) {
+  Geom gg;
+  if (!make_geom(g, &gg) || !deform_by_rows(gg, dtype, false)) return 0;
+  return align256(deform_forward_rows_workspace(gg, dtype == DK_F16 ? 2 : 4));
+}
+
+int dk_deform_sample_depthwise_forward_ws(const void* input, const void* offset, const void* rotation, const void* filter,
+                                          void* output, const dk_geom* g, int dtype, void* workspace, size_t workspace_bytes,
+                                          void* stream) {
+  Geom gg;
+  if (!input || !offset || !filter || !output || !make_geom(g, &gg)) return DK_ERR_BAD_ARGUMENT;
+  const size_t need = dk_deform_sample_depthwise_forward_workspace_bytes(g, dtype);
+  if (need == 0) return dk_deform_sample_depthwise_forward(input, offset, rotation, filter, output, g, dtype, stream);
+  if (!workspace || workspace_bytes < need) return DK_ERR_WORKSPACE;
+  if (dtype == DK_F16)
+    return deform_forward_rows<__half>(P_(__half, input), P_(__half, offset), P_(__half, rotation), P_(__half, filter),
+                                       M_(__half, output), gg, workspace, workspace_bytes, (cudaStream_t)stream);
+  return deform_forward_rows<float>(P_(float, input), P_(float, offset), P_(float, rotation), P_(float, filter),
+                                    M_(float, output), gg, workspace, workspace_bytes, (cudaStream_t)stream);
+}
+
 size_t dk_deform_sample_depthwise_backward_data_workspace_bytes(const dk_geom* g, int dtype) {
   Geom gg;
   if (!make_geom(g, &gg) || !dtype_ok(dtype)) return 0;
@@ -365,14 +394,6 @@ int dk_deform_sample_depthwise_backward_rotation(const void* grad_output, const 
                                                P_(T, filter), (T*)nullptr, M_(T, grad_rotation), gg, (cudaStream_t)stream))
 }
 
-/* Whether the fused backward takes the kernels with channels on the lanes: where no tensor-core kernel applies; for
- * grad-input alone (`data`) where that one has none. */
-static bool deform_by_rows(const Geom& g, int dtype, bool data) {
-  if (dtype != DK_F16) return dtype == DK_F32;
-  return deform_data_mma_workspace(g) == 0 &&
-         (data || (deform_coords_mma_workspace(g) == 0 && deform_filter_mma_workspace(g) == 0));
-}
-
 /* First region of the fused backward's workspace: used by grad-input, then (same stream) by the offset gradients. */
 static size_t deform_front_ws(const dk_geom* g, int dtype) {
   size_t need = dk_deform_sample_depthwise_backward_data_workspace_bytes(g, dtype);
@@ -411,6 +432,18 @@ int dk_deform_sample_depthwise_backward(const void* grad_output, const void* inp
   int rc = DK_OK;
   if (!rotation) {  // zero kernel-space offsets (see the forward); nothing to differentiate with respect to them
     if (grad_rotation) return DK_ERR_BAD_ARGUMENT;
+    if (deform_by_rows(gg, dtype, false)) {
+      if (grad_filter && (gg.scH > 4 || gg.scW > 4)) return DK_ERR_UNSUPPORTED;  // that kernel wants a tensor of zeros
+      bool bank_done = false;
+      const size_t room = workspace && workspace_bytes >= data_ws ? data_ws : 0;
+      return dtype == DK_F16
+                 ? deform_backward_rows<__half>(P_(__half, grad_output), P_(__half, input), P_(__half, offset), nullptr,
+                                                P_(__half, filter), M_(__half, grad_input), M_(__half, grad_offset), nullptr,
+                                                M_(__half, grad_filter), gg, workspace, room, (cudaStream_t)stream, &bank_done)
+                 : deform_backward_rows<float>(P_(float, grad_output), P_(float, input), P_(float, offset), nullptr,
+                                               P_(float, filter), M_(float, grad_input), M_(float, grad_offset), nullptr,
+                                               M_(float, grad_filter), gg, workspace, room, (cudaStream_t)stream, &bank_done);
+    }
     if (dtype != DK_F16 || !mma_path_enabled()) return DK_ERR_UNSUPPORTED;
     if (!workspace || workspace_bytes < data_ws + filt_ws) return DK_ERR_WORKSPACE;
     cudaStream_t s = (cudaStream_t)stream;

@@ -224,6 +224,9 @@ int tc_error_status();
 int local_rot_f32(const float* dy, const float* x, const float* rot, const float* w, float* drot, const Geom& g, cudaStream_t s);
 size_t local_filter_f32_workspace(const Geom& g);
 size_t deform_data_mma_workspace(const Geom& g);
+size_t deform_forward_rows_workspace(const Geom& g, size_t elem);
+template <typename T>
+int deform_forward_rows(const T* x, const T* off, const T* rot, const T* w, T* y, const Geom& g, void* ws, size_t ws_bytes, cudaStream_t s);
 size_t deform_rows_workspace(const Geom& g, size_t elem);
 template <typename T>
 int deform_backward_rows(const T* dy, const T* x, const T* off, const T* rot, const T* w, T* dx, T* doff, T* drot, T* dw, const Geom& g,

@@ -35,7 +35,7 @@ struct Rec {
   int4 at;
 };
 
-// where sample (n, tap, p) falls in the image and in the bank: upper left corner (-1 .. last) and the fractions
+// where sample (n, tap, p) falls in the image and in the bank (rot may be null: zeros): upper left corner (-1 .. last) and the fractions
 struct Point {
   int h0, w0, u0, v0;
   float lh, lw, lu, lv;
@@ -48,8 +48,8 @@ __device__ __forceinline__ bool sample_point(int n, int tap, int p, const T* __r
   const size_t o = ((size_t)n * g.taps + tap) * 2 * g.P + p;
   const float ph = (float)(oh * g.sH - g.pH + fh * g.dH) + ld<float>(off + o);
   const float pw = (float)(ow * g.sW - g.pW + fw * g.dW) + ld<float>(off + o + g.P);
-  const float u = ((float)fh + ld<float>(rot + o)) + (float)(g.scH - g.kH) * 0.5f;
-  const float v = ((float)fw + ld<float>(rot + o + g.P)) + (float)(g.scW - g.kW) * 0.5f;
+  const float u = ((float)fh + (rot ? ld<float>(rot + o) : 0.f)) + (float)(g.scH - g.kH) * 0.5f;
+  const float v = ((float)fw + (rot ? ld<float>(rot + o + g.P) : 0.f)) + (float)(g.scW - g.kW) * 0.5f;
   // written so that NaN fails; what passes is in range for the conversions below
   if (!(ph > -1.f && pw > -1.f && ph < (float)g.H && pw < (float)g.W)) return false;
   if (!(u > -1.f && v > -1.f && u < (float)g.scH && v < (float)g.scW)) return false;
@@ -115,7 +115,7 @@ __global__ void __launch_bounds__(kSortThreads, 2) dcn_bins_kernel(const T* __re
   __shared__ float tile[kMovePixels * 33];
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int n = blockIdx.x / kSortBlocks, rank = blockIdx.x - n * kSortBlocks;
-  move_channels(dy, dyt, g.P, g, t, tile);
+  if (dyt != nullptr) move_channels(dy, dyt, g.P, g, t, tile);
   if (xt != nullptr) {
     move_channels(x, xt, g.HW, g, t, tile);
     const int cells = (g.scH + 2) * (g.scW + 2);
@@ -377,6 +377,66 @@ __device__ __forceinline__ void tap_record(int flat, int total, int tap, const T
   *to = r;
 }
 
+// Forward: a block takes 32 pixels and all their taps, a warp four of the pixels, two at a time; results pass through shared memory so that
+// they are stored along the pixels.  14 multiply-adds per sample and channel.
+constexpr int kForwardTaps = 9;
+
+template <typename T, int V>
+__global__ void __launch_bounds__(32 * kRowWarps, 3) dcn_forward_kernel(const T* __restrict__ xt, const float* __restrict__ bankt,
+                                                                        const T* __restrict__ off, const T* __restrict__ rot,
+                                                                        T* __restrict__ y, const Geom g, const int Cp) {
+  constexpr int CB = 32 * V;
+  __shared__ TapRec recs[kForwardTaps][32];
+  __shared__ float out[CB][33];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, total = g.N * g.P, flat0 = blockIdx.x * 32;
+  for (int i = threadIdx.x; i < g.taps * 32; i += 32 * kRowWarps)
+    tap_record<T, false>(flat0 + (i & 31), total, i >> 5, off, rot, g, Cp, &recs[i >> 5][i & 31]);
+  __syncthreads();
+  const unsigned cell = Cp * sizeof(float), row = (g.scW + 2) * cell;
+  const bool live = flat0 + lane < total;
+  const int n = (flat0 + lane) / g.P, p = flat0 + lane - n * g.P;
+  for (int c0 = blockIdx.y * CB; c0 < Cp; c0 += gridDim.y * CB) {
+    const int c = c0 + V * lane;
+    const unsigned cb = c * (unsigned)sizeof(T), ck = c * (unsigned)sizeof(float);
+#pragma unroll 1
+    for (int j = warp * 4; j < warp * 4 + 4; j += 2) {
+      float acc[2][V] = {};
+#pragma unroll 1
+      for (int tap = 0; tap < g.taps; ++tap) {
+        float x[2][4][V], k[2][4][V];
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+          const TapRec& r = recs[tap][j + h];
+          const int4 idx = r.idx;
+          const unsigned bk = r.at.y + ck;
+          get_at<T, V>(xt, idx.x + cb, x[h][0]), get_at<T, V>(xt, idx.y + cb, x[h][1]), get_at<T, V>(xt, idx.z + cb, x[h][2]), get_at<T, V>(xt, idx.w + cb, x[h][3]);
+          get_at<float, V>(bankt, bk, k[h][0]), get_at<float, V>(bankt, bk + cell, k[h][1]);
+          get_at<float, V>(bankt, bk + row, k[h][2]), get_at<float, V>(bankt, bk + row + cell, k[h][3]);
+        }
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+          const float4 im = recs[tap][j + h].im, b = recs[tap][j + h].a;
+#pragma unroll
+          for (int e = 0; e < V; ++e) {
+            const float xs = im.x * (im.z * x[h][0][e] + im.w * x[h][1][e]) + im.y * (im.z * x[h][2][e] + im.w * x[h][3][e]);
+            acc[h][e] += xs * (b.x * (b.z * k[h][0][e] + b.w * k[h][1][e]) + b.y * (b.z * k[h][2][e] + b.w * k[h][3][e]));
+          }
+        }
+      }
+#pragma unroll
+      for (int h = 0; h < 2; ++h)
+#pragma unroll
+        for (int e = 0; e < V; ++e) out[V * lane + e][j + h] = acc[h][e];
+    }
+    __syncthreads();
+    if (live) {
+      T* to = y + ((size_t)n * g.C + c0) * g.P + p;
+      for (int ch = warp; ch < min(CB, g.C - c0); ch += kRowWarps) st<T, float>(to + (size_t)ch * g.P, out[ch][lane]);
+    }
+    __syncthreads();
+  }
+}
+
 // Both offset gradients.  S warps share the channels of a unit; the sum over the lanes leaves a quarter of the four sums on each.
 // 28 multiplications and additions per sample and channel, nine loads of a line.
 template <typename T, int V, bool ROT>
@@ -588,7 +648,7 @@ static int launch_bins(const T* dy, const T* x, const T* off, const T* rot, cons
   const int rc = enable_smem(dcn_bins_kernel<T>, t.sort_smem);
   if (rc) return rc;
   t.sorted = sort ? g.N : 0;
-  long long tiles = (long long)g.N * (t.Cp / 32) * (g.P / kMovePixels + 1);
+  long long tiles = dyt != nullptr ? (long long)g.N * (t.Cp / 32) * (g.P / kMovePixels + 1) : 0;
   if (xt != nullptr) tiles += (long long)g.N * (t.Cp / 32) * (g.HW / kMovePixels + 1);
   long long clusters = t.sorted + (tiles + kSortBlocks - 1) / kSortBlocks;
   if (clusters > 2 * device_sm_count() / kSortBlocks) clusters = 2 * device_sm_count() / kSortBlocks;
@@ -666,6 +726,37 @@ int deform_backward_rows(const T* dy, const T* x, const T* off, const T* rot, co
   }
   return DK_OK;
 }
+// Forward: x and the bank into channel order, then a lane per channel.  Not where lanes stay empty in a large call, nor where a
+// large x is moved for a quarter as many outputs of few channels.  Lane per pixel -> per channel, us: 16 x 192 of 28 x 28 75 -> 50,
+// 13 x 96 of 80 x 80 270 -> 188, 64 x 384 of 14 x 14 128 -> 98, 1 x 240 of 20 x 20 31 -> 17; 64 x 16 of 28 x 28 39 -> 46; stride
+// 2: 20 x 128 of 56 x 56 80 -> 71, 32 x 72 of 56 x 56 78 -> 90, 8 x 32 of 40 x 40 38 -> 16.
+static bool forward_rows(const Geom& g, size_t elem, BinPlan& t) {
+  if (g.taps > kForwardTaps || !bin_plan(g, elem, t) || !rows_shape(g, t)) return false;
+  return (g.C >= 32 || (long long)g.N * g.P < 16384) && (g.HW <= 2 * g.P || g.C >= 96 || (long long)g.N * g.HW * g.C < (1 << 21));
+}
+size_t deform_forward_rows_workspace(const Geom& g, size_t elem) {
+  BinPlan t;
+  return forward_rows(g, elem, t) ? t.xt_bytes + t.bankt_bytes : 0;
+}
+template <typename T>
+int deform_forward_rows(const T* x, const T* off, const T* rot, const T* w, T* y, const Geom& g, void* ws, size_t ws_bytes, cudaStream_t s) {
+  BinPlan t;
+  if (!forward_rows(g, sizeof(T), t)) return DK_ERR_UNSUPPORTED;
+  if (ws == nullptr || ws_bytes < t.xt_bytes + t.bankt_bytes) return DK_ERR_WORKSPACE;
+  T* xt = reinterpret_cast<T*>(ws);
+  float* bankt = reinterpret_cast<float*>(reinterpret_cast<char*>(ws) + t.xt_bytes);
+  const int rc = launch_bins<T>(nullptr, x, off, rot, w, false, nullptr, nullptr, nullptr, xt, bankt, g, t, s);
+  if (rc) return rc;
+  const int V = t.Cp % 64 == 0 ? 2 : 1, groups = t.Cp / (32 * V), tiles = (g.N * g.P + 31) / 32;
+  int split = (3 * device_sm_count() + tiles - 1) / tiles;  // blocks share the channels until there are three on every SM
+  if (split > groups) split = groups;
+  auto kern = V == 2 ? dcn_forward_kernel<T, 2> : dcn_forward_kernel<T, 1>;
+  kern<<<dim3(tiles, split), 32 * kRowWarps, 0, s>>>(xt, bankt, off, rot, y, g, t.Cp);
+  return check_launch();
+}
+template int deform_forward_rows<float>(const float*, const float*, const float*, const float*, float*, const Geom&, void*, size_t, cudaStream_t);
+template int deform_forward_rows<__half>(const __half*, const __half*, const __half*, const __half*, __half*, const Geom&, void*, size_t,
+                                         cudaStream_t);
 template int deform_backward_rows<float>(const float*, const float*, const float*, const float*, const float*, float*, float*, float*, float*,
                                         const Geom&, void*, size_t, cudaStream_t, bool*);
 template int deform_backward_rows<__half>(const __half*, const __half*, const __half*, const __half*, const __half*, __half*, __half*, __half*,

@@ -33,7 +33,8 @@ using torch::autograd::variable_list;
   X(dk_sample_depthwise_forward)                   \
   X(dk_sample_depthwise_backward_workspace_bytes)  \
   X(dk_sample_depthwise_backward)                  \
-  X(dk_deform_sample_depthwise_forward)            \
+  X(dk_deform_sample_depthwise_forward_workspace_bytes) \
+  X(dk_deform_sample_depthwise_forward_ws)         \
   X(dk_deform_sample_depthwise_backward_workspace_bytes) \
   X(dk_deform_sample_depthwise_backward)           \
   X(dk_nd_linear_sample_forward)                   \
@@ -290,8 +291,11 @@ Tensor deform_sample_depthwise(const Tensor& input, const Tensor& offset, const 
     x = input.contiguous(), o = offset.contiguous(), w = weight.contiguous();
     if (rotation.defined()) r = rotation.contiguous();
     out = empty_as(x, out_size);
+    const size_t bytes = lib.dk_deform_sample_depthwise_forward_workspace_bytes(&g, code);
+    Tensor ws = workspace(bytes, x);
     auto call = [&] {
-      return lib.dk_deform_sample_depthwise_forward(cptr(x), cptr(o), cptr(r), cptr(w), mptr(out), &g, code, stream_of(x));
+      return lib.dk_deform_sample_depthwise_forward_ws(cptr(x), cptr(o), cptr(r), cptr(w), mptr(out), &g, code, mptr(ws), bytes,
+                                                       stream_of(x));
     };
     int status = call();
     if (status == DK_ERR_UNSUPPORTED && !r.defined()) {

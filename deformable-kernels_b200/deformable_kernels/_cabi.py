@@ -48,6 +48,8 @@ _PROTOS = {
     "dk_sample_depthwise_backward": (_int, [_vp] * 7 + [_gp, _int, _vp, _sz, _vp]),
     "dk_sample_depthwise_backward_one_pass": (_int, [_vp] * 7 + [_gp, _int, _vp, _sz, _vp]),
     "dk_deform_sample_depthwise_forward": (_int, [_vp] * 5 + [_gp, _int, _vp]),
+    "dk_deform_sample_depthwise_forward_workspace_bytes": (_sz, [_gp, _int]),
+    "dk_deform_sample_depthwise_forward_ws": (_int, [_vp] * 5 + [_gp, _int, _vp, _sz, _vp]),
     "dk_deform_sample_depthwise_backward_data_workspace_bytes": (_sz, [_gp, _int]),
     "dk_deform_sample_depthwise_backward_data": (_int, [_vp] * 5 + [_gp, _int, _vp, _sz, _vp]),
     "dk_deform_sample_depthwise_backward_filter_workspace_bytes": (_sz, [_gp, _int]),

@@ -167,10 +167,18 @@ int dk_sample_depthwise_backward(const void *grad_output, const void *input, con
 /* replaces deformable_sample_depthwise_forward_cuda, csrc/filter_sample_depthwise_cuda.cpp:237-294.
  * `rotation` may be NULL here and in dk_deform_sample_depthwise_backward, meaning zero kernel-space offsets (what
  * DeformKernelConv2d / DeformConv2d pass, modules/deform_kernel.py:276): the sampled kernel is then the same for every
- * pixel and is built once.  Only the fp16 tensor-core path takes NULL; otherwise DK_ERR_UNSUPPORTED is returned and
- * the caller passes a tensor of zeros, as the reference does. */
+ * pixel and is built once.  The fp16 tensor-core path takes NULL, and so do dk_deform_sample_depthwise_forward_ws and the
+ * backward where they use their workspace; otherwise DK_ERR_UNSUPPORTED is returned and the caller passes a tensor of zeros, as
+ * the reference does. */
 int dk_deform_sample_depthwise_forward(const void *input, const void *offset, const void *rotation,
                                        const void *filter, void *output, const dk_geom *g, int dtype, void *stream);
+
+/* The same with scratch memory, in which fp32 (and the fp16 shapes outside the tensor-core path) first brings the input into
+ * channel order; 0 bytes: as without. */
+size_t dk_deform_sample_depthwise_forward_workspace_bytes(const dk_geom *g, int dtype);
+int dk_deform_sample_depthwise_forward_ws(const void *input, const void *offset, const void *rotation, const void *filter,
+                                          void *output, const dk_geom *g, int dtype, void *workspace, size_t workspace_bytes,
+                                          void *stream);
 
 /* replaces deformable_sample_depthwise_backward_data_cuda, csrc/filter_sample_depthwise_cuda.cpp:296-354.
  * For DK_F16 the scatter accumulates in an fp32 workspace of

@@ -1,4 +1,4 @@
-"""DK + DCN gradients where the tensor-core kernels do not apply (fp32; fp16 with channels that are no multiple of
+"""DK + DCN forward and gradients where the tensor-core kernels do not apply (fp32; fp16 with channels that are no multiple of
 16 or planes beyond 56 x 56): remainders of the 32-channel groups, of the 32-pixel tiles and of the bands and pieces of rows,
 single pixels, other strides, paddings and dilations, scopes other than 4 x 4, samples far outside, NaN offsets."""
 import pytest
@@ -24,12 +24,14 @@ def test_gradients(n, c, h, w, stride, pad, dil, scope, dtype):
         case["offset"][0, 0, 0, 0], case["offset"][0, 3, -1, -1], case["offset"][0, 8, 1, 1] = float("nan"), 1e9, -float("inf")
     x, o, r, wt, dy = (case[k].to(dtype).to(DEV) for k in ("input", "offset", "rotation", "weight", "grad_output"))
     leaves = [t.requires_grad_(True) for t in (x, o, r, wt)]
-    got = torch.autograd.grad(deform_sample_depthwise(*leaves, **case["args"]), leaves, dy)
+    y = deform_sample_depthwise(*leaves, **case["args"])
+    got = torch.autograd.grad(y, leaves, dy)
     up = torch.float32 if dtype == torch.float16 else torch.float64
     a = [case[k].to(dtype).to(up) for k in ("grad_output", "input", "offset", "rotation", "weight")]
     want = O.deform_sample_depthwise_backward(*a, **case["args"])
     tol = 2e-3 if dtype == torch.float16 else 1e-5
-    for g, w in zip(got, want):
+    want = (O.deform_sample_depthwise_forward(*a[1:], **case["args"]), *want)
+    for g, w in zip((y.detach(), *got), want):
         assert rel_err(g, w.to(dtype)) < tol
 
 
@@ -44,3 +46,16 @@ def test_subsets_of_the_gradients_agree(dtype):
         args = [t if t is leaf else t.detach() for t in leaves]
         one, = torch.autograd.grad(deform_sample_depthwise(*args, **case["args"]), [leaf], dy)
         assert rel_err(one, full[i]) < (2e-3 if dtype == torch.float16 else 1e-5)
+
+
+@pytest.mark.parametrize("c,scope", [(40, (3, 3)), (24, (6, 5))])
+@pytest.mark.parametrize("dtype", [torch.float32, torch.float16])
+def test_without_kernel_offsets(c, scope, dtype):
+    from deformable_kernels.ops.deform_kernel.functions import deform_sample_depthwise
+    case = make_case(2, c, 12, 9, scope=scope, off_std=1.5, seed=7)
+    x, o, r, wt, dy = (case[k].to(dtype).to(DEV) for k in ("input", "offset", "rotation", "weight", "grad_output"))
+    leaves = [t.requires_grad_(True) for t in (x, o, wt)]
+    a = deform_sample_depthwise(x, o, torch.zeros_like(r), wt, **case["args"])
+    b = deform_sample_depthwise(x, o, None, wt, **case["args"])
+    for p, q in zip((a, *torch.autograd.grad(a, leaves, dy)), (b, *torch.autograd.grad(b, leaves, dy))):
+        assert rel_err(q, p) < (2e-3 if dtype == torch.float16 else 1e-5)
