@@ -301,17 +301,32 @@ int dk_deform_sample_depthwise_forward(const void* input, const void* offset, co
                                        (cudaStream_t)stream))
 }
 
-/* Whether the forward and the fused backward take the kernels with channels on the lanes: where no tensor-core kernel applies; for
- * grad-input alone (`data`) where that one has none. */
-static bool deform_by_rows(const Geom& g, int dtype, bool data) {
+/* Which passes take the kernels with channels on the lanes: fp32, and fp16 where no tensor-core kernel applies, or where those
+ * are the slower ones.  Rows of odd width cost them pixel pairs (fp16, us): forward 40 x 128 of 15 x 17 44 -> 33, 16 x 160 of 45 x 31
+ * 125 -> 95, but 100 x 32 of 13 x 15 24 -> 27, 60 x 960 of 7 x 7 56 -> 72; backward 2 x 96 of 51 x 37 109 -> 81, 10 x 512 of
+ * 19 x 27 248 -> 193, but 9 x 240 of 55 x 55 451 -> 490.  Without kernel-space offsets theirs is the cheaper sampled kernel. */
+static bool deform_no_mma(const Geom& g, int dtype) {
   if (dtype != DK_F16) return dtype == DK_F32;
-  return deform_data_mma_workspace(g) == 0 &&
-         (data || (deform_coords_mma_workspace(g) == 0 && deform_filter_mma_workspace(g) == 0));
+  return deform_data_mma_workspace(g) == 0 && deform_coords_mma_workspace(g) == 0 && deform_filter_mma_workspace(g) == 0;
+}
+static bool odd_rows(const Geom& g, int dtype) { return dtype == DK_F16 && g.sH == 1 && g.sW == 1 && (g.W & 1); }
+static bool deform_rows_forward(const Geom& g, int dtype, bool rotation) {
+  return deform_no_mma(g, dtype) || (rotation && odd_rows(g, dtype) && g.C >= 48 && g.P >= 64);
+}
+static bool deform_rows_all(const Geom& g, int dtype, bool rotation) {
+  return deform_no_mma(g, dtype) || (rotation && odd_rows(g, dtype) && g.C >= 96 && g.HW <= 2000);
+}
+/* Grad-input by gathering sorted samples instead of fixed-point atomics into whole planes: small planes of many channels.  60 x 960
+ * of 7 x 7 182 -> 78, 64 x 320 of 9 x 9 109 -> 79, 32 x 384 of 14 x 14 82 -> 63 (stride 2: 48 -> 39), 16 x 256 of 28 x 28 95 -> 81
+ * (stride 2: 38 -> 42), 100 x 48 of 14 x 14 46 -> 72, 9 x 240 of 55 x 55 171 -> 208. */
+static bool deform_rows_data(const Geom& g, int dtype) {
+  if (dtype != DK_F16) return dtype == DK_F32;
+  return deform_data_mma_workspace(g) == 0 || (g.C >= 128 && g.HW <= (g.sH == 1 && g.sW == 1 ? 1400 : 256));
 }
 
 size_t dk_deform_sample_depthwise_forward_workspace_bytes(const dk_geom* g, int dtype) {
   Geom gg;
-  if (!make_geom(g, &gg) || !deform_by_rows(gg, dtype, false)) return 0;
+  if (!make_geom(g, &gg) || !deform_rows_forward(gg, dtype, true)) return 0;
   return align256(deform_forward_rows_workspace(gg, dtype == DK_F16 ? 2 : 4));
 }
 
@@ -321,7 +336,8 @@ int dk_deform_sample_depthwise_forward_ws(const void* input, const void* offset,
   Geom gg;
   if (!input || !offset || !filter || !output || !make_geom(g, &gg)) return DK_ERR_BAD_ARGUMENT;
   const size_t need = dk_deform_sample_depthwise_forward_workspace_bytes(g, dtype);
-  if (need == 0) return dk_deform_sample_depthwise_forward(input, offset, rotation, filter, output, g, dtype, stream);
+  if (need == 0 || !deform_rows_forward(gg, dtype, rotation != nullptr))
+    return dk_deform_sample_depthwise_forward(input, offset, rotation, filter, output, g, dtype, stream);
   if (!workspace || workspace_bytes < need) return DK_ERR_WORKSPACE;
   if (dtype == DK_F16)
     return deform_forward_rows<__half>(P_(__half, input), P_(__half, offset), P_(__half, rotation), P_(__half, filter),
@@ -402,7 +418,7 @@ static size_t deform_front_ws(const dk_geom* g, int dtype) {
     const size_t c = align256(deform_coords_mma_workspace(gg));
     if (c > need) need = c;
   }
-  if (make_geom(g, &gg) && deform_by_rows(gg, dtype, true)) {
+  if (make_geom(g, &gg) && (deform_rows_data(gg, dtype) || deform_rows_all(gg, dtype, true))) {
     const size_t rows = align256(deform_rows_workspace(gg, dtype == DK_F16 ? 2 : 4));
     if (rows > need) need = rows;
   }
@@ -432,7 +448,7 @@ int dk_deform_sample_depthwise_backward(const void* grad_output, const void* inp
   int rc = DK_OK;
   if (!rotation) {  // zero kernel-space offsets (see the forward); nothing to differentiate with respect to them
     if (grad_rotation) return DK_ERR_BAD_ARGUMENT;
-    if (deform_by_rows(gg, dtype, false)) {
+    if (deform_no_mma(gg, dtype)) {
       if (grad_filter && (gg.scH > 4 || gg.scW > 4)) return DK_ERR_UNSUPPORTED;  // that kernel wants a tensor of zeros
       bool bank_done = false;
       const size_t room = workspace && workspace_bytes >= data_ws ? data_ws : 0;
@@ -447,6 +463,13 @@ int dk_deform_sample_depthwise_backward(const void* grad_output, const void* inp
     if (dtype != DK_F16 || !mma_path_enabled()) return DK_ERR_UNSUPPORTED;
     if (!workspace || workspace_bytes < data_ws + filt_ws) return DK_ERR_WORKSPACE;
     cudaStream_t s = (cudaStream_t)stream;
+    if (grad_input && deform_rows_data(gg, dtype)) {
+      bool none = false;
+      rc = deform_backward_rows<__half>(P_(__half, grad_output), P_(__half, input), P_(__half, offset), nullptr, P_(__half, filter),
+                                        M_(__half, grad_input), nullptr, nullptr, nullptr, gg, workspace, data_ws, s, &none);
+      if (rc != DK_OK && rc != DK_ERR_UNSUPPORTED) return rc;
+      if (rc == DK_OK) grad_input = nullptr;
+    }
     if (grad_input) {
       rc = deform_data_mma(P_(__half, grad_output), P_(__half, offset), nullptr, P_(__half, filter), M_(__half, grad_input),
                            gg, workspace, data_ws, s);
@@ -464,8 +487,8 @@ int dk_deform_sample_depthwise_backward(const void* grad_output, const void* inp
                              gg, (char*)workspace + data_ws, filt_ws, s);
     return rc;
   }
-  if (deform_by_rows(gg, dtype, true)) {
-    const bool all = deform_by_rows(gg, dtype, false);
+  const bool all = deform_rows_all(gg, dtype, true);
+  if (all || deform_rows_data(gg, dtype)) {
     const size_t room = workspace && workspace_bytes >= data_ws ? data_ws : 0;
     bool bank_done = false;
 #define DK_ROWS(T)                                                                                                             \

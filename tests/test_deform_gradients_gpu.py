@@ -1,5 +1,5 @@
 """DK + DCN forward and gradients where the tensor-core kernels do not apply (fp32; fp16 with channels that are no multiple of
-16 or planes beyond 56 x 56): remainders of the 32-channel groups, of the 32-pixel tiles and of the bands and pieces of rows,
+16, planes beyond 56 x 56, rows of odd width, small planes of many channels): remainders of the 32-channel groups, of the 32-pixel tiles and of the bands and pieces of rows,
 single pixels, other strides, paddings and dilations, scopes other than 4 x 4, samples far outside, NaN offsets."""
 import pytest
 import torch
@@ -11,7 +11,8 @@ DEV = "cuda:0"
 
 SHAPES = [
     (1, 1, 1, 1, 1, 1, 1, (4, 4)), (2, 33, 5, 40, 1, 1, 1, (4, 4)), (3, 8, 9, 7, 2, 1, 1, (3, 3)), (1, 72, 33, 35, 1, 2, 2, (2, 4)),
-    (2, 24, 60, 61, 2, 0, 1, (4, 4)), (17, 40, 4, 4, 1, 1, 1, (1, 1)), (1, 8, 3, 120, 1, 1, 1, (6, 5))]
+    (2, 24, 60, 61, 2, 0, 1, (4, 4)), (17, 40, 4, 4, 1, 1, 1, (1, 1)), (1, 8, 3, 120, 1, 1, 1, (6, 5)),
+    (2, 96, 11, 13, 1, 1, 1, (4, 4)), (1, 128, 6, 8, 2, 1, 1, (4, 4))]
 
 
 @pytest.mark.parametrize("n,c,h,w,stride,pad,dil,scope", SHAPES)
@@ -48,7 +49,7 @@ def test_subsets_of_the_gradients_agree(dtype):
         assert rel_err(one, full[i]) < (2e-3 if dtype == torch.float16 else 1e-5)
 
 
-@pytest.mark.parametrize("c,scope", [(40, (3, 3)), (24, (6, 5))])
+@pytest.mark.parametrize("c,scope", [(40, (3, 3)), (24, (6, 5)), (128, (3, 3))])
 @pytest.mark.parametrize("dtype", [torch.float32, torch.float16])
 def test_without_kernel_offsets(c, scope, dtype):
     from deformable_kernels.ops.deform_kernel.functions import deform_sample_depthwise
