@@ -301,27 +301,26 @@ int dk_deform_sample_depthwise_forward(const void* input, const void* offset, co
                                        (cudaStream_t)stream))
 }
 
-/* Which passes take the kernels with channels on the lanes: fp32, and fp16 where no tensor-core kernel applies, or where those
- * are the slower ones.  Rows of odd width cost them pixel pairs (fp16, us): forward 40 x 128 of 15 x 17 44 -> 33, 16 x 160 of 45 x 31
- * 125 -> 95, but 100 x 32 of 13 x 15 24 -> 27, 60 x 960 of 7 x 7 56 -> 72; backward 2 x 96 of 51 x 37 109 -> 81, 10 x 512 of
- * 19 x 27 248 -> 193, but 9 x 240 of 55 x 55 451 -> 490.  Without kernel-space offsets theirs is the cheaper sampled kernel. */
+/* Which passes take the kernels with channels on the lanes: fp32, and fp16 where no tensor-core kernel applies or, forward, where
+ * rows of odd width cost that one its pixel pairs (us: 40 x 128 of 15 x 17 44 -> 33, 16 x 160 of 45 x 31 125 -> 95, but 100 x 32
+ * of 13 x 15 24 -> 27, 60 x 960 of 7 x 7 56 -> 72; without kernel-space offsets its sampled kernel is the cheaper one). */
 static bool deform_no_mma(const Geom& g, int dtype) {
   if (dtype != DK_F16) return dtype == DK_F32;
   return deform_data_mma_workspace(g) == 0 && deform_coords_mma_workspace(g) == 0 && deform_filter_mma_workspace(g) == 0;
 }
-static bool odd_rows(const Geom& g, int dtype) { return dtype == DK_F16 && g.sH == 1 && g.sW == 1 && (g.W & 1); }
 static bool deform_rows_forward(const Geom& g, int dtype, bool rotation) {
-  return deform_no_mma(g, dtype) || (rotation && odd_rows(g, dtype) && g.C >= 48 && g.P >= 64);
+  return deform_no_mma(g, dtype) ||
+         (rotation && dtype == DK_F16 && g.sH == 1 && g.sW == 1 && (g.W & 1) && g.C >= 48 && g.P >= 64);
 }
-static bool deform_rows_all(const Geom& g, int dtype, bool rotation) {
-  return deform_no_mma(g, dtype) || (rotation && odd_rows(g, dtype) && g.C >= 96 && g.HW <= 2000);
-}
-/* Grad-input by gathering sorted samples instead of fixed-point atomics into whole planes: small planes of many channels.  60 x 960
- * of 7 x 7 182 -> 78, 64 x 320 of 9 x 9 109 -> 79, 32 x 384 of 14 x 14 82 -> 63 (stride 2: 48 -> 39), 16 x 256 of 28 x 28 95 -> 81
- * (stride 2: 38 -> 42), 100 x 48 of 14 x 14 46 -> 72, 9 x 240 of 55 x 55 171 -> 208. */
+/* Grad-input, and with it the other gradients unless most lanes would stay empty: the preparation is paid for once (fp16, all
+ * gradients, us: 2 x 96 of 51 x 37 109 -> 81, 4 x 96 of 56 x 56 160 -> 147; 20 x 16 of 41 x 39 97 -> 138).  Where a tensor-core
+ * grad-input exists it stays: its fixed-point sums are the same bits in every run. */
 static bool deform_rows_data(const Geom& g, int dtype) {
   if (dtype != DK_F16) return dtype == DK_F32;
-  return deform_data_mma_workspace(g) == 0 || (g.C >= 128 && g.HW <= (g.sH == 1 && g.sW == 1 ? 1400 : 256));
+  return deform_data_mma_workspace(g) == 0;
+}
+static bool deform_rows_all(const Geom& g, int dtype) {
+  return deform_no_mma(g, dtype) || (deform_rows_data(g, dtype) && g.C >= 32);
 }
 
 size_t dk_deform_sample_depthwise_forward_workspace_bytes(const dk_geom* g, int dtype) {
@@ -418,7 +417,7 @@ static size_t deform_front_ws(const dk_geom* g, int dtype) {
     const size_t c = align256(deform_coords_mma_workspace(gg));
     if (c > need) need = c;
   }
-  if (make_geom(g, &gg) && (deform_rows_data(gg, dtype) || deform_rows_all(gg, dtype, true))) {
+  if (make_geom(g, &gg) && deform_rows_data(gg, dtype)) {
     const size_t rows = align256(deform_rows_workspace(gg, dtype == DK_F16 ? 2 : 4));
     if (rows > need) need = rows;
   }
@@ -448,17 +447,19 @@ int dk_deform_sample_depthwise_backward(const void* grad_output, const void* inp
   int rc = DK_OK;
   if (!rotation) {  // zero kernel-space offsets (see the forward); nothing to differentiate with respect to them
     if (grad_rotation) return DK_ERR_BAD_ARGUMENT;
-    if (deform_no_mma(gg, dtype)) {
+    if (deform_rows_all(gg, dtype)) {
       if (grad_filter && (gg.scH > 4 || gg.scW > 4)) return DK_ERR_UNSUPPORTED;  // that kernel wants a tensor of zeros
       bool bank_done = false;
       const size_t room = workspace && workspace_bytes >= data_ws ? data_ws : 0;
-      return dtype == DK_F16
+      rc = dtype == DK_F16
                  ? deform_backward_rows<__half>(P_(__half, grad_output), P_(__half, input), P_(__half, offset), nullptr,
                                                 P_(__half, filter), M_(__half, grad_input), M_(__half, grad_offset), nullptr,
                                                 M_(__half, grad_filter), gg, workspace, room, (cudaStream_t)stream, &bank_done)
                  : deform_backward_rows<float>(P_(float, grad_output), P_(float, input), P_(float, offset), nullptr,
                                                P_(float, filter), M_(float, grad_input), M_(float, grad_offset), nullptr,
                                                M_(float, grad_filter), gg, workspace, room, (cudaStream_t)stream, &bank_done);
+      if (rc != DK_ERR_UNSUPPORTED) return rc;
+      rc = DK_OK;
     }
     if (dtype != DK_F16 || !mma_path_enabled()) return DK_ERR_UNSUPPORTED;
     if (!workspace || workspace_bytes < data_ws + filt_ws) return DK_ERR_WORKSPACE;
@@ -487,8 +488,8 @@ int dk_deform_sample_depthwise_backward(const void* grad_output, const void* inp
                              gg, (char*)workspace + data_ws, filt_ws, s);
     return rc;
   }
-  const bool all = deform_rows_all(gg, dtype, true);
-  if (all || deform_rows_data(gg, dtype)) {
+  if (deform_rows_data(gg, dtype)) {
+    const bool all = deform_rows_all(gg, dtype);
     const size_t room = workspace && workspace_bytes >= data_ws ? data_ws : 0;
     bool bank_done = false;
 #define DK_ROWS(T)                                                                                                             \

@@ -1,5 +1,5 @@
 """DK + DCN forward and gradients where the tensor-core kernels do not apply (fp32; fp16 with channels that are no multiple of
-16, planes beyond 56 x 56, rows of odd width, small planes of many channels): remainders of the 32-channel groups, of the 32-pixel tiles and of the bands and pieces of rows,
+16, planes beyond 56 x 56, rows of odd width): remainders of the 32-channel groups, of the 32-pixel tiles and of the bands and pieces of rows,
 single pixels, other strides, paddings and dilations, scopes other than 4 x 4, samples far outside, NaN offsets."""
 import pytest
 import torch
