@@ -139,7 +139,12 @@ static int launch_local_conv(const T* src, const T* rot, const T* w, T* dst, con
       // 32 x 32: 45 -> 29 us); against the ring kernels (rows of 112 / 56) up to 96 channels only (C = 96, 112 x 112: 283 ->
       // 253 us, grad-input 300 -> 286; C = 144, 56 x 56, batch 32: 35 -> 40).
       const bool ring_row = g.W == 112 || g.W == 56;
-      if (g.sH == 1 && g.W % 8 == 0 && g.C > 64 && (!ring_row || g.C <= 96)) {
+      // grad-input at stride 2 where TMA fetches the rows of dy, against the gather of the band kernels (nine mma for 2.25 useful):
+      // 32 x 96 of 64 x 64 29 -> 19 us, 64 x 384 of 32 x 32 50 -> 27, 64 x 64 of 48 x 48 27 -> 19; rows of dy of 20 19 -> 25,
+      // odd rows of dx (32 x 96 of 63 x 63) 45 -> 129, 50 x 80 of 16 x 16 10.5 -> 11.3; the ring kernel of 112-wide rows takes half of
+      // its time.
+      const bool dx2 = TRANSPOSED && g.sH == 2 && g.W % 16 == 0 && g.W >= 32 && g.C >= 64 && g.W != 112;
+      if (dx2 || (g.sH == 1 && g.W % 8 == 0 && g.C > 64 && (!ring_row || g.C <= 96))) {
         rc = local_conv_tc<T>(src, rot, w, dst, g, TRANSPOSED, s);
         if (rc != DK_ERR_UNSUPPORTED) return rc;
       }

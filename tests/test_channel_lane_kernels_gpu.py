@@ -1,5 +1,5 @@
 """The local operator with any number of channels, against the CPU oracle: fp32 runs on the tcgen05 kernels (one channel per
-TMEM lane), fp16 on the mma.sync kernels with a partly filled last slab of channels.  The sizes are the edges of their tiles:
+TMEM lane), fp16 there on wide rows, else on the mma.sync kernels with a partly filled last slab of channels.  The sizes are the edges of their tiles:
 32-channel groups (1 to 5 of them, full and partial, so that every
 placement of the remaining groups on the lanes occurs), 8-pixel segments, rows with and without TMA, planes of one row or one
 pixel, steps that span samples, more channels than one block takes."""
@@ -15,6 +15,7 @@ SHAPES = [
     (1, 8, 1, 1), (5, 16, 1, 9), (3, 24, 7, 7), (2, 32, 8, 8), (2, 40, 9, 16), (1, 56, 17, 24), (2, 72, 19, 23),
     (1, 104, 12, 33), (2, 136, 5, 40), (1, 160, 28, 28), (1, 200, 14, 14), (1, 264, 3, 64), (9, 280, 4, 4), (1, 1096, 6, 10),
     (1, 24, 112, 112), (1, 8, 2, 200), (1, 32, 110, 110), (2, 48, 31, 57),
+    (2, 72, 31, 48), (5, 264, 2, 32),
 ]
 
 
