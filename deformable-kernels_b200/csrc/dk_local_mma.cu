@@ -107,9 +107,9 @@ __global__ void __launch_bounds__(448, 2) mma_conv_kernel(const __half* __restri
     const int j = i >> 4, cell = i & 15;
     bank[j * kBankPitch + cell] = (WHOLE || j < cnt) && cell < g.cells ? __ldg(w + (size_t)(c0 + j) * g.cells + cell) : __float2half(0.f);
   }
-  load_band(band, bx, src, n, g.C, c0, cnt, Hs, Ws);
+  load_band<S == 1 ? 96 : 72>(band, bx, src, n, g.C, c0, cnt, Hs, Ws);
   if (!WHOLE) zero_absent_channels(band, bx.pitch_c, cnt);
-  load_band(rband, br, rot, n, 18, 0, 18, g.Ho, g.Wo);
+  load_band<S == 1 ? 96 : 72>(rband, br, rot, n, 18, 0, 18, g.Ho, g.Wo);
   cp_async_wait_all();
   __syncthreads();
 
@@ -402,13 +402,13 @@ __global__ void __launch_bounds__(MAXT, MINB) mma_rot_kernel(const __half* __res
     const int cell = i / cnt16, c = i - cell * cnt16;
     bankT[cell * pitchT + c] = cell < g.cells && c < cnt ? __ldg(w + (size_t)(c0 + c) * g.cells + cell) : __float2half(0.f);
   }
-  load_band(xband, bx, x, n, g.C, c0, cnt, g.H, g.W);
+  load_band<S == 1 ? 96 : 0>(xband, bx, x, n, g.C, c0, cnt, g.H, g.W);
   zero_absent_channels(xband, bx.pitch_c, cnt);
   if (!DYD) {
-    load_band(yband, by, dy, n, g.C, c0, cnt, g.Ho, g.Wo);
+    load_band<S == 1 ? 96 : 0>(yband, by, dy, n, g.C, c0, cnt, g.Ho, g.Wo);
     zero_absent_channels(yband, by.pitch_c, cnt);
   }
-  load_band(rband, br, rot, n, 18, 0, 18, g.Ho, g.Wo);
+  load_band<S == 1 ? 96 : 0>(rband, br, rot, n, 18, 0, 18, g.Ho, g.Wo);
   cp_async_wait_all();
   __syncthreads();
 
@@ -692,9 +692,9 @@ __global__ void __launch_bounds__(MAXT, MINB) mma_filter_kernel(const __half* __
     const Band by = make_band(oh0, pl.BH, g.Ho, g.Wo, pl.mode_dy);
     const Band br = make_band(oh0, pl.BH, g.Ho, g.Wo, pl.mode_rot);
     __syncthreads();  // previous unit's readers are done
-    load_band<DYM == 0>(xband, bx, x, n, g.C, c0, cnt, g.H, g.W);
-    if (!DYM) load_band<DYM == 0>(yband, by, dy, n, g.C, c0, cnt, g.Ho, g.Wo);
-    load_band<DYM == 0>(rband, br, rot, n, 18, 0, 18, g.Ho, g.Wo);
+    load_band<DYM == 0 && S == 1 ? 96 : 0>(xband, bx, x, n, g.C, c0, cnt, g.H, g.W);
+    if (!DYM) load_band<DYM == 0 && S == 1 ? 96 : 0>(yband, by, dy, n, g.C, c0, cnt, g.Ho, g.Wo);
+    load_band<DYM == 0 && S == 1 ? 96 : 0>(rband, br, rot, n, 18, 0, 18, g.Ho, g.Wo);
     // DYM == 2: 16 bytes of every channel row of item it_ go to ring slot slot_, one row per lane and step
     auto ring_fill = [&](int it_, int slot_) {
       const int r_ = it_ / NB;
@@ -994,13 +994,13 @@ __global__ void __launch_bounds__(MAXT, MINB) mma_gw_kernel(const __half* __rest
     const Band by = make_band(oh0, pl.BH, g.Ho, g.Wo, pl.mode_dy);
     const Band br = make_band(oh0, pl.BH, g.Ho, g.Wo, pl.mode_rot);
     __syncthreads();  // previous unit's readers are done
-    load_band<false>(xband, bx, x, n, g.C, c0, cnt, g.H, g.W);
+    load_band<0>(xband, bx, x, n, g.C, c0, cnt, g.H, g.W);
     if (!WHOLE) zero_absent_channels(xband, bx.pitch_c, cnt);
     if (!DYD) {
-      load_band<false>(yband, by, dy, n, g.C, c0, cnt, g.Ho, g.Wo);
+      load_band<0>(yband, by, dy, n, g.C, c0, cnt, g.Ho, g.Wo);
       if (!WHOLE) zero_absent_channels(yband, by.pitch_c, cnt);
     }
-    load_band<false>(rband, br, rot, n, 18, 0, 18, g.Ho, g.Wo);
+    load_band<0>(rband, br, rot, n, 18, 0, 18, g.Ho, g.Wo);
     cp_async_wait_all();
     __syncthreads();
     __half* drot_n = drot + (size_t)n * 18 * g.P;

@@ -149,8 +149,8 @@ __device__ __forceinline__ void group_sync(int bar_id, int nt) {
   if (bar_id == 0) __syncthreads();
   else asm volatile("bar.sync %0, %1;\n" ::"r"(bar_id), "r"(nt) : "memory");
 }
-// WIDE: with the warp-per-row copies of odd widths above 64 (kernels short of registers leave them out where they meet no such rows)
-template <bool WIDE>
+// WIDE: odd widths above it are copied a warp per row; 0: none (kernels short of registers, or slower with them)
+template <int WIDE>
 __device__ __forceinline__ void load_band_group(__half* __restrict__ band, const Band& b, const __half* __restrict__ src, int n,
                                                 int C, int c0, int cnt, int Hs, int Ws, int tid, int nt, int bar_id) {
   const int lane = tid & 31, warp = tid >> 5, nwarps = nt >> 5;
@@ -166,10 +166,12 @@ __device__ __forceinline__ void load_band_group(__half* __restrict__ band, const
     group_sync(bar_id, nt);
     const int rows = r_e - r_s;
     const int tasks = cnt * rows;
-    if (WIDE && Ws > 64) {
+    if (WIDE && Ws > WIDE) {
       // 2-byte copies, a warp per (channel, row): neighbours on neighbouring lanes, up to four loads in flight each.  With a row per
       // thread every lane is on a line of its own, but the lines are reused and more loads are in flight: on rows of 31 that is
-      // the faster way (forward 29 against 49 us), on rows of 85 and 101 it is not (121 against 83, 66 against 41 us)
+      // the faster way (forward 29 against 49 us), on rows of 101 it is not (66 against 41 us).  The line, by kernel: 96 at stride 1
+      // (40 x 64 channels, rows of 81, offsets and bank gradients 393 against 470 us, of 111 549 against 450), 72 in the forward at stride 2
+      // (rows of 67 49 / 57, of 79 103 / 74), never in the gradients at stride 2 (rows of 101 280 / 327)
       for (int t = warp; t < tasks; t += nwarps) {
         const int j = t / rows, r = r_s + (t - j * rows);
         const __half* sp = s0 + (size_t)j * plane + (size_t)r * Ws + lane;
@@ -260,7 +262,7 @@ __device__ __forceinline__ void flat_copies(__half* __restrict__ band, int pitch
 // leave lanes idle on the last pass over a row and walk through the channels one after the other.  Same instruction count
 // (measured), 3-4 % less time in the four kernels.
 // Odd row widths, and bands without a row inside the image, go through load_band_group.
-template <bool WIDE>
+template <int WIDE>
 __device__ __forceinline__ void load_band_flat(__half* __restrict__ band, const Band& b, const __half* __restrict__ src, int n,
                                                int C, int c0, int cnt, int Hs, int Ws, int tid, int nt, int bar_id) {
   const int r_s = max(b.row_lo, 0), r_e = min(b.row_lo + b.RB, Hs);
@@ -296,7 +298,7 @@ __device__ __forceinline__ void load_band_flat(__half* __restrict__ band, const 
     }
   }
 }
-template <bool WIDE = true>
+template <int WIDE>
 __device__ __forceinline__ void load_band(__half* __restrict__ band, const Band& b, const __half* __restrict__ src, int n, int C,
                                           int c0, int cnt, int Hs, int Ws) {
   load_band_flat<WIDE>(band, b, src, n, C, c0, cnt, Hs, Ws, threadIdx.x, blockDim.x, 0);
