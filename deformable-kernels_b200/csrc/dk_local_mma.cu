@@ -692,9 +692,9 @@ __global__ void __launch_bounds__(MAXT, MINB) mma_filter_kernel(const __half* __
     const Band by = make_band(oh0, pl.BH, g.Ho, g.Wo, pl.mode_dy);
     const Band br = make_band(oh0, pl.BH, g.Ho, g.Wo, pl.mode_rot);
     __syncthreads();  // previous unit's readers are done
-    load_band<DYM == 0 && S == 1 ? 96 : 0>(xband, bx, x, n, g.C, c0, cnt, g.H, g.W);
-    if (!DYM) load_band<DYM == 0 && S == 1 ? 96 : 0>(yband, by, dy, n, g.C, c0, cnt, g.Ho, g.Wo);
-    load_band<DYM == 0 && S == 1 ? 96 : 0>(rband, br, rot, n, 18, 0, 18, g.Ho, g.Wo);
+    load_band<0>(xband, bx, x, n, g.C, c0, cnt, g.H, g.W);
+    if (!DYM) load_band<0>(yband, by, dy, n, g.C, c0, cnt, g.Ho, g.Wo);
+    load_band<0>(rband, br, rot, n, 18, 0, 18, g.Ho, g.Wo);
     // DYM == 2: 16 bytes of every channel row of item it_ go to ring slot slot_, one row per lane and step
     auto ring_fill = [&](int it_, int slot_) {
       const int r_ = it_ / NB;

@@ -170,8 +170,8 @@ __device__ __forceinline__ void load_band_group(__half* __restrict__ band, const
       // 2-byte copies, a warp per (channel, row): neighbours on neighbouring lanes, up to four loads in flight each.  With a row per
       // thread every lane is on a line of its own, but the lines are reused and more loads are in flight: on rows of 31 that is
       // the faster way (forward 29 against 49 us), on rows of 101 it is not (66 against 41 us).  The line, by kernel: 96 at stride 1
-      // (40 x 64 channels, rows of 81, offsets and bank gradients 393 against 470 us, of 111 549 against 450), 72 in the forward at stride 2
-      // (rows of 67 49 / 57, of 79 103 / 74), never in the gradients at stride 2 (rows of 101 280 / 327)
+      // (40 x 64 channels, rows of 81, offsets and bank gradients 393 against 470 us), 72 in the forward at stride 2
+      // (rows of 67 49 / 57, of 79 103 / 74), never in the bank gradient (its presence costs rows below 96 two percent) nor in the gradients at stride 2 (rows of 101 280 / 327)
       for (int t = warp; t < tasks; t += nwarps) {
         const int j = t / rows, r = r_s + (t - j * rows);
         const __half* sp = s0 + (size_t)j * plane + (size_t)r * Ws + lane;
