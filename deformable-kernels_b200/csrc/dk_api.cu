@@ -145,6 +145,7 @@ const char* dk_version(void) { return "dk_b200 0.1 (sm_100a)"; }
 int dk_local_plan_query(const dk_geom* g, int dtype, int pass, long long* out8) {
   Geom gg;
   if (!out8 || !make_geom(g, &gg)) return DK_ERR_BAD_ARGUMENT;
+  if (pass == 8) return tc_register_query(out8);
   if (dtype != DK_F16 || !mma_path_enabled()) return DK_ERR_UNSUPPORTED;
   if (pass >= 4 && pass <= 7) return local_ring_plan_query(gg, pass, out8);
   return local_mma_plan_query(gg, pass, out8);

@@ -220,6 +220,7 @@ int ring_error_status();
 template <typename T>
 int local_conv_tc(const T* src, const T* rot, const T* w, T* dst, const Geom& g, bool transposed, cudaStream_t s);
 int tc_error_status();
+int tc_register_query(long long out[8]);  // {kernels, fewest registers per thread of any, what the roles' shares need}
 // fp32 gradients towards offsets and bank (dk_local_f32.cu); the bank's leave as *blocks partial sums [block][C][cells]
 int local_rot_f32(const float* dy, const float* x, const float* rot, const float* w, float* drot, const Geom& g, cudaStream_t s);
 size_t local_filter_f32_workspace(const Geom& g);

@@ -28,6 +28,7 @@
 //   4 or 6 store warps results of a step from shared memory, consecutive pixels on consecutive lanes (written straight from
 //                      the consumers' registers, one channel per lane, every store touches 32 lines)
 // Every hand-over is an mbarrier used once per step (or per set of accumulators) by the same warps, in order.
+#include <atomic>
 #include <cstring>
 #include <type_traits>
 
@@ -902,6 +903,39 @@ ConvPlan plan_conv(const Geom& g, const void* src, const void* dst) {
   return pl;
 }
 
+// Registers per thread that a launch of KERN allocates; -1: the query failed.
+template <auto KERN>
+int launch_registers() {
+  cudaFuncAttributes at;
+  const cudaError_t e = cudaFuncGetAttributes(&at, KERN);
+  if (e == cudaSuccess) return at.numRegs;
+  (void)cudaGetLastError();
+  return -1;
+}
+// setmaxnreg.inc waits for registers that the launch did not allocate for ever: a kernel that was compiled to fewer than the
+// roles' shares add up to is not launched.  One answer per kernel (the kernels of a template share a pointer type, so KERN is
+// a template argument); a failed query is not kept.
+template <auto KERN>
+bool shares_fit() {
+  static std::atomic<int> regs{-1};
+  int r = regs.load(std::memory_order_relaxed);
+  if (r < 0) {
+    r = launch_registers<KERN>();
+    regs.store(r, std::memory_order_relaxed);
+  }
+  return r >= kRegsLaunch;
+}
+
+template <typename T, int MODE, bool SC44, int NL>
+int run_conv(const ConvPlan& pl, const CUtensorMap& tm, const T* src, const T* rot, const T* w, T* dst, cudaStream_t s) {
+  constexpr auto kern = tc_conv_kernel<T, MODE, SC44, NL>;
+  if (!shares_fit<kern>()) return DK_ERR_UNSUPPORTED;
+  const int rc = enable_smem(kern, pl.smem);
+  if (rc) return rc;
+  kern<<<dim3(pl.ctas, pl.splits), kThreads, pl.smem, s>>>(tm, src, rot, w, dst, pl.p);
+  return check_launch();
+}
+
 template <typename T, int MODE>
 int launch_conv(const T* src, const T* rot, const T* w, T* dst, const Geom& g, cudaStream_t s) {
   const ConvPlan pl = plan_conv<T, MODE>(g, src, dst);
@@ -911,20 +945,24 @@ int launch_conv(const T* src, const T* rot, const T* w, T* dst, const Geom& g, c
   if (pl.tma && !make_plane_row_map(&tm, src, sizeof(T), pl.p.Ws, pl.p.Hs, (long long)g.N * g.C, pl.p.pitch / (int)sizeof(T), pl.p.box_c))
     return DK_ERR_UNSUPPORTED;
   const bool sc44 = g.scH == 4 && g.scW == 4;
-  auto run = [&](auto kern) {
-    // the roles' register shares add up to what a launch with this many registers allocates, not to less
-    static const bool shares_fit = [&] {
-      cudaFuncAttributes at;
-      return cudaFuncGetAttributes(&at, kern) == cudaSuccess && at.numRegs >= kRegsLaunch;
-    }();
-    if (!shares_fit) return (int)DK_ERR_UNSUPPORTED;
-    const int rc = enable_smem(kern, pl.smem);
-    if (rc) return rc;
-    kern<<<dim3(pl.ctas, pl.splits), kThreads, pl.smem, s>>>(tm, src, rot, w, dst, pl.p);
-    return check_launch();
-  };
-  if (pl.tma) return sc44 ? run(tc_conv_kernel<T, MODE, true, 1>) : run(tc_conv_kernel<T, MODE, false, 1>);
-  return sc44 ? run(tc_conv_kernel<T, MODE, true, kLoaders>) : run(tc_conv_kernel<T, MODE, false, kLoaders>);
+  if (pl.tma) return sc44 ? run_conv<T, MODE, true, 1>(pl, tm, src, rot, w, dst, s) : run_conv<T, MODE, false, 1>(pl, tm, src, rot, w, dst, s);
+  return sc44 ? run_conv<T, MODE, true, kLoaders>(pl, tm, src, rot, w, dst, s) : run_conv<T, MODE, false, kLoaders>(pl, tm, src, rot, w, dst, s);
+}
+
+template <typename T, int MODE, bool SC44, int NL>
+void add_registers(long long out[8]) {
+  const int r = launch_registers<tc_conv_kernel<T, MODE, SC44, NL>>();
+  ++out[0];
+  if (out[1] < 0 || r < out[1]) out[1] = r;
+}
+template <typename T, int MODE>
+void add_registers_of(long long out[8]) {
+  add_registers<T, MODE, true, 1>(out), add_registers<T, MODE, false, 1>(out);
+  add_registers<T, MODE, true, kLoaders>(out), add_registers<T, MODE, false, kLoaders>(out);
+}
+template <typename T>
+void add_registers_of(long long out[8]) {
+  add_registers_of<T, kFwd1>(out), add_registers_of<T, kFwd2>(out), add_registers_of<T, kData1>(out), add_registers_of<T, kData2>(out);
 }
 
 }  // namespace
@@ -937,6 +975,14 @@ int local_conv_tc(const T* src, const T* rot, const T* w, T* dst, const Geom& g,
 }
 template int local_conv_tc<float>(const float*, const float*, const float*, float*, const Geom&, bool, cudaStream_t);
 template int local_conv_tc<__half>(const __half*, const __half*, const __half*, __half*, const Geom&, bool, cudaStream_t);
+
+int tc_register_query(long long out[8]) {
+  for (int i = 0; i < 8; ++i) out[i] = 0;
+  out[1] = -1, out[2] = kRegsLaunch;
+  add_registers_of<float>(out);
+  add_registers_of<__half>(out);
+  return out[1] < 0 ? DK_ERR_CUDA : DK_OK;
+}
 
 int tc_error_status() {
   int v = 0;

@@ -84,7 +84,9 @@ const char *dk_version(void);
  * block, channel groups, warps per block, bands, dynamic shared memory in bytes, blocks in the grid, workspace bytes}.
  * Row-ring kernels, pass: 4 forward, 5 grad-input, 6 grad-offsets + grad-bank, 7 the one-pass backward; out8 = {slots of
  * the source-row ring, slots of the per-output-row rings, warps per block, producer warps among them, channels per block,
- * channel groups, dynamic shared memory in bytes, blocks in the grid}.  DK_ERR_UNSUPPORTED when the geometry or dtype
+ * channel groups, dynamic shared memory in bytes, blocks in the grid}.  Pass 8 (any geometry and dtype, needs a device): the
+ * tcgen05 kernels; out8 = {kernels, fewest registers per thread that any of them is compiled to, registers that their roles'
+ * shares add up to}.  DK_ERR_UNSUPPORTED when the geometry or dtype
  * does not take that family of kernels. */
 int dk_local_plan_query(const dk_geom *g, int dtype, int pass, long long *out8);
 /* The producer / consumer kernels of the fp16 path bound every wait on a shared-memory barrier; a wait that

@@ -61,6 +61,16 @@ def test_offsets_that_sample_nothing():
     assert rel_err(y, want) < 1e-5
 
 
+def test_every_kernel_has_the_registers_of_its_roles():
+    """setmaxnreg moves registers between warps; what the shares add up to has to be there in every instantiation."""
+    import ctypes
+    from deformable_kernels import _cabi as C
+    out = (ctypes.c_longlong * 8)()
+    g = C.geom((1, 16, 8, 8), (3, 3), (1, 1), (1, 1), (1, 1), (4, 4), 1)
+    assert C.lib.dk_local_plan_query(g, C.DK_F32, 8, out) == 0
+    assert out[0] >= 32 and out[1] >= out[2] >= 72
+
+
 def _check(case, dtype):
     from deformable_kernels import _cabi as C
     from deformable_kernels.ops.deform_kernel.functions import sample_depthwise
