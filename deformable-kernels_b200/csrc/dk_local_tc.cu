@@ -13,9 +13,12 @@
 //
 // fp16: K leaves the tensor cores rounded to fp16 (relative 2^-11, like the tensors themselves) and meets x in the
 // mixed-precision multiply-add (exact product, fp32 sum), as in dk_local_ring.cu.
-// fp32: W and the hat products are split into two fp16 pieces each, scaled by powers of two so that no piece is subnormal
-// (W per channel, the hat products by 2^15); the four products of the pieces, summed in fp32, are exact to 2^-23 of the
-// channel's largest bank value, like the four fp32 products and additions it replaces.
+// fp32: W is split into three fp16 pieces and the hat products into two, scaled by powers of two (W per channel, its last piece
+// by 2^15 more; the hat products by 2^15).  The pieces hold W to 24 bits down to 2^-30 of the channel's largest value, below that
+// to 2^-55 of it, and the hat products to 23 bits down to 2^-15, below that to 2^-40.  Five products, the small ones first: the
+// tensor cores truncate each sum, and only the last one is at full size (kUnbias).  Error against fp64, 2-norm, N(0, 1) data, 56 x 56:
+// 1.36e-7, most of it the rounding of the coordinates (four gathered fp32 products and additions before: 1.40e-7; two pieces of W, large
+// products first: 1.94e-7).
 //
 // A block walks through a contiguous range of 8-pixel segments of the destination rows (sample, row, column octet, in
 // memory order) for up to CG channels; 8 segments are a step.  Roles:
@@ -48,9 +51,20 @@ constexpr int kTeams = 4;
 constexpr int kConsumers = 16;
 constexpr int kHelpers = 12;  // MMA, loaders, hat products, stores
 constexpr int kThreads = 32 * (kConsumers + kHelpers);
-// registers: 72 per thread at launch, then 88 for the four consumer warpgroups and 48 for the three of the helpers
-constexpr int kRegsLaunch = 72, kRegsConsumer = 88, kRegsHelper = 48;
-static_assert(kConsumers * kRegsConsumer + kHelpers * kRegsHelper <= (kConsumers + kHelpers) * kRegsLaunch, "register shares");
+// Registers per thread: 72 at launch, then more for the four consumer warpgroups than for the three of the helpers.  fp16 consumers
+// hold two items; fp32 ones hold one, and the hat products need what that leaves.
+constexpr int kRegsLaunch = 72;
+template <typename T>
+__host__ __device__ constexpr int consumer_regs() {
+  return sizeof(T) == 2 ? 88 : 80;
+}
+template <typename T>
+__host__ __device__ constexpr int helper_regs() {
+  return sizeof(T) == 2 ? 48 : 56;
+}
+template <typename T>
+constexpr bool kSharesAdd = kConsumers * consumer_regs<T>() + kHelpers * helper_regs<T>() <= (kConsumers + kHelpers) * kRegsLaunch;
+static_assert(kSharesAdd<float> && kSharesAdd<__half>, "register shares");
 constexpr int kLoaders = 3;                         // warps that fetch rows without TMA
 constexpr int kStepSegs = 8;
 constexpr int kSlotCols = 48;                       // three taps x 16 pixels
@@ -68,6 +82,11 @@ constexpr int kMinSmem = 120 * 1024;                // one block per SM: it take
 template <typename T>
 __host__ __device__ constexpr int beta_warps(int loaders) {
   return loaders == 1 && sizeof(T) == 2 ? 6 : 4;
+}
+
+template <typename T>
+__host__ __device__ constexpr int bank_piece_count() {
+  return sizeof(T) == 2 ? 1 : 3;
 }
 
 enum Mode { kFwd1 = 0, kFwd2 = 1, kData1 = 2, kData2 = 3 };  // forward, grad-input; stride 1, 2
@@ -217,34 +236,47 @@ __device__ __forceinline__ int rest_index(int rest, int v, int q) {
   return q == v ? -1 : q - (q > v);
 }
 
-// the 16 cells of one channel as fp16 pieces: hi[8], lo[8] (two cells each); `inv` undoes the scaling of fp32 banks and of
-// the hat products they meet
+// The tensor cores truncate a sum to 24 bits: 1/2 of the last place too low on average, 2^-24 / 1.44 of the value over a binade.
+// Banks are larger by that much; the truncation takes it off again (a sum of one term comes out exact: less than one place was added).
+constexpr float kUnbias = 4.1e-8f;
+
+// The 16 cells of one channel into the columns at `a` as fp16 pieces of 8 columns (two cells each): the values, or for fp32 their
+// upper and lower parts and, scaled by 2^15, what those leave.  Returns what undoes the scaling of fp32 banks and of the hat
+// products they meet.
 template <typename T>
-__device__ __forceinline__ void bank_pieces(unsigned (&hi)[8], unsigned (&lo)[8], float& inv, const T* __restrict__ w, int cells,
-                                            bool ok) {
-  float v[16];
+__device__ __forceinline__ float bank_to_tmem(unsigned a, const T* __restrict__ w, int cells, bool ok) {
+  float v[16], inv = 1.f;
 #pragma unroll
   for (int i = 0; i < 16; ++i) v[i] = ok && i < cells ? ld<float>(w + i) : 0.f;
-  if constexpr (std::is_same<T, __half>::value) {
-#pragma unroll
-    for (int i = 0; i < 8; ++i) hi[i] = mma::pack2(v[2 * i], v[2 * i + 1]), lo[i] = 0;
-    inv = 1.f;
-  } else {
+  if constexpr (std::is_same<T, float>::value) {
     float top = 0.f;
 #pragma unroll
     for (int i = 0; i < 16; ++i) top = fmaxf(top, fabsf(v[i]));
     int e = 0;
     if (top > 0.f && top < INFINITY) frexpf(top, &e);
-    const int shift = min(15 - e, 100);  // largest magnitude in [2^14, 2^15)
+    const int shift = min(15 - e, 111);  // largest magnitude in [2^14, 2^15), or less where `inv` would be subnormal
     const float sc = ldexpf(1.f, shift);
     inv = ldexpf(1.f, -15 - shift);
 #pragma unroll
-    for (int i = 0; i < 8; ++i) {
-      const float a = v[2 * i] * sc, b = v[2 * i + 1] * sc;
-      hi[i] = mma::pack2(a, b);
-      lo[i] = mma::pack2(a - mma::lo2f(hi[i]), b - mma::hi2f(hi[i]));
-    }
+    for (int i = 0; i < 16; ++i) v[i] *= sc;
   }
+  unsigned top_part[8];
+#pragma unroll
+  for (int piece = 0; piece < bank_piece_count<T>(); ++piece) {
+    unsigned r[8];
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+      if (piece == 2) {
+        v[2 * i] = 32768.f * fmaf(kUnbias, mma::lo2f(top_part[i]), v[2 * i]);
+        v[2 * i + 1] = 32768.f * fmaf(kUnbias, mma::hi2f(top_part[i]), v[2 * i + 1]);
+      }
+      r[i] = mma::pack2(v[2 * i], v[2 * i + 1]);
+      if (piece == 0) top_part[i] = r[i];
+      v[2 * i] -= mma::lo2f(r[i]), v[2 * i + 1] -= mma::hi2f(r[i]);
+    }
+    st8(a + 8 * piece, r);
+  }
+  return inv;
 }
 
 // ------------------------------------------------------------------ hat products
@@ -260,37 +292,34 @@ __device__ __forceinline__ void tap_of(int v, int t, int g, int x, int& qh, int&
   }
 }
 
-// 16 hat products of one tap: cells (2i, 2i + 1) in hi[i] (and, scaled by 2^15, the rest in lo[i] for fp32)
+// 16 hat products of one tap: cells (2i, 2i + 1) in hi[i].  SPLIT (fp32): scaled by 2^15, and what hi leaves of the unrounded
+// products in lo[i].  (Scalar instructions: packed pairs have to be moved into place, the forward of N = 64, C = 144, 56 x 56 took 170 us with them, 156 without.)
 template <bool SC44, bool SPLIT>
 __device__ __forceinline__ void hat_products(unsigned (&hi)[8], unsigned (&lo)[8], float u, float v, bool ok, int scW, int cells) {
-  float b[16];
+  constexpr float kScale = SPLIT ? 32768.f : 1.f;
+  float hv4[4];
   if (SC44) {
-    float hu[4], hv[4];
 #pragma unroll
-    for (int a = 0; a < 4; ++a) {
-      hu[a] = ok ? hat(u - (float)a) : 0.f;
-      hv[a] = hat(v - (float)a);
-      if (SPLIT) hu[a] *= 32768.f;
-    }
-    const uint64_t v01 = pack_f2(hv[0], hv[1]), v23 = pack_f2(hv[2], hv[3]);
-#pragma unroll
-    for (int a = 0; a < 4; ++a) {
-      const uint64_t uu = pack_f2(hu[a], hu[a]);
-      const float2 r = unpack_f2(mul2(uu, v01)), q = unpack_f2(mul2(uu, v23));
-      b[4 * a] = r.x, b[4 * a + 1] = r.y, b[4 * a + 2] = q.x, b[4 * a + 3] = q.y;
-    }
-  } else {
-    int a = 0, c = 0;
-#pragma unroll
-    for (int i = 0; i < 16; ++i) {
-      b[i] = ok && i < cells ? hat(u - (float)a) * hat(v - (float)c) * (SPLIT ? 32768.f : 1.f) : 0.f;
-      if (++c == scW) c = 0, ++a;
-    }
+    for (int a = 0; a < 4; ++a) hv4[a] = hat(v - (float)a);
   }
+  float hu4 = 0.f;
+  int a = 0, c = 0;
 #pragma unroll
   for (int i = 0; i < 8; ++i) {
-    hi[i] = mma::pack2(b[2 * i], b[2 * i + 1]);
-    if (SPLIT) lo[i] = mma::pack2(b[2 * i] - mma::lo2f(hi[i]), b[2 * i + 1] - mma::hi2f(hi[i]));
+    float hu[2], hv[2];
+    if (SC44) {
+      if (i % 2 == 0) hu4 = ok ? kScale * hat(u - (float)(i / 2)) : 0.f;
+      hu[0] = hu[1] = hu4, hv[0] = hv4[2 * i % 4], hv[1] = hv4[2 * i % 4 + 1];
+    } else {
+#pragma unroll
+      for (int k = 0; k < 2; ++k) {
+        hu[k] = ok && 2 * i + k < cells ? kScale * hat(u - (float)a) : 0.f;
+        hv[k] = hat(v - (float)c);
+        if (++c == scW) c = 0, ++a;
+      }
+    }
+    hi[i] = mma::pack2(hu[0] * hv[0], hu[1] * hv[1]);
+    if (SPLIT) lo[i] = mma::pack2(fmaf(hu[0], hv[0], -mma::lo2f(hi[i])), fmaf(hu[1], hv[1], -mma::hi2f(hi[i])));
   }
 }
 
@@ -336,8 +365,8 @@ __device__ __forceinline__ void write_hats(unsigned buf, const Offsets<T>& o, in
   for (int i = 0; i < 9; ++i) {
     int qh, qw, fh, fw;
     tap_of<MODE>(i / 3, i % 3, 0, 0, qh, qw, fh, fw);
-    // same association as the reference: (tap index + offset) + (scope - kernel) / 2
-    const float u = ((float)fh + static_cast<float>(o.r[i][0])) + p.uh0, w = ((float)fw + static_cast<float>(o.r[i][1])) + p.uw0;
+    // one rounding: tap + (scope - kernel) / 2 is exact
+    const float u = static_cast<float>(o.r[i][0]) + ((float)fh + p.uh0), w = static_cast<float>(o.r[i][1]) + ((float)fw + p.uw0);
     unsigned hi[8], lo[8];
     hat_products<SC44, SPLIT>(hi, lo, u, w, (o.ok >> i) & 1, p.scW, p.cells);
     const unsigned a = dst + (i / 3) * (kTeams * kPairRow) + (i % 3) * 256;
@@ -399,6 +428,21 @@ __device__ __forceinline__ void copy_row(char* slot, const T* __restrict__ src, 
 }
 
 // ------------------------------------------------------------------ forward and grad-input
+// d = bank at a (its pieces 8 columns apart) * hat products at b (kPiece apart), the smallest products first
+template <typename T>
+__device__ __forceinline__ void products(unsigned d, unsigned a, uint64_t b, unsigned idesc) {
+  if constexpr (sizeof(T) == 4) {
+    const uint64_t b_lo = b + (kPiece >> 4);
+    mma_ts(d, a + 16, b, idesc, false);
+    mma_ts_scaled<15>(d, a + 8, b_lo, idesc);
+    mma_ts(d, a + 8, b, idesc, true);
+    mma_ts(d, a, b_lo, idesc, true);
+    mma_ts(d, a, b, idesc, true);
+  } else {
+    mma_ts(d, a, b, idesc, false);
+  }
+}
+
 // staged results: [channel][64 pixels], an odd number of 16-byte units per channel (lanes = channels write 16 bytes each)
 template <typename T> __host__ __device__ constexpr int out_pitch() { return kStepSegs * 8 * (int)sizeof(T) + 16; }
 
@@ -425,7 +469,7 @@ __global__ void __launch_bounds__(kThreads, 1)
   extern __shared__ __align__(1024) char smem[];
   using Wk = Walk<MODE>;
   constexpr bool SPLIT = std::is_same<T, float>::value, STAGED = MODE != kData2;
-  constexpr int PIECES = SPLIT ? 2 : 1, E = sizeof(T);
+  constexpr int PIECES = SPLIT ? 2 : 1, E = sizeof(T), TILE = 8 * bank_piece_count<T>();  // columns of 128 channels' bank
   constexpr int NB = beta_warps<T>(NL), NBUF = NB / 2, NS = kHelpers - 1 - NL - NB;
   constexpr int kOutPitch = out_pitch<T>();
   const int warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0), lane = threadIdx.x & 31;
@@ -488,15 +532,9 @@ __global__ void __launch_bounds__(kThreads, 1)
       }
       const int ch = grp * 32 + lane;
       const bool ok = grp >= 0 && ch < cg;
-      unsigned h[8], l[8];
-      float inv;
-      bank_pieces<T>(h, l, inv, bank + (size_t)(c0 + (ok ? ch : 0)) * p.cells, p.cells, ok);
-      const unsigned a = tmem + ((unsigned)(q * 32) << 16) + kBankCol + i * 8 * PIECES;
-      st8(a, h);
-      if (SPLIT) {
-        st8(a + 8, l);
-        if (grp >= 0) inv_s[grp * 32 + lane] = inv;
-      }
+      const float inv = bank_to_tmem<T>(tmem + ((unsigned)(q * 32) << 16) + kBankCol + i * TILE, bank + (size_t)(c0 + (ok ? ch : 0)) * p.cells,
+                                        p.cells, ok);
+      if (SPLIT && grp >= 0) inv_s[grp * 32 + lane] = inv;
     }
     wait_st();
   }
@@ -506,7 +544,7 @@ __global__ void __launch_bounds__(kThreads, 1)
 
   if (warp < kConsumers) {
     // ================================================================ consumers
-    regs_inc<kRegsConsumer>();
+    regs_inc<consumer_regs<T>()>();
     const int q = warp & 3, team = warp >> 2;
     const unsigned lanes = (unsigned)(q * 32) << 16;
     const bool vec = p.store == 16;
@@ -630,7 +668,7 @@ __global__ void __launch_bounds__(kThreads, 1)
     }
   } else if (warp == kConsumers) {
     // ================================================================ MMA
-    regs_dec<kRegsHelper>();
+    regs_dec<helper_regs<T>()>();
     constexpr unsigned idesc_all = idesc_f16(128, kSetCols, false, false, SPLIT), idesc_pair = idesc_f16(128, kSlotCols, false, false, SPLIT);
     int use = 0;
     bool ok = true;
@@ -651,24 +689,11 @@ __global__ void __launch_bounds__(kThreads, 1)
           const uint64_t b = sdesc(buf + v * (kTeams * kPairRow), 128, 256);
           if (elect_one()) {
             if (rd < p.full) {
-              const unsigned a = tmem + kBankCol + rd * 8 * PIECES;
-              mma_ts(d, a, b, idesc_all, false);
-              if (SPLIT) {
-                mma_ts(d, a, b + (kPiece >> 4), idesc_all, true);
-                mma_ts(d, a + 8, b, idesc_all, true);
-                mma_ts(d, a + 8, b + (kPiece >> 4), idesc_all, true);
-              }
+              products<T>(d, tmem + kBankCol + rd * TILE, b, idesc_all);
             } else {  // the remaining groups sit on other lanes for every pair
 #pragma unroll
               for (int j = 0; j < kTeams; ++j) {
-                const unsigned a = tmem + kBankCol + (p.full + ((j + s) & 3)) * 8 * PIECES, dj = d + j * kSlotCols;
-                const uint64_t bj = b + j * (kPairRow >> 4);
-                mma_ts(dj, a, bj, idesc_pair, false);
-                if (SPLIT) {
-                  mma_ts(dj, a, bj + (kPiece >> 4), idesc_pair, true);
-                  mma_ts(dj, a + 8, bj, idesc_pair, true);
-                  mma_ts(dj, a + 8, bj + (kPiece >> 4), idesc_pair, true);
-                }
+                products<T>(d + j * kSlotCols, tmem + kBankCol + (p.full + ((j + s) & 3)) * TILE, b + j * (kPairRow >> 4), idesc_pair);
               }
             }
             commit(t_full + 8 * set);
@@ -682,7 +707,7 @@ __global__ void __launch_bounds__(kThreads, 1)
     }
   } else if (warp <= kConsumers + NL) {
     // ================================================================ source rows
-    regs_dec<kRegsHelper>();
+    regs_dec<helper_regs<T>()>();
     const int lw = warp - kConsumers - 1;
     int next = 0, done = 0;
     bool ok = true;
@@ -740,7 +765,7 @@ __global__ void __launch_bounds__(kThreads, 1)
     }
   } else if (warp <= kConsumers + NL + NB) {
     // ================================================================ hat products
-    regs_dec<kRegsHelper>();
+    regs_dec<helper_regs<T>()>();
     const int w = warp - kConsumers - 1 - NL, half = w & 1, bi = w >> 1;
     Offsets<T> off;
     if (bi < steps) fetch_offsets<T, MODE>(off, rot, lo + bi * kStepSegs + half * 4, hi, p, lane);
@@ -754,7 +779,7 @@ __global__ void __launch_bounds__(kThreads, 1)
     }
   } else {
     // ================================================================ results to memory
-    regs_dec<kRegsHelper>();
+    regs_dec<helper_regs<T>()>();
     const int w = warp - kConsumers - 1 - NL - NB;
     const size_t plane = (size_t)p.Hd * p.Wd;
     for (int s = 0; s < steps && STAGED; ++s) {
@@ -841,7 +866,7 @@ ConvPlan plan_conv(const Geom& g, const void* src, const void* dst) {
   pl.ok = false;
   ConvParams& p = pl.p;
   constexpr bool kData = MODE == kData1 || MODE == kData2;
-  constexpr int E = sizeof(T), PIECES = E == 4 ? 2 : 1;
+  constexpr int E = sizeof(T);
   p.N = g.N, p.C = g.C, p.Ho = g.Ho, p.Wo = g.Wo;
   p.Hs = kData ? g.Ho : g.H, p.Ws = kData ? g.Wo : g.W;
   p.Hd = kData ? g.H : g.Ho, p.Wd = kData ? g.W : g.Wo;
@@ -874,7 +899,7 @@ ConvPlan plan_conv(const Geom& g, const void* src, const void* dst) {
     const int splits = (groups + per - 1) / per;
     if ((groups + splits - 1) / splits != per || splits > 65535) continue;  // as many blocks with a better balance exist
     const int full = per / 4, rest = per % 4;
-    if ((full + (rest ? 4 : 0)) * 8 * PIECES > 512 - kBankCol) continue;
+    if ((full + (rest ? 4 : 0)) * 8 * bank_piece_count<T>() > 512 - kBankCol) continue;
     int cg = splits == 1 ? (g.C + 7) & ~7 : per * 32;
     const int boxes = (cg + 255) / 256;
     cg = (cg + 8 * boxes - 1) / (8 * boxes) * (8 * boxes);  // boxes start on 128 bytes

@@ -55,6 +55,14 @@ __device__ __forceinline__ void mma_ts(unsigned d, unsigned a, uint64_t b, unsig
       " tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n}\n" ::"r"(d), "r"(a), "l"(b), "r"(idesc), "r"((unsigned)acc)
       : "memory");
 }
+// D[tmem] = D * 2^-SHIFT + A[tmem] * B[smem]
+template <int SHIFT>
+__device__ __forceinline__ void mma_ts_scaled(unsigned d, unsigned a, uint64_t b, unsigned idesc) {
+  asm volatile(
+      "{\n .reg .pred p;\n setp.eq.u32 p, 0, 0;\n"
+      " tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p, %4;\n}\n" ::"r"(d), "r"(a), "l"(b), "r"(idesc), "n"(SHIFT)
+      : "memory");
+}
 
 // ---- TMEM <-> registers: lane l of a warp owns TMEM lane 32 (warp % 4) + l, one register per column
 __device__ __forceinline__ void st8(unsigned a, const unsigned (&r)[8]) {
@@ -104,19 +112,9 @@ __device__ __forceinline__ void wait_ld(unsigned (&r)[24]) {
 template <int N> __device__ __forceinline__ void regs_inc() { asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;\n" ::"n"(N)); }
 template <int N> __device__ __forceinline__ void regs_dec() { asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;\n" ::"n"(N)); }
 
-// ---- packed fp32 pairs
-__device__ __forceinline__ uint64_t pack_f2(float a, float b) {
-  uint64_t r;
-  asm("mov.b64 %0, {%1, %2};\n" : "=l"(r) : "f"(a), "f"(b));
-  return r;
-}
-__device__ __forceinline__ float2 unpack_f2(uint64_t v) {
-  float2 r;
-  asm("mov.b64 {%0, %1}, %2;\n" : "=f"(r.x), "=f"(r.y) : "l"(v));
-  return r;
-}
-__device__ __forceinline__ uint64_t mul2(uint64_t a, uint64_t b) {
-  uint64_t r;
+// ---- packed fp32 pairs (pair, unpair, fma2: dk_common.cuh)
+__device__ __forceinline__ unsigned long long mul2(unsigned long long a, unsigned long long b) {
+  unsigned long long r;
   asm("mul.rn.f32x2 %0, %1, %2;\n" : "=l"(r) : "l"(a), "l"(b));
   return r;
 }

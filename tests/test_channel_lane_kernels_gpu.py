@@ -45,6 +45,54 @@ def test_bank_magnitudes(scale):
     assert float(per.max()) < 1e-5
 
 
+@pytest.mark.parametrize("n,c,h,w,stride", [(2, 64, 28, 28, 1), (2, 144, 30, 37, 2), (3, 960, 7, 7, 1)])
+def test_error_against_fp64(n, c, h, w, stride):
+    """2-norm error of fp32 results.  Forward and grad-input: a coordinate between 1 and 4 is rounded at 2^-24 to 2^-22, which moves a
+    kernel value by 1.3e-7 of its size, the sampled kernel itself is off by 4.5e-8, products and store by 4e-8: 1.4e-7 in all for four
+    gathered fp32 products as for the split ones, here with a tenth more."""
+    from deformable_kernels.ops.deform_kernel.functions import sample_depthwise
+    from oracle import dk_oracle as O
+    case = make_case(n, c, h, w, stride=stride, rot_std=1.0, seed=c)
+    x, r, wt, dy = (case[k].to(DEV) for k in ("input", "rotation", "weight", "grad_output"))
+    x.requires_grad_(True)
+    y = sample_depthwise(x, r, wt, **case["args"])
+    got = (y.detach(),) + torch.autograd.grad(y, [x], dy)
+    a = {k: case[k].double() for k in ("input", "rotation", "weight", "grad_output")}
+    want = (O.sample_depthwise_forward(a["input"], a["rotation"], a["weight"], **case["args"]),)
+    want += tuple(O.sample_depthwise_backward(a["grad_output"], a["input"], a["rotation"], a["weight"], **case["args"])[:1])
+    for name, g, v, bound in zip(("output", "grad_input"), got, want, (1.55e-7, 1.55e-7)):
+        err = float((g.double().cpu() - v).norm() / v.norm())
+        assert err < bound, "%s %.3e (bound %.3e)" % (name, err, bound)
+
+
+@pytest.mark.parametrize("stride", [1, 2])
+def test_wide_range_inside_a_channel(stride):
+    """Cells from 1 down to 2^-40 of the channel's largest, sampled with offsets that are multiples of 1/64 (hat products exact).  The
+    sums of products are truncated five times at 2^-23 and the nine products with the input add ten roundings: 2^-20 of the sum of
+    magnitudes.  The pieces of the bank end at 2^-54 of the largest cell, and products with a hat of zero still take part in the
+    alignment of a sum (2^-53 of it seen): 2^-50 of the largest cell."""
+    from deformable_kernels.ops.deform_kernel.functions import sample_depthwise
+    from oracle import dk_oracle as O
+    case = make_case(2, 40, 13, 21, stride=stride, rot_std=1.0, seed=8)
+    gen = torch.Generator().manual_seed(9)
+    w = case["weight"] * torch.exp2(-40 * torch.rand(case["weight"].shape, generator=gen))
+    r = torch.round(case["rotation"] * 64) / 64
+    r[0] = torch.round(r[0])  # one cell alone
+    x, dy = case["input"], case["grad_output"]
+    xg = x.to(DEV).requires_grad_(True)
+    y = sample_depthwise(xg, r.to(DEV), w.to(DEV), **case["args"])
+    dx, = torch.autograd.grad(y, [xg], dy.to(DEV))
+
+    def both(x, r, w, dy):
+        args = [t.double() for t in (dy, x, r, w)]
+        return O.sample_depthwise_forward(*args[1:], **case["args"]), O.sample_depthwise_backward(*args, **case["args"])[0]
+    flat = w.abs().amax((2, 3), keepdim=True).expand_as(w)
+    for got, want, size, top in zip((y.detach(), dx), both(x, r, w, dy), both(x.abs(), r, w.abs(), dy.abs()),
+                                    both(x.abs(), torch.zeros_like(r), flat, dy.abs())):
+        over = (got.double().cpu() - want).abs() - (2.0 ** -20 * size + 2.0 ** -50 * top)
+        assert float(over.max()) <= 0
+
+
 def test_offsets_that_sample_nothing():
     case = make_case(1, 40, 9, 20, rot_std=1.0, seed=6)
     r = case["rotation"]
