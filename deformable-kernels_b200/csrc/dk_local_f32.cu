@@ -187,8 +187,13 @@ __global__ void __launch_bounds__(32 * kBankWarps, 2) f32_bank_kernel(const floa
 }
 
 // ------------------------------------------------------------------ offsets
-// 12 warps: kernel row x (PQ quads of 32 pixels, 4 / PQ shares of the channels); the shares' sums meet in shared memory.
+// 12 warps: kernel row x (PQ quads of 32 pixels, 4 / PQ shares of the channels).  A sum over L channels in one register is off by
+// about 8.6e-8 sqrt(L / 24) (each addition by up to half a unit of the sum so far).  The eight warps of the general kernel keep L at
+// C / 8 but lose another 1.1e-7 where the coordinate is rounded at its full size.  That part is kept here (`rest`), so chains of
+// C / 8 + 39 channels are as near to fp64; after one, a share contracts what it has and adds up two numbers per tap.  2-norm:
+// C = 960, 7 x 7 general kernel 2.3e-7, this one 2.2e-7, with chains of C / 4 3.0e-7.
 constexpr int kOffWarps = 12;
+constexpr int kChainSlack = 39;
 
 template <int S, int PQ>
 __global__ void __launch_bounds__(32 * kOffWarps, 2) f32_offsets_kernel(const float* __restrict__ dy, const float* __restrict__ x,
@@ -205,10 +210,52 @@ __global__ void __launch_bounds__(32 * kOffWarps, 2) f32_offsets_kernel(const fl
   const int px = t.TH * t.TW;
   const int p = quad * 32 + lane, pc = p < px ? p : 0, r = over(pc, t.TW, t.magic_y), col = pc - r * t.TW;
   const int xo = (r * S + fh) * t.XW + col * S;
+  const int oh = tp.oh0 + r, ow = tp.ow0 + col;
+  const bool live = p < px && oh < g.Ho && ow < g.Wo;
+  const size_t o0 = ((size_t)tp.n * 18 + 6 * fh) * g.P + (live ? oh * g.Wo + ow : 0);
   unsigned long long G2[3][8];  // cells (2i, 2i + 1)
+  float sum[3][2];
 #pragma unroll
   for (int i = 0; i < 24; ++i) G2[i / 8][i % 8] = 0;
-  for (int c0 = 0; c0 < g.C; c0 += 32) {
+#pragma unroll
+  for (int i = 0; i < 6; ++i) sum[i >> 1][i & 1] = 0.f;
+  // sum += G times the floor-based derivative weights of the tap's four cells; the other cells are not read
+  auto contract = [&]() {
+    const float uh0 = 0.5f * (float)(g.scH - 3), uw0 = 0.5f * (float)(g.scW - 3);
+    const int ih = oh * S - 1 + fh;
+#pragma unroll
+    for (int fw = 0; fw < 3; ++fw) {
+      const int iw = ow * S - 1 + fw;
+      const float ru = __ldg(rot + o0 + (size_t)(2 * fw) * g.P), rv = __ldg(rot + o0 + (size_t)(2 * fw + 1) * g.P);
+      const float u = ((float)fh + ru) + uh0, v = ((float)fw + rv) + uw0;
+      if (live && ih >= 0 && ih < g.H && iw >= 0 && iw < g.W && u > -1.f && v > -1.f && u < (float)g.scH && v < (float)g.scW) {
+        const float fu = floorf(u), fv = floorf(v);
+        // tap + shift is a small multiple of 1/2: u minus it is exact, and so is what the rounding of u lost
+        const float lh = (u - fu) + (ru - (u - ((float)fh + uh0))), lw = (v - fv) + (rv - (v - ((float)fw + uw0)));
+        const int a0 = (int)fu, b0 = (int)fv;
+        float gu = 0.f, gv = 0.f;
+#pragma unroll
+        for (int a = 0; a < 4; ++a) {
+          float su = 0.f, sv = 0.f;
+#pragma unroll
+          for (int b = 0; b < 4; ++b) {
+            const float2 two = unpair(G2[fw][2 * a + (b >> 1)]);
+            const float v2 = b & 1 ? two.y : two.x;
+            if (b == b0) su = fmaf(1.f - lw, v2, su), sv -= v2;
+            if (b == b0 + 1) su = fmaf(lw, v2, su), sv += v2;
+          }
+          if (a == a0) gu -= su, gv = fmaf(1.f - lh, sv, gv);
+          if (a == a0 + 1) gu += su, gv = fmaf(lh, sv, gv);
+        }
+        sum[fw][0] += gu, sum[fw][1] += gv;
+      }
+#pragma unroll
+      for (int i = 0; i < 8; ++i) G2[fw][i] = 0;
+    }
+  };
+  const int chunks = (g.C + 31) / 32, per = max((g.C / 8 + kChainSlack) * SH / 32, 1);
+  for (int chunk = 0, left = per; chunk < chunks; ++chunk) {
+    const int c0 = chunk * 32;
     __syncthreads();
     stage_tile<S, kOffWarps>(xs, ys, x, dy, g, t, tp, c0, warp, lane);
     for (int i = threadIdx.x; i < 32 * 16; i += 32 * kOffWarps) {
@@ -239,63 +286,26 @@ __global__ void __launch_bounds__(32 * kOffWarps, 2) f32_offsets_kernel(const fl
         }
       }
     }
+    if (--left == 0 || chunk + 1 == chunks) contract(), left = per;
   }
-  float G[3][16];
-#pragma unroll
-  for (int i = 0; i < 24; ++i) {
-    const float2 v = unpair(G2[i / 8][i % 8]);
-    G[i / 8][2 * (i % 8)] = v.x, G[i / 8][2 * (i % 8) + 1] = v.y;
-  }
-  float* red = smem_f + (size_t)(quad * 3 + fh) * 48 * 32;  // [tap, cell][lane]
-#pragma unroll
-  for (int s = 1; s < SH; ++s) {
+  if (SH > 1) {  // the shares' sums, in order
+    float* red = smem_f + (quad * 3 + fh) * ((SH - 1) * 6 * 32) + lane;  // [share - 1][tap, direction][lane]
     __syncthreads();
-    if (share == s) {
+    if (share > 0) {
 #pragma unroll
-      for (int i = 0; i < 48; ++i) red[i * 32 + lane] = G[i / 16][i % 16];
+      for (int i = 0; i < 6; ++i) red[((share - 1) * 6 + i) * 32] = sum[i >> 1][i & 1];
     }
     __syncthreads();
     if (share == 0) {
 #pragma unroll
-      for (int i = 0; i < 48; ++i) G[i / 16][i % 16] += red[i * 32 + lane];
+      for (int s = 1; s < SH; ++s)
+#pragma unroll
+        for (int i = 0; i < 6; ++i) sum[i >> 1][i & 1] += red[((s - 1) * 6 + i) * 32];
     }
   }
-  const int oh = tp.oh0 + r, ow = tp.ow0 + col;
-  if (share != 0 || p >= px || oh >= g.Ho || ow >= g.Wo) return;
-  const float uh0 = 0.5f * (float)(g.scH - 3), uw0 = 0.5f * (float)(g.scW - 3);
-  const int ih = oh * S - 1 + fh;
+  if (share != 0 || !live) return;
 #pragma unroll
-  for (int fw = 0; fw < 3; ++fw) {
-    const int iw = ow * S - 1 + fw, tap = fh * 3 + fw;
-    const size_t o = ((size_t)tp.n * 18 + 2 * tap) * g.P + oh * g.Wo + ow;
-    const float u = ((float)fh + __ldg(rot + o)) + uh0, v = ((float)fw + __ldg(rot + o + g.P)) + uw0;
-    const bool used = ih >= 0 && ih < g.H && iw >= 0 && iw < g.W && u > -1.f && v > -1.f && u < (float)g.scH && v < (float)g.scW;
-    float gu = 0.f, gv = 0.f;
-    if (used) {
-      const float fu = floorf(u), fv = floorf(v), lh = u - fu, lw = v - fv;
-      const int a0 = (int)fu, b0 = (int)fv;
-      float hv[4], dv[4];
-#pragma unroll
-      for (int b = 0; b < 4; ++b) {
-        hv[b] = b == b0 ? 1.f - lw : (b == b0 + 1 ? lw : 0.f);
-        dv[b] = b == b0 ? -1.f : (b == b0 + 1 ? 1.f : 0.f);
-      }
-#pragma unroll
-      for (int a = 0; a < 4; ++a) {
-        const float hu = a == a0 ? 1.f - lh : (a == a0 + 1 ? lh : 0.f), du = a == a0 ? -1.f : (a == a0 + 1 ? 1.f : 0.f);
-        float su = 0.f, sv = 0.f;
-#pragma unroll
-        for (int b = 0; b < 4; ++b) {
-          su = fmaf(hv[b], G[fw][4 * a + b], su);
-          sv = fmaf(dv[b], G[fw][4 * a + b], sv);
-        }
-        gu = fmaf(du, su, gu);
-        gv = fmaf(hu, sv, gv);
-      }
-    }
-    drot[o] = gu;
-    drot[o + g.P] = gv;
-  }
+  for (int i = 0; i < 6; ++i) drot[o0 + (size_t)i * g.P] = sum[i >> 1][i & 1];
 }
 
 // ------------------------------------------------------------------ bank of DK + DCN
@@ -472,7 +482,7 @@ int local_rot_f32(const float* dy, const float* x, const float* rot, const float
   t = tile_plan(g, 64);
   if (t.tiles < 2 * device_sm_count()) pq = 1, t = tile_plan(g, 32);
   size_t words = 512 + 32 * (size_t)(t.xpitch + t.ypitch);
-  const size_t red = (size_t)pq * 3 * 48 * 32;
+  const size_t red = (size_t)pq * 3 * (4 / pq - 1) * 6 * 32;
   if (words < red) words = red;
   t.smem = words * sizeof(float);
   if (t.smem > (size_t)device_smem_optin()) return DK_ERR_UNSUPPORTED;

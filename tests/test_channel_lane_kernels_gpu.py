@@ -49,18 +49,21 @@ def test_bank_magnitudes(scale):
 def test_error_against_fp64(n, c, h, w, stride):
     """2-norm error of fp32 results.  Forward and grad-input: a coordinate between 1 and 4 is rounded at 2^-24 to 2^-22, which moves a
     kernel value by 1.3e-7 of its size, the sampled kernel itself is off by 4.5e-8, products and store by 4e-8: 1.4e-7 in all for four
-    gathered fp32 products as for the split ones, here with a tenth more."""
+    gathered fp32 products as for the split ones, here with a tenth more.  Offsets: chains of C / 8 + 39 additions at
+    8.6e-8 sqrt(L / 24), beside 8e-8; a tenth more."""
     from deformable_kernels.ops.deform_kernel.functions import sample_depthwise
     from oracle import dk_oracle as O
     case = make_case(n, c, h, w, stride=stride, rot_std=1.0, seed=c)
     x, r, wt, dy = (case[k].to(DEV) for k in ("input", "rotation", "weight", "grad_output"))
-    x.requires_grad_(True)
+    for t in (x, r):
+        t.requires_grad_(True)
     y = sample_depthwise(x, r, wt, **case["args"])
-    got = (y.detach(),) + torch.autograd.grad(y, [x], dy)
+    got = (y.detach(),) + torch.autograd.grad(y, [x, r], dy)
     a = {k: case[k].double() for k in ("input", "rotation", "weight", "grad_output")}
     want = (O.sample_depthwise_forward(a["input"], a["rotation"], a["weight"], **case["args"]),)
-    want += tuple(O.sample_depthwise_backward(a["grad_output"], a["input"], a["rotation"], a["weight"], **case["args"])[:1])
-    for name, g, v, bound in zip(("output", "grad_input"), got, want, (1.55e-7, 1.55e-7)):
+    want += tuple(O.sample_depthwise_backward(a["grad_output"], a["input"], a["rotation"], a["weight"], **case["args"])[:2])
+    chain = 1.1 * ((8e-8) ** 2 + (8.6e-8) ** 2 * (c / 8 + 39) / 24) ** 0.5
+    for name, g, v, bound in zip(("output", "grad_input", "grad_rotation"), got, want, (1.55e-7, 1.55e-7, chain)):
         err = float((g.double().cpu() - v).norm() / v.norm())
         assert err < bound, "%s %.3e (bound %.3e)" % (name, err, bound)
 
