@@ -186,7 +186,7 @@ size_t dk_sample_depthwise_backward_filter_workspace_bytes(const dk_geom* g, int
     const size_t fast = local_filter_mma_workspace(gg);
     if (fast > need) need = fast;
   }
-  if (dtype == DK_F32) {
+  if (dtype != DK_F64) {
     const size_t fast = local_filter_f32_workspace(gg);
     if (fast > need) need = fast;
   }

@@ -216,13 +216,18 @@ bool local_bwd_ring_preferred(const Geom& g);  // the one-pass backward is expec
 int local_bwd_ring(const __half* dy, const __half* x, const __half* rot, const __half* w, __half* dx, __half* drot, __half* dw,
                    const Geom& g, void* ws, size_t ws_bytes, cudaStream_t s);  // all three gradients in one pass
 int ring_error_status();
-// tcgen05 kernels (dk_local_tc.cu), fp16 and fp32; DK_ERR_UNSUPPORTED = shape outside them
+// tcgen05 kernels (dk_local_tc.cu), fp16 and fp32, kernel values in fp32; DK_ERR_UNSUPPORTED = shape outside them
 template <typename T>
 int local_conv_tc(const T* src, const T* rot, const T* w, T* dst, const Geom& g, bool transposed, cudaStream_t s);
+// the same with kernel values rounded to fp16, in place of the mma.sync kernels only
+int local_conv_tc_rounded(const __half* src, const __half* rot, const __half* w, __half* dst, const Geom& g, bool transposed,
+                          cudaStream_t s);
+bool local_conv_mma_takes(const Geom& g, bool transposed);  // the band kernels have a block shape for this call
 int tc_error_status();
 int tc_register_query(long long out[8]);  // {kernels, fewest registers per thread of any, what the roles' shares need}
-// fp32 gradients towards offsets and bank (dk_local_f32.cu); the bank's leave as *blocks partial sums [block][C][cells]
-int local_rot_f32(const float* dy, const float* x, const float* rot, const float* w, float* drot, const Geom& g, cudaStream_t s);
+// gradients towards offsets and bank in fp32 arithmetic (dk_local_f32.cu); the bank's leave as *blocks partial sums [block][C][cells]
+template <typename T>
+int local_rot_f32(const T* dy, const T* x, const T* rot, const T* w, T* drot, const Geom& g, cudaStream_t s);
 size_t local_filter_f32_workspace(const Geom& g);
 size_t deform_data_mma_workspace(const Geom& g);
 size_t deform_forward_rows_workspace(const Geom& g, size_t elem);
@@ -238,7 +243,8 @@ size_t deform_bank_workspace(const Geom& g);
 template <typename T>
 int deform_bank(const T* dy, const T* x, const T* off, const T* rot, float* partial, const Geom& g, size_t ws_bytes, int* blocks,
                 cudaStream_t s);
-int local_filter_f32(const float* dy, const float* x, const float* rot, float* partial, const Geom& g, size_t ws_bytes, int* blocks,
+template <typename T>
+int local_filter_f32(const T* dy, const T* x, const T* rot, float* partial, const Geom& g, size_t ws_bytes, int* blocks,
                      cudaStream_t s);
 size_t local_rot_mma_workspace(const Geom& g);
 int local_rot_mma(const __half* dy, const __half* x, const __half* rot, const __half* w, __half* drot, const Geom& g,

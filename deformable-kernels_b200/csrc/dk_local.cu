@@ -144,8 +144,8 @@ static int launch_local_conv(const T* src, const T* rot, const T* w, T* dst, con
       // odd rows of dx (32 x 96 of 63 x 63) 45 -> 129, 50 x 80 of 16 x 16 10.5 -> 11.3; the ring kernel of 112-wide rows takes half of
       // its time.
       const bool dx2 = TRANSPOSED && g.sH == 2 && g.W % 16 == 0 && g.W >= 32 && g.C >= 64 && g.W != 112;
-      if (dx2 || (g.sH == 1 && g.W % 8 == 0 && g.C > 64 && (!ring_row || g.C <= 96))) {
-        rc = local_conv_tc<T>(src, rot, w, dst, g, TRANSPOSED, s);
+      if ((dx2 || (g.sH == 1 && g.W % 8 == 0 && g.C > 64 && (!ring_row || g.C <= 96))) && local_conv_mma_takes(g, TRANSPOSED)) {
+        rc = local_conv_tc_rounded(src, rot, w, dst, g, TRANSPOSED, s);
         if (rc != DK_ERR_UNSUPPORTED) return rc;
       }
       rc = local_conv_ring(src, rot, w, dst, g, TRANSPOSED, s);
@@ -154,9 +154,14 @@ static int launch_local_conv(const T* src, const T* rot, const T* w, T* dst, con
       if (rc != DK_ERR_UNSUPPORTED) return rc;
     }
   }
-  // fp32, and fp16 with channel counts the mma.sync kernels do not take (no multiple of 16)
+  // fp32, and fp16 with channel counts that are no multiple of 16: those have always been computed with fp32 kernel values.  fp16
+  // where TMA or 8-byte copies of 28 columns and more fetch the rows (us, below -> these: 8 x 72 of 56 x 56 49 -> 16, 32 x 200 of 28 x 28
+  // 104 -> 48, grad-input of 32 x 72 of 56 x 56 at stride 2 127 -> 28; not 64 x 72 of 14 x 14 27 -> 37, 8 x 72 of 75 x 101 100 -> 129,
+  // forward of 32 x 200 of 28 x 28 at stride 2 41 -> 55).
   if constexpr (sizeof(T) <= 4) {
-    if (mma_path_enabled()) {
+    const int Ws = TRANSPOSED ? g.Wo : g.W;
+    const bool rows = sizeof(T) == 4 || Ws % 8 == 0 || (Ws % 4 == 0 && Ws >= 28 && (TRANSPOSED || g.sW == 1));
+    if (rows && mma_path_enabled()) {
       const int rc = local_conv_tc<T>(src, rot, w, dst, g, TRANSPOSED, s);
       if (rc != DK_ERR_UNSUPPORTED) return rc;
     }
@@ -270,8 +275,8 @@ int local_backward_rotation(const T* dy, const T* x, const T* rot, const T* w, T
       if (rc != DK_ERR_UNSUPPORTED) return rc;
     }
   }
-  if constexpr (std::is_same<T, float>::value) {
-    const int rc = local_rot_f32(dy, x, rot, w, drot, g, s);
+  if constexpr (sizeof(T) <= 4) {
+    const int rc = local_rot_f32<T>(dy, x, rot, w, drot, g, s);
     if (rc != DK_ERR_UNSUPPORTED) return rc;
   }
   constexpr int NW = 8;
@@ -704,9 +709,9 @@ int local_backward_filter(const T* dy, const T* x, const T* rot, T* dw, const Ge
       if (rc != DK_ERR_UNSUPPORTED) return rc;
     }
   }
-  if constexpr (std::is_same<T, float>::value) {
+  if constexpr (sizeof(T) <= 4) {
     int blocks = 0;
-    const int rc = local_filter_f32(dy, x, rot, reinterpret_cast<float*>(ws), g, ws_bytes, &blocks, s);
+    const int rc = local_filter_f32<T>(dy, x, rot, reinterpret_cast<float*>(ws), g, ws_bytes, &blocks, s);
     if (rc == DK_OK) {
       const int n_out = g.C * g.cells;
       reduce_partials_kernel<T><<<(n_out + 31) / 32, 256, 0, s>>>(reinterpret_cast<const float*>(ws), dw, n_out, blocks);

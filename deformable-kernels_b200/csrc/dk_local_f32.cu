@@ -1,5 +1,5 @@
-// Offset and bank gradients of the local deformable kernel in fp32, and the bank gradient of DK + DCN where the tensor-core
-// kernels do not apply (3 x 3 taps, scopes up to 4 x 4).
+// Offset and bank gradients of the local deformable kernel in fp32 arithmetic (fp32 tensors, and fp16 where the tensor-core kernels do
+// not apply), and the bank gradient of DK + DCN where those do not apply (3 x 3 taps, scopes up to 4 x 4).
 //
 // Both consume the products dK = dy * x, and both are dense in the 16 bank cells here: with the hat products the sampled
 // cells need no data-dependent addresses, so every bank value and every hat product is one broadcast read for a whole warp.
@@ -77,28 +77,39 @@ __device__ __forceinline__ void copies_done() { asm volatile("cp.async.wait_all;
 // One tile (rows x cols from row r0, column q0 of H x W planes) of 32 planes, the first n_c of which exist, into shared
 // memory; zero outside the planes.  All of a warp's copies are in flight at once, and a lane keeps its place in the tile and
 // walks down the channels: two additions per copy (with the whole address computed for each, the copies were half of all
-// instructions).
-template <int WARPS>
-__device__ __forceinline__ void stage_planes(float* s, const float* __restrict__ g0, int rows, int cols, unsigned magic, int pitch, int r0,
+// instructions).  fp16 planes are widened on the way, through registers.
+template <int WARPS, typename T>
+__device__ __forceinline__ void stage_planes(float* s, const T* __restrict__ g0, int rows, int cols, unsigned magic, int pitch, int r0,
                                              int q0, int H, int W, int n_c, int warp, int lane) {
   const size_t plane = (size_t)H * W;
   const unsigned s0 = (unsigned)__cvta_generic_to_shared(s) + 4u * (unsigned)(warp * pitch);
   const unsigned d_step = 4u * (unsigned)(WARPS * pitch);
+#pragma unroll sizeof(T) == 2 ? 2 : 1
   for (int e = lane; e < rows * cols; e += 32) {
     const int r = over(e, cols, magic), ih = r0 + r, iw = q0 + (e - r * cols);
     const bool in = ih >= 0 && ih < H && iw >= 0 && iw < W;
-    const float* src = g0 + (size_t)warp * plane + (in ? ih * W + iw : 0);
-    unsigned dst = s0 + 4u * e;
+    const T* src = g0 + (size_t)warp * plane + (in ? ih * W + iw : 0);
+    if constexpr (sizeof(T) == 4) {
+      unsigned dst = s0 + 4u * e;
 #pragma unroll
-    for (int ch = 0; ch < 32; ch += WARPS) {
-      if (ch + warp < 32) copy4(dst, src, in && ch + warp < n_c);
-      dst += d_step;
-      src += WARPS * plane;
+      for (int ch = 0; ch < 32; ch += WARPS) {
+        if (ch + warp < 32) copy4(dst, src, in && ch + warp < n_c);
+        dst += d_step;
+        src += WARPS * plane;
+      }
+    } else {
+      constexpr int kEach = (32 + WARPS - 1) / WARPS;
+      float v[kEach];
+#pragma unroll
+      for (int i = 0; i < kEach; ++i) v[i] = in && i * WARPS + warp < n_c ? ld<float>(src + (size_t)(i * WARPS) * plane) : 0.f;
+#pragma unroll
+      for (int i = 0; i < kEach; ++i)
+        if (i * WARPS + warp < 32) s[(i * WARPS + warp) * pitch + e] = v[i];
     }
   }
 }
-template <int S, int WARPS>
-__device__ __forceinline__ void stage_tile(float* xs, float* ys, const float* __restrict__ x, const float* __restrict__ dy, const Geom& g,
+template <int S, int WARPS, typename T>
+__device__ __forceinline__ void stage_tile(float* xs, float* ys, const T* __restrict__ x, const T* __restrict__ dy, const Geom& g,
                                            const TilePlan& t, const TilePos& tp, int c0, int warp, int lane) {
   const int n_c = min(32, g.C - c0);
   stage_planes<WARPS>(xs, x + ((size_t)tp.n * g.C + c0) * g.HW, t.XH, t.XW, t.magic_x, t.xpitch, tp.oh0 * S - 1, tp.ow0 * S - 1, g.H, g.W,
@@ -109,9 +120,9 @@ __device__ __forceinline__ void stage_tile(float* xs, float* ys, const float* __
 // ------------------------------------------------------------------ bank
 constexpr int kBankWarps = 8;
 
-template <int S>
-__global__ void __launch_bounds__(32 * kBankWarps, 2) f32_bank_kernel(const float* __restrict__ dy, const float* __restrict__ x,
-                                                                      const float* __restrict__ rot, float* __restrict__ partial,
+template <typename T, int S>
+__global__ void __launch_bounds__(32 * kBankWarps, 2) f32_bank_kernel(const T* __restrict__ dy, const T* __restrict__ x,
+                                                                      const T* __restrict__ rot, float* __restrict__ partial,
                                                                       const Geom g, const TilePlan t) {
   extern __shared__ __align__(16) float smem_f[];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -133,9 +144,9 @@ __global__ void __launch_bounds__(32 * kBankWarps, 2) f32_bank_kernel(const floa
       const int oh = tp.oh0 + r, ow = tp.ow0 + (p - r * t.TW), fh = tap / 3, fw = tap - fh * 3;
       float u = -8.f, v = -8.f;  // samples nothing
       if (oh < g.Ho && ow < g.Wo) {
-        const float* rp = rot + ((size_t)tp.n * 18 + 2 * tap) * g.P + oh * g.Wo + ow;
-        u = ((float)fh + __ldg(rp)) + uh0;
-        v = ((float)fw + __ldg(rp + g.P)) + uw0;
+        const T* rp = rot + ((size_t)tp.n * 18 + 2 * tap) * g.P + oh * g.Wo + ow;
+        u = ((float)fh + ld<float>(rp)) + uh0;
+        v = ((float)fw + ld<float>(rp + g.P)) + uw0;
       }
       float4 hu, hv;
       hu.x = hat1(u), hu.y = g.scH > 1 ? hat1(u - 1.f) : 0.f, hu.z = g.scH > 2 ? hat1(u - 2.f) : 0.f, hu.w = g.scH > 3 ? hat1(u - 3.f) : 0.f;
@@ -195,10 +206,10 @@ __global__ void __launch_bounds__(32 * kBankWarps, 2) f32_bank_kernel(const floa
 constexpr int kOffWarps = 12;
 constexpr int kChainSlack = 39;
 
-template <int S, int PQ>
-__global__ void __launch_bounds__(32 * kOffWarps, 2) f32_offsets_kernel(const float* __restrict__ dy, const float* __restrict__ x,
-                                                                        const float* __restrict__ rot, const float* __restrict__ w,
-                                                                        float* __restrict__ drot, const Geom g, const TilePlan t) {
+template <typename T, int S, int PQ>
+__global__ void __launch_bounds__(32 * kOffWarps, 2) f32_offsets_kernel(const T* __restrict__ dy, const T* __restrict__ x,
+                                                                        const T* __restrict__ rot, const T* __restrict__ w,
+                                                                        T* __restrict__ drot, const Geom g, const TilePlan t) {
   constexpr int SH = 4 / PQ;
   extern __shared__ __align__(16) float smem_f[];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -226,7 +237,7 @@ __global__ void __launch_bounds__(32 * kOffWarps, 2) f32_offsets_kernel(const fl
 #pragma unroll
     for (int fw = 0; fw < 3; ++fw) {
       const int iw = ow * S - 1 + fw;
-      const float ru = __ldg(rot + o0 + (size_t)(2 * fw) * g.P), rv = __ldg(rot + o0 + (size_t)(2 * fw + 1) * g.P);
+      const float ru = ld<float>(rot + o0 + (size_t)(2 * fw) * g.P), rv = ld<float>(rot + o0 + (size_t)(2 * fw + 1) * g.P);
       const float u = ((float)fh + ru) + uh0, v = ((float)fw + rv) + uw0;
       if (live && ih >= 0 && ih < g.H && iw >= 0 && iw < g.W && u > -1.f && v > -1.f && u < (float)g.scH && v < (float)g.scW) {
         const float fu = floorf(u), fv = floorf(v);
@@ -260,7 +271,7 @@ __global__ void __launch_bounds__(32 * kOffWarps, 2) f32_offsets_kernel(const fl
     stage_tile<S, kOffWarps>(xs, ys, x, dy, g, t, tp, c0, warp, lane);
     for (int i = threadIdx.x; i < 32 * 16; i += 32 * kOffWarps) {
       const int c = c0 + (i >> 4), a = (i >> 2) & 3, b = i & 3;
-      ws[i] = c < g.C && a < g.scH && b < g.scW ? __ldg(w + (size_t)c * g.cells + a * g.scW + b) : 0.f;
+      ws[i] = c < g.C && a < g.scH && b < g.scW ? ld<float>(w + (size_t)c * g.cells + a * g.scW + b) : 0.f;
     }
     copies_done();
     __syncthreads();
@@ -305,7 +316,7 @@ __global__ void __launch_bounds__(32 * kOffWarps, 2) f32_offsets_kernel(const fl
   }
   if (share != 0 || !live) return;
 #pragma unroll
-  for (int i = 0; i < 6; ++i) drot[o0 + (size_t)i * g.P] = sum[i >> 1][i & 1];
+  for (int i = 0; i < 6; ++i) st<T, float>(drot + o0 + (size_t)i * g.P, sum[i >> 1][i & 1]);
 }
 
 // ------------------------------------------------------------------ bank of DK + DCN
@@ -457,13 +468,14 @@ size_t local_filter_f32_workspace(const Geom& g) {
   return f32_shape(g) ? (size_t)bank_plan(g).blocks * g.C * g.cells * sizeof(float) : 0;
 }
 
-int local_filter_f32(const float* dy, const float* x, const float* rot, float* partial, const Geom& g, size_t ws_bytes, int* blocks,
+template <typename T>
+int local_filter_f32(const T* dy, const T* x, const T* rot, float* partial, const Geom& g, size_t ws_bytes, int* blocks,
                      cudaStream_t s) {
   if (!f32_shape(g)) return DK_ERR_UNSUPPORTED;
   const TilePlan t = bank_plan(g);
   if (t.smem > (size_t)device_smem_optin() || (g.C + 31) / 32 > 65535) return DK_ERR_UNSUPPORTED;
   if (partial == nullptr || ws_bytes < (size_t)t.blocks * g.C * g.cells * sizeof(float)) return DK_ERR_WORKSPACE;
-  auto kern = g.sH == 1 ? f32_bank_kernel<1> : f32_bank_kernel<2>;
+  auto kern = g.sH == 1 ? f32_bank_kernel<T, 1> : f32_bank_kernel<T, 2>;
   const int rc = enable_smem(kern, t.smem);
   if (rc) return rc;
   kern<<<dim3(t.blocks, (g.C + 31) / 32), 32 * kBankWarps, t.smem, s>>>(dy, x, rot, partial, g, t);
@@ -471,13 +483,20 @@ int local_filter_f32(const float* dy, const float* x, const float* rot, float* p
   return check_launch();
 }
 
-int local_rot_f32(const float* dy, const float* x, const float* rot, const float* w, float* drot, const Geom& g, cudaStream_t s) {
+template int local_filter_f32<float>(const float*, const float*, const float*, float*, const Geom&, size_t, int*, cudaStream_t);
+template int local_filter_f32<__half>(const __half*, const __half*, const __half*, float*, const Geom&, size_t, int*, cudaStream_t);
+
+template <typename T>
+int local_rot_f32(const T* dy, const T* x, const T* rot, const T* w, T* drot, const Geom& g, cudaStream_t s) {
   if (!f32_shape(g)) return DK_ERR_UNSUPPORTED;
   // Calls with few pixels only: the general kernel (32 pixels per block, gathered cells) leaves SMs without a block there.
   // N = 2, C = 64, 28 x 28: 13.6 -> 10.7 us; N = 32, C = 960, 7 x 7: 109 -> 82.  With the GPU full it is as fast or faster
   // (N = 64, C = 144, 56 x 56: 383 against 392 us, stride 2: 117 against 161).
   TilePlan t = tile_plan(g, 128);
   if (t.tiles >= 2 * device_sm_count()) return DK_ERR_UNSUPPORTED;
+  // fp16: few channels too, its planes pass through registers (2 x 24 of 14 x 14 16.5 -> 12 us, 1 x 40 of 28 x 28 19.5 -> 17; 64 x 936 of
+  // 7 x 7 132 -> 177)
+  if (sizeof(T) == 2 && (g.C > 64 || tile_plan(g, 32).tiles >= device_sm_count())) return DK_ERR_UNSUPPORTED;
   int pq = 2;
   t = tile_plan(g, 64);
   if (t.tiles < 2 * device_sm_count()) pq = 1, t = tile_plan(g, 32);
@@ -486,13 +505,15 @@ int local_rot_f32(const float* dy, const float* x, const float* rot, const float
   if (words < red) words = red;
   t.smem = words * sizeof(float);
   if (t.smem > (size_t)device_smem_optin()) return DK_ERR_UNSUPPORTED;
-  void (*kern)(const float*, const float*, const float*, const float*, float*, const Geom, const TilePlan) =
-      g.sH == 1 ? (pq == 2 ? f32_offsets_kernel<1, 2> : f32_offsets_kernel<1, 1>) : (pq == 2 ? f32_offsets_kernel<2, 2> : f32_offsets_kernel<2, 1>);
+  auto kern = g.sH == 1 ? (pq == 2 ? f32_offsets_kernel<T, 1, 2> : f32_offsets_kernel<T, 1, 1>)
+                        : (pq == 2 ? f32_offsets_kernel<T, 2, 2> : f32_offsets_kernel<T, 2, 1>);
   const int rc = enable_smem(kern, t.smem);
   if (rc) return rc;
   kern<<<t.tiles, 32 * kOffWarps, t.smem, s>>>(dy, x, rot, w, drot, g, t);
   return check_launch();
 }
+template int local_rot_f32<float>(const float*, const float*, const float*, const float*, float*, const Geom&, cudaStream_t);
+template int local_rot_f32<__half>(const __half*, const __half*, const __half*, const __half*, __half*, const Geom&, cudaStream_t);
 
 size_t deform_bank_workspace(const Geom& g) {
   return deform_bank_shape(g) ? (size_t)deform_bank_plan(g).blocks * g.C * g.cells * sizeof(float) : 0;

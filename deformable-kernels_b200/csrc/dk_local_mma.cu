@@ -16,7 +16,7 @@
 // values and five FMAs per (pixel, tap, channel) and is bound by instruction issue.
 //
 // Covers: fp16, 3x3 kernel, dilation 1, pad 1, stride 1 or 2 (equal in h and w), one rotation
-// group, at most 16 bank cells.
+// group, at most 16 bank cells, channels a multiple of 16.
 // Everything else stays on the SIMT kernels of dk_local.cu.
 #include <cstdlib>
 #include <cstring>
@@ -58,15 +58,6 @@ Plan cached_plan(const Geom& g, int tag, F compute) {
 #endif
 }
 
-// Channels are worked on in slabs of 16; the channels of the last slab that do not exist are zeros in shared memory (bands
-// and bank alike, so that they add nothing to sums over channels) and are not stored.  WHOLE: every slab is full; the kernels
-// that use all their registers are compiled for that case on its own (with the tests they spill: 72 -> 78 us on C = 960, 7 x 7).
-__host__ __device__ inline int whole_slabs(int channels) { return (channels + 15) & ~15; }
-__device__ __forceinline__ void zero_absent_channels(__half* band, int pitch, int cnt) {
-  unsigned* z = reinterpret_cast<unsigned*>(band + (size_t)cnt * pitch);
-  for (int i = threadIdx.x; i < (whole_slabs(cnt) - cnt) * pitch / 2; i += blockDim.x) z[i] = 0u;
-}
-
 // ================================================================== forward / grad-input
 struct ConvPlan {
   int BH, CG, groups, warps, bands;
@@ -81,7 +72,7 @@ __host__ __device__ inline int conv_band_rows(int bh, int S, bool transposed) {
   return S == 1 ? bh + 2 : (bh >> 1) + 2;
 }
 
-template <int S, bool TRANSPOSED, bool WHOLE>
+template <int S, bool TRANSPOSED>
 __global__ void __launch_bounds__(448, 2) mma_conv_kernel(const __half* __restrict__ src, const __half* __restrict__ rot,
                                                           const __half* __restrict__ w, __half* __restrict__ dst, const Geom g,
                                                           const ConvPlan pl) {
@@ -103,12 +94,11 @@ __global__ void __launch_bounds__(448, 2) mma_conv_kernel(const __half* __restri
   __half* rband = band + pl.CG * bx.pitch_c;                                 // [18][br.pitch_c]
   __half* bank = rband + 18 * br.pitch_c;                                    // [CG][kBankPitch]
 
-  for (int i = threadIdx.x; i < whole_slabs(cnt) * 16; i += blockDim.x) {
+  for (int i = threadIdx.x; i < cnt * 16; i += blockDim.x) {
     const int j = i >> 4, cell = i & 15;
-    bank[j * kBankPitch + cell] = (WHOLE || j < cnt) && cell < g.cells ? __ldg(w + (size_t)(c0 + j) * g.cells + cell) : __float2half(0.f);
+    bank[j * kBankPitch + cell] = cell < g.cells ? __ldg(w + (size_t)(c0 + j) * g.cells + cell) : __float2half(0.f);
   }
   load_band<S == 1 ? 96 : 72>(band, bx, src, n, g.C, c0, cnt, Hs, Ws);
-  if (!WHOLE) zero_absent_channels(band, bx.pitch_c, cnt);
   load_band<S == 1 ? 96 : 72>(rband, br, rot, n, 18, 0, 18, g.Ho, g.Wo);
   cp_async_wait_all();
   __syncthreads();
@@ -197,18 +187,17 @@ __global__ void __launch_bounds__(448, 2) mma_conv_kernel(const __half* __restri
           fma_win<1 + S + C2, 1>(acc[3], v0, v1, v2, d[2][1]);
         }
       }
-      if (ow < Wd && (WHOLE || cb16 + gq < cnt)) {
+      if (ow < Wd) {
         __half* y1 = y0 + 8 * dplane;
-        const bool both = WHOLE || cb16 + gq + 8 < cnt;
         if (dst_even) {
           *reinterpret_cast<__half2*>(y0) = __floats2half2_rn(acc[0], acc[1]);
-          if (both) *reinterpret_cast<__half2*>(y1) = __floats2half2_rn(acc[2], acc[3]);
+          *reinterpret_cast<__half2*>(y1) = __floats2half2_rn(acc[2], acc[3]);
         } else {
           y0[0] = __float2half_rn(acc[0]);
-          if (both) y1[0] = __float2half_rn(acc[2]);
+          y1[0] = __float2half_rn(acc[2]);
           if (ow + 1 < Wd) {
             y0[1] = __float2half_rn(acc[1]);
-            if (both) y1[1] = __float2half_rn(acc[3]);
+            y1[1] = __float2half_rn(acc[3]);
           }
         }
       }
@@ -223,7 +212,7 @@ constexpr size_t kOnePerSm = 226 * 1024;
 bool fast_shape(const Geom& g) {
   if (g.kH != 3 || g.kW != 3 || g.dH != 1 || g.dW != 1 || g.pH != 1 || g.pW != 1) return false;
   if (g.sH != g.sW || (g.sH != 1 && g.sH != 2)) return false;
-  if (g.G != 1 || g.cells > 16 || g.N > 65535) return false;
+  if (g.G != 1 || g.cells > 16 || (g.C & 15) || g.N > 65535) return false;
   return true;
 }
 
@@ -332,14 +321,16 @@ ConvPlan conv_plan(const Geom& g, bool transposed) {
   return cached_plan<ConvPlan>(g, transposed ? 1 : 0, [&] { return conv_plan_search(g, transposed); });
 }
 
+bool plan_launches(const ConvPlan& pl) { return pl.BH && pl.smem <= (size_t)device_smem_optin() && pl.groups <= 65535; }
+
 template <int S, bool TRANSPOSED>
 int launch_conv(const __half* src, const __half* rot, const __half* w, __half* dst, const Geom& g, cudaStream_t s) {
   ConvPlan pl = conv_plan(g, TRANSPOSED);
-  if (!pl.BH || pl.smem > (size_t)device_smem_optin() || pl.groups > 65535) return DK_ERR_UNSUPPORTED;
+  if (!plan_launches(pl)) return DK_ERR_UNSUPPORTED;
   pl.mode_src = ptr_mode(src);
   pl.mode_rot = ptr_mode(rot);
   pl.pair_store = (((TRANSPOSED ? g.W : g.Wo) & 1) == 0) && ptr_mode(dst) >= 1;
-  auto kern = g.C & 15 ? mma_conv_kernel<S, TRANSPOSED, false> : mma_conv_kernel<S, TRANSPOSED, true>;
+  auto kern = mma_conv_kernel<S, TRANSPOSED>;
   int rc = enable_smem(kern, pl.smem);
   if (rc) return rc;
   kern<<<dim3(pl.bands, pl.groups, g.N), pl.warps * 32, pl.smem, s>>>(src, rot, w, dst, g, pl);
@@ -386,7 +377,7 @@ __global__ void __launch_bounds__(MAXT, MINB) mma_rot_kernel(const __half* __res
   const int n = blockIdx.y;
   const int oh0 = blockIdx.x * pl.BH;
   const int c0 = blockIdx.z * pl.CG;
-  const int cnt = min(pl.CG, g.C - c0), cnt16 = whole_slabs(cnt);
+  const int cnt = min(pl.CG, g.C - c0);
   const Band bx = make_band(oh0 * S - 1, (pl.BH - 1) * S + 3, g.H, g.W, pl.mode_x);
   const Band by = make_band(oh0, pl.BH, g.Ho, g.Wo, pl.mode_dy);
   const Band br = make_band(oh0, pl.BH, g.Ho, g.Wo, pl.mode_rot);
@@ -398,16 +389,12 @@ __global__ void __launch_bounds__(MAXT, MINB) mma_rot_kernel(const __half* __res
   __half* bankT = rband + (size_t)18 * br.pitch_c;                         // [16 cells][CG + 8]
   unsigned char* scratch = reinterpret_cast<unsigned char*>(bankT + 16 * pitchT);
 
-  for (int i = threadIdx.x; i < 16 * cnt16; i += blockDim.x) {
-    const int cell = i / cnt16, c = i - cell * cnt16;
-    bankT[cell * pitchT + c] = cell < g.cells && c < cnt ? __ldg(w + (size_t)(c0 + c) * g.cells + cell) : __float2half(0.f);
+  for (int i = threadIdx.x; i < 16 * cnt; i += blockDim.x) {
+    const int cell = i / cnt, c = i - cell * cnt;
+    bankT[cell * pitchT + c] = cell < g.cells ? __ldg(w + (size_t)(c0 + c) * g.cells + cell) : __float2half(0.f);
   }
   load_band<S == 1 ? 96 : 0>(xband, bx, x, n, g.C, c0, cnt, g.H, g.W);
-  zero_absent_channels(xband, bx.pitch_c, cnt);
-  if (!DYD) {
-    load_band<S == 1 ? 96 : 0>(yband, by, dy, n, g.C, c0, cnt, g.Ho, g.Wo);
-    zero_absent_channels(yband, by.pitch_c, cnt);
-  }
+  if (!DYD) load_band<S == 1 ? 96 : 0>(yband, by, dy, n, g.C, c0, cnt, g.Ho, g.Wo);
   load_band<S == 1 ? 96 : 0>(rband, br, rot, n, 18, 0, 18, g.Ho, g.Wo);
   cp_async_wait_all();
   __syncthreads();
@@ -442,8 +429,8 @@ __global__ void __launch_bounds__(MAXT, MINB) mma_rot_kernel(const __half* __res
     const size_t dstep8 = (size_t)8 * g.P / 2;  // words between channel rows gq and gq + 8
     unsigned ndy0 = 0u, ndy1 = 0u;
     if (DYD && dy_in) {
-      if (gq < cnt) ndy0 = __ldg(dp);
-      if (gq + 8 < cnt) ndy1 = __ldg(dp + dstep8);
+      ndy0 = __ldg(dp);
+      ndy1 = __ldg(dp + dstep8);
     }
     for (int cb16 = 0; cb16 < cnt; cb16 += 16) {
       unsigned dy0, dy1;
@@ -451,8 +438,8 @@ __global__ void __launch_bounds__(MAXT, MINB) mma_rot_kernel(const __half* __res
         dy0 = ndy0;
         dy1 = ndy1;
         if (dy_in && cb16 + 16 < cnt) {
-          ndy0 = cb16 + 16 + gq < cnt ? __ldg(dp + (size_t)(cb16 + 16) / 8 * dstep8) : 0u;
-          ndy1 = cb16 + 24 + gq < cnt ? __ldg(dp + (size_t)(cb16 + 24) / 8 * dstep8) : 0u;
+          ndy0 = __ldg(dp + (size_t)(cb16 + 16) / 8 * dstep8);
+          ndy1 = __ldg(dp + (size_t)(cb16 + 24) / 8 * dstep8);
         }
       } else {
         dy0 = *reinterpret_cast<const unsigned*>(yband + (size_t)(cb16 + gq) * by.pitch_c + yoff);
@@ -557,8 +544,7 @@ RotPlan rot_plan_search(const Geom& g) {
   pl.BH = 0;
   pl.big = false;
   pl.groups = 1;
-  const int channels = whole_slabs(g.C);
-  pl.CG = channels;
+  pl.CG = g.C;
   pl.dy_direct = rot_dy_direct(g);
   // One block of up to 16 warps per SM with a taller band first: the halo rows of x weigh less and a block's load is
   // spread over more items (measured: C = 144 at 56 x 56 0.38 -> 0.22 ms, never slower on the sweep's layers).
@@ -575,7 +561,7 @@ RotPlan rot_plan_search(const Geom& g) {
     int cap = g.Ho;
     if (const char* e = tuning_env("DK_B200_ROT_BH")) cap = atoi(e) > 0 ? atoi(e) : cap;  // tuning knob
     for (int bh = 1; bh <= g.Ho && bh <= cap; ++bh) {
-      if (rot_smem(g, channels, bh, pick_warps(bh * NB, maxw)) > budget) break;
+      if (rot_smem(g, g.C, bh, pick_warps(bh * NB, maxw)) > budget) break;
       tallest = bh;
       if (bh * NB >= 2 * maxw) break;
     }
@@ -584,7 +570,7 @@ RotPlan rot_plan_search(const Geom& g) {
     // Among the bands up to that height: time of a band = fixed part (latency of its loads, barriers) + rows staged
     // + rounds of items over the warps; nothing overlaps in a block that has the SM to itself.  Constants fitted to
     // 28 x 28 ... 112 x 112 planes (band heights 1-14), in instructions per warp.
-    const double t_item = 250.0 + 220.0 * (channels / 16);
+    const double t_item = 250.0 + 220.0 * (g.C / 16);
     const double per_half = 0.0645;
     double best_cost = 1e30;
     for (int bh = 1; bh <= tallest; ++bh) {
@@ -594,7 +580,7 @@ RotPlan rot_plan_search(const Geom& g) {
       const int rounds = (items + wfull - 1) / wfull;
       int w = (items + rounds - 1) / rounds;  // fewest warps that finish in as many rounds
       if (w < 2) w = 2;
-      if (rot_smem(g, channels, bh, w) > budget) continue;
+      if (rot_smem(g, g.C, bh, w) > budget) continue;
       const int bands = (g.Ho + bh - 1) / bh;
       auto band_time = [&](int rows) {
         const double staged = per_half * ((double)g.C * ((rows - 1) * g.sH + 3) * g.W + (pl.dy_direct ? 18.0 : g.C + 18.0) * rows * g.Wo);
@@ -610,7 +596,7 @@ RotPlan rot_plan_search(const Geom& g) {
     pl.big = attempt == 1;
   }
   if (!pl.BH) {
-    const int slabs = channels / 16;
+    const int slabs = g.C / 16;
     int bh = (14 + NB - 1) / NB;
     if (bh > g.Ho) bh = g.Ho;
     for (; bh >= 1 && !pl.BH; --bh) {
@@ -654,14 +640,14 @@ struct FiltPlan {
 };
 
 // DYM: 0 = dy band in shared memory, 1 = dy words from global memory into registers, 2 = per-warp ring (see FiltPlan)
-template <int S, int NS, int MAXT, int MINB, int DYM, bool WHOLE>
+template <int S, int NS, int MAXT, int MINB, int DYM>
 __global__ void __launch_bounds__(MAXT, MINB) mma_filter_kernel(const __half* __restrict__ dy, const __half* __restrict__ x,
                                                             const __half* __restrict__ rot, float* __restrict__ partial,
                                                             const Geom g, const FiltPlan pl) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   const int c0 = blockIdx.y * pl.CG;
   const int cnt = min(pl.CG, g.C - c0);
-  const int nslab = (WHOLE ? cnt : whole_slabs(cnt)) >> 4;
+  const int nslab = cnt >> 4;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nwarps = blockDim.x >> 5;
   const int gq = lane >> 2, q = lane & 3;
   const int NB = (g.Wo + 7) >> 3;
@@ -727,8 +713,8 @@ __global__ void __launch_bounds__(MAXT, MINB) mma_filter_kernel(const __half* __
       auto fetch_dy = [&](int sidx) {
         dyw[sidx][0] = dyw[sidx][1] = 0u;
         if (sidx < nslab && owl < g.Wo) {
-          if (WHOLE || (sidx << 4) + gq < cnt) dyw[sidx][0] = __ldg(reinterpret_cast<const unsigned*>(dp + (size_t)(sidx << 4) * g.P));
-          if (WHOLE || (sidx << 4) + gq + 8 < cnt) dyw[sidx][1] = __ldg(reinterpret_cast<const unsigned*>(dp + (size_t)((sidx << 4) + 8) * g.P));
+          dyw[sidx][0] = __ldg(reinterpret_cast<const unsigned*>(dp + (size_t)(sidx << 4) * g.P));
+          dyw[sidx][1] = __ldg(reinterpret_cast<const unsigned*>(dp + (size_t)((sidx << 4) + 8) * g.P));
         }
       };
       if (DYM == 1) {
@@ -854,17 +840,16 @@ FiltPlan filt_plan_search(const Geom& g) {
   // Two shapes of block: up to four channel slabs and two blocks per SM, or six slabs in one block of up to
   // 14 warps per SM.  The second halves the hat-product work per slab; it pays on wide rows where the first
   // would be stuck with three slabs (measured: C = 96 at 112 x 112).
-  const int channels = whole_slabs(g.C);
-  int cg_small = (channels % 64 == 0) ? 64 : (channels % 48 == 0) ? 48 : (channels % 32 == 0) ? 32 : 16;
+  int cg_small = (g.C % 64 == 0) ? 64 : (g.C % 48 == 0) ? 48 : (g.C % 32 == 0) ? 32 : 16;
   if (const char* e = tuning_env("DK_B200_FILT_CG")) {  // tuning knob: 16, 32, 48 or 64 channels per block
     const int v = atoi(e);
-    if ((v == 16 || v == 32 || v == 48 || v == 64) && channels % v == 0) cg_small = v;
+    if ((v == 16 || v == 32 || v == 48 || v == 64) && g.C % v == 0) cg_small = v;
   }
-  const int cg_big = (channels % 96 == 0) ? 96 : (channels % 80 == 0) ? 80 : cg_small;
+  const int cg_big = (g.C % 96 == 0) ? 96 : (g.C % 80 == 0) ? 80 : cg_small;
   pl.big = cg_big >= 2 * cg_small && (g.Wo + 7) / 8 >= 14;
   if (const char* e = tuning_env("DK_B200_FILT_BIG")) pl.big = atoi(e) != 0;  // tuning knob
   pl.CG = pl.big ? cg_big : cg_small;
-  pl.groups = channels / pl.CG;
+  pl.groups = g.C / pl.CG;
   const int NB = (g.Wo + 7) / 8;
   const int Wp = g.W + (g.W & 1), Wpo = g.Wo + (g.Wo & 1);
   const size_t budget = pl.big ? kOnePerSm : kTwoPerSm;
@@ -939,7 +924,7 @@ struct GwPlan {
 };
 constexpr int kGwBandScratch = 3 * 36 * 8 * 4 + 24 * 8;  // per warp: G of three taps on the padded grid + their (u, v)
 
-template <int S, int MAXT, int MINB, bool DYD, bool WHOLE>
+template <int S, int MAXT, int MINB, bool DYD>
 __global__ void __launch_bounds__(MAXT, MINB) mma_gw_kernel(const __half* __restrict__ dy, const __half* __restrict__ x,
                                                         const __half* __restrict__ rot, const __half* __restrict__ w,
                                                         __half* __restrict__ drot, float* __restrict__ gpart,
@@ -947,8 +932,8 @@ __global__ void __launch_bounds__(MAXT, MINB) mma_gw_kernel(const __half* __rest
   constexpr int NS = 6;
   extern __shared__ __align__(16) unsigned char smem_raw[];
   const int c0 = blockIdx.y * pl.CG;
-  const int cnt = WHOLE ? pl.CG : min(pl.CG, g.C - c0), cnt16 = WHOLE ? cnt : whole_slabs(cnt);  // WHOLE: the groups divide evenly
-  const int nslab = cnt16 >> 4;
+  const int cnt = pl.CG;  // the groups divide the channels evenly
+  const int nslab = cnt >> 4;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nwarps = blockDim.x >> 5;
   const int gq = lane >> 2, q = lane & 3;
   const int NB = (g.Wo + 7) >> 3;
@@ -967,9 +952,9 @@ __global__ void __launch_bounds__(MAXT, MINB) mma_gw_kernel(const __half* __rest
   const float cell_row = (float)(q >> 1), cell_col = (float)((q & 1) << 1);
   const float uh0 = 0.5f, uw0 = 0.5f;  // (scope - kernel) / 2 for a 4 x 4 scope and 3 x 3 taps
 
-  for (int i = threadIdx.x; i < 16 * cnt16; i += blockDim.x) {
-    const int cell = i / cnt16, c = i - cell * cnt16;
-    bankT[cell * pitchT + c] = WHOLE || c < cnt ? __ldg(w + (size_t)(c0 + c) * 16 + cell) : __float2half(0.f);
+  for (int i = threadIdx.x; i < 16 * cnt; i += blockDim.x) {
+    const int cell = i / cnt, c = i - cell * cnt;
+    bankT[cell * pitchT + c] = __ldg(w + (size_t)(c0 + c) * 16 + cell);
   }
   {
     float* gz = reinterpret_cast<float*>(bankT + 16 * pitchT);  // the border cells of the G grids stay zero
@@ -995,11 +980,7 @@ __global__ void __launch_bounds__(MAXT, MINB) mma_gw_kernel(const __half* __rest
     const Band br = make_band(oh0, pl.BH, g.Ho, g.Wo, pl.mode_rot);
     __syncthreads();  // previous unit's readers are done
     load_band<0>(xband, bx, x, n, g.C, c0, cnt, g.H, g.W);
-    if (!WHOLE) zero_absent_channels(xband, bx.pitch_c, cnt);
-    if (!DYD) {
-      load_band<0>(yband, by, dy, n, g.C, c0, cnt, g.Ho, g.Wo);
-      if (!WHOLE) zero_absent_channels(yband, by.pitch_c, cnt);
-    }
+    if (!DYD) load_band<0>(yband, by, dy, n, g.C, c0, cnt, g.Ho, g.Wo);
     load_band<0>(rband, br, rot, n, 18, 0, 18, g.Ho, g.Wo);
     cp_async_wait_all();
     __syncthreads();
@@ -1022,8 +1003,8 @@ __global__ void __launch_bounds__(MAXT, MINB) mma_gw_kernel(const __half* __rest
         for (int sidx = 0; sidx < NS; ++sidx) {
           dyw[sidx][0] = dyw[sidx][1] = 0u;
           if (sidx < nslab && ow < g.Wo) {
-            if (WHOLE || (sidx << 4) + gq < cnt) dyw[sidx][0] = __ldg(dp + (size_t)(2 * sidx) * dstep8);
-            if (WHOLE || (sidx << 4) + gq + 8 < cnt) dyw[sidx][1] = __ldg(dp + (size_t)(2 * sidx + 1) * dstep8);
+            dyw[sidx][0] = __ldg(dp + (size_t)(2 * sidx) * dstep8);
+            dyw[sidx][1] = __ldg(dp + (size_t)(2 * sidx + 1) * dstep8);
           }
         }
       }
@@ -1165,14 +1146,13 @@ GwPlan gw_plan_search(const Geom& g) {
   // 0.147 (there one block over all 192 channels does as well as two groups with partial sums), so those stay apart.
   if (g.P > 196 && !tuning_env("DK_B200_GW_ANY")) return pl;
   pl.CG = 0;
-  const int channels = whole_slabs(g.C);
   for (int cg = 96; cg >= 48; cg -= 16)
-    if (channels % cg == 0) { pl.CG = cg; break; }
+    if (g.C % cg == 0) { pl.CG = cg; break; }
   if (!pl.CG) {
-    if (channels <= 96) pl.CG = channels;
+    if (g.C <= 96) pl.CG = g.C;
     else return pl;
   }
-  pl.groups = channels / pl.CG;
+  pl.groups = g.C / pl.CG;
   const int S = g.sH;
   const int NB = (g.Wo + 7) / 8;
   const int Wp = g.W + (g.W & 1), Wpo = g.Wo + (g.Wo & 1);
@@ -1267,6 +1247,11 @@ int local_mma_plan_query(const Geom& g, int pass, long long out[8]) {
   return DK_OK;
 }
 
+bool local_conv_mma_takes(const Geom& g, bool transposed) {
+  if (!fast_shape(g)) return false;
+  return plan_launches(conv_plan(g, transposed));
+}
+
 int local_conv_mma(const __half* src, const __half* rot, const __half* w, __half* dst, const Geom& g, bool transposed,
                    cudaStream_t s) {
   if (!fast_shape(g)) return DK_ERR_UNSUPPORTED;
@@ -1340,7 +1325,7 @@ int local_filter_mma(const __half* dy, const __half* x, const __half* rot, __hal
   float* partial = reinterpret_cast<float*>(ws);
 #define DK_LAUNCH_FILT(SS, NS, MAXT, MINB, DD)                                                        \
   {                                                                                                 \
-    auto kern = g.C & 15 ? mma_filter_kernel<SS, NS, MAXT, MINB, DD, false> : mma_filter_kernel<SS, NS, MAXT, MINB, DD, true>; \
+    auto kern = mma_filter_kernel<SS, NS, MAXT, MINB, DD>;                                          \
     if ((rc = enable_smem(kern, pl.smem))) return rc;                                               \
     kern<<<dim3(pl.blocks_x, pl.groups), pl.warps * 32, pl.smem, s>>>(dy, x, rot, partial, g, pl);  \
   }
@@ -1385,7 +1370,7 @@ int local_gw_mma(const __half* dy, const __half* x, const __half* rot, const __h
   float* gpart = reinterpret_cast<float*>(reinterpret_cast<unsigned char*>(ws) + pl.dw_bytes);
 #define DK_LAUNCH_GW(SS, MAXT, MINB, DD)                                                                       \
   {                                                                                                          \
-    auto kern = g.C & 15 ? mma_gw_kernel<SS, MAXT, MINB, DD, false> : mma_gw_kernel<SS, MAXT, MINB, DD, true>; \
+    auto kern = mma_gw_kernel<SS, MAXT, MINB, DD>;                                                           \
     if ((rc = enable_smem(kern, pl.smem))) return rc;                                                        \
     kern<<<dim3(pl.blocks_x, pl.groups), pl.warps * 32, pl.smem, s>>>(dy, x, rot, w, drot, gpart, partial, g, pl); \
   }

@@ -12,7 +12,8 @@
 // warp is left with 72 multiply-adds, 15 loads and the stores per 256 outputs.
 //
 // fp16: K leaves the tensor cores rounded to fp16 (relative 2^-11, like the tensors themselves) and meets x in the
-// mixed-precision multiply-add (exact product, fp32 sum), as in dk_local_ring.cu.
+// mixed-precision multiply-add (exact product, fp32 sum), as in dk_local_ring.cu and dk_local_mma.cu, whose calls these are.  Calls
+// that those do not take (channels no multiple of 16) keep K in fp32: W is exact in one piece, the hat products take two.
 // fp32: W is split into three fp16 pieces and the hat products into two, scaled by powers of two (W per channel, its last piece
 // by 2^15 more; the hat products by 2^15).  The pieces hold W to 24 bits down to 2^-30 of the channel's largest value, below that
 // to 2^-55 of it, and the hat products to 23 bits down to 2^-15, below that to 2^-40.  Five products, the small ones first: the
@@ -51,20 +52,20 @@ constexpr int kTeams = 4;
 constexpr int kConsumers = 16;
 constexpr int kHelpers = 12;  // MMA, loaders, hat products, stores
 constexpr int kThreads = 32 * (kConsumers + kHelpers);
-// Registers per thread: 72 at launch, then more for the four consumer warpgroups than for the three of the helpers.  fp16 consumers
-// hold two items; fp32 ones hold one, and the hat products need what that leaves.
+// Registers per thread: 72 at launch, then more for the four consumer warpgroups than for the three of the helpers.  Consumers of
+// fp16 kernel values hold two items; of fp32 values (FULL) one, and the hat products need what that leaves.
 constexpr int kRegsLaunch = 72;
-template <typename T>
+template <bool FULL>
 __host__ __device__ constexpr int consumer_regs() {
-  return sizeof(T) == 2 ? 88 : 80;
+  return FULL ? 80 : 88;
 }
-template <typename T>
+template <bool FULL>
 __host__ __device__ constexpr int helper_regs() {
-  return sizeof(T) == 2 ? 48 : 56;
+  return FULL ? 56 : 48;
 }
-template <typename T>
-constexpr bool kSharesAdd = kConsumers * consumer_regs<T>() + kHelpers * helper_regs<T>() <= (kConsumers + kHelpers) * kRegsLaunch;
-static_assert(kSharesAdd<float> && kSharesAdd<__half>, "register shares");
+template <bool FULL>
+constexpr bool kSharesAdd = kConsumers * consumer_regs<FULL>() + kHelpers * helper_regs<FULL>() <= (kConsumers + kHelpers) * kRegsLaunch;
+static_assert(kSharesAdd<true> && kSharesAdd<false>, "register shares");
 constexpr int kLoaders = 3;                         // warps that fetch rows without TMA
 constexpr int kStepSegs = 8;
 constexpr int kSlotCols = 48;                       // three taps x 16 pixels
@@ -79,9 +80,9 @@ constexpr int kMinSmem = 120 * 1024;                // one block per SM: it take
 
 // Hat products: two warps per step, each pair of warps with a buffer of its own, so that a warp sees every reuse of its buffer
 // (a barrier's phase can only be told from the one before it).
-template <typename T>
+template <bool FULL>
 __host__ __device__ constexpr int beta_warps(int loaders) {
-  return loaders == 1 && sizeof(T) == 2 ? 6 : 4;
+  return loaders == 1 && !FULL ? 6 : 4;
 }
 
 template <typename T>
@@ -135,9 +136,9 @@ template <int MODE> struct Walk {
 // ------------------------------------------------------------------ consumers' operands
 // One item = one segment (8 pixels) and one kernel row of the lane's channel: 24 kernel values (tap-major; pixels p and
 // p + 4 in adjacent columns) and the source window.
-template <typename T, int MODE> struct Item;
+template <typename T, int MODE, bool FULL> struct Item;
 
-template <int MODE> struct Item<__half, MODE> {
+template <int MODE> struct Item<__half, MODE, false> {
   static constexpr int NW = MODE == kFwd2 ? 8 : 4;
   unsigned k[12];        // fp16 pairs (p, p + 4)
   unsigned w[NW];        // source columns 0 .. 7 (15) of the segment
@@ -165,20 +166,30 @@ template <int MODE> struct Item<__half, MODE> {
   }
 };
 
-template <int MODE> struct Item<float, MODE> {
+template <typename T, int MODE> struct Item<T, MODE, true> {
   static constexpr int NW = MODE == kFwd2 ? 16 : 8;
   unsigned k[24];
   float w[NW], left, right;
   __device__ __forceinline__ void load(unsigned tmem, const char* row) {
     ld24(k, tmem);
-    const float* x = reinterpret_cast<const float*>(row);
+    const T* x = reinterpret_cast<const T*>(row);
+    if constexpr (sizeof(T) == 4) {
 #pragma unroll
-    for (int i = 0; i < NW / 4; ++i) {
-      const float4 q = *reinterpret_cast<const float4*>(x + 4 * i);
-      w[4 * i] = q.x, w[4 * i + 1] = q.y, w[4 * i + 2] = q.z, w[4 * i + 3] = q.w;
+      for (int i = 0; i < NW / 4; ++i) {
+        const float4 q = *reinterpret_cast<const float4*>(x + 4 * i);
+        w[4 * i] = q.x, w[4 * i + 1] = q.y, w[4 * i + 2] = q.z, w[4 * i + 3] = q.w;
+      }
+    } else {
+#pragma unroll
+      for (int i = 0; i < NW / 8; ++i) {
+        const uint4 q = *reinterpret_cast<const uint4*>(x + 8 * i);
+        const unsigned h[4] = {q.x, q.y, q.z, q.w};
+#pragma unroll
+        for (int j = 0; j < 4; ++j) w[8 * i + 2 * j] = mma::lo2f(h[j]), w[8 * i + 2 * j + 1] = mma::hi2f(h[j]);
+      }
     }
-    if (MODE != kData2) left = x[-1];
-    if (MODE != kFwd2) right = x[8];
+    if (MODE != kData2) left = static_cast<float>(x[-1]);
+    if (MODE != kFwd2) right = static_cast<float>(x[8]);
   }
   template <int I> __device__ __forceinline__ float at() const {
     if constexpr (I < 0) return left;
@@ -193,8 +204,8 @@ template <int MODE> struct Item<float, MODE> {
 
 // acc += window * kernel row.  Source column of tap t and pixel p: p xs + t - 1 (kData2: p, and p + 1 for the third tap);
 // kData2 keeps the even destination columns in acc[0..8) and the odd ones in acc[8..16).
-template <typename T, int MODE, int N>
-__device__ __forceinline__ void multiply(float (&acc)[N], const Item<T, MODE>& it) {
+template <typename T, int MODE, bool FULL, int N>
+__device__ __forceinline__ void multiply(float (&acc)[N], const Item<T, MODE, FULL>& it) {
   constexpr int XS = Walk<MODE>::xs;
   constexpr bool D = MODE == kData2;
 #define DK_TAP(t, p)                                                                                             \
@@ -355,9 +366,8 @@ __device__ __forceinline__ void fetch_offsets(Offsets<T>& o, const T* __restrict
   }
 }
 
-template <typename T, int MODE, bool SC44>
+template <typename T, int MODE, bool SC44, bool SPLIT>
 __device__ __forceinline__ void write_hats(unsigned buf, const Offsets<T>& o, int half, const ConvParams& p, int lane) {
-  constexpr bool SPLIT = std::is_same<T, float>::value;
   const int sl = lane >> 3, px = lane & 7;
   // row of this pixel inside its 8-row core matrix: pixels p and p + 4 are neighbours
   const unsigned dst = buf + (half * 2 + (sl >> 1)) * kPairRow + (sl & 1) * (3 * 256) + ((px & 3) * 2 + (px >> 2)) * 16;
@@ -429,17 +439,18 @@ __device__ __forceinline__ void copy_row(char* slot, const T* __restrict__ src, 
 
 // ------------------------------------------------------------------ forward and grad-input
 // d = bank at a (its pieces 8 columns apart) * hat products at b (kPiece apart), the smallest products first
-template <typename T>
+template <typename T, bool FULL>
 __device__ __forceinline__ void products(unsigned d, unsigned a, uint64_t b, unsigned idesc) {
+  const uint64_t b_lo = b + (kPiece >> 4);
   if constexpr (sizeof(T) == 4) {
-    const uint64_t b_lo = b + (kPiece >> 4);
     mma_ts(d, a + 16, b, idesc, false);
     mma_ts_scaled<15>(d, a + 8, b_lo, idesc);
     mma_ts(d, a + 8, b, idesc, true);
     mma_ts(d, a, b_lo, idesc, true);
     mma_ts(d, a, b, idesc, true);
   } else {
-    mma_ts(d, a, b, idesc, false);
+    if (FULL) mma_ts(d, a, b_lo, idesc, false);
+    mma_ts(d, a, b, idesc, FULL);
   }
 }
 
@@ -449,34 +460,34 @@ template <typename T> __host__ __device__ constexpr int out_pitch() { return kSt
 struct ConvSmem {  // byte offsets behind the row ring
   unsigned beta, inv, out, segs, bars, total;
 };
-template <typename T, int MODE>
+template <typename T, int MODE, bool FULL>
 __host__ __device__ inline ConvSmem conv_smem(unsigned ring_bytes, int groups, int nbuf) {
-  constexpr bool SPLIT = std::is_same<T, float>::value;
   ConvSmem m;
   m.beta = (ring_bytes + 32 + 127) & ~127u;  // 32: what the last channel row's right edge may read
-  m.inv = m.beta + nbuf * kPiece * (SPLIT ? 2 : 1);
-  m.out = m.inv + (SPLIT ? groups * 128 : 0);
+  m.inv = m.beta + nbuf * kPiece * (FULL ? 2 : 1);
+  m.out = m.inv + (sizeof(T) == 4 ? groups * 128 : 0);
   m.segs = m.out + (MODE == kData2 ? 0 : groups * 32 * out_pitch<T>());
   m.bars = m.segs + kDepth * kStepSegs * 16;
   m.total = m.bars + kBars * 8 + 16;
   return m;
 }
 
-template <typename T, int MODE, bool SC44, int NL>
+// FULL: the kernel values leave the tensor cores as fp32 (fp32 tensors always)
+template <typename T, int MODE, bool SC44, int NL, bool FULL>
 __global__ void __launch_bounds__(kThreads, 1)
     tc_conv_kernel(const __grid_constant__ CUtensorMap tm, const T* __restrict__ src, const T* __restrict__ rot,
                    const T* __restrict__ bank, T* __restrict__ dst, const ConvParams p) {
   extern __shared__ __align__(1024) char smem[];
   using Wk = Walk<MODE>;
-  constexpr bool SPLIT = std::is_same<T, float>::value, STAGED = MODE != kData2;
-  constexpr int PIECES = SPLIT ? 2 : 1, E = sizeof(T), TILE = 8 * bank_piece_count<T>();  // columns of 128 channels' bank
-  constexpr int NB = beta_warps<T>(NL), NBUF = NB / 2, NS = kHelpers - 1 - NL - NB;
+  constexpr bool STAGED = MODE != kData2, SCALED = sizeof(T) == 4;
+  constexpr int PIECES = FULL ? 2 : 1, E = sizeof(T), TILE = 8 * bank_piece_count<T>();  // columns of 128 channels' bank
+  constexpr int NB = beta_warps<FULL>(NL), NBUF = NB / 2, NS = kHelpers - 1 - NL - NB;
   constexpr int kOutPitch = out_pitch<T>();
   const int warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0), lane = threadIdx.x & 31;
   const int c0 = blockIdx.y * p.CG, cg = min(p.CG, p.C - c0);
   const int groups = p.full * 4 + p.rest, rounds = p.full + (p.rest ? 1 : 0);
   const unsigned slot_bytes = (unsigned)p.CG * p.pitch, ring_bytes = slot_bytes * p.R;
-  const ConvSmem sm = conv_smem<T, MODE>(ring_bytes, groups, NBUF);
+  const ConvSmem sm = conv_smem<T, MODE, FULL>(ring_bytes, groups, NBUF);
   const unsigned base = smem_u32(smem);
   const unsigned x_full = base + sm.bars, step_done = x_full + 8 * kDepth, b_full = step_done + 8 * kDepth;
   const unsigned b_free = b_full + 8 * kMaxBuf, t_full = b_free + 8 * kMaxBuf, t_empty = t_full + 16, o_full = t_empty + 16,
@@ -534,7 +545,7 @@ __global__ void __launch_bounds__(kThreads, 1)
       const bool ok = grp >= 0 && ch < cg;
       const float inv = bank_to_tmem<T>(tmem + ((unsigned)(q * 32) << 16) + kBankCol + i * TILE, bank + (size_t)(c0 + (ok ? ch : 0)) * p.cells,
                                         p.cells, ok);
-      if (SPLIT && grp >= 0) inv_s[grp * 32 + lane] = inv;
+      if (SCALED && grp >= 0) inv_s[grp * 32 + lane] = inv;
     }
     wait_st();
   }
@@ -544,7 +555,7 @@ __global__ void __launch_bounds__(kThreads, 1)
 
   if (warp < kConsumers) {
     // ================================================================ consumers
-    regs_inc<consumer_regs<T>()>();
+    regs_inc<consumer_regs<FULL>()>();
     const int q = warp & 3, team = warp >> 2;
     const unsigned lanes = (unsigned)(q * 32) << 16;
     const bool vec = p.store == 16;
@@ -576,16 +587,16 @@ __global__ void __launch_bounds__(kThreads, 1)
         }
         const int ch = grp * 32 + lane;
         const char* xc = smem + ch * p.pitch;
-        const float inv = SPLIT ? inv_s[ch] : 1.f;
+        const float inv = SCALED ? inv_s[ch] : FULL ? 1.f / 32768.f : 1.f;
         float acc[2][NA];
 #pragma unroll
         for (int h = 0; h < 2; ++h)
 #pragma unroll
           for (int i = 0; i < NA; ++i) acc[h][i] = 0.f;
         // items (kernel row, segment) in order; fp16 fetches the next item while it multiplies this one
-        constexpr int NI = SPLIT ? 1 : 2;
-        Item<T, MODE> item[NI];
-        auto fetch = [&](Item<T, MODE>& it, int i) -> bool {
+        constexpr int NI = FULL ? 1 : 2;
+        Item<T, MODE, FULL> item[NI];
+        auto fetch = [&](Item<T, MODE, FULL>& it, int i) -> bool {
           const int v = i >> 1, h = i & 1, set = (use + v) & 1;
           if (h == 0) {
             if (!wait_bar(t_full + 8 * set, ((use + v) >> 1) & 1, abort_flag)) return false;
@@ -596,7 +607,7 @@ __global__ void __launch_bounds__(kThreads, 1)
           it.load(tmem + lanes + set * kSetCols + team * kSlotCols + h * 24, xc + (row_of[v] == 0 ? sd[h].x : row_of[v] == 1 ? sd[h].y : sd[h].z));
           return true;
         };
-        auto fetched = [&](Item<T, MODE>& it, int i) {
+        auto fetched = [&](Item<T, MODE, FULL>& it, int i) {
           wait_ld(it.k);
           if (i & 1) {  // both segments' accumulators of this kernel row are in registers
             fence_before();
@@ -615,13 +626,13 @@ __global__ void __launch_bounds__(kThreads, 1)
               ok = fetch(item[(i + 1) % NI], i + 1);
               if (!ok) break;
             }
-            multiply<T, MODE>(acc[i & 1], item[i % NI]);
+            multiply<T, MODE, FULL>(acc[i & 1], item[i % NI]);
             if (i < 5) fetched(item[(i + 1) % NI], i + 1);
           } else {
             ok = fetch(item[0], i);
             if (!ok) break;
             fetched(item[0], i);
-            multiply<T, MODE>(acc[i & 1], item[0]);
+            multiply<T, MODE, FULL>(acc[i & 1], item[0]);
           }
           if (MODE == kData2 && (i < 2 || i > 3)) {  // kernel row 0 completes the even row of the patch, 2 the odd one
             const int h = i & 1, row = 2 * (sd[h].w >> 8) + (i > 3), col = 16 * (sd[h].w & 255);
@@ -647,8 +658,10 @@ __global__ void __launch_bounds__(kThreads, 1)
 #pragma unroll
           for (int h = 0; h < 2; ++h) {
             if constexpr (E == 2) {
-              *reinterpret_cast<uint4*>(o + 16 * h) = make_uint4(mma::pack2(acc[h][0], acc[h][1]), mma::pack2(acc[h][2], acc[h][3]),
-                                                                 mma::pack2(acc[h][4], acc[h][5]), mma::pack2(acc[h][6], acc[h][7]));
+              unsigned r[4];
+#pragma unroll
+              for (int k = 0; k < 4; ++k) r[k] = mma::pack2(acc[h][2 * k] * inv, acc[h][2 * k + 1] * inv);
+              *reinterpret_cast<uint4*>(o + 16 * h) = make_uint4(r[0], r[1], r[2], r[3]);
             } else {
 #pragma unroll
               for (int k = 0; k < 8; k += 4)
@@ -668,8 +681,8 @@ __global__ void __launch_bounds__(kThreads, 1)
     }
   } else if (warp == kConsumers) {
     // ================================================================ MMA
-    regs_dec<helper_regs<T>()>();
-    constexpr unsigned idesc_all = idesc_f16(128, kSetCols, false, false, SPLIT), idesc_pair = idesc_f16(128, kSlotCols, false, false, SPLIT);
+    regs_dec<helper_regs<FULL>()>();
+    constexpr unsigned idesc_all = idesc_f16(128, kSetCols, false, false, FULL), idesc_pair = idesc_f16(128, kSlotCols, false, false, FULL);
     int use = 0;
     bool ok = true;
     for (int s = 0, bi = 0, turn = 0; s < steps && ok; ++s) {
@@ -689,11 +702,11 @@ __global__ void __launch_bounds__(kThreads, 1)
           const uint64_t b = sdesc(buf + v * (kTeams * kPairRow), 128, 256);
           if (elect_one()) {
             if (rd < p.full) {
-              products<T>(d, tmem + kBankCol + rd * TILE, b, idesc_all);
+              products<T, FULL>(d, tmem + kBankCol + rd * TILE, b, idesc_all);
             } else {  // the remaining groups sit on other lanes for every pair
 #pragma unroll
               for (int j = 0; j < kTeams; ++j) {
-                products<T>(d + j * kSlotCols, tmem + kBankCol + (p.full + ((j + s) & 3)) * TILE, b + j * (kPairRow >> 4), idesc_pair);
+                products<T, FULL>(d + j * kSlotCols, tmem + kBankCol + (p.full + ((j + s) & 3)) * TILE, b + j * (kPairRow >> 4), idesc_pair);
               }
             }
             commit(t_full + 8 * set);
@@ -707,7 +720,7 @@ __global__ void __launch_bounds__(kThreads, 1)
     }
   } else if (warp <= kConsumers + NL) {
     // ================================================================ source rows
-    regs_dec<helper_regs<T>()>();
+    regs_dec<helper_regs<FULL>()>();
     const int lw = warp - kConsumers - 1;
     int next = 0, done = 0;
     bool ok = true;
@@ -765,13 +778,13 @@ __global__ void __launch_bounds__(kThreads, 1)
     }
   } else if (warp <= kConsumers + NL + NB) {
     // ================================================================ hat products
-    regs_dec<helper_regs<T>()>();
+    regs_dec<helper_regs<FULL>()>();
     const int w = warp - kConsumers - 1 - NL, half = w & 1, bi = w >> 1;
     Offsets<T> off;
     if (bi < steps) fetch_offsets<T, MODE>(off, rot, lo + bi * kStepSegs + half * 4, hi, p, lane);
     for (int s = bi, turn = 0; s < steps; s += NBUF, ++turn) {
       if (turn > 0 && !wait_bar(b_free + 8 * bi, (turn - 1) & 1, abort_flag)) break;
-      write_hats<T, MODE, SC44>(base + sm.beta + bi * (PIECES * kPiece), off, half, p, lane);
+      write_hats<T, MODE, SC44, FULL>(base + sm.beta + bi * (PIECES * kPiece), off, half, p, lane);
       fence_proxy_async();
       __syncwarp();
       if (lane == 0) mbar_arrive(b_full + 8 * bi);
@@ -779,7 +792,7 @@ __global__ void __launch_bounds__(kThreads, 1)
     }
   } else {
     // ================================================================ results to memory
-    regs_dec<helper_regs<T>()>();
+    regs_dec<helper_regs<FULL>()>();
     const int w = warp - kConsumers - 1 - NL - NB;
     const size_t plane = (size_t)p.Hd * p.Wd;
     for (int s = 0; s < steps && STAGED; ++s) {
@@ -859,7 +872,7 @@ struct ConvPlan {
   ConvParams p;
 };
 
-template <typename T, int MODE>
+template <typename T, int MODE, bool FULL>
 ConvPlan plan_conv(const Geom& g, const void* src, const void* dst) {
   using Wk = Walk<MODE>;
   ConvPlan pl;
@@ -889,7 +902,7 @@ ConvPlan plan_conv(const Geom& g, const void* src, const void* dst) {
   p.pitch = ((1 + (p.nseg * 8 * Wk::xs * E) / 16) | 1) * 16;
   if (p.pitch < 16 + p.Ws * E || p.pitch > 1152 || p.Hg >= (1 << 22)) return pl;
   pl.tma = (reinterpret_cast<uintptr_t>(src) & 15) == 0 && (p.Ws * E) % 16 == 0 && p.pitch / E <= 256;
-  const int nbuf = beta_warps<T>(pl.tma ? 1 : kLoaders) / 2;
+  const int nbuf = beta_warps<FULL>(pl.tma ? 1 : kLoaders) / 2;
   const int need = step_rows(p.nseg, p.Hg, Wk::S, p.L, Wk::rows, kStepSegs);
   const int want = step_rows(p.nseg, p.Hg, Wk::S, p.L, Wk::rows, kStepSegs * kDepth);
   const int groups = (g.C + 31) / 32, steps = (p.segs + kStepSegs - 1) / kStepSegs, sms = device_sm_count();
@@ -904,7 +917,7 @@ ConvPlan plan_conv(const Geom& g, const void* src, const void* dst) {
     const int boxes = (cg + 255) / 256;
     cg = (cg + 8 * boxes - 1) / (8 * boxes) * (8 * boxes);  // boxes start on 128 bytes
     if (splits > 1 && cg != per * 32) continue;
-    const size_t slot = (size_t)cg * p.pitch, fixed = conv_smem<T, MODE>(0, per, nbuf).total + 160;
+    const size_t slot = (size_t)cg * p.pitch, fixed = conv_smem<T, MODE, FULL>(0, per, nbuf).total + 160;
     if (fixed + slot * (need + 1) > budget) continue;
     int R = (int)((budget - fixed) / slot);
     if (R > want + 2) R = want + 2;
@@ -921,7 +934,7 @@ ConvPlan plan_conv(const Geom& g, const void* src, const void* dst) {
       p.CG = cg, p.box_c = cg / boxes, p.full = full, p.rest = rest, p.R = R;
       p.steps_per_cta = spc;
       pl.ctas = (steps + spc - 1) / spc, pl.splits = splits;
-      pl.smem = conv_smem<T, MODE>((unsigned)(slot * R), per, nbuf).total;
+      pl.smem = conv_smem<T, MODE, FULL>((unsigned)(slot * R), per, nbuf).total;
       if (pl.smem < kMinSmem) pl.smem = kMinSmem;
     }
   }
@@ -951,9 +964,9 @@ bool shares_fit() {
   return r >= kRegsLaunch;
 }
 
-template <typename T, int MODE, bool SC44, int NL>
+template <typename T, int MODE, bool SC44, int NL, bool FULL>
 int run_conv(const ConvPlan& pl, const CUtensorMap& tm, const T* src, const T* rot, const T* w, T* dst, cudaStream_t s) {
-  constexpr auto kern = tc_conv_kernel<T, MODE, SC44, NL>;
+  constexpr auto kern = tc_conv_kernel<T, MODE, SC44, NL, FULL>;
   if (!shares_fit<kern>()) return DK_ERR_UNSUPPORTED;
   const int rc = enable_smem(kern, pl.smem);
   if (rc) return rc;
@@ -961,51 +974,62 @@ int run_conv(const ConvPlan& pl, const CUtensorMap& tm, const T* src, const T* r
   return check_launch();
 }
 
-template <typename T, int MODE>
+template <typename T, int MODE, bool FULL>
 int launch_conv(const T* src, const T* rot, const T* w, T* dst, const Geom& g, cudaStream_t s) {
-  const ConvPlan pl = plan_conv<T, MODE>(g, src, dst);
+  const ConvPlan pl = plan_conv<T, MODE, FULL>(g, src, dst);
   if (!pl.ok) return DK_ERR_UNSUPPORTED;
   CUtensorMap tm;
   std::memset(&tm, 0, sizeof(tm));
   if (pl.tma && !make_plane_row_map(&tm, src, sizeof(T), pl.p.Ws, pl.p.Hs, (long long)g.N * g.C, pl.p.pitch / (int)sizeof(T), pl.p.box_c))
     return DK_ERR_UNSUPPORTED;
   const bool sc44 = g.scH == 4 && g.scW == 4;
-  if (pl.tma) return sc44 ? run_conv<T, MODE, true, 1>(pl, tm, src, rot, w, dst, s) : run_conv<T, MODE, false, 1>(pl, tm, src, rot, w, dst, s);
-  return sc44 ? run_conv<T, MODE, true, kLoaders>(pl, tm, src, rot, w, dst, s) : run_conv<T, MODE, false, kLoaders>(pl, tm, src, rot, w, dst, s);
+  if (pl.tma) return sc44 ? run_conv<T, MODE, true, 1, FULL>(pl, tm, src, rot, w, dst, s) : run_conv<T, MODE, false, 1, FULL>(pl, tm, src, rot, w, dst, s);
+  return sc44 ? run_conv<T, MODE, true, kLoaders, FULL>(pl, tm, src, rot, w, dst, s)
+              : run_conv<T, MODE, false, kLoaders, FULL>(pl, tm, src, rot, w, dst, s);
 }
 
-template <typename T, int MODE, bool SC44, int NL>
+template <typename T, int MODE, bool SC44, int NL, bool FULL>
 void add_registers(long long out[8]) {
-  const int r = launch_registers<tc_conv_kernel<T, MODE, SC44, NL>>();
+  const int r = launch_registers<tc_conv_kernel<T, MODE, SC44, NL, FULL>>();
   ++out[0];
   if (out[1] < 0 || r < out[1]) out[1] = r;
 }
-template <typename T, int MODE>
+template <typename T, int MODE, bool FULL>
 void add_registers_of(long long out[8]) {
-  add_registers<T, MODE, true, 1>(out), add_registers<T, MODE, false, 1>(out);
-  add_registers<T, MODE, true, kLoaders>(out), add_registers<T, MODE, false, kLoaders>(out);
+  add_registers<T, MODE, true, 1, FULL>(out), add_registers<T, MODE, false, 1, FULL>(out);
+  add_registers<T, MODE, true, kLoaders, FULL>(out), add_registers<T, MODE, false, kLoaders, FULL>(out);
 }
-template <typename T>
+template <typename T, bool FULL>
 void add_registers_of(long long out[8]) {
-  add_registers_of<T, kFwd1>(out), add_registers_of<T, kFwd2>(out), add_registers_of<T, kData1>(out), add_registers_of<T, kData2>(out);
+  add_registers_of<T, kFwd1, FULL>(out), add_registers_of<T, kFwd2, FULL>(out), add_registers_of<T, kData1, FULL>(out),
+      add_registers_of<T, kData2, FULL>(out);
+}
+
+template <typename T, bool FULL>
+int launch_conv(const T* src, const T* rot, const T* w, T* dst, const Geom& g, bool transposed, cudaStream_t s) {
+  if (!tc_shape(g)) return DK_ERR_UNSUPPORTED;
+  if (!transposed) return g.sH == 1 ? launch_conv<T, kFwd1, FULL>(src, rot, w, dst, g, s) : launch_conv<T, kFwd2, FULL>(src, rot, w, dst, g, s);
+  return g.sH == 1 ? launch_conv<T, kData1, FULL>(src, rot, w, dst, g, s) : launch_conv<T, kData2, FULL>(src, rot, w, dst, g, s);
 }
 
 }  // namespace
 
 template <typename T>
 int local_conv_tc(const T* src, const T* rot, const T* w, T* dst, const Geom& g, bool transposed, cudaStream_t s) {
-  if (!tc_shape(g)) return DK_ERR_UNSUPPORTED;
-  if (!transposed) return g.sH == 1 ? launch_conv<T, kFwd1>(src, rot, w, dst, g, s) : launch_conv<T, kFwd2>(src, rot, w, dst, g, s);
-  return g.sH == 1 ? launch_conv<T, kData1>(src, rot, w, dst, g, s) : launch_conv<T, kData2>(src, rot, w, dst, g, s);
+  return launch_conv<T, true>(src, rot, w, dst, g, transposed, s);
 }
 template int local_conv_tc<float>(const float*, const float*, const float*, float*, const Geom&, bool, cudaStream_t);
 template int local_conv_tc<__half>(const __half*, const __half*, const __half*, __half*, const Geom&, bool, cudaStream_t);
 
+int local_conv_tc_rounded(const __half* src, const __half* rot, const __half* w, __half* dst, const Geom& g, bool transposed,
+                          cudaStream_t s) {
+  return launch_conv<__half, false>(src, rot, w, dst, g, transposed, s);
+}
+
 int tc_register_query(long long out[8]) {
   for (int i = 0; i < 8; ++i) out[i] = 0;
   out[1] = -1, out[2] = kRegsLaunch;
-  add_registers_of<float>(out);
-  add_registers_of<__half>(out);
+  add_registers_of<float, true>(out), add_registers_of<__half, false>(out), add_registers_of<__half, true>(out);
   return out[1] < 0 ? DK_ERR_CUDA : DK_OK;
 }
 

@@ -46,12 +46,13 @@ typedef enum dk_dtype { DK_F32 = 0, DK_F16 = 1, DK_F64 = 2 } dk_dtype;
 
 /* Devices and numeric limits.  Every pointer of a call must belong to the CURRENT device (cudaGetDevice()): the library
  * launches there, on the given stream, and never checks ownership.  fp16 calls on the tensor-core path (3x3, pad 1,
- * stride 1 or 2, at most 16 bank cells): forward and grad-input take the resampled kernel
+ * stride 1 or 2, at most 16 bank cells, channels a multiple of 16): forward and grad-input take the resampled kernel
  * value of a (pixel, tap, channel) from the tensor cores rounded to fp16 (relative 2^-11, the precision of the tensors
  * themselves), multiply it exactly with the fp16 input and sum in fp32;
  * grad-offsets and grad-bank feed the products grad_output * input to the tensor cores as fp16, so
  * |grad_output * input| must stay below 65504 (an overflow gives Inf / NaN gradients, which a loss scaler's
- * overflow check catches and answers by lowering its scale); all sums are fp32. */
+ * overflow check catches and answers by lowering its scale); all sums are fp32.  fp16 calls with other channel counts form
+ * kernel values and products in fp32. */
 
 /* Geometry of one depthwise call.  Same fields as the reference's
  * SampleDepthwiseArgs (csrc/filter_sample_depthwise_cuda.h:1-28) minus the output

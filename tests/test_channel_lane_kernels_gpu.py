@@ -1,8 +1,8 @@
 """The local operator with any number of channels, against the CPU oracle: fp32 runs on the tcgen05 kernels (one channel per
-TMEM lane), fp16 there on wide rows, else on the mma.sync kernels with a partly filled last slab of channels.  The sizes are the edges of their tiles:
-32-channel groups (1 to 5 of them, full and partial, so that every
-placement of the remaining groups on the lanes occurs), 8-pixel segments, rows with and without TMA, planes of one row or one
-pixel, steps that span samples, more channels than one block takes."""
+TMEM lane), fp16 there on wide rows, else on the mma.sync kernels (channels a multiple of 16) or the general ones.  The sizes are the
+edges of their tiles: 32-channel groups (1 to 5 of them, full and partial, so that every placement of the remaining groups on the
+lanes occurs), 8-pixel segments, rows with and without TMA, planes of one row or one pixel, steps that span samples, more channels
+than one block takes."""
 import pytest
 import torch
 
@@ -15,7 +15,7 @@ SHAPES = [
     (1, 8, 1, 1), (5, 16, 1, 9), (3, 24, 7, 7), (2, 32, 8, 8), (2, 40, 9, 16), (1, 56, 17, 24), (2, 72, 19, 23),
     (1, 104, 12, 33), (2, 136, 5, 40), (1, 160, 28, 28), (1, 200, 14, 14), (1, 264, 3, 64), (9, 280, 4, 4), (1, 1096, 6, 10),
     (1, 24, 112, 112), (1, 8, 2, 200), (1, 32, 110, 110), (2, 48, 31, 57),
-    (2, 72, 31, 48), (5, 264, 2, 32),
+    (2, 72, 31, 48), (5, 264, 2, 32), (2, 72, 9, 28), (1, 40, 5, 36), (2, 104, 6, 100),
 ]
 
 
@@ -94,6 +94,44 @@ def test_wide_range_inside_a_channel(stride):
                                     both(x.abs(), torch.zeros_like(r), flat, dy.abs())):
         over = (got.double().cpu() - want).abs() - (2.0 ** -20 * size + 2.0 ** -50 * top)
         assert float(over.max()) <= 0
+
+
+def _flat(t, skip):
+    """A copy of t that starts `skip` elements into its storage."""
+    out = torch.empty(t.numel() + skip, dtype=t.dtype, device=t.device)[skip:].view(t.shape)
+    return out.copy_(t)
+
+
+@pytest.mark.parametrize("skip", [0, 1])
+@pytest.mark.parametrize("n,c,h,w,stride", [(2, 24, 20, 24, 1), (2, 40, 11, 64, 2), (1, 72, 9, 28, 1), (2, 72, 13, 101, 1), (3, 104, 7, 7, 2)])
+def test_fp16_channels_no_multiple_of_16_are_computed_in_fp32(n, c, h, w, stride, skip):
+    """Results are off by their rounding to fp16 only: relative 2^-12 / sqrt(3) to 2^-11 / sqrt(3) depending on the mantissa, 2.1e-4 over
+    a binade, here with a fifth more (kernel values or products rounded to fp16: 3e-4 to 3.6e-4).  Products dy x beyond 65504 are no
+    limit either.  skip = 1: tensors on odd addresses."""
+    from deformable_kernels.ops.deform_kernel.functions import sample_depthwise
+    from oracle import dk_oracle as O
+    case = make_case(n, c, h, w, stride=stride, rot_std=1.0, seed=c)
+    half = {k: case[k].half() for k in ("input", "rotation", "weight", "grad_output")}
+
+    def run(a):
+        x, r, wt, dy = (_flat(a[k].to(DEV), skip) for k in ("input", "rotation", "weight", "grad_output"))
+        for t in (x, r, wt):
+            t.requires_grad_(True)
+        y = sample_depthwise(x, r, wt, **case["args"])
+        d = {k: v.double() for k, v in a.items()}
+        want = [O.sample_depthwise_forward(d["input"], d["rotation"], d["weight"], **case["args"])]
+        want += O.sample_depthwise_backward(d["grad_output"], d["input"], d["rotation"], d["weight"], **case["args"])
+        return zip(("output", "grad_input", "grad_rotation", "grad_weight"), (y.detach(),) + torch.autograd.grad(y, [x, r, wt], dy), want)
+    for name, g, v in run(half):
+        err = float((g.double().cpu() - v).norm() / v.norm())
+        assert err < 2.5e-4, "%s %.2e" % (name, err)
+    half["input"] = half["input"] * 128
+    half["grad_output"] = half["grad_output"] * 128
+    half["weight"] = half["weight"] / 128
+    assert float(half["input"].abs().max()) * float(half["grad_output"].abs().max()) > 65504
+    for name, g, v in run(half):
+        if name == "grad_rotation":
+            assert float((g.double().cpu() - v).norm() / v.norm()) < 2.5e-4
 
 
 def test_offsets_that_sample_nothing():
