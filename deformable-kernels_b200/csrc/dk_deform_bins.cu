@@ -29,6 +29,11 @@ struct BinPlan {
   size_t starts_bytes, recs_bytes, dyt_bytes, bytes, xt_bytes, bankt_bytes, all_bytes, sort_smem, gather_smem;
 };
 
+// The bank in channel order: [scH + 2][scW + 2] cells with a border of zeros, and behind them as many zeros as the four cells of a
+// sample span, for samples that are not used (zero weights alone would let a cell that is not finite through).
+__host__ __device__ inline int bank_unused_cell(const Geom& g) { return (g.scH + 2) * (g.scW + 2); }
+__host__ __device__ inline int bank_cells(const Geom& g) { return bank_unused_cell(g) + g.scW + 4; }
+
 // one sample point: corner coefficients of the image and of the bank, {bank cell * 32, column of the cell, pixel * Cp, 0}
 struct Rec {
   float4 ci, cb;
@@ -103,7 +108,7 @@ __device__ __forceinline__ void move_channels(const T* __restrict__ src, T* __re
 // share the prefix sums (an eighth of the cells each, through distributed shared memory), then every block places its samples.
 // The clusters beyond the first (or, where they are few, all blocks before they sort) bring dy, x and the bank into the order
 // in which the channels of a pixel or cell are neighbours: [P + 1][Cp] and [H W + 1][Cp] with a last pixel of zeros, and
-// [scH + 2][scW + 2][Cp] with a border of zeros.  x and the bank only where the other gradients want them.
+// [bank_cells][Cp].  x and the bank only where the other gradients want them.
 template <typename T>
 __global__ void __launch_bounds__(kSortThreads, 2) dcn_bins_kernel(const T* __restrict__ dy, const T* __restrict__ off,
                                                                 const T* __restrict__ rot, int* __restrict__ starts,
@@ -118,7 +123,7 @@ __global__ void __launch_bounds__(kSortThreads, 2) dcn_bins_kernel(const T* __re
   if (dyt != nullptr) move_channels(dy, dyt, g.P, g, t, tile);
   if (xt != nullptr) {
     move_channels(x, xt, g.HW, g, t, tile);
-    const int cells = (g.scH + 2) * (g.scW + 2);
+    const int cells = bank_cells(g);
     for (int i = (blockIdx.x - t.movers) * kSortThreads + tid; i >= 0 && i < cells * t.Cp; i += (gridDim.x - t.movers) * kSortThreads) {
       const int cell = i / t.Cp, c = i - cell * t.Cp, a = cell / (g.scW + 2) - 1, b = cell - (a + 1) * (g.scW + 2) - 1;
       bankt[i] = c < g.C && a >= 0 && a < g.scH && b >= 0 && b < g.scW ? ld<float>(w + (size_t)c * g.cells + a * g.scW + b) : 0.f;
@@ -219,9 +224,9 @@ __global__ void __launch_bounds__(32 * kGatherWarps, 3) dcn_gather_kernel(const 
   const int c0 = blockIdx.y * CB, n_c = min(CB, g.C - c0), bw = g.scW + 2, W1 = g.W + 1;
   float4* stage = smem4 + warp * 96;                                   // [32 records]
   float* bank = reinterpret_cast<float*>(smem4 + kGatherWarps * 96);   // [cell of the zero-bordered bank][channel]
-  float* seam = bank + (g.scH + 2) * bw * CB;                          // [row of cells][piece][upper | lower][channel]
+  float* seam = bank + bank_cells(g) * CB;                          // [row of cells][piece][upper | lower][channel]
   float* acc = seam + (t.R + 1) * t.segs * 2 * CB;                     // [row][column][PITCH]
-  for (int i = threadIdx.x; i < (g.scH + 2) * bw * CB; i += 32 * kGatherWarps) {
+  for (int i = threadIdx.x; i < bank_cells(g) * CB; i += 32 * kGatherWarps) {
     const int cell = i / CB, a = cell / bw - 1, b = cell - (a + 1) * bw - 1, c = i % CB;
     bank[i] = (c < n_c && a >= 0 && a < g.scH && b >= 0 && b < g.scW) ? ld<float>(w + (size_t)(c0 + c) * g.cells + a * g.scW + b) : 0.f;
   }
@@ -262,7 +267,7 @@ __global__ void __launch_bounds__(32 * kGatherWarps, 3) dcn_gather_kernel(const 
         for (int j = 0; j < V; ++j) cu[j] = s01[j], cl[j] = s11[j], s00[j] = s01[j] = s10[j] = s11[j] = 0.f;
         ++cur;
       };
-      // records beyond the last one: no weight, the zero pixel, no new cell
+      // records beyond the last one: no weight, the zero pixel, zero cells of the bank, no new cell
       float4 next[3];
       auto fetch = [&](int at) {
         const int lim = (last - at) * 3;
@@ -270,7 +275,7 @@ __global__ void __launch_bounds__(32 * kGatherWarps, 3) dcn_gather_kernel(const 
         for (int j = 0; j < 3; ++j) {
           const int e = lane + 32 * j;
           next[j] = e < lim ? __ldg(rc_n + (size_t)at * 3 + e) : none;
-          if (e >= lim && e % 3 == 2) next[j].z = __int_as_float(g.P * t.Cp);
+          if (e >= lim && e % 3 == 2) next[j].x = __int_as_float(bank_unused_cell(g) * 32), next[j].z = __int_as_float(g.P * t.Cp);
         }
       };
       if (first < last) fetch(first);
@@ -348,7 +353,7 @@ __device__ __forceinline__ void tap_record(int flat, int total, int tap, const T
   TapRec r;
   const unsigned px_bytes = Cp * (unsigned)sizeof(T);
   const int nothing = (int)(g.HW * px_bytes);  // the zero pixels of the first sample
-  r.idx = make_int4(nothing, nothing, nothing, nothing), r.im = r.a = r.b = zero, r.at = make_int4((int)(g.P * px_bytes), 0, 0, 0);
+  r.idx = make_int4(nothing, nothing, nothing, nothing), r.im = r.a = r.b = zero, r.at = make_int4((int)(g.P * px_bytes), bank_unused_cell(g) * Cp * (int)sizeof(float), 0, 0);
   if (flat < total) {
     const int n = flat / g.P, p = flat - n * g.P;
     Point q;
@@ -519,11 +524,45 @@ __global__ void __launch_bounds__(32 * kRowWarps, 3) dcn_coords_kernel(const T* 
   }
 }
 
+// The units of a warp of dcn_bank_kernel again, each product to the four cells of its sample only: what a block whose sums are not
+// finite does, because products that are not finite would reach all cells (times a hat of zero).  acc: [cell][channel], the lane's.
+template <typename T, int V>
+__device__ __noinline__ void rows_bank_by_cells(float* acc, const T* __restrict__ dyt, const T* __restrict__ xt, const T* __restrict__ off,
+                                                const T* __restrict__ rot, const Geom& g, int Cp, int c, int warp) {
+  constexpr int CB = 32 * V;
+  for (int i = 0; i < 16; ++i)
+    for (int e = 0; e < V; ++e) acc[i * CB + e] = 0.f;
+  const int total = g.N * g.P, tiles = (total + 31) / 32;
+  for (int u = blockIdx.x * kRowWarps + warp; u < g.taps * tiles; u += gridDim.x * kRowWarps) {
+    const int tap = u / tiles, flat0 = (u - tap * tiles) * 32, cnt = min(32, total - flat0);
+    for (int j = 0; j < cnt; ++j) {
+      const int n = (flat0 + j) / g.P, pix = flat0 + j - n * g.P;
+      Point q;
+      if (!sample_point(n, tap, pix, off, rot, g, q)) continue;
+      for (int e = 0; e < V; ++e) {
+        float xs = 0.f;
+        for (int k = 0; k < 4; ++k) {
+          const int ih = q.h0 + (k >> 1), iw = q.w0 + (k & 1);
+          if (ih >= 0 && ih < g.H && iw >= 0 && iw < g.W)
+            xs = fmaf((k >> 1 ? q.lh : 1.f - q.lh) * (k & 1 ? q.lw : 1.f - q.lw),
+                      static_cast<float>(xt[((size_t)n * (g.HW + 1) + ih * g.W + iw) * Cp + c + e]), xs);
+        }
+        const float dk = static_cast<float>(dyt[((size_t)n * (g.P + 1) + pix) * Cp + c + e]) * xs;
+        for (int k = 0; k < 4; ++k) {
+          const int a = q.u0 + (k >> 1), b = q.v0 + (k & 1);
+          if (a >= 0 && a < g.scH && b >= 0 && b < g.scW)
+            acc[(a * 4 + b) * CB + e] += (k >> 1 ? q.lu : 1.f - q.lu) * (k & 1 ? q.lv : 1.f - q.lv) * dk;
+        }
+      }
+    }
+  }
+}
+
 // Bank gradient, dense in up to 4 x 4 cells (deform_bank_kernel with the samples taken by the lanes that use them).
 template <typename T, int V>
 __global__ void __launch_bounds__(32 * kRowWarps, 2) dcn_bank_kernel(const T* __restrict__ dyt, const T* __restrict__ xt,
                                                                      const T* __restrict__ off, const T* __restrict__ rot,
-                                                                     float* __restrict__ partial, const Geom g, const int Cp) {
+                                                                     float* __restrict__ partial, const __grid_constant__ Geom g, const int Cp) {
   constexpr int CB = 32 * V;
   __shared__ __align__(16) float room[kRowWarps * 16 * CB > kRowWarps * 32 * 20 ? kRowWarps * 16 * CB : kRowWarps * 32 * 20];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, c0 = blockIdx.y * CB, cb = (c0 + V * lane) * (int)sizeof(T);
@@ -561,16 +600,26 @@ __global__ void __launch_bounds__(32 * kRowWarps, 2) dcn_bank_kernel(const T* __
       }
     }
   }
-  __syncthreads();
+  bool finite = true;
 #pragma unroll
-  for (int e = 0; e < V; ++e) {
+  for (int e = 0; e < V; ++e)
 #pragma unroll
     for (int i = 0; i < 8; ++i) {
       const float2 v = unpair(acc[e][i >> 2][i & 3]);
-      const int cell = (i >> 2) * 8 + (i & 3);
-      room[(warp * 16 + cell) * CB + V * lane + e] = v.x;
-      room[(warp * 16 + cell + 4) * CB + V * lane + e] = v.y;
+      finite &= fabsf(v.x) < INFINITY && fabsf(v.y) < INFINITY;
     }
+  if (__syncthreads_or(!finite)) {
+    rows_bank_by_cells<T, V>(room + warp * 16 * CB + V * lane, dyt, xt, off, rot, g, Cp, c0 + V * lane, warp);
+  } else {
+#pragma unroll
+    for (int e = 0; e < V; ++e)
+#pragma unroll
+      for (int i = 0; i < 8; ++i) {
+        const float2 v = unpair(acc[e][i >> 2][i & 3]);
+        const int cell = (i >> 2) * 8 + (i & 3);
+        room[(warp * 16 + cell) * CB + V * lane + e] = v.x;
+        room[(warp * 16 + cell + 4) * CB + V * lane + e] = v.y;
+      }
   }
   __syncthreads();
   for (int i = threadIdx.x; i < 16 * CB; i += 32 * kRowWarps) {
@@ -614,7 +663,7 @@ bool bin_plan(const Geom& g, size_t elem, BinPlan& t) {
   if ((long long)g.N * (t.Cp / 32) * (g.P / kMovePixels + 1) > 0x3fffffff) return false;
   t.bins = (int)bins, t.rec_per_n = (int)recs;
   t.sort_smem = (size_t)t.bins * 4;
-  t.gather_smem = (size_t)kGatherWarps * 1536 + ((size_t)(g.scH + 2) * (g.scW + 2) * 32 * t.V + (size_t)(t.R + 1) * t.segs * 64 * t.V) * 4 + (size_t)t.R * row;
+  t.gather_smem = (size_t)kGatherWarps * 1536 + ((size_t)bank_cells(g) * 32 * t.V + (size_t)(t.R + 1) * t.segs * 64 * t.V) * 4 + (size_t)t.R * row;
   if (t.gather_smem > 110 * 1024 || (long long)g.N * t.bands > 0x7fffffff || (long long)g.N * kSortBlocks > 0x3fffffff) return false;
   t.starts_bytes = round256((size_t)g.N * (t.bins + 1) * sizeof(int));
   t.recs_bytes = round256((size_t)g.N * t.rec_per_n * sizeof(Rec));
@@ -626,7 +675,7 @@ bool bin_plan(const Geom& g, size_t elem, BinPlan& t) {
   if (t.bank_blocks < 1) t.bank_blocks = 1;
   if (t.bank_blocks > most) t.bank_blocks = (int)most;
   t.xt_bytes = round256((size_t)g.N * (g.HW + 1) * t.Cp * elem);
-  t.bankt_bytes = round256((size_t)(g.scH + 2) * (g.scW + 2) * t.Cp * sizeof(float));
+  t.bankt_bytes = round256((size_t)bank_cells(g) * t.Cp * sizeof(float));
   t.all_bytes = t.bytes + t.xt_bytes + t.bankt_bytes + (size_t)t.bank_blocks * g.C * g.cells * sizeof(float);
   return true;
 }

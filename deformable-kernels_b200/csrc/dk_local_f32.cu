@@ -118,12 +118,74 @@ __device__ __forceinline__ void stage_tile(float* xs, float* ys, const T* __rest
 }
 
 // ------------------------------------------------------------------ bank
+// Dense in the cells, a product dy x that is not finite reaches all cells of its channel (times a hat of zero) where only those of its
+// sample should have it.  A block whose sums are not finite starts again with this: one product to the four cells it belongs to.
+// acc: the lane's sums, [cell 4 x 4][32].
+__device__ __forceinline__ void add_to_cells(float* acc, float dk, float u, float v, const Geom& g) {
+  if (!(u > -1.f && v > -1.f && u < (float)g.scH && v < (float)g.scW)) return;
+  const int a0 = (int)floorf(u), b0 = (int)floorf(v);
+#pragma unroll
+  for (int q = 0; q < 4; ++q) {
+    const int a = a0 + (q >> 1), b = b0 + (q & 1);
+    if (a >= 0 && a < g.scH && b >= 0 && b < g.scW) acc[(a * 4 + b) * 32] += hat1(u - (float)a) * hat1(v - (float)b) * dk;
+  }
+}
+
+// All tiles of a block, a pixel per warp; bilinear samples of x at `off`, or x itself (off null).  red: [warp][cell][lane].
+template <typename T>
+__device__ __noinline__ void bank_by_cells(float* red, const T* __restrict__ dy, const T* __restrict__ x, const T* __restrict__ off,
+                                           const T* __restrict__ rot, const Geom& g, const TilePlan& t, int c0, int warp, int warps, int lane) {
+  float* acc = red + warp * 512 + lane;
+  for (int i = 0; i < 16; ++i) acc[i * 32] = 0.f;
+  if (c0 + lane >= g.C) return;
+  const float uh0 = 0.5f * (float)(g.scH - 3), uw0 = 0.5f * (float)(g.scW - 3);
+  const int first = blockIdx.x * t.per_block, last = min(first + t.per_block, t.tiles);
+  for (int tile = first; tile < last; ++tile) {
+    const TilePos tp = tile_pos(tile, t);
+    const T* xc = x + ((size_t)tp.n * g.C + c0 + lane) * g.HW;
+    for (int p = warp; p < t.TH * t.TW; p += warps) {
+      const int oh = tp.oh0 + p / t.TW, ow = tp.ow0 + p % t.TW;
+      if (oh >= g.Ho || ow >= g.Wo) continue;
+      const int pix = oh * g.Wo + ow;
+      const float yv = ld<float>(dy + ((size_t)tp.n * g.C + c0 + lane) * g.P + pix);
+      for (int tap = 0; tap < 9; ++tap) {
+        const int fh = tap / 3, fw = tap - fh * 3, ih = oh * g.sH - g.pH + fh * g.dH, iw = ow * g.sW - g.pW + fw * g.dW;
+        const size_t o = ((size_t)tp.n * 18 + 2 * tap) * g.P + pix;
+        float xv = 0.f;
+        if (off != nullptr) {
+          Bilinear<float> bi;
+          if (!image_setup<float>((float)ih + ld<float>(off + o), (float)iw + ld<float>(off + o + g.P), g, bi)) continue;
+          float sc[4];
+          bilinear_value_coefs(bi, sc);
+#pragma unroll
+          for (int q = 0; q < 4; ++q)
+            if (bi.m[q]) xv = fmaf(sc[q], ld<float>(xc + bi.idx[q]), xv);
+        } else {
+          if (ih < 0 || ih >= g.H || iw < 0 || iw >= g.W) continue;
+          xv = ld<float>(xc + ih * g.W + iw);
+        }
+        add_to_cells(acc, yv * xv, ((float)fh + ld<float>(rot + o)) + uh0, ((float)fw + ld<float>(rot + o + g.P)) + uw0, g);
+      }
+    }
+  }
+}
+
+__device__ __forceinline__ bool all_finite(const unsigned long long (&acc)[2][4]) {
+  bool ok = true;
+#pragma unroll
+  for (int i = 0; i < 8; ++i) {
+    const float2 v = unpair(acc[i >> 2][i & 3]);
+    ok &= fabsf(v.x) < INFINITY && fabsf(v.y) < INFINITY;
+  }
+  return ok;
+}
+
 constexpr int kBankWarps = 8;
 
 template <typename T, int S>
 __global__ void __launch_bounds__(32 * kBankWarps, 2) f32_bank_kernel(const T* __restrict__ dy, const T* __restrict__ x,
                                                                       const T* __restrict__ rot, float* __restrict__ partial,
-                                                                      const Geom g, const TilePlan t) {
+                                                                      const __grid_constant__ Geom g, const __grid_constant__ TilePlan t) {
   extern __shared__ __align__(16) float smem_f[];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int c0 = blockIdx.y * 32, px = t.TH * t.TW;
@@ -176,14 +238,17 @@ __global__ void __launch_bounds__(32 * kBankWarps, 2) f32_bank_kernel(const T* _
       }
     }
   }
-  __syncthreads();
   float* red = smem_f;  // [warp][cell][lane]
+  if (__syncthreads_or(!all_finite(acc))) {
+    bank_by_cells<T>(red, dy, x, nullptr, rot, g, t, c0, warp, kBankWarps, lane);
+  } else {
 #pragma unroll
-  for (int i = 0; i < 8; ++i) {
-    const float2 v = unpair(acc[i >> 2][i & 3]);
-    const int cell = (i >> 2) * 8 + (i & 3);
-    red[(warp * 16 + cell) * 32 + lane] = v.x;
-    red[(warp * 16 + cell + 4) * 32 + lane] = v.y;
+    for (int i = 0; i < 8; ++i) {
+      const float2 v = unpair(acc[i >> 2][i & 3]);
+      const int cell = (i >> 2) * 8 + (i & 3);
+      red[(warp * 16 + cell) * 32 + lane] = v.x;
+      red[(warp * 16 + cell + 4) * 32 + lane] = v.y;
+    }
   }
   __syncthreads();
   for (int i = threadIdx.x; i < 32 * 16; i += 32 * kBankWarps) {
@@ -332,7 +397,8 @@ constexpr int kSamplePitch = 32 * 9 + 1;
 template <typename T>
 __global__ void __launch_bounds__(32 * kTapWarps, 2) deform_bank_kernel(const T* __restrict__ dy, const T* __restrict__ x,
                                                                         const T* __restrict__ off, const T* __restrict__ rot,
-                                                                        float* __restrict__ partial, const Geom g, const TilePlan t) {
+                                                                        float* __restrict__ partial, const __grid_constant__ Geom g,
+                                                                        const __grid_constant__ TilePlan t) {
   extern __shared__ __align__(16) float smem_f[];
   const int lane = threadIdx.x & 31, tap = threadIdx.x >> 5;
   const int c0 = blockIdx.y * 32, n_c = min(32, g.C - c0), px = t.TH * t.TW;
@@ -406,14 +472,17 @@ __global__ void __launch_bounds__(32 * kTapWarps, 2) deform_bank_kernel(const T*
       }
     }
   }
-  __syncthreads();
   float* red = smem_f;  // [warp][cell][lane]
+  if (__syncthreads_or(!all_finite(acc))) {
+    bank_by_cells<T>(red, dy, x, off, rot, g, t, c0, tap, kTapWarps, lane);
+  } else {
 #pragma unroll
-  for (int i = 0; i < 8; ++i) {
-    const float2 v = unpair(acc[i >> 2][i & 3]);
-    const int cell = (i >> 2) * 8 + (i & 3);
-    red[(tap * 16 + cell) * 32 + lane] = v.x;
-    red[(tap * 16 + cell + 4) * 32 + lane] = v.y;
+    for (int i = 0; i < 8; ++i) {
+      const float2 v = unpair(acc[i >> 2][i & 3]);
+      const int cell = (i >> 2) * 8 + (i & 3);
+      red[(tap * 16 + cell) * 32 + lane] = v.x;
+      red[(tap * 16 + cell + 4) * 32 + lane] = v.y;
+    }
   }
   __syncthreads();
   for (int i = threadIdx.x; i < 32 * 16; i += 32 * kTapWarps) {

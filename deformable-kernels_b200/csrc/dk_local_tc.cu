@@ -253,12 +253,15 @@ constexpr float kUnbias = 4.1e-8f;
 
 // The 16 cells of one channel into the columns at `a` as fp16 pieces of 8 columns (two cells each): the values, or for fp32 their
 // upper and lower parts and, scaled by 2^15, what those leave.  Returns what undoes the scaling of fp32 banks and of the hat
-// products they meet.
+// products they meet; `finite` is cleared where a value is not.
 template <typename T>
-__device__ __forceinline__ float bank_to_tmem(unsigned a, const T* __restrict__ w, int cells, bool ok) {
+__device__ __forceinline__ float bank_to_tmem(unsigned a, const T* __restrict__ w, int cells, bool ok, bool& finite) {
   float v[16], inv = 1.f;
 #pragma unroll
-  for (int i = 0; i < 16; ++i) v[i] = ok && i < cells ? ld<float>(w + i) : 0.f;
+  for (int i = 0; i < 16; ++i) {
+    v[i] = ok && i < cells ? ld<float>(w + i) : 0.f;
+    finite &= fabsf(v[i]) < INFINITY;
+  }
   if constexpr (std::is_same<T, float>::value) {
     float top = 0.f;
 #pragma unroll
@@ -437,6 +440,50 @@ __device__ __forceinline__ void copy_row(char* slot, const T* __restrict__ src, 
   }
 }
 
+// ------------------------------------------------------------------ banks with values that are not finite
+// Products with a hat of zero would carry such a value to every output of its channel.  A block that finds one among its
+// channels' cells gathers the four cells of a sample instead, a lane per output.
+template <typename T, int MODE>
+__device__ __noinline__ void gather_block(const T* __restrict__ src, const T* __restrict__ rot, const T* __restrict__ bank,
+                                          T* __restrict__ dst, const ConvParams& p, int c0, int cg, int lo, int hi) {
+  constexpr bool kData = MODE == kData1 || MODE == kData2;
+  constexpr int S = MODE == kFwd2 || MODE == kData2 ? 2 : 1, PX = MODE == kData2 ? 32 : 8;  // destination pixels of a segment
+  const int scH = p.cells / p.scW, px = (hi - lo) * PX, P = p.Ho * p.Wo;
+#pragma unroll 1
+  for (int c = c0; c < c0 + cg; ++c) {
+    const T* w = bank + (size_t)c * p.cells;
+#pragma unroll 1
+    for (int i = threadIdx.x; i < px; i += kThreads) {
+      const SegPos sp = seg_pos(lo + i / PX, p);
+      const int k = i % PX, oh = MODE == kData2 ? 2 * sp.g + (k >> 4) : sp.g, ow = MODE == kData2 ? 16 * sp.s + (k & 15) : 8 * sp.s + k;
+      if (oh >= p.Hd || ow >= p.Wd) continue;
+      const T* plane = src + ((size_t)sp.n * p.C + c) * p.Hs * p.Ws;
+      float acc = 0.f;
+#pragma unroll 1
+      for (int tap = 0; tap < 9; ++tap) {
+        const int fh = tap / 3, fw = tap - fh * 3;
+        int sh = kData ? oh + 1 - fh : oh * S - 1 + fh, sw = kData ? ow + 1 - fw : ow * S - 1 + fw;
+        if (sh < 0 || sw < 0 || (kData && S == 2 && ((sh | sw) & 1))) continue;
+        if (kData && S == 2) sh >>= 1, sw >>= 1;
+        if (sh >= p.Hs || sw >= p.Ws) continue;
+        const T* r = rot + ((size_t)sp.n * 18 + 2 * tap) * P + (kData ? sh * p.Wo + sw : oh * p.Wo + ow);
+        const float u = ld<float>(r) + ((float)fh + p.uh0), v = ld<float>(r + P) + ((float)fw + p.uw0);
+        float kv = 0.f;
+        if (u > -1.f && v > -1.f && u < (float)scH && v < (float)p.scW) {
+          const float fu = floorf(u), fv = floorf(v);
+#pragma unroll 1
+          for (int q = 0; q < 4; ++q) {
+            const int a = (int)fu + (q >> 1), b = (int)fv + (q & 1);
+            if (a >= 0 && a < scH && b >= 0 && b < p.scW) kv = fmaf(hat(u - (float)a) * hat(v - (float)b), ld<float>(w + a * p.scW + b), kv);
+          }
+        }
+        acc = fmaf(ld<float>(plane + (size_t)sh * p.Ws + sw), kv, acc);
+      }
+      st<T, float>(dst + (((size_t)sp.n * p.C + c) * p.Hd + oh) * p.Wd + ow, acc);
+    }
+  }
+}
+
 // ------------------------------------------------------------------ forward and grad-input
 // d = bank at a (its pieces 8 columns apart) * hat products at b (kPiece apart), the smallest products first
 template <typename T, bool FULL>
@@ -476,7 +523,7 @@ __host__ __device__ inline ConvSmem conv_smem(unsigned ring_bytes, int groups, i
 template <typename T, int MODE, bool SC44, int NL, bool FULL>
 __global__ void __launch_bounds__(kThreads, 1)
     tc_conv_kernel(const __grid_constant__ CUtensorMap tm, const T* __restrict__ src, const T* __restrict__ rot,
-                   const T* __restrict__ bank, T* __restrict__ dst, const ConvParams p) {
+                   const T* __restrict__ bank, T* __restrict__ dst, const __grid_constant__ ConvParams p) {
   extern __shared__ __align__(1024) char smem[];
   using Wk = Walk<MODE>;
   constexpr bool STAGED = MODE != kData2, SCALED = sizeof(T) == 4;
@@ -493,7 +540,7 @@ __global__ void __launch_bounds__(kThreads, 1)
   const unsigned b_free = b_full + 8 * kMaxBuf, t_full = b_free + 8 * kMaxBuf, t_empty = t_full + 16, o_full = t_empty + 16,
                  o_free = o_full + 8;
   float* inv_s = reinterpret_cast<float*>(smem + sm.inv);
-  volatile int* tail = reinterpret_cast<volatile int*>(smem + sm.bars + kBars * 8);  // TMEM address, abort flag
+  volatile int* tail = reinterpret_cast<volatile int*>(smem + sm.bars + kBars * 8);  // TMEM address, abort flag, a bank that is not finite
 
   const int lo = blockIdx.x * p.steps_per_cta * kStepSegs, hi = min(lo + p.steps_per_cta * kStepSegs, p.segs);
   const int steps = (hi - lo + kStepSegs - 1) / kStepSegs;
@@ -525,7 +572,7 @@ __global__ void __launch_bounds__(kThreads, 1)
     mbar_init(o_full, kConsumers);
     mbar_init(o_free, NS);
     fence_barrier_init();
-    tail[1] = 0;
+    tail[1] = tail[2] = 0;
   }
   if (warp == kConsumers) tmem_alloc_all(smem_u32(const_cast<int*>(tail)));
   fence_before();
@@ -543,9 +590,11 @@ __global__ void __launch_bounds__(kThreads, 1)
       }
       const int ch = grp * 32 + lane;
       const bool ok = grp >= 0 && ch < cg;
+      bool finite = true;
       const float inv = bank_to_tmem<T>(tmem + ((unsigned)(q * 32) << 16) + kBankCol + i * TILE, bank + (size_t)(c0 + (ok ? ch : 0)) * p.cells,
-                                        p.cells, ok);
+                                        p.cells, ok, finite);
       if (SCALED && grp >= 0) inv_s[grp * 32 + lane] = inv;
+      if (FULL && !finite) tail[2] = 1;
     }
     wait_st();
   }
@@ -553,7 +602,9 @@ __global__ void __launch_bounds__(kThreads, 1)
   __syncthreads();
   fence_after();
 
-  if (warp < kConsumers) {
+  if (FULL && tail[2]) {
+    gather_block<T, MODE>(src, rot, bank, dst, p, c0, cg, lo, hi);
+  } else if (warp < kConsumers) {
     // ================================================================ consumers
     regs_inc<consumer_regs<FULL>()>();
     const int q = warp & 3, team = warp >> 2;

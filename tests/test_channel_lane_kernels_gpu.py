@@ -96,6 +96,35 @@ def test_wide_range_inside_a_channel(stride):
         assert float(over.max()) <= 0
 
 
+@pytest.mark.parametrize("dtype", [torch.float32, torch.float16])
+@pytest.mark.parametrize("c,h,w,stride", [(40, 9, 24, 1), (40, 10, 24, 2), (136, 7, 28, 1), (24, 9, 13, 2)])
+def test_values_that_are_not_finite_stay_where_they_belong(c, h, w, stride, dtype):
+    """Wherever the oracle is finite, results are finite and agree: a bank cell reaches the outputs and gradients of the samples that
+    touch it, an input or upstream gradient the cells that its samples touch (kernel offsets near 1/4, so that each tap touches four
+    known cells, and the taps in the padding none)."""
+    from deformable_kernels.ops.deform_kernel.functions import sample_depthwise
+    from oracle import dk_oracle as O
+    case = make_case(2, c, h, w, stride=stride, rot_std=0.05, seed=21)
+    case["rotation"] += 0.25
+    case["weight"][5, 0, 0, 0], case["weight"][c - 1, 0, 2, 1] = float("inf"), float("nan")
+    case["grad_output"][0, 3, 0, 0], case["input"][1, 9, 0, 0] = float("inf"), -float("inf")
+    a = {k: case[k].to(dtype) for k in ("input", "rotation", "weight", "grad_output")}
+    x, r, wt, dy = (a[k].to(DEV) for k in ("input", "rotation", "weight", "grad_output"))
+    for t in (x, r, wt):
+        t.requires_grad_(True)
+    y = sample_depthwise(x, r, wt, **case["args"])
+    got = (y.detach(),) + torch.autograd.grad(y, [x, r, wt], dy)
+    d = {k: v.double() for k, v in a.items()}
+    want = [O.sample_depthwise_forward(d["input"], d["rotation"], d["weight"], **case["args"])]
+    want += O.sample_depthwise_backward(d["grad_output"], d["input"], d["rotation"], d["weight"], **case["args"])
+    for g, v in zip(got, want):
+        ok = torch.isfinite(v)
+        assert 0 < int((~ok).sum()) and int(ok.sum()) > v.numel() // 4
+        g = g.double().cpu()
+        assert torch.isfinite(g[ok]).all()
+        assert float((g[ok] - v[ok]).norm() / v[ok].norm()) < (2e-3 if dtype == torch.float16 else 1e-5)
+
+
 def _flat(t, skip):
     """A copy of t that starts `skip` elements into its storage."""
     out = torch.empty(t.numel() + skip, dtype=t.dtype, device=t.device)[skip:].view(t.shape)

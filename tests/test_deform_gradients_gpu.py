@@ -60,3 +60,32 @@ def test_without_kernel_offsets(c, scope, dtype):
     b = deform_sample_depthwise(x, o, None, wt, **case["args"])
     for p, q in zip((a, *torch.autograd.grad(a, leaves, dy)), (b, *torch.autograd.grad(b, leaves, dy))):
         assert rel_err(q, p) < (2e-3 if dtype == torch.float16 else 1e-5)
+
+
+@pytest.mark.parametrize("c", [40, 24, 104])
+@pytest.mark.parametrize("dtype", [torch.float32, torch.float16])
+def test_values_that_are_not_finite_stay_where_they_belong(c, dtype):
+    """Wherever the oracle is finite, all gradients together and the bank gradient alone are finite and agree (offsets that leave the
+    first row and column of taps of an image outside it, and let each tap touch four known cells of the bank)."""
+    from deformable_kernels.ops.deform_kernel.functions import deform_sample_depthwise
+    from oracle import dk_oracle as O
+    case = make_case(2, c, 12, 9, rot_std=0.05, off_std=0.05, seed=22)
+    case["rotation"] += 0.25
+    case["offset"] -= 0.3
+    case["weight"][5, 0, 0, 0] = float("inf")
+    case["grad_output"][0, 3, 0, 0], case["input"][1, 9, 0, 0] = float("inf"), -float("inf")
+    a = [case[k].to(dtype) for k in ("grad_output", "input", "offset", "rotation", "weight")]
+    dy, *leaves = (t.to(DEV) for t in a)
+    for t in leaves:
+        t.requires_grad_(True)
+    y = deform_sample_depthwise(*leaves, **case["args"])
+    got = (y.detach(),) + torch.autograd.grad(y, leaves, dy)
+    d = [t.double() for t in a]
+    want = (O.deform_sample_depthwise_forward(*d[1:], **case["args"]), *O.deform_sample_depthwise_backward(*d, **case["args"]))
+    alone, = torch.autograd.grad(deform_sample_depthwise(*[t.detach() for t in leaves[:3]], leaves[3], **case["args"]), [leaves[3]], dy)
+    for g, v in zip((*got, alone), (*want, want[-1])):
+        ok = torch.isfinite(v)
+        assert 0 < int((~ok).sum()) and int(ok.sum()) > v.numel() // 4
+        g = g.double().cpu()
+        assert torch.isfinite(g[ok]).all()
+        assert float((g[ok] - v[ok]).norm() / v[ok].norm()) < (2e-3 if dtype == torch.float16 else 1e-5)
