@@ -28,8 +28,8 @@
 //   1 MMA warp         issues the tcgen05.mma, two sets of accumulators
 //   1 or 3 loaders     source rows through a ring of row slots: TMA where rows are multiples of 16 bytes (out-of-range
 //                      elements arrive as zeros = the convolution padding), else cp.async pieces or elements, 3 warps
-//   6 or 4 beta warps  lane = destination pixel: 18 offsets, nine taps of 16 hat products, written as the B operand
-//   4 or 6 store warps results of a step from shared memory, consecutive pixels on consecutive lanes (written straight from
+//   6 or 4 hat warps   lane = destination pixel: offsets, taps of 16 hat products each, written as the B operand
+//   4 store warps      results of a step from shared memory, consecutive pixels on consecutive lanes (written straight from
 //                      the consumers' registers, one channel per lane, every store touches 32 lines)
 // Every hand-over is an mbarrier used once per step (or per set of accumulators) by the same warps, in order.
 #include <atomic>
@@ -53,37 +53,37 @@ constexpr int kConsumers = 16;
 constexpr int kHelpers = 12;  // MMA, loaders, hat products, stores
 constexpr int kThreads = 32 * (kConsumers + kHelpers);
 // Registers per thread: 72 at launch, then more for the four consumer warpgroups than for the three of the helpers.  Consumers of
-// fp16 kernel values hold two items; of fp32 values (FULL) one, and the hat products need what that leaves.
+// fp16 kernel values hold two items; of fp32 values (FULL) one, and with one loader the hat products get what that leaves (with
+// three, 88 / 48 is the faster split: 32 x 384 of 14 x 14 47 -> 45 us).
 constexpr int kRegsLaunch = 72;
-template <bool FULL>
+template <bool FULL, int NL>
 __host__ __device__ constexpr int consumer_regs() {
-  return FULL ? 80 : 88;
+  return FULL && NL == 1 ? 80 : 88;
 }
-template <bool FULL>
+template <bool FULL, int NL>
 __host__ __device__ constexpr int helper_regs() {
-  return FULL ? 56 : 48;
+  return FULL && NL == 1 ? 56 : 48;
 }
-template <bool FULL>
-constexpr bool kSharesAdd = kConsumers * consumer_regs<FULL>() + kHelpers * helper_regs<FULL>() <= (kConsumers + kHelpers) * kRegsLaunch;
-static_assert(kSharesAdd<true> && kSharesAdd<false>, "register shares");
+static_assert(kConsumers * consumer_regs<true, 1>() + kHelpers * helper_regs<true, 1>() <= (kConsumers + kHelpers) * kRegsLaunch &&
+                  kConsumers * consumer_regs<false, 1>() + kHelpers * helper_regs<false, 1>() <= (kConsumers + kHelpers) * kRegsLaunch,
+              "register shares");
 constexpr int kLoaders = 3;                         // warps that fetch rows without TMA
 constexpr int kStepSegs = 8;
 constexpr int kSlotCols = 48;                       // three taps x 16 pixels
 constexpr int kSetCols = kTeams * kSlotCols;        // one set of accumulators
 constexpr int kBankCol = 2 * kSetCols;              // the bank behind the two sets
 constexpr int kDepth = 4;                           // steps in flight, as seen by the row ring
-constexpr int kMaxBuf = 3;                          // buffers of hat products
-constexpr int kBars = 2 * kDepth + 2 * kMaxBuf + 6;
 constexpr int kPairRow = 6 * 256;                   // hat products of two segments and one kernel row: 48 columns x 32 bytes
 constexpr int kPiece = 3 * kTeams * kPairRow;       // of a step: [kernel row][pair][segment, tap: 8 columns][two halves of the cells]
 constexpr int kMinSmem = 120 * 1024;                // one block per SM: it takes all of TMEM
 
-// Hat products: two warps per step, each pair of warps with a buffer of its own, so that a warp sees every reuse of its buffer
-// (a barrier's phase can only be told from the one before it).
-template <bool FULL>
-__host__ __device__ constexpr int beta_warps(int loaders) {
-  return loaders == 1 && !FULL ? 6 : 4;
-}
+// Hat products: two buffers, each with two or three warps of its own, so that a warp sees every reuse of its buffer (a barrier's phase
+// can only be told from the one before it).  Two warps take half of a step's pixels each; three, where there is one loader, a kernel
+// row each (three buffers with two warps: fp16, 128 x 96 of 112 x 112 285 / 328 us against 268 / 264; two with two: fp32, 64 x 144 of
+// 56 x 56 178 / 178 against 150 / 148).
+constexpr int kBufs = 2;
+constexpr int kBars = 2 * kDepth + 2 * kBufs + 6;
+__host__ __device__ constexpr int warps_per_buffer(int loaders) { return loaders == 1 ? 3 : 2; }
 
 template <typename T>
 __host__ __device__ constexpr int bank_piece_count() {
@@ -307,33 +307,54 @@ __device__ __forceinline__ void tap_of(int v, int t, int g, int x, int& qh, int&
 }
 
 // 16 hat products of one tap: cells (2i, 2i + 1) in hi[i].  SPLIT (fp32): scaled by 2^15, and what hi leaves of the unrounded
-// products in lo[i].  (Scalar instructions: packed pairs have to be moved into place, the forward of N = 64, C = 144, 56 x 56 took 170 us with them, 156 without.)
+// products in lo[i].  Products in packed pairs only where nothing else is done with them: before the subtraction the pairs have to be
+// moved into place (forward of N = 64, C = 144, 56 x 56 170 us, 156 without).
 template <bool SC44, bool SPLIT>
 __device__ __forceinline__ void hat_products(unsigned (&hi)[8], unsigned (&lo)[8], float u, float v, bool ok, int scW, int cells) {
   constexpr float kScale = SPLIT ? 32768.f : 1.f;
-  float hv4[4];
-  if (SC44) {
+  if constexpr (SC44) {
+    float hv[4];
 #pragma unroll
-    for (int a = 0; a < 4; ++a) hv4[a] = hat(v - (float)a);
-  }
-  float hu4 = 0.f;
-  int a = 0, c = 0;
+    for (int a = 0; a < 4; ++a) hv[a] = hat(v - (float)a);
+    if constexpr (SPLIT) {
 #pragma unroll
-  for (int i = 0; i < 8; ++i) {
-    float hu[2], hv[2];
-    if (SC44) {
-      if (i % 2 == 0) hu4 = ok ? kScale * hat(u - (float)(i / 2)) : 0.f;
-      hu[0] = hu[1] = hu4, hv[0] = hv4[2 * i % 4], hv[1] = hv4[2 * i % 4 + 1];
+      for (int a = 0; a < 4; ++a) {
+        const float hu = ok ? kScale * hat(u - (float)a) : 0.f;
+#pragma unroll
+        for (int k = 0; k < 2; ++k) {
+          const float h0 = hv[2 * k], h1 = hv[2 * k + 1];
+          const unsigned h = hi[2 * a + k] = mma::pack2(hu * h0, hu * h1);
+          lo[2 * a + k] = mma::pack2(fmaf(hu, h0, -mma::lo2f(h)), fmaf(hu, h1, -mma::hi2f(h)));
+        }
+      }
     } else {
+      float hu[4], b[16];
+#pragma unroll
+      for (int a = 0; a < 4; ++a) hu[a] = ok ? hat(u - (float)a) : 0.f;
+      const unsigned long long v01 = pair(hv[0], hv[1]), v23 = pair(hv[2], hv[3]);
+#pragma unroll
+      for (int a = 0; a < 4; ++a) {
+        const unsigned long long uu = pair(hu[a], hu[a]);
+        const float2 r = unpair(mul2(uu, v01)), q = unpair(mul2(uu, v23));
+        b[4 * a] = r.x, b[4 * a + 1] = r.y, b[4 * a + 2] = q.x, b[4 * a + 3] = q.y;
+      }
+#pragma unroll
+      for (int i = 0; i < 8; ++i) hi[i] = mma::pack2(b[2 * i], b[2 * i + 1]);
+    }
+  } else {
+    int a = 0, c = 0;
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+      float hu[2], hv[2];
 #pragma unroll
       for (int k = 0; k < 2; ++k) {
         hu[k] = ok && 2 * i + k < cells ? kScale * hat(u - (float)a) : 0.f;
         hv[k] = hat(v - (float)c);
         if (++c == scW) c = 0, ++a;
       }
+      hi[i] = mma::pack2(hu[0] * hv[0], hu[1] * hv[1]);
+      if (SPLIT) lo[i] = mma::pack2(fmaf(hu[0], hv[0], -mma::lo2f(hi[i])), fmaf(hu[1], hv[1], -mma::hi2f(hi[i])));
     }
-    hi[i] = mma::pack2(hu[0] * hv[0], hu[1] * hv[1]);
-    if (SPLIT) lo[i] = mma::pack2(fmaf(hu[0], hv[0], -mma::lo2f(hi[i])), fmaf(hu[1], hv[1], -mma::hi2f(hi[i])));
   }
 }
 
@@ -341,26 +362,39 @@ __device__ __forceinline__ void sts16(unsigned a, unsigned x, unsigned y, unsign
   asm volatile("st.shared.v4.b32 [%0], {%1,%2,%3,%4};\n" ::"r"(a), "r"(x), "r"(y), "r"(z), "r"(w) : "memory");
 }
 
-// The offsets of one pixel as they lie in memory: nine (vertical, horizontal) pairs; absent ones read as zero.
-template <typename T> struct Offsets {
-  T r[9][2];
+// What a beta warp does in a step, WPB warps sharing it: 18 / WPB pieces of 32 pixels (lane = pixel: segment lane / 8, column lane % 8)
+// and one tap.  Offsets as they lie in memory, (vertical, horizontal); absent ones read as zero.
+template <typename T, int WPB> struct Offsets {
+  static constexpr int kPieces = 18 / WPB;
+  T r[kPieces][2];
   unsigned ok;  // taps whose offsets exist
 };
+template <int WPB>
+__device__ __forceinline__ void piece_of(int i, int w, int& half, int& v, int& t) {
+  half = WPB == 3 ? i / 3 : w, v = WPB == 3 ? w : i / 3, t = i % 3;
+}
 
-// one beta warp: half a step (32 pixels, lane = pixel: segment lane / 8, column lane % 8)
-template <typename T, int MODE>
-__device__ __forceinline__ void fetch_offsets(Offsets<T>& o, const T* __restrict__ rot, int seg, int hi_seg, const ConvParams& p,
-                                              int lane) {
-  const int b = seg + (lane >> 3);
-  const SegPos sp = seg_pos(min(b, hi_seg - 1), p);
-  const int x = sp.s * 8 + (lane & 7), P = p.Ho * p.Wo;
-  const bool live = b < hi_seg && x < p.Wg;
-  const T* rn = rot + (size_t)sp.n * 18 * P;
+template <typename T, int MODE, int WPB>
+__device__ __forceinline__ void fetch_offsets(Offsets<T, WPB>& o, const T* __restrict__ rot, int seg, int hi_seg, const ConvParams& p,
+                                              int w, int lane) {
+  const int P = p.Ho * p.Wo;
+  SegPos sp;
+  int x = 0;
+  const T* rn = rot;
+  bool live = false;
   o.ok = 0;
 #pragma unroll
-  for (int i = 0; i < 9; ++i) {
-    int qh, qw, fh, fw;
-    tap_of<MODE>(i / 3, i % 3, sp.g, x, qh, qw, fh, fw);
+  for (int i = 0; i < Offsets<T, WPB>::kPieces; ++i) {
+    int half, v, t, qh, qw, fh, fw;
+    piece_of<WPB>(i, w, half, v, t);
+    if (i == 0 || (WPB == 3 && i == 3)) {
+      const int b = seg + half * 4 + (lane >> 3);
+      sp = seg_pos(min(b, hi_seg - 1), p);
+      x = sp.s * 8 + (lane & 7);
+      live = b < hi_seg && x < p.Wg;
+      rn = rot + (size_t)sp.n * 18 * P;
+    }
+    tap_of<MODE>(v, t, sp.g, x, qh, qw, fh, fw);
     const bool ok = live && qh >= 0 && qh < p.Ho && qw >= 0 && qw < p.Wo;
     o.ok |= (unsigned)ok << i;
     const T* a = rn + ((fh * 3 + fw) * 2) * P + qh * p.Wo + qw;
@@ -369,20 +403,22 @@ __device__ __forceinline__ void fetch_offsets(Offsets<T>& o, const T* __restrict
   }
 }
 
-template <typename T, int MODE, bool SC44, bool SPLIT>
-__device__ __forceinline__ void write_hats(unsigned buf, const Offsets<T>& o, int half, const ConvParams& p, int lane) {
+template <typename T, int MODE, bool SC44, bool SPLIT, int WPB>
+__device__ __forceinline__ void write_hats(unsigned buf, const Offsets<T, WPB>& o, const ConvParams& p, int w, int lane) {
   const int sl = lane >> 3, px = lane & 7;
   // row of this pixel inside its 8-row core matrix: pixels p and p + 4 are neighbours
-  const unsigned dst = buf + (half * 2 + (sl >> 1)) * kPairRow + (sl & 1) * (3 * 256) + ((px & 3) * 2 + (px >> 2)) * 16;
+  const unsigned dst = buf + (sl >> 1) * kPairRow + (sl & 1) * (3 * 256) + ((px & 3) * 2 + (px >> 2)) * 16;
 #pragma unroll
-  for (int i = 0; i < 9; ++i) {
-    int qh, qw, fh, fw;
-    tap_of<MODE>(i / 3, i % 3, 0, 0, qh, qw, fh, fw);
-    // one rounding: tap + (scope - kernel) / 2 is exact
-    const float u = static_cast<float>(o.r[i][0]) + ((float)fh + p.uh0), w = static_cast<float>(o.r[i][1]) + ((float)fw + p.uw0);
+  for (int i = 0; i < Offsets<T, WPB>::kPieces; ++i) {
+    int half, v, t, qh, qw, fh, fw;
+    piece_of<WPB>(i, w, half, v, t);
+    tap_of<MODE>(v, t, 0, 0, qh, qw, fh, fw);
+    const float ru = static_cast<float>(o.r[i][0]), rv = static_cast<float>(o.r[i][1]);
+    // fp32: one rounding, tap + (scope - kernel) / 2 is exact; with fp16 offsets the reference's order is, too
+    const float u0 = SPLIT ? ru + ((float)fh + p.uh0) : ((float)fh + ru) + p.uh0, v0 = SPLIT ? rv + ((float)fw + p.uw0) : ((float)fw + rv) + p.uw0;
     unsigned hi[8], lo[8];
-    hat_products<SC44, SPLIT>(hi, lo, u, w, (o.ok >> i) & 1, p.scW, p.cells);
-    const unsigned a = dst + (i / 3) * (kTeams * kPairRow) + (i % 3) * 256;
+    hat_products<SC44, SPLIT>(hi, lo, u0, v0, (o.ok >> i) & 1, p.scW, p.cells);
+    const unsigned a = dst + v * (kTeams * kPairRow) + half * (2 * kPairRow) + t * 256;
     sts16(a, hi[0], hi[1], hi[2], hi[3]);
     sts16(a + 128, hi[4], hi[5], hi[6], hi[7]);
     if (SPLIT) {
@@ -508,10 +544,10 @@ struct ConvSmem {  // byte offsets behind the row ring
   unsigned beta, inv, out, segs, bars, total;
 };
 template <typename T, int MODE, bool FULL>
-__host__ __device__ inline ConvSmem conv_smem(unsigned ring_bytes, int groups, int nbuf) {
+__host__ __device__ inline ConvSmem conv_smem(unsigned ring_bytes, int groups) {
   ConvSmem m;
   m.beta = (ring_bytes + 32 + 127) & ~127u;  // 32: what the last channel row's right edge may read
-  m.inv = m.beta + nbuf * kPiece * (FULL ? 2 : 1);
+  m.inv = m.beta + kBufs * kPiece * (FULL ? 2 : 1);
   m.out = m.inv + (sizeof(T) == 4 ? groups * 128 : 0);
   m.segs = m.out + (MODE == kData2 ? 0 : groups * 32 * out_pitch<T>());
   m.bars = m.segs + kDepth * kStepSegs * 16;
@@ -521,23 +557,22 @@ __host__ __device__ inline ConvSmem conv_smem(unsigned ring_bytes, int groups, i
 
 // FULL: the kernel values leave the tensor cores as fp32 (fp32 tensors always)
 template <typename T, int MODE, bool SC44, int NL, bool FULL>
-__global__ void __launch_bounds__(kThreads, 1)
-    tc_conv_kernel(const __grid_constant__ CUtensorMap tm, const T* __restrict__ src, const T* __restrict__ rot,
-                   const T* __restrict__ bank, T* __restrict__ dst, const __grid_constant__ ConvParams p) {
+__device__ __forceinline__ void tc_conv(const CUtensorMap& tm, const T* __restrict__ src, const T* __restrict__ rot,
+                                        const T* __restrict__ bank, T* __restrict__ dst, const ConvParams& p) {
   extern __shared__ __align__(1024) char smem[];
   using Wk = Walk<MODE>;
   constexpr bool STAGED = MODE != kData2, SCALED = sizeof(T) == 4;
   constexpr int PIECES = FULL ? 2 : 1, E = sizeof(T), TILE = 8 * bank_piece_count<T>();  // columns of 128 channels' bank
-  constexpr int NB = beta_warps<FULL>(NL), NBUF = NB / 2, NS = kHelpers - 1 - NL - NB;
+  constexpr int WPB = warps_per_buffer(NL), NB = kBufs * WPB, NS = kHelpers - 1 - NL - NB;
   constexpr int kOutPitch = out_pitch<T>();
   const int warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0), lane = threadIdx.x & 31;
   const int c0 = blockIdx.y * p.CG, cg = min(p.CG, p.C - c0);
   const int groups = p.full * 4 + p.rest, rounds = p.full + (p.rest ? 1 : 0);
   const unsigned slot_bytes = (unsigned)p.CG * p.pitch, ring_bytes = slot_bytes * p.R;
-  const ConvSmem sm = conv_smem<T, MODE, FULL>(ring_bytes, groups, NBUF);
+  const ConvSmem sm = conv_smem<T, MODE, FULL>(ring_bytes, groups);
   const unsigned base = smem_u32(smem);
   const unsigned x_full = base + sm.bars, step_done = x_full + 8 * kDepth, b_full = step_done + 8 * kDepth;
-  const unsigned b_free = b_full + 8 * kMaxBuf, t_full = b_free + 8 * kMaxBuf, t_empty = t_full + 16, o_full = t_empty + 16,
+  const unsigned b_free = b_full + 8 * kBufs, t_full = b_free + 8 * kBufs, t_empty = t_full + 16, o_full = t_empty + 16,
                  o_free = o_full + 8;
   float* inv_s = reinterpret_cast<float*>(smem + sm.inv);
   volatile int* tail = reinterpret_cast<volatile int*>(smem + sm.bars + kBars * 8);  // TMEM address, abort flag, a bank that is not finite
@@ -561,8 +596,8 @@ __global__ void __launch_bounds__(kThreads, 1)
       mbar_init(x_full + 8 * i, NL == 1 ? 1 : 64 * NL);
       mbar_init(step_done + 8 * i, kConsumers);
     }
-    for (int i = 0; i < NBUF; ++i) {
-      mbar_init(b_full + 8 * i, 2);
+    for (int i = 0; i < kBufs; ++i) {
+      mbar_init(b_full + 8 * i, WPB);
       mbar_init(b_free + 8 * i, 1);
     }
     for (int i = 0; i < 2; ++i) {
@@ -606,7 +641,7 @@ __global__ void __launch_bounds__(kThreads, 1)
     gather_block<T, MODE>(src, rot, bank, dst, p, c0, cg, lo, hi);
   } else if (warp < kConsumers) {
     // ================================================================ consumers
-    regs_inc<consumer_regs<FULL>()>();
+    regs_inc<consumer_regs<FULL, NL>()>();
     const int q = warp & 3, team = warp >> 2;
     const unsigned lanes = (unsigned)(q * 32) << 16;
     const bool vec = p.store == 16;
@@ -732,7 +767,7 @@ __global__ void __launch_bounds__(kThreads, 1)
     }
   } else if (warp == kConsumers) {
     // ================================================================ MMA
-    regs_dec<helper_regs<FULL>()>();
+    regs_dec<helper_regs<FULL, NL>()>();
     constexpr unsigned idesc_all = idesc_f16(128, kSetCols, false, false, FULL), idesc_pair = idesc_f16(128, kSlotCols, false, false, FULL);
     int use = 0;
     bool ok = true;
@@ -767,11 +802,11 @@ __global__ void __launch_bounds__(kThreads, 1)
       }
       if (ok && elect_one()) commit(b_free + 8 * bi);
       __syncwarp();
-      if (++bi == NBUF) bi = 0, ++turn;
+      if (++bi == kBufs) bi = 0, ++turn;
     }
   } else if (warp <= kConsumers + NL) {
     // ================================================================ source rows
-    regs_dec<helper_regs<FULL>()>();
+    regs_dec<helper_regs<FULL, NL>()>();
     const int lw = warp - kConsumers - 1;
     int next = 0, done = 0;
     bool ok = true;
@@ -829,21 +864,21 @@ __global__ void __launch_bounds__(kThreads, 1)
     }
   } else if (warp <= kConsumers + NL + NB) {
     // ================================================================ hat products
-    regs_dec<helper_regs<FULL>()>();
-    const int w = warp - kConsumers - 1 - NL, half = w & 1, bi = w >> 1;
-    Offsets<T> off;
-    if (bi < steps) fetch_offsets<T, MODE>(off, rot, lo + bi * kStepSegs + half * 4, hi, p, lane);
-    for (int s = bi, turn = 0; s < steps; s += NBUF, ++turn) {
+    regs_dec<helper_regs<FULL, NL>()>();
+    const int w = (warp - kConsumers - 1 - NL) % WPB, bi = (warp - kConsumers - 1 - NL) / WPB;
+    Offsets<T, WPB> off;
+    if (bi < steps) fetch_offsets<T, MODE, WPB>(off, rot, lo + bi * kStepSegs, hi, p, w, lane);
+    for (int s = bi, turn = 0; s < steps; s += kBufs, ++turn) {
       if (turn > 0 && !wait_bar(b_free + 8 * bi, (turn - 1) & 1, abort_flag)) break;
-      write_hats<T, MODE, SC44, FULL>(base + sm.beta + bi * (PIECES * kPiece), off, half, p, lane);
+      write_hats<T, MODE, SC44, FULL, WPB>(base + sm.beta + bi * (PIECES * kPiece), off, p, w, lane);
       fence_proxy_async();
       __syncwarp();
       if (lane == 0) mbar_arrive(b_full + 8 * bi);
-      if (s + NBUF < steps) fetch_offsets<T, MODE>(off, rot, lo + (s + NBUF) * kStepSegs + half * 4, hi, p, lane);
+      if (s + kBufs < steps) fetch_offsets<T, MODE, WPB>(off, rot, lo + (s + kBufs) * kStepSegs, hi, p, w, lane);
     }
   } else {
     // ================================================================ results to memory
-    regs_dec<helper_regs<FULL>()>();
+    regs_dec<helper_regs<FULL, NL>()>();
     const int w = warp - kConsumers - 1 - NL - NB;
     const size_t plane = (size_t)p.Hd * p.Wd;
     for (int s = 0; s < steps && STAGED; ++s) {
@@ -901,6 +936,19 @@ __global__ void __launch_bounds__(kThreads, 1)
   }
 }
 
+template <typename T, int MODE, bool SC44, int NL>
+__global__ void __launch_bounds__(kThreads, 1)
+    tc_conv_kernel(const __grid_constant__ CUtensorMap tm, const T* __restrict__ src, const T* __restrict__ rot,
+                   const T* __restrict__ bank, T* __restrict__ dst, const __grid_constant__ ConvParams p) {
+  tc_conv<T, MODE, SC44, NL, true>(tm, src, rot, bank, dst, p);
+}
+template <int MODE, bool SC44, int NL>
+__global__ void __launch_bounds__(kThreads, 1)
+    tc_conv_rounded_kernel(const __grid_constant__ CUtensorMap tm, const __half* __restrict__ src, const __half* __restrict__ rot,
+                           const __half* __restrict__ bank, __half* __restrict__ dst, const ConvParams p) {
+  tc_conv<__half, MODE, SC44, NL, false>(tm, src, rot, bank, dst, p);
+}
+
 // ------------------------------------------------------------------ host side
 bool tc_shape(const Geom& g) {
   if (g.kH != 3 || g.kW != 3 || g.dH != 1 || g.dW != 1 || g.pH != 1 || g.pW != 1) return false;
@@ -953,7 +1001,6 @@ ConvPlan plan_conv(const Geom& g, const void* src, const void* dst) {
   p.pitch = ((1 + (p.nseg * 8 * Wk::xs * E) / 16) | 1) * 16;
   if (p.pitch < 16 + p.Ws * E || p.pitch > 1152 || p.Hg >= (1 << 22)) return pl;
   pl.tma = (reinterpret_cast<uintptr_t>(src) & 15) == 0 && (p.Ws * E) % 16 == 0 && p.pitch / E <= 256;
-  const int nbuf = beta_warps<FULL>(pl.tma ? 1 : kLoaders) / 2;
   const int need = step_rows(p.nseg, p.Hg, Wk::S, p.L, Wk::rows, kStepSegs);
   const int want = step_rows(p.nseg, p.Hg, Wk::S, p.L, Wk::rows, kStepSegs * kDepth);
   const int groups = (g.C + 31) / 32, steps = (p.segs + kStepSegs - 1) / kStepSegs, sms = device_sm_count();
@@ -968,7 +1015,7 @@ ConvPlan plan_conv(const Geom& g, const void* src, const void* dst) {
     const int boxes = (cg + 255) / 256;
     cg = (cg + 8 * boxes - 1) / (8 * boxes) * (8 * boxes);  // boxes start on 128 bytes
     if (splits > 1 && cg != per * 32) continue;
-    const size_t slot = (size_t)cg * p.pitch, fixed = conv_smem<T, MODE, FULL>(0, per, nbuf).total + 160;
+    const size_t slot = (size_t)cg * p.pitch, fixed = conv_smem<T, MODE, FULL>(0, per).total + 160;
     if (fixed + slot * (need + 1) > budget) continue;
     int R = (int)((budget - fixed) / slot);
     if (R > want + 2) R = want + 2;
@@ -985,7 +1032,7 @@ ConvPlan plan_conv(const Geom& g, const void* src, const void* dst) {
       p.CG = cg, p.box_c = cg / boxes, p.full = full, p.rest = rest, p.R = R;
       p.steps_per_cta = spc;
       pl.ctas = (steps + spc - 1) / spc, pl.splits = splits;
-      pl.smem = conv_smem<T, MODE, FULL>((unsigned)(slot * R), per, nbuf).total;
+      pl.smem = conv_smem<T, MODE, FULL>((unsigned)(slot * R), per).total;
       if (pl.smem < kMinSmem) pl.smem = kMinSmem;
     }
   }
@@ -1015,14 +1062,18 @@ bool shares_fit() {
   return r >= kRegsLaunch;
 }
 
-template <typename T, int MODE, bool SC44, int NL, bool FULL>
+template <auto KERN, typename T>
 int run_conv(const ConvPlan& pl, const CUtensorMap& tm, const T* src, const T* rot, const T* w, T* dst, cudaStream_t s) {
-  constexpr auto kern = tc_conv_kernel<T, MODE, SC44, NL, FULL>;
-  if (!shares_fit<kern>()) return DK_ERR_UNSUPPORTED;
-  const int rc = enable_smem(kern, pl.smem);
+  if (!shares_fit<KERN>()) return DK_ERR_UNSUPPORTED;
+  const int rc = enable_smem(KERN, pl.smem);
   if (rc) return rc;
-  kern<<<dim3(pl.ctas, pl.splits), kThreads, pl.smem, s>>>(tm, src, rot, w, dst, pl.p);
+  KERN<<<dim3(pl.ctas, pl.splits), kThreads, pl.smem, s>>>(tm, src, rot, w, dst, pl.p);
   return check_launch();
+}
+template <typename T, int MODE, bool SC44, int NL, bool FULL>
+constexpr auto conv_kernel() {
+  if constexpr (FULL) return &tc_conv_kernel<T, MODE, SC44, NL>;
+  else return &tc_conv_rounded_kernel<MODE, SC44, NL>;
 }
 
 template <typename T, int MODE, bool FULL>
@@ -1034,14 +1085,16 @@ int launch_conv(const T* src, const T* rot, const T* w, T* dst, const Geom& g, c
   if (pl.tma && !make_plane_row_map(&tm, src, sizeof(T), pl.p.Ws, pl.p.Hs, (long long)g.N * g.C, pl.p.pitch / (int)sizeof(T), pl.p.box_c))
     return DK_ERR_UNSUPPORTED;
   const bool sc44 = g.scH == 4 && g.scW == 4;
-  if (pl.tma) return sc44 ? run_conv<T, MODE, true, 1, FULL>(pl, tm, src, rot, w, dst, s) : run_conv<T, MODE, false, 1, FULL>(pl, tm, src, rot, w, dst, s);
-  return sc44 ? run_conv<T, MODE, true, kLoaders, FULL>(pl, tm, src, rot, w, dst, s)
-              : run_conv<T, MODE, false, kLoaders, FULL>(pl, tm, src, rot, w, dst, s);
+  if (pl.tma)
+    return sc44 ? run_conv<conv_kernel<T, MODE, true, 1, FULL>()>(pl, tm, src, rot, w, dst, s)
+                : run_conv<conv_kernel<T, MODE, false, 1, FULL>()>(pl, tm, src, rot, w, dst, s);
+  return sc44 ? run_conv<conv_kernel<T, MODE, true, kLoaders, FULL>()>(pl, tm, src, rot, w, dst, s)
+              : run_conv<conv_kernel<T, MODE, false, kLoaders, FULL>()>(pl, tm, src, rot, w, dst, s);
 }
 
 template <typename T, int MODE, bool SC44, int NL, bool FULL>
 void add_registers(long long out[8]) {
-  const int r = launch_registers<tc_conv_kernel<T, MODE, SC44, NL, FULL>>();
+  const int r = launch_registers<conv_kernel<T, MODE, SC44, NL, FULL>()>();
   ++out[0];
   if (out[1] < 0 || r < out[1]) out[1] = r;
 }
