@@ -704,7 +704,11 @@ template <typename T>
 int local_backward_filter(const T* dy, const T* x, const T* rot, T* dw, const Geom& g, void* ws, size_t ws_bytes,
                           cudaStream_t s) {
   if constexpr (std::is_same<T, __half>::value) {
-    if (mma_path_enabled()) {
+    // Odd rows above 96 at stride 1: the band kernel fetches 2 bytes at a time, a row per thread; the dense one below is faster
+    // (us, band -> dense: 8 x 64 channels of 75 x 95 87 -> 75, x 97 97 -> 75, x 101 99 -> 79, x 111 144 -> 83, 40 x 64 of 60 x 111 353 -> 253,
+    // 8 x 96 of 75 x 101 114 -> 106; x 79 50 -> 67, 90 x 32 of 80 x 81 243 -> 284; stride 2 x 101 44 -> 44, x 111 42 -> 46).
+    const bool wide = (g.W & 1) && g.W > 96 && g.sW == 1;
+    if (!wide && mma_path_enabled()) {
       const int rc = local_filter_mma(dy, x, rot, dw, g, ws, ws_bytes, s);
       if (rc != DK_ERR_UNSUPPORTED) return rc;
     }

@@ -171,7 +171,8 @@ __device__ __forceinline__ void load_band_group(__half* __restrict__ band, const
       // thread every lane is on a line of its own, but the lines are reused and more loads are in flight: on rows of 31 that is
       // the faster way (forward 29 against 49 us), on rows of 101 it is not (66 against 41 us).  The line, by kernel: 96 at stride 1
       // (40 x 64 channels, rows of 81, offsets and bank gradients 393 against 470 us), 72 in the forward at stride 2
-      // (rows of 67 49 / 57, of 79 103 / 74), never in the bank gradient (its presence costs rows below 96 two percent) nor in the gradients at stride 2 (rows of 101 280 / 327)
+      // (rows of 67 49 / 57, of 79 103 / 74), never in the gradients at stride 2 (rows of 101 280 / 327).  The bank gradient has none: their
+      // registers cost rows below 96 two percent, rows above it go to another kernel.
       for (int t = warp; t < tasks; t += nwarps) {
         const int j = t / rows, r = r_s + (t - j * rows);
         const __half* sp = s0 + (size_t)j * plane + (size_t)r * Ws + lane;

@@ -16,6 +16,7 @@ SHAPES = [
     (1, 104, 12, 33), (2, 136, 5, 40), (1, 160, 28, 28), (1, 200, 14, 14), (1, 264, 3, 64), (9, 280, 4, 4), (1, 1096, 6, 10),
     (1, 24, 112, 112), (1, 8, 2, 200), (1, 32, 110, 110), (2, 48, 31, 57),
     (2, 72, 31, 48), (5, 264, 2, 32), (2, 72, 9, 28), (1, 40, 5, 36), (2, 104, 6, 100),
+    (1, 16, 9, 73), (1, 32, 7, 97), (2, 48, 5, 101), (1, 96, 6, 111),  # rows of odd width, a warp per row and not
 ]
 
 
