@@ -490,17 +490,18 @@ int dk_deform_sample_depthwise_backward(const void* grad_output, const void* inp
     return rc;
   }
   if (deform_rows_data(gg, dtype)) {
-    const bool all = deform_rows_all(gg, dtype);
+    const bool all = deform_rows_all(gg, dtype), gathers = deform_rows_gathers(gg, dtype == DK_F16 ? 2 : 4);
     const size_t room = workspace && workspace_bytes >= data_ws ? data_ws : 0;
     bool bank_done = false;
 #define DK_ROWS(T)                                                                                                             \
-  deform_backward_rows<T>(P_(T, grad_output), P_(T, input), P_(T, offset), P_(T, rotation), P_(T, filter), M_(T, grad_input), \
+  deform_backward_rows<T>(P_(T, grad_output), P_(T, input), P_(T, offset), P_(T, rotation), P_(T, filter),                   \
+                          gathers ? M_(T, grad_input) : nullptr,                                                               \
                           all ? M_(T, grad_offset) : nullptr, all ? M_(T, grad_rotation) : nullptr,                           \
                           all ? M_(T, grad_filter) : nullptr, gg, workspace, room, (cudaStream_t)stream, &bank_done)
     rc = dtype == DK_F16 ? DK_ROWS(__half) : DK_ROWS(float);
 #undef DK_ROWS
     if (rc == DK_OK) {  // what is left
-      grad_input = nullptr;
+      if (gathers) grad_input = nullptr;
       if (all) grad_offset = grad_rotation = nullptr;
       if (bank_done) grad_filter = nullptr;
     } else if (rc != DK_ERR_UNSUPPORTED) {

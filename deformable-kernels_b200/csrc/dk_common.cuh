@@ -234,6 +234,7 @@ size_t deform_forward_rows_workspace(const Geom& g, size_t elem);
 template <typename T>
 int deform_forward_rows(const T* x, const T* off, const T* rot, const T* w, T* y, const Geom& g, void* ws, size_t ws_bytes, cudaStream_t s);
 size_t deform_rows_workspace(const Geom& g, size_t elem);
+bool deform_rows_gathers(const Geom& g, size_t elem);  // grad-input too: the plane fits the sort
 template <typename T>
 int deform_backward_rows(const T* dy, const T* x, const T* off, const T* rot, const T* w, T* dx, T* doff, T* drot, T* dw, const Geom& g,
                          void* ws, size_t ws_bytes, cudaStream_t s, bool* bank_done);

@@ -26,6 +26,7 @@ struct BinPlan {
   int movers, sorted;               // first block that transposes; samples to sort (N or none)
   int V, R, bands, segs;               // destination rows of a block, blocks per plane, pieces of a row of cells
   int bank_blocks;                  // partial bank gradients
+  bool sorts;                       // the sort's table and the gather's sums fit: grad-input, which no other pass needs
   size_t starts_bytes, recs_bytes, dyt_bytes, bytes, xt_bytes, bankt_bytes, all_bytes, sort_smem, gather_smem;
 };
 
@@ -655,17 +656,23 @@ bool bin_plan(const Geom& g, size_t elem, BinPlan& t) {
       t.segs = 2 * kGatherWarps / (R + 1);
     }
   }
-  if (best < 0) return false;
+  t.sorts = best >= 0;
+  if (!t.sorts) {
+    t.V = g.C > 32 ? 2 : 1, t.groups = (g.C + 32 * t.V - 1) / (32 * t.V);
+    t.R = t.bands = t.segs = 1;
+  }
   if (t.segs > (g.W + 1) / 4) t.segs = (g.W + 1) / 4 > 0 ? (g.W + 1) / 4 : 1;
   const int row = g.W * (t.V == 1 ? 33 : 66) * 4;
   t.Cp = 32 * t.V * t.groups;
-  if (g.G != 1 || bins * 4 > 160 * 1024 || recs > 0x3fffffff || ((long long)g.P + 1) * t.Cp > 0x7fffffff || t.groups > 65535) return false;
+  if (g.G != 1 || recs > 0x3fffffff || ((long long)g.P + 1) * t.Cp > 0x7fffffff || t.groups > 65535) return false;
   if ((long long)g.N * (t.Cp / 32) * (g.P / kMovePixels + 1) > 0x3fffffff) return false;
-  t.bins = (int)bins, t.rec_per_n = (int)recs;
+  t.sorts = t.sorts && bins * 4 <= 160 * 1024;
+  t.bins = t.sorts ? (int)bins : 0, t.rec_per_n = t.sorts ? (int)recs : 0;
   t.sort_smem = (size_t)t.bins * 4;
   t.gather_smem = (size_t)kGatherWarps * 1536 + ((size_t)bank_cells(g) * 32 * t.V + (size_t)(t.R + 1) * t.segs * 64 * t.V) * 4 + (size_t)t.R * row;
-  if (t.gather_smem > 110 * 1024 || (long long)g.N * t.bands > 0x7fffffff || (long long)g.N * kSortBlocks > 0x3fffffff) return false;
-  t.starts_bytes = round256((size_t)g.N * (t.bins + 1) * sizeof(int));
+  if (t.gather_smem > 110 * 1024 || (long long)g.N * t.bands > 0x7fffffff || (long long)g.N * kSortBlocks > 0x3fffffff)
+    t.sorts = false, t.bins = t.rec_per_n = 0;
+  t.starts_bytes = t.sorts ? round256((size_t)g.N * (t.bins + 1) * sizeof(int)) : 0;
   t.recs_bytes = round256((size_t)g.N * t.rec_per_n * sizeof(Rec));
   t.dyt_bytes = round256((size_t)g.N * (g.P + 1) * t.Cp * elem);
   t.bytes = t.starts_bytes + t.recs_bytes + t.dyt_bytes;
@@ -686,6 +693,10 @@ bool rows_shape(const Geom& g, const BinPlan& t) {
 
 }  // namespace
 
+bool deform_rows_gathers(const Geom& g, size_t elem) {
+  BinPlan t;
+  return bin_plan(g, elem, t) && t.sorts;
+}
 size_t deform_rows_workspace(const Geom& g, size_t elem) {
   BinPlan t;
   return bin_plan(g, elem, t) && rows_shape(g, t) ? t.all_bytes : 0;
@@ -694,7 +705,8 @@ size_t deform_rows_workspace(const Geom& g, size_t elem) {
 template <typename T>
 static int launch_bins(const T* dy, const T* x, const T* off, const T* rot, const T* w, bool sort, int* starts, Rec* recs, T* dyt, T* xt,
                        float* bankt, const Geom& g, BinPlan& t, cudaStream_t s) {
-  const int rc = enable_smem(dcn_bins_kernel<T>, t.sort_smem);
+  const size_t smem = sort ? t.sort_smem : 0;
+  const int rc = enable_smem(dcn_bins_kernel<T>, smem);
   if (rc) return rc;
   t.sorted = sort ? g.N : 0;
   long long tiles = dyt != nullptr ? (long long)g.N * (t.Cp / 32) * (g.P / kMovePixels + 1) : 0;
@@ -708,7 +720,7 @@ static int launch_bins(const T* dy, const T* x, const T* off, const T* rot, cons
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3((unsigned)(clusters * kSortBlocks));
   cfg.blockDim = dim3(kSortThreads);
-  cfg.dynamicSmemBytes = t.sort_smem;
+  cfg.dynamicSmemBytes = smem;
   cfg.stream = s;
   cudaLaunchAttribute attr;
   attr.id = cudaLaunchAttributeClusterDimension;
@@ -740,7 +752,7 @@ int deform_backward_rows(const T* dy, const T* x, const T* off, const T* rot, co
   BinPlan t;
   *bank_done = false;
   const bool bank = dw != nullptr && g.scH <= 4 && g.scW <= 4, coords = doff != nullptr || drot != nullptr;
-  if (!bin_plan(g, sizeof(T), t) || !rows_shape(g, t) || ws == nullptr || ws_bytes < t.all_bytes) return DK_ERR_UNSUPPORTED;
+  if (!bin_plan(g, sizeof(T), t) || !rows_shape(g, t) || ws == nullptr || ws_bytes < t.all_bytes || (dx && !t.sorts)) return DK_ERR_UNSUPPORTED;
   // one gradient alone has to pay for bringing x and dy into channel order: offsets of 16 x 192 of 28 x 28 120 -> 77 us, but
   // 32 x 72 of 56 x 56, stride 2, 100 -> 134; bank of 1 x 960 of 7 x 7 12 -> 19
   if (!dx && !(coords && bank) && (g.C < 96 || (!coords && (long long)g.N * g.P < 2048))) return DK_ERR_UNSUPPORTED;

@@ -63,6 +63,13 @@ def test_workspace_queries(cabi):
     n32 = cabi.lib.dk_sample_depthwise_backward_filter_workspace_bytes(g, cabi.DK_F32)
     assert n32 > 0 and n32 % 256 == 0 and n32 % (64 * 16 * 4) == 0
     assert cabi.lib.dk_deform_sample_depthwise_backward_data_workspace_bytes(g, cabi.DK_F32) == 0
+    # planes too large for the sort (or rows for the gather) of grad-input still have the passes that need neither
+    for h, w in ((204, 210), (4, 700)):
+        big = cabi.geom((1, 40, h, w), (3, 3), (1, 1), (1, 1), (1, 1), (4, 4), 1)
+        for dtype, size in ((cabi.DK_F32, 4), (cabi.DK_F16, 2)):
+            one = 64 * (h * w + 1) * size                               # x in channel order
+            assert cabi.lib.dk_deform_sample_depthwise_forward_workspace_bytes(big, dtype) >= one
+            assert cabi.lib.dk_deform_sample_depthwise_backward_workspace_bytes(big, dtype) >= 2 * one
     assert cabi.lib.dk_deform_sample_depthwise_backward_data_workspace_bytes(g, cabi.DK_F16) >= 4 * 64 * 28 * 28 * 4
 
 

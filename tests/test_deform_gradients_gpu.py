@@ -12,7 +12,8 @@ DEV = "cuda:0"
 SHAPES = [
     (1, 1, 1, 1, 1, 1, 1, (4, 4)), (2, 33, 5, 40, 1, 1, 1, (4, 4)), (3, 8, 9, 7, 2, 1, 1, (3, 3)), (1, 72, 33, 35, 1, 2, 2, (2, 4)),
     (2, 24, 60, 61, 2, 0, 1, (4, 4)), (17, 40, 4, 4, 1, 1, 1, (1, 1)), (1, 8, 3, 120, 1, 1, 1, (6, 5)),
-    (2, 96, 11, 13, 1, 1, 1, (4, 4)), (1, 128, 6, 8, 2, 1, 1, (4, 4))]
+    (2, 96, 11, 13, 1, 1, 1, (4, 4)), (1, 128, 6, 8, 2, 1, 1, (4, 4)),
+    (1, 40, 204, 210, 1, 1, 1, (4, 4)), (1, 34, 4, 700, 1, 1, 1, (3, 3))]  # no room for the sort or the sums of grad-input
 
 
 @pytest.mark.parametrize("n,c,h,w,stride,pad,dil,scope", SHAPES)
@@ -27,7 +28,8 @@ def test_gradients(n, c, h, w, stride, pad, dil, scope, dtype):
     leaves = [t.requires_grad_(True) for t in (x, o, r, wt)]
     y = deform_sample_depthwise(*leaves, **case["args"])
     got = torch.autograd.grad(y, leaves, dy)
-    up = torch.float32 if dtype == torch.float16 else torch.float64
+    # beyond 128 pixels fp32 rounds a coordinate at 2^-17 and more: samples (and cells, at the floor) are those of the fp32 oracle
+    up = torch.float32 if dtype == torch.float16 or max(h, w) > 128 else torch.float64
     a = [case[k].to(dtype).to(up) for k in ("grad_output", "input", "offset", "rotation", "weight")]
     want = O.deform_sample_depthwise_backward(*a, **case["args"])
     tol = 2e-3 if dtype == torch.float16 else 1e-5
