@@ -303,8 +303,9 @@ int dk_deform_sample_depthwise_forward(const void* input, const void* offset, co
 }
 
 /* Which passes take the kernels with channels on the lanes: fp32, and fp16 where no tensor-core kernel applies or, forward, where
- * rows of odd width cost that one its pixel pairs (us: 40 x 128 of 15 x 17 44 -> 33, 16 x 160 of 45 x 31 125 -> 95, but 100 x 32
- * of 13 x 15 24 -> 27, 60 x 960 of 7 x 7 56 -> 72; without kernel-space offsets its sampled kernel is the cheaper one). */
+ * rows of odd width cost that one its pixel pairs (us: 40 x 128 of 15 x 17 44 -> 33, 16 x 160 of 45 x 31 125 -> 95, 64 x 48 of 9 x 9
+ * 23 -> 22, but 64 x 32 of 9 x 9 16 -> 20, 100 x 32 of 13 x 15 24 -> 27, 64 x 96 of 7 x 7 17 -> 22, 60 x 960 56 -> 72; without
+ * kernel-space offsets its sampled kernel is the cheaper one). */
 static bool deform_no_mma(const Geom& g, int dtype) {
   if (dtype != DK_F16) return dtype == DK_F32;
   return deform_data_mma_workspace(g) == 0 && deform_coords_mma_workspace(g) == 0 && deform_filter_mma_workspace(g) == 0;

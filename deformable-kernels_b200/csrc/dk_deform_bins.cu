@@ -753,9 +753,10 @@ int deform_backward_rows(const T* dy, const T* x, const T* off, const T* rot, co
   *bank_done = false;
   const bool bank = dw != nullptr && g.scH <= 4 && g.scW <= 4, coords = doff != nullptr || drot != nullptr;
   if (!bin_plan(g, sizeof(T), t) || !rows_shape(g, t) || ws == nullptr || ws_bytes < t.all_bytes || (dx && !t.sorts)) return DK_ERR_UNSUPPORTED;
-  // one gradient alone has to pay for bringing x and dy into channel order: offsets of 16 x 192 of 28 x 28 120 -> 77 us, but
-  // 32 x 72 of 56 x 56, stride 2, 100 -> 134; bank of 1 x 960 of 7 x 7 12 -> 19
-  if (!dx && !(coords && bank) && (g.C < 96 || (!coords && (long long)g.N * g.P < 2048))) return DK_ERR_UNSUPPORTED;
+  // One gradient alone has to pay for bringing x and dy into channel order.  us, without -> with, image offsets / kernel offsets / bank:
+  // 16 x 64 of 28 x 28 47 -> 34 / 75 -> 38 / 75 -> 38, 64 x 40 101 -> 107 / 162 -> 118 / 149 -> 91; stride 2, 32 x 72 of 56 x 56 101 -> 110 / 132 -> 116 /
+  // 171 -> 106, 32 x 40 71 -> 75 / 94 -> 79 / 95 -> 69.  Bank alone with few pixels: 32 x 192 of 7 x 7 28 -> 28, 48 x 192 30 -> 32, 1 x 960 12 -> 19.
+  if (!dx && !(coords && bank) && (g.C < 64 || (!coords && (long long)g.N * g.P < 2048))) return DK_ERR_UNSUPPORTED;
   if (!dx && !coords && !bank) return DK_ERR_UNSUPPORTED;
   char* at = reinterpret_cast<char*>(ws);
   int* starts = reinterpret_cast<int*>(at);
@@ -787,13 +788,12 @@ int deform_backward_rows(const T* dy, const T* x, const T* off, const T* rot, co
   }
   return DK_OK;
 }
-// Forward: x and the bank into channel order, then a lane per channel.  Not where lanes stay empty in a large call, nor where a
-// large x is moved for a quarter as many outputs of few channels.  Lane per pixel -> per channel, us: 16 x 192 of 28 x 28 75 -> 50,
-// 13 x 96 of 80 x 80 270 -> 188, 64 x 384 of 14 x 14 128 -> 98, 1 x 240 of 20 x 20 31 -> 17; 64 x 16 of 28 x 28 39 -> 46; stride
-// 2: 20 x 128 of 56 x 56 80 -> 71, 32 x 72 of 56 x 56 78 -> 90, 8 x 32 of 40 x 40 38 -> 16.
+// Forward: x and the bank into channel order, then a lane per channel.  Not where most lanes stay empty in a large call.  Lane per
+// pixel -> per channel, us: 16 x 192 of 28 x 28 90 -> 56, 64 x 24 64 -> 50, 64 x 16 55 -> 50, 64 x 8 39 -> 48, 128 x 16 of 56 x 56 274 -> 296,
+// 8 x 16 of 32 x 32 50 -> 22; stride 2: 32 x 128 of 56 x 56 152 -> 106, 32 x 64 102 -> 59, 32 x 40 53 -> 60, 32 x 32 59 -> 40.
 static bool forward_rows(const Geom& g, size_t elem, BinPlan& t) {
   if (g.taps > kForwardTaps || !bin_plan(g, elem, t) || !rows_shape(g, t)) return false;
-  return (g.C >= 32 || (long long)g.N * g.P < 16384) && (g.HW <= 2 * g.P || g.C >= 96 || (long long)g.N * g.HW * g.C < (1 << 21));
+  return g.C >= 24 || (long long)g.N * g.P < 16384;
 }
 size_t deform_forward_rows_workspace(const Geom& g, size_t elem) {
   BinPlan t;

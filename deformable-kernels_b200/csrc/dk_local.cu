@@ -136,15 +136,16 @@ static int launch_local_conv(const T* src, const T* rot, const T* w, T* dst, con
       int rc = DK_ERR_UNSUPPORTED;
       // stride 1, rows that TMA fetches, three 32-channel groups or more: a pair of groups leaves half of the consumer warps
       // idle at a time.  Against the band kernels on rows of 16 .. 96, 72 .. 384 channels 1.0 to 1.6 times as fast (C = 384,
-      // 32 x 32: 45 -> 29 us); against the ring kernels (rows of 112 / 56) up to 96 channels only (C = 96, 112 x 112: 283 ->
-      // 253 us, grad-input 300 -> 286; C = 144, 56 x 56, batch 32: 35 -> 40).
+      // 32 x 32: 45 -> 29 us).  Against the ring kernels, forward and grad-input: rows of 112, batch 64 and 32, C = 80 137, 144 ->
+      // 141, 138 us, C = 96 154, 163 -> 144, 142, C = 112 463, 513 -> 259, 251, C = 128 121, 129 -> 137, 132, C = 160 137, 144 -> 197, 189; rows of
+      // 56, batch 32, C = 128 38, 39 -> 31, 31 (batch 8 21, 23 -> 18, 19), C = 144 41, 42 -> 46, 45.
       const bool ring_row = g.W == 112 || g.W == 56;
       // grad-input at stride 2 where TMA fetches the rows of dy, against the gather of the band kernels (nine mma for 2.25 useful):
       // 32 x 96 of 64 x 64 29 -> 19 us, 64 x 384 of 32 x 32 50 -> 27, 64 x 64 of 48 x 48 27 -> 19; rows of dy of 20 19 -> 25,
       // odd rows of dx (32 x 96 of 63 x 63) 45 -> 129, 50 x 80 of 16 x 16 10.5 -> 11.3; the ring kernel of 112-wide rows takes half of
       // its time.
       const bool dx2 = TRANSPOSED && g.sH == 2 && g.W % 16 == 0 && g.W >= 32 && g.C >= 64 && g.W != 112;
-      if ((dx2 || (g.sH == 1 && g.W % 8 == 0 && g.C > 64 && (!ring_row || g.C <= 96))) && local_conv_mma_takes(g, TRANSPOSED)) {
+      if ((dx2 || (g.sH == 1 && g.W % 8 == 0 && g.C > 64 && (!ring_row || g.C <= (g.W == 112 ? 112 : 128)))) && local_conv_mma_takes(g, TRANSPOSED)) {
         rc = local_conv_tc_rounded(src, rot, w, dst, g, TRANSPOSED, s);
         if (rc != DK_ERR_UNSUPPORTED) return rc;
       }
@@ -561,8 +562,8 @@ static PlanePlan plane_plan(const Geom& g) {
   if (slots > g.N) slots = g.N;
   if (slots < 1) slots = 1;
   pl.slots = (int)slots;
-  // fewer samples than it takes to fill the GPU: several blocks share a sample's pixels, each with a copy of the planes
-  // (N = 16, C = 192, 28 x 28 fp32: 96 blocks became 384, 213 -> 150 us)
+  // fewer samples than it takes to fill the GPU: several blocks share a sample's pixels, each with a copy of the planes (scopes
+  // beyond 4 x 4, fp32: 16 x 192 of 28 x 28, 6 x 6, 224 -> 181 us; 4 x 64 of 40 x 40, 5 x 5, 917 -> 134)
   long long parts = (2LL * 148 + slots * chan_ctas - 1) / (slots * chan_ctas);
   const long long most = g.P / (4 * pl.batch);
   if (parts > most) parts = most;
