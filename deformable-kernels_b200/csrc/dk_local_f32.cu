@@ -558,24 +558,28 @@ template int local_filter_f32<__half>(const __half*, const __half*, const __half
 template <typename T>
 int local_rot_f32(const T* dy, const T* x, const T* rot, const T* w, T* drot, const Geom& g, cudaStream_t s) {
   if (!f32_shape(g)) return DK_ERR_UNSUPPORTED;
-  // Calls with few pixels only: the general kernel (32 pixels per block, gathered cells) leaves SMs without a block there.
-  // N = 2, C = 64, 28 x 28: 13.6 -> 10.7 us; N = 32, C = 960, 7 x 7: 109 -> 82.  With the GPU full it is as fast or faster
-  // (N = 64, C = 144, 56 x 56: 383 against 392 us, stride 2: 117 against 161).
+  // Calls with few pixels: the general kernel (32 pixels per block, gathered cells) leaves SMs without a block there.  N = 2, C = 64,
+  // 28 x 28: 13.6 -> 10.7 us; N = 32, C = 960, 7 x 7: 109 -> 82.  With the GPU full, up to 32 channels, which that kernel's warps share
+  // too thinly: 64 x 24 of 112 x 112 666 -> 327 us (fp16 633 -> 443, stride 2 172 -> 156), 64 x 16 of 56 x 56 158 -> 79; 32 x 72 139 -> 137 (fp16
+  // 133 -> 195), 64 x 144 389 -> 438.
   TilePlan t = tile_plan(g, 128);
-  if (t.tiles >= 2 * device_sm_count()) return DK_ERR_UNSUPPORTED;
-  // fp16: few channels too, its planes pass through registers (2 x 24 of 14 x 14 16.5 -> 12 us, 1 x 40 of 28 x 28 19.5 -> 17; 64 x 936 of
-  // 7 x 7 132 -> 177)
-  if (sizeof(T) == 2 && (g.C > 64 || tile_plan(g, 32).tiles >= device_sm_count())) return DK_ERR_UNSUPPORTED;
-  int pq = 2;
-  t = tile_plan(g, 64);
-  if (t.tiles < 2 * device_sm_count()) pq = 1, t = tile_plan(g, 32);
+  int pq = 4;
+  if (t.tiles >= 2 * device_sm_count()) {
+    if (g.C > 32) return DK_ERR_UNSUPPORTED;
+  } else {
+    // fp16: few channels too, its planes pass through registers (2 x 24 of 14 x 14 16.5 -> 12 us, 1 x 40 of 28 x 28 19.5 -> 17; 64 x 936 of
+    // 7 x 7 132 -> 177)
+    if (sizeof(T) == 2 && (g.C > 64 || tile_plan(g, 32).tiles >= device_sm_count())) return DK_ERR_UNSUPPORTED;
+    pq = 2, t = tile_plan(g, 64);
+    if (t.tiles < 2 * device_sm_count()) pq = 1, t = tile_plan(g, 32);
+  }
   size_t words = 512 + 32 * (size_t)(t.xpitch + t.ypitch);
   const size_t red = (size_t)pq * 3 * (4 / pq - 1) * 6 * 32;
   if (words < red) words = red;
   t.smem = words * sizeof(float);
   if (t.smem > (size_t)device_smem_optin()) return DK_ERR_UNSUPPORTED;
-  auto kern = g.sH == 1 ? (pq == 2 ? f32_offsets_kernel<T, 1, 2> : f32_offsets_kernel<T, 1, 1>)
-                        : (pq == 2 ? f32_offsets_kernel<T, 2, 2> : f32_offsets_kernel<T, 2, 1>);
+  auto kern = g.sH == 1 ? (pq == 4 ? f32_offsets_kernel<T, 1, 4> : pq == 2 ? f32_offsets_kernel<T, 1, 2> : f32_offsets_kernel<T, 1, 1>)
+                        : (pq == 4 ? f32_offsets_kernel<T, 2, 4> : pq == 2 ? f32_offsets_kernel<T, 2, 2> : f32_offsets_kernel<T, 2, 1>);
   const int rc = enable_smem(kern, t.smem);
   if (rc) return rc;
   kern<<<t.tiles, 32 * kOffWarps, t.smem, s>>>(dy, x, rot, w, drot, g, t);

@@ -17,6 +17,7 @@ SHAPES = [
     (1, 24, 112, 112), (1, 8, 2, 200), (1, 32, 110, 110), (2, 48, 31, 57),
     (2, 72, 31, 48), (5, 264, 2, 32), (2, 72, 9, 28), (1, 40, 5, 36), (2, 104, 6, 100),
     (1, 16, 9, 73), (1, 32, 7, 97), (2, 48, 5, 101), (1, 96, 6, 111),  # rows of odd width, a warp per row and not
+    (13, 24, 57, 58), (13, 8, 113, 114),  # few channels, the GPU full
 ]
 
 
