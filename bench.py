@@ -88,7 +88,7 @@ def measured_traffic(n):
     ncu capture summarised under profiles/ (taken at a smaller batch; the traffic of these streaming kernels grows in
     proportion to the batch, so it is scaled to n images).  None when the summary is missing."""
     try:
-        rec = json.load(open(os.path.join(ROOT, "profiles", "local_dk_ring_kernels_traffic.json")))
+        rec = json.load(open(os.path.join(ROOT, "profiles", "local_dk_largest_layer_traffic.json")))
         return {k: v * n / rec["batch"] for k, v in rec["dram_bytes_per_launch"].items()}, rec.get("source")
     except Exception:
         return None, None
