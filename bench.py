@@ -872,8 +872,7 @@ def main():
         # launches of this library per step: ring layers (rows of 112 or 56, rows of 28 at stride 1) run forward,
         # grad-input, the fused offsets + bank pass (+ the reduction of its partial offset gradients when more than 144
         # channels are split into groups) and the bank reduction (or forward, the one-pass backward and the reduction); planes of
-        # 14 x 14 outputs and below forward, grad-input, the fused band pass, the reduction of its partial offset
-        # gradients when the channels are split into groups (more than 96 channels) and the bank reduction; the others
+        # 14 x 14 outputs and below forward, grad-input, the fused band pass and one launch for its reductions; the others
         # forward, grad-input, grad-offsets (+ the reduction of its partial sums when split), grad-bank + reduction
         def layer_launches(t):
             if t["hw"] in (112, 56) or (t["hw"] == 28 and t["s"] == 1):
@@ -881,7 +880,7 @@ def main():
                     return 3
                 return 5 if t["c"] > 144 else 4
             if t["ho"] * t["ho"] <= 196:
-                return 5 if t["c"] > 96 else 4
+                return 4
             q = (ctypes.c_longlong * 8)()
             geom = C.geom((n, t["c"], t["hw"], t["hw"]), (K, K), (t["s"], t["s"]), (PAD, PAD), (1, 1), (SCOPE, SCOPE), 1)
             split = C.lib.dk_local_plan_query(geom, C.DK_F16, 2, q) == 0 and q[2] > 1
