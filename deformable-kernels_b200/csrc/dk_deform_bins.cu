@@ -8,7 +8,8 @@
 // the cells of a row with 32 channels on its lanes and the four corner sums in registers: no atomics, no collisions, one
 // multiply-add per corner (dcn_gather_kernel).  16 x 192 of 28 x 28: 245 -> 71 us (19 of them the sort); 13 x 96 of 80 x 80:
 // 985 -> 281, in fp16 912 -> 281; 64 x 384 of 14 x 14: 640 -> 111; 32 x 72 of 56 x 56, stride 2: 124 -> 101.  The gather is
-// bound by issue (1.6 instructions per cycle and SM over about 20 warps), the sort by the latency of its five steps.
+// bound by latency: 1.6 instructions per cycle and SM (40 % of the issue slots) from one dependent walk per warp, 192 blocks of eight
+// warps on 148 SMs for 16 x 192 of 28 x 28; the sort by the latency of its five steps.
 #include <cooperative_groups.h>
 
 #include "dk_common.cuh"
@@ -335,8 +336,9 @@ __global__ void __launch_bounds__(32 * kGatherWarps, 3) dcn_gather_kernel(const 
 // read the zero pixel, cells outside the bank its zero border, so nothing is masked.  A unit of a warp is 32 pixels of a tap.
 // Offsets, with x and dy brought into channel order for it alone: 16 x 192 of 28 x 28 120 -> 70 us, 8 x 960 of 7 x 7 222 -> 33; bank
 // 167 -> 62.  All gradients from one preparation: 16 x 192 of 28 x 28 531 -> 183 us, 13 x 96 of 80 x 80 2704 -> 773, fp16 13 x 88
-// of 80 x 80 2424 -> 713, 64 x 384 of 14 x 14 1061 -> 300, 32 x 72 of 56 x 56 at stride 2 551 -> 265.  Bound by issue: 28
-// multiply-adds beside nine loads and their addresses.
+// of 80 x 80 2424 -> 713, 64 x 384 of 14 x 14 1061 -> 300, 32 x 72 of 56 x 56 at stride 2 551 -> 265.  Bound by the load
+// pipe (70 %, the forward 82 %): nine lines for 28 (14) multiply-adds; the bank gradient by the latency of five at 16 accumulators'
+// registers (FMA pipe 54 %).
 constexpr int kRowWarps = 8;
 
 // byte offsets of the four corners; {1 - lh, lh, 1 - lw, lw}; for the coordinates the same of the bank and {dy, bank cell}, for the bank

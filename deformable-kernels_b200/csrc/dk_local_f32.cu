@@ -8,8 +8,9 @@
 //             lanes, read back one channel per lane), the hats of a (pixel, tap) are two 16-byte broadcasts
 //   offsets   lanes = pixels: G[tap, cell] += dK * W[c, cell], a warp per kernel row (48 accumulators), channel after channel;
 //             then the floor-based derivative weights contract G
-// Bound by instruction issue: 21 (bank) and 17 (offsets) multiply-adds per pixel, tap and channel, packed in pairs, beside
-// the loads.  The bank kernel before gathered four cells per tap with an address per lane, read x and dy one channel per lane
+// 21 (bank) and 17 (offsets) multiply-adds per pixel, tap and channel, packed in pairs, beside the loads.  The bank kernel keeps the FMA
+// pipe at 55 % and the issue slots at 56 % with the 16 warps that its registers allow: bound by the latency of the loads between the
+// products.  The bank kernel before gathered four cells per tap with an address per lane, read x and dy one channel per lane
 // from global memory (a line per lane) and added into shared memory: N = 64, C = 144, 56 x 56 2088 -> 384 us (stride 2 562 ->
 // 119, N = 32, C = 384, 14 x 14 115 -> 39).
 #include <cuda_runtime.h>
