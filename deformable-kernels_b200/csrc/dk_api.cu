@@ -325,10 +325,29 @@ static bool deform_rows_all(const Geom& g, int dtype) {
   return deform_no_mma(g, dtype) || (deform_rows_data(g, dtype) && g.C >= 32);
 }
 
+/* fp16 with the operands in channel order (dk_deform_lines.cu): in place of the kernels with planes on chip, with their arithmetic,
+ * where there is enough to pay for bringing x (and dy) into that order, and for units of 64 channels that are not mostly empty.
+ * us, planes on chip -> lines, forward: 12 x 144 of 9 x 9 20 -> 19, 8 x 192 of 28 x 28 at stride 2 (301 k outputs) 18 -> 20, 100 x 32 of
+ * 13 x 14 (582 k) 27 -> 22, 16 x 96 of 28 x 28 37 -> 22; 128 x 16 of 28 x 28 at stride 2 18 -> 28.  Backward: 60 x 960 of 7 x 7
+ * 359 -> 114, 8 x 192 of 28 x 28 at stride 2 73 -> 58, 64 x 48 of 14 x 14 at stride 2 65 -> 63, 64 x 32 of 28 x 28 149 -> 153,
+ * 128 x 16 of 28 x 28 at stride 2 60 -> 121. */
+static bool deform_lines_takes_forward(const Geom& g, int dtype, bool rotation) {
+  return dtype == DK_F16 && mma_path_enabled() && g.C >= 32 && (long long)g.N * g.C * g.P >= (1 << 19) && deform_lines_shape(g) &&
+         deform_forward_mma_takes(g) && !deform_rows_forward(g, dtype, rotation);
+}
+static bool deform_lines_takes_backward(const Geom& g, int dtype) {
+  return dtype == DK_F16 && mma_path_enabled() && g.C >= 48 && deform_lines_shape(g) && !deform_rows_data(g, dtype);
+}
+
 size_t dk_deform_sample_depthwise_forward_workspace_bytes(const dk_geom* g, int dtype) {
   Geom gg;
-  if (!make_geom(g, &gg) || !deform_rows_forward(gg, dtype, true)) return 0;
-  return align256(deform_forward_rows_workspace(gg, dtype == DK_F16 ? 2 : 4));
+  if (!make_geom(g, &gg)) return 0;
+  size_t need = 0;
+  if (deform_rows_forward(gg, dtype, true)) need = deform_forward_rows_workspace(gg, dtype == DK_F16 ? 2 : 4);
+  for (int rotation = 0; rotation < 2; ++rotation)
+    if (deform_lines_takes_forward(gg, dtype, rotation != 0) && deform_lines_forward_workspace(gg) > need)
+      need = deform_lines_forward_workspace(gg);
+  return align256(need);
 }
 
 int dk_deform_sample_depthwise_forward_ws(const void* input, const void* offset, const void* rotation, const void* filter,
@@ -337,6 +356,11 @@ int dk_deform_sample_depthwise_forward_ws(const void* input, const void* offset,
   Geom gg;
   if (!input || !offset || !filter || !output || !make_geom(g, &gg)) return DK_ERR_BAD_ARGUMENT;
   const size_t need = dk_deform_sample_depthwise_forward_workspace_bytes(g, dtype);
+  if (deform_lines_takes_forward(gg, dtype, rotation != nullptr)) {
+    if (!workspace || workspace_bytes < need) return DK_ERR_WORKSPACE;
+    return deform_lines_forward(P_(__half, input), P_(__half, offset), P_(__half, rotation), P_(__half, filter), M_(__half, output),
+                                gg, workspace, workspace_bytes, (cudaStream_t)stream);
+  }
   if (need == 0 || !deform_rows_forward(gg, dtype, rotation != nullptr))
     return dk_deform_sample_depthwise_forward(input, offset, rotation, filter, output, g, dtype, stream);
   if (!workspace || workspace_bytes < need) return DK_ERR_WORKSPACE;
@@ -423,6 +447,10 @@ static size_t deform_front_ws(const dk_geom* g, int dtype) {
     const size_t rows = align256(deform_rows_workspace(gg, dtype == DK_F16 ? 2 : 4));
     if (rows > need) need = rows;
   }
+  if (make_geom(g, &gg) && deform_lines_takes_backward(gg, dtype)) {
+    const size_t lines = align256(deform_lines_backward_workspace(gg));
+    if (lines > need) need = lines;
+  }
   return need;
 }
 
@@ -447,8 +475,15 @@ int dk_deform_sample_depthwise_backward(const void* grad_output, const void* inp
   const size_t data_ws = deform_front_ws(g, dtype);
   const size_t filt_ws = dk_deform_sample_depthwise_backward_filter_workspace_bytes(g, dtype);
   int rc = DK_OK;
+  if (!rotation && grad_rotation) return DK_ERR_BAD_ARGUMENT;
+  if (deform_lines_takes_backward(gg, dtype) && workspace && workspace_bytes >= data_ws) {
+    rc = deform_lines_backward(P_(__half, grad_output), P_(__half, input), P_(__half, offset), P_(__half, rotation), P_(__half, filter),
+                               M_(__half, grad_input), M_(__half, grad_offset), M_(__half, grad_rotation), M_(__half, grad_filter), gg,
+                               workspace, data_ws, (cudaStream_t)stream);
+    if (rc != DK_ERR_UNSUPPORTED) return rc;
+    rc = DK_OK;
+  }
   if (!rotation) {  // zero kernel-space offsets (see the forward); nothing to differentiate with respect to them
-    if (grad_rotation) return DK_ERR_BAD_ARGUMENT;
     if (deform_rows_all(gg, dtype)) {
       if (grad_filter && (gg.scH > 4 || gg.scW > 4)) return DK_ERR_UNSUPPORTED;  // that kernel wants a tensor of zeros
       bool bank_done = false;

@@ -230,6 +230,14 @@ template <typename T>
 int local_rot_f32(const T* dy, const T* x, const T* rot, const T* w, T* drot, const Geom& g, cudaStream_t s);
 size_t local_filter_f32_workspace(const Geom& g);
 size_t deform_data_mma_workspace(const Geom& g);
+// fp16 with the operands in channel order (dk_deform_lines.cu)
+bool deform_lines_shape(const Geom& g);
+size_t deform_lines_forward_workspace(const Geom& g);
+int deform_lines_forward(const __half* x, const __half* off, const __half* rot, const __half* w, __half* y, const Geom& g, void* ws,
+                         size_t ws_bytes, cudaStream_t s);
+size_t deform_lines_backward_workspace(const Geom& g);
+int deform_lines_backward(const __half* dy, const __half* x, const __half* off, const __half* rot, const __half* w, __half* dx,
+                          __half* doff, __half* drot, __half* dw, const Geom& g, void* ws, size_t ws_bytes, cudaStream_t s);
 size_t deform_forward_rows_workspace(const Geom& g, size_t elem);
 template <typename T>
 int deform_forward_rows(const T* x, const T* off, const T* rot, const T* w, T* y, const Geom& g, void* ws, size_t ws_bytes, cudaStream_t s);
@@ -275,6 +283,7 @@ int deform_coords_mma(const __half* dy, const __half* x, const __half* off, cons
                       void* bank_ws = nullptr, size_t bank_ws_bytes = 0, bool* bank_done = nullptr);
 int deform_data_mma(const __half* dy, const __half* off, const __half* rot, const __half* w, __half* dx, const Geom& g,
                     void* ws, size_t ws_bytes, cudaStream_t s);
+bool deform_forward_mma_takes(const Geom& g);
 int deform_forward_mma(const __half* x, const __half* off, const __half* rot, const __half* w, __half* y, const Geom& g,
                        cudaStream_t s);  // fp16 tensor-core DK+DCN bank gradient (dk_deform_mma.cu)
 int deform_filter_mma(const __half* dy, const __half* x, const __half* off, const __half* rot, __half* dw, const Geom& g,

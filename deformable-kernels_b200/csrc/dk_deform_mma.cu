@@ -1242,6 +1242,11 @@ int deform_filter_mma(const __half* dy, const __half* x, const __half* off, cons
   return check_launch();
 }
 
+bool deform_forward_mma_takes(const Geom& g) {
+  const DcnPlan pl = dcn_plan(g, slab_cap(), 0);
+  return pl.BH != 0 && pl.smem <= (size_t)device_smem_optin() && g.C / (16 * pl.NS) <= 65535;
+}
+
 int deform_forward_mma(const __half* x, const __half* off, const __half* rot, const __half* w, __half* y, const Geom& g,
                        cudaStream_t s) {
   DcnPlan pl = dcn_plan(g, slab_cap(), 0);

@@ -1,0 +1,90 @@
+"""DK + DCN in fp16 with the operands in channel order: units of 64 channels, strips of 16 columns, windows of 8 columns and groups of 16
+pixels or samples, each with remainders, against the fp32 oracle (grad-input also bit for bit against itself)."""
+import os
+import sys
+
+import pytest
+import torch
+
+ROOT = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
+sys.path.insert(0, os.path.join(ROOT, "deformable-kernels_b200"))
+sys.path.insert(0, ROOT)
+
+from dk_cases import make_case, rel_err  # noqa: E402
+
+pytestmark = pytest.mark.gpu
+NAMES = ("grad_input", "grad_offset", "grad_rotation", "grad_weight")
+
+
+def _run(case, rotation=True):
+    from deformable_kernels.ops.deform_kernel.functions import deform_sample_depthwise
+    dy, x, o, r, w = (case[k].to(torch.float16).cuda() for k in ("grad_output", "input", "offset", "rotation", "weight"))
+    leaves = [t.requires_grad_(True) for t in ((x, o, r, w) if rotation else (x, o, w))]
+    y = deform_sample_depthwise(x, o, r if rotation else None, w, **case["args"])
+    names = NAMES if rotation else tuple(n for n in NAMES if n != "grad_rotation")
+    return dict(zip(("output",) + names, (y.detach(),) + torch.autograd.grad(y, leaves, dy)))
+
+
+def _want(case):
+    from oracle import dk_oracle as O
+    dy, x, o, r, w = (case[k].to(torch.float16).float() for k in ("grad_output", "input", "offset", "rotation", "weight"))
+    return dict(zip(("output",) + NAMES, (O.deform_sample_depthwise_forward(x, o, r, w, **case["args"]),) +
+                    tuple(O.deform_sample_depthwise_backward(dy, x, o, r, w, **case["args"]))))
+
+
+def _check(case, rotation=True):
+    if not rotation:
+        case["rotation"] = torch.zeros_like(case["rotation"])
+    got, want = _run(case, rotation), _want(case)
+    for k, v in got.items():
+        # corner weights, hat products, K and the products with dy rounded to fp16 (2^-11 each), the result as well
+        assert rel_err(v, want[k].half()) < 2e-3, k
+    return got
+
+
+@pytest.mark.parametrize("n,c,h,w,stride,scope,rotation", [
+    (32, 48, 17, 16, 1, (4, 4), True),     # part of a unit; a strip without remainder
+    (40, 64, 18, 34, 2, (4, 4), True),     # one unit, four groups of pixels per block; columns of y 17
+    (12, 144, 20, 20, 1, (3, 3), True),    # three units: a block of three warps
+    (7, 320, 16, 36, 1, (4, 4), True),     # five units: two sets of channels; strips 16, 16, 4
+    (6, 272, 25, 30, 2, (2, 4), True),     # odd rows of y, even columns of x
+    (20, 128, 9, 50, 1, (3, 3), False),    # no kernel-space offsets
+    (50, 64, 3, 200, 1, (1, 4), True),     # fewer rows than a band
+    (3, 960, 21, 15, 1, (4, 4), True),     # four sets; odd columns
+    (24, 96, 56, 6, 1, (4, 1), True),      # narrower than a window
+])
+def test_shapes(n, c, h, w, stride, scope, rotation):
+    case = make_case(n, c, h, w, scope=scope, stride=stride, rot_std=0.7, off_std=2.0, seed=7)
+    _check(case, rotation)
+
+
+def test_offsets_that_collapse_and_leave():
+    """Every tap of a sample on one point (one cell holds all records, far more than a chunk), and points far outside, infinite or NaN."""
+    case = make_case(10, 160, 14, 18, scope=(4, 4), rot_std=0.5, off_std=1.0, seed=8)
+    off = case["offset"].view(10, 9, 2, 14, 18)
+    rows, cols = torch.arange(14.).view(1, 14, 1), torch.arange(18.).view(1, 1, 18)
+    for t in range(9):
+        off[0, t, 0], off[0, t, 1] = 6.25 - (rows[0] - 1 + t // 3), 7.5 - (cols[0] - 1 + t % 3)
+    off[1] = 1e4
+    off[2, :, 0, 3, 4], off[2, :, 1, 5, 6], off[2, 4, 0, 7, 7] = float("nan"), float("inf"), -float("inf")
+    got = _check(case)
+    assert torch.equal(got["grad_input"][1], torch.zeros_like(got["grad_input"][1]))
+
+
+def test_grad_input_is_the_same_in_every_run():
+    case = make_case(16, 96, 31, 28, scope=(4, 4), rot_std=0.5, off_std=2.0, seed=9)
+    first = _run(case)["grad_input"]
+    for _ in range(3):
+        assert torch.equal(first, _run(case)["grad_input"])
+
+
+def test_values_that_are_not_finite_stay_with_their_samples():
+    """An infinite dy reaches the pixels its taps touch in its own channel; the rest of grad-input keeps its value."""
+    case = make_case(8, 192, 20, 24, scope=(4, 4), rot_std=0.3, off_std=1.0, seed=10)
+    plain = _run(case)["grad_input"]
+    case["grad_output"][3, 100, 9, 11] = float("inf")
+    got = _run(case)["grad_input"]
+    changed = ~torch.isfinite(got)
+    assert 4 <= int(changed.sum()) <= 36 and bool(changed[3, 100].any()) and int(changed.sum()) == int(changed[3, 100].sum())
+    # a window with such a value is summed pixel by pixel in fp32, not in pieces of 22 bits
+    torch.testing.assert_close(got[~changed], plain[~changed], rtol=2e-3, atol=2e-3)
