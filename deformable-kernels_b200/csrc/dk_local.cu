@@ -149,21 +149,30 @@ static int launch_local_conv(const T* src, const T* rot, const T* w, T* dst, con
         rc = local_conv_tc_rounded(src, rot, w, dst, g, TRANSPOSED, s);
         if (rc != DK_ERR_UNSUPPORTED) return rc;
       }
-      rc = local_conv_ring(src, rot, w, dst, g, TRANSPOSED, s);
-      if (rc != DK_ERR_UNSUPPORTED) return rc;
-      rc = local_conv_mma(src, rot, w, dst, g, TRANSPOSED, s);
+      if ((g.C & 15) == 0) {
+        rc = local_conv_ring(src, rot, w, dst, g, TRANSPOSED, s);
+        if (rc != DK_ERR_UNSUPPORTED) return rc;
+        rc = local_conv_mma(src, rot, w, dst, g, TRANSPOSED, s);
+        if (rc != DK_ERR_UNSUPPORTED) return rc;
+      }
+    }
+  }
+  // fp32, and fp16 with channel counts that are no multiple of 16: those have always been computed with fp32 kernel values.  fp16 with
+  // tcgen05 where TMA fetches the rows and there are three 32-channel groups or more, else with mma.sync (us, forward + grad-input,
+  // tcgen05 / mma.sync: 32 x 72 of 56 x 56 63 / 77, 64 x 72 of 16 x 16 21 / 23, 4 x 952 of 24 x 24 27 / 31; 128 x 104 of 8 x 8 23 / 18, 16 x 24 of
+  // 64 x 64 38 / 31, 64 x 24 of 112 x 112 364 / 278; rows that TMA does not fetch, 2 x 200 of 50 x 60 48 / 27, 32 x 200 of 28 x 28 77 / 58, but
+  // grad-input of 32 x 72 of 56 x 56 at stride 2 25 / 28).
+  if constexpr (sizeof(T) <= 4) {
+    const int Ws = TRANSPOSED ? g.Wo : g.W;
+    const bool rows = sizeof(T) == 4 || (g.C > 64 && ((Ws % 8 == 0 && Ws >= 16) || (TRANSPOSED && g.sW == 2 && Ws % 4 == 0 && Ws >= 28)));
+    if (rows && mma_path_enabled()) {
+      const int rc = local_conv_tc<T>(src, rot, w, dst, g, TRANSPOSED, s);
       if (rc != DK_ERR_UNSUPPORTED) return rc;
     }
   }
-  // fp32, and fp16 with channel counts that are no multiple of 16: those have always been computed with fp32 kernel values.  fp16
-  // where TMA or 8-byte copies of 28 columns and more fetch the rows (us, below -> these: 8 x 72 of 56 x 56 49 -> 16, 32 x 200 of 28 x 28
-  // 104 -> 48, grad-input of 32 x 72 of 56 x 56 at stride 2 127 -> 28; not 64 x 72 of 14 x 14 27 -> 37, 8 x 72 of 75 x 101 100 -> 129,
-  // forward of 32 x 200 of 28 x 28 at stride 2 41 -> 55).
-  if constexpr (sizeof(T) <= 4) {
-    const int Ws = TRANSPOSED ? g.Wo : g.W;
-    const bool rows = sizeof(T) == 4 || Ws % 8 == 0 || (Ws % 4 == 0 && Ws >= 28 && (TRANSPOSED || g.sW == 1));
-    if (rows && mma_path_enabled()) {
-      const int rc = local_conv_tc<T>(src, rot, w, dst, g, TRANSPOSED, s);
+  if constexpr (std::is_same<T, __half>::value) {
+    if (mma_path_enabled() && (g.C & 15)) {
+      const int rc = local_conv_mma(src, rot, w, dst, g, TRANSPOSED, s);
       if (rc != DK_ERR_UNSUPPORTED) return rc;
     }
   }

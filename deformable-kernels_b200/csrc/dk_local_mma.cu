@@ -205,14 +205,203 @@ __global__ void __launch_bounds__(448, 2) mma_conv_kernel(const __half* __restri
   }
 }
 
+// ------------------------------------------------------------------ the same in fp32 arithmetic, any number of channels
+// fp16 with channels that are no multiple of 16 has always been computed with fp32 kernel values: the hat products are two fp16 pieces (the
+// second the rest of the first, 2^-25 of the whole left out), the bank is exact, so two mma with fp32 sums give K, which then meets the
+// widened x.  Columns beside the image are zeros and not products with a zero kernel value, and a block whose bank holds a value that
+// is not finite computes every output by itself: such values stay with the samples that touch them.
+// Against gathered cells (local_conv_kernel: four reads and five multiply-adds per channel and tap), us, forward + grad-input: 8 x 72 of
+// 75 x 101 189 -> 133, 64 x 88 of 28 x 30 195 -> 55, 40 x 72 of 56 x 50 at stride 2 191 -> 53, 128 x 200 of 7 x 7 67 -> 30, 64 x 24 of 112 x 110
+// 790 -> 278, 64 x 8 of 56 x 54 at stride 2 54 -> 47, 1 x 72 of 28 x 30 21 -> 15.  Rows of odd width wait for their loader (8 x 72 of 75 x 102 73).
+template <int S, bool TRANSPOSED>
+__device__ __noinline__ float conv_alone(const __half* __restrict__ src, const __half* __restrict__ rot, const __half* __restrict__ w, const Geom& g,
+                                         int n, int c, int drow, int dcol) {
+  const int Hs = TRANSPOSED ? g.Ho : g.H, Ws = TRANSPOSED ? g.Wo : g.W;
+  const __half* plane = src + ((size_t)n * g.C + c) * Hs * Ws;
+  float sum = 0.f;
+  for (int t = 0; t < 9; ++t) {
+    const int fh = t / 3, fw = t - fh * 3;
+    int orow = drow, ocol = dcol, sr = drow * S - 1 + fh, sc = dcol * S - 1 + fw;
+    if (TRANSPOSED) {
+      const int tr = drow + 1 - fh, tc = dcol + 1 - fw;
+      if (tr < 0 || tc < 0 || tr % S || tc % S) continue;
+      orow = sr = tr / S, ocol = sc = tc / S;
+    }
+    if (sr < 0 || sr >= Hs || sc < 0 || sc >= Ws) continue;
+    const __half* r = rot + ((size_t)n * 18 + 2 * t) * g.P + orow * g.Wo + ocol;
+    Bilinear<float> b;
+    if (!bank_setup<float>(__half2float(r[0]), __half2float(r[g.P]), fh, fw, g, b)) continue;
+    float cf[4], k = 0.f;
+    bilinear_value_coefs(b, cf);
+    for (int e = 0; e < 4; ++e)
+      if (b.m[e]) k += cf[e] * __half2float(w[(size_t)c * g.cells + b.idx[e]]);
+    sum += k * __half2float(plane[sr * Ws + sc]);
+  }
+  return sum;
+}
+
+template <int S, bool TRANSPOSED>
+__global__ void __launch_bounds__(256, 2) mma_conv_full_kernel(const __half* __restrict__ src, const __half* __restrict__ rot,
+                                                               const __half* __restrict__ w, __half* __restrict__ dst, const Geom g,
+                                                               const ConvPlan pl) {
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  const int Hd = TRANSPOSED ? g.H : g.Ho, Wd = TRANSPOSED ? g.W : g.Wo;
+  const int Hs = TRANSPOSED ? g.Ho : g.H, Ws = TRANSPOSED ? g.Wo : g.W;
+  const int n = blockIdx.z;
+  const int c0 = blockIdx.y * pl.CG;
+  const int cnt = min(pl.CG, g.C - c0);
+  const int d_row0 = blockIdx.x * pl.BH;
+  const int RB = conv_band_rows(pl.BH, S, TRANSPOSED);
+  const int src_row_lo = TRANSPOSED ? (S == 1 ? d_row0 - 1 : d_row0 >> 1) : d_row0 * S - 1;
+  const Band bx = make_band(src_row_lo, RB, Hs, Ws, pl.mode_src);
+  const Band br = TRANSPOSED ? make_band(src_row_lo, RB, g.Ho, g.Wo, pl.mode_rot)
+                             : make_band(d_row0, pl.BH, g.Ho, g.Wo, pl.mode_rot);
+
+  __half* band = reinterpret_cast<__half*>(smem_raw);
+  __half* rband = band + pl.CG * bx.pitch_c;
+  __half* bank = rband + 18 * br.pitch_c;
+  bool finite = true;
+  for (int i = threadIdx.x; i < pl.CG * 16; i += blockDim.x) {
+    const int j = i >> 4, cell = i & 15;
+    const __half v = j < cnt && cell < g.cells ? __ldg(w + (size_t)(c0 + j) * g.cells + cell) : __float2half(0.f);
+    bank[j * kBankPitch + cell] = v;
+    finite &= fabsf(__half2float(v)) < INFINITY;
+  }
+  load_band<S == 1 ? 96 : 72>(band, bx, src, n, g.C, c0, cnt, Hs, Ws);
+  load_band<S == 1 ? 96 : 72>(rband, br, rot, n, 18, 0, 18, g.Ho, g.Wo);
+  cp_async_wait_all();
+  const size_t dplane = (size_t)Hd * Wd;
+  if (__syncthreads_or(!finite)) {
+    const int rows = min(pl.BH, Hd - d_row0);
+    for (int i = threadIdx.x; i < cnt * rows * Wd; i += blockDim.x) {
+      const int c = c0 + i / (rows * Wd), r = i % (rows * Wd);
+      dst[((size_t)n * g.C + c) * dplane + (size_t)d_row0 * Wd + r] =
+          __float2half_rn(conv_alone<S, TRANSPOSED>(src, rot, w, g, n, c, d_row0 + r / Wd, r % Wd));
+    }
+    return;
+  }
+
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nwarps = blockDim.x >> 5;
+  const int gq = lane >> 2, q = lane & 3;
+  const int NB = (Wd + 7) >> 3;
+  const int items = pl.BH * NB;
+  const LaneCells lc = lane_cells(g, q);
+  const float uh0 = (float)(g.scH - 3) * 0.5f, uw0 = (float)(g.scW - 3) * 0.5f;
+
+  for (int item = warp; item < items; item += nwarps) {
+    const int dr = item / NB;
+    const int drow = d_row0 + dr;
+    if (drow >= Hd) break;
+    const int ow0 = (item - dr * NB) << 3;
+    unsigned hi[9][2], lo[9][2];  // hat products of pixel ow0 + gq in cells 2 q, + 1 and 2 q + 8, + 9, as two pieces
+    {
+      const int pc = ow0 + gq;
+      const __half* base = rband + kSlack - br.org;
+#pragma unroll
+      for (int t = 0; t < 9; ++t) {
+        const int fh = t / 3, fw = t % 3;
+        int orow = drow, ocol = pc;
+        bool ok;
+        if (!TRANSPOSED) {
+          const int sr = drow * S - 1 + fh, sc = pc * S - 1 + fw;
+          ok = pc < Wd && sr >= 0 && sr < Hs && sc >= 0 && sc < Ws;
+        } else {
+          const int tr = drow + 1 - fh, tc = pc + 1 - fw;
+          orow = S == 1 ? tr : tr >> 1, ocol = S == 1 ? tc : tc >> 1;
+          ok = pc < Wd && tr >= 0 && tc >= 0 && (S == 1 || !((tr | tc) & 1)) && orow < Hs && ocol < Ws;
+          if (!ok) orow = max(br.row_lo, 0), ocol = 0;  // an unused tap reads (and ignores) some row of the band
+        }
+        if (!TRANSPOSED && !ok) ocol = 0;
+        const __half* rp = base + 2 * t * br.pitch_c + orow * br.Wp + ocol;
+        const float u = ((float)fh + __half2float(rp[0])) + uh0;
+        const float v = ok ? ((float)fw + __half2float(rp[br.pitch_c])) + uw0 : 1e30f;
+#pragma unroll
+        for (int k = 0; k < 2; ++k) {
+          const float b0 = lc.ok[2 * k] ? hat(u - lc.ca[2 * k]) * hat(v - lc.cb[2 * k]) : 0.f;
+          const float b1 = lc.ok[2 * k + 1] ? hat(u - lc.ca[2 * k + 1]) * hat(v - lc.cb[2 * k + 1]) : 0.f;
+          hi[t][k] = pack2(b0, b1);
+          lo[t][k] = pack2(b0 - lo2f(hi[t][k]), b1 - hi2f(hi[t][k]));
+        }
+      }
+    }
+    const int ow = ow0 + 2 * q;
+    const int j0 = ow >> 1;
+    const int wbase = (TRANSPOSED && S == 2) ? kSlack + (j0 & ~1) - bx.org
+                                             : window_offset(bx, TRANSPOSED ? drow - 1 : drow * S - 1, ow, S);
+    // rows of even width lie end to end: what a window reads beside the image is the neighbouring row
+    const bool left = ow == 0, right = S == 1 ? ow + 2 >= Ws : j0 + 1 >= Ws;
+    const unsigned* bkp = reinterpret_cast<const unsigned*>(bank + gq * kBankPitch) + q;
+    const __half* x0 = band + gq * bx.pitch_c + wbase;
+    const int xstep = 16 * bx.pitch_c, x8 = 8 * bx.pitch_c;
+    __half* y0 = dst + ((size_t)n * g.C + c0 + gq) * dplane + (size_t)drow * Wd + ow;
+#pragma unroll 1
+    for (int cb16 = 0; cb16 < cnt; cb16 += 16, bkp += 16 * kBankPitch / 2, x0 += xstep, y0 += 16 * dplane) {
+      const unsigned a[4] = {bkp[0], bkp[8 * kBankPitch / 2], bkp[4], bkp[8 * kBankPitch / 2 + 4]};
+      const __half* x1 = x0 + x8;
+      float acc[4] = {0.f, 0.f, 0.f, 0.f};
+      auto kernel_value = [&](float (&d)[4], int t) {
+        mma16816(d, a, lo[t][0], lo[t][1]);
+        mma16816_acc(d, a[0], a[1], a[2], a[3], hi[t][0], hi[t][1]);
+      };
+#pragma unroll
+      for (int fh = 0; fh < 3; ++fh) {
+        float d[3][4];
+        if (TRANSPOSED && S == 2) {
+          const int tr = drow + 1 - fh;
+          if (tr < 0 || (tr & 1)) continue;  // uniform over the warp
+          const unsigned sel = (j0 & 1) ? 0x5432u : 0x3210u;  // -> (dy[j0], dy[j0 + 1]) in one word
+          const unsigned* p0 = reinterpret_cast<const unsigned*>(x0 + (tr >> 1) * bx.Wp);
+          const unsigned* p1 = reinterpret_cast<const unsigned*>(x1 + (tr >> 1) * bx.Wp);
+          const unsigned ab0 = __byte_perm(p0[0], p0[1], sel), ab1 = __byte_perm(p1[0], p1[1], sel);
+          const float b0 = right ? 0.f : hi2f(ab0), b1 = right ? 0.f : hi2f(ab1);
+#pragma unroll
+          for (int fw = 0; fw < 3; ++fw) kernel_value(d[fw], fh * 3 + fw);
+          acc[1] = fmaf(b0, d[0][1], acc[1]), acc[3] = fmaf(b1, d[0][3], acc[3]);
+          acc[0] = fmaf(lo2f(ab0), d[1][0], acc[0]), acc[2] = fmaf(lo2f(ab1), d[1][2], acc[2]);
+          acc[1] = fmaf(lo2f(ab0), d[2][1], acc[1]), acc[3] = fmaf(lo2f(ab1), d[2][3], acc[3]);
+        } else {
+          const int rsel = TRANSPOSED ? 2 - fh : fh;
+          const unsigned* p0 = reinterpret_cast<const unsigned*>(x0 + rsel * bx.Wp);
+          const unsigned* p1 = reinterpret_cast<const unsigned*>(x1 + rsel * bx.Wp);
+          const unsigned w0 = p0[0], w1 = p0[1], w2 = p0[2], v0 = p1[0], v1 = p1[1], v2 = p1[2];
+          // halves 1 .. 5 of the windows
+          const float xa[5] = {left ? 0.f : hi2f(w0), lo2f(w1), hi2f(w1), S == 1 && right ? 0.f : lo2f(w2), hi2f(w2)};
+          const float xb[5] = {left ? 0.f : hi2f(v0), lo2f(v1), hi2f(v1), S == 1 && right ? 0.f : lo2f(v2), hi2f(v2)};
+#pragma unroll
+          for (int fw = 0; fw < 3; ++fw) kernel_value(d[fw], fh * 3 + fw);
+#pragma unroll
+          for (int fw = 0; fw < 3; ++fw) {
+            const int c = TRANSPOSED ? 2 - fw : fw;
+            acc[0] = fmaf(xa[c], d[fw][0], acc[0]), acc[1] = fmaf(xa[S + c], d[fw][1], acc[1]);
+            acc[2] = fmaf(xb[c], d[fw][2], acc[2]), acc[3] = fmaf(xb[S + c], d[fw][3], acc[3]);
+          }
+        }
+      }
+      if (ow < Wd) {
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+          if (cb16 + gq + 8 * h >= cnt) continue;
+          __half* y = y0 + 8 * h * dplane;
+          if (pl.pair_store) {
+            *reinterpret_cast<__half2*>(y) = __floats2half2_rn(acc[2 * h], acc[2 * h + 1]);
+          } else {
+            y[0] = __float2half_rn(acc[2 * h]);
+            if (ow + 1 < Wd) y[1] = __float2half_rn(acc[2 * h + 1]);
+          }
+        }
+      }
+    }
+  }
+}
+
 // shared memory per block that still lets two blocks share an SM (228 KB per SM, 1 KB reserved per block)
 constexpr size_t kTwoPerSm = 113 * 1024;
 constexpr size_t kOnePerSm = 226 * 1024;
 
-bool fast_shape(const Geom& g) {
+bool fast_shape(const Geom& g, bool any_channels = false) {
   if (g.kH != 3 || g.kW != 3 || g.dH != 1 || g.dW != 1 || g.pH != 1 || g.pW != 1) return false;
   if (g.sH != g.sW || (g.sH != 1 && g.sH != 2)) return false;
-  if (g.G != 1 || g.cells > 16 || (g.C & 15) || g.N > 65535) return false;
+  if (g.G != 1 || g.cells > 16 || (!any_channels && (g.C & 15)) || g.N > 65535) return false;
   return true;
 }
 
@@ -248,7 +437,7 @@ size_t conv_smem(const Geom& g, bool transposed, int cg, int bh) {
 }
 
 // Channel group, band height and warps per block are chosen together by an estimate of the time per output row.
-ConvPlan conv_plan_search(const Geom& g, bool transposed) {
+ConvPlan conv_plan_search(const Geom& g, bool transposed, bool full) {
   ConvPlan pl;
   const int S = g.sH;
   const int Hd = transposed ? g.H : g.Ho, Wd = transposed ? g.W : g.Wo;
@@ -285,16 +474,17 @@ ConvPlan conv_plan_search(const Geom& g, bool transposed) {
       const int rb = conv_band_rows(bh, S, transposed);
       const double staged = ((double)cg * rb * Ws + 18.0 * (transposed ? rb : bh) * g.Wo) / ((double)cg * bh * Wd);
       const double band_fill = (double)Hd / (bands * bh);
-      const int wmax = items < 2 ? 2 : (items < 14 ? items : 14);
+      const int most = full ? 8 : 14, sm_warps = full ? 16 : 28;  // 128 or 72 registers per thread
+      const int wmax = items < 2 ? 2 : (items < most ? items : most);
       for (int w = wmax; w >= 2 && w >= wmax / 2; --w) {
         int bpsm = (int)((228 * 1024) / (smem + 1024));
-        if (bpsm > 28 / w) bpsm = 28 / w;  // 72 registers per thread: 28 warps per SM
+        if (bpsm > sm_warps / w) bpsm = sm_warps / w;
         if (bpsm > 16) bpsm = 16;
         if (bpsm < 1) continue;
         const int rounds = (items + w - 1) / w;
         const double util = (double)items / (rounds * w);
         const int resident = bpsm * w;
-        const double occ = resident >= 20 ? 1.0 : 0.6 + 0.02 * resident;
+        const double occ = resident >= 20 || (full && resident >= 14) ? 1.0 : 0.6 + 0.02 * resident;
         const double cost = (per_item / (util * occ) + 46.0 * staged) / (wave_fill(ctas, bpsm) * band_fill);
         if (cost < best_cost) {
           best_cost = cost;
@@ -317,8 +507,8 @@ ConvPlan conv_plan_search(const Geom& g, bool transposed) {
   return pl;
 }
 
-ConvPlan conv_plan(const Geom& g, bool transposed) {
-  return cached_plan<ConvPlan>(g, transposed ? 1 : 0, [&] { return conv_plan_search(g, transposed); });
+ConvPlan conv_plan(const Geom& g, bool transposed) {  // channels that are no multiple of 16: of the fp32 kernel
+  return cached_plan<ConvPlan>(g, transposed ? 1 : 0, [&] { return conv_plan_search(g, transposed, g.C & 15); });
 }
 
 bool plan_launches(const ConvPlan& pl) { return pl.BH && pl.smem <= (size_t)device_smem_optin() && pl.groups <= 65535; }
@@ -330,7 +520,7 @@ int launch_conv(const __half* src, const __half* rot, const __half* w, __half* d
   pl.mode_src = ptr_mode(src);
   pl.mode_rot = ptr_mode(rot);
   pl.pair_store = (((TRANSPOSED ? g.W : g.Wo) & 1) == 0) && ptr_mode(dst) >= 1;
-  auto kern = mma_conv_kernel<S, TRANSPOSED>;
+  auto kern = g.C & 15 ? mma_conv_full_kernel<S, TRANSPOSED> : mma_conv_kernel<S, TRANSPOSED>;
   int rc = enable_smem(kern, pl.smem);
   if (rc) return rc;
   kern<<<dim3(pl.bands, pl.groups, g.N), pl.warps * 32, pl.smem, s>>>(src, rot, w, dst, g, pl);
@@ -1254,7 +1444,7 @@ bool local_conv_mma_takes(const Geom& g, bool transposed) {
 
 int local_conv_mma(const __half* src, const __half* rot, const __half* w, __half* dst, const Geom& g, bool transposed,
                    cudaStream_t s) {
-  if (!fast_shape(g)) return DK_ERR_UNSUPPORTED;
+  if (!fast_shape(g, true)) return DK_ERR_UNSUPPORTED;
   if (transposed) return g.sH == 1 ? launch_conv<1, true>(src, rot, w, dst, g, s) : launch_conv<2, true>(src, rot, w, dst, g, s);
   if (g.sH == 1) return launch_conv<1, false>(src, rot, w, dst, g, s);
   return launch_conv<2, false>(src, rot, w, dst, g, s);
