@@ -234,8 +234,8 @@ __global__ void __launch_bounds__(512, 1) mma_deform_fwd_kernel(const __half* __
     const Band br = make_band(oh0, pl.BH, g.Ho, g.Wo, pl.mode_rot);
     const Band bo = make_band(oh0, pl.BH, g.Ho, g.Wo, pl.mode_off);
     __syncthreads();  // readers of the previous unit are done
-    if (!zero_rot) load_band<0>(rband, br, rot, n, 18, 0, 18, g.Ho, g.Wo);
-    load_band<0>(oband, bo, off, n, 18, 0, 18, g.Ho, g.Wo);
+    if (!zero_rot) load_band(rband, br, rot, n, 18, 0, 18, g.Ho, g.Wo);
+    load_band(oband, bo, off, n, 18, 0, 18, g.Ho, g.Wo);
     if (n != cur_n) {
 #pragma unroll
       for (int sidx = 0; sidx < NS; ++sidx) load_pair_planes<S>(xw + (size_t)sidx * HW16 * 8, x, n, g.C, c0 + 16 * sidx, g.HW, pl.vec);
@@ -356,9 +356,9 @@ __global__ void __launch_bounds__(512, 1) mma_deform_filter_kernel(const __half*
     const Band br = make_band(oh0, pl.BH, g.Ho, g.Wo, pl.mode_rot);
     const Band bo = make_band(oh0, pl.BH, g.Ho, g.Wo, pl.mode_off);
     __syncthreads();  // readers of the previous unit are done
-    load_band<0>(yband, by, dy, n, g.C, c0, CG, g.Ho, g.Wo);
-    if (!zero_rot) load_band<0>(rband, br, rot, n, 18, 0, 18, g.Ho, g.Wo);
-    load_band<0>(oband, bo, off, n, 18, 0, 18, g.Ho, g.Wo);
+    load_band(yband, by, dy, n, g.C, c0, CG, g.Ho, g.Wo);
+    if (!zero_rot) load_band(rband, br, rot, n, 18, 0, 18, g.Ho, g.Wo);
+    load_band(oband, bo, off, n, 18, 0, 18, g.Ho, g.Wo);
     if (n != cur_n) {
 #pragma unroll
       for (int sidx = 0; sidx < NS; ++sidx) load_pair_planes<S>(xw + (size_t)sidx * HW16 * 8, x, n, g.C, c0 + 16 * sidx, g.HW, pl.vec);
@@ -846,9 +846,9 @@ __global__ void __launch_bounds__(DO_BANK ? 384 : 512, 1)  // the bank accumulat
     const Band br = make_band(oh0, pl.BH, g.Ho, g.Wo, pl.mode_rot);
     const Band bo = make_band(oh0, pl.BH, g.Ho, g.Wo, pl.mode_off);
     __syncthreads();  // readers of the previous unit are done
-    load_band<0>(yband, by, dy, n, g.C, c0, CG, g.Ho, g.Wo);
-    if (!zero_rot) load_band<0>(rband, br, rot, n, 18, 0, 18, g.Ho, g.Wo);
-    load_band<0>(oband, bo, off, n, 18, 0, 18, g.Ho, g.Wo);
+    load_band(yband, by, dy, n, g.C, c0, CG, g.Ho, g.Wo);
+    if (!zero_rot) load_band(rband, br, rot, n, 18, 0, 18, g.Ho, g.Wo);
+    load_band(oband, bo, off, n, 18, 0, 18, g.Ho, g.Wo);
     if (n != cur_n) {
 #pragma unroll
       for (int sidx = 0; sidx < NS; ++sidx) load_pair_planes<S>(xw + (size_t)sidx * HW16 * 8, x, n, g.C, c0 + 16 * sidx, g.HW, pl.vec);

@@ -98,8 +98,8 @@ __global__ void __launch_bounds__(448, 2) mma_conv_kernel(const __half* __restri
     const int j = i >> 4, cell = i & 15;
     bank[j * kBankPitch + cell] = cell < g.cells ? __ldg(w + (size_t)(c0 + j) * g.cells + cell) : __float2half(0.f);
   }
-  load_band<S == 1 ? 96 : 72>(band, bx, src, n, g.C, c0, cnt, Hs, Ws);
-  load_band<S == 1 ? 96 : 72>(rband, br, rot, n, 18, 0, 18, g.Ho, g.Wo);
+  load_band(band, bx, src, n, g.C, c0, cnt, Hs, Ws);
+  load_band(rband, br, rot, n, 18, 0, 18, g.Ho, g.Wo);
   cp_async_wait_all();
   __syncthreads();
 
@@ -212,7 +212,8 @@ __global__ void __launch_bounds__(448, 2) mma_conv_kernel(const __half* __restri
 // is not finite computes every output by itself: such values stay with the samples that touch them.
 // Against gathered cells (local_conv_kernel: four reads and five multiply-adds per channel and tap), us, forward + grad-input: 8 x 72 of
 // 75 x 101 189 -> 133, 64 x 88 of 28 x 30 195 -> 55, 40 x 72 of 56 x 50 at stride 2 191 -> 53, 128 x 200 of 7 x 7 67 -> 30, 64 x 24 of 112 x 110
-// 790 -> 278, 64 x 8 of 56 x 54 at stride 2 54 -> 47, 1 x 72 of 28 x 30 21 -> 15.  Rows of odd width wait for their loader (8 x 72 of 75 x 102 73).
+// 790 -> 278, 64 x 8 of 56 x 54 at stride 2 54 -> 47, 1 x 72 of 28 x 30 21 -> 15.  Rows of odd width wait for their loader (8 x 72 of 75 x 101 115
+// with its rows word by word, of 75 x 102 73).
 template <int S, bool TRANSPOSED>
 __device__ __noinline__ float conv_alone(const __half* __restrict__ src, const __half* __restrict__ rot, const __half* __restrict__ w, const Geom& g,
                                          int n, int c, int drow, int dcol) {
@@ -267,8 +268,8 @@ __global__ void __launch_bounds__(256, 2) mma_conv_full_kernel(const __half* __r
     bank[j * kBankPitch + cell] = v;
     finite &= fabsf(__half2float(v)) < INFINITY;
   }
-  load_band<S == 1 ? 96 : 72>(band, bx, src, n, g.C, c0, cnt, Hs, Ws);
-  load_band<S == 1 ? 96 : 72>(rband, br, rot, n, 18, 0, 18, g.Ho, g.Wo);
+  load_band(band, bx, src, n, g.C, c0, cnt, Hs, Ws);
+  load_band(rband, br, rot, n, 18, 0, 18, g.Ho, g.Wo);
   cp_async_wait_all();
   const size_t dplane = (size_t)Hd * Wd;
   if (__syncthreads_or(!finite)) {
@@ -583,9 +584,9 @@ __global__ void __launch_bounds__(MAXT, MINB) mma_rot_kernel(const __half* __res
     const int cell = i / cnt, c = i - cell * cnt;
     bankT[cell * pitchT + c] = cell < g.cells ? __ldg(w + (size_t)(c0 + c) * g.cells + cell) : __float2half(0.f);
   }
-  load_band<S == 1 ? 96 : 0>(xband, bx, x, n, g.C, c0, cnt, g.H, g.W);
-  if (!DYD) load_band<S == 1 ? 96 : 0>(yband, by, dy, n, g.C, c0, cnt, g.Ho, g.Wo);
-  load_band<S == 1 ? 96 : 0>(rband, br, rot, n, 18, 0, 18, g.Ho, g.Wo);
+  load_band(xband, bx, x, n, g.C, c0, cnt, g.H, g.W);
+  if (!DYD) load_band(yband, by, dy, n, g.C, c0, cnt, g.Ho, g.Wo);
+  load_band(rband, br, rot, n, 18, 0, 18, g.Ho, g.Wo);
   cp_async_wait_all();
   __syncthreads();
 
@@ -868,9 +869,9 @@ __global__ void __launch_bounds__(MAXT, MINB) mma_filter_kernel(const __half* __
     const Band by = make_band(oh0, pl.BH, g.Ho, g.Wo, pl.mode_dy);
     const Band br = make_band(oh0, pl.BH, g.Ho, g.Wo, pl.mode_rot);
     __syncthreads();  // previous unit's readers are done
-    load_band<0>(xband, bx, x, n, g.C, c0, cnt, g.H, g.W);
-    if (!DYM) load_band<0>(yband, by, dy, n, g.C, c0, cnt, g.Ho, g.Wo);
-    load_band<0>(rband, br, rot, n, 18, 0, 18, g.Ho, g.Wo);
+    load_band<false>(xband, bx, x, n, g.C, c0, cnt, g.H, g.W);
+    if (!DYM) load_band<false>(yband, by, dy, n, g.C, c0, cnt, g.Ho, g.Wo);
+    load_band<false>(rband, br, rot, n, 18, 0, 18, g.Ho, g.Wo);
     // DYM == 2: 16 bytes of every channel row of item it_ go to ring slot slot_, one row per lane and step
     auto ring_fill = [&](int it_, int slot_) {
       const int r_ = it_ / NB;
@@ -1169,9 +1170,9 @@ __global__ void __launch_bounds__(MAXT, MINB) mma_gw_kernel(const __half* __rest
     const Band by = make_band(oh0, pl.BH, g.Ho, g.Wo, pl.mode_dy);
     const Band br = make_band(oh0, pl.BH, g.Ho, g.Wo, pl.mode_rot);
     __syncthreads();  // previous unit's readers are done
-    load_band<0>(xband, bx, x, n, g.C, c0, cnt, g.H, g.W);
-    if (!DYD) load_band<0>(yband, by, dy, n, g.C, c0, cnt, g.Ho, g.Wo);
-    load_band<0>(rband, br, rot, n, 18, 0, 18, g.Ho, g.Wo);
+    load_band(xband, bx, x, n, g.C, c0, cnt, g.H, g.W);
+    if (!DYD) load_band(yband, by, dy, n, g.C, c0, cnt, g.Ho, g.Wo);
+    load_band(rband, br, rot, n, 18, 0, 18, g.Ho, g.Wo);
     cp_async_wait_all();
     __syncthreads();
     __half* drot_n = drot + (size_t)n * 18 * g.P;

@@ -141,16 +141,49 @@ inline int ptr_mode(const void* p) {
 // Copy the in-range source rows [row_lo, row_lo+RB) of channels c0 .. c0+cnt-1 of sample n into
 // the band with cp.async (16- or 4-byte pieces) and zero everything else of the band (slack,
 // rows outside the image).  Called by the whole block; the caller must execute
-// cp_async_wait_all() and __syncthreads() before reading.  Odd row widths fall back to plain
-// 2-byte copies behind an extra barrier.
+// cp_async_wait_all() and __syncthreads() before reading.  Odd row widths pass through
+// registers behind an extra barrier.
 // load_band_group: the same for a group of nt threads (whole warps) numbered tid = 0 .. nt-1 that synchronises on
 // named barrier bar_id (bar_id 0: the whole block, __syncthreads).
 __device__ __forceinline__ void group_sync(int bar_id, int nt) {
   if (bar_id == 0) __syncthreads();
   else asm volatile("bar.sync %0, %1;\n" ::"r"(bar_id), "r"(nt) : "memory");
 }
-// WIDE: odd widths above it are copied a warp per row; 0: none (kernels short of registers, or slower with them)
-template <int WIDE>
+// Rows of odd width.  The rows of a channel are one run of halves in global memory that starts on an odd half for every other channel or so;
+// the threads take its aligned words, four in flight each, and store the halves one by one: in the band a row starts on an even
+// half.  From `dst` (row 0 of the run, channel 0) on; `pitch` halves per channel, `Wp` per row.
+__device__ __forceinline__ void odd_rows(__half* __restrict__ dst, int pitch, int Wp, const __half* __restrict__ run, size_t plane, int cnt,
+                                         int rows, int Ws, int tid, int nt) {
+  const int span = rows * Ws, words = (span >> 1) + 1, total = cnt * words;
+  const unsigned by_words = words == 1 ? 0u : 0xffffffffu / words + 1, by_row = Ws == 1 ? 0u : 0xffffffffu / Ws + 1;
+  const int phase0 = (int)((reinterpret_cast<uintptr_t>(run) >> 1) & 1), step = (int)(plane & 1);
+  for (int first = tid; first < total; first += 4 * nt) {
+    unsigned v[4];
+    int c[4], p[4];
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+      const int idx = min(first + k * nt, total - 1);
+      c[k] = by_words ? (int)__umulhi((unsigned)idx, by_words) : idx;
+      p[k] = 2 * (idx - c[k] * words) - ((phase0 + c[k] * step) & 1);  // the word's first half in the run
+      const __half* a = run + (size_t)c[k] * plane + p[k];
+      if (p[k] >= 0 && p[k] + 1 < span) {
+        v[k] = __ldg(reinterpret_cast<const unsigned*>(a));
+      } else {  // the word hangs over an end of the run: nothing beside it is read
+        v[k] = p[k] >= 0 && p[k] < span ? __half_as_ushort(__ldg(a)) : 0u;
+        if (p[k] < 0) v[k] = (unsigned)__half_as_ushort(__ldg(a + 1)) << 16;
+      }
+    }
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+      if (first + k * nt >= total) break;
+      const int at = max(p[k], 0), r = by_row ? (int)__umulhi((unsigned)at, by_row) : at, col = p[k] - r * Ws;
+      __half* d = dst + c[k] * pitch + r * Wp + col;
+      if (p[k] >= 0 && p[k] < span) d[0] = __ushort_as_half((unsigned short)v[k]);
+      if (p[k] + 1 < span) d[col + 1 == Ws ? 1 + Wp - Ws : 1] = __ushort_as_half((unsigned short)(v[k] >> 16));
+    }
+  }
+}
+template <bool WORDS>
 __device__ __forceinline__ void load_band_group(__half* __restrict__ band, const Band& b, const __half* __restrict__ src, int n,
                                                 int C, int c0, int cnt, int Hs, int Ws, int tid, int nt, int bar_id) {
   const int lane = tid & 31, warp = tid >> 5, nwarps = nt >> 5;
@@ -164,34 +197,17 @@ __device__ __forceinline__ void load_band_group(__half* __restrict__ band, const
     for (int i = tid; i < nv; i += nt) b4[i] = z;
     if (r_e <= r_s) return;
     group_sync(bar_id, nt);
-    const int rows = r_e - r_s;
-    const int tasks = cnt * rows;
-    if (WIDE && Ws > WIDE) {
-      // 2-byte copies, a warp per (channel, row): neighbours on neighbouring lanes, up to four loads in flight each.  With a row per
-      // thread every lane is on a line of its own, but the lines are reused and more loads are in flight: on rows of 31 that is
-      // the faster way (forward 29 against 49 us), on rows of 101 it is not (66 against 41 us).  The line, by kernel: 96 at stride 1
-      // (40 x 64 channels, rows of 81, offsets and bank gradients 393 against 470 us), 72 in the forward at stride 2
-      // (rows of 67 49 / 57, of 79 103 / 74), never in the gradients at stride 2 (rows of 101 280 / 327).  The bank gradient has none: their
-      // registers cost rows below 96 two percent, rows above it go to another kernel.
-      for (int t = warp; t < tasks; t += nwarps) {
-        const int j = t / rows, r = r_s + (t - j * rows);
-        const __half* sp = s0 + (size_t)j * plane + (size_t)r * Ws + lane;
-        __half* dp = band + j * b.pitch_c + kSlack + (r * b.Wp - b.org) + lane;
-        for (int left = Ws - lane; left > 0; left -= 128, sp += 128, dp += 128) {
-          __half v[4];
-#pragma unroll
-          for (int k = 0; k < 4; ++k)
-            if (32 * k < left) v[k] = __ldg(sp + 32 * k);
-#pragma unroll
-          for (int k = 0; k < 4; ++k)
-            if (32 * k < left) dp[32 * k] = v[k];
-        }
-      }
+    // Short rows: a thread takes one (channel, row) and walks along it, eight independent loads in flight; every lane is on a line of its
+    // own, but the lines are reused (forward + backward of 128 x 384 of 7 x 7 67 us, word by word 86; 16 x 160 of 45 x 31 149 / 162, 4 x 32 of
+    // 73 x 79 79 / 87).  Longer rows word by word (8 x 64 of 75 x 101 209 -> 198, 20 x 64 of 63 x 97 at stride 2 221 -> 182), except in the
+    // bank gradient (!WORDS: 4 x 48 of 20 x 99 at stride 2 22 -> 30).
+    if (WORDS && Ws > 96) {
+      odd_rows(band + kSlack + (r_s * b.Wp - b.org), b.pitch_c, b.Wp, s0 + (size_t)r_s * Ws, plane, cnt, r_e - r_s, Ws, tid, nt);
       return;
     }
-    // short rows: a thread takes one (channel, row) and walks along it, eight independent loads in flight
+    const int tasks = cnt * (r_e - r_s);
     for (int t = tid; t < tasks; t += nt) {
-      const int j = t / rows, r = r_s + (t - j * rows);
+      const int j = t / (r_e - r_s), r = r_s + (t - j * (r_e - r_s));
       const __half* sp = s0 + (size_t)j * plane + (size_t)r * Ws;
       __half* dp = band + (size_t)j * b.pitch_c + kSlack + (r * b.Wp - b.org);
       for (int c0w = 0; c0w < Ws; c0w += 8) {
@@ -263,12 +279,12 @@ __device__ __forceinline__ void flat_copies(__half* __restrict__ band, int pitch
 // leave lanes idle on the last pass over a row and walk through the channels one after the other.  Same instruction count
 // (measured), 3-4 % less time in the four kernels.
 // Odd row widths, and bands without a row inside the image, go through load_band_group.
-template <int WIDE>
+template <bool WORDS>
 __device__ __forceinline__ void load_band_flat(__half* __restrict__ band, const Band& b, const __half* __restrict__ src, int n,
                                                int C, int c0, int cnt, int Hs, int Ws, int tid, int nt, int bar_id) {
   const int r_s = max(b.row_lo, 0), r_e = min(b.row_lo + b.RB, Hs);
   if (b.mode == 0 || r_e <= r_s) {
-    load_band_group<WIDE>(band, b, src, n, C, c0, cnt, Hs, Ws, tid, nt, bar_id);
+    load_band_group<WORDS>(band, b, src, n, C, c0, cnt, Hs, Ws, tid, nt, bar_id);
     return;
   }
   const size_t plane = (size_t)Hs * Ws;
@@ -299,10 +315,10 @@ __device__ __forceinline__ void load_band_flat(__half* __restrict__ band, const 
     }
   }
 }
-template <int WIDE>
+template <bool WORDS = true>
 __device__ __forceinline__ void load_band(__half* __restrict__ band, const Band& b, const __half* __restrict__ src, int n, int C,
                                           int c0, int cnt, int Hs, int Ws) {
-  load_band_flat<WIDE>(band, b, src, n, C, c0, cnt, Hs, Ws, threadIdx.x, blockDim.x, 0);
+  load_band_flat<WORDS>(band, b, src, n, C, c0, cnt, Hs, Ws, threadIdx.x, blockDim.x, 0);
 }
 
 // Offset (in halves, even) of the window of pixel pair (ow, ow+1), row selector 0, inside a channel band.
