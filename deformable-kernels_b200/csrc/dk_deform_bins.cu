@@ -36,6 +36,11 @@ struct BinPlan {
 __host__ __device__ inline int bank_unused_cell(const Geom& g) { return (g.scH + 2) * (g.scW + 2); }
 __host__ __device__ inline int bank_cells(const Geom& g) { return bank_unused_cell(g) + g.scW + 4; }
 
+// Without kernel-space offsets (rot null) the sampled kernel is the same at every pixel: in place of the bank its value per (tap,
+// channel) is laid out, and one read stands for four and their multiply-adds; the bank gradient meets the cells once per tap.  16 x 192
+// of 28 x 28, 3 x 3 scope: forward 39 -> 25 us, gather 53 -> 44, offsets 43 -> 31, bank 42 -> 33; 13 x 88 of 80 x 80 in fp16, all, 848 -> 646.
+__host__ __device__ inline bool fixed_kernel(const Geom& g, const void* rot) { return rot == nullptr && g.taps <= bank_cells(g); }
+
 // one sample point: corner coefficients of the image and of the bank, {bank cell * 32, column of the cell, pixel * Cp, 0}
 struct Rec {
   float4 ci, cb;
@@ -77,9 +82,22 @@ __device__ __forceinline__ int sample_cell(int i, int n, const T* __restrict__ o
     const float hh = 1.f - q.lh, hw = 1.f - q.lw, hu = 1.f - q.lu, hv = 1.f - q.lv;
     rec->ci = make_float4(hh * hw, hh * q.lw, q.lh * hw, q.lh * q.lw);
     rec->cb = make_float4(hu * hv, hu * q.lv, q.lu * hv, q.lu * q.lv);
-    rec->at = make_int4(((q.u0 + 1) * (g.scW + 2) + q.v0 + 1) * 32, q.w0 + 1, p * Cp, 0);
+    rec->at = make_int4((fixed_kernel(g, rot) ? tap : (q.u0 + 1) * (g.scW + 2) + q.v0 + 1) * 32, q.w0 + 1, p * Cp, 0);
   }
   return (q.h0 + 1) * (g.W + 1) + q.w0 + 1;
+}
+
+template <typename T>
+__device__ __forceinline__ float fixed_kernel_value(int tap, int c, const T* __restrict__ w, const Geom& g) {
+  const int fh = tap / g.kW, fw = tap - fh * g.kW;
+  Bilinear<float> b;
+  float k = 0.f;
+  if (bank_setup<float>(0.f, 0.f, fh, fw, g, b)) {
+    const float t[4] = {b.hh, b.hh, b.lh, b.lh}, u[4] = {b.hw, b.lw, b.hw, b.lw};
+    for (int e = 0; e < 4; ++e)
+      if (b.m[e]) k += t[e] * u[e] * ld<float>(w + (size_t)c * g.cells + b.idx[e]);
+  }
+  return k;
 }
 
 template <typename T>
@@ -128,7 +146,8 @@ __global__ void __launch_bounds__(kSortThreads, 2) dcn_bins_kernel(const T* __re
     const int cells = bank_cells(g);
     for (int i = (blockIdx.x - t.movers) * kSortThreads + tid; i >= 0 && i < cells * t.Cp; i += (gridDim.x - t.movers) * kSortThreads) {
       const int cell = i / t.Cp, c = i - cell * t.Cp, a = cell / (g.scW + 2) - 1, b = cell - (a + 1) * (g.scW + 2) - 1;
-      bankt[i] = c < g.C && a >= 0 && a < g.scH && b >= 0 && b < g.scW ? ld<float>(w + (size_t)c * g.cells + a * g.scW + b) : 0.f;
+      if (fixed_kernel(g, rot)) bankt[i] = c < g.C && cell < g.taps ? fixed_kernel_value<T>(cell, c, w, g) : 0.f;
+      else bankt[i] = c < g.C && a >= 0 && a < g.scH && b >= 0 && b < g.scW ? ld<float>(w + (size_t)c * g.cells + a * g.scW + b) : 0.f;
     }
   }
   if (n >= t.sorted) return;
@@ -215,7 +234,7 @@ __device__ __forceinline__ void put(float* p, const float (&v)[V]) {
 // of cells write their two rows of dx first, then the odd rows add theirs, so no element has two writers.  What a piece
 // carries past its end waits in `seam`.  A sample costs four shared loads of its record, one line of dy, four bank reads
 // and nine multiplications or multiply-adds per channel.
-template <typename T, int V>
+template <typename T, int V, bool FIXED>
 __global__ void __launch_bounds__(32 * kGatherWarps, 3) dcn_gather_kernel(const T* __restrict__ dyt, const int* __restrict__ starts,
                                                                        const Rec* __restrict__ recs, const T* __restrict__ w,
                                                                        T* __restrict__ dx, const Geom g, const BinPlan t) {
@@ -230,7 +249,8 @@ __global__ void __launch_bounds__(32 * kGatherWarps, 3) dcn_gather_kernel(const 
   float* acc = seam + (t.R + 1) * t.segs * 2 * CB;                     // [row][column][PITCH]
   for (int i = threadIdx.x; i < bank_cells(g) * CB; i += 32 * kGatherWarps) {
     const int cell = i / CB, a = cell / bw - 1, b = cell - (a + 1) * bw - 1, c = i % CB;
-    bank[i] = (c < n_c && a >= 0 && a < g.scH && b >= 0 && b < g.scW) ? ld<float>(w + (size_t)(c0 + c) * g.cells + a * g.scW + b) : 0.f;
+    if (FIXED) bank[i] = c < n_c && cell < g.taps ? fixed_kernel_value<T>(cell, c0 + c, w, g) : 0.f;
+    else bank[i] = (c < n_c && a >= 0 && a < g.scH && b >= 0 && b < g.scW) ? ld<float>(w + (size_t)(c0 + c) * g.cells + a * g.scW + b) : 0.f;
   }
   __syncthreads();
   const T* yl = dyt + (size_t)n * (g.P + 1) * t.Cp + c0 + V * lane;
@@ -294,15 +314,16 @@ __global__ void __launch_bounds__(32 * kGatherWarps, 3) dcn_gather_kernel(const 
           for (int j = 0; j < 8; ++j) get<T, V>(yl + reinterpret_cast<const int*>(stage + (k0 + j) * 3 + 2)[2], yv[j]);
 #pragma unroll
           for (int j = 0; j < 8; ++j) {
-            const float4 ci = stage[(k0 + j) * 3], cb = stage[(k0 + j) * 3 + 1];
+            const float4 ci = stage[(k0 + j) * 3], cb = FIXED ? none : stage[(k0 + j) * 3 + 1];
             const int2 at2 = *reinterpret_cast<const int2*>(stage + (k0 + j) * 3 + 2);
             while (cur < at2.y) flush();
             const float* bk = bl + at2.x * V;
             float b0v[V], b1v[V], b2v[V], b3v[V];
-            get<float, V>(bk, b0v), get<float, V>(bk + CB, b1v), get<float, V>(bk + bw * CB, b2v), get<float, V>(bk + bw * CB + CB, b3v);
+            get<float, V>(bk, b0v);
+            if (!FIXED) get<float, V>(bk + CB, b1v), get<float, V>(bk + bw * CB, b2v), get<float, V>(bk + bw * CB + CB, b3v);
 #pragma unroll
             for (int e = 0; e < V; ++e) {
-              const float kv = cb.x * b0v[e] + cb.y * b1v[e] + cb.z * b2v[e] + cb.w * b3v[e];
+              const float kv = FIXED ? b0v[e] : cb.x * b0v[e] + cb.y * b1v[e] + cb.z * b2v[e] + cb.w * b3v[e];
               const float v = kv * yv[j][e];
               s00[e] += ci.x * v, s01[e] += ci.y * v, s10[e] += ci.z * v, s11[e] += ci.w * v;
             }
@@ -389,7 +410,7 @@ __device__ __forceinline__ void tap_record(int flat, int total, int tap, const T
 // they are stored along the pixels.  14 multiply-adds per sample and channel.
 constexpr int kForwardTaps = 9;
 
-template <typename T, int V>
+template <typename T, int V, bool FIXED>
 __global__ void __launch_bounds__(32 * kRowWarps, 3) dcn_forward_kernel(const T* __restrict__ xt, const float* __restrict__ bankt,
                                                                         const T* __restrict__ off, const T* __restrict__ rot,
                                                                         T* __restrict__ y, const Geom g, const int Cp) {
@@ -418,8 +439,12 @@ __global__ void __launch_bounds__(32 * kRowWarps, 3) dcn_forward_kernel(const T*
           const int4 idx = r.idx;
           const unsigned bk = r.at.y + ck;
           get_at<T, V>(xt, idx.x + cb, x[h][0]), get_at<T, V>(xt, idx.y + cb, x[h][1]), get_at<T, V>(xt, idx.z + cb, x[h][2]), get_at<T, V>(xt, idx.w + cb, x[h][3]);
-          get_at<float, V>(bankt, bk, k[h][0]), get_at<float, V>(bankt, bk + cell, k[h][1]);
-          get_at<float, V>(bankt, bk + row, k[h][2]), get_at<float, V>(bankt, bk + row + cell, k[h][3]);
+          if (FIXED) {
+            if (h == 0) get_at<float, V>(bankt, tap * cell + ck, k[0][0]);
+          } else {
+            get_at<float, V>(bankt, bk, k[h][0]), get_at<float, V>(bankt, bk + cell, k[h][1]);
+            get_at<float, V>(bankt, bk + row, k[h][2]), get_at<float, V>(bankt, bk + row + cell, k[h][3]);
+          }
         }
 #pragma unroll
         for (int h = 0; h < 2; ++h) {
@@ -427,7 +452,8 @@ __global__ void __launch_bounds__(32 * kRowWarps, 3) dcn_forward_kernel(const T*
 #pragma unroll
           for (int e = 0; e < V; ++e) {
             const float xs = im.x * (im.z * x[h][0][e] + im.w * x[h][1][e]) + im.y * (im.z * x[h][2][e] + im.w * x[h][3][e]);
-            acc[h][e] += xs * (b.x * (b.z * k[h][0][e] + b.w * k[h][1][e]) + b.y * (b.z * k[h][2][e] + b.w * k[h][3][e]));
+            if (FIXED) acc[h][e] += xs * k[0][0][e];
+            else acc[h][e] += xs * (b.x * (b.z * k[h][0][e] + b.w * k[h][1][e]) + b.y * (b.z * k[h][2][e] + b.w * k[h][3][e]));
           }
         }
       }
@@ -447,7 +473,7 @@ __global__ void __launch_bounds__(32 * kRowWarps, 3) dcn_forward_kernel(const T*
 
 // Both offset gradients.  S warps share the channels of a unit; the sum over the lanes leaves a quarter of the four sums on each.
 // 28 multiplications and additions per sample and channel, nine loads of a line.
-template <typename T, int V, bool ROT>
+template <typename T, int V, bool ROT, bool FIXED>
 __global__ void __launch_bounds__(32 * kRowWarps, 3) dcn_coords_kernel(const T* __restrict__ dyt, const T* __restrict__ xt,
                                                                        const float* __restrict__ bankt, const T* __restrict__ off,
                                                                        const T* __restrict__ rot, T* __restrict__ doff,
@@ -474,8 +500,12 @@ __global__ void __launch_bounds__(32 * kRowWarps, 3) dcn_coords_kernel(const T* 
         get_at<T, V>(xt, idx.x + cb, x[h][0]), get_at<T, V>(xt, idx.y + cb, x[h][1]), get_at<T, V>(xt, idx.z + cb, x[h][2]), get_at<T, V>(xt, idx.w + cb, x[h][3]);
         get_at<T, V>(dyt, at.x + cb, y[h]);
         const unsigned bk = at.y + c * (unsigned)sizeof(float);
-        get_at<float, V>(bankt, bk, k[h][0]), get_at<float, V>(bankt, bk + cell, k[h][1]);
-        get_at<float, V>(bankt, bk + row, k[h][2]), get_at<float, V>(bankt, bk + row + cell, k[h][3]);
+        if (FIXED) {
+          if (h == 0) get_at<float, V>(bankt, tap * cell + c * (unsigned)sizeof(float), k[0][0]);
+        } else {
+          get_at<float, V>(bankt, bk, k[h][0]), get_at<float, V>(bankt, bk + cell, k[h][1]);
+          get_at<float, V>(bankt, bk + row, k[h][2]), get_at<float, V>(bankt, bk + row + cell, k[h][3]);
+        }
       }
 #pragma unroll
       for (int h = 0; h < 2; ++h) {
@@ -483,8 +513,8 @@ __global__ void __launch_bounds__(32 * kRowWarps, 3) dcn_coords_kernel(const T* 
 #pragma unroll
         for (int e = 0; e < V; ++e) {
           const float top = im.z * x[h][0][e] + im.w * x[h][1][e], low = im.z * x[h][2][e] + im.w * x[h][3][e];
-          const float ktop = b.z * k[h][0][e] + b.w * k[h][1][e], klow = b.z * k[h][2][e] + b.w * k[h][3][e];
-          const float yk = y[h][e] * (b.x * ktop + b.y * klow);
+          const float ktop = FIXED ? 0.f : b.z * k[h][0][e] + b.w * k[h][1][e], klow = FIXED ? 0.f : b.z * k[h][2][e] + b.w * k[h][3][e];
+          const float yk = y[h][e] * (FIXED ? k[0][0][e] : b.x * ktop + b.y * klow);
           s[h][0] += yk * (low - top);
           s[h][1] += yk * (im.x * (x[h][1][e] - x[h][0][e]) + im.y * (x[h][3][e] - x[h][2][e]));
           if (ROT) {
@@ -558,6 +588,75 @@ __device__ __noinline__ void rows_bank_by_cells(float* acc, const T* __restrict_
         }
       }
     }
+  }
+}
+
+// Bank gradient without kernel-space offsets: the samples of a tap go to the same cells at every pixel, so their products are summed per tap and
+// only the nine sums meet the cells.  A warp takes a run of units (32 pixels of a tap) and lays a sum down where the tap changes.
+template <typename T, int V>
+__global__ void __launch_bounds__(32 * kRowWarps, 3) dcn_fixed_bank_kernel(const T* __restrict__ dyt, const T* __restrict__ xt,
+                                                                           const T* __restrict__ off, float* __restrict__ partial,
+                                                                           const __grid_constant__ Geom g, const int Cp) {
+  constexpr int CB = 32 * V;
+  extern __shared__ __align__(16) unsigned char smem[];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, c0 = blockIdx.y * CB, cb = (c0 + V * lane) * (int)sizeof(T);
+  TapRec* recs = reinterpret_cast<TapRec*>(smem) + warp * 32;
+  float* sums = reinterpret_cast<float*>(reinterpret_cast<TapRec*>(smem) + kRowWarps * 32);  // [warp][tap][CB]
+  float* mine = sums + warp * g.taps * CB + V * lane;
+  for (int tap = 0; tap < g.taps; ++tap)
+    for (int e = 0; e < V; ++e) mine[tap * CB + e] = 0.f;
+  const int total = g.N * g.P, tiles = (total + 31) / 32, units = g.taps * tiles, runs = gridDim.x * kRowWarps, run = blockIdx.x * kRowWarps + warp;
+  const int first = (int)((long long)units * run / runs), last = (int)((long long)units * (run + 1) / runs);
+  float acc[V] = {};
+  for (int u = first; u < last; ++u) {
+    const int tap = u / tiles, flat0 = (u - tap * tiles) * 32, cnt = min(32, total - flat0);
+    __syncwarp();
+    tap_record<T, false>(flat0 + lane, total, tap, off, (const T*)nullptr, g, Cp, recs + lane);
+    __syncwarp();
+    float part[V] = {};
+    for (int j = 0; j < cnt; j += 4) {
+      float x[4][4][V], y[4][V];
+#pragma unroll
+      for (int h = 0; h < 4; ++h) {
+        const int4 idx = recs[j + h].idx;
+        get_at<T, V>(xt, idx.x + cb, x[h][0]), get_at<T, V>(xt, idx.y + cb, x[h][1]), get_at<T, V>(xt, idx.z + cb, x[h][2]), get_at<T, V>(xt, idx.w + cb, x[h][3]);
+        get_at<T, V>(dyt, recs[j + h].at.x + cb, y[h]);
+      }
+#pragma unroll
+      for (int h = 0; h < 4; ++h) {
+        const float4 im = recs[j + h].im;
+#pragma unroll
+        for (int e = 0; e < V; ++e)
+          part[e] += y[h][e] * (im.x * (im.z * x[h][0][e] + im.w * x[h][1][e]) + im.y * (im.z * x[h][2][e] + im.w * x[h][3][e]));
+      }
+    }
+#pragma unroll
+    for (int e = 0; e < V; ++e) acc[e] += part[e];
+    if (u + 1 == last || (u + 1) / tiles != tap) {
+#pragma unroll
+      for (int e = 0; e < V; ++e) mine[tap * CB + e] = acc[e], acc[e] = 0.f;
+    }
+  }
+  __syncthreads();
+  for (int i = threadIdx.x; i < g.taps * CB; i += 32 * kRowWarps) {
+    float s = 0.f;
+#pragma unroll
+    for (int k = 0; k < kRowWarps; ++k) s += sums[k * g.taps * CB + i];
+    sums[i] = s;  // in the first warp's room, which this thread alone has read at i
+  }
+  __syncthreads();
+  for (int i = threadIdx.x; i < g.cells * CB; i += 32 * kRowWarps) {
+    const int cell = i / CB, a = cell / g.scW, b = cell - a * g.scW, ch = i % CB;
+    if (c0 + ch >= g.C) continue;
+    float s = 0.f;
+    for (int tap = 0; tap < g.taps; ++tap) {
+      const int fh = tap / g.kW, fw = tap - fh * g.kW;
+      const float u = (float)fh + (float)(g.scH - g.kH) * 0.5f, v = (float)fw + (float)(g.scW - g.kW) * 0.5f;
+      const int da = a - (int)floorf(u), db = b - (int)floorf(v);  // one of the four cells of the tap's samples?
+      if (da < 0 || da > 1 || db < 0 || db > 1 || !(u > -1.f && v > -1.f && u < (float)g.scH && v < (float)g.scW)) continue;
+      s += (1.f - fabsf(u - (float)a)) * (1.f - fabsf(v - (float)b)) * sums[tap * CB + ch];
+    }
+    partial[((size_t)blockIdx.x * g.C + c0 + ch) * g.cells + cell] = s;
   }
 }
 
@@ -738,8 +837,10 @@ static int launch_bins(const T* dy, const T* x, const T* off, const T* rot, cons
 }
 
 template <typename T>
-static int launch_gather(const T* dyt, const int* starts, const Rec* recs, const T* w, T* dx, const Geom& g, const BinPlan& t, cudaStream_t s) {
-  auto gather = t.V == 1 ? dcn_gather_kernel<T, 1> : dcn_gather_kernel<T, 2>;
+static int launch_gather(const T* dyt, const int* starts, const Rec* recs, const T* w, T* dx, const Geom& g, const BinPlan& t, bool fixed,
+                         cudaStream_t s) {
+  auto gather = fixed ? (t.V == 1 ? dcn_gather_kernel<T, 1, true> : dcn_gather_kernel<T, 2, true>)
+                      : (t.V == 1 ? dcn_gather_kernel<T, 1, false> : dcn_gather_kernel<T, 2, false>);
   const int rc = enable_smem(gather, t.gather_smem);
   if (rc) return rc;
   gather<<<dim3((unsigned)(g.N * t.bands), t.groups), 32 * kGatherWarps, t.gather_smem, s>>>(dyt, starts, recs, w, dx, g, t);
@@ -769,21 +870,30 @@ int deform_backward_rows(const T* dy, const T* x, const T* off, const T* rot, co
   float* partial = reinterpret_cast<float*>(at + t.bytes + t.xt_bytes + t.bankt_bytes);
   int rc = launch_bins<T>(dy, x, off, rot, w, dx != nullptr, starts, recs, dyt, coords || bank ? xt : nullptr, bankt, g, t, s);
   if (rc) return rc;
-  if (dx && (rc = launch_gather<T>(dyt, starts, recs, w, dx, g, t, s))) return rc;
+  const bool fixed = fixed_kernel(g, rot);
+  if (dx && (rc = launch_gather<T>(dyt, starts, recs, w, dx, g, t, fixed, s))) return rc;
   const int V = t.Cp % 64 == 0 ? 2 : 1, groups = t.Cp / (32 * V), units = g.taps * ((g.N * g.P + 31) / 32);
   if (coords) {
     // warps share a unit's channels until there are 16 on every SM
     int S = 1;
     while (S < kRowWarps && 2 * S <= groups && (long long)units * S < 16 * device_sm_count()) S *= 2;
-    auto kern = V == 2 ? (drot ? dcn_coords_kernel<T, 2, true> : dcn_coords_kernel<T, 2, false>)
-                       : (drot ? dcn_coords_kernel<T, 1, true> : dcn_coords_kernel<T, 1, false>);
+    auto kern = fixed ? (V == 2 ? dcn_coords_kernel<T, 2, false, true> : dcn_coords_kernel<T, 1, false, true>)
+                : V == 2 ? (drot ? dcn_coords_kernel<T, 2, true, false> : dcn_coords_kernel<T, 2, false, false>)
+                         : (drot ? dcn_coords_kernel<T, 1, true, false> : dcn_coords_kernel<T, 1, false, false>);
     const int per_block = kRowWarps / S;
     kern<<<(units + per_block - 1) / per_block, 32 * kRowWarps, 0, s>>>(dyt, xt, bankt, off, rot, doff, drot, g, t.Cp, S);
     if ((rc = check_launch())) return rc;
   }
   if (bank) {
-    auto kern = V == 2 ? dcn_bank_kernel<T, 2> : dcn_bank_kernel<T, 1>;
-    kern<<<dim3(t.bank_blocks, groups), 32 * kRowWarps, 0, s>>>(dyt, xt, off, rot, partial, g, t.Cp);
+    const size_t fixed_smem = kRowWarps * (32 * sizeof(TapRec) + (size_t)g.taps * 32 * V * sizeof(float));
+    if (fixed && fixed_smem <= 100 * 1024) {
+      auto kern = V == 2 ? dcn_fixed_bank_kernel<T, 2> : dcn_fixed_bank_kernel<T, 1>;
+      if ((rc = enable_smem(kern, fixed_smem))) return rc;
+      kern<<<dim3(t.bank_blocks, groups), 32 * kRowWarps, fixed_smem, s>>>(dyt, xt, off, partial, g, t.Cp);
+    } else {
+      auto kern = V == 2 ? dcn_bank_kernel<T, 2> : dcn_bank_kernel<T, 1>;
+      kern<<<dim3(t.bank_blocks, groups), 32 * kRowWarps, 0, s>>>(dyt, xt, off, rot, partial, g, t.Cp);
+    }
     if ((rc = check_launch())) return rc;
     if ((rc = reduce_bank<T>(partial, dw, g.C * g.cells, t.bank_blocks, s))) return rc;
     *bank_done = true;
@@ -813,7 +923,8 @@ int deform_forward_rows(const T* x, const T* off, const T* rot, const T* w, T* y
   const int V = t.Cp % 64 == 0 ? 2 : 1, groups = t.Cp / (32 * V), tiles = (g.N * g.P + 31) / 32;
   int split = (3 * device_sm_count() + tiles - 1) / tiles;  // blocks share the channels until there are three on every SM
   if (split > groups) split = groups;
-  auto kern = V == 2 ? dcn_forward_kernel<T, 2> : dcn_forward_kernel<T, 1>;
+  auto kern = fixed_kernel(g, rot) ? (V == 2 ? dcn_forward_kernel<T, 2, true> : dcn_forward_kernel<T, 1, true>)
+                                   : (V == 2 ? dcn_forward_kernel<T, 2, false> : dcn_forward_kernel<T, 1, false>);
   kern<<<dim3(tiles, split), 32 * kRowWarps, 0, s>>>(xt, bankt, off, rot, y, g, t.Cp);
   return check_launch();
 }
