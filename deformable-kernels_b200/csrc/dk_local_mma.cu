@@ -437,6 +437,41 @@ size_t conv_smem(const Geom& g, bool transposed, int cg, int bh) {
          (size_t)cg * kBankPitch * 2;
 }
 
+// A call of up to some 26 (item, slab) pairs per SM (20 with rows of odd width) is a chain of latencies: the loads of a band one after the other (rows of odd width pass through
+// registers, eight halves a trip), then the hat products of a warp's items and their slabs; the warps of a scheduler and the blocks of
+// an SM add what they issue.  Few channels a block, and one item a warp, shorten the chain as long as each SM has one block.  The weights
+// are us, from 384 x 14 x 14 (channels / rows / warps: 16/4/8 4.0, 32/4/8 4.6, 96/4/8 6.8, 16/4/6 4.7, 16/7/14 4.6, 16/2/4 with 168 blocks 4.3),
+// 960 x 7 x 7 (16/4/4 4.4, 16/2/2 with 240 blocks 5.0) and 3 x 56 of 16 x 17 (16/2/6 5.6, 64/2/6 8.0).
+void small_conv_plan(const Geom& g, bool transposed, bool full, size_t budget, ConvPlan& pl) {
+  const int S = g.sH, Hd = transposed ? g.H : g.Ho, Wd = transposed ? g.W : g.Wo, Hs = transposed ? g.Ho : g.H, Ws = transposed ? g.Wo : g.W;
+  const int NB = (Wd + 7) / 8, slabs_all = (g.C + 15) / 16, most = full ? 8 : 14;
+  double best = 1e30;
+  for (int ngrp = slabs_all; ngrp >= 1; --ngrp) {
+    const int slabs = (slabs_all + ngrp - 1) / ngrp, cg = 16 * slabs, groups = (g.C + cg - 1) / cg;
+    if (groups != ngrp) continue;
+    for (int bh = 1; bh <= Hd; ++bh) {
+      const size_t smem = conv_smem(g, transposed, cg, bh);
+      if (smem > budget) break;
+      const int items = bh * NB, rb = conv_band_rows(bh, S, transposed), rot_rows = transposed ? rb : bh;
+      const int per_sm = (int)(((long long)((Hd + bh - 1) / bh) * groups * g.N + 147) / 148);
+      for (int rounds = (items + most - 1) / most, last = rounds + 2; rounds <= last; ++rounds) {
+        const int w = max((items + rounds - 1) / rounds, 2), threads = 32 * w;
+        auto trips = [&](int channels, int rows, int width) {
+          return width & 1 ? (double)((channels * rows + threads - 1) / threads) * ((width + 7) / 8) : 0.025 * channels * rows * width / threads;
+        };
+        const double load = 0.27 * (trips(cg, min(rb, Hs), Ws) + trips(18, min(rot_rows, g.Ho), g.Wo)) + 0.1 * (cg * 16 / threads);
+        const double chain = rounds * (0.1 + 0.55 * slabs);
+        const double issue = (per_sm * ((w + 3) / 4) - 1) * rounds * ((full ? 0.25 : 0.13) + 0.115 * slabs);
+        const double cost = load + chain + issue + 0.3 * (per_sm - 1);
+        if (cost < best) {
+          best = cost;
+          pl.BH = bh, pl.CG = cg, pl.groups = groups, pl.warps = w;
+        }
+      }
+    }
+  }
+}
+
 // Channel group, band height and warps per block are chosen together by an estimate of the time per output row.
 ConvPlan conv_plan_search(const Geom& g, bool transposed, bool full) {
   ConvPlan pl;
@@ -498,6 +533,8 @@ ConvPlan conv_plan_search(const Geom& g, bool transposed, bool full) {
     }
     if (cg_only) break;
   }
+  const bool odd = (transposed ? g.Wo : g.W) & 1;
+  if (!cg_only && (long long)g.N * Hd * NB * ((g.C + 15) / 16) <= 148LL * (odd ? 20 : 26)) small_conv_plan(g, transposed, full, budget, pl);
   if (!pl.BH) {  // no block shape fits the budget: the caller falls back to the SIMT kernels
     pl.CG = pl.groups = pl.warps = pl.bands = 0;
     pl.smem = 0;
