@@ -134,6 +134,12 @@ static int launch_local_conv(const T* src, const T* rot, const T* w, T* dst, con
   if constexpr (std::is_same<T, __half>::value) {
     if (mma_path_enabled()) {
       int rc = DK_ERR_UNSUPPORTED;
+      // small calls: the band kernels in their own block shape, against the ring and tcgen05 kernels (192 x 28 x 28, forward and grad-input,
+      // 10.4, 9.8 -> 4.8, 4.2 us; 160 x 32 x 32 8.5, 7.9 -> 4.6, 4.2; 72 x 64 x 64 9.3, 8.9 -> 6.7, 5.9)
+      if (local_conv_mma_small(g, TRANSPOSED)) {
+        rc = local_conv_mma(src, rot, w, dst, g, TRANSPOSED, s);
+        if (rc != DK_ERR_UNSUPPORTED) return rc;
+      }
       // stride 1, rows that TMA fetches, three 32-channel groups or more: a pair of groups leaves half of the consumer warps
       // idle at a time.  Against the band kernels on rows of 16 .. 96, 72 .. 384 channels 1.0 to 1.6 times as fast (C = 384,
       // 32 x 32: 45 -> 29 us).  Against the ring kernels, forward and grad-input: rows of 112, batch 64 and 32, C = 80 137, 144 ->

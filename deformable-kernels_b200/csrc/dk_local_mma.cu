@@ -72,7 +72,9 @@ __host__ __device__ inline int conv_band_rows(int bh, int S, bool transposed) {
   return S == 1 ? bh + 2 : (bh >> 1) + 2;
 }
 
-template <int S, bool TRANSPOSED>
+// EDGES: what a window reads beside the image is set to zero.  Without it the neighbouring row's element meets a kernel value of zero, which is
+// the same for finite elements only; small calls take the place of kernels whose padding is real zeros (ring, tcgen05) and pay the selects.
+template <int S, bool TRANSPOSED, bool EDGES>
 __global__ void __launch_bounds__(448, 2) mma_conv_kernel(const __half* __restrict__ src, const __half* __restrict__ rot,
                                                           const __half* __restrict__ w, __half* __restrict__ dst, const Geom g,
                                                           const ConvPlan pl) {
@@ -125,6 +127,7 @@ __global__ void __launch_bounds__(448, 2) mma_conv_kernel(const __half* __restri
     const int j0 = ow >> 1;
     const int wbase = (TRANSPOSED && S == 2) ? kSlack + (j0 & ~1) - bx.org
                                              : window_offset(bx, TRANSPOSED ? drow - 1 : drow * S - 1, ow, S);
+    const bool left = EDGES && ow == 0, right = EDGES && (S == 1 ? ow + 2 >= Ws : j0 + 1 >= Ws);
     const unsigned* bkp = reinterpret_cast<const unsigned*>(bank + gq * kBankPitch) + q;
     const __half* x0 = band + gq * bx.pitch_c + wbase;
     const int xstep = 16 * bx.pitch_c, x8 = 8 * bx.pitch_c;
@@ -148,7 +151,8 @@ __global__ void __launch_bounds__(448, 2) mma_conv_kernel(const __half* __restri
           const int orow = tr >> 1;
           const unsigned* p0 = reinterpret_cast<const unsigned*>(x0 + orow * bx.Wp);
           const unsigned* p1 = reinterpret_cast<const unsigned*>(x1 + orow * bx.Wp);
-          const unsigned ab0 = __byte_perm(p0[0], p0[1], sel), ab1 = __byte_perm(p1[0], p1[1], sel);
+          unsigned ab0 = __byte_perm(p0[0], p0[1], sel), ab1 = __byte_perm(p1[0], p1[1], sel);
+          if (right) ab0 &= 0xffffu, ab1 &= 0xffffu;
           unsigned d[2];
           mma16816_h(d, a, bf[fh * 3 + 0][0], bf[fh * 3 + 0][1]);
           fma_hh<1, 1>(acc[1], ab0, d[0]);
@@ -166,8 +170,8 @@ __global__ void __launch_bounds__(448, 2) mma_conv_kernel(const __half* __restri
           const int rsel = TRANSPOSED ? 2 - fh : fh;
           const unsigned* p0 = reinterpret_cast<const unsigned*>(x0 + rsel * bx.Wp);
           const unsigned* p1 = reinterpret_cast<const unsigned*>(x1 + rsel * bx.Wp);
-          const unsigned w0 = p0[0], w1 = p0[1], w2 = p0[2];
-          const unsigned v0 = p1[0], v1 = p1[1], v2 = p1[2];
+          const unsigned w0 = left ? 0u : p0[0], w1 = p0[1], w2 = S == 1 && right ? 0u : p0[2];
+          const unsigned v0 = left ? 0u : p1[0], v1 = p1[1], v2 = S == 1 && right ? 0u : p1[2];
           unsigned d[3][2];
 #pragma unroll
           for (int fw = 0; fw < 3; ++fw) mma16816_h(d[fw], a, bf[fh * 3 + fw][0], bf[fh * 3 + fw][1]);
@@ -437,7 +441,17 @@ size_t conv_smem(const Geom& g, bool transposed, int cg, int bh) {
          (size_t)cg * kBankPitch * 2;
 }
 
-// A call of up to some 26 (item, slab) pairs per SM (20 with rows of odd width) is a chain of latencies: the loads of a band one after the other (rows of odd width pass through
+// The line between small calls and the others, in (item, slab) pairs per SM.  The other side is the ring and tcgen05 kernels or a block shape
+// from the estimate for large calls (us, small / other): 8 x 192 of 28 x 28 (73) forward 8.9 / 12.9, 96 x 112 x 112 (64) 9.5 / 11.8, 4 x 144 of 56 x 56
+// (95) 14.8 / 11.8; fp32 kernel values 2 x 88 of 64 x 64 (42) 9.0 / 10.9, 8 x 72 of 40 x 40 (54) 15.4 / 13.7; grad-input at stride 2, 256 of 32 x 32
+// (14) 4.5 / 7.7, 64 of 96 x 96 (31) 8.3 / 7.5; odd rows 24 x 40 of 15 x 15 (15) 7.0 / 9.3, 6 x 24 of 50 x 51 (28) 21 / 15.
+bool small_conv(const Geom& g, bool transposed) {
+  const int Hd = transposed ? g.H : g.Ho, Wd = transposed ? g.W : g.Wo;
+  const int most = (transposed ? g.Wo : g.W) & 1 ? 20 : transposed && g.sH == 2 ? 26 : g.C & 15 ? 44 : 76;
+  return (long long)g.N * Hd * ((Wd + 7) / 8) * ((g.C + 15) / 16) <= 148LL * most;
+}
+
+// A small call is a chain of latencies: the loads of a band one after the other (rows of odd width pass through
 // registers, eight halves a trip), then the hat products of a warp's items and their slabs; the warps of a scheduler and the blocks of
 // an SM add what they issue.  Few channels a block, and one item a warp, shorten the chain as long as each SM has one block.  The weights
 // are us, from 384 x 14 x 14 (channels / rows / warps: 16/4/8 4.0, 32/4/8 4.6, 96/4/8 6.8, 16/4/6 4.7, 16/7/14 4.6, 16/2/4 with 168 blocks 4.3),
@@ -533,8 +547,7 @@ ConvPlan conv_plan_search(const Geom& g, bool transposed, bool full) {
     }
     if (cg_only) break;
   }
-  const bool odd = (transposed ? g.Wo : g.W) & 1;
-  if (!cg_only && (long long)g.N * Hd * NB * ((g.C + 15) / 16) <= 148LL * (odd ? 20 : 26)) small_conv_plan(g, transposed, full, budget, pl);
+  if (!cg_only && small_conv(g, transposed)) small_conv_plan(g, transposed, full, budget, pl);
   if (!pl.BH) {  // no block shape fits the budget: the caller falls back to the SIMT kernels
     pl.CG = pl.groups = pl.warps = pl.bands = 0;
     pl.smem = 0;
@@ -558,7 +571,9 @@ int launch_conv(const __half* src, const __half* rot, const __half* w, __half* d
   pl.mode_src = ptr_mode(src);
   pl.mode_rot = ptr_mode(rot);
   pl.pair_store = (((TRANSPOSED ? g.W : g.Wo) & 1) == 0) && ptr_mode(dst) >= 1;
-  auto kern = g.C & 15 ? mma_conv_full_kernel<S, TRANSPOSED> : mma_conv_kernel<S, TRANSPOSED>;
+  auto kern = g.C & 15                    ? mma_conv_full_kernel<S, TRANSPOSED>
+              : small_conv(g, TRANSPOSED) ? mma_conv_kernel<S, TRANSPOSED, true>
+                                          : mma_conv_kernel<S, TRANSPOSED, false>;
   int rc = enable_smem(kern, pl.smem);
   if (rc) return rc;
   kern<<<dim3(pl.bands, pl.groups, g.N), pl.warps * 32, pl.smem, s>>>(src, rot, w, dst, g, pl);
@@ -1478,6 +1493,10 @@ int local_mma_plan_query(const Geom& g, int pass, long long out[8]) {
 bool local_conv_mma_takes(const Geom& g, bool transposed) {
   if (!fast_shape(g)) return false;
   return plan_launches(conv_plan(g, transposed));
+}
+
+bool local_conv_mma_small(const Geom& g, bool transposed) {
+  return small_conv(g, transposed) && fast_shape(g, true) && plan_launches(conv_plan(g, transposed));
 }
 
 int local_conv_mma(const __half* src, const __half* rot, const __half* w, __half* dst, const Geom& g, bool transposed,
