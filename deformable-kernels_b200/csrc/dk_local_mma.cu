@@ -442,12 +442,13 @@ size_t conv_smem(const Geom& g, bool transposed, int cg, int bh) {
 }
 
 // The line between small calls and the others, in (item, slab) pairs per SM.  The other side is the ring and tcgen05 kernels or a block shape
-// from the estimate for large calls (us, small / other): 8 x 192 of 28 x 28 (73) forward 8.9 / 12.9, 96 x 112 x 112 (64) 9.5 / 11.8, 4 x 144 of 56 x 56
-// (95) 14.8 / 11.8; fp32 kernel values 2 x 88 of 64 x 64 (42) 9.0 / 10.9, 8 x 72 of 40 x 40 (54) 15.4 / 13.7; grad-input at stride 2, 256 of 32 x 32
-// (14) 4.5 / 7.7, 64 of 96 x 96 (31) 8.3 / 7.5; odd rows 24 x 40 of 15 x 15 (15) 7.0 / 9.3, 6 x 24 of 50 x 51 (28) 21 / 15.
+// from the estimate for large calls.  Below the line (us, other -> small): 144 x 56 x 56 (24) forward 9.5 -> 6.0, 4 x 384 of 16 x 16 (21) 9.5 -> 5.6,
+// 32 x 112 x 112 (21) 7.1 -> 6.3, 10 x 96 of 30 x 36 at stride 2 (18) 7.9 -> 6.6, odd rows 24 x 40 of 15 x 15 (15) 9.3 -> 7.0.  Above it some gain and some
+// lose: 7 x 176 of 20 x 20 (31) 8.3 -> 6.1, 12 x 112 of 20 x 22 (34) 8.4 -> 9.3, 43 x 48 of 28 x 18 (73) 9.6 -> 12.0, grad-input of 64 x 96 x 96 at stride
+// 2 (31) 7.5 -> 8.3, odd rows 6 x 24 of 50 x 51 (28) 15 -> 21.
 bool small_conv(const Geom& g, bool transposed) {
   const int Hd = transposed ? g.H : g.Ho, Wd = transposed ? g.W : g.Wo;
-  const int most = (transposed ? g.Wo : g.W) & 1 ? 20 : transposed && g.sH == 2 ? 26 : g.C & 15 ? 44 : 76;
+  const int most = (transposed ? g.Wo : g.W) & 1 ? 20 : 24;
   return (long long)g.N * Hd * ((Wd + 7) / 8) * ((g.C + 15) / 16) <= 148LL * most;
 }
 
