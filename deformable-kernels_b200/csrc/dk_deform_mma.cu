@@ -10,6 +10,7 @@
 // The products with beta are mma.sync.m16n8k16 as for the local operator.  The offset gradients and grad-input
 // (a scatter into on-chip planes) are described at their kernels further down.
 //
+// dk_deform_lines.cu takes forwards of 32 channels or more that are not small and backwards of 48 or more.
 // Covers fp16, 3x3, pad 1, dilation 1, stride 1 or 2, one rotation group, <= 16 bank cells, C % 16 == 0 and
 // planes small enough for 16 of them to fit on chip (56 x 56 and below); other shapes use the SIMT kernels.
 #include <cstdlib>

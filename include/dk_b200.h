@@ -176,8 +176,8 @@ int dk_sample_depthwise_backward(const void *grad_output, const void *input, con
 int dk_deform_sample_depthwise_forward(const void *input, const void *offset, const void *rotation,
                                        const void *filter, void *output, const dk_geom *g, int dtype, void *stream);
 
-/* The same with scratch memory, in which fp32 (and the fp16 shapes outside the tensor-core path) first brings the input into
- * channel order; 0 bytes: as without. */
+/* The same with scratch memory, in which fp32 and fp16 (except small fp16 calls) first bring the input into channel order;
+ * 0 bytes: as without. */
 size_t dk_deform_sample_depthwise_forward_workspace_bytes(const dk_geom *g, int dtype);
 int dk_deform_sample_depthwise_forward_ws(const void *input, const void *offset, const void *rotation, const void *filter,
                                           void *output, const dk_geom *g, int dtype, void *workspace, size_t workspace_bytes,
