@@ -8,9 +8,9 @@
 // A load of 16 bytes per lane is served eight lanes at a time, 4.2 cycles of the load pipe if those read one line, 8.0 if
 // they read the same 64 bytes of two.  So eight lanes read the 64 channels of one pixel: lane = 4 g + t has the channels
 // 32 (g & 1) + 8 t .. + 7 of the pixels 4 (g >> 1) + i, i = 0 .. 3, of a group of 16.  The products with the hat functions come
-// out of mma.sync in that layout: the rows 2 q and 2 q + 1 are the same pixel, the even rows meet the bank of the lower 32 channels
-// and the odd rows that of the upper ones (two mma on operands that have the other rows zeroed), and the columns 2 t, 2 t + 1 of
-// tile j are the channels 8 t + 2 j, + 1.  mma.sync, because its results are needed in registers beside the gathered values.
+// out of mma.sync in that layout: the rows 2 q and 2 q + 1 are the same pixel, the even rows count for the lower 32 channels and the odd
+// rows for the upper ones (two mma, one with the bank of each half, and a lane keeps the result of its rows: zeroed rows instead would let a
+// bank value that is not finite reach the channel 32 away), and the columns 2 t, 2 t + 1 of tile j are the channels 8 t + 2 j, + 1.  mma.sync, because its results are needed in registers beside the gathered values.
 //
 // 64 x 256 of 56 x 56, forward and backward 3384 -> 1294 us: lines 51 each way, forward 296, sort 54, gather 285, offsets and bank
 // 543.  Forward: load pipe 60 % (64 of its 109 passes per 16 pixels, tap and 64 channels are the corners, 44 % of the
@@ -246,11 +246,6 @@ __device__ __forceinline__ void mul16h(unsigned (&d)[2], const unsigned (&a)[4],
       : "=r"(d[0]), "=r"(d[1])
       : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1), "r"(0u));
 }
-__device__ __forceinline__ void mad16h(unsigned (&d)[2], const unsigned (&a)[4], unsigned b0, unsigned b1) {
-  asm("mma.sync.aligned.m16n8k16.row.col.f16.f16.f16.f16 {%0,%1}, {%2,%3,%4,%5}, {%6,%7}, {%0,%1};\n"
-      : "+r"(d[0]), "+r"(d[1])
-      : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
-}
 __device__ __forceinline__ unsigned fma2h(unsigned a, unsigned b, unsigned c) {
   const __half2 r = __hfma2(*reinterpret_cast<const __half2*>(&a), *reinterpret_cast<const __half2*>(&b), *reinterpret_cast<const __half2*>(&c));
   return *reinterpret_cast<const unsigned*>(&r);
@@ -306,14 +301,15 @@ __device__ __forceinline__ unsigned kernel_rows(const uint4* rows, int lane) {
 // K of the pixels 4 q + I, + I + 1
 template <int I>
 __device__ __forceinline__ void kernel_values(unsigned (&kk)[4][2], unsigned rows, const unsigned (&wb)[2][4][2], bool upper) {
-  unsigned a[4], even[4], odd[4];
+  unsigned a[4];
   ldsm4<I * 128>(a, rows);
 #pragma unroll
-  for (int k = 0; k < 4; ++k) even[k] = upper ? 0u : a[k], odd[k] = upper ? a[k] : 0u;
-#pragma unroll
-  for (int j = 0; j < 4; ++j) mul16h(kk[j], even, wb[0][j][0], wb[0][j][1]);
-#pragma unroll
-  for (int j = 0; j < 4; ++j) mad16h(kk[j], odd, wb[1][j][0], wb[1][j][1]);
+  for (int j = 0; j < 4; ++j) {
+    unsigned low[2], high[2];
+    mul16h(low, a, wb[0][j][0], wb[0][j][1]);
+    mul16h(high, a, wb[1][j][0], wb[1][j][1]);
+    kk[j][0] = upper ? high[0] : low[0], kk[j][1] = upper ? high[1] : low[1];
+  }
 }
 
 // ------------------------------------------------------------------ forward

@@ -88,3 +88,18 @@ def test_values_that_are_not_finite_stay_with_their_samples():
     assert 4 <= int(changed.sum()) <= 36 and bool(changed[3, 100].any()) and int(changed.sum()) == int(changed[3, 100].sum())
     # a window with such a value is summed pixel by pixel in fp32, not in pieces of 22 bits
     torch.testing.assert_close(got[~changed], plain[~changed], rtol=2e-3, atol=2e-3)
+
+
+@pytest.mark.parametrize("value", [float("inf"), float("nan")])
+def test_bank_values_that_are_not_finite_stay_in_their_channel(value):
+    """K of a channel comes out of the same products as that of the channel 32 away."""
+    case = make_case(8, 192, 20, 24, scope=(4, 4), rot_std=0.3, off_std=1.0, seed=11)
+    plain = _run(case)
+    for c in (5, 70, 127):
+        case["weight"][c, 0, 1, 2] = value
+    got = _run(case)
+    rest = [c for c in range(192) if c not in (5, 70, 127)]
+    for k in ("output", "grad_input"):
+        torch.testing.assert_close(got[k][:, rest], plain[k][:, rest], rtol=2e-3, atol=2e-3)
+        assert all(not torch.isfinite(got[k][:, c]).all() for c in (5, 70, 127)), k
+    assert torch.equal(got["grad_weight"], plain["grad_weight"])  # does not depend on the bank
