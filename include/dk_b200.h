@@ -177,7 +177,8 @@ int dk_deform_sample_depthwise_forward(const void *input, const void *offset, co
                                        const void *filter, void *output, const dk_geom *g, int dtype, void *stream);
 
 /* The same with scratch memory, in which fp32 and fp16 (except small fp16 calls) first bring the input into channel order;
- * 0 bytes: as without. */
+ * 0 bytes: as without.  fp16 calls that the kernels without scratch take as well fall back to them when there is too little; fp32 ones return
+ * DK_ERR_WORKSPACE. */
 size_t dk_deform_sample_depthwise_forward_workspace_bytes(const dk_geom *g, int dtype);
 int dk_deform_sample_depthwise_forward_ws(const void *input, const void *offset, const void *rotation, const void *filter,
                                           void *output, const dk_geom *g, int dtype, void *workspace, size_t workspace_bytes,

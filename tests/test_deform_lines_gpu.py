@@ -103,3 +103,21 @@ def test_bank_values_that_are_not_finite_stay_in_their_channel(value):
         torch.testing.assert_close(got[k][:, rest], plain[k][:, rest], rtol=2e-3, atol=2e-3)
         assert all(not torch.isfinite(got[k][:, c]).all() for c in (5, 70, 127)), k
     assert torch.equal(got["grad_weight"], plain["grad_weight"])  # does not depend on the bank
+
+
+@pytest.mark.parametrize("rotation", [True, False])
+def test_forward_without_its_scratch(rotation):
+    """The kernels with planes on chip take the same calls: no scratch, or too little, is not an error."""
+    from deformable_kernels import _cabi as C
+    case = make_case(6, 128, 28, 30, scope=(4, 4) if rotation else (3, 3), rot_std=0.5, off_std=1.0, seed=12)
+    want = _run(case, rotation)["output"]
+    x, o, r, w = (case[k].to(torch.float16).cuda() for k in ("input", "offset", "rotation", "weight"))
+    g = C.geom(tuple(x.shape), (3, 3), (1, 1), (1, 1), (1, 1), tuple(w.shape[2:]), 1)
+    need = C.lib.dk_deform_sample_depthwise_forward_workspace_bytes(g, C.DK_F16)
+    assert need > 0
+    for size in (0, 256, need - 256, need):
+        ws, y = torch.empty(max(size, 1), dtype=torch.uint8, device="cuda"), torch.empty_like(want)
+        status = C.lib.dk_deform_sample_depthwise_forward_ws(C.ptr(x), C.ptr(o), C.ptr(r if rotation else None), C.ptr(w), C.ptr(y), g, C.DK_F16,
+                                                             C.ptr(ws if size else None), size, C.stream_ptr(x.device))
+        assert status == 0, size
+        assert rel_err(y, want) < 2e-3, size  # both round corner weights, hat products and K to fp16
