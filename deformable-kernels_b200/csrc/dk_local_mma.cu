@@ -100,8 +100,8 @@ __global__ void __launch_bounds__(448, 2) mma_conv_kernel(const __half* __restri
     const int j = i >> 4, cell = i & 15;
     bank[j * kBankPitch + cell] = cell < g.cells ? __ldg(w + (size_t)(c0 + j) * g.cells + cell) : __float2half(0.f);
   }
-  load_band(band, bx, src, n, g.C, c0, cnt, Hs, Ws);
-  load_band(rband, br, rot, n, 18, 0, 18, g.Ho, g.Wo);
+  load_band<S == 2 ? 74 : 96>(band, bx, src, n, g.C, c0, cnt, Hs, Ws);
+  load_band<S == 2 ? 74 : 96>(rband, br, rot, n, 18, 0, 18, g.Ho, g.Wo);
   cp_async_wait_all();
   __syncthreads();
 
@@ -922,9 +922,9 @@ __global__ void __launch_bounds__(MAXT, MINB) mma_filter_kernel(const __half* __
     const Band by = make_band(oh0, pl.BH, g.Ho, g.Wo, pl.mode_dy);
     const Band br = make_band(oh0, pl.BH, g.Ho, g.Wo, pl.mode_rot);
     __syncthreads();  // previous unit's readers are done
-    load_band<false>(xband, bx, x, n, g.C, c0, cnt, g.H, g.W);
-    if (!DYM) load_band<false>(yband, by, dy, n, g.C, c0, cnt, g.Ho, g.Wo);
-    load_band<false>(rband, br, rot, n, 18, 0, 18, g.Ho, g.Wo);
+    load_band<0>(xband, bx, x, n, g.C, c0, cnt, g.H, g.W);
+    if (!DYM) load_band<0>(yband, by, dy, n, g.C, c0, cnt, g.Ho, g.Wo);
+    load_band<0>(rband, br, rot, n, 18, 0, 18, g.Ho, g.Wo);
     // DYM == 2: 16 bytes of every channel row of item it_ go to ring slot slot_, one row per lane and step
     auto ring_fill = [&](int it_, int slot_) {
       const int r_ = it_ / NB;

@@ -183,7 +183,8 @@ __device__ __forceinline__ void odd_rows(__half* __restrict__ dst, int pitch, in
     }
   }
 }
-template <bool WORDS>
+// WORDS: odd widths above it are copied word by word; 0: none
+template <int WORDS>
 __device__ __forceinline__ void load_band_group(__half* __restrict__ band, const Band& b, const __half* __restrict__ src, int n,
                                                 int C, int c0, int cnt, int Hs, int Ws, int tid, int nt, int bar_id) {
   const int lane = tid & 31, warp = tid >> 5, nwarps = nt >> 5;
@@ -200,8 +201,12 @@ __device__ __forceinline__ void load_band_group(__half* __restrict__ band, const
     // Short rows: a thread takes one (channel, row) and walks along it, eight independent loads in flight; every lane is on a line of its
     // own, but the lines are reused (forward + backward of 128 x 384 of 7 x 7 67 us, word by word 86; 16 x 160 of 45 x 31 149 / 162, 4 x 32 of
     // 73 x 79 79 / 87).  Longer rows word by word (8 x 64 of 75 x 101 209 -> 198, 20 x 64 of 63 x 97 at stride 2 221 -> 182), except in the
-    // bank gradient (!WORDS: 4 x 48 of 20 x 99 at stride 2 22 -> 30).
-    if (WORDS && Ws > 96) {
+    // bank gradient (WORDS = 0: 4 x 48 of 20 x 99 at stride 2 22 -> 30).  The line lies where the lanes' lines of two blocks stop fitting in what
+    // shared memory leaves of L1, which bands of twice the rows reach earlier: forward at stride 2, a row per thread / words, us, 40 x 64 of 56 x 75
+    // 66 / 39, x 79 70 / 41, x 85 86 / 48, x 89 69 / 74, x 95 76 / 70; 24 x 96 of 45 x 83 41 / 31; 8 x 128 of 100 x 73 35 / 49, x 75 33 / 35, x 95
+    // 45 / 39 (a warp per row 53, 53, 55, 90, 84; 39; 51, 48, 47).  The kernel with fp32 kernel values has smaller blocks: 40 x 72 of 56 x 75
+    // 54 / 72, x 95 70 / 76, 16 x 40 of 90 x 79 33 / 29.
+    if (WORDS && Ws > WORDS) {
       odd_rows(band + kSlack + (r_s * b.Wp - b.org), b.pitch_c, b.Wp, s0 + (size_t)r_s * Ws, plane, cnt, r_e - r_s, Ws, tid, nt);
       return;
     }
@@ -279,7 +284,7 @@ __device__ __forceinline__ void flat_copies(__half* __restrict__ band, int pitch
 // leave lanes idle on the last pass over a row and walk through the channels one after the other.  Same instruction count
 // (measured), 3-4 % less time in the four kernels.
 // Odd row widths, and bands without a row inside the image, go through load_band_group.
-template <bool WORDS>
+template <int WORDS>
 __device__ __forceinline__ void load_band_flat(__half* __restrict__ band, const Band& b, const __half* __restrict__ src, int n,
                                                int C, int c0, int cnt, int Hs, int Ws, int tid, int nt, int bar_id) {
   const int r_s = max(b.row_lo, 0), r_e = min(b.row_lo + b.RB, Hs);
@@ -315,7 +320,7 @@ __device__ __forceinline__ void load_band_flat(__half* __restrict__ band, const 
     }
   }
 }
-template <bool WORDS = true>
+template <int WORDS = 96>
 __device__ __forceinline__ void load_band(__half* __restrict__ band, const Band& b, const __half* __restrict__ src, int n, int C,
                                           int c0, int cnt, int Hs, int Ws) {
   load_band_flat<WORDS>(band, b, src, n, C, c0, cnt, Hs, Ws, threadIdx.x, blockDim.x, 0);
