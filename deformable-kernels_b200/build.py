@@ -17,7 +17,7 @@ LIB_DIR = os.path.join(HERE, "lib")
 LIB = os.path.join(LIB_DIR, "libdk_b200.so")
 TORCH_SOURCE = os.path.join(CSRC, "dk_torch.cpp")
 TORCH_LIB = os.path.join(LIB_DIR, "dk_torch.so")
-SOURCES = ["dk_api.cu", "dk_local.cu", "dk_local_mma.cu", "dk_local_ring.cu", "dk_local_tc.cu", "dk_local_f32.cu", "dk_local_tf32.cu", "dk_deform.cu", "dk_deform_bins.cu", "dk_deform_lines.cu", "dk_deform_mma.cu", "dk_nd.cu", "dk_scale.cu", "dk_global.cu", "dk_static_scratch.cu"]
+SOURCES = ["dk_api.cu", "dk_local.cu", "dk_local_mma.cu", "dk_local_ring.cu", "dk_local_tc.cu", "dk_local_f32.cu", "dk_local_pieces.cu", "dk_deform.cu", "dk_deform_bins.cu", "dk_deform_lines.cu", "dk_deform_mma.cu", "dk_nd.cu", "dk_scale.cu", "dk_global.cu", "dk_static_scratch.cu"]
 NVCC_FLAGS = [
     "-gencode", "arch=compute_100a,code=sm_100a", "-lineinfo", "-O3", "-std=c++17",
     "-Xcompiler", "-fPIC",

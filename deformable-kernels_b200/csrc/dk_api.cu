@@ -217,11 +217,11 @@ int dk_sample_depthwise_backward_rotation(const void* grad_output, const void* i
                                                 M_(T, grad_rotation), gg, workspace, workspace_bytes, (cudaStream_t)stream))
 }
 
-/* Offset and bank gradients in one pass with fp32 arithmetic on the tensor cores (dk_local_tf32.cu): fp32, and fp16 where the
+/* Offset and bank gradients in one pass with fp32 arithmetic on the tensor cores (dk_local_pieces.cu): fp32, and fp16 where the
  * channels are no multiple of 16. */
-static bool local_tf32_gradients(const Geom& g, int dtype) {
+static bool local_pieces_gradients(const Geom& g, int dtype) {
   if (!mma_path_enabled() || (dtype != DK_F32 && (dtype != DK_F16 || (g.C & 15) == 0))) return false;
-  return local_gradients_tf32_takes(g, dtype == DK_F16 ? 2 : 4);
+  return local_gradients_pieces_takes(g, dtype == DK_F16 ? 2 : 4);
 }
 
 size_t dk_sample_depthwise_backward_workspace_bytes(const dk_geom* g, int dtype) {
@@ -236,8 +236,8 @@ size_t dk_sample_depthwise_backward_workspace_bytes(const dk_geom* g, int dtype)
     if (d > need) need = d;
     if (e > need) need = e;
   }
-  if (make_geom(g, &gg) && local_tf32_gradients(gg, dtype)) {
-    const size_t f = align256(local_gradients_tf32_workspace(gg, dtype == DK_F16 ? 2 : 4));
+  if (make_geom(g, &gg) && local_pieces_gradients(gg, dtype)) {
+    const size_t f = align256(local_gradients_pieces_workspace(gg, dtype == DK_F16 ? 2 : 4));
     if (f > need) need = f;
   }
   return need;
@@ -277,11 +277,11 @@ int dk_sample_depthwise_backward(const void* grad_output, const void* input, con
   if (grad_rotation && grad_filter) {
     Geom gg;
     if (!grad_output || !input || !rotation || !filter || !make_geom(g, &gg)) return DK_ERR_BAD_ARGUMENT;
-    if (local_tf32_gradients(gg, dtype)) {
-      rc = dtype == DK_F16 ? local_gradients_tf32<__half>(P_(__half, grad_output), P_(__half, input), P_(__half, rotation), P_(__half, filter),
+    if (local_pieces_gradients(gg, dtype)) {
+      rc = dtype == DK_F16 ? local_gradients_pieces<__half>(P_(__half, grad_output), P_(__half, input), P_(__half, rotation), P_(__half, filter),
                                                           M_(__half, grad_rotation), M_(__half, grad_filter), gg, workspace, workspace_bytes,
                                                           (cudaStream_t)stream)
-                           : local_gradients_tf32<float>(P_(float, grad_output), P_(float, input), P_(float, rotation), P_(float, filter),
+                           : local_gradients_pieces<float>(P_(float, grad_output), P_(float, input), P_(float, rotation), P_(float, filter),
                                                          M_(float, grad_rotation), M_(float, grad_filter), gg, workspace, workspace_bytes,
                                                          (cudaStream_t)stream);
       if (rc != DK_ERR_UNSUPPORTED) return rc;

@@ -230,11 +230,11 @@ int tc_register_query(long long out[8]);  // {kernels, fewest registers per thre
 template <typename T>
 int local_rot_f32(const T* dy, const T* x, const T* rot, const T* w, T* drot, const Geom& g, cudaStream_t s);
 size_t local_filter_f32_workspace(const Geom& g);
-// both in one pass on the tensor cores (dk_local_tf32.cu)
-bool local_gradients_tf32_takes(const Geom& g, size_t elem);
-size_t local_gradients_tf32_workspace(const Geom& g, size_t elem);
+// both in one pass on the tensor cores (dk_local_pieces.cu)
+bool local_gradients_pieces_takes(const Geom& g, size_t elem);
+size_t local_gradients_pieces_workspace(const Geom& g, size_t elem);
 template <typename T>
-int local_gradients_tf32(const T* dy, const T* x, const T* rot, const T* w, T* drot, T* dw, const Geom& g, void* ws, size_t ws_bytes,
+int local_gradients_pieces(const T* dy, const T* x, const T* rot, const T* w, T* drot, T* dw, const Geom& g, void* ws, size_t ws_bytes,
                          cudaStream_t s);
 size_t deform_data_mma_workspace(const Geom& g);
 // fp16 with the operands in channel order (dk_deform_lines.cu)

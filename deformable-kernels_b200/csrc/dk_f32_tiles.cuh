@@ -1,5 +1,5 @@
 // Tiles of output pixels with their source windows in shared memory, channel by channel, for the gradient kernels in fp32 arithmetic
-// (dk_local_f32.cu, dk_local_tf32.cu).
+// (dk_local_f32.cu, dk_local_pieces.cu).
 #pragma once
 
 #include "dk_common.cuh"

@@ -2,19 +2,22 @@
 // the fp16 kernels do not apply; 3 x 3 taps, scopes up to 4 x 4).
 //
 // Both are contractions of dK = dy * x with 16 cells: G[pixel, tap][cell] = sum_c dK W[c, cell] (then the floor-based derivative
-// weights) and dW[c][cell] = sum over pixels and taps of dK beta[(pixel, tap), cell].  An fp32 value is two tf32 pieces, 11 bits rounded and
-// the rest, so a product is three mma.m16n8k8: small * large, large * small, large * large in this order; what is left out is 2^-24 of it.
-// The tensor cores truncate their sums, so no accumulator runs longer than these three: a step of 8 channels (G) or 8 pixels (dW) of a tap is
-// added to the sums with one rounded addition.  fp16 banks are one piece.
+// weights) and dW[c][cell] = sum over pixels and taps of dK beta[(pixel, tap), cell].  An fp32 value is three bf16 pieces, 8 bits rounded each time,
+// which together are all of it (down to 2^-110, below which the last ones underflow); a product is six of their products, the smallest first,
+// and what is left out is 2^-23 of it at the most, 2^-26 in the mean (a rounding: 2^-24 and 2^-25.8).  The tensor cores truncate their sums, so no accumulator runs longer than
+// these six: a step of 16 channels (G) or of 8 pixels at two taps (dW) is added to the sums with one rounded addition.  Against fp64, separate fp32
+// kernels -> this one, 2-norm: 16 x 16 of 61 x 63 at stride 2 offsets 7.5e-8 -> 6.9e-8, bank 1.9e-7 -> 1.7e-7 (most of it the rounding of the
+// coordinates), 64 x 144 of 56 x 56 1.4e-7 -> 0.9e-7 and 5.2e-7 -> 2.0e-7.
 //
 // Block: a tile of up to 96 pixels, a warp 8 of them, over all channels, 32 at a time, whose dy and x are staged while the previous ones are
 // multiplied.  G stays in registers (9 taps x 16 cells x 8 pixels per warp); the warps' bank sums of 32 channels meet in
-// shared memory, in their order, and are added to the block's partial sums.
+// shared memory, in their order, and are added to the block's partial sums.  dK is split once: movmatrix turns the pieces from the lanes'
+// order of the offsets (k = channels) to that of the bank (k = pixels).  Pairs of steps and pairs of taps fill the 16 k-slots so that every operand lies
+// in registers as it was loaded or made; two pieces of one step beside each other need copies of one of them and take 629 us below.
 //
-// fp32 64 x 144 of 56 x 56: 758 us in two kernels that gather or hold the cells with one fp32 multiply-add each -> 557.  Tensor pipe 39 %,
-// issue 44 %: mma.sync and the fp32 work around it (two pieces, rounded additions) do not overlap much, three products with their pieces
-// take 10.2 cycles of an SM in a loop by themselves, 6.2 of them the products (here 17, with staging, the warps' sums and tiles that do not
-// fill).  At 128 registers and two blocks of eight warps the compiler moves operands about (663 us), 8 warps with 254 take as long as 12 with 168.
+// fp32 64 x 144 of 56 x 56: 753 us in two kernels that gather or hold the cells with one fp32 multiply-add each -> 561.  Tensor pipe 42 %,
+// issue 40 %: products, the pieces that feed them and the additions behind them follow each other in a warp, and 3 warps per scheduler (168 registers)
+// overlap part of it; tiles that do not fill and the tenth tap of the pairs are 15 % of the products.
 #include "dk_f32_tiles.cuh"
 
 namespace dk {
@@ -22,7 +25,7 @@ namespace dk {
 namespace {
 
 constexpr int kWarps = 12, kPixels = 8 * kWarps, kRedPitch = 40;
-constexpr int kBetaBytes = kWarps * 9 * 32 * 16, kRedBytes = kWarps * 16 * kRedPitch * 4, kBankBytes = 4 * 32 * 32;
+constexpr int kBetaBytes = kWarps * 5 * 3 * 32 * 16, kRedBytes = kWarps * 16 * kRedPitch * 4, kBankBytes = 2 * 3 * 32 * 16;
 // Words of a channel of x and of dy in shared memory: 12 modulo 32, so that neither way of reading them has bank conflicts.  At stride 2 two
 // buffers do not fit.
 template <int S> struct Room {
@@ -46,51 +49,50 @@ __device__ __forceinline__ f2 sub2(f2 a, f2 b) {
   asm("sub.rn.f32x2 %0, %1, %2;\n" : "=l"(r) : "l"(a), "l"(b));
   return r;
 }
-__device__ __forceinline__ unsigned large(float v) {
-  return (__float_as_uint(v) + 0x1000u) & 0xffffe000u;
-}
-// two values as pieces: 11 bits rounded, and the rest (of which the tensor cores see 11 bits)
+// Two values as three pieces of bf16, 8 bits rounded and the rest: together they are the values, all 24 bits.  Low half: the first value.
 struct Pieces {
-  unsigned hi[2], lo[2];
+  unsigned p[3];
 };
-__device__ __forceinline__ Pieces split2(f2 v) {
+__device__ __forceinline__ unsigned two_bf16(f2 v) {
   const float2 w = unpair(v);
-  Pieces p;
-  p.hi[0] = large(w.x), p.hi[1] = large(w.y);
-  const float2 l = unpair(sub2(v, pair(__uint_as_float(p.hi[0]), __uint_as_float(p.hi[1]))));
-  p.lo[0] = __float_as_uint(l.x), p.lo[1] = __float_as_uint(l.y);
-  return p;
+  unsigned r;
+  asm("cvt.rn.bf16x2.f32 %0, %1, %2;\n" : "=r"(r) : "f"(w.y), "f"(w.x));
+  return r;
 }
-__device__ __forceinline__ void mul8(float (&d)[4], const unsigned (&a)[4], const unsigned (&b)[2]) {
-  asm("mma.sync.aligned.m16n8k8.row.col.f32.tf32.tf32.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%10,%10,%10,%10};\n"
+__device__ __forceinline__ f2 widened(unsigned p) { return pair(__uint_as_float(p << 16), __uint_as_float(p & 0xffff0000u)); }
+__device__ __forceinline__ Pieces split3(f2 v) {
+  Pieces s;
+  s.p[0] = two_bf16(v);
+  v = sub2(v, widened(s.p[0]));
+  s.p[1] = two_bf16(v);
+  s.p[2] = two_bf16(sub2(v, widened(s.p[1])));
+  return s;
+}
+__device__ __forceinline__ unsigned turned(unsigned v) {
+  unsigned r;
+  asm("movmatrix.sync.aligned.m8n8.trans.b16 %0, %1;\n" : "=r"(r) : "r"(v));
+  return r;
+}
+__device__ __forceinline__ void mul16(float (&d)[4], const uint4& a, unsigned b0, unsigned b1) {
+  asm("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%10,%10,%10,%10};\n"
       : "=f"(d[0]), "=f"(d[1]), "=f"(d[2]), "=f"(d[3])
-      : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b[0]), "r"(b[1]), "f"(0.f));
+      : "r"(a.x), "r"(a.y), "r"(a.z), "r"(a.w), "r"(b0), "r"(b1), "f"(0.f));
 }
-__device__ __forceinline__ void mad8(float (&d)[4], const unsigned (&a)[4], const unsigned (&b)[2]) {
-  asm("mma.sync.aligned.m16n8k8.row.col.f32.tf32.tf32.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};\n"
+__device__ __forceinline__ void mad16(float (&d)[4], const uint4& a, unsigned b0, unsigned b1) {
+  asm("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};\n"
       : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3])
-      : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b[0]), "r"(b[1]));
+      : "r"(a.x), "r"(a.y), "r"(a.z), "r"(a.w), "r"(b0), "r"(b1));
 }
-// sums += a * b for N of b, side by side: each is a chain of three products.  ONE: a has no small piece.
-template <bool ONE, int N>
-__device__ __forceinline__ void add8(f2 (&sum)[N][2], const unsigned (&hi)[4], const unsigned (&lo)[4], const Pieces (&b)[N]) {
-  float d[N][4];
-#pragma unroll
-  for (int i = 0; i < N; ++i) {
-    if (ONE) mul8(d[i], hi, b[i].lo);
-    else mul8(d[i], lo, b[i].hi);
-  }
-  if (!ONE) {
-#pragma unroll
-    for (int i = 0; i < N; ++i) mad8(d[i], hi, b[i].lo);
-  }
-#pragma unroll
-  for (int i = 0; i < N; ++i) mad8(d[i], hi, b[i].hi);
-#pragma unroll
-  for (int i = 0; i < N; ++i) {
-    sum[i][0] = add2(sum[i][0], pair(d[i][0], d[i][1]));
-    sum[i][1] = add2(sum[i][1], pair(d[i][2], d[i][3]));
-  }
+// Product E of the six of two operands in pieces.  a: [piece], b and c: the pieces of the k-slots 0-7 and 8-15.
+template <int E>
+__device__ __forceinline__ void product(float (&d)[4], const uint4 (&a)[3], const Pieces& b, const Pieces& c) {
+  constexpr int A = E == 0 || E > 3 ? 0 : E == 1 ? 2 : 1, B = E == 0 ? 2 : E == 2 || E == 4 ? 1 : 0;
+  if (E == 0) mul16(d, a[A], b.p[B], c.p[B]);
+  else mad16(d, a[A], b.p[B], c.p[B]);
+}
+__device__ __forceinline__ void add4(f2 (&s)[2], const float (&d)[4]) {
+  s[0] = add2(s[0], pair(d[0], d[1]));
+  s[1] = add2(s[1], pair(d[2], d[3]));
 }
 
 // derivative towards the kernel-space offset (u: !dv, v: dv) from G [cell][8 pixels]
@@ -125,19 +127,19 @@ __device__ __noinline__ void cells_alone(float* G, const T* __restrict__ dy, con
 }
 
 template <typename T, int S>
-__global__ void __launch_bounds__(32 * kWarps, 1) tf32_gradients_kernel(const T* __restrict__ dy, const T* __restrict__ x,
+__global__ void __launch_bounds__(32 * kWarps, 1) pieces_gradients_kernel(const T* __restrict__ dy, const T* __restrict__ x,
                                                                         const T* __restrict__ rot, const T* __restrict__ w,
                                                                         T* __restrict__ drot, float* __restrict__ partial,
                                                                         const __grid_constant__ Geom g, const __grid_constant__ TilePlan t) {
   extern __shared__ __align__(16) unsigned char smem[];
   using R = Room<S>;
-  constexpr bool kOnePiece = sizeof(T) == 2, kTwo = R::kBuffers == 2;
+  constexpr bool kTwo = R::kBuffers == 2;
   constexpr int NX = (R::X + 31) / 32, NY = (kPixels + 31) / 32;  // words of a lane per channel
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, gq = lane >> 2, q = lane & 3;
-  float4* beta = reinterpret_cast<float4*>(smem) + warp * 9 * 32 + lane;            // the warp's hat products as mma operands, [tap][lane]
+  uint4* beta = reinterpret_cast<uint4*>(smem) + warp * 15 * 32 + lane;             // the warp's hat products as mma operands, [taps 2 i, + 1][piece][lane]
   float* red = reinterpret_cast<float*>(smem + kBetaBytes);                         // [warp][cell][kRedPitch]
-  uint4* banks = reinterpret_cast<uint4*>(smem + kBetaBytes + kRedBytes);           // [buffer][step of 8 channels][hi | lo][lane]
-  float* stage = reinterpret_cast<float*>(banks + R::kBuffers * kBankBytes / 16);   // [buffer] of x [32][X], dy [32][Y]
+  uint4* banks = reinterpret_cast<uint4*>(smem + kBetaBytes + kRedBytes) + lane;    // [buffer][steps 2 i, + 1 of 8 channels][piece][lane]
+  float* stage = reinterpret_cast<float*>(smem + kBetaBytes + kRedBytes + R::kBuffers * kBankBytes);  // [buffer] of x [32][X], dy [32][Y]
   const int px = t.TH * t.TW, chunks = (g.C + 31) / 32;
   const float uh0 = 0.5f * (float)(g.scH - 3), uw0 = 0.5f * (float)(g.scW - 3);
   float* mine = partial + (size_t)blockIdx.x * g.C * g.cells;
@@ -165,6 +167,11 @@ __global__ void __launch_bounds__(32 * kWarps, 1) tf32_gradients_kernel(const T*
       const int e = lane + 32 * i, r = over(e, t.TW, t.magic_y), oh = tp.oh0 + r, ow = tp.ow0 + (e - r * t.TW);
       from_y[i] = e < px && oh < g.Ho && ow < g.Wo ? oh * g.Wo + ow : -1;
     }
+    // half `h` (eight k-slots) of an operand in pieces: rows gq and gq + 8
+    auto put = [](uint4* to, int h, const Pieces& r0, const Pieces& r1) {
+#pragma unroll
+      for (int k = 0; k < 3; ++k) reinterpret_cast<uint2*>(to + 32 * k)[h] = make_uint2(r0.p[k], r1.p[k]);
+    };
     auto fill = [&](int chunk) {
       const int c0 = chunk * 32, buffer = kTwo ? chunk & 1 : 0;
       float* xs = stage + buffer * R::kWords + warp * R::X + lane;
@@ -195,38 +202,42 @@ __global__ void __launch_bounds__(32 * kWarps, 1) tf32_gradients_kernel(const T*
           for (int i = 0; i < NY; ++i) ys[k * kWarps * R::Y + 32 * i] = v[NX + i];
         }
       }
-      if (warp < 4) {  // the bank of step `warp`: {cell gq, cell gq + 8} of channel 2 q, then of 2 q + 1
+      if (warp < 4) {  // the bank of step `warp`: channels 2 q, + 1 of cell gq, then of gq + 8
         float v[4];
 #pragma unroll
         for (int i = 0; i < 4; ++i) {
-          const int c = c0 + warp * 8 + 2 * q + (i >> 1), a = (gq >> 2) + 2 * (i & 1), b = gq & 3;
+          const int c = c0 + warp * 8 + 2 * q + (i & 1), a = (gq >> 2) + 2 * (i >> 1), b = gq & 3;
           v[i] = c < g.C && a < g.scH && b < g.scW ? ld<float>(w + (size_t)c * g.cells + a * g.scW + b) : 0.f;
         }
-        const Pieces p0 = split2(pair(v[0], v[1])), p1 = split2(pair(v[2], v[3]));
-        uint4* to = banks + (buffer * 4 + warp) * 64 + lane;
-        to[0] = make_uint4(p0.hi[0], p0.hi[1], p1.hi[0], p1.hi[1]);
-        if (!kOnePiece) to[32] = make_uint4(p0.lo[0], p0.lo[1], p1.lo[0], p1.lo[1]);
+        put(banks + (buffer * 2 + (warp >> 1)) * 96, warp & 1, split3(pair(v[0], v[1])), split3(pair(v[2], v[3])));
       }
     };
     __syncthreads();  // the previous tile's last sums have been read
     fill(0);
-    int xg, yg, xk[2], yk[2];
-    bool live_k[2];
+    int xg, yg;
+    bool live_g;
     {
-      int oh, ow;
-      place(warp * 8 + gq, xg, yg, oh, ow);
+      int oh, ow, xk, yk;
+      live_g = place(warp * 8 + gq, xg, yg, oh, ow);
+      bool live_k[2];
+      const T* rp[2];
 #pragma unroll
-      for (int e = 0; e < 2; ++e) {  // k-slots q and q + 4 of the bank's operands: the warp's pixels of these numbers; cells gq and gq + 8
-        live_k[e] = place(warp * 8 + q + 4 * e, xk[e], yk[e], oh, ow);
-        const T* rp = rot + (size_t)tp.n * 18 * g.P + (live_k[e] ? oh * g.Wo + ow : 0);
+      for (int e = 0; e < 2; ++e) {
+        live_k[e] = place(warp * 8 + 2 * q + e, xk, yk, oh, ow);
+        rp[e] = rot + (size_t)tp.n * 18 * g.P + (live_k[e] ? oh * g.Wo + ow : 0);
+      }
 #pragma unroll
-        for (int tap = 0; tap < 9; ++tap) {
-          const float u = live_k[e] ? ((float)(tap / 3) + ld<float>(rp + (size_t)(2 * tap) * g.P)) + uh0 : -8.f;
-          const float v = ((float)(tap % 3) + ld<float>(rp + (size_t)(2 * tap + 1) * g.P)) + uw0;
+      for (int tap = 0; tap < 9; ++tap) {
+        float b[2][2];  // cells gq and gq + 8, pixels 2 q and 2 q + 1
+#pragma unroll
+        for (int e = 0; e < 2; ++e) {
+          const float u = live_k[e] ? ((float)(tap / 3) + ld<float>(rp[e] + (size_t)(2 * tap) * g.P)) + uh0 : -8.f;
+          const float v = ((float)(tap % 3) + ld<float>(rp[e] + (size_t)(2 * tap + 1) * g.P)) + uw0;
           const float hv = (gq & 3) < g.scW ? hat1(v - (float)(gq & 3)) : 0.f;
-          const float h0 = (gq >> 2) < g.scH ? hat1(u - (float)(gq >> 2)) : 0.f, h1 = (gq >> 2) + 2 < g.scH ? hat1(u - (float)((gq >> 2) + 2)) : 0.f;
-          reinterpret_cast<float2*>(beta + tap * 32)[e] = make_float2(h0 * hv, h1 * hv);
+          b[0][e] = (gq >> 2) < g.scH ? hat1(u - (float)(gq >> 2)) * hv : 0.f;
+          b[1][e] = (gq >> 2) + 2 < g.scH ? hat1(u - (float)((gq >> 2) + 2)) * hv : 0.f;
         }
+        put(beta + (tap >> 1) * 96, tap & 1, split3(pair(b[0][0], b[0][1])), split3(pair(b[1][0], b[1][1])));
       }
     }
     f2 G[3][3][2];  // cell gq, then gq + 8, of the warp's pixels 2 q, + 1
@@ -240,51 +251,59 @@ __global__ void __launch_bounds__(32 * kWarps, 1) tf32_gradients_kernel(const T*
       if (kTwo && chunk + 1 < chunks) fill(chunk + 1);
       const float* xs = stage + buffer * R::kWords;
       const float* ys = xs + 32 * R::X;
-      // offsets: k-slots q and q + 4 are the channels 2 q and 2 q + 1 of a step of 8
+      // Two taps and two steps at a time: 16 k-slots are the channels of both steps (offsets), or the warp's pixels at both taps (bank).  The
+      // products of a tap and a step are split once, in the lanes as the offsets want them, and movmatrix turns the pieces for the bank.
       const int steps = min(4, (g.C - c0 + 7) >> 3);
+      float* r = red + (warp * 16 + gq) * kRedPitch + 2 * q;
 #pragma unroll 1
-      for (int ks = 0; ks < steps; ++ks) {
-        const uint4* wp = banks + (buffer * 4 + ks) * 64 + lane;
-        const uint4 h4 = wp[0], l4 = kOnePiece ? make_uint4(0, 0, 0, 0) : wp[32];
-        const unsigned hi[4] = {h4.x, h4.y, h4.z, h4.w}, lo[4] = {l4.x, l4.y, l4.z, l4.w};
-        const float* xp = xs + (ks * 8 + 2 * q) * R::X + xg;
-        const float* yp = ys + (ks * 8 + 2 * q) * R::Y + yg;
-        const f2 d = pair(yp[0], yp[R::Y]);
+      for (int h = 0; h < steps; h += 2, r += 16) {
+        f2 acc[2][2], d[2];
+        uint4 wp[3];
 #pragma unroll
-        for (int fh = 0; fh < 3; ++fh, xp += t.XW) {
-          Pieces p[3];
+        for (int k = 0; k < 3; ++k) wp[k] = banks[(buffer * 6 + (h >> 1) * 3 + k) * 32];
 #pragma unroll
-          for (int fw = 0; fw < 3; ++fw) p[fw] = split2(mul2(d, pair(xp[fw], xp[R::X + fw])));
-          add8<kOnePiece, 3>(G[fh], hi, lo, p);
-        }
-      }
-      // bank
-      {
-        f2 acc[4][2], d[4];
-#pragma unroll
-        for (int j = 0; j < 4; ++j) {
+        for (int j = 0; j < 2; ++j) {
+          const float* yp = ys + ((h + j) * 8 + 2 * q) * R::Y + yg;
+          d[j] = live_g ? pair(yp[0], yp[R::Y]) : 0;
           acc[j][0] = acc[j][1] = 0;
-          const float* yp = ys + (8 * j + gq) * R::Y;
-          d[j] = pair(live_k[0] ? yp[yk[0]] : 0.f, live_k[1] ? yp[yk[1]] : 0.f);
         }
-        const float* xa = xs + gq * R::X + xk[0];
-        const float* xb = xs + gq * R::X + xk[1];
-        const float4* bp = beta;
-#pragma unroll 1
-        for (int fh = 0; fh < 3; ++fh, xa += t.XW, xb += t.XW)
+        const float* xp = xs + (h * 8 + 2 * q) * R::X + xg;
 #pragma unroll
-          for (int fw = 0; fw < 3; ++fw, bp += 32) {
-            const float4 b = *bp;
-            const Pieces p0 = split2(pair(b.x, b.y)), p1 = split2(pair(b.z, b.w));
-            const unsigned hi[4] = {p0.hi[0], p0.hi[1], p1.hi[0], p1.hi[1]}, lo[4] = {p0.lo[0], p0.lo[1], p1.lo[0], p1.lo[1]};
-            Pieces p[4];
+        for (int t0 = 0; t0 < 9; t0 += 2) {
+          uint4 bp[3];
 #pragma unroll
-            for (int j = 0; j < 4; ++j) p[j] = split2(mul2(d[j], pair(xa[8 * j * R::X + fw], xb[8 * j * R::X + fw])));
-            add8<false, 4>(acc, hi, lo, p);
+          for (int k = 0; k < 3; ++k) bp[k] = beta[(t0 >> 1) * 96 + 32 * k];
+          Pieces p[2][2], pt[2][2];  // [tap][step]
+          float u[2][4], v[2][4];
+#pragma unroll
+          for (int i = 0; i < 2; ++i) {
+            const int tap = t0 + i;
+            if (tap > 8) break;
+            const float* at = xp + (tap / 3) * t.XW + tap % 3;
+#pragma unroll
+            for (int j = 0; j < 2; ++j) p[i][j] = split3(mul2(d[j], pair(at[j * 8 * R::X], at[j * 8 * R::X + R::X])));
           }
-        float* r = red + (warp * 16 + gq) * kRedPitch + 2 * q;
 #pragma unroll
-        for (int j = 0; j < 4; ++j) {
+          for (int i = 0; i < 2; ++i)
+#pragma unroll
+            for (int j = 0; j < 2; ++j)
+#pragma unroll
+              for (int k = 0; k < 3; ++k) pt[i][j].p[k] = t0 + i < 9 ? turned(p[i][j].p[k]) : 0u;
+          if (t0 == 8) bp[0].z = bp[0].w = bp[1].z = bp[1].w = bp[2].z = bp[2].w = 0u;
+#define DK_PRODUCT(E)                                                                    \
+  if (E != 1 || sizeof(T) == 4) { /* fp16 banks are two pieces */                        \
+    product<E>(u[0], wp, p[0][0], p[0][1]);                                              \
+    if (t0 < 8) product<E>(u[1], wp, p[1][0], p[1][1]);                                  \
+  }                                                                                      \
+  product<E>(v[0], bp, pt[0][0], pt[1][0]), product<E>(v[1], bp, pt[0][1], pt[1][1]);
+          DK_PRODUCT(0) DK_PRODUCT(1) DK_PRODUCT(2) DK_PRODUCT(3) DK_PRODUCT(4) DK_PRODUCT(5)
+#undef DK_PRODUCT
+          add4(G[t0 / 3][t0 % 3], u[0]);
+          if (t0 < 8) add4(G[(t0 + 1) / 3 % 3][(t0 + 1) % 3], u[1]);
+          add4(acc[0], v[0]), add4(acc[1], v[1]);
+        }
+#pragma unroll
+        for (int j = 0; j < 2; ++j) {
           *reinterpret_cast<f2*>(r + 8 * j) = acc[j][0];
           *reinterpret_cast<f2*>(r + 8 * kRedPitch + 8 * j) = acc[j][1];
         }
@@ -367,7 +386,7 @@ TilePlan search_plan(const Geom& g) {
       const int across = (g.Wo + wide - 1) / wide, TW = (g.Wo + across - 1) / across, down = (g.Ho + high - 1) / high, TH = (g.Ho + down - 1) / down;
       const int words = ((TH - 1) * g.sH + 3) * ((TW - 1) * g.sW + 3);
       if (words > most) continue;
-      // a tile costs its eight warps' steps whatever part of their pixels there is, and a fiftieth of a pixel per staged word
+      // a tile costs its twelve warps' steps whatever part of their pixels there is, and a fiftieth of a pixel per staged word
       const long long cost = (long long)across * down * (kPixels * 50 + words + TH * TW);
       if (best < 0 || cost < best) best = cost, t.TW = TW, t.TH = TH, t.across = across, t.down = down;
       break;
@@ -403,32 +422,32 @@ const TilePlan& gradients_plan(const Geom& g) {
 // 28 x 28 (72 tiles) 24 -> 19, 4 x 64 (36 tiles) 17 -> 19, 40 x 40 of 60 x 111 455 -> 289, 128 x 960 of 7 x 7 221 -> 175; stride 2, 40 x 96 of
 // 30 x 41 74 -> 51, 16 x 96 of 28 x 28 (48 tiles) 23 -> 27.  fp16 8 x 72 of 75 x 101 165 -> 118, 6 x 104 of 40 x 44 54 -> 34, 24 x 104 of
 // 28 x 28 77 -> 62, 64 x 200 of 14 x 14 (1.3 tiles per SM) 90 -> 97, 128 x 200 160 -> 150; stride 2, 40 x 72 of 56 x 50 114 -> 121.
-bool local_gradients_tf32_takes(const Geom& g, size_t elem) {
+bool local_gradients_pieces_takes(const Geom& g, size_t elem) {
   if (g.kH != 3 || g.kW != 3 || g.dH != 1 || g.dW != 1 || g.pH != 1 || g.pW != 1 || g.sH != g.sW || (g.sH != 1 && g.sH != 2)) return false;
   if (g.G != 1 || g.scH > 4 || g.scW > 4 || (long long)g.N * g.P >= 0x3fffffff) return false;
   if ((long long)g.N * g.P < 1536) return false;  // few tiles whatever their shape
   const int tiles = gradients_plan(g).tiles, sms = device_sm_count();
   return tiles >= 64 && (elem == 4 || (g.sH == 1 && (tiles <= sms || 2 * tiles >= 3 * sms)));
 }
-size_t local_gradients_tf32_workspace(const Geom& g, size_t elem) {
-  return local_gradients_tf32_takes(g, elem) ? (size_t)gradients_plan(g).blocks * g.C * g.cells * sizeof(float) : 0;
+size_t local_gradients_pieces_workspace(const Geom& g, size_t elem) {
+  return local_gradients_pieces_takes(g, elem) ? (size_t)gradients_plan(g).blocks * g.C * g.cells * sizeof(float) : 0;
 }
 template <typename T>
-int local_gradients_tf32(const T* dy, const T* x, const T* rot, const T* w, T* drot, T* dw, const Geom& g, void* ws, size_t ws_bytes,
+int local_gradients_pieces(const T* dy, const T* x, const T* rot, const T* w, T* drot, T* dw, const Geom& g, void* ws, size_t ws_bytes,
                          cudaStream_t s) {
-  if (!local_gradients_tf32_takes(g, sizeof(T))) return DK_ERR_UNSUPPORTED;
+  if (!local_gradients_pieces_takes(g, sizeof(T))) return DK_ERR_UNSUPPORTED;
   const TilePlan& t = gradients_plan(g);
   if (t.smem > (size_t)device_smem_optin() || ws == nullptr || ws_bytes < (size_t)t.blocks * g.C * g.cells * sizeof(float)) return DK_ERR_UNSUPPORTED;
-  auto kern = g.sH == 1 ? tf32_gradients_kernel<T, 1> : tf32_gradients_kernel<T, 2>;
+  auto kern = g.sH == 1 ? pieces_gradients_kernel<T, 1> : pieces_gradients_kernel<T, 2>;
   if (int rc = enable_smem(kern, t.smem)) return rc;
   float* partial = reinterpret_cast<float*>(ws);
   kern<<<t.blocks, 32 * kWarps, t.smem, s>>>(dy, x, rot, w, drot, partial, g, t);
   if (int rc = check_launch()) return rc;
   return reduce_bank<T>(partial, dw, g.C * g.cells, t.blocks, s);
 }
-template int local_gradients_tf32<float>(const float*, const float*, const float*, const float*, float*, float*, const Geom&, void*, size_t,
+template int local_gradients_pieces<float>(const float*, const float*, const float*, const float*, float*, float*, const Geom&, void*, size_t,
                                          cudaStream_t);
-template int local_gradients_tf32<__half>(const __half*, const __half*, const __half*, const __half*, __half*, __half*, const Geom&, void*,
+template int local_gradients_pieces<__half>(const __half*, const __half*, const __half*, const __half*, __half*, __half*, const Geom&, void*,
                                           size_t, cudaStream_t);
 
 }  // namespace dk

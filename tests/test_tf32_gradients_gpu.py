@@ -1,4 +1,4 @@
-"""Offset and bank gradients of the local operator from tf32 pieces: calls of 64 tiles and more, with channels that do not fill a step of 8 or a
+"""Offset and bank gradients of the local operator from bf16 pieces of fp32 values: calls of 64 tiles and more, with channels that do not fill a step of 8 or a
 chunk of 32, tiles of odd shapes, pixels that do not fill a warp, both strides, and values that are not finite."""
 import pytest
 import torch
@@ -37,9 +37,9 @@ def test_shapes(n, c, h, w, stride, scope, dtype):
 
 @pytest.mark.parametrize("n,c,h,w,stride", [(8, 64, 56, 56, 1), (40, 96, 30, 41, 2), (64, 384, 14, 14, 1)])
 def test_error_against_fp64(n, c, h, w, stride):
-    """2-norm of fp32 results.  Pieces: 2^-24 of a product; a step's three products are truncated at 2^-23 of their sum, 6e-8 in the mean; the
-    coordinate is rounded at its size for the hat products (1.2e-7 of a kernel value, bank only); rounded additions of C / 8 steps
-    (offsets) or of the pixels' steps (bank), 8.6e-8 sqrt(L / 24) for chains of L = C / 8 and of 12 steps a tile: 1.4e-7 and 2.6e-7."""
+    """2-norm of fp32 results.  Pieces: 2^-26 of a product in the mean; the products of a step are truncated at 2^-23 of their sum, 6e-8 in the mean; the
+    coordinate is rounded at its size for the hat products (1.2e-7 of a kernel value, bank only); rounded additions of C / 16 steps
+    (offsets) or of the pixels' steps (bank), 8.6e-8 sqrt(L / 24) for chains of L = C / 16 and of 12 steps a tile: 1.2e-7 and 2.6e-7."""
     case = make_case(n, c, h, w, stride=stride, rot_std=1.0, seed=c)
     for name, g, v, bound in zip(("rotation", "weight"), _run(case, torch.float32), _want(case, torch.float32), (1.7e-7, 2.9e-7)):
         err = float((g.double().cpu() - v).norm() / v.norm())
@@ -67,3 +67,18 @@ def test_products_that_are_not_finite():
                 if 0 <= i < 4 and 0 <= j < 4:
                     u[i, j] = True
     assert not changed[17, 0][~u.to(DEV)].any()
+
+
+@pytest.mark.parametrize("n,c,h,w,stride", [(16, 16, 61, 63, 2), (27, 16, 11, 17, 1), (5, 40, 80, 86, 2), (4, 120, 53, 57, 1), (8, 200, 30, 28, 1)])
+def test_no_less_exact_than_each_gradient_alone(n, c, h, w, stride):
+    """Either gradient alone comes from a kernel with an fp32 multiply-add per term; how many are wanted must not cost precision."""
+    from deformable_kernels.ops.deform_kernel.functions import sample_depthwise
+    case = make_case(n, c, h, w, stride=stride, rot_std=1.0, seed=c + h)
+    both, want = _run(case, torch.float32), _want(case, torch.float32)
+    x, r, k, dy = (case[name].to(DEV) for name in ("input", "rotation", "weight", "grad_output"))
+    for i, (name, leaf) in enumerate((("rotation", r), ("weight", k))):
+        leaf.requires_grad_(True)
+        alone, = torch.autograd.grad(sample_depthwise(x, r, k, **case["args"]), leaf, dy)
+        leaf.requires_grad_(False)
+        error = [float((g.double().cpu() - want[i]).norm()) for g in (both[i], alone)]
+        assert error[0] < 1.01 * error[1], "%s %.3e %.3e" % (name, *error)  # a 2-norm over 2e4 elements and more: 1 % is its own scatter
