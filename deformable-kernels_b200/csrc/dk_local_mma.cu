@@ -211,13 +211,15 @@ __global__ void __launch_bounds__(448, 2) mma_conv_kernel(const __half* __restri
 
 // ------------------------------------------------------------------ the same in fp32 arithmetic, any number of channels
 // fp16 with channels that are no multiple of 16 has always been computed with fp32 kernel values: the hat products are two fp16 pieces (the
-// second the rest of the first, 2^-25 of the whole left out), the bank is exact, so two mma with fp32 sums give K, which then meets the
-// widened x.  Columns beside the image are zeros and not products with a zero kernel value, and a block whose bank holds a value that
+// second the rest of the first), the bank is exact, so two mma with fp32 sums give K, which then meets the widened x.  The pieces are those of
+// 2^15 times the product, so that 2^-23 of a product is left out and not 2^-25 of one: small ones keep their bits.  Columns beside the image are zeros and not products with a zero kernel value, and a block whose bank holds a value that
 // is not finite computes every output by itself: such values stay with the samples that touch them.
 // Against gathered cells (local_conv_kernel: four reads and five multiply-adds per channel and tap), us, forward + grad-input: 8 x 72 of
 // 75 x 101 189 -> 133, 64 x 88 of 28 x 30 195 -> 55, 40 x 72 of 56 x 50 at stride 2 191 -> 53, 128 x 200 of 7 x 7 67 -> 30, 64 x 24 of 112 x 110
 // 790 -> 278, 64 x 8 of 56 x 54 at stride 2 54 -> 47, 1 x 72 of 28 x 30 21 -> 15.  Rows of odd width wait for their loader (8 x 72 of 75 x 101 115
 // with its rows word by word, of 75 x 102 73).
+constexpr float kHatScale = 32768.f;
+
 template <int S, bool TRANSPOSED>
 __device__ __noinline__ float conv_alone(const __half* __restrict__ src, const __half* __restrict__ rot, const __half* __restrict__ w, const Geom& g,
                                          int n, int c, int drow, int dcol) {
@@ -322,8 +324,8 @@ __global__ void __launch_bounds__(256, 2) mma_conv_full_kernel(const __half* __r
         const float v = ok ? ((float)fw + __half2float(rp[br.pitch_c])) + uw0 : 1e30f;
 #pragma unroll
         for (int k = 0; k < 2; ++k) {
-          const float b0 = lc.ok[2 * k] ? hat(u - lc.ca[2 * k]) * hat(v - lc.cb[2 * k]) : 0.f;
-          const float b1 = lc.ok[2 * k + 1] ? hat(u - lc.ca[2 * k + 1]) * hat(v - lc.cb[2 * k + 1]) : 0.f;
+          const float b0 = lc.ok[2 * k] ? hat(u - lc.ca[2 * k]) * hat(v - lc.cb[2 * k]) * kHatScale : 0.f;
+          const float b1 = lc.ok[2 * k + 1] ? hat(u - lc.ca[2 * k + 1]) * hat(v - lc.cb[2 * k + 1]) * kHatScale : 0.f;
           hi[t][k] = pack2(b0, b1);
           lo[t][k] = pack2(b0 - lo2f(hi[t][k]), b1 - hi2f(hi[t][k]));
         }
@@ -387,11 +389,12 @@ __global__ void __launch_bounds__(256, 2) mma_conv_full_kernel(const __half* __r
         for (int h = 0; h < 2; ++h) {
           if (cb16 + gq + 8 * h >= cnt) continue;
           __half* y = y0 + 8 * h * dplane;
+          const float r0 = acc[2 * h] * (1.f / kHatScale), r1 = acc[2 * h + 1] * (1.f / kHatScale);
           if (pl.pair_store) {
-            *reinterpret_cast<__half2*>(y) = __floats2half2_rn(acc[2 * h], acc[2 * h + 1]);
+            *reinterpret_cast<__half2*>(y) = __floats2half2_rn(r0, r1);
           } else {
-            y[0] = __float2half_rn(acc[2 * h]);
-            if (ow + 1 < Wd) y[1] = __float2half_rn(acc[2 * h + 1]);
+            y[0] = __float2half_rn(r0);
+            if (ow + 1 < Wd) y[1] = __float2half_rn(r1);
           }
         }
       }

@@ -37,6 +37,22 @@ def test_only_the_result_is_rounded(n, c, h, w, scope, stride):
         assert float((got - v).norm()) < 1.02 * float((rounded - v).norm()) + 1e-6 * float(v.norm())
 
 
+@pytest.mark.parametrize("stride", [1, 2])
+def test_small_hat_products_keep_their_bits(stride):
+    """Kernel values that come from the far edge of a hat alone.  Fractions of 2^-22 and 2^-10 keep every coordinate exact, so only the rounding
+    of the result is left; their products have up to 20 bits, the last of them 2^-32."""
+    case = make_case(2, 24, 14, 18, scope=(3, 5), stride=stride, seed=3)
+    rot = case["rotation"]
+    g = torch.Generator().manual_seed(4)
+    rot[:, 0::2] = torch.randint(-900, 900, rot[:, 0::2].shape, generator=g).to(rot.dtype) * 2.0 ** -10
+    rot[:, 1::2] = torch.randint(40, 400, rot[:, 1::2].shape, generator=g).to(rot.dtype) * 2.0 ** -22
+    case["weight"][..., :4] = 0
+    case["weight"][..., 4] *= 1000  # the last column of cells: taps of the last column, a fraction beyond the cell beside it
+    for got, v in zip(_run(case), _want(case)):
+        got, rounded = got.double().cpu(), v.half().double()
+        assert float((got - v).norm()) < 1.02 * float((rounded - v).norm()) + 1e-6 * float(v.norm())
+
+
 @pytest.mark.parametrize("w,stride", [(22, 1), (26, 2), (21, 1), (23, 2)])
 def test_values_that_are_not_finite(w, stride):
     case = make_case(2, 24, 10, w, stride=stride, rot_std=0.4, seed=w)
