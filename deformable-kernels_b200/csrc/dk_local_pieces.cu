@@ -4,20 +4,23 @@
 // Both are contractions of dK = dy * x with 16 cells: G[pixel, tap][cell] = sum_c dK W[c, cell] (then the floor-based derivative
 // weights) and dW[c][cell] = sum over pixels and taps of dK beta[(pixel, tap), cell].  An fp32 value is three bf16 pieces, 8 bits rounded each time,
 // which together are all of it (down to 2^-110, below which the last ones underflow); a product is six of their products, the smallest first,
-// and what is left out is 2^-23 of it at the most, 2^-26 in the mean (a rounding: 2^-24 and 2^-25.8).  The tensor cores truncate their sums, so no accumulator runs longer than
-// these six: a step of 16 channels (G) or of 8 pixels at two taps (dW) is added to the sums with one rounded addition.  Against fp64, separate fp32
-// kernels -> this one, 2-norm: 16 x 16 of 61 x 63 at stride 2 offsets 7.5e-8 -> 6.9e-8, bank 1.9e-7 -> 1.7e-7 (most of it the rounding of the
-// coordinates), 64 x 144 of 56 x 56 1.4e-7 -> 0.9e-7 and 5.2e-7 -> 2.0e-7.
+// and what is left out is 2^-23 of it at the most, 2^-26 in the mean (a rounding: 2^-24 and 2^-25.8).  The tensor cores truncate their
+// sums, so no accumulator runs longer than these six: a step of 16 channels (G) or of 8 pixels at two taps (dW) is added to the sums with
+// one rounded addition.  Against fp64, separate fp32 kernels -> this one, 2-norm: 16 x 16 of 61 x 63 at stride 2 offsets 7.5e-8 -> 6.9e-8,
+// bank 1.9e-7 -> 1.7e-7 (most of it the rounding of the coordinates), 64 x 144 of 56 x 56 1.4e-7 -> 0.9e-7 and 5.2e-7 -> 2.0e-7.
 //
 // Block: a tile of up to 96 pixels, a warp 8 of them, over all channels, 32 at a time, whose dy and x are staged while the previous ones are
 // multiplied.  G stays in registers (9 taps x 16 cells x 8 pixels per warp); the warps' bank sums of 32 channels meet in
 // shared memory, in their order, and are added to the block's partial sums.  dK is split once: movmatrix turns the pieces from the lanes'
 // order of the offsets (k = channels) to that of the bank (k = pixels).  Pairs of steps and pairs of taps fill the 16 k-slots so that every operand lies
-// in registers as it was loaded or made; two pieces of one step beside each other need copies of one of them and take 629 us below.
+// in registers as it was loaded or made; two pieces of one step beside each other need copies of one of them and take 629 us below.  A step left
+// over takes them that way for the offsets (64 x 24 of 112 x 110: 674 us beside a step of zeros, 617 so, 637 in separate kernels).
 //
-// fp32 64 x 144 of 56 x 56: 753 us in two kernels that gather or hold the cells with one fp32 multiply-add each -> 561.  Tensor pipe 42 %,
+// fp32 64 x 144 of 56 x 56: 753 us in two kernels that gather or hold the cells with one fp32 multiply-add each -> 558.  Tensor pipe 42 %,
 // issue 40 %: products, the pieces that feed them and the additions behind them follow each other in a warp, and 3 warps per scheduler (168 registers)
 // overlap part of it; tiles that do not fill and the tenth tap of the pairs are 15 % of the products.
+#include <type_traits>
+
 #include "dk_f32_tiles.cuh"
 
 namespace dk {
@@ -89,6 +92,12 @@ __device__ __forceinline__ void product(float (&d)[4], const uint4 (&a)[3], cons
   constexpr int A = E == 0 || E > 3 ? 0 : E == 1 ? 2 : 1, B = E == 0 ? 2 : E == 2 || E == 4 ? 1 : 0;
   if (E == 0) mul16(d, a[A], b.p[B], c.p[B]);
   else mad16(d, a[A], b.p[B], c.p[B]);
+}
+// The same in three products of two pieces each.  a: {third | first}, {second | second}, {first | first} from a[2] on down.
+template <int E>
+__device__ __forceinline__ void beside(float (&d)[4], const uint4 (&a)[3], const Pieces& b) {
+  if (E == 0) mul16(d, a[2], b.p[0], b.p[2]);
+  else mad16(d, a[2 - E], b.p[0], b.p[1]);
 }
 __device__ __forceinline__ void add4(f2 (&s)[2], const float (&d)[4]) {
   s[0] = add2(s[0], pair(d[0], d[1]));
@@ -253,61 +262,74 @@ __global__ void __launch_bounds__(32 * kWarps, 1) pieces_gradients_kernel(const 
       const float* ys = xs + 32 * R::X;
       // Two taps and two steps at a time: 16 k-slots are the channels of both steps (offsets), or the warp's pixels at both taps (bank).  The
       // products of a tap and a step are split once, in the lanes as the offsets want them, and movmatrix turns the pieces for the bank.
+      // A step that is left over by itself has two pieces beside each other in the products of the offsets.
       const int steps = min(4, (g.C - c0 + 7) >> 3);
       float* r = red + (warp * 16 + gq) * kRedPitch + 2 * q;
-#pragma unroll 1
-      for (int h = 0; h < steps; h += 2, r += 16) {
-        f2 acc[2][2], d[2];
+      const uint4* wq = banks + buffer * 6 * 32;
+      const float* yq = ys + 2 * q * R::Y + yg;
+      const float* xq = xs + 2 * q * R::X + xg;
+      auto pass = [&](auto pair_of_steps) {
+        constexpr int N = decltype(pair_of_steps)::value ? 2 : 1;
+        f2 acc[N][2], d[N];
         uint4 wp[3];
 #pragma unroll
-        for (int k = 0; k < 3; ++k) wp[k] = banks[(buffer * 6 + (h >> 1) * 3 + k) * 32];
+        for (int k = 0; k < 3; ++k) wp[k] = wq[32 * k];
+        if (N == 1) {
+          const uint2 w0 = make_uint2(wp[0].x, wp[0].y), w1 = make_uint2(wp[1].x, wp[1].y);
+          wp[2] = make_uint4(wp[2].x, wp[2].y, w0.x, w0.y), wp[1] = make_uint4(w1.x, w1.y, w1.x, w1.y), wp[0] = make_uint4(w0.x, w0.y, w0.x, w0.y);
+        }
 #pragma unroll
-        for (int j = 0; j < 2; ++j) {
-          const float* yp = ys + ((h + j) * 8 + 2 * q) * R::Y + yg;
+        for (int j = 0; j < N; ++j) {
+          const float* yp = yq + j * 8 * R::Y;
           d[j] = live_g ? pair(yp[0], yp[R::Y]) : 0;
           acc[j][0] = acc[j][1] = 0;
         }
-        const float* xp = xs + (h * 8 + 2 * q) * R::X + xg;
 #pragma unroll
         for (int t0 = 0; t0 < 9; t0 += 2) {
           uint4 bp[3];
 #pragma unroll
           for (int k = 0; k < 3; ++k) bp[k] = beta[(t0 >> 1) * 96 + 32 * k];
-          Pieces p[2][2], pt[2][2];  // [tap][step]
-          float u[2][4], v[2][4];
+          Pieces p[2][N], pt[2][N];  // [tap][step]
+          float u[2][4], v[N][4];
 #pragma unroll
           for (int i = 0; i < 2; ++i) {
             const int tap = t0 + i;
             if (tap > 8) break;
-            const float* at = xp + (tap / 3) * t.XW + tap % 3;
+            const float* at = xq + (tap / 3) * t.XW + tap % 3;
 #pragma unroll
-            for (int j = 0; j < 2; ++j) p[i][j] = split3(mul2(d[j], pair(at[j * 8 * R::X], at[j * 8 * R::X + R::X])));
+            for (int j = 0; j < N; ++j) p[i][j] = split3(mul2(d[j], pair(at[j * 8 * R::X], at[j * 8 * R::X + R::X])));
           }
 #pragma unroll
           for (int i = 0; i < 2; ++i)
 #pragma unroll
-            for (int j = 0; j < 2; ++j)
+            for (int j = 0; j < N; ++j)
 #pragma unroll
               for (int k = 0; k < 3; ++k) pt[i][j].p[k] = t0 + i < 9 ? turned(p[i][j].p[k]) : 0u;
           if (t0 == 8) bp[0].z = bp[0].w = bp[1].z = bp[1].w = bp[2].z = bp[2].w = 0u;
 #define DK_PRODUCT(E)                                                                    \
-  if (E != 1 || sizeof(T) == 4) { /* fp16 banks are two pieces */                        \
-    product<E>(u[0], wp, p[0][0], p[0][1]);                                              \
-    if (t0 < 8) product<E>(u[1], wp, p[1][0], p[1][1]);                                  \
+  if (N == 2 && (E != 1 || sizeof(T) == 4)) { /* fp16 banks are two pieces */            \
+    product<E>(u[0], wp, p[0][0], p[0][N - 1]);                                          \
+    if (t0 < 8) product<E>(u[1], wp, p[1][0], p[1][N - 1]);                              \
   }                                                                                      \
-  product<E>(v[0], bp, pt[0][0], pt[1][0]), product<E>(v[1], bp, pt[0][1], pt[1][1]);
+  if (N == 1 && E < 3)                                                                   \
+    for (int i = 0; i < (t0 < 8 ? 2 : 1); ++i) beside<E>(u[i], wp, p[i][0]);             \
+  for (int j = 0; j < N; ++j) product<E>(v[j], bp, pt[0][j], pt[1][j]);
           DK_PRODUCT(0) DK_PRODUCT(1) DK_PRODUCT(2) DK_PRODUCT(3) DK_PRODUCT(4) DK_PRODUCT(5)
 #undef DK_PRODUCT
           add4(G[t0 / 3][t0 % 3], u[0]);
           if (t0 < 8) add4(G[(t0 + 1) / 3 % 3][(t0 + 1) % 3], u[1]);
-          add4(acc[0], v[0]), add4(acc[1], v[1]);
+#pragma unroll
+          for (int j = 0; j < N; ++j) add4(acc[j], v[j]);
         }
 #pragma unroll
-        for (int j = 0; j < 2; ++j) {
+        for (int j = 0; j < N; ++j) {
           *reinterpret_cast<f2*>(r + 8 * j) = acc[j][0];
           *reinterpret_cast<f2*>(r + 8 * kRedPitch + 8 * j) = acc[j][1];
         }
-      }
+      };
+#pragma unroll 1
+      for (int h = 1; h < steps; h += 2, r += 16, wq += 96, yq += 16 * R::Y, xq += 16 * R::X) pass(std::true_type());
+      if (steps & 1) pass(std::false_type());
       __syncthreads();
 #pragma unroll
       for (int i = threadIdx.x; i < 512; i += 32 * kWarps) {
