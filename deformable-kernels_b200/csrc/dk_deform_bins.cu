@@ -39,7 +39,8 @@ __host__ __device__ inline int bank_cells(const Geom& g) { return bank_unused_ce
 // Without kernel-space offsets (rot null) the sampled kernel is the same at every pixel: in place of the bank its value per (tap,
 // channel) is laid out, and one read stands for four and their multiply-adds; the bank gradient meets the cells once per tap.  16 x 192
 // of 28 x 28, 3 x 3 scope: forward 39 -> 25 us, gather 53 -> 44, offsets 43 -> 31, bank 42 -> 33; 13 x 88 of 80 x 80 in fp16, all, 848 -> 646.
-__host__ __device__ inline bool fixed_kernel(const Geom& g, const void* rot) { return rot == nullptr && g.taps <= bank_cells(g); }
+// The unused cell keeps its zeros; samples that are not used select zero in place of their tap's value, which may not be finite.
+__host__ __device__ inline bool fixed_kernel(const Geom& g, const void* rot) { return rot == nullptr && g.taps <= bank_unused_cell(g); }
 
 // one sample point: corner coefficients of the image and of the bank, {bank cell * 32, column of the cell, pixel * Cp, 0}
 struct Rec {
@@ -449,10 +450,11 @@ __global__ void __launch_bounds__(32 * kRowWarps, 3) dcn_forward_kernel(const T*
 #pragma unroll
         for (int h = 0; h < 2; ++h) {
           const float4 im = recs[tap][j + h].im, b = recs[tap][j + h].a;
+          const bool used = im.x + im.y > 0.f;  // the two are 1 - lh and lh, or zeros
 #pragma unroll
           for (int e = 0; e < V; ++e) {
             const float xs = im.x * (im.z * x[h][0][e] + im.w * x[h][1][e]) + im.y * (im.z * x[h][2][e] + im.w * x[h][3][e]);
-            if (FIXED) acc[h][e] += xs * k[0][0][e];
+            if (FIXED) acc[h][e] += xs * (used ? k[0][0][e] : 0.f);
             else acc[h][e] += xs * (b.x * (b.z * k[h][0][e] + b.w * k[h][1][e]) + b.y * (b.z * k[h][2][e] + b.w * k[h][3][e]));
           }
         }
@@ -510,11 +512,12 @@ __global__ void __launch_bounds__(32 * kRowWarps, 3) dcn_coords_kernel(const T* 
 #pragma unroll
       for (int h = 0; h < 2; ++h) {
         const float4 im = recs[warp][j + h].im, b = recs[warp][j + h].a;
+        const bool used = im.x + im.y > 0.f;
 #pragma unroll
         for (int e = 0; e < V; ++e) {
           const float top = im.z * x[h][0][e] + im.w * x[h][1][e], low = im.z * x[h][2][e] + im.w * x[h][3][e];
           const float ktop = FIXED ? 0.f : b.z * k[h][0][e] + b.w * k[h][1][e], klow = FIXED ? 0.f : b.z * k[h][2][e] + b.w * k[h][3][e];
-          const float yk = y[h][e] * (FIXED ? k[0][0][e] : b.x * ktop + b.y * klow);
+          const float yk = y[h][e] * (FIXED ? (used ? k[0][0][e] : 0.f) : b.x * ktop + b.y * klow);
           s[h][0] += yk * (low - top);
           s[h][1] += yk * (im.x * (x[h][1][e] - x[h][0][e]) + im.y * (x[h][3][e] - x[h][2][e]));
           if (ROT) {

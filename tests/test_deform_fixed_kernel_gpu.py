@@ -42,3 +42,23 @@ def test_values_that_are_not_finite():
     assert bad[:, 7].any() and not bad[:, [c for c in range(24) if c != 7]].any()
     bad = ~torch.isfinite(dw)
     assert bad[9].any() and not bad[[c for c in range(24) if c != 9]].any()
+
+
+@pytest.mark.parametrize("n,c,stride,dtype", [(2, 24, 1, torch.float32), (2, 64, 2, torch.float32), (3, 72, 1, torch.float16)])
+def test_samples_outside_the_image_meet_no_value_that_is_not_finite(n, c, stride, dtype):
+    """Finite wherever the oracle is: a tap that falls outside the image has no kernel value, whatever the bank holds."""
+    from deformable_kernels.ops.deform_kernel.functions import deform_sample_depthwise
+    from oracle import dk_oracle as O
+    case = make_case(n, c, 12, 14, scope=(3, 3), stride=stride, rot_std=0.0, off_std=3.0, seed=c)
+    case["weight"][7, 0, 0, 1], case["weight"][11, 0, 2, 2], case["weight"][c - 1, 0, 1, 0] = float("inf"), float("nan"), -float("inf")
+    x, o, wt, dy = (case[i].to(dtype).cuda() for i in ("input", "offset", "weight", "grad_output"))
+    leaves = [t.requires_grad_(True) for t in (x, o)]
+    y = deform_sample_depthwise(x, o, None, wt, **case["args"])
+    got = (y.detach(),) + torch.autograd.grad(y, leaves, dy)
+    a = [case[i].to(dtype).float() for i in ("grad_output", "input", "offset", "rotation", "weight")]
+    want = (O.deform_sample_depthwise_forward(*a[1:], **case["args"]),) + tuple(O.deform_sample_depthwise_backward(*a, **case["args"])[:2])
+    for name, g, v in zip(("output", "input", "offset"), got, want):
+        finite = torch.isfinite(v)
+        assert (~finite).any() and finite.any(), name
+        assert torch.isfinite(g.cpu()[finite]).all(), name
+        assert rel_err(g.cpu()[finite], v[finite].to(dtype)) < (1e-5 if dtype == torch.float32 else 2e-3), name
