@@ -221,7 +221,7 @@ __global__ void __launch_bounds__(512, 1) mma_deform_fwd_kernel(const __half* __
   const int total_units = g.N * pl.bands;
   const int u_begin = blockIdx.x * pl.units_per_block;
   const int u_end = min(u_begin + pl.units_per_block, total_units);
-  const bool even_w = (g.Wo & 1) == 0;
+  const bool even_w = (g.Wo & 1) == 0 && (reinterpret_cast<uintptr_t>(y) & 3) == 0;  // pairs of pixels lie on words
   constexpr bool zero_rot = ZR;  // rot == nullptr
   unsigned bf[9][2];
   if (zero_rot) {

@@ -121,3 +121,35 @@ def test_forward_without_its_scratch(rotation):
                                                              C.ptr(ws if size else None), size, C.stream_ptr(x.device))
         assert status == 0, size
         assert rel_err(y, want) < 2e-3, size  # both round corner weights, hat products and K to fp16
+
+
+def _behind(t, halves):
+    """The same values so many halves behind an aligned address."""
+    buf = torch.empty(t.numel() + 8, dtype=t.dtype, device=t.device)
+    return buf[halves:halves + t.numel()].view(t.shape).copy_(t)
+
+
+@pytest.mark.parametrize("n,c,h,w,stride", [(8, 64, 24, 40, 1), (24, 64, 24, 40, 1), (40, 48, 32, 60, 2)])  # forward of the first: planes on chip
+@pytest.mark.parametrize("halves", [1, 2, 4])
+def test_operands_at_any_address(n, c, h, w, stride, halves):
+    """Widths and planes allow the wide loads and stores, the addresses do not: the results are the same, of most kernels bit for bit."""
+    from deformable_kernels import _cabi as C
+    case = make_case(n, c, h, w, scope=(4, 4), stride=stride, rot_std=0.7, off_std=2.0, seed=14)
+    dy, x, o, r, wt = (case[k].to(torch.float16).cuda() for k in ("grad_output", "input", "offset", "rotation", "weight"))
+    g = C.geom(tuple(x.shape), (3, 3), (stride, stride), (1, 1), (1, 1), (4, 4), 1)
+    size = max(C.lib.dk_deform_sample_depthwise_forward_workspace_bytes(g, C.DK_F16), C.lib.dk_deform_sample_depthwise_backward_workspace_bytes(g, C.DK_F16))
+    ws = torch.empty(size, dtype=torch.uint8, device="cuda")
+    s = C.stream_ptr(x.device)
+    results = []
+    for k in (0, halves):
+        a, b, d, e, f = (_behind(t, k) for t in (dy, x, o, r, wt))
+        y, dx, do, dr, dw = (_behind(torch.zeros_like(t), k) for t in (dy, x, o, r, wt))
+        assert C.lib.dk_deform_sample_depthwise_forward_ws(C.ptr(b), C.ptr(d), C.ptr(e), C.ptr(f), C.ptr(y), g, C.DK_F16, C.ptr(ws), size, s) == 0
+        assert C.lib.dk_deform_sample_depthwise_backward(C.ptr(a), C.ptr(b), C.ptr(d), C.ptr(e), C.ptr(f), C.ptr(dx), C.ptr(do), C.ptr(dr), C.ptr(dw), g,
+                                                         C.DK_F16, C.ptr(ws), size, s) == 0
+        results.append([t.clone() for t in (y, dx, do, dr, dw)])
+    for k, (first, other) in enumerate(zip(*results)):
+        if n > 8 or k == 0:
+            assert torch.equal(first, other)
+        else:  # the kernels of few samples add in the order of the day: two roundings to fp16
+            assert rel_err(first, other) < 1e-3
