@@ -252,6 +252,14 @@ __device__ __forceinline__ unsigned fma2h(unsigned a, unsigned b, unsigned c) {
 }
 __device__ __forceinline__ unsigned word(const uint4& v, int k) { return k == 0 ? v.x : k == 1 ? v.y : k == 2 ? v.z : v.w; }
 __device__ __forceinline__ uint4 line16(const char* p) { return __ldg(reinterpret_cast<const uint4*>(p)); }
+__device__ __forceinline__ unsigned sub2h(unsigned a, unsigned b) {
+  const __half2 r = __hsub2(*reinterpret_cast<const __half2*>(&a), *reinterpret_cast<const __half2*>(&b));
+  return *reinterpret_cast<const unsigned*>(&r);
+}
+// differences of the corners: lower - upper on the left and on the right, right - left above and below
+__device__ __forceinline__ unsigned across(const uint4 (&x)[4], int k, int j) {
+  return k < 2 ? sub2h(word(x[k + 2], j), word(x[k], j)) : sub2h(word(x[2 * k - 3], j), word(x[2 * k - 4], j));
+}
 // the four corners of a sample
 __device__ __forceinline__ void corners(uint4 (&x)[4], const char* upper, size_t below) {
   const char* lower = upper + below;
@@ -443,9 +451,10 @@ __global__ void __launch_bounds__(128, 3) line_forward_kernel(const __half* __re
 
 // ------------------------------------------------------------------ offset and bank gradients
 // d(kernel offset) = sum_c dy xs dK/d(u|v): G = (dy xs) W as an mma over the channels, then the four cells around the sample
-// with the derivatives of the hats.  d(image offset) = sum_c dy K dxs/d(h|w): differences of the four sums S_k = sum_c (dy K) x_k over
-// the corners, an mma of the products whose other operand is one in the columns k, k + 4; a pixel's two rows are its two halves of the
-// channels.  dW = beta^T (dy xs) over the pixels, for which movmatrix turns the products.
+// with the derivatives of the hats.  d(image offset) = sum_c dy K dxs/d(h|w): from the four sums S_k = sum_c (dy K) dx_k over
+// the differences of neighbouring corners, an mma of the products whose other operand is one in the columns k, k + 4; a pixel's two rows are its two
+// halves of the channels.  Products with the corners themselves, subtracted afterwards, overflow where only the corners are large (x of 100, dy
+// of 500) and lose what they have in common: 8 x 512 of 28 x 28 with x around 10, 1.1e-3 off fp64 against 4.5e-4 (4.6e-4 and 5.1e-4 around 0).  dW = beta^T (dy xs) over the pixels, for which movmatrix turns the products.
 // A warp has 64 channels for the whole run of its block (the bank sums stay in registers) and walks over groups of 16 pixels;
 // the warps of a stream have different channels of the same pixels, and their sums over channels meet in shared memory.
 struct CoordPlan {
@@ -463,7 +472,7 @@ __global__ void __launch_bounds__(128, 3) line_coords_kernel(const __half* __res
   extern __shared__ __align__(16) unsigned char smem_raw[];
   const Geom& g = lg.g;
   const int npx = 16 * pl.streams, nwarps = blockDim.x >> 5;
-  constexpr int NP = ROT ? 160 : 128;  // floats that a warp leaves for 16 pixels and a tap: S [half][pixel][corner], then u and v
+  constexpr int NP = ROT ? 160 : 128;  // floats that a warp leaves for 16 pixels and a tap: S [half][pixel][difference], then u and v
   uint4* beta = reinterpret_cast<uint4*>(smem_raw);                               // [tap][npx][2]
   uint4* wgs = beta + kLineTaps * npx * 2;                                        // [unit][4 steps of 16 channels][lane]
   float* grids = reinterpret_cast<float*>(wgs + (ROT ? pl.upb * 128 : 0));        // [warp][kGridCells][kGridPitch]
@@ -574,8 +583,8 @@ __global__ void __launch_bounds__(128, 3) line_coords_kernel(const __half* __res
           for (int k = 0; k < 4; ++k)
 #pragma unroll
             for (int j = 0; j < 4; j += 2) {
-              const unsigned a[4] = {hmul2u(yk[j][0], word(xa[k], j)), hmul2u(yk[j][1], word(xe[k], j)), hmul2u(yk[j + 1][0], word(xa[k], j + 1)),
-                                     hmul2u(yk[j + 1][1], word(xe[k], j + 1))};
+              const unsigned a[4] = {hmul2u(yk[j][0], across(xa, k, j)), hmul2u(yk[j][1], across(xe, k, j)),
+                                     hmul2u(yk[j + 1][0], across(xa, k, j + 1)), hmul2u(yk[j + 1][1], across(xe, k, j + 1))};
               if (k == 0) mul16(j ? E : D, a, one[k], one[k]);
               else mad16(j ? E : D, a[0], a[1], a[2], a[3], one[k], one[k]);
             }
@@ -652,8 +661,8 @@ __global__ void __launch_bounds__(128, 3) line_coords_kernel(const __half* __res
           s.x += v.x, s.y += v.y, s.z += v.z, s.w += v.w;
         }
         const float2 l = frac[flip * kLineTaps * npx + tap * npx + st * 16 + px];
-        a = (1.f - l.y) * (s.z - s.x) + l.y * (s.w - s.y);
-        b = (1.f - l.x) * (s.y - s.x) + l.x * (s.w - s.z);
+        a = (1.f - l.y) * s.x + l.y * s.y;
+        b = (1.f - l.x) * s.z + l.x * s.w;
       }
       if (pl.sets == 1) {
         __half* to = kernel_space ? drot : doff;

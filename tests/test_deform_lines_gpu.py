@@ -123,6 +123,25 @@ def test_forward_without_its_scratch(rotation):
         assert rel_err(y, want) < 2e-3, size  # both round corner weights, hat products and K to fp16
 
 
+@pytest.mark.parametrize("top,mean", [(800, 70), (1600, 30)])
+def test_offset_gradients_where_only_the_corners_are_large(top, mean):
+    """|dy K x| beyond fp16 with |dy x| and |dy K dx| inside it: a scaled loss and an input far from zero.  The differences of the corners are exact."""
+    case = make_case(32, 64, 30, 28, scope=(4, 4), rot_std=0.7, off_std=2.0, seed=13)
+    case["grad_output"] = case["grad_output"].clamp(-1, 1) * top
+    case["input"] = mean + case["input"]
+    case["weight"] *= 3.0
+    assert top * case["input"].abs().max() < 65504 < top * mean * case["weight"].abs().max() * 0.75
+    got, want = _run(case)["grad_offset"].cpu(), _want(case)["grad_offset"]
+    # samples whose four corners lie in the image: beside it the difference is the value itself
+    off = case["offset"].half().float().view(32, 9, 2, 30, 28)
+    tap = torch.arange(9.).view(9, 1, 1)
+    h, w = off[:, :, 0] + torch.arange(30.).view(30, 1) - 1 + tap // 3, off[:, :, 1] + torch.arange(28.) - 1 + tap % 3
+    inside = ((h >= 0) & (h < 29) & (w >= 0) & (w < 27)).repeat_interleave(2, 1)
+    got, want = got[inside], want[inside]
+    assert want.abs().max() < 65504 and torch.isfinite(got).all()
+    assert rel_err(got, want.half()) < 2e-3
+
+
 def _behind(t, halves):
     """The same values so many halves behind an aligned address."""
     buf = torch.empty(t.numel() + 8, dtype=t.dtype, device=t.device)
