@@ -828,31 +828,75 @@ struct GatherPlan {
   int R, bands, windows, warps, sets, bins;
 };
 
-// one element of grad-input, every product to its own corners only: where the sums of a window are not finite
-__device__ __noinline__ float gather_alone(const float4* __restrict__ rec_n, const int* __restrict__ st_n, const __half* __restrict__ dyt,
-                                           const __half* __restrict__ w, const LineGeom& lg, int n, int c, int r, int col) {
+// Grad-input of a row of a window, every product to its own corners only: for the elements whose sums in the window are not finite.  A lane has
+// the channels c, c + 1; bit t (4 + t) of `wanted`: the columns 2 t, 2 t + 1 of c (c + 1).  The warp walks over the records of the two rows of
+// cells once for all its channels and columns (an element at a time, all of 64 x 256 of 56 x 56 17 ms, so 3).
+__device__ __noinline__ void gather_row_alone(const float4* __restrict__ rec_n, const int* __restrict__ st_n, const __half* __restrict__ dyt,
+                                              const __half* __restrict__ w, __half* __restrict__ dx, const LineGeom& lg, int n, int c, int r, int w0,
+                                              unsigned wanted) {
   const Geom& g = lg.g;
-  const __half* y = reinterpret_cast<const __half*>(reinterpret_cast<const char*>(dyt) + (c >> 6) * lg.yu) + (c & 63);
-  float sum = 0.f;
-  for (int h0 = r - 1; h0 <= r; ++h0) {
-    const int* s = st_n + (h0 + 1) * (g.W + 1) + col;
-    for (int i = s[0]; i < s[2]; ++i) {
-      const float4 rec = rec_n[i];
-      const unsigned id = __float_as_uint(rec.w), r2 = __float_as_uint(rec.z);
-      Sample q;
-      bank_point(q, id >> 27, lo2f(r2), hi2f(r2), g);
-      const float fl = floorf(rec.x), lw = rec.x - fl;
-      const float coef = (h0 == r ? 1.f - rec.y : rec.y) * ((int)fl == col ? 1.f - lw : lw);
-      float k = 0.f;
-      for (int e = 0; e < 4; ++e) {
-        const int a = q.u0 + (e >> 1), b = q.v0 + (e & 1);
-        if (a >= 0 && a < g.scH && b >= 0 && b < g.scW)
-          k += (e >> 1 ? q.lu : 1.f - q.lu) * (e & 1 ? q.lv : 1.f - q.lv) * __half2float(w[(size_t)c * g.cells + a * g.scW + b]);
-      }
-      sum += coef * (k * __half2float(y[((size_t)n * g.P + (id & 0x7ffffffu)) * 64]));
-    }
+  const char* yl = reinterpret_cast<const char*>(dyt) + (c >> 6) * lg.yu + (size_t)n * g.P * kLine + (c & 63) * 2;
+  const int lane = threadIdx.x & 31;
+  unsigned bank[36];  // both channels, the first one's in the low halves: 4 x 4 cells with a border of zeros
+#pragma unroll
+  for (int k = 0; k < 36; ++k) {
+    const int a = k / 6 - 1, b = k - (k / 6) * 6 - 1;
+    bank[k] = a >= 0 && a < 4 && b >= 0 && b < 4 ? chans2(w, c, a * 4 + b, g) : 0u;
   }
-  return sum;
+  float2 sum[10];  // columns w0 - 1 .. w0 + 8
+#pragma unroll
+  for (int k = 0; k < 10; ++k) sum[k] = make_float2(0.f, 0.f);
+  for (int h0 = r - 1; h0 <= r; ++h0) {
+    const int* s = st_n + (h0 + 1) * (g.W + 1) + w0;
+    const int last = s[min(9, g.W + 1 - w0)];
+    int cur = 0;  // records come by column: the sums of two neighbours stay in registers
+    float2 left = sum[0], right = sum[1];
+    for (int i0 = s[0]; i0 < last; i0 += 32) {
+      Sample q;  // a record per lane
+      q.u0 = q.v0 = 0, q.lu = q.lv = 0.f;
+      float lw = 0.f, row = 0.f;
+      int col = 0, px = 0;
+      if (i0 + lane < last) {
+        const float4 rec = __ldg(rec_n + i0 + lane);
+        const unsigned id = __float_as_uint(rec.w), r2 = __float_as_uint(rec.z);
+        bank_point(q, id >> 27, lo2f(r2), hi2f(r2), g);
+        const float fl = floorf(rec.x);
+        lw = rec.x - fl, row = h0 == r ? 1.f - rec.y : rec.y, col = (int)fl - w0, px = id & 0x7ffffffu;
+      }
+      const int at = ((q.u0 + 1) * 6 + q.v0 + 1) << 4 | (col + 1), cnt = min(32, last - i0);
+      const float cl = row * (1.f - lw), cr = row * lw;
+      auto line = [&](int k) { return __ldg(reinterpret_cast<const unsigned*>(yl + (size_t)__shfl_sync(0xffffffffu, px, k) * kLine)); };
+      unsigned y0 = line(0), y1 = line(1), y2 = line(2), y3 = line(3);
+      // not unrolled: a body of eight records took twice as long, two thirds of it waiting for instructions
+#pragma unroll 1
+      for (int k = 0; k < cnt; ++k) {
+        const unsigned y = y0;
+        y0 = y1, y1 = y2, y2 = y3, y3 = line((k + 4) & 31);
+        const int o = __shfl_sync(0xffffffffu, at, k);
+        const float u = __shfl_sync(0xffffffffu, q.lu, k), t = __shfl_sync(0xffffffffu, q.lv, k);
+        const float l = __shfl_sync(0xffffffffu, cl, k), m = __shfl_sync(0xffffffffu, cr, k);
+        const unsigned* b = bank + (o >> 4);
+        float a0 = 0.f, a1 = 0.f;
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+          const float h = (e >> 1 ? u : 1.f - u) * (e & 1 ? t : 1.f - t);
+          const unsigned cell = b[(e >> 1) * 6 + (e & 1)];
+          a0 += h * lo2f(cell), a1 += h * hi2f(cell);
+        }
+        const float v0 = a0 * lo2f(y), v1 = a1 * hi2f(y);
+        while (cur < (o & 15)) sum[cur++] = left, left = right, right = sum[cur + 1];
+        left.x += l * v0, left.y += l * v1;
+        right.x += m * v0, right.y += m * v1;
+      }
+    }
+    sum[cur] = left, sum[cur + 1] = right;
+  }
+  __half* o = dx + ((size_t)n * g.C + c) * g.HW + (size_t)r * g.W + w0;
+  for (int k = 0; k < 8; ++k) {
+    if (w0 + k >= g.W) break;
+    if (c < g.C && (wanted >> (k >> 1) & 1)) o[k] = __float2half_rn(sum[k + 1].x);
+    if (c + 1 < g.C && (wanted >> (4 + (k >> 1)) & 1)) o[g.HW + k] = __float2half_rn(sum[k + 1].y);
+  }
 }
 
 // A block has 8 columns of R rows of dx and up to four units of 64 channels, a warp each.  It walks over the rows of cells that
@@ -991,17 +1035,15 @@ __global__ void __launch_bounds__(128, 4) line_gather_kernel(const __half* __res
     }
     if (up && active) {
       const int col = w0 + 2 * t;
+      bool all = true;
 #pragma unroll
       for (int j = 0; j < 4; ++j)
 #pragma unroll
         for (int h = 0; h < 2; ++h) {
           const int c = c0 + 8 * (gq >> 1) + 2 * j + (gq & 1) + 32 * h;
           if (c < g.C && col < g.W) {
-            float v0 = acc[0][j][2 * h], v1 = acc[0][j][2 * h + 1];
-            if (!(fabsf(v0) < INFINITY && fabsf(v1) < INFINITY)) {
-              v0 = gather_alone(rec_n, st_n, dyt, w, lg, n, c, h0, col);
-              if (col + 1 < g.W) v1 = gather_alone(rec_n, st_n, dyt, w, lg, n, c, h0, col + 1);
-            }
+            const float v0 = acc[0][j][2 * h], v1 = acc[0][j][2 * h + 1];
+            all &= fabsf(v0) < INFINITY && fabsf(v1) < INFINITY;
             __half* o = dx + ((size_t)n * g.C + c) * g.HW + (size_t)h0 * g.W + col;
             if (pairs) {
               *reinterpret_cast<unsigned*>(o) = pack2(v0, v1);
@@ -1011,6 +1053,18 @@ __global__ void __launch_bounds__(128, 4) line_gather_kernel(const __half* __res
             }
           }
         }
+      if (__any_sync(0xffffffffu, !all)) {
+        unsigned wanted = 0;  // the lane's channels there: c0 + 2 lane, + 1
+#pragma unroll
+        for (int j = 0; j < 4; ++j)
+#pragma unroll
+          for (int h = 0; h < 2; ++h) {
+            const unsigned b = __ballot_sync(0xffffffffu, !(fabsf(acc[0][j][2 * h]) < INFINITY && fabsf(acc[0][j][2 * h + 1]) < INFINITY));
+            if ((lane & 3) == j && (lane >> 4) == h) wanted = b >> (lane & 12) * 2 & 0xffu;
+          }
+        __syncwarp();  // the stores above come first
+        gather_row_alone(rec_n, st_n, dyt, w, dx, lg, n, c0 + 2 * lane, h0, w0, wanted);
+      }
     }
 #pragma unroll
     for (int j = 0; j < 4; ++j)

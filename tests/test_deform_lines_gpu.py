@@ -142,6 +142,23 @@ def test_offset_gradients_where_only_the_corners_are_large(top, mean):
     assert rel_err(got, want.half()) < 2e-3
 
 
+@pytest.mark.parametrize("n,c,h,w,stride", [(8, 192, 20, 24, 1), (6, 272, 25, 30, 2), (4, 144, 26, 29, 1)])
+def test_grad_input_of_values_that_are_not_finite(n, c, h, w, stride):
+    """Not finite exactly where the oracle is not: channels of every lane and half, both columns of a pair, windows with a remainder."""
+    case = make_case(n, c, h, w, scope=(4, 4), stride=stride, rot_std=0.3, off_std=1.5, seed=w)
+    gen = torch.Generator().manual_seed(5)
+    dy = case["grad_output"]
+    for k in range(40):
+        at = [int(torch.randint(s, (1,), generator=gen)) for s in dy.shape]
+        dy[at[0] // 2, at[1], at[2], at[3]] = (float("inf"), -float("inf"), float("nan"))[k % 3]
+    case["weight"][c - 3, 0, 1, 1], case["weight"][36, 0, 2, 0] = float("inf"), float("nan")
+    got, want = _run(case)["grad_input"].cpu(), _want(case)["grad_input"]
+    finite = torch.isfinite(want)
+    assert 100 < int((~finite).sum()) < finite.numel() // 10
+    assert torch.equal(torch.isfinite(got), finite)
+    assert rel_err(got[finite], want[finite].half()) < 2e-3
+
+
 def _behind(t, halves):
     """The same values so many halves behind an aligned address."""
     buf = torch.empty(t.numel() + 8, dtype=t.dtype, device=t.device)
