@@ -124,10 +124,18 @@ __device__ __noinline__ void bank_by_cells(float* red, const T* __restrict__ dy,
                                            const T* __restrict__ rot, const Geom& g, const TilePlan& t, int c0, int warp, int warps, int lane) {
   float* acc = red + warp * 512 + lane;
   for (int i = 0; i < 16; ++i) acc[i * 32] = 0.f;
+  const unsigned live = __ballot_sync(0xffffffffu, c0 + lane < g.C);
   if (c0 + lane >= g.C) return;
   const float uh0 = 0.5f * (float)(g.scH - 3), uw0 = 0.5f * (float)(g.scW - 3);
   const int first = blockIdx.x * t.per_block, last = min(first + t.per_block, t.tiles);
-  for (int tile = first; tile < last; ++tile) {
+  // a NaN stays: once every sum of the warp is one there is nothing left to find out
+  auto settled = [&]() {
+    bool all = true;
+    for (int i = 0; i < 16; ++i)
+      if ((i >> 2) < g.scH && (i & 3) < g.scW) all &= acc[i * 32] != acc[i * 32];
+    return __all_sync(live, all);
+  };
+  for (int tile = first; tile < last && !settled(); ++tile) {
     const TilePos tp = tile_pos(tile, t);
     const T* xc = x + ((size_t)tp.n * g.C + c0 + lane) * g.HW;
     for (int p = warp; p < t.TH * t.TW; p += warps) {

@@ -104,35 +104,88 @@ __device__ __forceinline__ void add4(f2 (&s)[2], const float (&d)[4]) {
   s[1] = add2(s[1], pair(d[2], d[3]));
 }
 
-// derivative towards the kernel-space offset (u: !dv, v: dv) from G [cell][8 pixels]
-__device__ __forceinline__ float derivative(const float* G, float r_h, float r_w, int fh, int fw, bool dv, const Geom& g) {
+// where a sample falls in the bank: upper left cell (-1 .. last) and the fractions
+struct Cells {
+  int a, b;
+  float lh, lw;
+};
+__device__ __forceinline__ bool cells_at(Cells& q, float r_h, float r_w, int fh, int fw, const Geom& g) {
   const float uh0 = 0.5f * (float)(g.scH - 3), uw0 = 0.5f * (float)(g.scW - 3);
   const float u = ((float)fh + r_h) + uh0, v = ((float)fw + r_w) + uw0;
-  if (!(u > -1.f && v > -1.f && u < (float)g.scH && v < (float)g.scW)) return 0.f;
+  if (!(u > -1.f && v > -1.f && u < (float)g.scH && v < (float)g.scW)) return false;
   const float fu = floorf(u), fv = floorf(v);
   // tap + shift is a small multiple of 1/2: u minus it is exact, and so is what the rounding of u lost
-  const float lh = (u - fu) + (r_h - (u - ((float)fh + uh0))), lw = (v - fv) + (r_w - (v - ((float)fw + uw0)));
-  const int a0 = (int)fu, b0 = (int)fv;
-  float c[2][2];
-#pragma unroll
-  for (int k = 0; k < 4; ++k) {
-    const int a = a0 + (k >> 1), b = b0 + (k & 1);
-    c[k >> 1][k & 1] = a >= 0 && a < g.scH && b >= 0 && b < g.scW ? G[(a * 4 + b) * 8] : 0.f;
-  }
-  return dv ? (1.f - lh) * (c[0][1] - c[0][0]) + lh * (c[1][1] - c[1][0]) : (1.f - lw) * (c[1][0] - c[0][0]) + lw * (c[1][1] - c[0][1]);
+  q.lh = (u - fu) + (r_h - (u - ((float)fh + uh0))), q.lw = (v - fv) + (r_w - (v - ((float)fw + uw0)));
+  q.a = (int)fu, q.b = (int)fv;
+  return true;
+}
+__device__ __forceinline__ bool cell_in(const Cells& q, int k, const Geom& g) {  // k-th of the four
+  return (unsigned)(q.a + (k >> 1)) < (unsigned)g.scH && (unsigned)(q.b + (k & 1)) < (unsigned)g.scW;
+}
+// derivatives towards the kernel-space offset from G of the four cells
+__device__ __forceinline__ float2 derivatives(const Cells& q, const float (&c)[4]) {
+  return make_float2((1.f - q.lw) * (c[2] - c[0]) + q.lw * (c[3] - c[1]), (1.f - q.lh) * (c[1] - c[0]) + q.lh * (c[3] - c[2]));
 }
 
-// G of one pixel and tap, cell by cell, where a product that is not finite would have reached the others' pieces (Inf - Inf)
+// The derivatives of one pixel and tap where G [cell][8 pixels] is not finite in a cell of theirs: the pieces of an infinite product are infinite and NaN.
+// Its four cells again, a multiply-add each.  Where other cells are finite every dK is, and only the bank's values that are not (or round to
+// infinity) count; else all channels do, until a NaN settles both derivatives.  64 x 144 of 56 x 56, offsets and bank, us, with all sixteen cells for
+// either derivative -> so: every dy NaN 36144 -> 1278, one infinite bank value 29929 -> 1725 (in
+// separate kernels 4326 and 767).
 template <typename T>
-__device__ __noinline__ void cells_alone(float* G, const T* __restrict__ dy, const T* __restrict__ x, const T* __restrict__ w, const Geom& g) {
-  float sum[16];
-  for (int k = 0; k < 16; ++k) sum[k] = 0.f;
-  for (int c = 0; c < g.C; ++c) {
-    const float dk = ld<float>(dy + (size_t)c * g.P) * ld<float>(x + (size_t)c * g.HW);
-    for (int k = 0; k < 16; ++k)
-      if ((k >> 2) < g.scH && (k & 3) < g.scW) sum[k] += dk * ld<float>(w + (size_t)c * g.cells + (k >> 2) * g.scW + (k & 3));
+__device__ __noinline__ float2 cells_alone(const Cells& q, const float* G, const T* __restrict__ dy, const T* __restrict__ x, const T* __restrict__ w,
+                                           const Geom& g) {
+  constexpr float kRounds = 3.3961e38f;  // bf16 values end at 2^128 (1 - 2^-8), those from 2^128 (1 - 2^-9) on round to infinity
+  float sum[4];
+  bool bad[4], by_bank = false;
+#pragma unroll
+  for (int k = 0; k < 16; ++k) by_bank |= fabsf(G[k * 8]) < INFINITY;
+#pragma unroll
+  for (int k = 0; k < 4; ++k) {
+    const bool in = cell_in(q, k, g);
+    sum[k] = in ? G[((q.a + (k >> 1)) * 4 + q.b + (k & 1)) * 8] : 0.f;
+    bad[k] = !(fabsf(sum[k]) < INFINITY);
   }
-  for (int k = 0; k < 16; ++k) G[k * 8] = sum[k];
+  const T* wk = w + q.a * g.scW + q.b;
+  if (by_bank) {
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+      if (!bad[k]) continue;
+      sum[k] = 0.f;
+      for (int c0 = 0; c0 < g.C; c0 += 8) {
+        float v[8];
+#pragma unroll
+        for (int i = 0; i < 8; ++i) v[i] = ld<float>(wk + (size_t)min(c0 + i, g.C - 1) * g.cells + (k >> 1) * g.scW + (k & 1));
+#pragma unroll
+        for (int i = 0; i < 8; ++i)
+          if (c0 + i < g.C && !(fabsf(v[i]) < kRounds)) sum[k] += ld<float>(dy + (size_t)(c0 + i) * g.P) * ld<float>(x + (size_t)(c0 + i) * g.HW) * v[i];
+      }
+      by_bank &= !(fabsf(sum[k]) < INFINITY);
+    }
+    if (by_bank) return derivatives(q, sum);
+  }
+#pragma unroll
+  for (int k = 0; k < 4; ++k) sum[k] = 0.f;
+  for (int c0 = 0; c0 < g.C; c0 += 4) {
+    float dk[4], b[4][4];
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      const int c = min(c0 + i, g.C - 1);
+      dk[i] = ld<float>(dy + (size_t)c * g.P) * ld<float>(x + (size_t)c * g.HW);
+#pragma unroll
+      for (int k = 0; k < 4; ++k) b[i][k] = cell_in(q, k, g) ? ld<float>(wk + (size_t)c * g.cells + (k >> 1) * g.scW + (k & 1)) : 0.f;
+    }
+    bool settled = false;
+#pragma unroll
+    for (int i = 0; i < 4; ++i)
+#pragma unroll
+      for (int k = 0; k < 4; ++k) {
+        if (c0 + i < g.C && cell_in(q, k, g)) sum[k] += dk[i] * b[i][k];
+        settled |= sum[k] != sum[k];
+      }
+    if (settled) break;
+  }
+  return derivatives(q, sum);
 }
 
 template <typename T, int S>
@@ -360,41 +413,40 @@ __global__ void __launch_bounds__(32 * kWarps, 1) pieces_gradients_kernel(const 
         *reinterpret_cast<f2*>(cells + (fw * 16 + gq + 8) * 8 + 2 * q) = G[fh][fw][1];
       }
       __syncwarp();
-      for (int e = part; e < 6; e += 4) {
-        const int fw = e >> 1, tap = fh * 3 + fw;
-        const bool dv = e & 1;
-        const int ih = oh * S - 1 + fh, iw = ow * S - 1 + fw;
-        if (!live) continue;
-        float d = 0.f;
-        if (ih >= 0 && ih < g.H && iw >= 0 && iw < g.W) {
-          const float r_h = ld<float>(rot + o0 + (size_t)(2 * tap) * g.P), r_w = ld<float>(rot + o0 + (size_t)(2 * tap + 1) * g.P);
-          d = derivative(cells + fw * 128 + p, r_h, r_w, fh, fw, dv, g);
-          if (!(fabsf(d) < INFINITY)) {
-            float alone[16 * 8];
-            cells_alone<T>(alone, dy + (size_t)tp.n * g.C * g.P + oh * g.Wo + ow, x + (size_t)tp.n * g.C * g.HW + ih * g.W + iw, w, g);
-            d = derivative(alone, r_h, r_w, fh, fw, dv, g);
-          }
+      if (part < 3 && live) {
+        const int fw = part, tap = fh * 3 + fw, ih = oh * S - 1 + fh, iw = ow * S - 1 + fw;
+        const size_t o = o0 + (size_t)(2 * tap) * g.P;
+        float2 d = make_float2(0.f, 0.f);
+        Cells at;
+        if (ih >= 0 && ih < g.H && iw >= 0 && iw < g.W && cells_at(at, ld<float>(rot + o), ld<float>(rot + o + g.P), fh, fw, g)) {
+          const float* G4 = cells + fw * 128 + p;
+          float c[4];
+#pragma unroll
+          for (int k = 0; k < 4; ++k) c[k] = cell_in(at, k, g) ? G4[((at.a + (k >> 1)) * 4 + at.b + (k & 1)) * 8] : 0.f;
+          d = derivatives(at, c);
+          if (!(fabsf(d.x) < INFINITY && fabsf(d.y) < INFINITY))
+            d = cells_alone<T>(at, G4, dy + (size_t)tp.n * g.C * g.P + oh * g.Wo + ow, x + (size_t)tp.n * g.C * g.HW + ih * g.W + iw, w, g);
         }
-        st<T, float>(drot + o0 + (size_t)(2 * tap + dv) * g.P, d);
+        st<T, float>(drot + o, d.x);
+        st<T, float>(drot + o + g.P, d.y);
       }
     }
   }
-  bool finite = true;
-  __syncthreads();
-  for (int i = threadIdx.x; i < g.C * g.cells; i += 32 * kWarps) finite &= fabsf(__ldcg(mine + i)) < INFINITY;
-  if (__syncthreads_or(!finite)) {  // one product to the four cells it belongs to, the whole run of the block again
-    float* sums = reinterpret_cast<float*>(smem);
-    for (int c0 = 0; c0 < g.C; c0 += 32) {
-      __syncthreads();
-      bank_by_cells<T>(sums, dy, x, nullptr, rot, g, t, c0, warp, kWarps, lane);
-      __syncthreads();
-      for (int i = threadIdx.x; i < 512; i += 32 * kWarps) {
-        const int cell = i >> 5, a = cell >> 2, b = cell & 3, c = c0 + (i & 31);
-        if (c >= g.C || a >= g.scH || b >= g.scW) continue;
-        float s = 0.f;
-        for (int k = 0; k < kWarps; ++k) s += sums[k * 512 + i];
-        mine[(size_t)c * g.cells + a * g.scW + b] = s;
-      }
+  // one product to the four cells it belongs to, the whole run of the block again, for 32 channels with a sum that is not finite
+  float* sums = reinterpret_cast<float*>(smem);
+  for (int c0 = 0; c0 < g.C; c0 += 32) {
+    bool finite = true;
+    __syncthreads();
+    for (int i = threadIdx.x; i < min(32, g.C - c0) * g.cells; i += 32 * kWarps) finite &= fabsf(__ldcg(mine + c0 * g.cells + i)) < INFINITY;
+    if (!__syncthreads_or(!finite)) continue;
+    bank_by_cells<T>(sums, dy, x, nullptr, rot, g, t, c0, warp, kWarps, lane);
+    __syncthreads();
+    for (int i = threadIdx.x; i < 512; i += 32 * kWarps) {
+      const int cell = i >> 5, a = cell >> 2, b = cell & 3, c = c0 + (i & 31);
+      if (c >= g.C || a >= g.scH || b >= g.scW) continue;
+      float s = 0.f;
+      for (int k = 0; k < kWarps; ++k) s += sums[k * 512 + i];
+      mine[(size_t)c * g.cells + a * g.scW + b] = s;
     }
   }
 }

@@ -82,3 +82,31 @@ def test_no_less_exact_than_each_gradient_alone(n, c, h, w, stride):
         leaf.requires_grad_(False)
         error = [float((g.double().cpu() - want[i]).norm()) for g in (both[i], alone)]
         assert error[0] < 1.01 * error[1], "%s %.3e %.3e" % (name, *error)  # a 2-norm over 2e4 elements and more: 1 % is its own scatter
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.float16])
+@pytest.mark.parametrize("value", [float("inf"), -float("inf"), float("nan")])
+@pytest.mark.parametrize("where", ["weight", "grad_output", "input", "both"])
+def test_where_the_offset_gradients_are_not_finite(where, value, dtype):
+    """Exactly where the oracle's are not: a value of the bank reaches the samples of its cell, one of dy or x those of its pixel."""
+    case = make_case(16, 40, 20, 24, rot_std=0.8, seed=6)
+    if where in ("weight", "both"):
+        case["weight"][11, 0, 1, 2] = case["weight"][39, 0, 3, 0] = value
+    if where in ("grad_output", "both"):
+        case["grad_output"][3, 17, 9, 11] = case["grad_output"][7, 2, 19, 23] = value
+    if where in ("input", "both"):
+        case["input"][2, 5, 0, 7] = case["input"][15, 39, 13, 23] = value
+    (got, dw), (want, dw_want) = _run(case, dtype), _want(case, dtype)
+    finite = torch.isfinite(want)
+    assert (~finite).any() and finite.any()
+    assert torch.equal(torch.isfinite(got).cpu(), finite)
+    assert rel_err(got.cpu()[finite], want[finite].to(dtype)) < (1e-5 if dtype == torch.float32 else 2e-3)
+    assert torch.isfinite(dw).cpu()[torch.isfinite(dw_want)].all()
+
+
+def test_an_infinite_bank_value_gives_infinities():
+    """Its sign and that of dy * x decide, as with a multiply-add per term: not the NaN of the pieces of infinity."""
+    case = make_case(16, 40, 20, 24, rot_std=0.8, seed=6)
+    case["weight"][11, 0, 1, 2] = float("inf")
+    got, want = _run(case, torch.float32)[0].double().cpu(), _want(case, torch.float32)[0]
+    assert torch.isinf(want).any() and torch.equal(got[torch.isinf(want)], want[torch.isinf(want)])
