@@ -212,8 +212,9 @@ __global__ void __launch_bounds__(448, 2) mma_conv_kernel(const __half* __restri
 // ------------------------------------------------------------------ the same in fp32 arithmetic, any number of channels
 // fp16 with channels that are no multiple of 16 has always been computed with fp32 kernel values: the hat products are two fp16 pieces (the
 // second the rest of the first), the bank is exact, so two mma with fp32 sums give K, which then meets the widened x.  The pieces are those of
-// 2^15 times the product, so that 2^-23 of a product is left out and not 2^-25 of one: small ones keep their bits.  Columns beside the image are zeros and not products with a zero kernel value, and a block whose bank holds a value that
-// is not finite computes every output by itself: such values stay with the samples that touch them.
+// 2^15 times the product, so that 2^-23 of a product is left out and not 2^-25 of one: small ones keep their bits.  Columns beside the image are zeros and not products with a zero kernel value, and a channel
+// whose bank holds a value that is not finite is computed again output by output: such values stay with the samples that touch them (forward with one
+// such value, all channels of a block by themselves -> that one, us: 8 x 72 of 75 x 101 740 -> 79, 64 x 88 of 28 x 30 493 -> 55).
 // Against gathered cells (local_conv_kernel: four reads and five multiply-adds per channel and tap), us, forward + grad-input: 8 x 72 of
 // 75 x 101 189 -> 133, 64 x 88 of 28 x 30 195 -> 55, 40 x 72 of 56 x 50 at stride 2 191 -> 53, 128 x 200 of 7 x 7 67 -> 30, 64 x 24 of 112 x 110
 // 790 -> 278, 64 x 8 of 56 x 54 at stride 2 54 -> 47, 1 x 72 of 28 x 30 21 -> 15.  Rows of odd width wait for their loader (8 x 72 of 75 x 101 115
@@ -278,15 +279,7 @@ __global__ void __launch_bounds__(256, 2) mma_conv_full_kernel(const __half* __r
   load_band(rband, br, rot, n, 18, 0, 18, g.Ho, g.Wo);
   cp_async_wait_all();
   const size_t dplane = (size_t)Hd * Wd;
-  if (__syncthreads_or(!finite)) {
-    const int rows = min(pl.BH, Hd - d_row0);
-    for (int i = threadIdx.x; i < cnt * rows * Wd; i += blockDim.x) {
-      const int c = c0 + i / (rows * Wd), r = i % (rows * Wd);
-      dst[((size_t)n * g.C + c) * dplane + (size_t)d_row0 * Wd + r] =
-          __float2half_rn(conv_alone<S, TRANSPOSED>(src, rot, w, g, n, c, d_row0 + r / Wd, r % Wd));
-    }
-    return;
-  }
+  const bool alone = __syncthreads_or(!finite);
 
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nwarps = blockDim.x >> 5;
   const int gq = lane >> 2, q = lane & 3;
@@ -398,6 +391,18 @@ __global__ void __launch_bounds__(256, 2) mma_conv_full_kernel(const __half* __r
           }
         }
       }
+    }
+  }
+  if (alone) {
+    __syncthreads();  // these stores come after the ones above
+    const int rows = min(pl.BH, Hd - d_row0);
+    for (int j = 0; j < cnt; ++j) {
+      bool ok = true;
+      for (int cell = 0; cell < g.cells; ++cell) ok &= fabsf(__half2float(bank[j * kBankPitch + cell])) < INFINITY;
+      if (ok) continue;
+      for (int i = threadIdx.x; i < rows * Wd; i += blockDim.x)
+        dst[((size_t)n * g.C + c0 + j) * dplane + (size_t)d_row0 * Wd + i] =
+            __float2half_rn(conv_alone<S, TRANSPOSED>(src, rot, w, g, n, c0 + j, d_row0 + i / Wd, i % Wd));
     }
   }
 }
