@@ -451,7 +451,7 @@ __global__ void __launch_bounds__(32 * kWarps, 1) pieces_gradients_kernel(const 
   }
 }
 
-TilePlan search_plan(const Geom& g) {
+TilePlan search_plan(const Geom& g, int sms) {
   TilePlan t;
   const int most = g.sH == 1 ? Room<1>::X : Room<2>::X;
   long long best = -1;
@@ -473,8 +473,7 @@ TilePlan search_plan(const Geom& g) {
   t.magic_x = (unsigned)((0x100000000ull + t.XW - 1) / t.XW);
   t.magic_y = t.TW == 1 ? 0 : (unsigned)((0x100000000ull + t.TW - 1) / t.TW);
   t.smem = g.sH == 1 ? Room<1>::kBytes : Room<2>::kBytes;
-  const int want = 1 * device_sm_count();
-  t.per_block = (t.tiles + want - 1) / want;
+  t.per_block = (t.tiles + sms - 1) / sms;
   t.blocks = (t.tiles + t.per_block - 1) / t.per_block;
   return t;
 }
@@ -482,11 +481,13 @@ TilePlan search_plan(const Geom& g) {
 // A call asks for its plan several times (is it taken, scratch, launch); a search takes some microseconds, so a thread keeps its last one.
 const TilePlan& gradients_plan(const Geom& g) {
   struct Last {
-    int n = 0, h = 0, w = 0, s = 0;
+    int n = 0, h = 0, w = 0, s = 0, sms = 0;
     TilePlan t;
   };
   static thread_local Last last;
-  if (last.n != g.N || last.h != g.H || last.w != g.W || last.s != g.sH) last.t = search_plan(g), last.n = g.N, last.h = g.H, last.w = g.W, last.s = g.sH;
+  const int sms = device_sm_count();  // of the thread's current device
+  if (last.n != g.N || last.h != g.H || last.w != g.W || last.s != g.sH || last.sms != sms)
+    last.t = search_plan(g, sms), last.n = g.N, last.h = g.H, last.w = g.W, last.s = g.sH, last.sms = sms;
   return last.t;
 }
 
