@@ -167,11 +167,12 @@ int device_smem_optin();  // max dynamic shared memory per block (opt-in), cache
 int device_sm_count();
 
 // Raises the kernel's dynamic shared-memory limit on the current device to `bytes`.  The driver is asked once per (kernel,
-// device, larger size): the call costs about as much host time as the launch itself.
+// device, larger size): the call costs about as much host time as the launch itself.  Below 48 KB too: what a launch may have without being
+// asked for is 48 KB less the kernel's static arrays.
 int raise_smem_limit(const void* kernel, size_t bytes);
 template <typename K>
 inline int enable_smem(K kernel, size_t bytes) {
-  return bytes > 48 * 1024 ? raise_smem_limit(reinterpret_cast<const void*>(kernel), bytes) : DK_OK;
+  return bytes > 0 ? raise_smem_limit(reinterpret_cast<const void*>(kernel), bytes) : DK_OK;
 }
 
 // typed launchers implemented in dk_local.cu / dk_deform.cu / dk_nd.cu

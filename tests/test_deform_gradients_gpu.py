@@ -38,6 +38,22 @@ def test_gradients(n, c, h, w, stride, pad, dil, scope, dtype):
         assert rel_err(g, w.to(dtype)) < tol
 
 
+@pytest.mark.parametrize("h,w", [(105, 112), (127, 95)])
+@pytest.mark.parametrize("dtype", [torch.float32, torch.float16])
+def test_planes_whose_cells_take_almost_48_kilobytes(h, w, dtype):
+    """The sort's counters and its static arrays together take more shared memory than a launch has without asking."""
+    from deformable_kernels.ops.deform_kernel.functions import deform_sample_depthwise
+    from oracle import dk_oracle as O
+    case = make_case(1, 24, h, w, scope=(4, 4), rot_std=0.5, off_std=2.0, seed=h)
+    names = ("grad_output", "input", "offset", "rotation", "weight")
+    want = O.deform_sample_depthwise_backward(*(case[k].to(dtype).float() for k in names), **case["args"])
+    dy, *leaves = (case[k].to(dtype).to(DEV) for k in names)
+    leaves = [t.requires_grad_(True) for t in leaves]
+    got = torch.autograd.grad(deform_sample_depthwise(*leaves, **case["args"]), leaves, dy)
+    for g, v in zip(got, want):
+        assert rel_err(g, v.to(dtype)) < (1e-5 if dtype == torch.float32 else 2e-3)
+
+
 @pytest.mark.parametrize("dtype", [torch.float32, torch.float16])
 def test_subsets_of_the_gradients_agree(dtype):
     from deformable_kernels.ops.deform_kernel.functions import deform_sample_depthwise
