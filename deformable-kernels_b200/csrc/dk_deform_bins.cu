@@ -12,6 +12,8 @@
 // warps on 148 SMs for 16 x 192 of 28 x 28; the sort by the latency of its five steps.
 #include <cooperative_groups.h>
 
+#include <type_traits>
+
 #include "dk_common.cuh"
 
 namespace dk {
@@ -39,7 +41,8 @@ __host__ __device__ inline int bank_cells(const Geom& g) { return bank_unused_ce
 // Without kernel-space offsets (rot null) the sampled kernel is the same at every pixel: in place of the bank its value per (tap,
 // channel) is laid out, and one read stands for four and their multiply-adds; the bank gradient meets the cells once per tap.  16 x 192
 // of 28 x 28, 3 x 3 scope: forward 39 -> 25 us, gather 53 -> 44, offsets 43 -> 31, bank 42 -> 33; 13 x 88 of 80 x 80 in fp16, all, 848 -> 646.
-// The unused cell keeps its zeros; samples that are not used select zero in place of their tap's value, which may not be finite.
+// The unused cell keeps its zeros; samples that are not used meet their tap's value with zeros, and where that leaves sums that are not finite
+// they are formed again with zero selected in its place.
 __host__ __device__ inline bool fixed_kernel(const Geom& g, const void* rot) { return rot == nullptr && g.taps <= bank_unused_cell(g); }
 
 // one sample point: corner coefficients of the image and of the bank, {bank cell * 32, column of the cell, pixel * Cp, 0}
@@ -431,32 +434,49 @@ __global__ void __launch_bounds__(32 * kRowWarps, 3) dcn_forward_kernel(const T*
 #pragma unroll 1
     for (int j = warp * 4; j < warp * 4 + 4; j += 2) {
       float acc[2][V] = {};
+      auto taps = [&](auto select) {
 #pragma unroll 1
-      for (int tap = 0; tap < g.taps; ++tap) {
-        float x[2][4][V], k[2][4][V];
+        for (int tap = 0; tap < g.taps; ++tap) {
+          float x[2][4][V], k[2][4][V];
 #pragma unroll
-        for (int h = 0; h < 2; ++h) {
-          const TapRec& r = recs[tap][j + h];
-          const int4 idx = r.idx;
-          const unsigned bk = r.at.y + ck;
-          get_at<T, V>(xt, idx.x + cb, x[h][0]), get_at<T, V>(xt, idx.y + cb, x[h][1]), get_at<T, V>(xt, idx.z + cb, x[h][2]), get_at<T, V>(xt, idx.w + cb, x[h][3]);
-          if (FIXED) {
-            if (h == 0) get_at<float, V>(bankt, tap * cell + ck, k[0][0]);
-          } else {
-            get_at<float, V>(bankt, bk, k[h][0]), get_at<float, V>(bankt, bk + cell, k[h][1]);
-            get_at<float, V>(bankt, bk + row, k[h][2]), get_at<float, V>(bankt, bk + row + cell, k[h][3]);
+          for (int h = 0; h < 2; ++h) {
+            const TapRec& r = recs[tap][j + h];
+            const int4 idx = r.idx;
+            const unsigned bk = r.at.y + ck;
+            get_at<T, V>(xt, idx.x + cb, x[h][0]), get_at<T, V>(xt, idx.y + cb, x[h][1]), get_at<T, V>(xt, idx.z + cb, x[h][2]), get_at<T, V>(xt, idx.w + cb, x[h][3]);
+            if (FIXED) {
+              if (h == 0) get_at<float, V>(bankt, tap * cell + ck, k[0][0]);
+            } else {
+              get_at<float, V>(bankt, bk, k[h][0]), get_at<float, V>(bankt, bk + cell, k[h][1]);
+              get_at<float, V>(bankt, bk + row, k[h][2]), get_at<float, V>(bankt, bk + row + cell, k[h][3]);
+            }
+          }
+#pragma unroll
+          for (int h = 0; h < 2; ++h) {
+            const float4 im = recs[tap][j + h].im, b = recs[tap][j + h].a;
+            const bool used = !decltype(select)::value || im.x + im.y > 0.f;  // the two are 1 - lh and lh, or zeros
+#pragma unroll
+            for (int e = 0; e < V; ++e) {
+              const float xs = im.x * (im.z * x[h][0][e] + im.w * x[h][1][e]) + im.y * (im.z * x[h][2][e] + im.w * x[h][3][e]);
+              if (FIXED) acc[h][e] += xs * (used ? k[0][0][e] : 0.f);
+              else acc[h][e] += xs * (b.x * (b.z * k[h][0][e] + b.w * k[h][1][e]) + b.y * (b.z * k[h][2][e] + b.w * k[h][3][e]));
+            }
           }
         }
+      };
+      taps(std::false_type());
+      if constexpr (FIXED) {
+        bool finite = true;
 #pragma unroll
-        for (int h = 0; h < 2; ++h) {
-          const float4 im = recs[tap][j + h].im, b = recs[tap][j + h].a;
-          const bool used = im.x + im.y > 0.f;  // the two are 1 - lh and lh, or zeros
+        for (int h = 0; h < 2; ++h)
 #pragma unroll
-          for (int e = 0; e < V; ++e) {
-            const float xs = im.x * (im.z * x[h][0][e] + im.w * x[h][1][e]) + im.y * (im.z * x[h][2][e] + im.w * x[h][3][e]);
-            if (FIXED) acc[h][e] += xs * (used ? k[0][0][e] : 0.f);
-            else acc[h][e] += xs * (b.x * (b.z * k[h][0][e] + b.w * k[h][1][e]) + b.y * (b.z * k[h][2][e] + b.w * k[h][3][e]));
-          }
+          for (int e = 0; e < V; ++e) finite &= fabsf(acc[h][e]) < INFINITY;
+        if (!finite) {
+#pragma unroll
+          for (int h = 0; h < 2; ++h)
+#pragma unroll
+            for (int e = 0; e < V; ++e) acc[h][e] = 0.f;
+          taps(std::true_type());
         }
       }
 #pragma unroll
@@ -490,43 +510,50 @@ __global__ void __launch_bounds__(32 * kRowWarps, 3) dcn_coords_kernel(const T* 
   const unsigned cell = Cp * sizeof(float), row = (g.scW + 2) * cell;
   for (int j = 0; j < cnt; j += 2) {
     float s[2][4] = {};
+    auto channels = [&](auto select) {
 #pragma unroll 1
-    for (int c = (share * 32 + lane) * V; c < Cp; c += S * 32 * V) {
-      const unsigned cb = c * (unsigned)sizeof(T);
-      float x[2][4][V], k[2][4][V], y[2][V];
+      for (int c = (share * 32 + lane) * V; c < Cp; c += S * 32 * V) {
+        const unsigned cb = c * (unsigned)sizeof(T);
+        float x[2][4][V], k[2][4][V], y[2][V];
 #pragma unroll
-      for (int h = 0; h < 2; ++h) {
-        const TapRec& r = recs[warp][j + h];
-        const int4 idx = r.idx;
-        const int2 at = *reinterpret_cast<const int2*>(&r.at);
-        get_at<T, V>(xt, idx.x + cb, x[h][0]), get_at<T, V>(xt, idx.y + cb, x[h][1]), get_at<T, V>(xt, idx.z + cb, x[h][2]), get_at<T, V>(xt, idx.w + cb, x[h][3]);
-        get_at<T, V>(dyt, at.x + cb, y[h]);
-        const unsigned bk = at.y + c * (unsigned)sizeof(float);
-        if (FIXED) {
-          if (h == 0) get_at<float, V>(bankt, tap * cell + c * (unsigned)sizeof(float), k[0][0]);
-        } else {
-          get_at<float, V>(bankt, bk, k[h][0]), get_at<float, V>(bankt, bk + cell, k[h][1]);
-          get_at<float, V>(bankt, bk + row, k[h][2]), get_at<float, V>(bankt, bk + row + cell, k[h][3]);
+        for (int h = 0; h < 2; ++h) {
+          const TapRec& r = recs[warp][j + h];
+          const int4 idx = r.idx;
+          const int2 at = *reinterpret_cast<const int2*>(&r.at);
+          get_at<T, V>(xt, idx.x + cb, x[h][0]), get_at<T, V>(xt, idx.y + cb, x[h][1]), get_at<T, V>(xt, idx.z + cb, x[h][2]), get_at<T, V>(xt, idx.w + cb, x[h][3]);
+          get_at<T, V>(dyt, at.x + cb, y[h]);
+          const unsigned bk = at.y + c * (unsigned)sizeof(float);
+          if (FIXED) {
+            if (h == 0) get_at<float, V>(bankt, tap * cell + c * (unsigned)sizeof(float), k[0][0]);
+          } else {
+            get_at<float, V>(bankt, bk, k[h][0]), get_at<float, V>(bankt, bk + cell, k[h][1]);
+            get_at<float, V>(bankt, bk + row, k[h][2]), get_at<float, V>(bankt, bk + row + cell, k[h][3]);
+          }
         }
-      }
 #pragma unroll
-      for (int h = 0; h < 2; ++h) {
-        const float4 im = recs[warp][j + h].im, b = recs[warp][j + h].a;
-        const bool used = im.x + im.y > 0.f;
+        for (int h = 0; h < 2; ++h) {
+          const float4 im = recs[warp][j + h].im, b = recs[warp][j + h].a;
+          const bool used = !decltype(select)::value || im.x + im.y > 0.f;
 #pragma unroll
-        for (int e = 0; e < V; ++e) {
-          const float top = im.z * x[h][0][e] + im.w * x[h][1][e], low = im.z * x[h][2][e] + im.w * x[h][3][e];
-          const float ktop = FIXED ? 0.f : b.z * k[h][0][e] + b.w * k[h][1][e], klow = FIXED ? 0.f : b.z * k[h][2][e] + b.w * k[h][3][e];
-          const float yk = y[h][e] * (FIXED ? (used ? k[0][0][e] : 0.f) : b.x * ktop + b.y * klow);
-          s[h][0] += yk * (low - top);
-          s[h][1] += yk * (im.x * (x[h][1][e] - x[h][0][e]) + im.y * (x[h][3][e] - x[h][2][e]));
-          if (ROT) {
-            const float yx = y[h][e] * (im.x * top + im.y * low);
-            s[h][2] += yx * (klow - ktop);
-            s[h][3] += yx * (b.x * (k[h][1][e] - k[h][0][e]) + b.y * (k[h][3][e] - k[h][2][e]));
+          for (int e = 0; e < V; ++e) {
+            const float top = im.z * x[h][0][e] + im.w * x[h][1][e], low = im.z * x[h][2][e] + im.w * x[h][3][e];
+            const float ktop = FIXED ? 0.f : b.z * k[h][0][e] + b.w * k[h][1][e], klow = FIXED ? 0.f : b.z * k[h][2][e] + b.w * k[h][3][e];
+            const float yk = y[h][e] * (FIXED ? (used ? k[0][0][e] : 0.f) : b.x * ktop + b.y * klow);
+            s[h][0] += yk * (low - top);
+            s[h][1] += yk * (im.x * (x[h][1][e] - x[h][0][e]) + im.y * (x[h][3][e] - x[h][2][e]));
+            if (ROT) {
+              const float yx = y[h][e] * (im.x * top + im.y * low);
+              s[h][2] += yx * (klow - ktop);
+              s[h][3] += yx * (b.x * (k[h][1][e] - k[h][0][e]) + b.y * (k[h][3][e] - k[h][2][e]));
+            }
           }
         }
       }
+    };
+    channels(std::false_type());
+    if (FIXED && !(fabsf(s[0][0]) < INFINITY && fabsf(s[0][1]) < INFINITY && fabsf(s[1][0]) < INFINITY && fabsf(s[1][1]) < INFINITY)) {
+      s[0][0] = s[0][1] = s[1][0] = s[1][1] = 0.f;
+      channels(std::true_type());
     }
 #pragma unroll
     for (int h = 0; h < 2; ++h) {

@@ -38,9 +38,9 @@ def test_gradients(n, c, h, w, stride, pad, dil, scope, dtype):
         assert rel_err(g, w.to(dtype)) < tol
 
 
-@pytest.mark.parametrize("h,w", [(105, 112), (127, 95)])
+@pytest.mark.parametrize("h,w", [(90, 91), (105, 112), (127, 95)])
 @pytest.mark.parametrize("dtype", [torch.float32, torch.float16])
-def test_planes_whose_cells_take_almost_48_kilobytes(h, w, dtype):
+def test_planes_whose_cells_take_32_to_48_kilobytes(h, w, dtype):
     """The sort's counters and its static arrays together take more shared memory than a launch has without asking."""
     from deformable_kernels.ops.deform_kernel.functions import deform_sample_depthwise
     from oracle import dk_oracle as O
