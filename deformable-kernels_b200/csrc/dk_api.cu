@@ -381,9 +381,11 @@ int dk_deform_sample_depthwise_forward_ws(const void* input, const void* offset,
   if (!input || !offset || !filter || !output || !make_geom(g, &gg)) return DK_ERR_BAD_ARGUMENT;
   const size_t need = dk_deform_sample_depthwise_forward_workspace_bytes(g, dtype);
   const bool lines = deform_lines_takes_forward(gg, dtype, rotation != nullptr);
-  if (lines && workspace && workspace_bytes >= deform_lines_forward_workspace(gg))
-    return deform_lines_forward(P_(__half, input), P_(__half, offset), P_(__half, rotation), P_(__half, filter), M_(__half, output),
-                                gg, workspace, workspace_bytes, (cudaStream_t)stream);
+  if (lines) {
+    const int rc = deform_lines_forward(P_(__half, input), P_(__half, offset), P_(__half, rotation), P_(__half, filter), M_(__half, output),
+                                        gg, workspace, workspace_bytes, (cudaStream_t)stream);
+    if (rc != DK_ERR_UNSUPPORTED) return rc;
+  }
   if (lines || need == 0 || !deform_rows_forward(gg, dtype, rotation != nullptr))
     return dk_deform_sample_depthwise_forward(input, offset, rotation, filter, output, g, dtype, stream);
   if (!workspace || workspace_bytes < need) return DK_ERR_WORKSPACE;

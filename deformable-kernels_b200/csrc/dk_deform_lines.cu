@@ -1145,6 +1145,9 @@ void line_plan(const Geom& g, LinePlan& p) {
   p.bytes = p.xt + p.dyt + p.starts + p.recs + p.sums + p.bank;
 }
 
+// lines are read and written 16 bytes at a time; the kernels without them take scratch at any word
+bool lines_fit(const void* ws) { return (reinterpret_cast<uintptr_t>(ws) & 15) == 0; }
+
 int to_lines(const __half* x, __half* xt, const __half* dy, __half* dyt, const LineGeom& lg, cudaStream_t s) {
   const Geom& g = lg.g;
   auto job = [&](const __half* src, __half* dst, int P) { return LineJob{src, dst, P, (P & 7) == 0 && ptr_mode(src) == 2}; };
@@ -1170,7 +1173,7 @@ int deform_lines_forward(const __half* x, const __half* off, const __half* rot, 
   if (!lines_shape(g)) return DK_ERR_UNSUPPORTED;
   LinePlan p;
   line_plan(g, p);
-  if (ws == nullptr || ws_bytes < p.xt) return DK_ERR_WORKSPACE;
+  if (ws == nullptr || ws_bytes < p.xt || !lines_fit(ws)) return DK_ERR_UNSUPPORTED;
   __half* xt = reinterpret_cast<__half*>(ws);
   if (int rc = to_lines(x, xt, nullptr, nullptr, p.lg, s)) return rc;
   const int units = p.lg.units, tiles = (int)(((long long)g.N * g.P + kFwdPixels - 1) / kFwdPixels);
@@ -1196,7 +1199,7 @@ int deform_lines_backward(const __half* dy, const __half* x, const __half* off, 
   if (!lines_shape(g)) return DK_ERR_UNSUPPORTED;
   LinePlan p;
   line_plan(g, p);
-  if (p.sort_smem > 200 * 1024 || ws == nullptr || ws_bytes < p.bytes) return DK_ERR_UNSUPPORTED;
+  if (p.sort_smem > 200 * 1024 || ws == nullptr || ws_bytes < p.bytes || !lines_fit(ws)) return DK_ERR_UNSUPPORTED;
   const bool coords = doff || drot || dw;
   char* at = reinterpret_cast<char*>(ws);
   auto take = [&](size_t bytes) {

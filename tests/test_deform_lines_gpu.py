@@ -189,3 +189,19 @@ def test_operands_at_any_address(n, c, h, w, stride, halves):
             assert torch.equal(first, other)
         else:  # the kernels of few samples add in the order of the day: two roundings to fp16
             assert rel_err(first, other) < 1e-3
+
+
+def test_scratch_at_any_word():
+    """Lines want 16 bytes; scratch that begins between them is left to the kernels that take it."""
+    from deformable_kernels import _cabi as C
+    case = make_case(24, 64, 24, 40, scope=(4, 4), rot_std=0.7, off_std=2.0, seed=14)
+    dy, x, o, r, w = (case[k].to(torch.float16).cuda() for k in ("grad_output", "input", "offset", "rotation", "weight"))
+    g = C.geom(tuple(x.shape), (3, 3), (1, 1), (1, 1), (1, 1), (4, 4), 1)
+    size = max(C.lib.dk_deform_sample_depthwise_forward_workspace_bytes(g, C.DK_F16), C.lib.dk_deform_sample_depthwise_backward_workspace_bytes(g, C.DK_F16))
+    s, want = C.stream_ptr(x.device), _want(case)
+    ws = torch.empty(size // 4 + 4, dtype=torch.float32, device="cuda")[1:]
+    got = [torch.empty_like(t) for t in (x, x, o, r, w)]
+    assert C.lib.dk_deform_sample_depthwise_forward_ws(*(C.ptr(t) for t in (x, o, r, w, got[0])), g, C.DK_F16, C.ptr(ws), size, s) == 0
+    assert C.lib.dk_deform_sample_depthwise_backward(*(C.ptr(t) for t in (dy, x, o, r, w, *got[1:])), g, C.DK_F16, C.ptr(ws), size, s) == 0
+    for k, v in zip(("output",) + NAMES, got):
+        assert rel_err(v, want[k].half()) < 2e-3, k
