@@ -10,13 +10,15 @@
 // 32 (g & 1) + 8 t .. + 7 of the pixels 4 (g >> 1) + i, i = 0 .. 3, of a group of 16.  The products with the hat functions come
 // out of mma.sync in that layout: the rows 2 q and 2 q + 1 are the same pixel, the even rows count for the lower 32 channels and the odd
 // rows for the upper ones (two mma, one with the bank of each half, and a lane keeps the result of its rows: zeroed rows instead would let a
-// bank value that is not finite reach the channel 32 away), and the columns 2 t, 2 t + 1 of tile j are the channels 8 t + 2 j, + 1.  mma.sync, because its results are needed in registers beside the gathered values.
+// bank value that is not finite reach the channel 32 away), and the columns 2 t, 2 t + 1 of tile j are the channels 8 t + 2 j, + 1.  mma.sync,
+// because its results are needed in registers beside the gathered values.
 //
-// 64 x 256 of 56 x 56, forward and backward 3384 -> 1294 us: lines 51 each way, forward 296, sort 54, gather 285, offsets and bank
-// 543.  Forward: load pipe 60 % (64 of its 109 passes per 16 pixels, tap and 64 channels are the corners, 44 % of the
+// 64 x 256 of 56 x 56, forward and backward 3384 -> 1342 us: lines 35 and 65, forward 300, sort 56, gather 290, offsets and bank
+// 590.  Forward: load pipe 69 % (64 of its 109 passes per 16 pixels, tap and 64 channels are the corners, 44 % of the
 // rest misses and offsets), 2.8 warps per scheduler at 168 registers; 8 loads in flight instead of 16 with 16 warps instead of
-// 12 takes as long.  Offsets and bank: load pipe 48 %, half-rate fp16 pipe 37 %, tensor pipe 33 %, issue 42 %: latency at ten warps, which
-// the 64 registers of bank sums and bank operands leave.  Gather: load pipe 55 %, tensor 33 %, issue 48 %.
+// 12 takes as long.  Offsets and bank: load pipe 46 %, tensor pipe 33 %, issue 44 %, the half-rate fp16 pipe with 14 instructions where the tensor
+// pipe has 10: latency at twelve warps of an SM in three blocks, which the 64 registers of bank sums and bank operands leave.  Gather: load pipe
+// 60 %, tensor 37 %, issue 52 %.
 #include <cooperative_groups.h>
 
 #include "dk_mma_common.cuh"
@@ -454,7 +456,8 @@ __global__ void __launch_bounds__(128, 3) line_forward_kernel(const __half* __re
 // with the derivatives of the hats.  d(image offset) = sum_c dy K dxs/d(h|w): from the four sums S_k = sum_c (dy K) dx_k over
 // the differences of neighbouring corners, an mma of the products whose other operand is one in the columns k, k + 4; a pixel's two rows are its two
 // halves of the channels.  Products with the corners themselves, subtracted afterwards, overflow where only the corners are large (x of 100, dy
-// of 500) and lose what they have in common: 8 x 512 of 28 x 28 with x around 10, 1.1e-3 off fp64 against 4.5e-4 (4.6e-4 and 5.1e-4 around 0).  dW = beta^T (dy xs) over the pixels, for which movmatrix turns the products.
+// of 500) and lose what they have in common: 8 x 512 of 28 x 28 with x around 10, 1.1e-3 off fp64 against 4.5e-4 (4.6e-4 and 5.1e-4 around 0).
+// 543 -> 590 us for the differences.  dW = beta^T (dy xs) over the pixels, for which movmatrix turns the products.
 // A warp has 64 channels for the whole run of its block (the bank sums stay in registers) and walks over groups of 16 pixels;
 // the warps of a stream have different channels of the same pixels, and their sums over channels meet in shared memory.
 struct CoordPlan {

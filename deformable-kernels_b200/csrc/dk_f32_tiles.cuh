@@ -12,7 +12,7 @@ struct TilePlan {
   int across, down;           // tiles per row of tiles, per sample
   int tiles;                  // over the batch
   int XH, XW;                 // source rows and columns of a tile
-  int xpitch, ypitch;         // words per channel in shared memory, odd
+  int xpitch, ypitch;         // words per channel in shared memory
   unsigned magic_x, magic_y;  // ceil(2^32 / XW), ceil(2^32 / TW)
   int per_block, blocks;      // tiles per block, blocks (bank)
   size_t smem;

@@ -16,8 +16,8 @@
 // in registers as it was loaded or made; two pieces of one step beside each other need copies of one of them and take 629 us below.  A step left
 // over takes them that way for the offsets (64 x 24 of 112 x 110: 674 us beside a step of zeros, 617 so, 637 in separate kernels).
 //
-// fp32 64 x 144 of 56 x 56: 753 us in two kernels that gather or hold the cells with one fp32 multiply-add each -> 558.  Tensor pipe 42 %,
-// issue 40 %: products, the pieces that feed them and the additions behind them follow each other in a warp, and 3 warps per scheduler (168 registers)
+// fp32 64 x 144 of 56 x 56: 753 us in two kernels that gather or hold the cells with one fp32 multiply-add each -> 558.  Tensor pipe 40 %,
+// issue 37 %: products, the pieces that feed them and the additions behind them follow each other in a warp, and 3 warps per scheduler (168 registers)
 // overlap part of it; tiles that do not fill and the tenth tap of the pairs are 15 % of the products.
 #include <type_traits>
 

@@ -51,7 +51,8 @@ typedef enum dk_dtype { DK_F32 = 0, DK_F16 = 1, DK_F64 = 2 } dk_dtype;
  * themselves), multiply it exactly with the fp16 input and sum in fp32;
  * grad-offsets and grad-bank feed the products grad_output * input to the tensor cores as fp16, so
  * |grad_output * input| must stay below 65504 (an overflow gives Inf / NaN gradients, which a loss scaler's
- * overflow check catches and answers by lowering its scale); all sums are fp32.  fp16 calls with other channel counts form
+ * overflow check catches and answers by lowering its scale); all sums are fp32.  DK + DCN feeds them |grad_output * kernel value *
+ * (difference of neighbouring inputs)| as well, with the same bound.  fp16 calls with other channel counts form
  * kernel values and products in fp32. */
 
 /* Geometry of one depthwise call.  Same fields as the reference's
