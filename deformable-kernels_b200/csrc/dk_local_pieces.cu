@@ -493,16 +493,26 @@ const TilePlan& gradients_plan(const Geom& g) {
 
 }  // namespace
 
-// us, separate kernels (f32_offsets_kernel or local_rot_kernel, f32_bank_kernel) -> this one: fp32 64 x 144 of 56 x 56 758 -> 557, 8 x 64 of
-// 28 x 28 (72 tiles) 24 -> 19, 4 x 64 (36 tiles) 17 -> 19, 40 x 40 of 60 x 111 455 -> 289, 128 x 960 of 7 x 7 221 -> 175; stride 2, 40 x 96 of
-// 30 x 41 74 -> 51, 16 x 96 of 28 x 28 (48 tiles) 23 -> 27.  fp16 8 x 72 of 75 x 101 165 -> 118, 6 x 104 of 40 x 44 54 -> 34, 24 x 104 of
-// 28 x 28 77 -> 62, 64 x 200 of 14 x 14 (1.3 tiles per SM) 90 -> 97, 128 x 200 160 -> 150; stride 2, 40 x 72 of 56 x 50 114 -> 121.
+// A block's tiles take the time of their twelve warps whatever part of them is pixels, so planes that leave tiles half empty (4 x 4 outputs: 16
+// of 96 pixels) and one tile too many for a round make this kernel the slower one.  Both sides are estimated in us, from 2000 measured calls of
+// 16 to 968 channels, planes of 7 x 7 to 56 x 56, 1536 to 70 k pixels, inputs in L2 and not: this one within 4 to 8 %, the separate kernels
+// (f32_offsets_kernel or local_rot_kernel, f32_bank_kernel) within 5 to 13 %; of the faster choice 0.5 % are lost in the mean, a quarter at most.  us,
+// separate -> this one, taken: fp32 64 x 144 of 56 x 56 758 -> 557, 8 x 64 of 28 x 28 (72 tiles) 24 -> 19, 40 x 40 of 60 x 111 455 -> 289, 128 x 960
+// of 7 x 7 217 -> 172; stride 2, 40 x 96 of 30 x 41 74 -> 51.  fp16 8 x 72 of 75 x 101 165 -> 118, 6 x 104 of 40 x 44 54 -> 34, 24 x 104 of 28 x 28
+// 77 -> 62.  Not taken: fp32 4 x 64 of 28 x 28 (36 tiles) 17 -> 19; stride 2, 16 x 96 of 28 x 28 (48 tiles) 23 -> 27, 128 x 960 of 7 x 7
+// 132 -> 195, 388 x 192 of 7 x 7 55 -> 127, 317 x 192 of 9 x 12 71 -> 130; fp16 64 x 200 of 14 x 14 (1.3 tiles per SM) 90 -> 97, 153 x 584 of 9 x 12
+// 267 -> 350; stride 2, 40 x 72 of 56 x 50 114 -> 121.
 bool local_gradients_pieces_takes(const Geom& g, size_t elem) {
   if (g.kH != 3 || g.kW != 3 || g.dH != 1 || g.dW != 1 || g.pH != 1 || g.pW != 1 || g.sH != g.sW || (g.sH != 1 && g.sH != 2)) return false;
   if (g.G != 1 || g.scH > 4 || g.scW > 4 || (long long)g.N * g.P >= 0x3fffffff) return false;
   if ((long long)g.N * g.P < 1536) return false;  // few tiles whatever their shape
-  const int tiles = gradients_plan(g).tiles, sms = device_sm_count();
-  return tiles >= 64 && (elem == 4 || (g.sH == 1 && (tiles <= sms || 2 * tiles >= 3 * sms)));
+  const TilePlan& t = gradients_plan(g);
+  const int sms = device_sm_count();
+  if (t.tiles < 64 || (elem == 2 && (g.sH == 2 || (t.tiles > sms && 2 * t.tiles < 3 * sms)))) return false;
+  const double steps = (g.C + 7) / 8, thousands = (double)g.N * g.P / 1000 * 148 / sms;
+  const double here = 4.6 + t.per_block * (3.6 + (elem == 2 ? 1.95 : g.sH == 1 ? 1.5 : 1.7) * steps);
+  const double separate = 14 + 0.08 * g.C + thousands * (0.5 + (elem == 2 ? 0.19 : g.sH == 1 ? 0.195 : 0.22) * steps);
+  return here < separate;
 }
 size_t local_gradients_pieces_workspace(const Geom& g, size_t elem) {
   return local_gradients_pieces_takes(g, elem) ? (size_t)gradients_plan(g).blocks * g.C * g.cells * sizeof(float) : 0;
