@@ -100,8 +100,8 @@ __global__ void __launch_bounds__(448, 2) mma_conv_kernel(const __half* __restri
     const int j = i >> 4, cell = i & 15;
     bank[j * kBankPitch + cell] = cell < g.cells ? __ldg(w + (size_t)(c0 + j) * g.cells + cell) : __float2half(0.f);
   }
-  load_band<S == 2 ? 74 : 96>(band, bx, src, n, g.C, c0, cnt, Hs, Ws);
-  load_band<S == 2 ? 74 : 96>(rband, br, rot, n, 18, 0, 18, g.Ho, g.Wo);
+  load_band<S == 2 ? 74 : 96, S == 1 && !EDGES>(band, bx, src, n, g.C, c0, cnt, Hs, Ws);
+  load_band<S == 2 ? 74 : 96, S == 1 && !EDGES>(rband, br, rot, n, 18, 0, 18, g.Ho, g.Wo);
   cp_async_wait_all();
   __syncthreads();
 

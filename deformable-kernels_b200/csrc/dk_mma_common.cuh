@@ -183,8 +183,8 @@ __device__ __forceinline__ void odd_rows(__half* __restrict__ dst, int pitch, in
     }
   }
 }
-// WORDS: odd widths above it are copied word by word; 0: none
-template <int WORDS>
+// WORDS: odd widths above it are copied word by word (BY_WARP: a warp per row); 0: none
+template <int WORDS, bool BY_WARP>
 __device__ __forceinline__ void load_band_group(__half* __restrict__ band, const Band& b, const __half* __restrict__ src, int n,
                                                 int C, int c0, int cnt, int Hs, int Ws, int tid, int nt, int bar_id) {
   const int lane = tid & 31, warp = tid >> 5, nwarps = nt >> 5;
@@ -206,6 +206,27 @@ __device__ __forceinline__ void load_band_group(__half* __restrict__ band, const
     // 66 / 39, x 79 70 / 41, x 85 86 / 48, x 89 69 / 74, x 95 76 / 70; 24 x 96 of 45 x 83 41 / 31; 8 x 128 of 100 x 73 35 / 49, x 75 33 / 35, x 95
     // 45 / 39 (a warp per row 53, 53, 55, 90, 84; 39; 51, 48, 47).  The kernel with fp32 kernel values has smaller blocks: 40 x 72 of 56 x 75
     // 54 / 72, x 95 70 / 76, 16 x 40 of 90 x 79 33 / 29.
+    if (WORDS && Ws > WORDS && BY_WARP) {
+      // 2-byte copies, neighbours on neighbouring lanes, up to four loads in flight each.  Forward and grad-input at stride 1, large calls: word by
+      // word / so, us, 4 x 96 of 70 x 109 26.9, 29.1 / 24.3, 25.6, 2 x 240 of 64 x 103 30.7, 33.0 / 27.7, 28.1, 24 x 96 of 111 x 111 193, 198 / 187, 190 (grad-input
+      // of 32 x 48 of 99 x 99 117 / 126); the gradients of offsets and bank are faster word by word (16 x 32 of 100 x 99 141 / 151).
+      const int rows = r_e - r_s;
+      for (int t = warp; t < cnt * rows; t += nwarps) {
+        const int j = t / rows, r = r_s + (t - j * rows);
+        const __half* sp = s0 + (size_t)j * plane + (size_t)r * Ws + lane;
+        __half* dp = band + j * b.pitch_c + kSlack + (r * b.Wp - b.org) + lane;
+        for (int left = Ws - lane; left > 0; left -= 128, sp += 128, dp += 128) {
+          __half v[4];
+#pragma unroll
+          for (int k = 0; k < 4; ++k)
+            if (32 * k < left) v[k] = __ldg(sp + 32 * k);
+#pragma unroll
+          for (int k = 0; k < 4; ++k)
+            if (32 * k < left) dp[32 * k] = v[k];
+        }
+      }
+      return;
+    }
     if (WORDS && Ws > WORDS) {
       odd_rows(band + kSlack + (r_s * b.Wp - b.org), b.pitch_c, b.Wp, s0 + (size_t)r_s * Ws, plane, cnt, r_e - r_s, Ws, tid, nt);
       return;
@@ -284,12 +305,12 @@ __device__ __forceinline__ void flat_copies(__half* __restrict__ band, int pitch
 // leave lanes idle on the last pass over a row and walk through the channels one after the other.  Same instruction count
 // (measured), 3-4 % less time in the four kernels.
 // Odd row widths, and bands without a row inside the image, go through load_band_group.
-template <int WORDS>
+template <int WORDS, bool BY_WARP>
 __device__ __forceinline__ void load_band_flat(__half* __restrict__ band, const Band& b, const __half* __restrict__ src, int n,
                                                int C, int c0, int cnt, int Hs, int Ws, int tid, int nt, int bar_id) {
   const int r_s = max(b.row_lo, 0), r_e = min(b.row_lo + b.RB, Hs);
   if (b.mode == 0 || r_e <= r_s) {
-    load_band_group<WORDS>(band, b, src, n, C, c0, cnt, Hs, Ws, tid, nt, bar_id);
+    load_band_group<WORDS, BY_WARP>(band, b, src, n, C, c0, cnt, Hs, Ws, tid, nt, bar_id);
     return;
   }
   const size_t plane = (size_t)Hs * Ws;
@@ -320,10 +341,10 @@ __device__ __forceinline__ void load_band_flat(__half* __restrict__ band, const 
     }
   }
 }
-template <int WORDS = 96>
+template <int WORDS = 96, bool BY_WARP = false>
 __device__ __forceinline__ void load_band(__half* __restrict__ band, const Band& b, const __half* __restrict__ src, int n, int C,
                                           int c0, int cnt, int Hs, int Ws) {
-  load_band_flat<WORDS>(band, b, src, n, C, c0, cnt, Hs, Ws, threadIdx.x, blockDim.x, 0);
+  load_band_flat<WORDS, BY_WARP>(band, b, src, n, C, c0, cnt, Hs, Ws, threadIdx.x, blockDim.x, 0);
 }
 
 // Offset (in halves, even) of the window of pixel pair (ow, ow+1), row selector 0, inside a channel band.

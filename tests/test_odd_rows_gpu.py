@@ -1,4 +1,4 @@
-"""fp16 band kernels at stride 2 on rows of odd width from 71 to 97 columns, on either side of the line from which rows are copied word by word:
+"""fp16 band kernels, mostly at stride 2 on rows of odd width from 71 to 97 columns, on either side of the line from which rows are copied word by word:
 planes that start on an even or odd half, bands at both ends of a plane, blocks of one and of several slabs of channels."""
 import pytest
 import torch
@@ -14,13 +14,10 @@ def _odd_start(t):
     return buf[1:].view(t.shape).copy_(t)
 
 
-@pytest.mark.parametrize("n,c,h", [(2, 32, 9), (24, 96, 45), (3, 64, 100), (2, 40, 31)])
-@pytest.mark.parametrize("w", [71, 73, 75, 79, 89, 95, 97])
-@pytest.mark.parametrize("shifted", [False, True])
-def test_forward_and_gradients(n, c, h, w, shifted):
+def _check(n, c, h, w, stride, shifted):
     from deformable_kernels.ops.deform_kernel.functions import sample_depthwise
     from oracle import dk_oracle as O
-    case = make_case(n, c, h, w, stride=2, rot_std=0.7, seed=c + w)
+    case = make_case(n, c, h, w, stride=stride, rot_std=0.7, seed=c + w)
     x, r, k, dy = (case[name].half() for name in ("input", "rotation", "weight", "grad_output"))
     want = (O.sample_depthwise_forward(x.float(), r.float(), k.float(), **case["args"]),
             *O.sample_depthwise_backward(dy.float(), x.float(), r.float(), k.float(), **case["args"]))
@@ -31,3 +28,17 @@ def test_forward_and_gradients(n, c, h, w, shifted):
     y = sample_depthwise(*leaves, **case["args"])
     for name, g, v in zip(("output", "input", "rotation", "weight"), (y.detach(),) + torch.autograd.grad(y, leaves, dy), want):
         assert rel_err(g, v.half()) < 2e-3, name  # hat products, K and products with dy rounded to fp16, the result as well
+
+
+@pytest.mark.parametrize("n,c,h", [(2, 32, 9), (24, 96, 45), (3, 64, 100), (2, 40, 31)])
+@pytest.mark.parametrize("w", [71, 73, 75, 79, 89, 95, 97])
+@pytest.mark.parametrize("shifted", [False, True])
+def test_forward_and_gradients(n, c, h, w, shifted):
+    _check(n, c, h, w, 2, shifted)
+
+
+@pytest.mark.parametrize("n,c,h,w", [(3, 64, 75, 101), (2, 96, 60, 97), (7, 16, 99, 111), (1, 240, 61, 129)])
+@pytest.mark.parametrize("shifted", [False, True])
+def test_stride_1(n, c, h, w, shifted):
+    """Rows above 96 a warp each: calls that are not small."""
+    _check(n, c, h, w, 1, shifted)
