@@ -223,6 +223,7 @@ int local_conv_tc(const T* src, const T* rot, const T* w, T* dst, const Geom& g,
 // the same with kernel values rounded to fp16, in place of the mma.sync kernels only
 int local_conv_tc_rounded(const __half* src, const __half* rot, const __half* w, __half* dst, const Geom& g, bool transposed,
                           cudaStream_t s);
+double local_conv_mma_items(const Geom& g, bool transposed);  // of 8 pixels and 16 channels, per SM
 bool local_conv_mma_small(const Geom& g, bool transposed);  // and the call is so small that its block shape makes it the fastest one
 bool local_conv_mma_takes(const Geom& g, bool transposed);  // the band kernels have a block shape for this call
 int tc_error_status();

@@ -164,20 +164,31 @@ static int launch_local_conv(const T* src, const T* rot, const T* w, T* dst, con
     }
   }
   // fp32, and fp16 with channel counts that are no multiple of 16: those have always been computed with fp32 kernel values.  fp16 with
-  // tcgen05 where TMA fetches the rows and there are three 32-channel groups or more, else with mma.sync (us, forward + grad-input,
-  // tcgen05 / mma.sync: 32 x 72 of 56 x 56 63 / 77, 64 x 72 of 16 x 16 21 / 23, 4 x 952 of 24 x 24 27 / 31; 128 x 104 of 8 x 8 23 / 18, 16 x 24 of
-  // 64 x 64 38 / 31, 64 x 24 of 112 x 112 364 / 278; rows that TMA does not fetch, 2 x 200 of 50 x 60 48 / 27, 32 x 200 of 28 x 28 77 / 58, but
-  // grad-input of 32 x 72 of 56 x 56 at stride 2 25 / 28).
+  // tcgen05 where TMA fetches the rows and the lanes of its channel groups are full enough, else with mma.sync.  us, tcgen05 / mma.sync, taken: forward + grad-input
+  // of 32 x 72 of 56 x 56 63 / 77, 64 x 72 of 16 x 16 21 / 23, 4 x 952 of 24 x 24 27 / 31; grad-input at stride 2, where a lane's patch has four outputs
+  // and few channels are no loss, 32 x 24 of 112 x 112 28 / 62, 32 x 40 of 48 x 48 11 / 17, 32 x 72 of 56 x 56 25 / 28, 6 x 24 of 101 x 88 12 / 15.  Not
+  // taken: 128 x 104 of 8 x 8 23 / 18, 16 x 24 of 64 x 64 38 / 31, 64 x 24 of 112 x 112 364 / 278; rows that TMA does not fetch, 2 x 200 of
+  // 50 x 60 48 / 27, 32 x 200 of 28 x 28 77 / 58; forward at stride 2 beyond five groups (1.2 in the mean), with few items (1.35 below 60 per SM), and of two
+  // groups (32 x 56 of 112 x 112 31 / 41, taken) where they are half empty or the planes have odd heights (38 x 56 of 91 x 88 50 / 35); grad-input at
+  // stride 2 whose rows end on half a patch, 65 x 392 of 31 x 31 433 / 86.
   if constexpr (sizeof(T) <= 4) {
     const int Ws = TRANSPOSED ? g.Wo : g.W;
-    const bool rows = sizeof(T) == 4 || (g.C > 64 && ((Ws % 8 == 0 && Ws >= 16) || (TRANSPOSED && g.sW == 2 && Ws % 4 == 0 && Ws >= 28)));
+    bool rows = sizeof(T) == 4;
+    if (sizeof(T) == 2 && (g.C & 15)) {
+      const double items = local_conv_mma_items(g, TRANSPOSED);
+      if (TRANSPOSED && g.sW == 2) rows = g.W % 2 == 0 && ((Ws % 8 == 0 && items >= 40) || (Ws % 4 == 0 && Ws >= 28 && items >= 80));
+      else if (g.sW == 2) rows = g.C <= 136 && (g.C > 64 || (g.C >= 48 && g.H % 2 == 0)) && Ws % 8 == 0 && Ws >= 16 && items >= 60;
+      else rows = g.C > 64 && Ws % 8 == 0 && Ws >= 16;
+    }
     if (rows && mma_path_enabled()) {
       const int rc = local_conv_tc<T>(src, rot, w, dst, g, TRANSPOSED, s);
       if (rc != DK_ERR_UNSUPPORTED) return rc;
     }
   }
   if constexpr (std::is_same<T, __half>::value) {
-    if (mma_path_enabled() && (g.C & 15)) {
+    // half a slab, and rows that pass through registers: gathered cells (stride 1, mma.sync -> these, 61 x 8 of 45 x 41 29 -> 21 us, 49 x 8 of 99 x 91 91 -> 75)
+    const bool few = g.C <= 8 && ((TRANSPOSED ? g.Wo : g.W) & 1) && g.sW == 1 && local_conv_mma_items(g, TRANSPOSED) >= 24;
+    if (mma_path_enabled() && (g.C & 15) && !few) {
       const int rc = local_conv_mma(src, rot, w, dst, g, TRANSPOSED, s);
       if (rc != DK_ERR_UNSUPPORTED) return rc;
     }

@@ -27,6 +27,11 @@
 
 namespace dk {
 
+double local_conv_mma_items(const Geom& g, bool transposed) {
+  const int Hd = transposed ? g.H : g.Ho, Wd = transposed ? g.W : g.Wo;
+  return (double)g.N * Hd * ((Wd + 7) / 8) * ((g.C + 15) / 16) / 148;
+}
+
 using namespace mma;
 
 namespace {
@@ -454,10 +459,12 @@ size_t conv_smem(const Geom& g, bool transposed, int cg, int bh) {
 // 32 x 112 x 112 (21) 7.1 -> 6.3, 10 x 96 of 30 x 36 at stride 2 (18) 7.9 -> 6.6, odd rows 24 x 40 of 15 x 15 (15) 9.3 -> 7.0.  Above it some gain and some
 // lose: 7 x 176 of 20 x 20 (31) 8.3 -> 6.1, 12 x 112 of 20 x 22 (34) 8.4 -> 9.3, 43 x 48 of 28 x 18 (73) 9.6 -> 12.0, grad-input of 64 x 96 x 96 at stride
 // 2 (31) 7.5 -> 8.3, odd rows 6 x 24 of 50 x 51 (28) 15 -> 21.
+// In fp32 arithmetic (channels outside a multiple of 16) the block shape for large calls loses until 30 items, whatever the rows: forward of 16 x 104 of
+// 28 x 27 at stride 2 (21) 14.4 -> 7.5 us, 51 x 72 of 16 x 23 at stride 2 (28) 15.2 -> 9.5; in the mean of 700 calls 0.98 at 20 to 24 items, 0.88 at
+// 24 to 30, 1.05 at 30 to 40; grad-input at stride 2 0.81, 0.94, 1.05.
 bool small_conv(const Geom& g, bool transposed) {
-  const int Hd = transposed ? g.H : g.Ho, Wd = transposed ? g.W : g.Wo;
-  const int most = (transposed ? g.Wo : g.W) & 1 ? 20 : 24;
-  return (long long)g.N * Hd * ((Wd + 7) / 8) * ((g.C + 15) / 16) <= 148LL * most;
+  const int most = g.C & 15 ? (transposed && g.sH == 2 ? 24 : 30) : (transposed ? g.Wo : g.W) & 1 ? 20 : 24;
+  return local_conv_mma_items(g, transposed) <= most;
 }
 
 // A small call is a chain of latencies: the loads of a band one after the other (rows of odd width pass through

@@ -42,3 +42,9 @@ def test_forward_and_gradients(n, c, h, w, shifted):
 def test_stride_1(n, c, h, w, shifted):
     """Rows above 96 a warp each: calls that are not small."""
     _check(n, c, h, w, 1, shifted)
+
+
+@pytest.mark.parametrize("n,c,h,w,stride", [(61, 8, 45, 41, 1), (6, 24, 64, 64, 2), (2, 40, 110, 112, 2), (3, 56, 96, 104, 2), (4, 24, 62, 62, 2), (9, 72, 33, 40, 2)])
+def test_calls_between_the_kernels(n, c, h, w, stride):
+    """Channels outside a multiple of 16: few of them on odd rows, and grad-input at stride 2 with full, half and no patches at the ends of its rows."""
+    _check(n, c, h, w, stride, False)
