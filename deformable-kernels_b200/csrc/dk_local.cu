@@ -131,12 +131,17 @@ static int launch_local_conv_simt(const T* src, const T* rot, const T* w, T* dst
 template <typename T, bool TRANSPOSED>
 static int launch_local_conv(const T* src, const T* rot, const T* w, T* dst, const Geom& g, cudaStream_t s) {
   using A = typename Compute<T>::type;
+  // half a slab, and rows that pass through registers: gathered cells (mma.sync -> these, us, 61 x 8 of 45 x 41 29 -> 21, 49 x 8 of 99 x 91 91 -> 75; at
+  // stride 2, forward of 91 x 8 of 67 x 47 17 -> 14, of 128 x 8 of 17 x 17 11 -> 9, grad-input of 12 x 8 of 79 x 109 35 -> 19; not 110 x 8 of 67 x 66
+  // 68 -> 77)
+  const int fewest = g.sW == 1 ? 24 : 15;
+  const bool few = g.C <= 8 && (g.W & 1) && (!TRANSPOSED || (g.Wo & 1)) && (!TRANSPOSED || g.sW == 1 || (g.H & 1)) && local_conv_mma_items(g, TRANSPOSED) >= fewest;
   if constexpr (std::is_same<T, __half>::value) {
     if (mma_path_enabled()) {
       int rc = DK_ERR_UNSUPPORTED;
       // small calls: the band kernels in their own block shape, against the ring and tcgen05 kernels (192 x 28 x 28, forward and grad-input,
       // 10.4, 9.8 -> 4.8, 4.2 us; 160 x 32 x 32 8.5, 7.9 -> 4.6, 4.2; 72 x 64 x 64 9.3, 8.9 -> 6.7, 5.9)
-      if (local_conv_mma_small(g, TRANSPOSED)) {
+      if (!few && local_conv_mma_small(g, TRANSPOSED)) {
         rc = local_conv_mma(src, rot, w, dst, g, TRANSPOSED, s);
         if (rc != DK_ERR_UNSUPPORTED) return rc;
       }
@@ -168,16 +173,17 @@ static int launch_local_conv(const T* src, const T* rot, const T* w, T* dst, con
   // of 32 x 72 of 56 x 56 63 / 77, 64 x 72 of 16 x 16 21 / 23, 4 x 952 of 24 x 24 27 / 31; grad-input at stride 2, where a lane's patch has four outputs
   // and few channels are no loss, 32 x 24 of 112 x 112 28 / 62, 32 x 40 of 48 x 48 11 / 17, 32 x 72 of 56 x 56 25 / 28, 6 x 24 of 101 x 88 12 / 15.  Not
   // taken: 128 x 104 of 8 x 8 23 / 18, 16 x 24 of 64 x 64 38 / 31, 64 x 24 of 112 x 112 364 / 278; rows that TMA does not fetch, 2 x 200 of
-  // 50 x 60 48 / 27, 32 x 200 of 28 x 28 77 / 58; forward at stride 2 beyond five groups (1.2 in the mean), with few items (1.35 below 60 per SM), and of two
-  // groups (32 x 56 of 112 x 112 31 / 41, taken) where they are half empty or the planes have odd heights (38 x 56 of 91 x 88 50 / 35); grad-input at
-  // stride 2 whose rows end on half a patch, 65 x 392 of 31 x 31 433 / 86.
+  // 50 x 60 48 / 27, 32 x 200 of 28 x 28 77 / 58; forward at stride 2 of more than five groups on rows of 112 or 16 (11 x 232 of 95 x 112 67 / 47, 128 x 296 of
+  // 15 x 16 26 / 17; rows between 1.02 in the mean), with few items (1.35 below 60 per SM), and of two groups (32 x 56 of 112 x 112 31 / 41, taken) where
+  // they are half empty or the planes have odd heights (38 x 56 of 91 x 88 50 / 35); grad-input at stride 2 whose rows end on half a patch, 65 x 392
+  // of 31 x 31 433 / 86 (with 8 channels 128 x 8 of 37 x 47 25 / 37, taken).
   if constexpr (sizeof(T) <= 4) {
     const int Ws = TRANSPOSED ? g.Wo : g.W;
     bool rows = sizeof(T) == 4;
     if (sizeof(T) == 2 && (g.C & 15)) {
       const double items = local_conv_mma_items(g, TRANSPOSED);
-      if (TRANSPOSED && g.sW == 2) rows = g.W % 2 == 0 && ((Ws % 8 == 0 && items >= 40) || (Ws % 4 == 0 && Ws >= 28 && items >= 80));
-      else if (g.sW == 2) rows = g.C <= 136 && (g.C > 64 || (g.C >= 48 && g.H % 2 == 0)) && Ws % 8 == 0 && Ws >= 16 && items >= 60;
+      if (TRANSPOSED && g.sW == 2) rows = (g.W % 2 == 0 || g.C <= 8) && ((Ws % 8 == 0 && items >= 40) || (Ws % 4 == 0 && Ws >= 28 && items >= 80));
+      else if (g.sW == 2) rows = (g.C > 64 || (g.C >= 48 && g.H % 2 == 0)) && Ws % 8 == 0 && Ws >= (g.C > 136 ? 24 : 16) && (g.C <= 136 || Ws <= 96) && items >= 60;
       else rows = g.C > 64 && Ws % 8 == 0 && Ws >= 16;
     }
     if (rows && mma_path_enabled()) {
@@ -186,8 +192,6 @@ static int launch_local_conv(const T* src, const T* rot, const T* w, T* dst, con
     }
   }
   if constexpr (std::is_same<T, __half>::value) {
-    // half a slab, and rows that pass through registers: gathered cells (stride 1, mma.sync -> these, 61 x 8 of 45 x 41 29 -> 21 us, 49 x 8 of 99 x 91 91 -> 75)
-    const bool few = g.C <= 8 && ((TRANSPOSED ? g.Wo : g.W) & 1) && g.sW == 1 && local_conv_mma_items(g, TRANSPOSED) >= 24;
     if (mma_path_enabled() && (g.C & 15) && !few) {
       const int rc = local_conv_mma(src, rot, w, dst, g, TRANSPOSED, s);
       if (rc != DK_ERR_UNSUPPORTED) return rc;

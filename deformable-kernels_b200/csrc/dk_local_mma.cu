@@ -460,7 +460,7 @@ size_t conv_smem(const Geom& g, bool transposed, int cg, int bh) {
 // lose: 7 x 176 of 20 x 20 (31) 8.3 -> 6.1, 12 x 112 of 20 x 22 (34) 8.4 -> 9.3, 43 x 48 of 28 x 18 (73) 9.6 -> 12.0, grad-input of 64 x 96 x 96 at stride
 // 2 (31) 7.5 -> 8.3, odd rows 6 x 24 of 50 x 51 (28) 15 -> 21.
 // In fp32 arithmetic (channels outside a multiple of 16) the block shape for large calls loses until 30 items, whatever the rows: forward of 16 x 104 of
-// 28 x 27 at stride 2 (21) 14.4 -> 7.5 us, 51 x 72 of 16 x 23 at stride 2 (28) 15.2 -> 9.5; in the mean of 700 calls 0.98 at 20 to 24 items, 0.88 at
+// 28 x 27 at stride 2 (21) 14.4 -> 11.8 us, 51 x 72 of 16 x 23 at stride 2 (28) 15.2 -> 9.6; in the mean of 700 calls 0.98 at 20 to 24 items, 0.88 at
 // 24 to 30, 1.05 at 30 to 40; grad-input at stride 2 0.81, 0.94, 1.05.
 bool small_conv(const Geom& g, bool transposed) {
   const int most = g.C & 15 ? (transposed && g.sH == 2 ? 24 : 30) : (transposed ? g.Wo : g.W) & 1 ? 20 : 24;
@@ -471,7 +471,8 @@ bool small_conv(const Geom& g, bool transposed) {
 // registers, eight halves a trip), then the hat products of a warp's items and their slabs; the warps of a scheduler and the blocks of
 // an SM add what they issue.  Few channels a block, and one item a warp, shorten the chain as long as each SM has one block.  The weights
 // are us, from 384 x 14 x 14 (channels / rows / warps: 16/4/8 4.0, 32/4/8 4.6, 96/4/8 6.8, 16/4/6 4.7, 16/7/14 4.6, 16/2/4 with 168 blocks 4.3),
-// 960 x 7 x 7 (16/4/4 4.4, 16/2/2 with 240 blocks 5.0) and 3 x 56 of 16 x 17 (16/2/6 5.6, 64/2/6 8.0).
+// 960 x 7 x 7 (16/4/4 4.4, 16/2/2 with 240 blocks 5.0) and 3 x 56 of 16 x 17 (16/2/6 5.6, 64/2/6 8.0).  Blocks that share an SM wait for some of each
+// other's loads (128 x 48 of 8 x 8, forward and grad-input, 6.2 and 6.0 without that term, 5.0 and 5.1 with it).
 void small_conv_plan(const Geom& g, bool transposed, bool full, size_t budget, ConvPlan& pl) {
   const int S = g.sH, Hd = transposed ? g.H : g.Ho, Wd = transposed ? g.W : g.Wo, Hs = transposed ? g.Ho : g.H, Ws = transposed ? g.Wo : g.W;
   const int NB = (Wd + 7) / 8, slabs_all = (g.C + 15) / 16, most = full ? 8 : 14;
@@ -492,7 +493,7 @@ void small_conv_plan(const Geom& g, bool transposed, bool full, size_t budget, C
         const double load = 0.27 * (trips(cg, min(rb, Hs), Ws) + trips(18, min(rot_rows, g.Ho), g.Wo)) + 0.1 * (cg * 16 / threads);
         const double chain = rounds * (0.1 + 0.55 * slabs);
         const double issue = (per_sm * ((w + 3) / 4) - 1) * rounds * ((full ? 0.25 : 0.13) + 0.115 * slabs);
-        const double cost = load + chain + issue + 0.3 * (per_sm - 1);
+        const double cost = load + chain + issue + (0.3 + (full ? 0.0 : 0.15 * load)) * (per_sm - 1);
         if (cost < best) {
           best = cost;
           pl.BH = bh, pl.CG = cg, pl.groups = groups, pl.warps = w;
