@@ -13,8 +13,8 @@
 // bank value that is not finite reach the channel 32 away), and the columns 2 t, 2 t + 1 of tile j are the channels 8 t + 2 j, + 1.  mma.sync,
 // because its results are needed in registers beside the gathered values.
 //
-// 64 x 256 of 56 x 56, forward and backward 3384 -> 1342 us: lines 35 and 65, forward 300, sort 56, gather 290, offsets and bank
-// 590.  Forward: load pipe 69 % (64 of its 109 passes per 16 pixels, tap and 64 channels are the corners, 44 % of the
+// 64 x 256 of 56 x 56, forward and backward 3384 -> 1324 us: lines 35 and 65, forward 300, sort 56, gather 290, offsets and bank
+// 573.  Forward: load pipe 69 % (64 of its 109 passes per 16 pixels, tap and 64 channels are the corners, 44 % of the
 // rest misses and offsets), 2.8 warps per scheduler at 168 registers; 8 loads in flight instead of 16 with 16 warps instead of
 // 12 takes as long.  Offsets and bank: load pipe 46 %, tensor pipe 33 %, issue 44 %, the half-rate fp16 pipe with 14 instructions where the tensor
 // pipe has 10: latency at twelve warps of an SM in three blocks, which the 64 registers of bank sums and bank operands leave.  Gather: load pipe
@@ -457,11 +457,11 @@ __global__ void __launch_bounds__(128, 3) line_forward_kernel(const __half* __re
 // the differences of neighbouring corners, an mma of the products whose other operand is one in the columns k, k + 4; a pixel's two rows are its two
 // halves of the channels.  Products with the corners themselves, subtracted afterwards, overflow where only the corners are large (x of 100, dy
 // of 500) and lose what they have in common: 8 x 512 of 28 x 28 with x around 10, 1.1e-3 off fp64 against 4.5e-4 (4.6e-4 and 5.1e-4 around 0).
-// 543 -> 590 us for the differences.  dW = beta^T (dy xs) over the pixels, for which movmatrix turns the products.
+// 543 -> 590 us for the differences, 573 with runs of tiles as equal as they can be.  dW = beta^T (dy xs) over the pixels, for which movmatrix turns the products.
 // A warp has 64 channels for the whole run of its block (the bank sums stay in registers) and walks over groups of 16 pixels;
 // the warps of a stream have different channels of the same pixels, and their sums over channels meet in shared memory.
 struct CoordPlan {
-  int units, upb, streams, sets, tiles, per_block, blocks;  // units of channels, of a block; groups of pixels of a block; channel sets
+  int units, upb, streams, sets, tiles, blocks;  // units of channels, of a block; groups of pixels of a block; channel sets
   size_t smem;
 };
 constexpr int kGridRow = 6, kGridNone = 36, kGridCells = 44, kGridPitch = 16;  // 6 x 6 cells with a border of zeros, and zeros behind; 16 pixels
@@ -519,8 +519,8 @@ __global__ void __launch_bounds__(128, 3) line_coords_kernel(const __half* __res
   const int my_px = threadIdx.x & (npx - 1), tap0 = threadIdx.x / npx, taps_step = blockDim.x / npx;  // npx is a power of two
   // the hat products turned: the two k-slots of a lane are the pixels 4 t, + 1 and 4 t + 2, + 3
   const int trow = stream * 16 + ((lane & 1) + 2 * (lane >> 4)) * 4 + ((lane & 7) >> 1);
-  const int tile_end = min((int)((blockIdx.x + 1) * pl.per_block), pl.tiles);
-  for (int tile = blockIdx.x * pl.per_block; tile < tile_end; ++tile) {
+  const int tile_end = (int)((long long)pl.tiles * (blockIdx.x + 1) / pl.blocks);
+  for (int tile = (int)((long long)pl.tiles * blockIdx.x / pl.blocks); tile < tile_end; ++tile) {
     const int f0 = tile * npx, flip = tile & 1;
     {
       const int f = f0 + my_px;
@@ -1117,8 +1117,10 @@ void line_plan(const Geom& g, LinePlan& p) {
   int blocks = 3 * sms / c.sets;
   if (blocks < 1) blocks = 1;
   if (blocks > c.tiles) blocks = c.tiles;
-  c.per_block = (c.tiles + blocks - 1) / blocks;
-  c.blocks = (c.tiles + c.per_block - 1) / c.per_block;
+  // runs of equal length up to one; short ones take the fewest blocks that are no slower, each lays down bank sums (64 x 256 of 56 x 56, runs of 28 and 29
+  // instead of 29: 1341 -> 1324 us; 128 x 160 of 8 x 7, runs of 1 and 2 instead of 2: 99.8 -> 102.4)
+  const int run = (c.tiles + blocks - 1) / blocks;
+  c.blocks = run >= 8 ? blocks : (c.tiles + run - 1) / run;
   const int warps = c.upb * c.streams;
   c.smem = (size_t)kLineTaps * npx * 76 + npx * 12 + (size_t)c.upb * 2048 + (size_t)warps * (kLineTaps * 160 + kGridCells * kGridPitch) * 4;
   const size_t red = (size_t)warps * 1024 * 4;
